@@ -145,12 +145,12 @@ class GPT2:
             P = lambda n: p[f"h{l}.{n}"]
             qkv = buf(("qkv", l), (T, 3 * C))
             gemm.linear(ln_in, P("w_qkv"), P("b_qkv"), out=qkv)
-            qkv_leaf = qkv.detach().requires_grad_(not loss_only)
+            q, k, v = (t.requires_grad_(not loss_only) for t in qkv.detach().view(B, S, 3, H, D).permute(2, 0, 3, 1, 4).unbind(0))
             with torch.enable_grad():
-                q, k, v = qkv_leaf.view(B, S, 3, H, D).permute(2, 0, 3, 1, 4).unbind(0)
-                att = F.scaled_dot_product_attention(q, k, v, is_causal=True).transpose(1, 2).reshape(T, C)
+                att4 = F.scaled_dot_product_attention(q, k, v, is_causal=True)
+            att = att4.detach().transpose(1, 2).reshape(T, C)
             a = buf("a", (T, C))
-            gemm.linear(att.detach(), P("w_o"), P("b_o"), out=a)
+            gemm.linear(att, P("w_o"), P("b_o"), out=a)
             x2, ln2 = buf(("x2", l), (T, C)), buf(("ln2", l), (T, C))
             mean2, rstd2 = buf(("mean2", l), (T,), f32), buf(("rstd2", l), (T,), f32)
             ops.layernorm_fwd(a, xin, P("ln2_g"), P("ln2_b"), x2, ln2, mean2, rstd2, cfg.ln_eps)
@@ -165,7 +165,7 @@ class GPT2:
                 ops.layernorm_fwd(pr, x2, p[f"h{l + 1}.ln1_g"], p[f"h{l + 1}.ln1_b"], x3, nxt, nmean, nrstd, cfg.ln_eps)
             else:
                 ops.layernorm_fwd(pr, x2, p["lnf_g"], p["lnf_b"], x3, nxt, nmean, nrstd, cfg.ln_eps)
-            saved.append((xin, ln_in, mean1, rstd1, qkv_leaf, att, x2, ln2, mean2, rstd2, h, gl))
+            saved.append((xin, ln_in, mean1, rstd1, (q, k, v, att4), att, x2, ln2, mean2, rstd2, h, gl))
             xin, ln_in, mean1, rstd1 = x3, nxt, nmean, nrstd
 
         logits = buf("logits", (T, cfg.padded_vocab))
@@ -182,36 +182,45 @@ class GPT2:
         dln = buf("dlnf", (T, C))
         gemm.grad_input(logits, p["wte"], out=dln)
         dx = buf("dx_a", (T, C))
-        ops.layernorm_bwd(dln, xin, p["lnf_g"], mean1, rstd1, None, dx, g["lnf_g"], g["lnf_b"])
+        # Bias, gamma and beta gradients are column sums of tensors that some kernel below holds in registers: each leaves partial rows
+        # in fp32, one launch per layer folds the partial rows of all eight vectors.
+        n_ln, n_fc, n_qkv = ops.layernorm_bwd_parts(T, C), ops.col_parts(T, 4 * C), ops.col_parts(T, 3 * C)
+        ws = buf("parts", (6 * n_ln * C + n_fc * 4 * C + n_qkv * 3 * C,), f32).data_ptr()
+        row = 4 * n_ln * C                                     # bytes of one vector's partial rows
+        ws1, ws_fc, ws_qkv = ws + 3 * row, ws + 6 * row, ws + 6 * row + 16 * n_fc * C
+        ops.layernorm_bwd_partial(dln, xin, p["lnf_g"], mean1, rstd1, None, dx, ws1, True)
+        ops.finish_parts([(ws1, n_ln, g["lnf_g"], False), (ws1 + row, n_ln, g["lnf_b"], False), (ws1 + 2 * row, n_ln, g[f"h{L - 1}.b_proj"], False)])
         ready(self.offset["lnf_b"][1])
         for l in reversed(range(L)):
             P = lambda n: p[f"h{l}.{n}"]
             G = lambda n: g[f"h{l}.{n}"]
-            xin_l, ln1_l, m1, r1, qkv_leaf, att, x2, ln2, m2, r2, h, gl = saved[l]
+            xin_l, ln1_l, m1, r1, (q, k, v, att4), att, x2, ln2, m2, r2, h, gl = saved[l]
             # x3 = x2 + gelu(ln2 @ Wfc + bfc) @ Wproj + bproj
-            ops.colsum(dx, G("b_proj"))
             gemm.grad_weight(dx, gl, out=G("w_proj"))
             dg = buf("dg", (T, 4 * C))
             gemm.grad_input(dx, P("w_proj"), out=dg)
-            ops.gelu_bwd(dg, h, dg)
-            ops.colsum(dg, G("b_fc"))
+            ops.gelu_bwd(dg, h, dg, ws_fc)
             gemm.grad_weight(dg, ln2, out=G("w_fc"))
             dln2 = buf("dln2", (T, C))
             gemm.grad_input(dg, P("w_fc"), out=dln2)
             dx2 = buf("dx_b", (T, C))
-            ops.layernorm_bwd(dln2, x2, P("ln2_g"), m2, r2, dx, dx2, G("ln2_g"), G("ln2_b"))
+            ops.layernorm_bwd_partial(dln2, x2, P("ln2_g"), m2, r2, dx, dx2, ws, True)
             # x2 = xin + att @ Wo + bo
-            ops.colsum(dx2, G("b_o"))
-            gemm.grad_weight(dx2, att.detach(), out=G("w_o"))
+            gemm.grad_weight(dx2, att, out=G("w_o"))
             datt = buf("datt", (T, C))
             gemm.grad_input(dx2, P("w_o"), out=datt)
-            (dqkv,) = torch.autograd.grad(att, qkv_leaf, datt)
-            dqkv = dqkv.reshape(T, 3 * C)
-            ops.colsum(dqkv, G("b_qkv"))
+            grads = torch.autograd.grad(att4, (q, k, v), datt.view(B, S, H, D).transpose(1, 2))
+            dqkv = buf("dqkv", (T, 3 * C))
+            ops.qkv_grad(*grads, dqkv, ws_qkv)
             gemm.grad_weight(dqkv, ln1_l, out=G("w_qkv"))
             dln1 = buf("dln1", (T, C))
             gemm.grad_input(dqkv, P("w_qkv"), out=dln1)
-            ops.layernorm_bwd(dln1, xin_l, P("ln1_g"), m1, r1, dx2, dx, G("ln1_g"), G("ln1_b"))
+            ops.layernorm_bwd_partial(dln1, xin_l, P("ln1_g"), m1, r1, dx2, dx, ws1, l > 0)
+            jobs = [(ws, n_ln, G("ln2_g"), False), (ws + row, n_ln, G("ln2_b"), False), (ws + 2 * row, n_ln, G("b_o"), False), (ws_fc, n_fc, G("b_fc"), False),
+                    (ws_qkv, n_qkv, G("b_qkv"), False), (ws1, n_ln, G("ln1_g"), False), (ws1 + row, n_ln, G("ln1_b"), False)]
+            if l > 0:
+                jobs.append((ws1 + 2 * row, n_ln, g[f"h{l - 1}.b_proj"], False))
+            ops.finish_parts(jobs)
             ready(self.offset[f"h{l}.b_proj"][1])
         ops.wpe_bwd(dx, g["wpe"], B, S)
         ready(self.offset["wpe"][1])

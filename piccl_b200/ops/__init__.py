@@ -58,14 +58,35 @@ def layernorm_fwd(x, res, gamma, beta, sum_out, y, mean, rstd, eps: float = 1e-5
     _bump()
 
 
-def layernorm_bwd(dy, xin, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate: bool = False, rows_per_block: int = 32):
+class _FinishJob(C.Structure):
+    _fields_ = [("part", C.c_void_p), ("out", C.c_void_p), ("nparts", C.c_int), ("C", C.c_int), ("accumulate", C.c_int), ("pad", C.c_int)]
+
+
+def finish_parts(jobs) -> None:
+    """jobs: up to 16 tuples (address of fp32 partial rows, number of rows, bf16 output vector, accumulate): out (+)= sum of the rows."""
+    arr = (_FinishJob * len(jobs))(*[(p, o.data_ptr(), n, o.numel(), int(acc), 0) for p, n, o, acc in jobs])
+    _chk(N.ops_lib().piccl_ops_finish_parts(arr, len(jobs), C.c_void_p(_s())), "finish_parts")
+    _bump()
+
+
+def layernorm_bwd_parts(rows: int, cols: int) -> int:
+    return N.ops_lib().piccl_ops_ln_bwd_parts(rows, cols)
+
+
+def layernorm_bwd_partial(dy, xin, gamma, mean, rstd, dres, dx, part: int, with_dsum: bool) -> None:
+    """dx = dLN(dy) + dres; partial rows of dgamma, dbeta (and of the column sum of dx) at address `part`: [2 or 3][layernorm_bwd_parts][C] floats."""
+    rows, Cc = dy.shape
+    _chk(N.ops_lib().piccl_ops_ln_bwd(_p(dy), _p(xin), _p(gamma), _p(mean), _p(rstd), _p(dres), _p(dx), C.c_void_p(part), int(with_dsum), rows, Cc, C.c_void_p(_s())), "ln_bwd")
+    _bump()
+
+
+def layernorm_bwd(dy, xin, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate: bool = False):
     """dx = dLN(dy) + dres; dgamma / dbeta (bf16) written or accumulated."""
     rows, Cc = dy.shape
-    nblocks = (rows + rows_per_block - 1) // rows_per_block
-    ws = _workspace(2 * nblocks * Cc, dy.device)
-    _chk(N.ops_lib().piccl_ops_ln_bwd(_p(dy), _p(xin), _p(gamma), _p(mean), _p(rstd), _p(dres), _p(dx), _p(dgamma), _p(dbeta), _p(ws), rows, Cc,
-                                      rows_per_block, int(accumulate), C.c_void_p(_s())), "ln_bwd")
-    _bump(3)
+    n = layernorm_bwd_parts(rows, Cc)
+    ws = _workspace(2 * max(n, 1) * Cc, dy.device)
+    layernorm_bwd_partial(dy, xin, gamma, mean, rstd, dres, dx, ws.data_ptr(), False)
+    finish_parts([(ws.data_ptr(), n, dgamma, accumulate), (ws.data_ptr() + 4 * n * Cc, n, dbeta, accumulate)])
 
 
 def bias_gelu_fwd(h, bias, h_out, g):
@@ -74,8 +95,25 @@ def bias_gelu_fwd(h, bias, h_out, g):
     _bump()
 
 
-def gelu_bwd(dg, h, dh):
-    _chk(N.ops_lib().piccl_ops_gelu_bwd(_p(dg), _p(h), _p(dh), C.c_longlong(dg.numel()), C.c_void_p(_s())), "gelu_bwd")
+def col_parts(rows: int, cols: int) -> int:
+    """Partial rows that gelu_bwd and qkv_grad leave."""
+    return N.ops_lib().piccl_ops_col_parts(C.c_longlong(rows), cols)
+
+
+def gelu_bwd(dg, h, dh, part: int = 0):
+    """dh = dg * gelu'(h); part: address of col_parts(*h.shape) * h.shape[1] floats for partial column sums of dh (0: none)."""
+    rows, Cc = h.shape
+    _chk(N.ops_lib().piccl_ops_gelu_bwd(_p(dg), _p(h), _p(dh), C.c_void_p(part), C.c_longlong(rows), Cc, C.c_void_p(_s())), "gelu_bwd")
+    _bump()
+
+
+def qkv_grad(dq, dk, dv, dqkv, part: int):
+    """dqkv[b * S + s, (which, head, d)] from the [B, H, S, D] gradients of the attention, with partial column sums at address `part`."""
+    B, H, S, D = dq.shape
+    ptrs = (C.c_void_p * 3)(dq.data_ptr(), dk.data_ptr(), dv.data_ptr())
+    st = (C.c_longlong * 9)(*[t.stride(i) for t in (dq, dk, dv) for i in (0, 1, 2)])
+    assert dq.stride(3) == dk.stride(3) == dv.stride(3) == 1
+    _chk(N.ops_lib().piccl_ops_qkv_grad(ptrs, st, _p(dqkv), C.c_void_p(part), B, S, H, D, C.c_void_p(_s())), "qkv_grad")
     _bump()
 
 

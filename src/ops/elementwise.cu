@@ -1,9 +1,26 @@
 // Fused element-wise model kernels: bias + GELU (forward / backward), bias
 // gradient (column sums), softmax cross entropy with in-place gradient, and a
 // flat AdamW step with fp32 master weights.
+#include <cstring>
 #include "ops_common.cuh"
 
 namespace piccl_ops {
+
+// The 8 warps of a block hold sums of columns [blockIdx.x * 256, + 256), 8 to a lane: their total is row blockIdx.y of part[][C].
+__device__ __forceinline__ void block_colsum(const float (&acc)[8], float* __restrict__ part, int C) {
+  __shared__ float sh[8][256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int e = 0; e < 8; e++) sh[warp][lane * 8 + e] = acc[e];
+  __syncthreads();
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c < C) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) s += sh[w][threadIdx.x];
+    part[(size_t)blockIdx.y * C + c] = s;
+  }
+}
 
 // g = gelu(h + bias); h_out = h + bias (kept for the backward pass); h may alias h_out
 __global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const bf16* __restrict__ h, const bf16* __restrict__ bias, bf16* __restrict__ h_out,
@@ -21,16 +38,69 @@ __global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const bf16* __restri
   }
 }
 
-// dh = dg * gelu'(h)    (h includes the bias); dh may alias dg
-__global__ void __launch_bounds__(256) gelu_bwd_kernel(const bf16* __restrict__ dg, const bf16* __restrict__ h, bf16* __restrict__ dh, size_t n8) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
-    float d[8], v[8], o[8];
-    unpack8(reinterpret_cast<const bf16x8*>(dg)[i], d);
-    unpack8(reinterpret_cast<const bf16x8*>(h)[i], v);
+// dh = dg * gelu'(h)    (h includes the bias); dh may alias dg.  Block (bx, by): 256 columns, every gridDim.y-th group of 8 rows.
+// part (optional): [gridDim.y][C] column sums of the dh written, the bias gradient of the layer, taken while the rows are in
+// registers instead of by a second pass over dh.
+constexpr int kColRows = 4;      // rows in flight per warp
+__global__ void __launch_bounds__(256) gelu_bwd_kernel(const bf16* __restrict__ dg, const bf16* __restrict__ h, bf16* __restrict__ dh, float* __restrict__ part,
+                                                       long long rows, int C) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c8 = blockIdx.x * 32 + lane, C8 = C / 8;
+  float acc[8];
 #pragma unroll
-    for (int e = 0; e < 8; e++) o[e] = d[e] * gelu_grad_f(v[e]);
-    reinterpret_cast<bf16x8*>(dh)[i] = pack8(o);
+  for (int e = 0; e < 8; e++) acc[e] = 0.f;
+  if (c8 < C8)
+    for (long long r0 = (blockIdx.y * 8ll + warp) * kColRows; r0 < rows; r0 += gridDim.y * 8ll * kColRows) {
+      bf16x8 pd[kColRows], ph[kColRows];
+#pragma unroll
+      for (int r = 0; r < kColRows; r++)
+        if (r0 + r < rows) { const size_t i = (size_t)(r0 + r) * C8 + c8; pd[r] = reinterpret_cast<const bf16x8*>(dg)[i]; ph[r] = reinterpret_cast<const bf16x8*>(h)[i]; }
+#pragma unroll
+      for (int r = 0; r < kColRows; r++)
+        if (r0 + r < rows) {
+          float d[8], v[8];
+          unpack8(pd[r], d); unpack8(ph[r], v);
+#pragma unroll
+          for (int e = 0; e < 8; e++) d[e] *= gelu_grad_f(v[e]);
+          const bf16x8 p = pack8(d);
+          reinterpret_cast<bf16x8*>(dh)[(size_t)(r0 + r) * C8 + c8] = p;
+          unpack8(p, d);
+#pragma unroll
+          for (int e = 0; e < 8; e++) acc[e] += d[e];
+        }
+    }
+  if (part) block_colsum(acc, part, C);
+}
+
+// dqkv[b * S + s, which * H * D + head * D + d] from the three gradients of the attention, which lie as [B, H, S, D] views with
+// strides sb / sh / ss (elements) and contiguous rows of D; part: [gridDim.y][3 * H * D] column sums of what is written.
+struct QkvGrads { const bf16* p[3]; long long sb[3], sh[3], ss[3]; };
+__global__ void __launch_bounds__(256) qkv_grad_kernel(const QkvGrads q, bf16* __restrict__ dqkv, float* __restrict__ part, int rows, int S, int H, int D) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = H * D, C3 = 3 * C;
+  const int c = (blockIdx.x * 32 + lane) * 8;
+  float acc[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) acc[e] = 0.f;
+  if (c < C3) {
+    const int which = c / C, head = (c - which * C) / D, d = c - which * C - head * D;
+    const bf16* src = (which == 0 ? q.p[0] : which == 1 ? q.p[1] : q.p[2]) + d + head * (which == 0 ? q.sh[0] : which == 1 ? q.sh[1] : q.sh[2]);
+    const long long sb = which == 0 ? q.sb[0] : which == 1 ? q.sb[1] : q.sb[2], ss = which == 0 ? q.ss[0] : which == 1 ? q.ss[1] : q.ss[2];
+    for (int r0 = (blockIdx.y * 8 + warp) * kColRows; r0 < rows; r0 += gridDim.y * 8 * kColRows) {
+      bf16x8 v[kColRows];
+#pragma unroll
+      for (int r = 0; r < kColRows; r++)
+        if (r0 + r < rows) { const int b = (r0 + r) / S, s = (r0 + r) - b * S; v[r] = *reinterpret_cast<const bf16x8*>(src + b * sb + s * ss); }
+#pragma unroll
+      for (int r = 0; r < kColRows; r++)
+        if (r0 + r < rows) {
+          *reinterpret_cast<bf16x8*>(dqkv + (size_t)(r0 + r) * C3 + c) = v[r];
+          float f[8]; unpack8(v[r], f);
+#pragma unroll
+          for (int e = 0; e < 8; e++) acc[e] += f[e];
+        }
+    }
   }
+  block_colsum(acc, part, C3);
 }
 
 // partial column sums: block (bx, by) sums rows [by*rpb, ...) of 8*32 = 256 columns starting at bx*256
@@ -47,25 +117,41 @@ __global__ void __launch_bounds__(256) colsum_kernel(const bf16* __restrict__ x,
 #pragma unroll
       for (int e = 0; e < 8; e++) acc[e] += v[e];
     }
-  __shared__ float sh[8][256];
-#pragma unroll
-  for (int e = 0; e < 8; e++) sh[warp][lane * 8 + e] = acc[e];
-  __syncthreads();
-  int c = blockIdx.x * 256 + threadIdx.x;
-  if (c < C) {
-    float s = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; w++) s += sh[w][threadIdx.x];
-    part[(size_t)blockIdx.y * C + c] = s;
-  }
+  block_colsum(acc, part, C);
 }
-__global__ void colsum_finish_kernel(const float* __restrict__ part, int nparts, int C, bf16* __restrict__ out, int accumulate) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
+
+// out[c] (+)= sum over parts of part[p][c] for several vectors in one launch (blockIdx.y: vector, blockIdx.x: 32 columns).
+// Latency bound: the partial rows are spread over the 16 warps of the block, each with 8 loads in flight, so a vector of 296 partial
+// rows takes three round trips to L2 (one thread per column walked them one after the other: 10 us at 256 rows of 1024 columns).
+struct FinishJob { const float* part; bf16* out; int nparts, C, accumulate, pad; };
+constexpr int kMaxFinish = 16;
+struct FinishJobs { FinishJob j[kMaxFinish]; };
+__global__ void __launch_bounds__(512) finish_parts_kernel(const __grid_constant__ FinishJobs jobs) {
+  const FinishJob& j = jobs.j[blockIdx.y];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = j.C, n = j.nparts;
+  const int c = blockIdx.x * 32 + lane;
+  if (blockIdx.x * 32 >= C) return;
   float s = 0.f;
-  for (int p = 0; p < nparts; p++) s += part[(size_t)p * C + c];
-  if (accumulate) s += __bfloat162float(out[c]);
-  out[c] = __float2bfloat16_rn(s);
+  if (c < C) {
+    const float* p = j.part + c;
+    for (int r = warp; r < n; r += 16 * 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = r + u * 16 < n ? p[(size_t)(r + u * 16) * C] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; u++) s += v[u];
+    }
+  }
+  __shared__ float sh[16][32];
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && c < C) {
+    s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 16; w++) s += sh[w][lane];
+    if (j.accumulate) s += __bfloat162float(j.out[c]);
+    j.out[c] = __float2bfloat16_rn(s);
+  }
 }
 
 // One block per row: loss[row] = logsumexp(logits[:V]) - logits[target]; logits <- (softmax - onehot) * gscale
@@ -211,9 +297,38 @@ int piccl_ops_bias_gelu_fwd(const void* h, const void* bias, void* h_out, void* 
   bias_gelu_fwd_kernel<<<grid_for(n8, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)h, (const bf16*)bias, (bf16*)h_out, (bf16*)g, n8, C / 8);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
-int piccl_ops_gelu_bwd(const void* dg, const void* h, void* dh, long long n, void* stream) {
-  if (n % 8) return -1;
-  gelu_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)dg, (const bf16*)h, (bf16*)dh, (size_t)n / 8);
+// Row groups (partial rows) of the kernels that walk C columns of a [rows, C] matrix 256 at a time: four blocks per SM
+int piccl_ops_col_parts(long long rows, int C) {
+  const long long bx = (C + 255) / 256, most = (rows + 8 * kColRows - 1) / (8 * kColRows);
+  const long long n = 148 * 4 / bx;
+  return (int)(n < 1 ? 1 : n < most ? n : most > 0 ? most : 1);
+}
+// part: null, or piccl_ops_col_parts(rows, C) * C floats that receive partial column sums of dh
+int piccl_ops_gelu_bwd(const void* dg, const void* h, void* dh, float* part, long long rows, int C, void* stream) {
+  if (C % 8) return -1;
+  gelu_bwd_kernel<<<dim3((C + 255) / 256, piccl_ops_col_parts(rows, C)), 256, 0, (cudaStream_t)stream>>>((const bf16*)dg, (const bf16*)h, (bf16*)dh, part, rows, C);
+  PICCL_OPS_CHECK_LAUNCH(); return 0;
+}
+// g[3]: gradients of q, k, v; strides: {sb, sh, ss} of each in elements (multiples of 8, the rows 16-byte aligned);
+// part: piccl_ops_col_parts(B * S, 3 * H * D) * 3 * H * D floats
+int piccl_ops_qkv_grad(const void* const* g, const long long* strides, void* dqkv, float* part, int B, int S, int H, int D, void* stream) {
+  if (D % 8) return -1;
+  QkvGrads q;
+  for (int i = 0; i < 3; i++) {
+    q.p[i] = (const bf16*)g[i]; q.sb[i] = strides[3 * i]; q.sh[i] = strides[3 * i + 1]; q.ss[i] = strides[3 * i + 2];
+    if ((q.sb[i] | q.sh[i] | q.ss[i]) % 8 || (uintptr_t)g[i] % 16) return -2;
+  }
+  const int C3 = 3 * H * D;
+  qkv_grad_kernel<<<dim3((C3 + 255) / 256, piccl_ops_col_parts((long long)B * S, C3)), 256, 0, (cudaStream_t)stream>>>(q, (bf16*)dqkv, part, B * S, S, H, D);
+  PICCL_OPS_CHECK_LAUNCH(); return 0;
+}
+// Folds the partial rows of up to 16 vectors into their bf16 results in one launch.
+int piccl_ops_finish_parts(const void* jobs, int n, void* stream) {
+  if (n < 1 || n > kMaxFinish) return -1;
+  FinishJobs a; memset(&a, 0, sizeof a); memcpy(&a, jobs, n * sizeof(FinishJob));
+  int c = 0;
+  for (int i = 0; i < n; i++) c = a.j[i].C > c ? a.j[i].C : c;
+  finish_parts_kernel<<<dim3((c + 31) / 32, n), 512, 0, (cudaStream_t)stream>>>(a);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // workspace: ceil(rows / rows_per_block) * C floats
@@ -221,8 +336,9 @@ int piccl_ops_colsum(const void* x, void* out, float* workspace, int rows, int C
   if (C % 8) return -1;
   int nparts = (rows + rows_per_block - 1) / rows_per_block;
   colsum_kernel<<<dim3((C + 255) / 256, nparts), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, workspace, rows, C, rows_per_block);
-  colsum_finish_kernel<<<(C + 255) / 256, 256, 0, (cudaStream_t)stream>>>(workspace, nparts, C, (bf16*)out, accumulate);
-  PICCL_OPS_CHECK_LAUNCH(); return 0;
+  PICCL_OPS_CHECK_LAUNCH();
+  const FinishJob j{workspace, (bf16*)out, nparts, C, accumulate, 0};
+  return piccl_ops_finish_parts(&j, 1, stream);
 }
 int piccl_ops_ce_fwd_bwd(void* logits, const long long* targets, float* loss, int rows, int V, int Vp, float gscale, void* stream) {
   if (Vp % 8 || V > Vp) return -1;

@@ -17,19 +17,14 @@
 #include <mutex>
 #include <tuple>
 #include "../include/sm100_gemm.cuh"
+#include "ops_common.cuh"
 
 namespace piccl_ops {
 
 using namespace sm100;
-typedef __nv_bfloat16 bf16;
 
 constexpr int BM = GEMM_BM, BK = GEMM_BK;
 template <int BN, int STAGES> using SmemLayout = GemmSmem<BN, STAGES>;
-
-__device__ __forceinline__ float gelu_tanh(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
-}
 
 // Plain GEMM: tiles in m-fastest order, nothing to wait for, bias / GELU epilogue.
 template <int BN>
@@ -68,7 +63,7 @@ struct PlainPolicy {
       for (int i = 0; i < 32; i++) {
         // activation of the value as stored (bf16), so that backward sees the same pre-activation
         float x = C_pre ? __bfloat162float(__float2bfloat16_rn(v[i])) : v[i];
-        v[i] = gelu_tanh(x);
+        v[i] = gelu_f(x);
       }
     }
     store_row32_bf16(C + off, v);

@@ -51,76 +51,108 @@ __global__ void __launch_bounds__(128) ln_fwd_kernel(const bf16* __restrict__ x,
   }
 }
 
-// dx = LN-backward(dy) + dres ; per-block partial dgamma / dbeta in fp32
-template <int V>
-__global__ void __launch_bounds__(128) ln_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ xin, const bf16* __restrict__ gamma,
-                                                     const float* __restrict__ mean, const float* __restrict__ rstd, const bf16* __restrict__ dres,
-                                                     bf16* __restrict__ dx, float* __restrict__ dgamma_part, float* __restrict__ dbeta_part,
-                                                     int rows, int rows_per_block) {
-  const int C = 256 * V;
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float dg[V][8], db[V][8];
+// dx = LN-backward(dy) + dres ; per-block partial column sums in fp32: part[0] = dgamma, part[1] = dbeta and, with_dsum, part[2] = sum
+// of the dx written (dx is the gradient that enters the layer before, whose bias gradient is exactly that sum: the kernel that
+// has the rows in registers adds them up, so nobody reads dx again for it).
+// Memory bound: 4 tensors of rows * C bf16.  A row is spread over V warps (8 columns a thread), so the three accumulators cost 24
+// registers instead of the 96 of a warp per row at C = 1024, and R rows are in flight per group; G groups of V warps make a
+// block of about 8 warps.  The grid is what the chip holds at once: each block leaves one partial row per vector.
+template <int V, int G, int R>   // C = 256 * V
+__global__ void __launch_bounds__(32 * V * G, 2) ln_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ xin, const bf16* __restrict__ gamma,
+                                                               const float* __restrict__ mean, const float* __restrict__ rstd, const bf16* __restrict__ dres,
+                                                               bf16* __restrict__ dx, float* __restrict__ part, int rows, int with_dsum) {
+  constexpr int C = 256 * V;
+  __shared__ float red[2][G][V][2 * R];
+  __shared__ float sh[G][C];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = warp / V, wv = warp % V;
+  const int c8 = wv * 32 + lane;
+  float ga[8], dg[8], db[8], ds[8];
+  unpack8(reinterpret_cast<const bf16x8*>(gamma)[c8], ga);
 #pragma unroll
-  for (int i = 0; i < V; i++)
+  for (int e = 0; e < 8; e++) { dg[e] = 0.f; db[e] = 0.f; ds[e] = 0.f; }
+  int buf = 0;
+  for (int r0 = (blockIdx.x * G + g) * R; r0 < rows; r0 += gridDim.x * G * R, buf ^= 1) {
+    bf16x8 py[R], px[R], pr[R];
+    float mu[R], rs[R];
 #pragma unroll
-    for (int e = 0; e < 8; e++) { dg[i][e] = 0.f; db[i][e] = 0.f; }
-  float g[V][8];
-#pragma unroll
-  for (int i = 0; i < V; i++) unpack8(reinterpret_cast<const bf16x8*>(gamma)[lane + 32 * i], g[i]);
-  int row0 = blockIdx.x * rows_per_block;
-  for (int r = row0 + warp; r < min(rows, row0 + rows_per_block); r += 4) {
-    float mu = mean[r], rs = rstd[r];
-    float xh[V][8], dyv[V][8];
-    float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < V; i++) {
-      unpack8(reinterpret_cast<const bf16x8*>(xin + (size_t)r * C)[lane + 32 * i], xh[i]);
-      unpack8(reinterpret_cast<const bf16x8*>(dy + (size_t)r * C)[lane + 32 * i], dyv[i]);
-#pragma unroll
-      for (int e = 0; e < 8; e++) {
-        xh[i][e] = (xh[i][e] - mu) * rs;
-        dg[i][e] += dyv[i][e] * xh[i][e]; db[i][e] += dyv[i][e];
-        float t = dyv[i][e] * g[i][e];
-        s1 += t; s2 += t * xh[i][e];
-        dyv[i][e] = t;
+    for (int r = 0; r < R; r++) {
+      if (r0 + r < rows) {
+        const size_t o = (size_t)(r0 + r) * (C / 8) + c8;
+        py[r] = reinterpret_cast<const bf16x8*>(dy)[o];
+        px[r] = reinterpret_cast<const bf16x8*>(xin)[o];
+        if (dres) pr[r] = reinterpret_cast<const bf16x8*>(dres)[o];
+        mu[r] = mean[r0 + r]; rs[r] = rstd[r0 + r];
       }
     }
-    s1 = warp_sum(s1) / C; s2 = warp_sum(s2) / C;
+    float s[2 * R];
 #pragma unroll
-    for (int i = 0; i < V; i++) {
-      float o[8];
-      if (dres) unpack8(reinterpret_cast<const bf16x8*>(dres + (size_t)r * C)[lane + 32 * i], o);
-      else {
+    for (int r = 0; r < R; r++) {
+      s[2 * r] = 0.f; s[2 * r + 1] = 0.f;
+      if (r0 + r < rows) {
+        float x[8], y[8];
+        unpack8(px[r], x); unpack8(py[r], y);
 #pragma unroll
-        for (int e = 0; e < 8; e++) o[e] = 0.f;
+        for (int e = 0; e < 8; e++) {
+          const float xh = (x[e] - mu[r]) * rs[r], t = y[e] * ga[e];
+          dg[e] += y[e] * xh; db[e] += y[e];
+          s[2 * r] += t; s[2 * r + 1] += t * xh;
+        }
       }
+    }
 #pragma unroll
-      for (int e = 0; e < 8; e++) o[e] += rs * (dyv[i][e] - s1 - xh[i][e] * s2);
-      reinterpret_cast<bf16x8*>(dx + (size_t)r * C)[lane + 32 * i] = pack8(o);
+    for (int i = 0; i < 2 * R; i++) s[i] = warp_sum(s[i]);
+    if (V > 1) {
+      if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < 2 * R; i++) red[buf][g][wv][i] = s[i];
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(32 * V) : "memory");      // the other buffer is free: its readers have passed this barrier
+#pragma unroll
+      for (int i = 0; i < 2 * R; i++) {
+        s[i] = 0.f;
+#pragma unroll
+        for (int w = 0; w < V; w++) s[i] += red[buf][g][w][i];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      if (r0 + r < rows) {
+        const float s1 = s[2 * r] * (1.f / C), s2 = s[2 * r + 1] * (1.f / C);
+        float x[8], y[8], o[8];
+        unpack8(px[r], x); unpack8(py[r], y);
+        if (dres) unpack8(pr[r], o);
+        else {
+#pragma unroll
+          for (int e = 0; e < 8; e++) o[e] = 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) o[e] += rs[r] * (y[e] * ga[e] - s1 - (x[e] - mu[r]) * rs[r] * s2);
+        const bf16x8 p = pack8(o);
+        reinterpret_cast<bf16x8*>(dx)[(size_t)(r0 + r) * (C / 8) + c8] = p;
+        if (with_dsum) {
+          unpack8(p, o);
+#pragma unroll
+          for (int e = 0; e < 8; e++) ds[e] += o[e];
+        }
+      }
     }
   }
-  // combine the 4 warps of the block, then one partial row per block
-  __shared__ float sh[4][256 * V];   // reused for gamma then beta
-  for (int pass = 0; pass < 2; pass++) {
+  // one partial row per block and vector
 #pragma unroll
-    for (int i = 0; i < V; i++)
+  for (int vec = 0; vec < 3; vec++) {
+    if (vec == 2 && !with_dsum) break;
 #pragma unroll
-      for (int e = 0; e < 8; e++) sh[warp][(lane + 32 * i) * 8 + e] = pass == 0 ? dg[i][e] : db[i][e];
+    for (int e = 0; e < 8; e++) sh[g][c8 * 8 + e] = vec == 0 ? dg[e] : vec == 1 ? db[e] : ds[e];
     __syncthreads();
-    float* dst = (pass == 0 ? dgamma_part : dbeta_part) + (size_t)blockIdx.x * C;
-    for (int c = threadIdx.x; c < C; c += 128) dst[c] = sh[0][c] + sh[1][c] + sh[2][c] + sh[3][c];
+    float* dst = part + ((size_t)vec * gridDim.x + blockIdx.x) * C;
+    for (int c = threadIdx.x; c < C; c += 32 * V * G) {
+      float t = 0.f;
+#pragma unroll
+      for (int q = 0; q < G; q++) t += sh[q][c];
+      dst[c] = t;
+    }
     __syncthreads();
   }
-}
-
-// out[c] (+)= sum over parts of part[p][c]   (bf16 output, fp32 partials)
-__global__ void colsum_parts_kernel(const float* __restrict__ part, int nparts, int C, bf16* __restrict__ out, int accumulate) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float s = 0.f;
-  for (int p = 0; p < nparts; p++) s += part[(size_t)p * C + c];
-  if (accumulate) s += __bfloat162float(out[c]);
-  out[c] = __float2bfloat16_rn(s);
 }
 
 }  // namespace piccl_ops
@@ -141,18 +173,23 @@ int piccl_ops_ln_fwd(const void* x, const void* res, const void* gamma, const vo
   return 0;
 }
 
-// workspace: 2 * nblocks * C floats, nblocks = ceil(rows / rows_per_block).  dgamma/dbeta are bf16 and accumulated if accumulate != 0.
+// Blocks, that is partial rows per vector, that piccl_ops_ln_bwd leaves for `rows` rows of C columns (0: C is not supported).
+int piccl_ops_ln_bwd_parts(int rows, int C) {
+  int per = 0;                                       // rows a block has in flight
+  switch (C) { case 256: per = 8 * 2; break; case 512: per = 4 * 2; break; case 768: case 1024: per = 2 * 2; break; default: return 0; }
+  const int n = (rows + per - 1) / per;
+  return n < 296 ? (n > 0 ? n : 1) : 296;            // two blocks on each of 148 SMs
+}
+
+// part: [2 or 3][piccl_ops_ln_bwd_parts(rows, C)][C] floats, see the kernel; piccl_ops_finish_parts folds them.
 int piccl_ops_ln_bwd(const void* dy, const void* xin, const void* gamma, const float* mean, const float* rstd, const void* dres, void* dx,
-                     void* dgamma, void* dbeta, float* workspace, int rows, int C, int rows_per_block, int accumulate, void* stream) {
-  int nblocks = (rows + rows_per_block - 1) / rows_per_block;
+                     float* part, int with_dsum, int rows, int C, void* stream) {
+  const int nb = piccl_ops_ln_bwd_parts(rows, C);
+  if (!nb) return -1;
   cudaStream_t s = (cudaStream_t)stream;
-  float* pg = workspace; float* pb = workspace + (size_t)nblocks * C;
-#define LN_CASE(V) case 256 * V: ln_bwd_kernel<V><<<nblocks, 128, 0, s>>>((const bf16*)dy, (const bf16*)xin, (const bf16*)gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, pg, pb, rows, rows_per_block); break;
-  switch (C) { LN_CASE(1) LN_CASE(2) LN_CASE(3) LN_CASE(4) default: return -1; }
+#define LN_CASE(V, G) case 256 * V: ln_bwd_kernel<V, G, 2><<<nb, 32 * V * G, 0, s>>>((const bf16*)dy, (const bf16*)xin, (const bf16*)gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, part, rows, with_dsum); break;
+  switch (C) { LN_CASE(1, 8) LN_CASE(2, 4) LN_CASE(3, 2) LN_CASE(4, 2) default: return -1; }
 #undef LN_CASE
-  PICCL_OPS_CHECK_LAUNCH();
-  colsum_parts_kernel<<<(C + 255) / 256, 256, 0, s>>>(pg, nblocks, C, (bf16*)dgamma, accumulate);
-  colsum_parts_kernel<<<(C + 255) / 256, 256, 0, s>>>(pb, nblocks, C, (bf16*)dbeta, accumulate);
   PICCL_OPS_CHECK_LAUNCH();
   return 0;
 }
