@@ -50,11 +50,6 @@ def targets() -> dict[str, dict]:
             "src": _sources("ops/*.cu", "ops/*.cc"),
             "link": ["-shared", "-cudart", "static", "-ldl", "-lpthread", "-lrt"],
         },
-        # CTA-pair GEMM: a library of its own, left out of runs on several GPUs (see the header of its source)
-        "libpiccl_gemm2.so": {
-            "src": _sources("ops2/*.cu"),
-            "link": ["-shared", "-cudart", "static", "-ldl", "-lpthread", "-lrt"],
-        },
         "piccl_sched": {
             "src": _sources("coll/*.cc", "tools/piccl_sched.cc"),
             "link": [],

@@ -154,7 +154,7 @@ class GPT2:
             x2, ln2 = buf(("x2", l), (T, C)), buf(("ln2", l), (T, C))
             mean2, rstd2 = buf(("mean2", l), (T,), f32), buf(("rstd2", l), (T,), f32)
             ops.layernorm_fwd(a, xin, P("ln2_g"), P("ln2_b"), x2, ln2, mean2, rstd2, cfg.ln_eps)
-            h, gl = buf(("h", l), (T, 4 * C)), buf(("g", l), (T, 4 * C))
+            h, gl = None if loss_only else buf(("h", l), (T, 4 * C)), buf(("g", l), (T, 4 * C))
             gemm.linear_gelu(ln2, P("w_fc"), P("b_fc"), h, gl)
             pr = buf("pr", (T, C))
             gemm.linear(gl, P("w_proj"), P("b_proj"), out=pr)
@@ -184,7 +184,7 @@ class GPT2:
         dx = buf("dx_a", (T, C))
         # Bias, gamma and beta gradients are column sums of tensors that some kernel below holds in registers: each leaves partial rows
         # in fp32, one launch per layer folds the partial rows of all eight vectors.
-        n_ln, n_fc, n_qkv = ops.layernorm_bwd_parts(T, C), ops.col_parts(T, 4 * C), ops.col_parts(T, 3 * C)
+        n_ln, n_fc, n_qkv = ops.layernorm_bwd_parts(T, C), gemm.gelu_grad_parts(T, 4 * C), ops.col_parts(T, 3 * C)
         ws = buf("parts", (6 * n_ln * C + n_fc * 4 * C + n_qkv * 3 * C,), f32).data_ptr()
         row = 4 * n_ln * C                                     # bytes of one vector's partial rows
         ws1, ws_fc, ws_qkv = ws + 3 * row, ws + 6 * row, ws + 6 * row + 16 * n_fc * C
@@ -198,8 +198,7 @@ class GPT2:
             # x3 = x2 + gelu(ln2 @ Wfc + bfc) @ Wproj + bproj
             gemm.grad_weight(dx, gl, out=G("w_proj"))
             dg = buf("dg", (T, 4 * C))
-            gemm.grad_input(dx, P("w_proj"), out=dg)
-            ops.gelu_bwd(dg, h, dg, ws_fc)
+            n_fc = gemm.grad_input_gelu(dx, P("w_proj"), h, dg, ws_fc)
             gemm.grad_weight(dg, ln2, out=G("w_fc"))
             dln2 = buf("dln2", (T, C))
             gemm.grad_input(dg, P("w_fc"), out=dln2)

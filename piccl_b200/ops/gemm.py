@@ -31,8 +31,8 @@ def counts() -> dict:
 
 
 def _own_kernel_ok(x, w, out, fused_epilogue: bool = False) -> bool:
-    """"auto": the tcgen05 kernel where its fused epilogue saves a pass over the activations (bias + GELU);
-    plain products stay on cuBLAS, which is still a little faster on those shapes.  "tcgen05": wherever supported."""
+    """"auto": the tcgen05 kernel where its fused epilogue saves a pass over the activations (GELU and its derivative);
+    plain products stay on cuBLAS.  "tcgen05": wherever supported."""
     if _backend == "cublas" or (_backend == "auto" and not fused_epilogue):
         return False
     from . import gemm_sm100
@@ -43,7 +43,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out: torch.Tensor) -> torch.T
     """out[M, N] = x[M, K] @ w[N, K]^T + bias[N]"""
     if _own_kernel_ok(x, w, out):
         from . import gemm_sm100
-        gemm_sm100.gemm_nt(x, w, out, bias=bias)
+        gemm_sm100.gemm(gemm_sm100.NT, gemm_sm100.BIAS, x, w, out, bias=bias)
         _counts["tcgen05"] += 1
         return out
     _counts["cublas"] += 1
@@ -52,17 +52,36 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out: torch.Tensor) -> torch.T
     return torch.addmm(bias, x, w.t(), out=out)
 
 
-def linear_gelu(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor, h_out: torch.Tensor, g_out: torch.Tensor) -> None:
-    """h_out = x @ w^T + bias;  g_out = gelu_tanh(h_out)   — one kernel where the tcgen05 GEMM is usable."""
+def linear_gelu(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor, h_out, g_out: torch.Tensor) -> None:
+    """h_out = x @ w^T + bias (None: not wanted);  g_out = gelu_tanh(h_out)   — one kernel where the tcgen05 GEMM is usable."""
     if _own_kernel_ok(x, w, g_out, fused_epilogue=True):
         from . import gemm_sm100
-        gemm_sm100.gemm_nt(x, w, g_out, bias=bias, gelu=True, pre=h_out)
+        gemm_sm100.gemm(gemm_sm100.NT, gemm_sm100.GELU, x, w, g_out, bias=bias, pre=h_out)
         _counts["tcgen05"] += 1
         return
     from . import bias_gelu_fwd
     _counts["cublas"] += 1
-    torch.mm(x, w.t(), out=h_out)
-    bias_gelu_fwd(h_out, bias, h_out, g_out)
+    h = g_out if h_out is None else h_out
+    torch.mm(x, w.t(), out=h)
+    bias_gelu_fwd(h, bias, h_out, g_out)
+
+
+def gelu_grad_parts(rows: int, cols: int) -> int:
+    """Partial rows that grad_input_gelu leaves at most."""
+    from . import col_parts, gemm_sm100
+    return max(gemm_sm100.partial_rows(rows), col_parts(rows, cols))
+
+
+def grad_input_gelu(dy: torch.Tensor, w: torch.Tensor, h: torch.Tensor, out: torch.Tensor, part: int) -> int:
+    """out = (dy @ w) * gelu'(h), with partial column sums of it at address `part`: returns how many rows of them."""
+    from . import col_parts, gelu_bwd, gemm_sm100
+    if _own_kernel_ok(dy, w, out, fused_epilogue=True):
+        gemm_sm100.gemm(gemm_sm100.NN, gemm_sm100.GELU_GRAD, dy, w, out, aux=h, part=part)
+        _counts["tcgen05"] += 1
+        return gemm_sm100.partial_rows(out.shape[0])
+    grad_input(dy, w, out)
+    gelu_bwd(out, h, out, part)
+    return col_parts(*out.shape)
 
 
 def grad_input(dy: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:

@@ -22,21 +22,42 @@ def available() -> bool:
     return _checked
 
 
+NT, NN, TN = 0, 1, 2                                   # C = A B^T, A B, A^T B
+BIAS, GELU, RESIDUAL, GELU_GRAD = 0, 1, 2, 3           # epilogues, see src/ops/gemm_sm100.cu
+
+
 def supports(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
-    M, K = x.shape
-    Nn = w.shape[0]
+    """Contiguous bf16 operands whose rows are a multiple of 16 bytes."""
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and x.is_contiguous() and w.is_contiguous()
-            and out.is_contiguous() and K % 64 == 0 and Nn % 128 == 0 and M % 128 == 0 and K >= 64)
+            and out.is_contiguous() and x.shape[1] % 8 == 0 and w.shape[1] % 8 == 0 and out.shape[1] % 8 == 0)
+
+
+def _ptr(t) -> C.c_void_p:
+    return C.c_void_p(t.data_ptr() if t is not None else 0)
+
+
+def gemm(layout: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bias=None, aux=None, pre=None, part: int = 0) -> torch.Tensor:
+    """The general entry: layouts and epilogues of src/ops/gemm_sm100.cu; `part` is the address of partial_rows(M) x N floats."""
+    M, Nn = out.shape
+    K = a.shape[0] if layout == TN else a.shape[1]
+    rc = N.ops_lib().piccl_ops_gemm(layout, epilogue, _ptr(a), _ptr(b), _ptr(out), _ptr(pre), _ptr(bias), _ptr(aux), C.c_void_p(part), M, Nn, K,
+                                    C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    if rc != 0:
+        raise RuntimeError(f"piccl_ops_gemm failed (code {rc}) for layout {layout} epilogue {epilogue} M={M} N={Nn} K={K}")
+    _bump()
+    return out
+
+
+def partial_rows(M: int) -> int:
+    """Rows of column sums that the GELU_GRAD epilogue leaves: one per 32 rows."""
+    return (M + 31) // 32
 
 
 def gemm_nt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, gelu: bool = False, pre=None) -> torch.Tensor:
     """out[M, N] = act(x[M, K] @ w[N, K]^T + bias); `pre` (optional) receives the value before the activation"""
     M, K = x.shape
     Nn = w.shape[0]
-    rc = N.ops_lib().piccl_ops_gemm_bf16_nt_ex(C.c_void_p(x.data_ptr()), C.c_void_p(w.data_ptr()), C.c_void_p(out.data_ptr()),
-                                               C.c_void_p(pre.data_ptr() if pre is not None else 0),
-                                               C.c_void_p(bias.data_ptr() if bias is not None else 0), M, Nn, K, int(gelu),
-                                               C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    rc = N.ops_lib().piccl_ops_gemm_bf16_nt_ex(_ptr(x), _ptr(w), _ptr(out), _ptr(pre), _ptr(bias), M, Nn, K, int(gelu), C.c_void_p(torch.cuda.current_stream().cuda_stream))
     if rc != 0:
         raise RuntimeError(f"piccl_ops_gemm_bf16_nt failed (code {rc}) for M={M} N={Nn} K={K}")
     _bump()
@@ -44,19 +65,10 @@ def gemm_nt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, gelu
 
 
 def gemm_nt_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None) -> torch.Tensor:
-    """out[M, N] = x[M, K] @ w[N, K]^T + bias on CTA pairs (`tcgen05.mma.cta_group::2`, src/ops2/gemm_sm100_2cta.cu).
-    M and N multiples of 256, K a multiple of 64.  Opt-in: nothing in the package calls it by default."""
-    M, K = x.shape
-    Nn = w.shape[0]
-    rc = N.gemm2_lib().piccl_ops2_gemm_bf16_nt(C.c_void_p(x.data_ptr()), C.c_void_p(w.data_ptr()), C.c_void_p(out.data_ptr()),
-                                               C.c_void_p(bias.data_ptr() if bias is not None else 0), M, Nn, K,
-                                               C.c_void_p(torch.cuda.current_stream().cuda_stream))
-    if rc != 0:
-        raise RuntimeError(f"piccl_ops2_gemm_bf16_nt failed (code {rc}) for M={M} N={Nn} K={K}")
-    _bump()
-    return out
+    """out[M, N] = x[M, K] @ w[N, K]^T + bias on CTA pairs, which is how every product of this module runs."""
+    return gemm(NT, BIAS, x, w, out, bias=bias)
 
 
 def pair_status() -> int:
-    """0, or the role whose bounded wait ran out in the CTA-pair GEMM since the last call (synchronises the device)."""
-    return int(N.gemm2_lib().piccl_ops2_gemm_status())
+    """0, or the role whose bounded wait ran out in a GEMM on this device (synchronises the device)."""
+    return int(N.ops_lib().piccl_ops_gemm_status())

@@ -26,15 +26,14 @@ __device__ __forceinline__ void block_colsum(const float (&acc)[8], float* __res
 __global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const bf16* __restrict__ h, const bf16* __restrict__ bias, bf16* __restrict__ h_out,
                                                             bf16* __restrict__ g, size_t n8, int C8) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
-    float v[8], b[8], o[8];
+    float v[8], b[8];
     unpack8(reinterpret_cast<const bf16x8*>(h)[i], v);
     if (bias) { unpack8(reinterpret_cast<const bf16x8*>(bias)[i % C8], b);
 #pragma unroll
       for (int e = 0; e < 8; e++) v[e] += b[e]; }
     if (h_out) { bf16x8 p = pack8(v); reinterpret_cast<bf16x8*>(h_out)[i] = p; unpack8(p, v); }
-#pragma unroll
-    for (int e = 0; e < 8; e++) o[e] = gelu_f(v[e]);
-    reinterpret_cast<bf16x8*>(g)[i] = pack8(o);
+    gelu_n(v);
+    reinterpret_cast<bf16x8*>(g)[i] = pack8(v);
   }
 }
 
@@ -60,8 +59,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const bf16* __restrict__ 
         if (r0 + r < rows) {
           float d[8], v[8];
           unpack8(pd[r], d); unpack8(ph[r], v);
-#pragma unroll
-          for (int e = 0; e < 8; e++) d[e] *= gelu_grad_f(v[e]);
+          mul_gelu_grad_n(d, v);
           const bf16x8 p = pack8(d);
           reinterpret_cast<bf16x8*>(dh)[(size_t)(r0 + r) * C8 + c8] = p;
           unpack8(p, d);

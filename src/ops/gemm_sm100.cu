@@ -1,96 +1,185 @@
-// bf16 GEMM for sm_100a:  C[M,N] = act(A[M,K] · B[N,K]^T + bias)
+// bf16 GEMM for sm_100a with fused epilogues, on the CTA-pair core of sm100_gemm_pair.cuh.
 //
-// Persistent, warp-specialised CTAs (one per SM):
-//   warp 0      TMA producer: 128x64 A tiles and BNx64 B tiles -> 128B-swizzled shared memory,
-//               STAGES-deep ring guarded by full/empty mbarriers
-//   warp 1      allocates TMEM; one elected lane issues tcgen05.mma (128 x BN x 16 per instruction),
-//               accumulating in TMEM; tcgen05.commit releases shared-memory stages and publishes
-//               finished accumulators
-//   warps 2-5   epilogue: tcgen05.ld (each warp its own 32-lane quarter) -> bias / GELU in fp32 ->
-//               bf16 -> global.  Two TMEM accumulators, so the epilogue of tile i overlaps the
-//               main loop of tile i+1.
-// All mbarrier waits are bounded; a wait that runs out raises a CTA-wide flag, every role leaves its
-// loop, TMEM is released and the kernel returns with a status word set.
+//   layout 0  C[M,N] = A[M,K] B[N,K]^T      (forward products)
+//   layout 1  C[M,N] = A[M,K] B[K,N]        (input gradients)
+//   layout 2  C[M,N] = A[K,M]^T B[K,N]      (weight gradients)
+//
+//   epilogue 0  C = acc + bias
+//   epilogue 1  pre = acc + bias (optional), C = gelu(pre as stored)
+//   epilogue 2  C = acc + bias + aux                     (residual stream)
+//   epilogue 3  C = acc * gelu'(aux), part = partial column sums of C: the input gradient of the GELU's product and the bias
+//               gradient below it, without a pass over C
+// M, N and K need not be multiples of the tile: what a load finds beyond the extents is zero, what a store would put there is dropped.
 #include <cuda_bf16.h>
 #include <cstdio>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <tuple>
-#include "../include/sm100_gemm.cuh"
+#include "../include/sm100_gemm_pair.cuh"
 #include "ops_common.cuh"
 
 namespace piccl_ops {
 
 using namespace sm100;
 
-constexpr int BM = GEMM_BM, BK = GEMM_BK;
-template <int BN, int STAGES> using SmemLayout = GemmSmem<BN, STAGES>;
+enum Epi : int { EPI_BIAS = 0, EPI_GELU = 1, EPI_RESIDUAL = 2, EPI_GELU_GRAD = 3 };
 
-// Plain GEMM: tiles in m-fastest order, nothing to wait for, bias / GELU epilogue.
-template <int BN>
+struct GemmArgs {
+  CUtensorMap ta, tb, tc, tpre;
+  const bf16* bias; const bf16* aux; float* part;
+  int M, N, K, has_pre;
+  int* status;
+};
+
+template <int TN, int EPI>
 struct PlainPolicy {
-  const CUtensorMap* ta; bf16* C; bf16* C_pre; const bf16* bias; int N, num_m, num_n, act_gelu;
+  const GemmArgs& a;
+  int num_m, num_n;                                    // tiles of 256 rows, of TN columns
+  __device__ PlainPolicy(const GemmArgs& g) : a(g), num_m((g.M + 2 * PAIR_BM - 1) / (2 * PAIR_BM)), num_n((g.N + TN - 1) / TN) {}
   __device__ int num_tiles() const { return num_m * num_n; }
-  // Bands of 32 row blocks, inside a band column blocks outer / row blocks inner: the CTAs that run together share a
-  // band of A (about 30 MB at K = 3584) that stays in L2 while B streams through once per band.
-  __device__ void tile(int idx, int& m_blk, int& n_blk) const {
-    constexpr int GM = 32;
+  // Bands of 16 row tiles, inside a band column tiles outer / row tiles inner: the pairs that run together share a band of A
+  // (about 30 MB at K = 3584) that stays in L2 while B streams through once per band.
+  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) const {
+    constexpr int GM = 16;
     const int per_band = GM * num_n, band = idx / per_band, within = idx % per_band;
     const int rows = min(GM, num_m - band * GM);
-    m_blk = band * GM + within % rows; n_blk = within / rows;
+    m_blk = 2 * (band * GM + within % rows) + v; n_blk = within / rows;
   }
-  __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = m_blk * BM; return ta; }
+  __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = m_blk * PAIR_BM; return &a.ta; }
   __device__ bool gate(int, volatile int*) const { return true; }
-  static constexpr int STAGING = 0;
-  __device__ void set_staging(uint8_t*) {}
-  __device__ bool tile_begin(int, int, int, volatile int*) { return true; }
-  __device__ void tile_end(int, int, int) {}
-  __device__ void store(int m_blk, int n_blk, int row, int col0, float (&v)[32]) {
-    const size_t off = (size_t)(m_blk * BM + row) * N + (size_t)n_blk * BN + col0;
-    if (bias) {
-      const bf16* brow = bias + (size_t)n_blk * BN + col0;
+
+  // 64 bf16 of one row -> this warp's staging buffer (16-byte pieces XOR-ed with the row: conflict free, and the layout the store's map expects)
+  __device__ static void stage_row(const EpiCtx& e, const float (&v)[64]) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        uint4 bb = *reinterpret_cast<const uint4*>(brow + i);
-        const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bb);
+    for (int j = 0; j < 8; j++) {
+      uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-        for (int j = 0; j < 4; j++) { float2 f = __bfloat1622float2(b2[j]); v[i + 2 * j] += f.x; v[i + 2 * j + 1] += f.y; }
+      for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
+      *reinterpret_cast<uint4*>(e.staging + e.lane * 128 + ((j ^ (e.lane & 7)) << 4)) = o;
+    }
+    fence_proxy_async();                               // these stores must be visible to the bulk-copy engine
+    __syncwarp();
+  }
+  __device__ static void ship(const EpiCtx& e, const CUtensorMap* map, int x, int y) {
+    if (e.lane == 0) { tma_store_2d(map, e.staging, x, y); bulk_commit(); }
+  }
+  __device__ static void staging_free(const EpiCtx& e) {
+    if (e.lane == 0) bulk_wait_read_all();             // the last store has been read out of the staging buffer
+    __syncwarp();
+  }
+
+  static constexpr bool AUX = EPI == EPI_RESIDUAL || EPI == EPI_GELU_GRAD;
+  static constexpr int PIECES = TN / 64;               // 64-column pieces of the tile; the halves of the warps share them
+  static constexpr int PER = PIECES >= 2 ? PIECES / 2 : 1;
+  uint4 x[8];                                          // the piece of aux that comes next, in flight
+  // Four rows of 128 bytes per instruction (a thread that loads its own row touches 32 lines at a time, more than the L1 that 225 KB of
+  // shared memory leave can keep: 74 us instead of 61 for 8192 x 4096 x 1024).
+  __device__ void load_aux(const EpiCtx& e, int m_blk, int n_blk, int pc) {
+    const int row0 = m_blk * PAIR_BM + e.quarter * 32 + (e.lane >> 3), col = n_blk * TN + pc * 64 + (e.lane & 7) * 8;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      x[i] = (row0 + 4 * i < a.M && col < a.N) ? *reinterpret_cast<const uint4*>(a.aux + (size_t)(row0 + 4 * i) * a.N + col) : make_uint4(0, 0, 0, 0);
+  }
+  __device__ int first_piece(const EpiCtx& e) const { return PIECES >= 2 ? e.half * PER : e.half; }
+  __device__ void prefetch(const EpiCtx& e, int m_blk, int n_blk) {
+    if (AUX && (PIECES >= 2 || e.half == 0)) load_aux(e, m_blk, n_blk, first_piece(e));
+  }
+
+  __device__ bool epilogue(const EpiCtx& e, int m_blk, int n_blk, volatile int*) {
+    const int row0 = m_blk * PAIR_BM + e.quarter * 32;
+    if (row0 >= a.M || (PIECES < 2 && e.half)) return true;
+    const int p0 = first_piece(e), p1 = p0 + PER;
+#pragma unroll 1
+    for (int pc = p0; pc < p1; pc++) {
+      const int col = n_blk * TN + pc * 64;
+      if (col >= a.N) break;
+      uint4 y[8];                                      // this thread's row of aux
+      staging_free(e);
+      if (AUX) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) { const int r = 4 * i + (e.lane >> 3); *reinterpret_cast<uint4*>(e.staging + r * 128 + (((e.lane & 7) ^ (r & 7)) << 4)) = x[i]; }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; j++) y[j] = *reinterpret_cast<const uint4*>(e.staging + e.lane * 128 + ((j ^ (e.lane & 7)) << 4));
+        __syncwarp();
+        if (pc + 1 < p1) load_aux(e, m_blk, n_blk, pc + 1);
+      }
+      float v[64];
+      epi_load64(e, pc * 64, v);
+      if (EPI != EPI_GELU_GRAD && a.bias) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          if (col + 8 * j < a.N) {
+            float b[8]; unpack8(*reinterpret_cast<const bf16x8*>(a.bias + col + 8 * j), b);
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[8 * j + q] += b[q];
+          }
+        }
+      }
+      if (EPI == EPI_RESIDUAL) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          float b[8]; unpack8(*reinterpret_cast<const bf16x8*>(&y[j]), b);
+#pragma unroll
+          for (int q = 0; q < 8; q++) v[8 * j + q] += b[q];
+        }
+      }
+      if (EPI == EPI_GELU_GRAD) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          float b[8]; unpack8(*reinterpret_cast<const bf16x8*>(&y[j]), b);
+          mul_gelu_grad_n(v + 8 * j, b);
+        }
+      }
+      if (EPI == EPI_GELU) {
+        if (a.has_pre) { stage_row(e, v); ship(e, &a.tpre, col, row0); }
+        if (a.has_pre) {                               // of the value as stored, which the backward pass sees
+#pragma unroll
+          for (int i = 0; i < 64; i++) v[i] = __bfloat162float(__float2bfloat16_rn(v[i]));
+        }
+        gelu_n(v);
+        if (a.has_pre) staging_free(e);
+      }
+      stage_row(e, v);
+      ship(e, &a.tc, col, row0);
+      if (EPI == EPI_GELU_GRAD && a.part) {            // two columns a lane, down the 32 rows of the staging buffer (rows beyond M hold zeros)
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int r = 0; r < 32; r++) {
+          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(e.staging + r * 128 + (((e.lane >> 2) ^ (r & 7)) << 4) + (e.lane & 3) * 4));
+          s0 += f.x; s1 += f.y;
+        }
+        if (col + 2 * e.lane < a.N) *reinterpret_cast<float2*>(a.part + (size_t)(m_blk * 4 + e.quarter) * a.N + col + 2 * e.lane) = make_float2(s0, s1);
       }
     }
-    if (C_pre) store_row32_bf16(C_pre + off, v);
-    if (act_gelu) {
-#pragma unroll
-      for (int i = 0; i < 32; i++) {
-        // activation of the value as stored (bf16), so that backward sees the same pre-activation
-        float x = C_pre ? __bfloat162float(__float2bfloat16_rn(v[i])) : v[i];
-        v[i] = gelu_f(x);
-      }
-    }
-    store_row32_bf16(C + off, v);
+    return true;
   }
 };
 
-template <int BN, int STAGES>
-__global__ void __launch_bounds__(192, 1)
-gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, bf16* __restrict__ C, bf16* __restrict__ C_pre,
-                    const bf16* __restrict__ bias, int M, int N, int K, int act_gelu, int* __restrict__ status) {
+template <int TN, int STAGES, bool A_MN, bool B_MN, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) gemm_pair_kernel(const __grid_constant__ GemmArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int s_abort;
-  if (threadIdx.x == 0) s_abort = 0;
-  if (threadIdx.x == 0) tma_prefetch_desc(&tmap_a);
-  PlainPolicy<BN> pol{&tmap_a, C, C_pre, bias, N, M / BM, N / BN, act_gelu};
-  gemm_persistent<BN, STAGES>(smem_raw, &tmap_b, pol, K, blockIdx.x, gridDim.x, status, &s_abort);
+  if (threadIdx.x == 0) { s_abort = 0; tma_prefetch_desc(&a.ta); tma_prefetch_desc(&a.tc); }
+  PlainPolicy<TN, EPI> pol(a);
+  gemm_pair_persistent<TN, STAGES, A_MN, B_MN>(smem_raw, &a.tb, pol, a.K, blockIdx.x >> 1, gridDim.x >> 1, a.status, &s_abort);
 }
 
 // ------------------------------------------------------------------ host
-struct MapKey { const void* p; long rows, cols; int box; bool operator<(const MapKey& o) const { return std::tie(p, rows, cols, box) < std::tie(o.p, o.rows, o.cols, o.box); } };
+struct MapKey {
+  const void* p; long rows, cols; int box;
+  bool operator<(const MapKey& o) const { return std::tie(p, rows, cols, box) < std::tie(o.p, o.rows, o.cols, o.box); }
+};
 static std::mutex g_mu;
 static std::map<MapKey, CUtensorMap> g_maps;
 static int* g_status[64] = {nullptr};
+static int g_pairs[64] = {0};
 
+// box rows x 64 columns of a row-major [rows, cols] matrix
 static bool get_map(const void* p, long rows, long cols, int box, CUtensorMap* out) {
   std::lock_guard<std::mutex> l(g_mu);
-  MapKey k{p, rows, cols, box};
+  const MapKey k{p, rows, cols, box};
   auto it = g_maps.find(k);
   if (it != g_maps.end()) { *out = it->second; return true; }
   CUtensorMap m;
@@ -100,41 +189,99 @@ static bool get_map(const void* p, long rows, long cols, int box, CUtensorMap* o
   return true;
 }
 
-template <int BN, int STAGES>
-static int launch(const void* A, const void* B, void* C, void* C_pre, const void* bias, int M, int N, int K, int gelu, int* status, cudaStream_t s) {
-  typedef SmemLayout<BN, STAGES> L;
-  CUtensorMap ta, tb;
-  if (!get_map(A, M, K, BM, &ta) || !get_map(B, N, K, BN, &tb)) return -3;
-  static bool attr_set = false;
-  const int smem = L::DYNAMIC;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_bf16_nt_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;
-    attr_set = true;
+typedef void (*GemmFn)(GemmArgs);
+struct Variant { int tn, layout, epi; GemmFn fn; int smem; bool ready[64]; };
+#define V_(TN, ST, L, AM, BM_, E) {TN, L, E, gemm_pair_kernel<TN, ST, AM, BM_, E>, PairSmem<TN, ST>::DYNAMIC, {false}}
+static Variant g_variants[] = {
+  V_(256, 6, 0, false, false, EPI_BIAS), V_(128, 8, 0, false, false, EPI_BIAS), V_(64, 9, 0, false, false, EPI_BIAS),
+  V_(256, 6, 0, false, false, EPI_GELU), V_(128, 8, 0, false, false, EPI_GELU), V_(64, 9, 0, false, false, EPI_GELU),
+  V_(256, 6, 0, false, false, EPI_RESIDUAL), V_(128, 8, 0, false, false, EPI_RESIDUAL), V_(64, 9, 0, false, false, EPI_RESIDUAL),
+  V_(256, 6, 1, false, true, EPI_BIAS), V_(128, 8, 1, false, true, EPI_BIAS),
+  V_(256, 6, 1, false, true, EPI_GELU_GRAD), V_(128, 8, 1, false, true, EPI_GELU_GRAD),
+  V_(256, 6, 2, true, true, EPI_BIAS), V_(128, 8, 2, true, true, EPI_BIAS),
+};
+#undef V_
+
+// Prepares the device state; pairs that can be resident at once (a pair needs two SMs of one GPC): the persistent grid is never larger.
+static int device_ready(int dev) {
+  std::lock_guard<std::mutex> l(g_mu);
+  if (!g_status[dev]) {
+    if (cudaMalloc(&g_status[dev], sizeof(int)) != cudaSuccess) return -7;
+    cudaMemset(g_status[dev], 0, sizeof(int));
   }
-  int dev = 0, sms = 148; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int tiles = (M / BM) * (N / BN);
-  int grid = tiles < sms ? tiles : sms;
-  gemm_bf16_nt_kernel<BN, STAGES><<<grid, 192, smem, s>>>(ta, tb, (bf16*)C, (bf16*)C_pre, (const bf16*)bias, M, N, K, gelu, status);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  if (!g_pairs[dev]) {
+    Variant& v = g_variants[0];
+    if (cudaFuncSetAttribute((const void*)v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem) != cudaSuccess) return -4;
+    int sms = 148; cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sms / 2 * 2); cfg.blockDim = dim3(PAIR_THREADS); cfg.dynamicSmemBytes = v.smem;
+    cudaLaunchAttribute at; memset(&at, 0, sizeof at);
+    at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    int active = 0, n = sms / 2;
+    if (cudaOccupancyMaxActiveClusters(&active, v.fn, &cfg) == cudaSuccess && active > 0) n = active < n ? active : n;
+    else cudaGetLastError();
+    g_pairs[dev] = n;
+  }
+  return 0;
+}
+
+// Tile width: waves of the persistent grid times the clocks of a tile.  A k-step of 16 takes the larger of the MMA (TN / 4 clocks) and
+// reading the operands out of shared memory (128 rows of A and TN / 2 of B at 128 bytes a clock: 32 + TN / 8), which favours wide
+// tiles (64 against 48 clocks for twice the columns) until the tiles no longer fill the pairs; ten clocks a column for the epilogue.
+static Variant* choose(int layout, int epi, int M, int N, int K, int pairs) {
+  Variant* best = nullptr; double best_cost = 0;
+  for (auto& v : g_variants) {
+    if (v.layout != layout || v.epi != epi) continue;
+    const long tiles = (long)((M + 255) / 256) * ((N + v.tn - 1) / v.tn);
+    const double cost = (double)((tiles + pairs - 1) / pairs) * ((32 + v.tn / 8) * ((K + 15) / 16) + 10.0 * v.tn);
+    if (!best || cost < best_cost) { best = &v; best_cost = cost; }
+  }
+  return best;
 }
 
 }  // namespace piccl_ops
 
 extern "C" {
 
+// Row-major, contiguous bf16 operands, 16-byte aligned, rows a multiple of 16 bytes.  bias [N], aux / pre [M, N] or null as the epilogue
+// says; part: [ceil(M / 32)][N] floats or null.  Returns 0 on launch, a negative code if the shape is unsupported or set-up failed.
+int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, void* pre, const void* bias, const void* aux, float* part, int M, int N, int K, void* stream) {
+  using namespace piccl_ops;
+  if (layout < 0 || layout > 2 || M <= 0 || N <= 0 || K <= 0 || N % 8 || (layout != 2 && K % 8) || (layout == 2 && M % 8)) return -1;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(pre) |
+       reinterpret_cast<uintptr_t>(aux) | reinterpret_cast<uintptr_t>(part)) & 15) return -2;
+  if ((epi == EPI_RESIDUAL || epi == EPI_GELU_GRAD) && !aux) return -2;
+  int dev = 0; cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return -6;
+  int rc = device_ready(dev); if (rc) return rc;
+  Variant* v = choose(layout, epi, M, N, K, g_pairs[dev]);
+  if (!v) return -1;
+  if (!v->ready[dev]) {
+    if (cudaFuncSetAttribute((const void*)v->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v->smem) != cudaSuccess) return -4;
+    v->ready[dev] = true;
+  }
+  GemmArgs a;
+  const bool a_ok = layout == 2 ? get_map(A, K, M, 64, &a.ta) : get_map(A, M, K, PAIR_BM, &a.ta);
+  const bool b_ok = layout == 0 ? get_map(B, N, K, v->tn / 2, &a.tb) : get_map(B, K, N, 64, &a.tb);
+  if (!a_ok || !b_ok || !get_map(C, M, N, 32, &a.tc)) return -3;
+  a.has_pre = pre != nullptr;
+  if (pre) { if (!get_map(pre, M, N, 32, &a.tpre)) return -3; } else a.tpre = a.tc;
+  a.bias = (const bf16*)bias; a.aux = (const bf16*)aux; a.part = part;
+  a.M = M; a.N = N; a.K = K; a.status = g_status[dev];
+  const long tiles = (long)((M + 255) / 256) * ((N + v->tn - 1) / v->tn);
+  const int pairs = (int)(tiles < g_pairs[dev] ? tiles : g_pairs[dev]);
+  void* args[] = {&a};
+  return cudaLaunchKernel((const void*)v->fn, dim3(2 * pairs), dim3(PAIR_THREADS), args, v->smem, (cudaStream_t)stream) == cudaSuccess ? 0 : -5;
+}
+
 // C = act(A · B^T + bias).  A [M,K], B [N,K], C [M,N], all bf16 row-major and contiguous; bias [N] bf16 or null;
 // c_pre (optional) receives the value before the activation.  Requires M % 128 == 0, N % 128 == 0, K % 64 == 0.
 // Returns 0 on launch, a negative code if the shape is unsupported or set-up failed.
 int piccl_ops_gemm_bf16_nt_ex(const void* A, const void* B, void* C, void* c_pre, const void* bias, int M, int N, int K, int gelu, void* stream) {
   using namespace piccl_ops;
-  if (M <= 0 || N <= 0 || K <= 0 || M % BM || N % 128 || K % BK) return -1;
-  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(c_pre)) & 15) return -2;
-  int dev = 0; cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return -6;
-  if (!g_status[dev]) { if (cudaMalloc(&g_status[dev], sizeof(int)) != cudaSuccess) return -7; cudaMemset(g_status[dev], 0, sizeof(int)); }
-  cudaStream_t s = (cudaStream_t)stream;
-  if (N % 256 == 0) return launch<256, 4>(A, B, C, c_pre, bias, M, N, K, gelu, g_status[dev], s);
-  return launch<128, 6>(A, B, C, c_pre, bias, M, N, K, gelu, g_status[dev], s);
+  if (M <= 0 || N <= 0 || K <= 0 || M % 128 || N % 128 || K % 64) return -1;
+  return piccl_ops_gemm(0, gelu ? EPI_GELU : EPI_BIAS, A, B, C, c_pre, bias, nullptr, nullptr, M, N, K, stream);
 }
 int piccl_ops_gemm_bf16_nt(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int gelu, void* stream) {
   return piccl_ops_gemm_bf16_nt_ex(A, B, C, nullptr, bias, M, N, K, gelu, stream);

@@ -30,17 +30,41 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-// GPT-2's tanh GELU and its derivative, through 0.5 (1 + tanh u) = 1 / (1 + exp(-2u)): two special-function instructions in place of
-// the branches of tanhf, and no cancellation in 1 + tanh u for negative u.
-__device__ __forceinline__ float gelu_sigmoid(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return __fdividef(1.f, 1.f + __expf(-2.f * k0 * x * (1.f + k1 * x * x)));      // exp may be inf: 1 / inf is the 0 that is wanted
+// GPT-2's tanh GELU and its derivative, through 0.5 (1 + tanh u) = 1 / (1 + exp(-2u)), u = k0 (x + k1 x^3): two special-function
+// instructions in place of the branches of tanhf, and no cancellation in 1 + tanh u for negative u.  Two values at a time: the
+// polynomial parts run as packed fp32 pairs, since the GEMM epilogues that call these are bound by instruction issue.
+__device__ __forceinline__ float ex2_approx(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float rcp_approx(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 both2(float a) { return pack2(a, a); }
+
+__device__ __forceinline__ f32x2 gelu_sigmoid2(f32x2 x, f32x2 xx) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f, c = -2.f * k0 * 1.4426950408889634f;
+  const f32x2 z = mul2(x, fma2(both2(c * k1), xx, both2(c)));
+  float a, b; unpack2(z, a, b);
+  unpack2(add2(pack2(ex2_approx(a), ex2_approx(b)), both2(1.f)), a, b);      // exp may be inf: 1 / inf is the 0 that is wanted
+  return pack2(rcp_approx(a), rcp_approx(b));
 }
-__device__ __forceinline__ float gelu_f(float x) { return x * gelu_sigmoid(x); }
-__device__ __forceinline__ float gelu_grad_f(float x) {
+__device__ __forceinline__ f32x2 gelu2(f32x2 x) { return mul2(x, gelu_sigmoid2(x, mul2(x, x))); }
+__device__ __forceinline__ f32x2 gelu_grad2(f32x2 x) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float s = gelu_sigmoid(x);
-  return s + 2.f * x * s * (1.f - s) * (k0 + 3.f * k0 * k1 * x * x);
+  const f32x2 xx = mul2(x, x), s = gelu_sigmoid2(x, xx);
+  const f32x2 t = fma2(mul2(s, both2(-1.f)), s, s);                          // s (1 - s)
+  return fma2(t, mul2(x, fma2(both2(6.f * k0 * k1), xx, both2(2.f * k0))), s);
+}
+// arrays of an even number of values in registers
+template <int N> __device__ __forceinline__ void gelu_n(float (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) unpack2(gelu2(pack2(v[i], v[i + 1])), v[i], v[i + 1]);
+}
+template <int N> __device__ __forceinline__ void mul_gelu_grad_n(float* v, const float (&x)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) unpack2(mul2(pack2(v[i], v[i + 1]), gelu_grad2(pack2(x[i], x[i + 1]))), v[i], v[i + 1]);
 }
 
 }  // namespace piccl_ops

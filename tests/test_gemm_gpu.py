@@ -66,3 +66,38 @@ def test_gemm_back_to_back_and_unsupported_shapes():
     # shapes the kernel does not cover are refused with an error code, not computed wrongly
     rc = N.ops_lib().piccl_ops_gemm_bf16_nt(C.c_void_p(a.data_ptr()), C.c_void_p(b.data_ptr()), C.c_void_p(outs[0].data_ptr()), C.c_void_p(0), 100, 256, 512, 0, C.c_void_p(0))
     assert rc != 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (127, 72, 40), (129, 264, 72), (257, 520, 192), (2331, 768, 200)])
+@pytest.mark.parametrize("layout,epilogue", [(0, 0), (0, 1), (0, 2), (1, 0), (1, 3), (2, 0)])
+def test_gemm_layouts_epilogues_and_edges(M, N, K, layout, epilogue):
+    """Ragged tiles of every operand layout and epilogue against fp32.  The result is rounded to bf16 once (2^-9 relative, 2^-8 where
+    GELU reads the rounded pre-activation) on top of an fp32 sum, so the error norm stays below 4e-3 of the result's."""
+    from piccl_b200.ops import gemm_sm100 as G
+    if layout == 2:
+        M = (M + 7) // 8 * 8                      # rows of A^T are a multiple of 16 bytes
+    a = _bf(M, K, seed=1) if layout != 2 else _bf(K, M, seed=1)
+    b = _bf(N, K, seed=2, scale=0.05) if layout == 0 else _bf(K, N, seed=2, scale=0.05)
+    bias = _bf(N, seed=3) if epilogue != 3 else None
+    aux = _bf(M, N, seed=4) if epilogue >= 2 else None
+    guard = torch.full((M + 1, N), float("nan"), device="cuda", dtype=torch.bfloat16)      # the row after the result must stay untouched
+    out, pre = guard[:M], (torch.empty(M, N, device="cuda", dtype=torch.bfloat16) if epilogue == 1 else None)
+    part = torch.full((G.partial_rows(M), N), float("nan"), device="cuda") if epilogue == 3 else None
+    G.gemm(layout, epilogue, a, b, out, bias=bias, aux=aux, pre=pre, part=part.data_ptr() if part is not None else 0)
+    torch.cuda.synchronize()
+    assert _status() == 0
+    ref = (a.float().t() if layout == 2 else a.float()).double() @ (b.float().t() if layout == 0 else b.float()).double()
+    if bias is not None:
+        ref = ref + bias.double()
+    if epilogue == 1:
+        assert (pre.double() - ref).norm() <= 4e-3 * ref.norm()
+        ref = F.gelu(pre.double(), approximate="tanh")
+    if epilogue == 2:
+        ref = ref + aux.double()
+    if epilogue == 3:
+        x = aux.double().requires_grad_()
+        F.gelu(x, approximate="tanh").backward(ref)
+        ref = x.grad
+        assert (part.double().sum(0) - out.double().sum(0)).norm() <= 1e-5 * out.double().abs().sum(0).norm()      # fp32 sums of M values
+    assert (out.double() - ref).norm() <= 4e-3 * ref.norm()
+    assert torch.isnan(guard[M]).all()
