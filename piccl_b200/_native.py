@@ -98,6 +98,22 @@ def ops_lib() -> C.CDLL:
         return _libs["ops"]
 
 
+def model_lib() -> C.CDLL:
+    """The native training step (libpiccl_model.so); PyTorch's libraries are already in the process."""
+    with _lock:
+        if "model" not in _libs:
+            import torch  # noqa: F401
+            _ensure_built("libpiccl_ops.so")
+            l = C.CDLL(str(_ensure_built("libpiccl_model.so")), mode=C.RTLD_LOCAL)
+            vp, i, ll = C.c_void_p, C.c_int, C.c_longlong
+            l.piccl_gpt2_create.argtypes, l.piccl_gpt2_create.restype = [vp], vp
+            l.piccl_gpt2_destroy.argtypes = [vp]
+            l.piccl_gpt2_run.argtypes = [vp, vp, vp, i, i, vp, i, i, vp, C.POINTER(ll)]
+            l.piccl_gpt2_error.restype = C.c_char_p
+            _libs["model"] = l
+        return _libs["model"]
+
+
 def last_error() -> str:
     return (lib().piccl_last_error() or b"").decode()
 

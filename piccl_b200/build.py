@@ -2,6 +2,7 @@
 
   piccl_b200/lib/piccl.so        collectives library + NCCL-ABI preload shim + fused TP kernels
   piccl_b200/lib/libpiccl_ops.so model kernels (tcgen05 GEMM, layer norm, cross entropy, AdamW, ...)
+  piccl_b200/lib/libpiccl_model.so native training step (launches the kernels of libpiccl_ops.so, attention through ATen)
   piccl_b200/lib/piccl_sched     schedule dump / validation command line tool
   piccl_b200/lib/coll_bench      OSU-style collective benchmark (fork per GPU, no MPI)
   piccl_b200/lib/loggp_bench     PRTT measurements between two GPUs (input of tools/loggp_param)
@@ -15,6 +16,7 @@ Run:  python -m piccl_b200.build [--force] [--verbose]
 from __future__ import annotations
 
 import concurrent.futures as cf
+import importlib.util
 import os
 import shlex
 import subprocess
@@ -26,6 +28,7 @@ SRC = ROOT / "src"
 OUT = ROOT / "piccl_b200" / "lib"
 OBJ = ROOT / "build"
 
+TORCH = Path(importlib.util.find_spec("torch").submodule_search_locations[0])     # its headers and libraries, without importing it
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -49,6 +52,13 @@ def targets() -> dict[str, dict]:
         "libpiccl_ops.so": {
             "src": _sources("ops/*.cu", "ops/*.cc"),
             "link": ["-shared", "-cudart", "static", "-ldl", "-lpthread", "-lrt"],
+        },
+        # the training step: calls libpiccl_ops.so and, for attention, ATen
+        "libpiccl_model.so": {
+            "src": _sources("model/*.cc"),
+            "flags": [f"-I{p}" for p in (TORCH / "include", TORCH / "include" / "torch" / "csrc" / "api" / "include")],
+            "link": ["-shared", "-cudart", "none", f"-L{OUT}", "-lpiccl_ops", f"-L{TORCH / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+                     "-Xlinker", "-rpath,$ORIGIN", "-Xlinker", f"-rpath,{TORCH / 'lib'}"],
         },
         "piccl_sched": {
             "src": _sources("coll/*.cc", "tools/piccl_sched.cc"),
@@ -104,7 +114,7 @@ def build(force: bool = False, verbose: bool = False, only: list[str] | None = N
             objs.append(o)
             stale = force or _newer(s, o) or (o.exists() and hdr_m > o.stat().st_mtime)
             if stale and o not in jobs:
-                cmd = [NVCC, *ARCH, *CXXFLAGS, *INCLUDES, "-c", str(s), "-o", str(o)]
+                cmd = [NVCC, *ARCH, *CXXFLAGS, *INCLUDES, *t.get("flags", []), "-c", str(s), "-o", str(o)]
                 if ptxas_info:
                     cmd.insert(1, "-Xptxas=-v")
                 jobs[o] = cmd

@@ -62,31 +62,15 @@ class _FinishJob(C.Structure):
     _fields_ = [("part", C.c_void_p), ("out", C.c_void_p), ("nparts", C.c_int), ("C", C.c_int), ("accumulate", C.c_int), ("pad", C.c_int)]
 
 
-def finish_parts(jobs) -> None:
-    """jobs: up to 16 tuples (address of fp32 partial rows, number of rows, bf16 output vector, accumulate): out (+)= sum of the rows."""
-    arr = (_FinishJob * len(jobs))(*[(p, o.data_ptr(), n, o.numel(), int(acc), 0) for p, n, o, acc in jobs])
-    _chk(N.ops_lib().piccl_ops_finish_parts(arr, len(jobs), C.c_void_p(_s())), "finish_parts")
-    _bump()
-
-
-def layernorm_bwd_parts(rows: int, cols: int) -> int:
-    return N.ops_lib().piccl_ops_ln_bwd_parts(rows, cols)
-
-
-def layernorm_bwd_partial(dy, xin, gamma, mean, rstd, dres, dx, part: int, with_dsum: bool) -> None:
-    """dx = dLN(dy) + dres; partial rows of dgamma, dbeta (and of the column sum of dx) at address `part`: [2 or 3][layernorm_bwd_parts][C] floats."""
-    rows, Cc = dy.shape
-    _chk(N.ops_lib().piccl_ops_ln_bwd(_p(dy), _p(xin), _p(gamma), _p(mean), _p(rstd), _p(dres), _p(dx), C.c_void_p(part), int(with_dsum), rows, Cc, C.c_void_p(_s())), "ln_bwd")
-    _bump()
-
-
 def layernorm_bwd(dy, xin, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate: bool = False):
     """dx = dLN(dy) + dres; dgamma / dbeta (bf16) written or accumulated."""
     rows, Cc = dy.shape
-    n = layernorm_bwd_parts(rows, Cc)
+    n = N.ops_lib().piccl_ops_ln_bwd_parts(rows, Cc)
     ws = _workspace(2 * max(n, 1) * Cc, dy.device)
-    layernorm_bwd_partial(dy, xin, gamma, mean, rstd, dres, dx, ws.data_ptr(), False)
-    finish_parts([(ws.data_ptr(), n, dgamma, accumulate), (ws.data_ptr() + 4 * n * Cc, n, dbeta, accumulate)])
+    _chk(N.ops_lib().piccl_ops_ln_bwd(_p(dy), _p(xin), _p(gamma), _p(mean), _p(rstd), _p(dres), _p(dx), _p(ws), 0, rows, Cc, C.c_void_p(_s())), "ln_bwd")
+    jobs = (_FinishJob * 2)(*[(ws.data_ptr() + 4 * i * n * Cc, o.data_ptr(), n, Cc, int(accumulate), 0) for i, o in enumerate((dgamma, dbeta))])
+    _chk(N.ops_lib().piccl_ops_finish_parts(jobs, 2, C.c_void_p(_s())), "finish_parts")
+    _bump(2)
 
 
 def bias_gelu_fwd(h, bias, h_out, g):
@@ -95,25 +79,9 @@ def bias_gelu_fwd(h, bias, h_out, g):
     _bump()
 
 
-def col_parts(rows: int, cols: int) -> int:
-    """Partial rows that gelu_bwd and qkv_grad leave."""
-    return N.ops_lib().piccl_ops_col_parts(C.c_longlong(rows), cols)
-
-
-def gelu_bwd(dg, h, dh, part: int = 0):
-    """dh = dg * gelu'(h); part: address of col_parts(*h.shape) * h.shape[1] floats for partial column sums of dh (0: none)."""
+def gelu_bwd(dg, h, dh):
     rows, Cc = h.shape
-    _chk(N.ops_lib().piccl_ops_gelu_bwd(_p(dg), _p(h), _p(dh), C.c_void_p(part), C.c_longlong(rows), Cc, C.c_void_p(_s())), "gelu_bwd")
-    _bump()
-
-
-def qkv_grad(dq, dk, dv, dqkv, part: int):
-    """dqkv[b * S + s, (which, head, d)] from the [B, H, S, D] gradients of the attention, with partial column sums at address `part`."""
-    B, H, S, D = dq.shape
-    ptrs = (C.c_void_p * 3)(dq.data_ptr(), dk.data_ptr(), dv.data_ptr())
-    st = (C.c_longlong * 9)(*[t.stride(i) for t in (dq, dk, dv) for i in (0, 1, 2)])
-    assert dq.stride(3) == dk.stride(3) == dv.stride(3) == 1
-    _chk(N.ops_lib().piccl_ops_qkv_grad(ptrs, st, _p(dqkv), C.c_void_p(part), B, S, H, D, C.c_void_p(_s())), "qkv_grad")
+    _chk(N.ops_lib().piccl_ops_gelu_bwd(_p(dg), _p(h), _p(dh), C.c_void_p(0), C.c_longlong(rows), Cc, C.c_void_p(_s())), "gelu_bwd")
     _bump()
 
 
@@ -143,6 +111,14 @@ def adamw_devstep(p, master, m, v, g, lr: float, b1: float, b2: float, eps: floa
     """AdamW with the step number in a device int32 tensor (replayable from a CUDA graph)."""
     _chk(N.ops_lib().piccl_ops_adamw_devstep(_p(p), _p(master), _p(m), _p(v), _p(g), C.c_longlong(p.numel()), C.c_float(lr), C.c_float(b1), C.c_float(b2),
                                              C.c_float(eps), C.c_float(wd), _p(step_dev), C.c_float(gscale), C.c_void_p(_s())), "adamw_devstep")
+    _bump()
+
+
+def adamw_runs(p, master, m, v, g, ends, decay_parity: int, lr: float, b1: float, b2: float, eps: float, wd: float, step_dev, ticket):
+    """AdamW over flat buffers in one launch: run i ends before pack `ends[i]` of 8 elements (device int32), runs of parity `decay_parity` decay;
+    `step_dev` (device int32, steps done so far) is advanced by the launch, `ticket` is a device int32 that holds zero."""
+    _chk(N.ops_lib().piccl_ops_adamw_runs(_p(p), _p(master), _p(m), _p(v), _p(g), C.c_longlong(p.numel()), _p(ends), ends.numel(), decay_parity, C.c_float(lr), C.c_float(b1),
+                                          C.c_float(b2), C.c_float(eps), C.c_float(wd), _p(step_dev), _p(ticket), C.c_void_p(_s())), "adamw_runs")
     _bump()
 
 

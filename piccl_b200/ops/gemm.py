@@ -26,8 +26,19 @@ def backend() -> str:
     return _backend
 
 
+def backend_code() -> int:
+    """The backend as the native training step numbers it."""
+    return ("auto", "tcgen05", "cublas").index(_backend)
+
+
 def counts() -> dict:
     return dict(_counts)
+
+
+def count(tcgen05: int, cublas: int) -> None:
+    """Adds the products of a native training step."""
+    _counts["tcgen05"] += tcgen05
+    _counts["cublas"] += cublas
 
 
 def _own_kernel_ok(x, w, out, fused_epilogue: bool = False) -> bool:
@@ -64,24 +75,6 @@ def linear_gelu(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor, h_out, g_o
     h = g_out if h_out is None else h_out
     torch.mm(x, w.t(), out=h)
     bias_gelu_fwd(h, bias, h_out, g_out)
-
-
-def gelu_grad_parts(rows: int, cols: int) -> int:
-    """Partial rows that grad_input_gelu leaves at most."""
-    from . import col_parts, gemm_sm100
-    return max(gemm_sm100.partial_rows(rows), col_parts(rows, cols))
-
-
-def grad_input_gelu(dy: torch.Tensor, w: torch.Tensor, h: torch.Tensor, out: torch.Tensor, part: int) -> int:
-    """out = (dy @ w) * gelu'(h), with partial column sums of it at address `part`: returns how many rows of them."""
-    from . import col_parts, gelu_bwd, gemm_sm100
-    if _own_kernel_ok(dy, w, out, fused_epilogue=True):
-        gemm_sm100.gemm(gemm_sm100.NN, gemm_sm100.GELU_GRAD, dy, w, out, aux=h, part=part)
-        _counts["tcgen05"] += 1
-        return gemm_sm100.partial_rows(out.shape[0])
-    grad_input(dy, w, out)
-    gelu_bwd(out, h, out, part)
-    return col_parts(*out.shape)
 
 
 def grad_input(dy: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:

@@ -54,7 +54,7 @@ class DataParallelTrainer:
 
     def _eager_step(self, idx: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
         self.averager.begin_step()
-        loss = self.model.forward_backward(idx, targets, on_grads_ready=self.averager.ready)
+        loss = self.model.forward_backward(idx, targets, on_grads_ready=self.averager.ready if self.averager.stream is not None else None)
         self.averager.finish()
         self.model.optimizer_step(lr=self.lr, weight_decay=self.weight_decay)
         return loss

@@ -1,0 +1,280 @@
+// Forward and backward pass of the GPT-2 training step as one native call (piccl_b200/models/gpt2.py keeps the parameters).
+//
+// Why native: the step is a few dozen launches per layer, and issued from Python each cost about 15 us of host time: two layers of
+// 256 columns took 1.4 ms for 0.3 ms of kernels, eight layers of 768 columns 4.5 ms for 2.7 ms.  Here a launch of this framework's
+// own kernels is a plain call (2 to 3 us); attention goes through ATen's fused kernels without autograd.
+//
+// The gradient buffer is laid out in the order in which the backward pass finishes it; `ready(end)` tells the caller that elements
+// [0, end) are final, which is where bucketed all-reduces start (the overlap that the reference gets from torch DDP).
+// Bias, gamma and beta gradients are column sums of tensors that some kernel holds in registers: each leaves partial rows in fp32,
+// one launch per layer folds the partial rows of all eight vectors.
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/core/GradMode.h>
+#include <torch/csrc/autograd/autograd.h>
+#include <cstdint>
+#include <cstring>
+#include <string>
+#include <vector>
+#include "../ops/piccl_ops.h"
+
+namespace {
+
+thread_local std::string g_error;
+
+enum { W_QKV, W_O, W_FC, W_PROJ, LN1_G, LN1_B, B_QKV, B_O, LN2_G, LN2_B, B_FC, B_PROJ, PER_LAYER };
+enum { NT = 0, NN = 1, TN = 2 };
+enum { EPI_BIAS = 0, EPI_GELU = 1, EPI_GELU_GRAD = 3 };
+typedef uint16_t b16;       // storage of a bf16 value
+typedef void (*ReadyFn)(long long end);
+
+struct Desc {               // mirrored in piccl_b200/models/gpt2.py
+  int L, C, H, V, Vp, seq_len;
+  float eps;
+  int pad;
+  b16 *p, *g;               // flat parameters and gradients
+  const long long* off;     // element offsets: lnf_g, lnf_b, wpe, wte, then PER_LAYER per layer
+};
+
+struct Saved { at::Tensor q, k, v, out, lse, cq, ck, seed, offset; c10::SymInt mq = 0, mk = 0; bool direct = false; };
+
+struct Model {
+  Desc d;
+  std::vector<long long> off;
+  at::Tensor arena;         // activations and workspace, grown to the largest shape so far
+  at::Tensor stage, owner;  // fp32 table of embedding gradients (all zero between calls), one row of the batch per token id
+  std::vector<Saved> saved;
+  long long launches = 0, cublas = 0, tcgen05 = 0;
+  int backend = 0;          // 0 / 1: this framework's GEMM, 2: cuBLAS
+
+  b16* p(int l, int which) const { return d.p + off[4 + l * PER_LAYER + which]; }
+  b16* g(int l, int which) const { return d.g + off[4 + l * PER_LAYER + which]; }
+};
+
+#define TRY(expr)                                                                             \
+  do {                                                                                        \
+    const int rc_ = (expr);                                                                   \
+    if (rc_ != 0) { g_error = std::string(#expr) + " failed (code " + std::to_string(rc_) + ")"; return rc_; } \
+    m.launches++;                                                                             \
+  } while (0)
+
+// hands out 256-byte aligned pieces of the arena; with base = null it only adds up
+struct Carve {
+  char* base; size_t used = 0;
+  template <typename T> T* get(size_t n) {
+    T* r = reinterpret_cast<T*>(base + used);
+    used += (n * sizeof(T) + 255) / 256 * 256;
+    return base ? r : nullptr;
+  }
+};
+
+struct Layer { b16 *ln1, *qkv, *x2, *ln2, *h, *gl, *x3; float *mean1, *rstd1, *mean2, *rstd2; };
+struct Buffers {
+  b16 *x0, *a, *pr, *logits, *dln, *dxa, *dxb, *dg, *dln2, *datt, *dqkv, *dln1;
+  float *loss_rows, *parts;
+  std::vector<Layer> layer;         // L + 1: the last one holds the input of the head
+};
+
+void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, Buffers& b) {
+  const size_t C = d.C;
+  b.x0 = c.get<b16>(T * C); b.a = c.get<b16>(T * C); b.pr = c.get<b16>(T * C);
+  b.layer.resize(d.L + 1);
+  for (int l = 0; l <= d.L; l++) {
+    Layer& y = b.layer[l];
+    if (!train && l >= 2) { y = b.layer[l - 2]; continue; }      // nothing is kept for a backward pass: two sets take turns
+    y.ln1 = c.get<b16>(T * C); y.mean1 = c.get<float>(T); y.rstd1 = c.get<float>(T);
+    if (train && l == d.L) continue;
+    y.qkv = c.get<b16>(T * 3 * C); y.x2 = c.get<b16>(T * C); y.ln2 = c.get<b16>(T * C); y.mean2 = c.get<float>(T); y.rstd2 = c.get<float>(T);
+    y.h = train ? c.get<b16>(T * 4 * C) : nullptr; y.gl = c.get<b16>(T * 4 * C); y.x3 = c.get<b16>(T * C);
+  }
+  b.logits = c.get<b16>(T * d.Vp); b.loss_rows = c.get<float>(T);
+  if (!train) return;
+  b.dln = c.get<b16>(T * C); b.dxa = c.get<b16>(T * C); b.dxb = c.get<b16>(T * C); b.dg = c.get<b16>(T * 4 * C); b.dln2 = c.get<b16>(T * C);
+  b.datt = c.get<b16>(T * C); b.dqkv = c.get<b16>(T * 3 * C); b.dln1 = c.get<b16>(T * C); b.parts = c.get<float>(part_floats);
+}
+
+at::Tensor view(b16* p, at::IntArrayRef sizes, at::IntArrayRef strides = {}) {
+  static thread_local int dev = -1;
+  dev = at::cuda::current_device();
+  const auto opt = at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, dev);
+  return strides.empty() ? at::from_blob(p, sizes, opt) : at::from_blob(p, sizes, strides, [](void*) {}, opt);
+}
+
+// C[M, N] = A op B, bf16 row-major: layout NT A [M,K] B [N,K], NN A [M,K] B [K,N], TN A [K,M] B [K,N]
+int product(Model& m, int layout, b16* A, b16* B, b16* C, const b16* bias, int M, int N, int K, void* s) {
+  if (m.backend == 2) {
+    at::Tensor out = view(C, {M, N});
+    at::Tensor a = layout == TN ? view(A, {K, M}).t() : view(A, {M, K}), b = layout == NT ? view(B, {N, K}).t() : view(B, {K, N});
+    if (bias) at::addmm_out(out, view(const_cast<b16*>(bias), {N}), a, b); else at::mm_out(out, a, b);
+    m.cublas++;
+    return 0;
+  }
+  TRY(piccl_ops_gemm(layout, EPI_BIAS, A, B, C, nullptr, bias, nullptr, nullptr, M, N, K, s));
+  m.tcgen05++;
+  return 0;
+}
+#define DO(expr) do { const int rc_ = (expr); if (rc_ != 0) return rc_; } while (0)
+
+// Causal attention of qkv [B * S, 3 C]; the [B, S, H, D] output is contiguous.
+at::Tensor attention(Saved& sv, b16* qkv, int B, int S, int H, int D, bool train) {
+  const int64_t C = (int64_t)H * D, sizes[4] = {B, H, S, D}, strides[4] = {(int64_t)S * 3 * C, D, 3 * C, 1};
+  sv.q = view(qkv, sizes, strides); sv.k = view(qkv + C, sizes, strides); sv.v = view(qkv + 2 * C, sizes, strides);
+  // the kernel that scaled_dot_product_attention would pick: cuDNN's is called without autograd, any other through it
+  sv.direct = at::_fused_sdp_choice(sv.q, sv.k, sv.v, {}, 0.0, true) == 3 /* sdp::SDPBackend::cudnn_attention */;
+  if (sv.direct) {
+    auto r = at::_scaled_dot_product_cudnn_attention(sv.q, sv.k, sv.v, {}, train, 0.0, true, false);
+    sv.out = std::get<0>(r); sv.lse = std::get<1>(r); sv.cq = std::get<2>(r); sv.ck = std::get<3>(r); sv.mq = std::get<4>(r); sv.mk = std::get<5>(r);
+    sv.seed = std::get<6>(r); sv.offset = std::get<7>(r);
+    return sv.out.transpose(1, 2).contiguous();
+  }
+  c10::AutoGradMode grad(train);
+  if (train) { sv.q.requires_grad_(true); sv.k.requires_grad_(true); sv.v.requires_grad_(true); }
+  sv.out = at::scaled_dot_product_attention(sv.q, sv.k, sv.v, {}, 0.0, true);
+  return sv.out.detach().transpose(1, 2).contiguous();
+}
+
+void attention_grad(const Saved& sv, b16* dout, int B, int S, int H, int D, at::Tensor (&d)[3]) {
+  const at::Tensor go = view(dout, {B, S, H, D}).transpose(1, 2);
+  if (sv.direct) {
+    auto r = at::_scaled_dot_product_cudnn_attention_backward_symint(go, sv.q, sv.k, sv.v, sv.out, sv.lse, sv.seed, sv.offset, at::Tensor(), sv.cq, sv.ck, sv.mq, sv.mk, 0.0, true);
+    d[0] = std::get<0>(r); d[1] = std::get<1>(r); d[2] = std::get<2>(r);
+  } else {
+    auto r = torch::autograd::grad({sv.out}, {sv.q, sv.k, sv.v}, {go});
+    for (int i = 0; i < 3; i++) d[i] = r[i];
+  }
+  for (auto& t : d) if (t.stride(3) != 1) t = t.contiguous();
+}
+
+int run(Model& m, const long long* idx, const long long* tgt, int B, int S, float* loss, bool train, ReadyFn ready) {
+  const Desc& d = m.d;
+  const int T = B * S, C = d.C, L = d.L, H = d.H, D = C / H;
+  void* s = at::cuda::getCurrentCUDAStream().stream();
+  c10::NoGradGuard no_grad;
+  const auto opt = at::TensorOptions().device(at::kCUDA, at::cuda::current_device());
+
+  // partial rows of the column sums: dgamma, dbeta and bias gradient of both LayerNorms, the MLP's and the attention's bias gradients
+  const int n_ln = piccl_ops_ln_bwd_parts(T, C), n_qkv = piccl_ops_col_parts(T, 3 * C), n_fc_own = (T + 31) / 32, n_fc_sep = piccl_ops_col_parts(T, 4 * C);
+  const size_t row = (size_t)n_ln * C, fc_floats = (size_t)std::max(n_fc_own, n_fc_sep) * 4 * C;
+  Buffers b;
+  Carve count{nullptr};
+  carve(count, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
+  if (!m.arena.defined() || (size_t)m.arena.numel() < count.used) { m.arena = at::Tensor(); m.arena = at::empty({(int64_t)count.used}, opt.dtype(at::kByte)); }
+  Carve c{static_cast<char*>(m.arena.data_ptr())};
+  carve(c, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
+  b16 *const lnf_g = d.p + m.off[0], *const lnf_b = d.p + m.off[1], *const wpe = d.p + m.off[2], *const wte = d.p + m.off[3];
+  if ((int)m.saved.size() < L) m.saved.resize(L);
+
+  // ---------------- forward
+  TRY(piccl_ops_embed_fwd(idx, wte, wpe, b.x0, T, S, C, s));
+  TRY(piccl_ops_ln_fwd(b.x0, nullptr, m.p(0, LN1_G), m.p(0, LN1_B), nullptr, b.layer[0].ln1, b.layer[0].mean1, b.layer[0].rstd1, T, C, d.eps, s));
+  const b16* xin = b.x0;
+  std::vector<at::Tensor> att(L);
+  for (int l = 0; l < L; l++) {
+    Layer& y = b.layer[l]; Layer& z = b.layer[l + 1];
+    DO(product(m, NT, y.ln1, m.p(l, W_QKV), y.qkv, m.p(l, B_QKV), T, 3 * C, C, s));
+    att[l] = attention(m.saved[l], y.qkv, B, S, H, D, train);
+    DO(product(m, NT, static_cast<b16*>(att[l].data_ptr()), m.p(l, W_O), b.a, m.p(l, B_O), T, C, C, s));
+    if (!train) { m.saved[l] = Saved(); att[l] = at::Tensor(); }
+    TRY(piccl_ops_ln_fwd(b.a, xin, m.p(l, LN2_G), m.p(l, LN2_B), y.x2, y.ln2, y.mean2, y.rstd2, T, C, d.eps, s));
+    if (m.backend == 2) {
+      b16* h = y.h ? y.h : y.gl;
+      DO(product(m, NT, y.ln2, m.p(l, W_FC), h, nullptr, T, 4 * C, C, s));
+      TRY(piccl_ops_bias_gelu_fwd(h, m.p(l, B_FC), y.h, y.gl, T, 4 * C, s));
+    } else {
+      TRY(piccl_ops_gemm(NT, EPI_GELU, y.ln2, m.p(l, W_FC), y.gl, y.h, m.p(l, B_FC), nullptr, nullptr, T, 4 * C, C, s));
+      m.tcgen05++;
+    }
+    DO(product(m, NT, y.gl, m.p(l, W_PROJ), b.pr, m.p(l, B_PROJ), T, C, 4 * C, s));
+    const bool last = l + 1 == L;
+    TRY(piccl_ops_ln_fwd(b.pr, y.x2, last ? lnf_g : m.p(l + 1, LN1_G), last ? lnf_b : m.p(l + 1, LN1_B), y.x3, z.ln1, z.mean1, z.rstd1, T, C, d.eps, s));
+    xin = y.x3;
+  }
+  Layer& f = b.layer[L];
+  DO(product(m, NT, f.ln1, wte, b.logits, nullptr, T, d.Vp, C, s));
+  TRY(piccl_ops_ce(b.logits, tgt, b.loss_rows, T, d.V, d.Vp, 1.0f / (float)T, train, s));
+  TRY(piccl_ops_mean(b.loss_rows, loss, T, s));
+  if (!train) return 0;
+
+  // ---------------- backward (logits now hold d loss / d logits)
+  b16 *const g_lnf_g = d.g + m.off[0], *const g_lnf_b = d.g + m.off[1], *const g_wpe = d.g + m.off[2], *const g_wte = d.g + m.off[3];
+  float *const ws2 = b.parts, *const ws1 = ws2 + 3 * row, *const ws_fc = ws1 + 3 * row, *const ws_qkv = ws_fc + fc_floats;
+  auto done = [&](const b16* last_of, size_t n) { if (ready) ready((long long)(last_of - d.g) + (long long)n); };
+  DO(product(m, TN, b.logits, f.ln1, g_wte, nullptr, d.Vp, C, T, s));
+  DO(product(m, NN, b.logits, wte, b.dln, nullptr, T, C, d.Vp, s));
+  TRY(piccl_ops_ln_bwd(b.dln, xin, lnf_g, f.mean1, f.rstd1, nullptr, b.dxa, ws1, 1, T, C, s));
+  {
+    const piccl_finish_job jobs[3] = {{ws1, g_lnf_g, n_ln, C, 0, 0}, {ws1 + row, g_lnf_b, n_ln, C, 0, 0}, {ws1 + 2 * row, m.g(L - 1, B_PROJ), n_ln, C, 0, 0}};
+    TRY(piccl_ops_finish_parts(jobs, 3, s));
+  }
+  done(g_lnf_b, C);
+  for (int l = L - 1; l >= 0; l--) {
+    Layer& y = b.layer[l];
+    // x3 = x2 + gelu(ln2 Wfc + bfc) Wproj + bproj
+    DO(product(m, TN, b.dxa, y.gl, m.g(l, W_PROJ), nullptr, C, 4 * C, T, s));
+    int n_fc = n_fc_own;
+    if (m.backend == 2) {
+      n_fc = n_fc_sep;
+      DO(product(m, NN, b.dxa, m.p(l, W_PROJ), b.dg, nullptr, T, 4 * C, C, s));
+      TRY(piccl_ops_gelu_bwd(b.dg, y.h, b.dg, ws_fc, T, 4 * C, s));
+    } else {
+      TRY(piccl_ops_gemm(NN, EPI_GELU_GRAD, b.dxa, m.p(l, W_PROJ), b.dg, nullptr, nullptr, y.h, ws_fc, T, 4 * C, C, s));
+      m.tcgen05++;
+    }
+    DO(product(m, TN, b.dg, y.ln2, m.g(l, W_FC), nullptr, 4 * C, C, T, s));
+    DO(product(m, NN, b.dg, m.p(l, W_FC), b.dln2, nullptr, T, C, 4 * C, s));
+    TRY(piccl_ops_ln_bwd(b.dln2, y.x2, m.p(l, LN2_G), y.mean2, y.rstd2, b.dxa, b.dxb, ws2, 1, T, C, s));
+    // x2 = xin + attention Wo + bo
+    DO(product(m, TN, b.dxb, static_cast<b16*>(att[l].data_ptr()), m.g(l, W_O), nullptr, C, C, T, s));
+    DO(product(m, NN, b.dxb, m.p(l, W_O), b.datt, nullptr, T, C, C, s));
+    at::Tensor dq[3];
+    attention_grad(m.saved[l], b.datt, B, S, H, D, dq);
+    const void* ptr[3]; long long st[9];
+    for (int i = 0; i < 3; i++) { ptr[i] = dq[i].data_ptr(); for (int j = 0; j < 3; j++) st[3 * i + j] = dq[i].stride(j); }
+    TRY(piccl_ops_qkv_grad(ptr, st, b.dqkv, ws_qkv, B, S, H, D, s));
+    DO(product(m, TN, b.dqkv, y.ln1, m.g(l, W_QKV), nullptr, 3 * C, C, T, s));
+    DO(product(m, NN, b.dqkv, m.p(l, W_QKV), b.dln1, nullptr, T, C, 3 * C, s));
+    TRY(piccl_ops_ln_bwd(b.dln1, l ? b.layer[l - 1].x3 : b.x0, m.p(l, LN1_G), y.mean1, y.rstd1, b.dxb, b.dxa, ws1, l > 0, T, C, s));
+    const piccl_finish_job jobs[8] = {{ws2, m.g(l, LN2_G), n_ln, C, 0, 0}, {ws2 + row, m.g(l, LN2_B), n_ln, C, 0, 0}, {ws2 + 2 * row, m.g(l, B_O), n_ln, C, 0, 0},
+                                      {ws_fc, m.g(l, B_FC), n_fc, 4 * C, 0, 0}, {ws_qkv, m.g(l, B_QKV), n_qkv, 3 * C, 0, 0}, {ws1, m.g(l, LN1_G), n_ln, C, 0, 0},
+                                      {ws1 + row, m.g(l, LN1_B), n_ln, C, 0, 0}, {ws1 + 2 * row, l ? m.g(l - 1, B_PROJ) : nullptr, n_ln, C, 0, 0}};
+    TRY(piccl_ops_finish_parts(jobs, l ? 8 : 7, s));
+    done(m.g(l, B_PROJ), C);
+    m.saved[l] = Saved();
+    att[l] = at::Tensor();
+  }
+  TRY(piccl_ops_wpe_bwd(b.dxa, g_wpe, B, S, C, 0, s));
+  done(g_wpe, (size_t)d.seq_len * C);
+  if (!m.stage.defined()) { m.stage = at::zeros({d.Vp, C}, opt.dtype(at::kFloat)); m.owner = at::zeros({d.Vp}, opt.dtype(at::kInt)); }
+  TRY(piccl_ops_wte_bwd_rows(idx, b.dxa, m.stage.data_ptr<float>(), m.owner.data_ptr<int>(), g_wte, T, C, s));
+  m.launches++;                       // two kernels
+  done(g_wte, (size_t)d.Vp * C);
+  return 0;
+}
+
+}  // namespace
+
+extern "C" {
+
+void* piccl_gpt2_create(const void* desc) {
+  Model* m = new Model();
+  memcpy(&m->d, desc, sizeof(Desc));
+  m->off.assign(m->d.off, m->d.off + 4 + m->d.L * PER_LAYER);
+  return m;
+}
+void piccl_gpt2_destroy(void* h) { delete static_cast<Model*>(h); }
+
+// idx / tgt: int64 [B * S] on the device; loss: one float on the device.  counts[4] (optional): launches of this framework's kernels,
+// products on tcgen05, products on cuBLAS since the last call.  0, or an error code whose text piccl_gpt2_error() holds.
+int piccl_gpt2_run(void* h, const long long* idx, const long long* tgt, int B, int S, float* loss, int train, int backend, ReadyFn ready, long long* counts) {
+  Model& m = *static_cast<Model*>(h);
+  m.launches = m.cublas = m.tcgen05 = 0;
+  m.backend = backend;
+  int rc;
+  try { rc = run(m, idx, tgt, B, S, loss, train != 0, ready); }
+  catch (const std::exception& e) { g_error = e.what(); rc = -1000; }
+  if (counts) { counts[0] = m.launches; counts[1] = m.tcgen05; counts[2] = m.cublas; }
+  return rc;
+}
+const char* piccl_gpt2_error(void) { return g_error.c_str(); }
+
+}  // extern "C"
