@@ -1,9 +1,10 @@
 """Matrix products of the model: y = x W^T (+ bias), dx = dy W, dW = dy^T x.
 
-Two back ends, chosen once per process (`set_backend`):
+Back ends, chosen once per process (`set_backend`):
+  "auto"     (default) the better one for the product at hand: this framework's kernel for small products and
+             wherever its epilogue saves a pass (GELU and its derivative), cuBLAS for large plain ones
   "tcgen05"  this framework's sm_100a kernel (src/ops/gemm_sm100.cu: TMA -> shared memory ->
-             tcgen05.mma with TMEM accumulators) for the forward products whose shapes it
-             supports; everything else through cuBLAS
+             tcgen05.mma with TMEM accumulators) for every product of the training step
   "cublas"   cuBLAS through torch.mm / torch.addmm for all three
 """
 from __future__ import annotations

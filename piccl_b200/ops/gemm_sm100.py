@@ -36,11 +36,12 @@ def _ptr(t) -> C.c_void_p:
     return C.c_void_p(t.data_ptr() if t is not None else 0)
 
 
-def gemm(layout: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bias=None, aux=None, pre=None, part: int = 0) -> torch.Tensor:
-    """The general entry: layouts and epilogues of src/ops/gemm_sm100.cu; `part` is the address of partial_rows(M) x N floats."""
+def gemm(layout: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bias=None, aux=None, pre=None, part: int = 0, ws=None) -> torch.Tensor:
+    """The general entry: layouts and epilogues of src/ops/gemm_sm100.cu; `part` is the address of partial_rows(M) x N floats;
+    `ws` (uint8, its first 64 KiB zero, one stream at a time) lets deep products with few tiles split K."""
     M, Nn = out.shape
     K = a.shape[0] if layout == TN else a.shape[1]
-    rc = N.ops_lib().piccl_ops_gemm(layout, epilogue, _ptr(a), _ptr(b), _ptr(out), _ptr(pre), _ptr(bias), _ptr(aux), C.c_void_p(part), M, Nn, K,
+    rc = N.ops_lib().piccl_ops_gemm(layout, epilogue, _ptr(a), _ptr(b), _ptr(out), _ptr(pre), _ptr(bias), _ptr(aux), C.c_void_p(part), _ptr(ws), C.c_size_t(ws.numel() if ws is not None else 0), M, Nn, K,
                                     C.c_void_p(torch.cuda.current_stream().cuda_stream))
     if rc != 0:
         raise RuntimeError(f"piccl_ops_gemm failed (code {rc}) for layout {layout} epilogue {epilogue} M={M} N={Nn} K={K}")

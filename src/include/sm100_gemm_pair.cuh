@@ -18,12 +18,14 @@
 //              next tile (4096 clocks at K = 1024).
 //
 //   struct Policy {
+//     void begin() const;                                           // every thread, after the set-up (barriers, TMEM) and before global memory is touched
 //     int  num_tiles() const;
 //     void tile(int idx, int v, int& m_blk, int& n_blk) const;     // 128-row block of CTA v (< 0: none), block of TN columns
+//     void k_range(int idx, int num_kb, int& kb0, int& kb1) const; // k-blocks that this entry of the tile order sums, not empty
 //     const CUtensorMap* a_map(int m_blk, int& row0) const;        // tensor map and first row of A for it
 //     bool gate(int m_blk, volatile int* abort) const;             // producer: wait until the row block may be loaded
 //     void prefetch(const EpiCtx&, int m_blk, int n_blk);          // epilogue warps, before they wait for the accumulator
-//     bool epilogue(const EpiCtx&, int m_blk, int n_blk, volatile int* abort);  // called by all eight warps; false: gave up
+//     bool epilogue(const EpiCtx&, int idx, int m_blk, int n_blk, volatile int* abort);  // called by all eight warps; false: gave up
 //   };
 // Every wait is bounded; a wait that runs out sets the status word (1 producer, 2 / 3 MMA issuer, 4 epilogue, 5 gate, 6 policy), every
 // role leaves its loop, copies in flight get time to land, TMEM is released.
@@ -146,6 +148,7 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
   cluster_sync_all();                                       // the partner's barriers exist before anything is signalled across
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pol.begin();                                              // nothing of global memory has been touched so far
 
   if (warp == 0) {
     const bool issuer = elect_one();
@@ -155,8 +158,9 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
       if (!pol.gate(m_blk, s_abort)) { *s_abort = 1; if (issuer) atomicExch(status, 5); break; }
       int row0; const CUtensorMap* ta = pol.a_map(m_blk, row0);
       const int col0 = n_blk * TN + v * (TN / 2);
+      int kb0, kb1; pol.k_range(t, num_kb, kb0, kb1);
       bool ok = true;
-      for (int kb = 0; kb < num_kb; kb++) {
+      for (int kb = kb0; kb < kb1; kb++) {
         if (!mbar_wait(&empty[stage], phase ^ 1, s_abort, kPairWaitLimitNs)) { if (issuer) atomicExch(status, 1); ok = false; break; }
         uint8_t* sa = smem + stage * L::STAGE_BYTES; uint8_t* sb = sa + L::A_BYTES;
         if (issuer) {
@@ -187,8 +191,9 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
         if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, s_abort, kPairWaitLimitNs)) { if (issuer) atomicExch(status, 2); break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN;
+        int kb0, kb1; pol.k_range(t, num_kb, kb0, kb1);
         bool ok = true;
-        for (int kb = 0; kb < num_kb; kb++) {
+        for (int kb = kb0; kb < kb1; kb++) {
           if (!mbar_wait(&full[stage], phase, s_abort, kPairWaitLimitNs)) { if (issuer) atomicExch(status, 3); ok = false; break; }
           tc_fence_after();
           const uint64_t da = desc_advance(da0, stage * L::STAGE_BYTES), db = desc_advance(db0, stage * L::STAGE_BYTES);
@@ -196,7 +201,7 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
             // 16 k are 32 bytes of a K-major row, or 16 rows of 128 bytes of an MN-major box
 #pragma unroll
             for (int k = 0; k < PAIR_BK / 16; k++)
-              umma_f16_pair(d_tmem, desc_advance(da, k * (A_MN ? 2048 : 32)), desc_advance(db, k * (B_MN ? 2048 : 32)), idesc, (kb | k) != 0);
+              umma_f16_pair(d_tmem, desc_advance(da, k * (A_MN ? 2048 : 32)), desc_advance(db, k * (B_MN ? 2048 : 32)), idesc, kb != kb0 || k != 0);
             umma_commit_pair(&empty[stage]);
           }
           __syncwarp();
@@ -219,16 +224,20 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
       pol.prefetch(e, m_blk, n_blk);
       if (!mbar_wait(&tmem_full[acc], acc_phase, s_abort, kPairWaitLimitNs)) { atomicExch(status, 4); break; }
       tc_fence_after();
-      if (!pol.epilogue(e, m_blk, n_blk, s_abort)) { *s_abort = 1; atomicExch(status, 6); break; }
+      if (!pol.epilogue(e, t, m_blk, n_blk, s_abort)) { *s_abort = 1; atomicExch(status, 6); break; }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(&tmem_empty[acc]);      // this warp's part of the accumulator may be overwritten
     }
-    if (lane == 0) bulk_wait_read_all();                        // the stores that this lane issued have read their staging buffer
   }
+  // Neither CTA leaves while the other may still touch its shared memory or barriers, TMEM is freed after the last read of it.  The
+  // arrival goes out before the wait for the stores' reads of the staging buffers, so the two latencies overlap.
   tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();                             // neither CTA leaves while the other may still touch its shared memory or barriers
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (warp >= 2 && lane == 0) bulk_wait_read_all();
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (*s_abort) {
     unsigned long long t0 = gtime_ns();
     while (gtime_ns() - t0 < 2000000ull) __nanosleep(1000);

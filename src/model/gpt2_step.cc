@@ -38,14 +38,18 @@ struct Desc {               // mirrored in piccl_b200/models/gpt2.py
 
 struct Saved { at::Tensor q, k, v, out, lse, cq, ck, seed, offset; c10::SymInt mq = 0, mk = 0; bool direct = false; };
 
+constexpr size_t kSplitBytes = (size_t)40 << 20;
+
 struct Model {
   Desc d;
   std::vector<long long> off;
   at::Tensor arena;         // activations and workspace, grown to the largest shape so far
   at::Tensor stage, owner;  // fp32 table of embedding gradients (all zero between calls), one row of the batch per token id
+  at::Tensor split;         // workspace of the products that split K
+  void* ws = nullptr;
   std::vector<Saved> saved;
   long long launches = 0, cublas = 0, tcgen05 = 0;
-  int backend = 0;          // 0 / 1: this framework's GEMM, 2: cuBLAS
+  int backend = 0;          // 0: by size, 1: this framework's GEMM, 2: cuBLAS
 
   b16* p(int l, int which) const { return d.p + off[4 + l * PER_LAYER + which]; }
   b16* g(int l, int which) const { return d.g + off[4 + l * PER_LAYER + which]; }
@@ -101,15 +105,20 @@ at::Tensor view(b16* p, at::IntArrayRef sizes, at::IntArrayRef strides = {}) {
 }
 
 // C[M, N] = A op B, bf16 row-major: layout NT A [M,K] B [N,K], NN A [M,K] B [K,N], TN A [K,M] B [K,N]
+// Plain products of more than 2 GFLOP go to cuBLAS unless the "tcgen05" backend is asked for: it has more tile shapes to fit ragged sizes
+// to the chip, and under the power cap it draws less for the same tile (GPT-2 medium step 23.5 ms with it, 24.7 without; 8 layers of
+// 768 columns on 3 x 777 tokens 2.97 / 3.10 ms).  Below, the launch counts: this framework's kernel costs a third of the host time and
+// overlaps its set-up with the kernel before it (2 layers of 256 columns 342 us, 500 with cuBLAS).
+constexpr double kOwnProductFlops = 2e9;
 int product(Model& m, int layout, b16* A, b16* B, b16* C, const b16* bias, int M, int N, int K, void* s) {
-  if (m.backend == 2) {
+  if (m.backend == 2 || (m.backend == 0 && 2.0 * M * N * K > kOwnProductFlops)) {
     at::Tensor out = view(C, {M, N});
     at::Tensor a = layout == TN ? view(A, {K, M}).t() : view(A, {M, K}), b = layout == NT ? view(B, {N, K}).t() : view(B, {K, N});
     if (bias) at::addmm_out(out, view(const_cast<b16*>(bias), {N}), a, b); else at::mm_out(out, a, b);
     m.cublas++;
     return 0;
   }
-  TRY(piccl_ops_gemm(layout, EPI_BIAS, A, B, C, nullptr, bias, nullptr, nullptr, M, N, K, s));
+  TRY(piccl_ops_gemm(layout, EPI_BIAS, A, B, C, nullptr, bias, nullptr, nullptr, m.ws, kSplitBytes, M, N, K, s));
   m.tcgen05++;
   return 0;
 }
@@ -162,6 +171,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   Carve c{static_cast<char*>(m.arena.data_ptr())};
   carve(c, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
   b16 *const lnf_g = d.p + m.off[0], *const lnf_b = d.p + m.off[1], *const wpe = d.p + m.off[2], *const wte = d.p + m.off[3];
+  if (!m.split.defined()) { m.split = at::empty({(int64_t)kSplitBytes}, opt.dtype(at::kByte)); m.split.narrow(0, 0, 64 << 10).zero_(); m.ws = m.split.data_ptr(); }
   if ((int)m.saved.size() < L) m.saved.resize(L);
 
   // ---------------- forward
@@ -181,7 +191,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
       DO(product(m, NT, y.ln2, m.p(l, W_FC), h, nullptr, T, 4 * C, C, s));
       TRY(piccl_ops_bias_gelu_fwd(h, m.p(l, B_FC), y.h, y.gl, T, 4 * C, s));
     } else {
-      TRY(piccl_ops_gemm(NT, EPI_GELU, y.ln2, m.p(l, W_FC), y.gl, y.h, m.p(l, B_FC), nullptr, nullptr, T, 4 * C, C, s));
+      TRY(piccl_ops_gemm(NT, EPI_GELU, y.ln2, m.p(l, W_FC), y.gl, y.h, m.p(l, B_FC), nullptr, nullptr, nullptr, 0, T, 4 * C, C, s));
       m.tcgen05++;
     }
     DO(product(m, NT, y.gl, m.p(l, W_PROJ), b.pr, m.p(l, B_PROJ), T, C, 4 * C, s));
@@ -217,7 +227,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
       DO(product(m, NN, b.dxa, m.p(l, W_PROJ), b.dg, nullptr, T, 4 * C, C, s));
       TRY(piccl_ops_gelu_bwd(b.dg, y.h, b.dg, ws_fc, T, 4 * C, s));
     } else {
-      TRY(piccl_ops_gemm(NN, EPI_GELU_GRAD, b.dxa, m.p(l, W_PROJ), b.dg, nullptr, nullptr, y.h, ws_fc, T, 4 * C, C, s));
+      TRY(piccl_ops_gemm(NN, EPI_GELU_GRAD, b.dxa, m.p(l, W_PROJ), b.dg, nullptr, nullptr, y.h, ws_fc, nullptr, 0, T, 4 * C, C, s));
       m.tcgen05++;
     }
     DO(product(m, TN, b.dg, y.ln2, m.g(l, W_FC), nullptr, 4 * C, C, T, s));

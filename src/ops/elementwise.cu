@@ -25,6 +25,7 @@ __device__ __forceinline__ void block_colsum(const float (&acc)[8], float* __res
 // g = gelu(h + bias); h_out = h + bias (kept for the backward pass); h may alias h_out
 __global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const bf16* __restrict__ h, const bf16* __restrict__ bias, bf16* __restrict__ h_out,
                                                             bf16* __restrict__ g, size_t n8, int C8) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
     float v[8], b[8];
     unpack8(reinterpret_cast<const bf16x8*>(h)[i], v);
@@ -43,6 +44,7 @@ __global__ void __launch_bounds__(256) bias_gelu_fwd_kernel(const bf16* __restri
 constexpr int kColRows = 4;      // rows in flight per warp
 __global__ void __launch_bounds__(256) gelu_bwd_kernel(const bf16* __restrict__ dg, const bf16* __restrict__ h, bf16* __restrict__ dh, float* __restrict__ part,
                                                        long long rows, int C) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c8 = blockIdx.x * 32 + lane, C8 = C / 8;
   float acc[8];
@@ -74,6 +76,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const bf16* __restrict__ 
 // strides sb / sh / ss (elements) and contiguous rows of D; part: [gridDim.y][3 * H * D] column sums of what is written.
 struct QkvGrads { const bf16* p[3]; long long sb[3], sh[3], ss[3]; };
 __global__ void __launch_bounds__(256) qkv_grad_kernel(const QkvGrads q, bf16* __restrict__ dqkv, float* __restrict__ part, int rows, int S, int H, int D) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = H * D, C3 = 3 * C;
   const int c = (blockIdx.x * 32 + lane) * 8;
   float acc[8];
@@ -103,6 +106,7 @@ __global__ void __launch_bounds__(256) qkv_grad_kernel(const QkvGrads q, bf16* _
 
 // partial column sums: block (bx, by) sums rows [by*rpb, ...) of 8*32 = 256 columns starting at bx*256
 __global__ void __launch_bounds__(256) colsum_kernel(const bf16* __restrict__ x, float* __restrict__ part, int rows, int C, int rows_per_block) {
+  pdl_begin();
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int c8 = blockIdx.x * 32 + lane;                 // index of the 8-column group
   float acc[8];
@@ -125,6 +129,7 @@ struct FinishJob { const float* part; bf16* out; int nparts, C, accumulate, pad;
 constexpr int kMaxFinish = 16;
 struct FinishJobs { FinishJob j[kMaxFinish]; };
 __global__ void __launch_bounds__(512) finish_parts_kernel(const __grid_constant__ FinishJobs jobs) {
+  pdl_begin();
   const FinishJob& j = jobs.j[blockIdx.y];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = j.C, n = j.nparts;
   const int c = blockIdx.x * 32 + lane;
@@ -156,6 +161,7 @@ __global__ void __launch_bounds__(512) finish_parts_kernel(const __grid_constant
 // (columns V..Vp-1 are padding: ignored in the sum, gradient zero).
 __global__ void __launch_bounds__(512) ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss,
                                                          int V, int Vp, float gscale) {
+  pdl_begin();
   int row = blockIdx.x, tid = threadIdx.x;
   bf16* lp = logits + (size_t)row * Vp;
   const int n8 = Vp / 8;
@@ -208,6 +214,7 @@ __global__ void __launch_bounds__(512) ce_fwd_bwd_kernel(bf16* __restrict__ logi
 // the blocks that share an SM overlap: one loads its row while the other computes.  GRAD = false leaves the logits as they are.
 template <bool GRAD>
 __global__ void __launch_bounds__(512) ce_row_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss, int V, int Vp, float gscale) {
+  pdl_begin();
   extern __shared__ __align__(16) unsigned char ce_smem[];
   bf16x8* const row_s = reinterpret_cast<bf16x8*>(ce_smem);
   __shared__ float sh[16];
@@ -274,6 +281,7 @@ __global__ void __launch_bounds__(512) ce_row_kernel(bf16* __restrict__ logits, 
 
 // out[0] = mean of x[0..n), one block
 __global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ x, float* __restrict__ out, int n) {
+  pdl_begin();
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += 1024) s += x[i];
   __shared__ float sh[32];
@@ -290,6 +298,7 @@ __global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ x,
 __global__ void __launch_bounds__(256) adamw_kernel(bf16* __restrict__ p, float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
                                                     const bf16* __restrict__ g, size_t n8, float lr, float b1, float b2, float eps, float wd,
                                                     float bc1, float bc2, float gscale, const int* __restrict__ step_dev) {
+  pdl_begin();
   if (step_dev) {   // step number kept on the device (the launch can then be replayed from a CUDA graph)
     const float st = (float)*step_dev;
     bc1 = 1.f - powf(b1, st); bc2 = 1.f - powf(b2, st);
@@ -326,6 +335,7 @@ constexpr int kMaxRuns = 1024;
 __global__ void __launch_bounds__(256) adamw_runs_kernel(bf16* __restrict__ p, float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
                                                          const bf16* __restrict__ g, const int* __restrict__ ends, int nruns, int decay_parity, size_t n8,
                                                          float lr, float b1, float b2, float eps, float wd, int* __restrict__ step, unsigned* __restrict__ ticket) {
+  pdl_begin();
   __shared__ int s_end[kMaxRuns];
   for (int i = threadIdx.x; i < nruns; i += 256) s_end[i] = ends[i];
   const float st = (float)(*(volatile int*)step + 1);
@@ -362,6 +372,7 @@ __global__ void __launch_bounds__(256) adamw_runs_kernel(bf16* __restrict__ p, f
 // out[r, :] = wte[idx[r], :] + wpe[r % S, :]
 __global__ void __launch_bounds__(128) embed_fwd_kernel(const long long* __restrict__ idx, const bf16* __restrict__ wte, const bf16* __restrict__ wpe,
                                                         bf16* __restrict__ out, int rows, int S, int C8) {
+  pdl_begin();
   int row = blockIdx.x;
   long long t = idx[row];
   const bf16x8* a = reinterpret_cast<const bf16x8*>(wte) + (size_t)t * C8;
@@ -376,6 +387,7 @@ __global__ void __launch_bounds__(128) embed_fwd_kernel(const long long* __restr
 
 // dwpe[s, :] += sum over batch of dx[b*S + s, :]   (one block per position; deterministic)
 __global__ void __launch_bounds__(128) wpe_bwd_kernel(const bf16* __restrict__ dx, bf16* __restrict__ dwpe, int B, int S, int C8, int accumulate) {
+  pdl_begin();
   int s = blockIdx.x;
   for (int i = threadIdx.x; i < C8; i += blockDim.x) {
     float acc[8];
@@ -395,10 +407,12 @@ __global__ void __launch_bounds__(128) wpe_bwd_kernel(const bf16* __restrict__ d
 
 // dwte[idx[r], :] += dx[r, :] in fp32 (atomics on an fp32 staging table), then folded into the bf16 gradient
 __global__ void __launch_bounds__(128) wte_bwd_scatter_kernel(const long long* __restrict__ idx, const bf16* __restrict__ dx, float* __restrict__ stage, int C) {
+  pdl_begin();
   int row = blockIdx.x; long long t = idx[row];
   for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&stage[(size_t)t * C + c], __bfloat162float(dx[(size_t)row * C + c]));
 }
 __global__ void __launch_bounds__(256) add_f32_into_bf16_kernel(const float* __restrict__ src, bf16* __restrict__ dst, size_t n) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     dst[i] = __float2bfloat16_rn(__bfloat162float(dst[i]) + src[i]);
 }
@@ -406,6 +420,7 @@ __global__ void __launch_bounds__(256) add_f32_into_bf16_kernel(const float* __r
 // dwte[v, :] += sum of dx[r, :] over the rows with idx[r] = v, touching only the rows of the table that occur.  stage (fp32 [V, C]) is
 // all zero before and after; owner[v] names one of the rows that hold v: its block folds the sum and clears it again.
 __global__ void __launch_bounds__(128) wte_scatter_rows_kernel(const long long* __restrict__ idx, const bf16* __restrict__ dx, float* __restrict__ stage, int* __restrict__ owner, int C8) {
+  pdl_begin();
   const int row = blockIdx.x; const long long t = idx[row];
   if (threadIdx.x == 0) owner[t] = row;
   float4* dst = reinterpret_cast<float4*>(stage) + (size_t)t * C8 * 2;
@@ -417,6 +432,7 @@ __global__ void __launch_bounds__(128) wte_scatter_rows_kernel(const long long* 
   }
 }
 __global__ void __launch_bounds__(128) wte_fold_rows_kernel(const long long* __restrict__ idx, float* __restrict__ stage, const int* __restrict__ owner, bf16* __restrict__ dwte, int C8) {
+  pdl_begin();
   const int row = blockIdx.x; const long long t = idx[row];
   if (owner[t] != row) return;
   float4* src = reinterpret_cast<float4*>(stage) + (size_t)t * C8 * 2;
@@ -441,7 +457,7 @@ extern "C" {
 int piccl_ops_bias_gelu_fwd(const void* h, const void* bias, void* h_out, void* g, long long rows, int C, void* stream) {
   if (C % 8) return -1;
   size_t n8 = (size_t)rows * C / 8;
-  bias_gelu_fwd_kernel<<<grid_for(n8, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)h, (const bf16*)bias, (bf16*)h_out, (bf16*)g, n8, C / 8);
+  launch_pdl(bias_gelu_fwd_kernel, grid_for(n8, 256), 256, 0, (cudaStream_t)stream, (const bf16*)h, (const bf16*)bias, (bf16*)h_out, (bf16*)g, n8, C / 8);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // Row groups (partial rows) of the kernels that walk C columns of a [rows, C] matrix 256 at a time: four blocks per SM
@@ -453,7 +469,7 @@ int piccl_ops_col_parts(long long rows, int C) {
 // part: null, or piccl_ops_col_parts(rows, C) * C floats that receive partial column sums of dh
 int piccl_ops_gelu_bwd(const void* dg, const void* h, void* dh, float* part, long long rows, int C, void* stream) {
   if (C % 8) return -1;
-  gelu_bwd_kernel<<<dim3((C + 255) / 256, piccl_ops_col_parts(rows, C)), 256, 0, (cudaStream_t)stream>>>((const bf16*)dg, (const bf16*)h, (bf16*)dh, part, rows, C);
+  launch_pdl(gelu_bwd_kernel, dim3((C + 255) / 256, piccl_ops_col_parts(rows, C)), 256, 0, (cudaStream_t)stream, (const bf16*)dg, (const bf16*)h, (bf16*)dh, part, rows, C);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // g[3]: gradients of q, k, v; strides: {sb, sh, ss} of each in elements (multiples of 8, the rows 16-byte aligned);
@@ -466,7 +482,7 @@ int piccl_ops_qkv_grad(const void* const* g, const long long* strides, void* dqk
     if ((q.sb[i] | q.sh[i] | q.ss[i]) % 8 || (uintptr_t)g[i] % 16) return -2;
   }
   const int C3 = 3 * H * D;
-  qkv_grad_kernel<<<dim3((C3 + 255) / 256, piccl_ops_col_parts((long long)B * S, C3)), 256, 0, (cudaStream_t)stream>>>(q, (bf16*)dqkv, part, B * S, S, H, D);
+  launch_pdl(qkv_grad_kernel, dim3((C3 + 255) / 256, piccl_ops_col_parts((long long)B * S, C3)), 256, 0, (cudaStream_t)stream, q, (bf16*)dqkv, part, B * S, S, H, D);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // Folds the partial rows of up to 16 vectors into their bf16 results in one launch.
@@ -475,14 +491,14 @@ int piccl_ops_finish_parts(const void* jobs, int n, void* stream) {
   FinishJobs a; memset(&a, 0, sizeof a); memcpy(&a, jobs, n * sizeof(FinishJob));
   int c = 0;
   for (int i = 0; i < n; i++) c = a.j[i].C > c ? a.j[i].C : c;
-  finish_parts_kernel<<<dim3((c + 31) / 32, n), 512, 0, (cudaStream_t)stream>>>(a);
+  launch_pdl(finish_parts_kernel, dim3((c + 31) / 32, n), 512, 0, (cudaStream_t)stream, a);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // workspace: ceil(rows / rows_per_block) * C floats
 int piccl_ops_colsum(const void* x, void* out, float* workspace, int rows, int C, int rows_per_block, int accumulate, void* stream) {
   if (C % 8) return -1;
   int nparts = (rows + rows_per_block - 1) / rows_per_block;
-  colsum_kernel<<<dim3((C + 255) / 256, nparts), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, workspace, rows, C, rows_per_block);
+  launch_pdl(colsum_kernel, dim3((C + 255) / 256, nparts), 256, 0, (cudaStream_t)stream, (const bf16*)x, workspace, rows, C, rows_per_block);
   PICCL_OPS_CHECK_LAUNCH();
   const FinishJob j{workspace, (bf16*)out, nparts, C, accumulate, 0};
   return piccl_ops_finish_parts(&j, 1, stream);
@@ -499,9 +515,9 @@ int piccl_ops_ce(void* logits, const long long* targets, float* loss, int rows, 
           cudaFuncSetAttribute(ce_row_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return -4;
       ready[dev] = true;
     }
-    if (grad) ce_row_kernel<true><<<rows, 512, smem, (cudaStream_t)stream>>>((bf16*)logits, targets, loss, V, Vp, gscale);
-    else ce_row_kernel<false><<<rows, 512, smem, (cudaStream_t)stream>>>((bf16*)logits, targets, loss, V, Vp, gscale);
-  } else ce_fwd_bwd_kernel<<<rows, 512, 0, (cudaStream_t)stream>>>((bf16*)logits, targets, loss, V, Vp, gscale);
+    if (grad) launch_pdl(ce_row_kernel<true>, rows, 512, smem, (cudaStream_t)stream, (bf16*)logits, targets, loss, V, Vp, gscale);
+    else launch_pdl(ce_row_kernel<false>, rows, 512, smem, (cudaStream_t)stream, (bf16*)logits, targets, loss, V, Vp, gscale);
+  } else launch_pdl(ce_fwd_bwd_kernel, rows, 512, 0, (cudaStream_t)stream, (bf16*)logits, targets, loss, V, Vp, gscale);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 int piccl_ops_ce_fwd_bwd(void* logits, const long long* targets, float* loss, int rows, int V, int Vp, float gscale, void* stream) {
@@ -509,7 +525,7 @@ int piccl_ops_ce_fwd_bwd(void* logits, const long long* targets, float* loss, in
 }
 int piccl_ops_mean(const float* x, float* out, int n, void* stream) {
   if (n < 1) return -1;
-  mean_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(x, out, n);
+  launch_pdl(mean_kernel, 1, 1024, 0, (cudaStream_t)stream, x, out, n);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // One AdamW step over flat buffers of n elements that alternate between decaying and non-decaying runs: ends[i] (device) is the end of
@@ -518,46 +534,46 @@ int piccl_ops_adamw_runs(void* p, float* master, float* m, float* v, const void*
                          float eps, float wd, int* step, unsigned* ticket, void* stream) {
   if (n % 8 || nruns < 1 || nruns > kMaxRuns || n / 8 > 0x7fffffffll) return -1;
   const size_t n8 = (size_t)n / 8;
-  adamw_runs_kernel<<<grid_for(n8, 256), 256, 0, (cudaStream_t)stream>>>((bf16*)p, master, m, v, (const bf16*)g, ends, nruns, decay_parity, n8, lr, b1, b2, eps, wd, step, ticket);
+  launch_pdl(adamw_runs_kernel, grid_for(n8, 256), 256, 0, (cudaStream_t)stream, (bf16*)p, master, m, v, (const bf16*)g, ends, nruns, decay_parity, n8, lr, b1, b2, eps, wd, step, ticket);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 int piccl_ops_adamw(void* p, float* master, float* m, float* v, const void* g, long long n, float lr, float b1, float b2, float eps, float wd,
                     int step, float gscale, void* stream) {
   if (n % 8) return -1;
   float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-  adamw_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((bf16*)p, master, m, v, (const bf16*)g, (size_t)n / 8, lr, b1, b2, eps, wd, bc1, bc2, gscale, nullptr);
+  launch_pdl(adamw_kernel, grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream, (bf16*)p, master, m, v, (const bf16*)g, (size_t)n / 8, lr, b1, b2, eps, wd, bc1, bc2, gscale, nullptr);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // Same update with the step number read from device memory (`step_dev`, an int the caller advances on the device).
 int piccl_ops_adamw_devstep(void* p, float* master, float* m, float* v, const void* g, long long n, float lr, float b1, float b2, float eps, float wd,
                             const int* step_dev, float gscale, void* stream) {
   if (n % 8 || !step_dev) return -1;
-  adamw_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((bf16*)p, master, m, v, (const bf16*)g, (size_t)n / 8, lr, b1, b2, eps, wd, 1.f, 1.f, gscale, step_dev);
+  launch_pdl(adamw_kernel, grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream, (bf16*)p, master, m, v, (const bf16*)g, (size_t)n / 8, lr, b1, b2, eps, wd, 1.f, 1.f, gscale, step_dev);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 int piccl_ops_embed_fwd(const long long* idx, const void* wte, const void* wpe, void* out, int rows, int S, int C, void* stream) {
   if (C % 8) return -1;
-  embed_fwd_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>(idx, (const bf16*)wte, (const bf16*)wpe, (bf16*)out, rows, S, C / 8);
+  launch_pdl(embed_fwd_kernel, rows, 128, 0, (cudaStream_t)stream, idx, (const bf16*)wte, (const bf16*)wpe, (bf16*)out, rows, S, C / 8);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 int piccl_ops_wpe_bwd(const void* dx, void* dwpe, int B, int S, int C, int accumulate, void* stream) {
   if (C % 8) return -1;
-  wpe_bwd_kernel<<<S, 128, 0, (cudaStream_t)stream>>>((const bf16*)dx, (bf16*)dwpe, B, S, C / 8, accumulate);
+  launch_pdl(wpe_bwd_kernel, S, 128, 0, (cudaStream_t)stream, (const bf16*)dx, (bf16*)dwpe, B, S, C / 8, accumulate);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // stage: fp32 [V, C], zeroed by the caller
 int piccl_ops_wte_bwd(const long long* idx, const void* dx, float* stage, void* dwte, int rows, long long V, int C, void* stream) {
-  wte_bwd_scatter_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>(idx, (const bf16*)dx, stage, C);
+  launch_pdl(wte_bwd_scatter_kernel, rows, 128, 0, (cudaStream_t)stream, idx, (const bf16*)dx, stage, C);
   size_t n = (size_t)V * C;
-  add_f32_into_bf16_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(stage, (bf16*)dwte, n);
+  launch_pdl(add_f32_into_bf16_kernel, grid_for(n, 256), 256, 0, (cudaStream_t)stream, stage, (bf16*)dwte, n);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 
 // stage: fp32 [V, C], all zero (and left so); owner: V ints, any content
 int piccl_ops_wte_bwd_rows(const long long* idx, const void* dx, float* stage, int* owner, void* dwte, int rows, int C, void* stream) {
   if (C % 8) return -1;
-  wte_scatter_rows_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>(idx, (const bf16*)dx, stage, owner, C / 8);
-  wte_fold_rows_kernel<<<rows, 128, 0, (cudaStream_t)stream>>>(idx, stage, owner, (bf16*)dwte, C / 8);
+  launch_pdl(wte_scatter_rows_kernel, rows, 128, 0, (cudaStream_t)stream, idx, (const bf16*)dx, stage, owner, C / 8);
+  launch_pdl(wte_fold_rows_kernel, rows, 128, 0, (cudaStream_t)stream, idx, stage, owner, (bf16*)dwte, C / 8);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 

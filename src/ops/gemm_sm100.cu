@@ -28,23 +28,31 @@ enum Epi : int { EPI_BIAS = 0, EPI_GELU = 1, EPI_RESIDUAL = 2, EPI_GELU_GRAD = 3
 struct GemmArgs {
   CUtensorMap ta, tb, tc, tpre;
   const bf16* bias; const bf16* aux; float* part;
-  int M, N, K, has_pre;
+  float4* split; unsigned* ticket;                     // split K: fp32 partial accumulators, arrivals per tile and warp (all zero between launches)
+  int M, N, K, has_pre, slices;
   int* status;
 };
 
-template <int TN, int EPI>
+template <int TN, int EPI, bool SPLIT>
 struct PlainPolicy {
   const GemmArgs& a;
   int num_m, num_n;                                    // tiles of 256 rows, of TN columns
   __device__ PlainPolicy(const GemmArgs& g) : a(g), num_m((g.M + 2 * PAIR_BM - 1) / (2 * PAIR_BM)), num_n((g.N + TN - 1) / TN) {}
-  __device__ int num_tiles() const { return num_m * num_n; }
+  __device__ void begin() const { pdl_begin(); }
+  __device__ int num_tiles() const { return num_m * num_n * a.slices; }
   // Bands of 16 row tiles, inside a band column tiles outer / row tiles inner: the pairs that run together share a band of A
   // (about 30 MB at K = 3584) that stays in L2 while B streams through once per band.
+  // With K split, the slices of one tile follow each other, so they run at the same time on different pairs.
   __device__ void tile(int idx, int v, int& m_blk, int& n_blk) const {
     constexpr int GM = 16;
+    idx /= a.slices;
     const int per_band = GM * num_n, band = idx / per_band, within = idx % per_band;
     const int rows = min(GM, num_m - band * GM);
     m_blk = 2 * (band * GM + within % rows) + v; n_blk = within / rows;
+  }
+  __device__ void k_range(int idx, int num_kb, int& kb0, int& kb1) const {
+    const int sl = idx % a.slices;
+    kb0 = (int)((long long)num_kb * sl / a.slices); kb1 = (int)((long long)num_kb * (sl + 1) / a.slices);
   }
   __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = m_blk * PAIR_BM; return &a.ta; }
   __device__ bool gate(int, volatile int*) const { return true; }
@@ -86,10 +94,46 @@ struct PlainPolicy {
     if (AUX && (PIECES >= 2 || e.half == 0)) load_aux(e, m_blk, n_blk, first_piece(e));
   }
 
-  __device__ bool epilogue(const EpiCtx& e, int m_blk, int n_blk, volatile int*) {
+  // Split K: every slice leaves its accumulator in fp32; the warp whose slice arrives last (nobody waits) adds the slices in their
+  // order and goes on to the epilogue.  Pieces are kept as the threads hold them, so all accesses are coalesced.
+  __device__ float4* split_at(int tile, int slice, int v8, int piece) const { return a.split + ((((size_t)tile * a.slices + slice) * 16 + v8) * PER + piece) * 512; }
+  __device__ bool last_slice(const EpiCtx& e, int idx, int m_blk, int p0) {
+    const int tile = idx / a.slices, v8 = (m_blk & 1) * 8 + e.half * 4 + e.quarter;
+    for (int pc = p0; pc < p0 + PER; pc++) {
+      float v[64];
+      epi_load64(e, pc * 64, v);
+      float4* dst = split_at(tile, idx % a.slices, v8, pc - p0) + e.lane;
+#pragma unroll
+      for (int j = 0; j < 16; j++) dst[j * 32] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+    __threadfence();
+    __syncwarp();
+    unsigned n = 0;
+    if (e.lane == 0) {
+      n = atomicAdd(a.ticket + tile * 16 + v8, 1u);
+      if (n == (unsigned)a.slices - 1) a.ticket[tile * 16 + v8] = 0;
+    }
+    n = __shfl_sync(0xffffffffu, n, 0);
+    __threadfence();
+    return n == (unsigned)a.slices - 1;
+  }
+  __device__ void add_slices(const EpiCtx& e, int idx, int m_blk, int piece, float (&v)[64]) const {
+    const int tile = idx / a.slices, v8 = (m_blk & 1) * 8 + e.half * 4 + e.quarter;
+#pragma unroll
+    for (int i = 0; i < 64; i++) v[i] = 0.f;
+#pragma unroll 1
+    for (int sl = 0; sl < a.slices; sl++) {
+      const float4* src = split_at(tile, sl, v8, piece) + e.lane;
+#pragma unroll
+      for (int j = 0; j < 16; j++) { const float4 f = __ldcg(src + j * 32); v[4 * j] += f.x; v[4 * j + 1] += f.y; v[4 * j + 2] += f.z; v[4 * j + 3] += f.w; }
+    }
+  }
+
+  __device__ bool epilogue(const EpiCtx& e, int idx, int m_blk, int n_blk, volatile int*) {
     const int row0 = m_blk * PAIR_BM + e.quarter * 32;
     if (row0 >= a.M || (PIECES < 2 && e.half)) return true;
     const int p0 = first_piece(e), p1 = p0 + PER;
+    if (SPLIT && !last_slice(e, idx, m_blk, p0)) return true;
 #pragma unroll 1
     for (int pc = p0; pc < p1; pc++) {
       const int col = n_blk * TN + pc * 64;
@@ -106,7 +150,7 @@ struct PlainPolicy {
         if (pc + 1 < p1) load_aux(e, m_blk, n_blk, pc + 1);
       }
       float v[64];
-      epi_load64(e, pc * 64, v);
+      if (SPLIT) add_slices(e, idx, m_blk, pc - p0, v); else epi_load64(e, pc * 64, v);
       if (EPI != EPI_GELU_GRAD && a.bias) {
 #pragma unroll
         for (int j = 0; j < 8; j++) {
@@ -157,12 +201,12 @@ struct PlainPolicy {
   }
 };
 
-template <int TN, int STAGES, bool A_MN, bool B_MN, int EPI>
+template <int TN, int STAGES, bool A_MN, bool B_MN, int EPI, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) gemm_pair_kernel(const __grid_constant__ GemmArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int s_abort;
   if (threadIdx.x == 0) { s_abort = 0; tma_prefetch_desc(&a.ta); tma_prefetch_desc(&a.tc); }
-  PlainPolicy<TN, EPI> pol(a);
+  PlainPolicy<TN, EPI, SPLIT> pol(a);
   gemm_pair_persistent<TN, STAGES, A_MN, B_MN>(smem_raw, &a.tb, pol, a.K, blockIdx.x >> 1, gridDim.x >> 1, a.status, &s_abort);
 }
 
@@ -190,15 +234,15 @@ static bool get_map(const void* p, long rows, long cols, int box, CUtensorMap* o
 }
 
 typedef void (*GemmFn)(GemmArgs);
-struct Variant { int tn, layout, epi; GemmFn fn; int smem; bool ready[64]; };
-#define V_(TN, ST, L, AM, BM_, E) {TN, L, E, gemm_pair_kernel<TN, ST, AM, BM_, E>, PairSmem<TN, ST>::DYNAMIC, {false}}
+struct Variant { int tn, layout, epi, split; GemmFn fn; int smem; bool ready[64]; };
+#define V_(TN, ST, L, E, SP) {TN, L, E, SP, gemm_pair_kernel<TN, ST, L == 2, L != 0, E, SP != 0>, PairSmem<TN, ST>::DYNAMIC, {false}}
 static Variant g_variants[] = {
-  V_(256, 6, 0, false, false, EPI_BIAS), V_(128, 8, 0, false, false, EPI_BIAS), V_(64, 9, 0, false, false, EPI_BIAS),
-  V_(256, 6, 0, false, false, EPI_GELU), V_(128, 8, 0, false, false, EPI_GELU), V_(64, 9, 0, false, false, EPI_GELU),
-  V_(256, 6, 0, false, false, EPI_RESIDUAL), V_(128, 8, 0, false, false, EPI_RESIDUAL), V_(64, 9, 0, false, false, EPI_RESIDUAL),
-  V_(256, 6, 1, false, true, EPI_BIAS), V_(128, 8, 1, false, true, EPI_BIAS),
-  V_(256, 6, 1, false, true, EPI_GELU_GRAD), V_(128, 8, 1, false, true, EPI_GELU_GRAD),
-  V_(256, 6, 2, true, true, EPI_BIAS), V_(128, 8, 2, true, true, EPI_BIAS),
+  V_(256, 6, 0, EPI_BIAS, 0), V_(128, 8, 0, EPI_BIAS, 0), V_(64, 9, 0, EPI_BIAS, 0), V_(256, 6, 0, EPI_BIAS, 1), V_(128, 8, 0, EPI_BIAS, 1),
+  V_(256, 6, 0, EPI_GELU, 0), V_(128, 8, 0, EPI_GELU, 0), V_(64, 9, 0, EPI_GELU, 0),
+  V_(256, 6, 0, EPI_RESIDUAL, 0), V_(128, 8, 0, EPI_RESIDUAL, 0), V_(64, 9, 0, EPI_RESIDUAL, 0),
+  V_(256, 6, 1, EPI_BIAS, 0), V_(128, 8, 1, EPI_BIAS, 0), V_(256, 6, 1, EPI_BIAS, 1), V_(128, 8, 1, EPI_BIAS, 1),
+  V_(256, 6, 1, EPI_GELU_GRAD, 0), V_(128, 8, 1, EPI_GELU_GRAD, 0),
+  V_(256, 6, 2, EPI_BIAS, 0), V_(128, 8, 2, EPI_BIAS, 0), V_(256, 6, 2, EPI_BIAS, 1), V_(128, 8, 2, EPI_BIAS, 1),
 };
 #undef V_
 
@@ -226,16 +270,24 @@ static int device_ready(int dev) {
   return 0;
 }
 
-// Tile width: waves of the persistent grid times the clocks of a tile.  A k-step of 16 takes the larger of the MMA (TN / 4 clocks) and
-// reading the operands out of shared memory (128 rows of A and TN / 2 of B at 128 bytes a clock: 32 + TN / 8), which favours wide
-// tiles (64 against 48 clocks for twice the columns) until the tiles no longer fill the pairs; ten clocks a column for the epilogue.
-static Variant* choose(int layout, int epi, int M, int N, int K, int pairs) {
+// Tile width and slices of K: waves of the persistent grid times the clocks of a tile.  A k-step of 16 takes 136 / 68 / 51 clocks at
+// 256 / 128 / 64 columns (measured; the MMA alone needs TN / 2), which favours wide tiles until they no longer fill the pairs.
+// K is split where the tiles of a deep product leave pairs idle (weight gradients, few rows): a slice then writes its accumulator and
+// the last one reads the others' (about 30 clocks a column and slice: 1024 x 1024 x 8192 gains, 23.1 -> 18.7 us, 3072 x 1024 x 8192 does not).  A slice keeps at least 8 k-blocks.
+constexpr size_t kTicketBytes = 64 * 1024;
+static size_t split_bytes(long tiles, int slices, int tn) { return kTicketBytes + (size_t)tiles * slices * 256 * tn * 4; }
+static Variant* choose(int layout, int epi, int M, int N, int K, int pairs, size_t ws_bytes, int* slices) {
   Variant* best = nullptr; double best_cost = 0;
+  const int kb = (K + PAIR_BK - 1) / PAIR_BK;
   for (auto& v : g_variants) {
     if (v.layout != layout || v.epi != epi) continue;
     const long tiles = (long)((M + 255) / 256) * ((N + v.tn - 1) / v.tn);
-    const double cost = (double)((tiles + pairs - 1) / pairs) * ((32 + v.tn / 8) * ((K + 15) / 16) + 10.0 * v.tn);
-    if (!best || cost < best_cost) { best = &v; best_cost = cost; }
+    const double step = v.tn == 256 ? 136 : v.tn == 128 ? 68 : 51;
+    for (int s = v.split ? 2 : 1; s <= (v.split ? 16 : 1) && (s == 1 || kb / s >= 8); s++) {
+      if (s > 1 && (split_bytes(tiles, s, v.tn) > ws_bytes || tiles * 64 > (long)kTicketBytes)) break;
+      const double cost = (double)((tiles * s + pairs - 1) / pairs) * (step * 4 * ((kb + s - 1) / s) + 10.0 * v.tn) + (s > 1 ? 30.0 * v.tn * (s + 1) : 0);
+      if (!best || cost < best_cost) { best = &v; best_cost = cost; *slices = s; }
+    }
   }
   return best;
 }
@@ -245,8 +297,10 @@ static Variant* choose(int layout, int epi, int M, int N, int K, int pairs) {
 extern "C" {
 
 // Row-major, contiguous bf16 operands, 16-byte aligned, rows a multiple of 16 bytes.  bias [N], aux / pre [M, N] or null as the epilogue
-// says; part: [ceil(M / 32)][N] floats or null.  Returns 0 on launch, a negative code if the shape is unsupported or set-up failed.
-int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, void* pre, const void* bias, const void* aux, float* part, int M, int N, int K, void* stream) {
+// says; part: [ceil(M / 32)][N] floats or null; ws: workspace of ws_bytes for splitting K, its first 64 KiB zero (and left so), used by
+// one stream at a time, or null.  Returns 0 on launch, a negative code if the shape is unsupported or set-up failed.
+int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, void* pre, const void* bias, const void* aux, float* part, void* ws, size_t ws_bytes, int M, int N, int K,
+                   void* stream) {
   using namespace piccl_ops;
   if (layout < 0 || layout > 2 || M <= 0 || N <= 0 || K <= 0 || N % 8 || (layout != 2 && K % 8) || (layout == 2 && M % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(pre) |
@@ -255,7 +309,8 @@ int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, v
   int dev = 0; cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return -6;
   int rc = device_ready(dev); if (rc) return rc;
-  Variant* v = choose(layout, epi, M, N, K, g_pairs[dev]);
+  int slices = 1;
+  Variant* v = choose(layout, epi, M, N, K, g_pairs[dev], ws ? ws_bytes : 0, &slices);
   if (!v) return -1;
   if (!v->ready[dev]) {
     if (cudaFuncSetAttribute((const void*)v->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v->smem) != cudaSuccess) return -4;
@@ -268,11 +323,11 @@ int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, v
   a.has_pre = pre != nullptr;
   if (pre) { if (!get_map(pre, M, N, 32, &a.tpre)) return -3; } else a.tpre = a.tc;
   a.bias = (const bf16*)bias; a.aux = (const bf16*)aux; a.part = part;
+  a.slices = slices; a.ticket = (unsigned*)ws; a.split = (float4*)((char*)ws + kTicketBytes);
   a.M = M; a.N = N; a.K = K; a.status = g_status[dev];
-  const long tiles = (long)((M + 255) / 256) * ((N + v->tn - 1) / v->tn);
+  const long tiles = (long)((M + 255) / 256) * ((N + v->tn - 1) / v->tn) * slices;
   const int pairs = (int)(tiles < g_pairs[dev] ? tiles : g_pairs[dev]);
-  void* args[] = {&a};
-  return cudaLaunchKernel((const void*)v->fn, dim3(2 * pairs), dim3(PAIR_THREADS), args, v->smem, (cudaStream_t)stream) == cudaSuccess ? 0 : -5;
+  return launch_pdl(v->fn, dim3(2 * pairs), dim3(PAIR_THREADS), v->smem, (cudaStream_t)stream, a) == cudaSuccess ? 0 : -5;
 }
 
 // C = act(A · B^T + bias).  A [M,K], B [N,K], C [M,N], all bf16 row-major and contiguous; bias [N] bf16 or null;
@@ -281,7 +336,7 @@ int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, v
 int piccl_ops_gemm_bf16_nt_ex(const void* A, const void* B, void* C, void* c_pre, const void* bias, int M, int N, int K, int gelu, void* stream) {
   using namespace piccl_ops;
   if (M <= 0 || N <= 0 || K <= 0 || M % 128 || N % 128 || K % 64) return -1;
-  return piccl_ops_gemm(0, gelu ? EPI_GELU : EPI_BIAS, A, B, C, c_pre, bias, nullptr, nullptr, M, N, K, stream);
+  return piccl_ops_gemm(0, gelu ? EPI_GELU : EPI_BIAS, A, B, C, c_pre, bias, nullptr, nullptr, nullptr, 0, M, N, K, stream);
 }
 int piccl_ops_gemm_bf16_nt(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int gelu, void* stream) {
   return piccl_ops_gemm_bf16_nt_ex(A, B, C, nullptr, bias, M, N, K, gelu, stream);

@@ -11,6 +11,7 @@ template <int V>   // V 16-byte vectors per lane: C = 256 * V
 __global__ void __launch_bounds__(128) ln_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, const bf16* __restrict__ gamma,
                                                      const bf16* __restrict__ beta, bf16* __restrict__ sum_out, bf16* __restrict__ y,
                                                      float* __restrict__ mean, float* __restrict__ rstd, int rows, float eps) {
+  pdl_begin();
   const int C = 256 * V;
   int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -61,6 +62,7 @@ template <int V, int G, int R>   // C = 256 * V
 __global__ void __launch_bounds__(32 * V * G, 2) ln_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ xin, const bf16* __restrict__ gamma,
                                                                const float* __restrict__ mean, const float* __restrict__ rstd, const bf16* __restrict__ dres,
                                                                bf16* __restrict__ dx, float* __restrict__ part, int rows, int with_dsum) {
+  pdl_begin();
   constexpr int C = 256 * V;
   __shared__ float red[2][G][V][2 * R];
   __shared__ float sh[G][C];
@@ -166,7 +168,7 @@ int piccl_ops_ln_fwd(const void* x, const void* res, const void* gamma, const vo
                      int rows, int C, float eps, void* stream) {
   dim3 grid((rows + 3) / 4), block(128);
   cudaStream_t s = (cudaStream_t)stream;
-#define LN_CASE(V) case 256 * V: ln_fwd_kernel<V><<<grid, block, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)gamma, (const bf16*)beta, (bf16*)sum_out, (bf16*)y, mean, rstd, rows, eps); break;
+#define LN_CASE(V) case 256 * V: launch_pdl(ln_fwd_kernel<V>, grid, block, 0, s, (const bf16*)x, (const bf16*)res, (const bf16*)gamma, (const bf16*)beta, (bf16*)sum_out, (bf16*)y, mean, rstd, rows, eps); break;
   switch (C) { LN_CASE(1) LN_CASE(2) LN_CASE(3) LN_CASE(4) LN_CASE(5) LN_CASE(6) LN_CASE(8) default: return -1; }
 #undef LN_CASE
   PICCL_OPS_CHECK_LAUNCH();
@@ -187,7 +189,7 @@ int piccl_ops_ln_bwd(const void* dy, const void* xin, const void* gamma, const f
   const int nb = piccl_ops_ln_bwd_parts(rows, C);
   if (!nb) return -1;
   cudaStream_t s = (cudaStream_t)stream;
-#define LN_CASE(V, G) case 256 * V: ln_bwd_kernel<V, G, 2><<<nb, 32 * V * G, 0, s>>>((const bf16*)dy, (const bf16*)xin, (const bf16*)gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, part, rows, with_dsum); break;
+#define LN_CASE(V, G) case 256 * V: launch_pdl(ln_bwd_kernel<V, G, 2>, nb, 32 * V * G, 0, s, (const bf16*)dy, (const bf16*)xin, (const bf16*)gamma, mean, rstd, (const bf16*)dres, (bf16*)dx, part, rows, with_dsum); break;
   switch (C) { LN_CASE(1, 8) LN_CASE(2, 4) LN_CASE(3, 2) LN_CASE(4, 2) default: return -1; }
 #undef LN_CASE
   PICCL_OPS_CHECK_LAUNCH();

@@ -8,6 +8,24 @@ namespace piccl_ops {
 
 typedef __nv_bfloat16 bf16;
 
+// Programmatic dependent launch: the grid may start while the kernel before it on the stream still runs; what it does before
+// pdl_begin() overlaps that kernel's tail, everything after it sees the kernel before completed.  A step is hundreds of kernels of 2 to
+// 50 us, so the launch latency between two of them (1 us and more) counts.  Every kernel launched by launch_pdl calls pdl_begin()
+// before it touches global memory, reads as well as writes.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 struct alignas(16) bf16x8 { __nv_bfloat162 v[4]; };
 
 __device__ __forceinline__ void unpack8(const bf16x8& p, float (&f)[8]) {

@@ -1,5 +1,6 @@
 // C interface of the model kernels (libpiccl_ops.so) that the native training step calls; each returns 0 or an error code.
 #pragma once
+#include <stddef.h>
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -7,7 +8,7 @@ int piccl_ops_embed_fwd(const long long* idx, const void* wte, const void* wpe, 
 int piccl_ops_ln_fwd(const void* x, const void* res, const void* gamma, const void* beta, void* sum_out, void* y, float* mean, float* rstd, int rows, int C, float eps, void* stream);
 int piccl_ops_ln_bwd_parts(int rows, int C);
 int piccl_ops_ln_bwd(const void* dy, const void* xin, const void* gamma, const float* mean, const float* rstd, const void* dres, void* dx, float* part, int with_dsum, int rows, int C, void* stream);
-int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, void* pre, const void* bias, const void* aux, float* part, int M, int N, int K, void* stream);
+int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, void* pre, const void* bias, const void* aux, float* part, void* ws, size_t ws_bytes, int M, int N, int K, void* stream);
 int piccl_ops_bias_gelu_fwd(const void* h, const void* bias, void* h_out, void* g, long long rows, int C, void* stream);
 int piccl_ops_gelu_bwd(const void* dg, const void* h, void* dh, float* part, long long rows, int C, void* stream);
 int piccl_ops_col_parts(long long rows, int C);
