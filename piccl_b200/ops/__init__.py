@@ -26,8 +26,12 @@ def _bump(n: int = 1) -> None:
     _launches += n
 
 
-def _s() -> int:
-    return torch.cuda.current_stream().cuda_stream
+def current_stream_ptr(device=None) -> int:
+    """The raw handle of the current stream (of the current device), without building a Stream object (0.2 us instead of 3.4)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice() if device is None else device)
+
+
+_s = current_stream_ptr
 
 
 def _p(t: Optional[torch.Tensor]) -> C.c_void_p:

@@ -6,7 +6,7 @@ import ctypes as C
 import torch
 
 from .. import _native as N
-from . import _bump
+from . import _bump, _s
 
 _checked = None
 
@@ -32,8 +32,25 @@ def supports(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
             and out.is_contiguous() and x.shape[1] % 8 == 0 and w.shape[1] % 8 == 0 and out.shape[1] % 8 == 0)
 
 
-def _ptr(t) -> C.c_void_p:
-    return C.c_void_p(t.data_ptr() if t is not None else 0)
+_fn: dict = {}
+
+
+def _native(name: str, argtypes):
+    """A function of the library with its argument types declared, so that plain integers pass (half the cost of building ctypes objects)."""
+    f = _fn.get(name)
+    if f is None:
+        f = getattr(N.ops_lib(), name)
+        f.argtypes = argtypes
+        _fn[name] = f
+    return f
+
+
+_GEMM = [C.c_int] * 2 + [C.c_void_p] * 8 + [C.c_size_t] + [C.c_int] * 3 + [C.c_void_p]
+_GEMM_NT = [C.c_void_p] * 5 + [C.c_int] * 4 + [C.c_void_p]
+
+
+def _ptr(t):
+    return None if t is None else t.data_ptr()
 
 
 def gemm(layout: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bias=None, aux=None, pre=None, part: int = 0, ws=None) -> torch.Tensor:
@@ -41,8 +58,8 @@ def gemm(layout: int, epilogue: int, a: torch.Tensor, b: torch.Tensor, out: torc
     `ws` (uint8, its first 64 KiB zero, one stream at a time) lets deep products with few tiles split K."""
     M, Nn = out.shape
     K = a.shape[0] if layout == TN else a.shape[1]
-    rc = N.ops_lib().piccl_ops_gemm(layout, epilogue, _ptr(a), _ptr(b), _ptr(out), _ptr(pre), _ptr(bias), _ptr(aux), C.c_void_p(part), _ptr(ws), C.c_size_t(ws.numel() if ws is not None else 0), M, Nn, K,
-                                    C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    rc = _native("piccl_ops_gemm", _GEMM)(layout, epilogue, a.data_ptr(), b.data_ptr(), out.data_ptr(), _ptr(pre), _ptr(bias), _ptr(aux), part or None, _ptr(ws),
+                                          ws.numel() if ws is not None else 0, M, Nn, K, _s())
     if rc != 0:
         raise RuntimeError(f"piccl_ops_gemm failed (code {rc}) for layout {layout} epilogue {epilogue} M={M} N={Nn} K={K}")
     _bump()
@@ -58,7 +75,7 @@ def gemm_nt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias=None, gelu
     """out[M, N] = act(x[M, K] @ w[N, K]^T + bias); `pre` (optional) receives the value before the activation"""
     M, K = x.shape
     Nn = w.shape[0]
-    rc = N.ops_lib().piccl_ops_gemm_bf16_nt_ex(_ptr(x), _ptr(w), _ptr(out), _ptr(pre), _ptr(bias), M, Nn, K, int(gelu), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    rc = _native("piccl_ops_gemm_bf16_nt_ex", _GEMM_NT)(x.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(pre), _ptr(bias), M, Nn, K, gelu, _s())
     if rc != 0:
         raise RuntimeError(f"piccl_ops_gemm_bf16_nt failed (code {rc}) for M={M} N={Nn} K={K}")
     _bump()

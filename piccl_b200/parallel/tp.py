@@ -25,8 +25,8 @@ def _declare():
     lib.piccl_tp_workspace_bytes.restype = C.c_longlong
     lib.piccl_gemm_rs.argtypes = [vp, vp, vp, vp, i, i, i, vp]
     lib.piccl_ag_gemm.argtypes = [vp, vp, vp, vp, i, i, i, vp]
-    lib.piccl_gemm_rs_group.argtypes = [C.POINTER(vp), i, C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), i, i, i, vp]
-    lib.piccl_ag_gemm_group.argtypes = [C.POINTER(vp), i, C.POINTER(vp), C.POINTER(vp), C.POINTER(vp), i, i, i, vp]
+    lib.piccl_gemm_rs_group.argtypes = [vp, i, vp, vp, vp, i, i, i, vp]
+    lib.piccl_ag_gemm_group.argtypes = [vp, i, vp, vp, vp, i, i, i, vp]
     lib.piccl_tp_status.argtypes = [vp]
     lib._tp_declared = True
     return lib
@@ -63,12 +63,7 @@ def tp_status(comm_or_handle) -> int:
 
 def _group(fn_name, g: LoopbackGroup, As, Bs, outs, M, N_, K, stream):
     lib = _declare()
-    n = g.nranks
-    comms = (C.c_void_p * n)(*[h.value for h in g._hs])
-    a = (C.c_void_p * n)(*[t.data_ptr() for t in As])
-    b = (C.c_void_p * n)(*[t.data_ptr() for t in Bs])
-    o = (C.c_void_p * n)(*[t.data_ptr() for t in outs])
-    N.check(getattr(lib, fn_name)(comms, n, a, b, o, M, N_, K, _stream_ptr(stream)), fn_name)
+    N.check(getattr(lib, fn_name)(g.handles(), g.nranks, g.table(As), g.table(Bs), g.table(outs), M, N_, K, _stream_ptr(stream)), fn_name)
 
 
 def gemm_rs_group(g: LoopbackGroup, As, Bs, outs, stream=None):

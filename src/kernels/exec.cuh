@@ -22,7 +22,7 @@ namespace piccl {
 constexpr int kFlagStride = 128;          // bytes between two counters
 constexpr int kMaxVRanks = 8;             // virtual ranks one launch can carry (single-GPU emulation)
 constexpr int kMaxBlock = 512;
-constexpr int kLLFifoCta = 8, kLLFifoSlots = 8, kLLFifoSlotBytes = 8192;   // low-latency FIFO: CTAs, ring depth, bytes per slot (half of it payload)
+constexpr int kLLFifoCta = 16, kLLFifoSlots = 8, kLLFifoSlotBytes = 8192;   // low-latency FIFO: CTAs, ring depth, bytes per slot (half of it payload)
 
 struct RankCtx {
   int rank, nranks, max_cta, nslot;

@@ -240,7 +240,7 @@ __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, 
 }
 
 // ---------------------------------------------------------------- the kernel
-constexpr int kSliceCache = 192;      // actions whose CTA slice is precomputed in shared memory
+constexpr int kSliceCache = 192;      // actions whose CTA slice is precomputed in shared memory (the low-latency executor: the actions themselves)
 
 // DEFER = true (PICCL_EXEC_DEFER=1) postpones the counter updates that end an action: a release store to another GPU waits
 // for the action's data to be acknowledged (a round trip through the switch), and a chain of independent actions, such as the

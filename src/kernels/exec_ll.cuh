@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
 
   __shared__ unsigned s_send_seq[kMaxRanks], s_recv_seq[kMaxRanks];
   __shared__ char* s_heap[kMaxRanks];
+  __shared__ Action s_act[kSliceCache];
   __shared__ int s_fail, s_maxseg;
 
   const int rank = ctx->rank, nranks = ctx->nranks;
@@ -41,7 +42,11 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
   const long long seg_elems = (kPayload / 16) * (16 / esz);
   {
     int m = 0;
-    for (int ai = tid; ai < L.n_actions; ai += blockDim.x) m = max(m, slice_of(L.actions[ai].count, esz, cta, ka.n_cta, kPayload).nseg);
+    for (int ai = tid; ai < L.n_actions; ai += blockDim.x) {
+      const Action a = L.actions[ai];
+      if (ai < kSliceCache) s_act[ai] = a;
+      m = max(m, slice_of(a.count, esz, cta, ka.n_cta, kPayload).nseg);
+    }
     if (m) atomicMax(&s_maxseg, m);
   }
   __syncthreads();
@@ -53,7 +58,7 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
 
   for (int seg = 0; seg < maxseg && !failed; seg++) {
     for (int ai = 0; ai < L.n_actions; ai++) {
-      const Action ac = L.actions[ai];
+      const Action& ac = ai < kSliceCache ? s_act[ai] : L.actions[ai];
       const Slice sl = slice_of(ac.count, esz, cta, ka.n_cta, kPayload);
       const long long lo = sl.lo + (long long)seg * seg_elems;
       if (lo >= sl.hi) continue;

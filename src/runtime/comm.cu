@@ -394,6 +394,47 @@ static bool fault_now(piccl_comm* c) {
   return false;
 }
 
+// CTAs of a low-latency kernel: one line per thread as far as the SMs go (a thread takes its lines one after the other, each with its
+// own round trip: 32 KiB among eight ranks 12.3 us with four lines a thread, 6.3 us with one), never fewer than the kernel's most lines per thread need.
+static int ll_ctas(long long nlines, int most_lines, int sms) {
+  const long long spread = std::min<long long>((nlines + kLLBlock - 1) / kLLBlock, std::max(1, sms));
+  return (int)std::max(spread, (nlines + most_lines - 1) / most_lines);
+}
+
+// Fills `out` with the call-independent part of a low-latency all-reduce; false: the schedule is not one of exchanges among all ranks.
+static bool ll_plan(piccl_comm** comms, int n, Algo algo, int k, LLArgs* out) {
+  piccl_comm* c0 = comms[0];
+  std::lock_guard<std::mutex> l(c0->mu);
+  for (const LLPlan& p : c0->ll_plans) {
+    if (p.n != n || p.algo != (int)algo || p.k != k) continue;
+    bool same = true;
+    for (int i = 0; i < n; i++) same &= p.ranks[i] == comms[i]->rank;
+    if (same) { if (p.usable) *out = p.args; return p.usable; }
+  }
+  LLPlan p; memset(&p, 0, sizeof p);
+  p.n = n; p.algo = (int)algo; p.k = k;
+  for (int i = 0; i < n; i++) p.ranks[i] = comms[i]->rank;
+  const Resolved rs = resolve(COLL_ALLREDUCE, algo, k, c0->nranks);
+  p.usable = rs.core == c0->nranks && !rs.radices.empty() && (int)rs.radices.size() <= kLLMaxSteps && rs.algo == algo;
+  if (p.usable) {
+    const bool permuted = algo == ALGO_PRD || algo == ALGO_PRM;
+    p.args.n_vrank = n; p.args.nsteps = (int)rs.radices.size();
+    for (int i = 0; i < n; i++)
+      for (int s = 0; s < p.args.nsteps; s++) {
+        std::vector<int> pe = step_peers(comms[i]->rank, s, rs.radices, c0->nranks, permuted);
+        std::sort(pe.begin(), pe.end());
+        p.args.npeers[s] = (uint8_t)pe.size();
+        int below = 0;
+        for (size_t j = 0; j < pe.size(); j++) { p.args.peers[i][s][j] = (uint8_t)pe[j]; if (pe[j] < comms[i]->rank) below++; }
+        p.args.self_pos[i][s] = (uint8_t)below;
+      }
+  }
+  if (c0->ll_plans.size() >= 64) c0->ll_plans.clear();      // a program uses a handful of algorithms
+  c0->ll_plans.push_back(p);
+  if (p.usable) *out = p.args;
+  return p.usable;
+}
+
 struct CallDesc { Coll coll; const void* send; void* recv; size_t count; int dtype, op, root; Algo algo; int k; };
 
 // Runs one collective over `n` communicators of this process (n == 1: the normal case).
@@ -435,29 +476,20 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
   if (cudaStreamIsCapturing(stream, &cap_state) != cudaSuccess) { cudaGetLastError(); cap_state = cudaStreamCaptureStatusNone; }
   if (cap_state == cudaStreamCaptureStatusNone && d0.coll == COLL_ALLREDUCE && c0->ll_max_bytes > 0 && (long long)d0.count * esz_real <= c0->ll_max_bytes &&
       (d0.algo == ALGO_RD || d0.algo == ALGO_RM || d0.algo == ALGO_PRD || d0.algo == ALGO_PRM)) {
-    Resolved rs = resolve(COLL_ALLREDUCE, d0.algo, d0.k, c0->nranks);
     LLKernelFn lf = ll_kernel_for(d0.dtype, op);
-    if (rs.core == c0->nranks && !rs.radices.empty() && (int)rs.radices.size() <= kLLMaxSteps && rs.algo == d0.algo && lf) {
-      const bool permuted = d0.algo == ALGO_PRD || d0.algo == ALGO_PRM;
-      LLArgs la; memset(&la, 0, sizeof la);
-      la.n_vrank = n; la.nsteps = (int)rs.radices.size(); la.avg = avg ? 1 : 0; la.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
+    LLArgs la;
+    if (lf && ll_plan(comms, n, d0.algo, d0.k, &la)) {
+      la.avg = avg ? 1 : 0; la.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
       la.count = (long long)d0.count; la.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
       const int E = 8 / esz_real;
       long long nlines = ((long long)d0.count + E - 1) / E;
-      la.n_cta = (int)((nlines + ll_lines_per_cta() - 1) / ll_lines_per_cta());
+      // (the persistent server is one CTA: what fits one goes to it)
+      la.n_cta = env().launch_persistent && nlines <= ll_lines_per_cta() ? 1 : ll_ctas(nlines, ll_lines_per_cta(), c0->sm_count / n);
       if (n * la.n_cta <= c0->sm_count) {
         bool skip = false;
         for (int i = 0; i < n; i++) {
           piccl_comm* c = comms[i];
           std::lock_guard<std::mutex> l(c->mu);
-          for (int s = 0; s < la.nsteps; s++) {
-            std::vector<int> pe = step_peers(c->rank, s, rs.radices, c->nranks, permuted);
-            std::sort(pe.begin(), pe.end());
-            la.npeers[s] = (uint8_t)pe.size();
-            int below = 0;
-            for (size_t j = 0; j < pe.size(); j++) { la.peers[i][s][j] = (uint8_t)pe[j]; if (pe[j] < c->rank) below++; }
-            la.self_pos[i][s] = (uint8_t)below;
-          }
           la.r[i].ctx = c->d_ctx; la.r[i].in = calls[i].send; la.r[i].out = calls[i].recv;
           la.epoch = ++c->ll_epoch;
           c->stats.launches++; c->stats.calls[COLL_ALLREDUCE]++; c->stats.bytes[COLL_ALLREDUCE] += (unsigned long long)d0.count * esz_real;
@@ -492,7 +524,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     xa.count = d0.coll == COLL_ALLGATHER ? (long long)d0.count * esz_real : (long long)d0.count;
     xa.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
     const long long nlines = d0.coll == COLL_ALLGATHER ? (xa.count + 7) / 8 : ((long long)d0.count + (8 / esz_real) - 1) / (8 / esz_real);
-    xa.n_cta = (int)((nlines + llx_lines_per_cta() - 1) / llx_lines_per_cta());
+    xa.n_cta = ll_ctas(nlines, llx_lines_per_cta(), c0->sm_count / n);
     if (xf && esz_real <= 8 && n * xa.n_cta <= c0->sm_count) {
       bool skip = false;
       for (int i = 0; i < n; i++) {
@@ -549,10 +581,18 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
   // slabs: bound the local scratch of the recursive reduce-scatters
   long long slab = count, stride = 0;
   if (d0.coll == COLL_REDUCE_SCATTER) {
-    CollArgs probe; probe.coll = d0.coll; probe.algo = d0.algo; probe.k = d0.k; probe.nranks = c0->nranks; probe.count = count; probe.elem_size = esz;
-    Program p = compile(probe, 0);
-    if (p.scratch_elems * esz > c0->h_ctx.scratch_bytes) {
-      long long blocks = (p.scratch_elems + count - 1) / count + 1;
+    const ProgKey pk{(int)d0.coll, (int)d0.algo, d0.k, 0, esz, 0, count, 0};
+    long long scratch_elems = -1;
+    { std::lock_guard<std::mutex> l(c0->mu); auto it = c0->scratch_need.find(pk); if (it != c0->scratch_need.end()) scratch_elems = it->second; }
+    if (scratch_elems < 0) {
+      CollArgs probe; probe.coll = d0.coll; probe.algo = d0.algo; probe.k = d0.k; probe.nranks = c0->nranks; probe.count = count; probe.elem_size = esz;
+      scratch_elems = compile(probe, 0).scratch_elems;
+      std::lock_guard<std::mutex> l(c0->mu);
+      if (c0->scratch_need.size() >= 65536) c0->scratch_need.clear();
+      c0->scratch_need.emplace(pk, scratch_elems);
+    }
+    if (scratch_elems * esz > c0->h_ctx.scratch_bytes) {
+      long long blocks = (scratch_elems + count - 1) / count + 1;
       slab = c0->h_ctx.scratch_bytes / esz / blocks / 64 * 64;
       if (slab <= 0) return fail(PICCL_UNSUPPORTED, "scratch too small");
       stride = count;
@@ -581,11 +621,11 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       rc = get_program(c, a, stream, &pe); if (rc) break;
       if (i == 0) {
         n_cta = choose_cta(c, a, n);
-        if (use_llf) {   // 4 KiB of payload per CTA and segment, at most kLLFifoCta CTAs
+        if (use_llf) {   // a line (8 bytes) per thread and action while there are CTAs, then several; a segment holds 4 KiB
           long long ab = a.count * a.elem_size;
           if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) ab /= std::max(1, a.nranks);
           if (a.algo == ALGO_DIRECT && a.coll != COLL_ALLGATHER && a.coll != COLL_REDUCE_SCATTER) ab /= std::max(1, a.coll == COLL_ALLREDUCE ? a.nranks : a.nranks - 1);
-          n_cta = (int)std::max<long long>(1, std::min<long long>((ab + 4095) / 4096, kLLFifoCta));
+          n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
           if (n > 1) n_cta = std::min(n_cta, std::max(1, c->sm_count / n));
         }
         ka.n_cta = n_cta; ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;

@@ -37,6 +37,10 @@ struct ProgKeyHash {
 struct ProgEntry { const Action* dev = nullptr; int n_actions = 0; long long scratch_elems = 0; cudaEvent_t ready = nullptr; cudaStream_t origin = nullptr; bool synced = false; };
 struct ProgChunk { char* dev = nullptr; char* host = nullptr; size_t cap = 0, used = 0; };
 
+// What a low-latency all-reduce of one algorithm and radix looks like for the communicators of a launch: the arguments that do not
+// change from call to call (schedule arithmetic with a dozen small vectors), kept by the first communicator.
+struct LLPlan { int n, algo, k, ranks[kMaxVRanks]; bool usable; LLArgs args; };
+
 struct TraceRec { int coll, algo, k, n_cta; long long bytes; double host_us; cudaEvent_t start = nullptr, stop = nullptr; };
 
 struct TuneRow { int coll, nranks; long long max_bytes; Algo algo; int k; };
@@ -64,6 +68,8 @@ struct piccl_comm {
   piccl_stats_t stats{};
   std::unordered_map<piccl::ProgKey, piccl::ProgEntry, piccl::ProgKeyHash> cache;
   std::vector<piccl::ProgChunk> chunks;
+  std::vector<piccl::LLPlan> ll_plans;                                                     // bounded, see comm.cu
+  std::unordered_map<piccl::ProgKey, long long, piccl::ProgKeyHash> scratch_need;          // scratch elements of a reduce-scatter by its arguments
   std::vector<piccl::TraceRec> trace;
   std::mutex mu;
 };

@@ -302,3 +302,30 @@ def test_bounded_wait_reports_instead_of_hanging():
     # the context is still usable
     assert float((x + 1).sum()) == 32.0
     g.close()
+
+
+@pytest.mark.parametrize("count", [511, 512, 513, 9215, 9216, 9217, 18 * 512 * 4])
+@pytest.mark.parametrize("coll,algo", [("allreduce", "PRM"), ("allgather", "DIRECT"), ("reduce_scatter", "DIRECT"), ("broadcast", "RING"), ("allgather", "RING")])
+def test_low_latency_lines_spread_over_ctas(count, coll, algo):
+    """Eight ranks leave 18 CTAs each: one line of 8 bytes per thread up to 18 x 256 lines (9216 fp32 elements), several beyond; the executor's low-latency
+    variant spreads over up to 16 CTAs.  Sums of eight values below 1 in fp32: each of the seven additions errs by at most 2^-24 x 8."""
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    n = 8
+    g = LoopbackGroup(n, config=make_config(max_cta=8, nslot=2, slot_bytes=4096, scratch_bytes=1 << 20, timeout_ms=5000))
+    n_in = count * n if coll == "reduce_scatter" else count
+    n_out = count * n if coll == "allgather" else count
+    for seed in range(3):                                   # both parities of the call epoch
+        xs = _inputs(n, n_in, torch.float32, seed=seed)
+        outs = [torch.full((n_out,), float("nan"), device="cuda") for _ in range(n)]
+        g.run(coll, xs, outs, count, op="sum", algo=algo, k=8)
+        _check_ok(g)
+        for r in range(n):
+            if coll == "allgather":
+                assert torch.equal(outs[r], torch.cat(xs))
+            elif coll == "broadcast":
+                assert torch.equal(outs[r], xs[0])
+            else:
+                ref = _ref_reduce(xs, "sum")
+                ref = ref[r * count:(r + 1) * count] if coll == "reduce_scatter" else ref
+                assert torch.allclose(outs[r], ref, atol=7 * 8 * 2.0 ** -24, rtol=0)
+    g.close()
