@@ -10,12 +10,13 @@
 // Operand layouts: K-major (rows of 64 k, one 128-byte swizzled row each) or MN-major (the operand lies transposed: 64 k-rows of
 // 64 elements each per box), so C = A B^T, C = A B and C = A^T B need no transposed copy.
 //
-// Roles inside a CTA of 320 threads:
+// Roles inside a CTA of 320 threads (352 with a policy's extra warp):
 //   warp 0     TMA producer; the bytes of both CTAs are counted on the LEADER's `full` barrier
 //   warp 1     TMEM allocation; in the leader one lane issues the MMAs and commits to the barriers of both CTAs
 //   warps 2-9  epilogue: warp w reads TMEM lanes of quarter w & 3, columns of half (w - 2) / 4, through 64-column pieces.
 //              Eight warps, because an epilogue of a few dozen instructions per element has to fit under the main loop of the
 //              next tile (4096 clocks at K = 1024).
+//   warp 10    Policy::extra_warp, where the policy has one (EXTRA_BYTES > 0: shared memory it gets)
 //
 //   struct Policy {
 //     void begin() const;                                           // every thread, after the set-up (barriers, TMEM) and before global memory is touched
@@ -26,10 +27,12 @@
 //     bool gate(int m_blk, volatile int* abort) const;             // producer: wait until the row block may be loaded
 //     void prefetch(const EpiCtx&, int m_blk, int n_blk);          // epilogue warps, before they wait for the accumulator
 //     bool epilogue(const EpiCtx&, int idx, int m_blk, int n_blk, volatile int* abort);  // called by all eight warps; false: gave up
+//     static constexpr int EXTRA_BYTES; void extra_warp(uint8_t* smem, int lane, volatile int* abort);           // all lanes of warp 10
 //   };
 // Every wait is bounded; a wait that runs out sets the status word (1 producer, 2 / 3 MMA issuer, 4 epilogue, 5 gate, 6 policy), every
 // role leaves its loop, copies in flight get time to land, TMEM is released.
 #pragma once
+#include <cuda_bf16.h>
 #include "sm100_ptx.cuh"
 
 namespace sm100 {
@@ -39,12 +42,13 @@ constexpr int PAIR_STAGING = 4096;                                  // bytes of 
 constexpr unsigned long long kPairWaitLimitNs = 4000000000ull;      // 4 s
 constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;      // clears the bit that tells the two CTAs of a pair apart in a shared::cluster address
 
-template <int TN, int STAGES>
+template <int TN, int STAGES, int EXTRA_BYTES = 0>
 struct PairSmem {
   static constexpr int A_BYTES = PAIR_BM * PAIR_BK * 2, B_BYTES = (TN / 2) * PAIR_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;
   static constexpr int BAR_OFF = STAGING_OFF + PAIR_EPI_WARPS * PAIR_STAGING;
-  static constexpr int TOTAL = BAR_OFF + (2 * STAGES + 4) * 8 + 16;
+  static constexpr int EXTRA_OFF = (BAR_OFF + (2 * STAGES + 4) * 8 + 16 + 127) / 128 * 128;
+  static constexpr int TOTAL = EXTRA_OFF + EXTRA_BYTES;
   static constexpr int DYNAMIC = TOTAL + 1024;                      // slack for the 1024-byte alignment of the tiles
   static_assert(DYNAMIC <= 232448, "more shared memory than a CTA can have");
 };
@@ -117,10 +121,31 @@ __device__ __forceinline__ void epi_load64(const EpiCtx& e, int col0, float (&v)
   for (int i = 0; i < 32; i++) { v[i] = __uint_as_float(r0[i]); v[32 + i] = __uint_as_float(r1[i]); }
 }
 
+// 64 bf16 of this thread's row -> the warp's staging buffer: 16-byte pieces XOR-ed with the row, conflict free and the layout that a
+// store through a 128-byte swizzled map of 32 x 64 boxes expects
+__device__ __forceinline__ void epi_stage_row(const EpiCtx& e, const float (&v)[64]) {
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
+    *reinterpret_cast<uint4*>(e.staging + e.lane * 128 + ((j ^ (e.lane & 7)) << 4)) = o;
+  }
+  fence_proxy_async();                                 // these stores must be visible to the bulk-copy engine
+  __syncwarp();
+}
+__device__ __forceinline__ void epi_ship(const EpiCtx& e, const CUtensorMap* map, int x, int y) {
+  if (e.lane == 0) { tma_store_2d(map, e.staging, x, y); bulk_commit(); }
+}
+__device__ __forceinline__ void epi_staging_free(const EpiCtx& e) {
+  if (e.lane == 0) bulk_wait_read_all();               // the last store has been read out of the staging buffer
+  __syncwarp();
+}
+
 template <int TN, int STAGES, bool A_MN, bool B_MN, class Policy>
 __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CUtensorMap* tmap_b, Policy& pol, int K, int first_tile, int tile_stride,
                                                      int* status, volatile int* s_abort) {
-  typedef PairSmem<TN, STAGES> L;
+  typedef PairSmem<TN, STAGES, Policy::EXTRA_BYTES> L;
   static_assert(!B_MN || TN >= 128, "an MN-major half of B is at least one box of 64 columns");
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
@@ -212,6 +237,8 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
         __syncwarp();
       }
     }
+  } else if (Policy::EXTRA_BYTES > 0 && warp >= 2 + PAIR_EPI_WARPS) {
+    if constexpr (Policy::EXTRA_BYTES > 0) pol.extra_warp(smem + L::EXTRA_OFF, lane, s_abort);
   } else {
     EpiCtx e;
     e.quarter = warp & 3; e.half = (warp - 2) >> 2; e.lane = lane;
@@ -235,7 +262,7 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
   tc_fence_before();
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  if (warp >= 2 && lane == 0) bulk_wait_read_all();
+  if (warp >= 2 && lane == 0) bulk_wait_read_all();            // (the extra warp has waited for its own copies)
   __syncwarp();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (*s_abort) {

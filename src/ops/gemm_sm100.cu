@@ -57,26 +57,7 @@ struct PlainPolicy {
   __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = m_blk * PAIR_BM; return &a.ta; }
   __device__ bool gate(int, volatile int*) const { return true; }
 
-  // 64 bf16 of one row -> this warp's staging buffer (16-byte pieces XOR-ed with the row: conflict free, and the layout the store's map expects)
-  __device__ static void stage_row(const EpiCtx& e, const float (&v)[64]) {
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-      for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
-      *reinterpret_cast<uint4*>(e.staging + e.lane * 128 + ((j ^ (e.lane & 7)) << 4)) = o;
-    }
-    fence_proxy_async();                               // these stores must be visible to the bulk-copy engine
-    __syncwarp();
-  }
-  __device__ static void ship(const EpiCtx& e, const CUtensorMap* map, int x, int y) {
-    if (e.lane == 0) { tma_store_2d(map, e.staging, x, y); bulk_commit(); }
-  }
-  __device__ static void staging_free(const EpiCtx& e) {
-    if (e.lane == 0) bulk_wait_read_all();             // the last store has been read out of the staging buffer
-    __syncwarp();
-  }
-
+  static constexpr int EXTRA_BYTES = 0;
   static constexpr bool AUX = EPI == EPI_RESIDUAL || EPI == EPI_GELU_GRAD;
   static constexpr int PIECES = TN / 64;               // 64-column pieces of the tile; the halves of the warps share them
   static constexpr int PER = PIECES >= 2 ? PIECES / 2 : 1;
@@ -139,7 +120,7 @@ struct PlainPolicy {
       const int col = n_blk * TN + pc * 64;
       if (col >= a.N) break;
       uint4 y[8];                                      // this thread's row of aux
-      staging_free(e);
+      epi_staging_free(e);
       if (AUX) {
 #pragma unroll
         for (int i = 0; i < 8; i++) { const int r = 4 * i + (e.lane >> 3); *reinterpret_cast<uint4*>(e.staging + r * 128 + (((e.lane & 7) ^ (r & 7)) << 4)) = x[i]; }
@@ -177,16 +158,16 @@ struct PlainPolicy {
         }
       }
       if (EPI == EPI_GELU) {
-        if (a.has_pre) { stage_row(e, v); ship(e, &a.tpre, col, row0); }
+        if (a.has_pre) { epi_stage_row(e, v); epi_ship(e, &a.tpre, col, row0); }
         if (a.has_pre) {                               // of the value as stored, which the backward pass sees
 #pragma unroll
           for (int i = 0; i < 64; i++) v[i] = __bfloat162float(__float2bfloat16_rn(v[i]));
         }
         gelu_n(v);
-        if (a.has_pre) staging_free(e);
+        if (a.has_pre) epi_staging_free(e);
       }
-      stage_row(e, v);
-      ship(e, &a.tc, col, row0);
+      epi_stage_row(e, v);
+      epi_ship(e, &a.tc, col, row0);
       if (EPI == EPI_GELU_GRAD && a.part) {            // two columns a lane, down the 32 rows of the staging buffer (rows beyond M hold zeros)
         float s0 = 0.f, s1 = 0.f;
 #pragma unroll

@@ -1,18 +1,21 @@
 // Fused tensor-parallel kernels: one launch does the tcgen05 GEMM AND the
 // collective that follows or precedes it, tile by tile, over peer memory.
+// Both run on the CTA-pair core of sm100_gemm_pair.cuh.
 //
 //  gemm_rs   C = A_r · B_r^T per rank, summed over ranks, row block r kept by rank r.
-//            Every CTA runs the persistent GEMM; tiles owned by OTHER ranks come first and their
-//            epilogue stores the bf16 partial tile straight into the owner's heap (plain peer
-//            stores over NVLink) and raises a per-(source, tile) epoch flag.  The rank's OWN tiles
-//            come last: their epilogue waits (bounded) for the n-1 partials of that tile, adds them
-//            in rank order to the accumulator it just read from TMEM, and writes the final result.
+//            Row blocks owned by OTHER ranks come first: an epilogue warp ships each piece of 32 rows x 64
+//            columns as bf16 with one 4 KiB bulk store into the owner's heap, the last of the tile's eight
+//            warps raises a per-(source, tile) epoch flag.  The rank's OWN blocks come last: their epilogue
+//            waits (bounded) for the n-1 partials of that tile, adds them in rank order to the accumulator it
+//            just read from TMEM, and writes the final result.
 //            No partial of an own tile ever goes to memory; transfer overlaps the remaining MMA work.
-//  ag_gemm   A is row-sharded over ranks; C = concat(A_r) · B^T.  A few "feeder" CTAs push this
-//            rank's shard, 128 rows at a time, into every peer's gathered buffer (nearest consumer
-//            first) and raise per-(source, row block) flags; the GEMM CTAs start on the local shard
-//            and gate the TMA loads of a remote row block on its flag.  TMA only ever reads LOCAL
-//            memory (the local shard or the local gathered buffer), never a peer's.
+//  ag_gemm   A is row-sharded over ranks; C = concat(A_r) · B^T.  One more warp in EVERY CTA pushes parts of
+//            this rank's shard into every peer's gathered buffer (the peer that needs them next first) with
+//            bulk copies through a small ring in shared memory, and raises per-part flags; it takes neither an SM nor
+//            issue slots from the products.  (24 CTAs set aside for it cost a sixth of the SMs for the whole call:
+//            two ranks of 4096 x 2048 x 4096 166 us.)  The GEMM starts on the local shard and gates the TMA
+//            loads of a remote row block on its flags.  TMA only ever reads LOCAL memory (the local
+//            shard or the local gathered buffer), never a peer's.
 //
 // Buffers are double buffered by call parity, flags carry the call epoch, so nothing is reset
 // between calls.  All waits are bounded; a wait that gives up is reported through
@@ -20,15 +23,15 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cstring>
-#include "../include/sm100_gemm.cuh"
+#include "../include/sm100_gemm_pair.cuh"
 #include "../runtime/comm.h"
 
 namespace piccl {
 
 using namespace sm100;
 typedef __nv_bfloat16 bf16;
-constexpr int TP_BN = 256, TP_STAGES = 4, TP_MAX_RANKS = 8;
-constexpr int RS_STAGES = 3, RS_STAGING = GEMM_BM * TP_BN * 2;   // reduce-scatter: one ring stage gives way to a 64 KiB staging tile
+constexpr int TP_BN = 256, RS_STAGES = 6, AG_STAGES = 5, TP_MAX_RANKS = 8;
+constexpr int TP_BM = PAIR_BM, TP_BK = PAIR_BK;
 
 __device__ __forceinline__ unsigned ld_acquire_sys_u32(const unsigned* p) {
   unsigned v; asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v;
@@ -44,7 +47,7 @@ __device__ __forceinline__ bool wait_flag(const unsigned* flag, unsigned epoch, 
     if ((it & 63u) == 0) {
       if (*abort_flag) return false;
       unsigned long long now = gtime_ns();
-      if (!t0) t0 = now; else if (now - t0 > kGemmWaitLimitNs) return false;
+      if (!t0) t0 = now; else if (now - t0 > kPairWaitLimitNs) return false;
     }
   }
 }
@@ -53,6 +56,7 @@ struct TpRank {
   CUtensorMap ta;            // gemm_rs: A [M, K_local];   ag_gemm: local shard [M/n, K]
   CUtensorMap ta2;           // ag_gemm: gathered buffer [2*M, K] in this rank's heap
   CUtensorMap tb;
+  CUtensorMap tc;            // this rank's output, boxes of 32 rows x 64 columns
   char* heap[TP_MAX_RANKS];  // all ranks' heaps as mapped here
   const bf16* a_shard;       // ag_gemm: the local shard (feeder source)
   bf16* out;
@@ -61,7 +65,7 @@ struct TpRank {
 };
 struct TpArgs {
   int n, M, N, K;            // gemm_rs: K = K_local, N full;  ag_gemm: N = N_local, K full
-  int ctas_per_rank, n_feed;
+  int ctas_per_rank, n_part; // ag_gemm: parts of a row block, each with a flag of its own
   unsigned epoch;
   long long flag_off, data_off;
   TpRank r[TP_MAX_RANKS];    // one entry per virtual rank of the launch
@@ -69,177 +73,243 @@ struct TpArgs {
 
 // ------------------------------------------------------------------ GEMM -> reduce-scatter
 struct RsPolicy {
-  const TpRank* R; int n, rank, N, mb_per_owner, num_n, tiles_per_owner, parity; unsigned epoch;
-  long long flag_off, data_off; int* s_ok; uint8_t* staging;
-  static constexpr int STAGING = RS_STAGING;
-  __device__ void set_staging(uint8_t* p) { staging = p; }
-  // A tile travels as 128 rows of 512 bytes; inside every 128-byte group the 16-byte pieces are XOR-ed with the
-  // row number, which makes the epilogue's shared-memory stores conflict free.  Writer and reader use the same map.
-  __device__ static int piece_off(int row, int piece) { return row * (TP_BN * 2) + (((piece & ~7) | ((piece & 7) ^ (row & 7))) << 4); }
-  __device__ int num_tiles() const { return n * tiles_per_owner; }
-  // Order: panels of 16 column blocks (one panel of B stays in L2); inside a panel the owners (rank+1, rank+2, ..., myself
-  // last); inside an owner's block rows fastest.  All ranks walk the panels in the same order, so the partials of my own
-  // tiles of a panel are on their way while I still compute the other owners' tiles of that panel.
-  __device__ void tile(int idx, int& m_blk, int& n_blk) const {
+  const TpRank* R; int n, rank, mb_per_owner, num_n, parity; unsigned epoch;
+  long long flag_off, data_off; unsigned* s_arrived;
+  int row_pairs, tiles_per_owner, group;
+  int seq = 0;
+  static constexpr int EXTRA_BYTES = 0;
+  __device__ RsPolicy(const TpArgs& a, const TpRank* r, unsigned* arrived)
+      : R(r), n(a.n), rank(r->rank), mb_per_owner(a.M / a.n / TP_BM), num_n(a.N / TP_BN), parity((int)(a.epoch & 1)), epoch(a.epoch), flag_off(a.flag_off), data_off(a.data_off),
+        s_arrived(arrived), row_pairs((a.M / TP_BM + 1) / 2), tiles_per_owner(mb_per_owner * num_n), group(min(16, (mb_per_owner + 1) / 2)) {}
+  __device__ void begin() const {}
+  __device__ int num_tiles() const { return row_pairs * num_n; }
+  // Row blocks in the order rank+1, rank+2, ..., myself last, two to a pair.  Panels of 16 column blocks (one panel of B stays in
+  // L2); inside a panel groups of row pairs (about one owner), inside a group rows fastest.  All ranks walk the panels in the same order, so the
+  // partials of my own tiles of a panel are on their way while I still compute the other owners' tiles of that panel.
+  // No cycle of waits: within a panel an own tile comes after every remote tile of its column, and what the remote tile that it
+  // waits for comes after are own tiles of earlier panels, or of earlier columns in the one group that holds both kinds.
+  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) const {
     constexpr int PN = 16;
-    const int per_panel = PN * mb_per_owner * n;              // tiles of a full panel
-    const int panel = idx / per_panel; int within = idx % per_panel;
+    const int per_panel = PN * row_pairs, panel = idx / per_panel;
+    int within = idx % per_panel;
     const int cols = min(PN, num_n - panel * PN);             // last panel may be narrower
-    const int per_owner = cols * mb_per_owner;
-    const int owner = (rank + 1 + within / per_owner) % n; within %= per_owner;
-    m_blk = owner * mb_per_owner + within % mb_per_owner; n_blk = panel * PN + within / mb_per_owner;
+    const int g = within / (group * cols); within %= group * cols;
+    const int rows = min(group, row_pairs - g * group);
+    const int i = 2 * (g * group + within % rows) + v;        // position in the order of row blocks
+    n_blk = panel * PN + within / rows;
+    m_blk = i < n * mb_per_owner ? (rank + 1 + i / mb_per_owner) % n * mb_per_owner + i % mb_per_owner : -1;
   }
-  __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = m_blk * GEMM_BM; return &R->ta; }
+  __device__ void k_range(int, int num_kb, int& kb0, int& kb1) const { kb0 = 0; kb1 = num_kb; }
+  __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = max(m_blk, 0) * TP_BM; return &R->ta; }
   __device__ bool gate(int, volatile int*) const { return true; }
   __device__ int tile_id(int m_blk, int n_blk) const { return (m_blk % mb_per_owner) + n_blk * mb_per_owner; }
-  __device__ unsigned* flag_ptr(int owner, int src, int tid_) const {
-    return reinterpret_cast<unsigned*>(R->heap[owner] + flag_off) + ((size_t)(parity * n + src) * tiles_per_owner + tid_);
+  __device__ unsigned* flag_ptr(int owner, int src, int t) const {
+    return reinterpret_cast<unsigned*>(R->heap[owner] + flag_off) + ((size_t)(parity * n + src) * tiles_per_owner + t);
   }
-  __device__ bf16* inbox(int owner, int src, int tid_) const {
-    return reinterpret_cast<bf16*>(R->heap[owner] + data_off) + ((size_t)src * tiles_per_owner + tid_) * (size_t)(GEMM_BM * TP_BN);      // data_off: this call's half of the region
+  // A tile travels as pieces of 32 rows x 64 columns: 4 KiB each, the 16-byte words of a row 512 bytes apart, so that both the
+  // staging stores of the writer and the loads of the reader take consecutive words.  data_off: this call's half of the region.
+  __device__ char* piece(int owner, int src, int t, const EpiCtx& e, int pc) const {
+    return R->heap[owner] + data_off + ((size_t)src * tiles_per_owner + t) * (size_t)(TP_BM * TP_BN * 2) + (e.quarter * 4 + pc) * PAIR_STAGING;
   }
-  __device__ bool tile_begin(int m_blk, int n_blk, int et, volatile int* abort_flag) {
-    if (m_blk / mb_per_owner != rank) return true;
-    // own tile: all other ranks' partials of this tile must have landed
-    if (et == 0) *s_ok = 1;
-    epilogue_barrier();
-    if (et < n && et != rank && !wait_flag(flag_ptr(rank, et, tile_id(m_blk, n_blk)), epoch, abort_flag)) *s_ok = 0;
-    epilogue_barrier();
-    return *s_ok != 0;
-  }
-  __device__ void store(int m_blk, int n_blk, int row, int col0, float (&v)[32]) {
+  __device__ void prefetch(const EpiCtx&, int, int) {}
+  __device__ bool epilogue(const EpiCtx& e, int, int m_blk, int n_blk, volatile int* abort_flag) {
+    const int slot = seq++ & 1;
+    if (m_blk < 0) return true;
     const int owner = m_blk / mb_per_owner, t = tile_id(m_blk, n_blk);
     if (owner != rank) {
-      // remote tile: into the staging tile; tile_end ships it with one bulk store
+#pragma unroll 1
+      for (int pc = e.half * 2; pc < e.half * 2 + 2; pc++) {
+        float v[64];
+        epi_load64(e, pc * 64, v);
+        epi_staging_free(e);
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+        for (int j = 0; j < 8; j++) {
+          uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-        for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
-        *reinterpret_cast<uint4*>(staging + piece_off(row, col0 / 8 + j)) = o;
+          for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
+          *reinterpret_cast<uint4*>(e.staging + j * 512 + e.lane * 16) = o;
+        }
+        fence_proxy_async();                             // these stores must be visible to the bulk-copy engine
+        __syncwarp();
+        if (e.lane == 0) { bulk_store(piece(owner, rank, t, e, pc), e.staging, PAIR_STAGING); bulk_commit(); }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these stores must be visible to the bulk-copy engine
-      return;
-    }
-    float sum[32];
-#pragma unroll
-    for (int i = 0; i < 32; i++) sum[i] = 0.f;
-    for (int src = 0; src < n; src++) {            // rank order: the same result whatever the arrival order
-      if (src == rank) {
-#pragma unroll
-        for (int i = 0; i < 32; i++) sum[i] += v[i];
-      } else {
-        const char* tile = reinterpret_cast<const char*>(inbox(rank, src, t));
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          uint4 b;
-          asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "l"(tile + piece_off(row, col0 / 8 + j)) : "memory");
-          const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
-#pragma unroll
-          for (int q = 0; q < 4; q++) { float2 f = __bfloat1622float2(b2[q]); sum[8 * j + 2 * q] += f.x; sum[8 * j + 2 * q + 1] += f.y; }
+      if (e.lane == 0) {
+        bulk_wait_all();                                 // data written; the last of the eight warps tells the owner
+        asm volatile("fence.proxy.async;" ::: "memory");
+        __threadfence_system();
+        if (atomicAdd(&s_arrived[slot], 1u) == PAIR_EPI_WARPS - 1) {
+          s_arrived[slot] = 0;                           // used again two tiles on, after every warp has left this one
+          __threadfence_system();
+          st_release_sys_u32(flag_ptr(owner, rank, t), epoch);
         }
       }
+      __syncwarp();
+      return true;
     }
-    store_row32_bf16(R->out + (size_t)((m_blk % mb_per_owner) * GEMM_BM + row) * N + (size_t)n_blk * TP_BN + col0, sum);
-  }
-  __device__ void tile_end(int m_blk, int n_blk, int et) {
-    const int owner = m_blk / mb_per_owner;
-    if (owner == rank) return;
-    // all 128 threads have written the staging tile (barrier passed): one asynchronous bulk store moves the 64 KiB over NVLink
-    if (et == 0) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      bulk_store(inbox(owner, rank, tile_id(m_blk, n_blk)), staging, RS_STAGING);
-      bulk_commit();
-      bulk_wait_all();                              // data written; then tell the owner
-      asm volatile("fence.proxy.async;" ::: "memory");
-      st_release_sys_u32(flag_ptr(owner, rank, tile_id(m_blk, n_blk)), epoch);
+    // own tile: all other ranks' partials of this tile must have landed
+    const bool ok = e.lane >= n || e.lane == rank || wait_flag(flag_ptr(rank, e.lane, t), epoch, abort_flag);
+    if (!__all_sync(0xffffffffu, ok)) return false;
+#pragma unroll 1
+    for (int pc = e.half * 2; pc < e.half * 2 + 2; pc++) {
+      float sum[64];
+#pragma unroll
+      for (int i = 0; i < 64; i++) sum[i] = 0.f;
+#pragma unroll 1
+      for (int src = 0; src < n; src++) {                // rank order: the same result whatever the arrival order
+        if (src == rank) {
+          float v[64];
+          epi_load64(e, pc * 64, v);
+#pragma unroll
+          for (int i = 0; i < 64; i++) sum[i] += v[i];
+        } else {
+          const char* p = piece(rank, src, t, e, pc) + e.lane * 16;
+          uint4 w[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++)
+            asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[j].x), "=r"(w[j].y), "=r"(w[j].z), "=r"(w[j].w) : "l"(p + j * 512) : "memory");
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&w[j]);
+#pragma unroll
+            for (int q = 0; q < 4; q++) { float2 f = __bfloat1622float2(b2[q]); sum[8 * j + 2 * q] += f.x; sum[8 * j + 2 * q + 1] += f.y; }
+          }
+        }
+      }
+      epi_staging_free(e);
+      epi_stage_row(e, sum);
+      epi_ship(e, &R->tc, n_blk * TP_BN + pc * 64, (m_blk % mb_per_owner) * TP_BM + e.quarter * 32);
     }
-    epilogue_barrier();                             // the staging tile is free again
+    return true;
   }
 };
 
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_rs_kernel(const __grid_constant__ TpArgs a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) gemm_rs_kernel(const __grid_constant__ TpArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ int s_abort, s_ok;
+  __shared__ int s_abort;
+  __shared__ unsigned s_arrived[2];
   const int vr = blockIdx.x / a.ctas_per_rank, cta = blockIdx.x % a.ctas_per_rank;
   const TpRank* R = &a.r[vr];
-  if (threadIdx.x == 0) { s_abort = 0; s_ok = 1; tma_prefetch_desc(&R->ta); }
-  RsPolicy pol{R, a.n, R->rank, a.N, a.M / a.n / GEMM_BM, a.N / TP_BN, (a.M / a.n / GEMM_BM) * (a.N / TP_BN), (int)(a.epoch & 1), a.epoch, a.flag_off, a.data_off, &s_ok, nullptr};
-  gemm_persistent<TP_BN, RS_STAGES>(smem_raw, &R->tb, pol, a.K, cta, a.ctas_per_rank, R->status, &s_abort);
+  if (threadIdx.x == 0) { s_abort = 0; s_arrived[0] = 0; s_arrived[1] = 0; tma_prefetch_desc(&R->ta); tma_prefetch_desc(&R->tc); }
+  RsPolicy pol(a, R, s_arrived);
+  gemm_pair_persistent<TP_BN, RS_STAGES, false, false>(smem_raw, &R->tb, pol, a.K, cta >> 1, a.ctas_per_rank >> 1, R->status, &s_abort);
 }
 
 // ------------------------------------------------------------------ all-gather -> GEMM
+constexpr int FEED_PIECE = 4096, FEED_STAGES = 8, FEED_AHEAD = 5;
 struct AgPolicy {
-  const TpRank* R; int n, rank, M, N, mb_per_shard, num_n, parity; unsigned epoch; long long flag_off;
-  __device__ int num_tiles() const { return n * mb_per_shard * num_n; }
-  __device__ void tile(int idx, int& m_blk, int& n_blk) const {
-    const int per = mb_per_shard * num_n, src = (rank + idx / per) % n, within = idx % per;   // own shard first, then rank+1, ...
-    m_blk = src * mb_per_shard + within / num_n; n_blk = within % num_n;
+  const TpArgs& a; const TpRank* R; int cta, rank, mb_per_shard, num_n, parity;
+  static constexpr int EXTRA_BYTES = FEED_STAGES * FEED_PIECE + FEED_STAGES * 8;
+  __device__ AgPolicy(const TpArgs& args, const TpRank* r, int c)
+      : a(args), R(r), cta(c), rank(r->rank), mb_per_shard(args.M / args.n / TP_BM), num_n(args.N / TP_BN), parity((int)(args.epoch & 1)) {}
+  __device__ void begin() const {}
+  __device__ int num_tiles() const { return (a.M / TP_BM + 1) / 2 * num_n; }
+  // row blocks of the own shard first, then rank+1, ..., two to a pair
+  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) const {
+    const int i = 2 * (idx / num_n) + v;
+    n_blk = idx % num_n;
+    m_blk = i < a.n * mb_per_shard ? (rank + i / mb_per_shard) % a.n * mb_per_shard + i % mb_per_shard : -1;
   }
+  __device__ void k_range(int, int num_kb, int& kb0, int& kb1) const { kb0 = 0; kb1 = num_kb; }
   __device__ const CUtensorMap* a_map(int m_blk, int& row0) const {
-    if (m_blk / mb_per_shard == rank) { row0 = (m_blk % mb_per_shard) * GEMM_BM; return &R->ta; }
-    row0 = m_blk * GEMM_BM; return &R->ta2;             // ta2 covers this call's half of the region
+    if (m_blk < 0) { row0 = 0; return &R->ta; }
+    if (m_blk / mb_per_shard == rank) { row0 = (m_blk % mb_per_shard) * TP_BM; return &R->ta; }
+    row0 = m_blk * TP_BM; return &R->ta2;               // ta2 covers this call's half of the region
+  }
+  __device__ unsigned* flags(int dest, int src, int mb) const {
+    return reinterpret_cast<unsigned*>(R->heap[dest] + a.flag_off) + ((size_t)(parity * a.n + src) * mb_per_shard + mb) * a.n_part;
   }
   __device__ bool gate(int m_blk, volatile int* abort_flag) const {
-    const int src = m_blk / mb_per_shard;
-    if (src == rank) return true;
-    const unsigned* f = reinterpret_cast<const unsigned*>(R->heap[rank] + flag_off) + ((size_t)(parity * n + src) * mb_per_shard + m_blk % mb_per_shard);
-    if (!wait_flag(f, epoch, abort_flag)) return false;
-    asm volatile("fence.proxy.async;" ::: "memory");   // the rows were written with ordinary stores; TMA reads them through the async proxy
+    if (m_blk < 0 || m_blk / mb_per_shard == rank) return true;
+    const int lane = threadIdx.x & 31;
+    const unsigned* f = flags(rank, m_blk / mb_per_shard, m_blk % mb_per_shard);
+    const bool ok = lane >= a.n_part || wait_flag(f + lane, a.epoch, abort_flag);
+    const bool all = __all_sync(0xffffffffu, ok);
+    asm volatile("fence.proxy.async;" ::: "memory");    // the rows arrived before the flags; TMA reads them through the async proxy
+    return all;
+  }
+  __device__ void prefetch(const EpiCtx&, int, int) {}
+  __device__ bool epilogue(const EpiCtx& e, int, int m_blk, int n_blk, volatile int*) {
+    if (m_blk < 0) return true;
+#pragma unroll 1
+    for (int pc = e.half * 2; pc < e.half * 2 + 2; pc++) {
+      float v[64];
+      epi_load64(e, pc * 64, v);
+      epi_staging_free(e);
+      epi_stage_row(e, v);
+      epi_ship(e, &R->tc, n_blk * TP_BN + pc * 64, m_blk * TP_BM + e.quarter * 32);
+    }
     return true;
   }
-  static constexpr int STAGING = 0;
-  __device__ void set_staging(uint8_t*) {}
-  __device__ bool tile_begin(int, int, int, volatile int*) { return true; }
-  __device__ void tile_end(int, int, int) {}
-  __device__ void store(int m_blk, int n_blk, int row, int col0, float (&v)[32]) {
-    store_row32_bf16(R->out + (size_t)(m_blk * GEMM_BM + row) * N + (size_t)n_blk * TP_BN + col0, v);
+  // The feeding warp: parts of the shard's row blocks to the peers, distance-major (the peer that needs my shard next comes first), spread over
+  // all CTAs.  One lane streams a part through the ring, FEED_AHEAD loads in flight, and raises the part's flag when its stores have been performed.
+  __device__ void extra_warp(uint8_t* smem, int lane, volatile int* abort_flag) {
+    if (lane != 0) return;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + FEED_STAGES * FEED_PIECE);
+    for (int i = 0; i < FEED_STAGES; i++) mbar_init(&bar[i], 1);
+    fence_barrier_init();
+    uint32_t phase = 0;                                  // bit s: the parity the next wait on stage s looks for
+    const size_t block_bytes = (size_t)TP_BM * a.K * 2, part_bytes = block_bytes / a.n_part;
+    const int per_dest = mb_per_shard * a.n_part, units = (a.n - 1) * per_dest, np = (int)((part_bytes + FEED_PIECE - 1) / FEED_PIECE);
+    bool ok = true;
+    for (int u = cta; u < units && ok; u += a.ctas_per_rank) {
+      const int dest = (rank - 1 - u / per_dest + a.n) % a.n, mb = u % per_dest / a.n_part, part = u % a.n_part;
+      const size_t off = (size_t)mb * block_bytes + (size_t)part * part_bytes;
+      const char* src = reinterpret_cast<const char*>(R->a_shard) + off;
+      char* dst = R->heap[dest] + a.data_off + (size_t)rank * (a.M / a.n) * a.K * 2 + off;
+      int issued = 0;
+      for (int i = 0; i < np + FEED_AHEAD; i++) {
+        if (i < np && ok) {
+          issued = i + 1;
+          const uint32_t bytes = (uint32_t)min((size_t)FEED_PIECE, part_bytes - (size_t)i * FEED_PIECE);
+          const int st = i % FEED_STAGES;
+          // the stage last held piece i - FEED_STAGES: all but the newest stores have been read out of shared memory
+          if (i >= FEED_STAGES) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(FEED_STAGES - 1 - FEED_AHEAD) : "memory");
+          mbar_arrive_expect_tx(&bar[st], bytes);
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem + st * FEED_PIECE)),
+                       "l"(src + (size_t)i * FEED_PIECE), "r"(bytes), "r"(smem_u32(&bar[st])) : "memory");
+        }
+        const int j = i - FEED_AHEAD;
+        if (j >= 0 && j < issued) {                      // every issued load is waited for, also after a failure
+          const int st = j % FEED_STAGES;
+          const bool landed = mbar_wait(&bar[st], (phase >> st) & 1u, abort_flag, kPairWaitLimitNs);
+          phase ^= 1u << st;
+          if (!landed) { ok = false; continue; }
+          const uint32_t bytes = (uint32_t)min((size_t)FEED_PIECE, part_bytes - (size_t)j * FEED_PIECE);
+          bulk_store(dst + (size_t)j * FEED_PIECE, smem + st * FEED_PIECE, bytes); bulk_commit();
+        }
+      }
+      bulk_wait_all();                                   // the writes are performed; then tell the reader
+      asm volatile("fence.proxy.async;" ::: "memory");
+      if (ok) st_release_sys_u32(flags(dest, rank, mb) + part, a.epoch);
+    }
+    if (!ok) { *abort_flag = 1; atomicExch(R->status, 7); }
   }
 };
 
-// Feeder CTAs: copy row blocks of the local shard into the peers' gathered buffers.
-__device__ void ag_feed(const TpArgs& a, const TpRank* R, int feeder, int n_feed) {
-  const int n = a.n, rank = R->rank, mbs = a.M / n / GEMM_BM, parity = a.epoch & 1;
-  const size_t block_bytes = (size_t)GEMM_BM * a.K * 2;
-  const int pairs = (n - 1) * mbs;
-  for (int p = feeder; p < pairs; p += n_feed) {
-    const int d = 1 + p / mbs, mb = p % mbs;             // distance-major: the peer that needs my shard next comes first
-    const int dest = (rank - d + n) % n;
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(R->a_shard) + (size_t)mb * block_bytes);
-    uint4* dst = reinterpret_cast<uint4*>(R->heap[dest] + a.data_off + ((size_t)rank * (a.M / n) + (size_t)mb * GEMM_BM) * a.K * 2);
-    const size_t nvec = block_bytes / 16;
-    size_t i = threadIdx.x;
-    for (; i + 7 * GEMM_THREADS < nvec; i += 8 * GEMM_THREADS) {
-      uint4 v[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) v[u] = src[i + u * GEMM_THREADS];
-#pragma unroll
-      for (int u = 0; u < 8; u++) dst[i + u * GEMM_THREADS] = v[u];
-    }
-    for (; i < nvec; i += GEMM_THREADS) dst[i] = src[i];
-    __syncthreads();
-    if (threadIdx.x == 0)
-      st_release_sys_u32(reinterpret_cast<unsigned*>(R->heap[dest] + a.flag_off) + ((size_t)(parity * n + rank) * mbs + mb), a.epoch);
-  }
-}
-
-__global__ void __launch_bounds__(GEMM_THREADS, 1) ag_gemm_kernel(const __grid_constant__ TpArgs a) {
+constexpr int AG_THREADS = PAIR_THREADS + 32;
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(AG_THREADS, 1) ag_gemm_kernel(const __grid_constant__ TpArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int s_abort;
   const int vr = blockIdx.x / a.ctas_per_rank, cta = blockIdx.x % a.ctas_per_rank;
   const TpRank* R = &a.r[vr];
-  if (cta < a.n_feed) { ag_feed(a, R, cta, a.n_feed); return; }     // feeders come first in the grid so they start first
-  if (threadIdx.x == 0) { s_abort = 0; tma_prefetch_desc(&R->ta); tma_prefetch_desc(&R->ta2); }
-  AgPolicy pol{R, a.n, R->rank, a.M, a.N, a.M / a.n / GEMM_BM, a.N / TP_BN, (int)(a.epoch & 1), a.epoch, a.flag_off};
-  gemm_persistent<TP_BN, TP_STAGES>(smem_raw, &R->tb, pol, a.K, cta - a.n_feed, a.ctas_per_rank - a.n_feed, R->status, &s_abort);
+  if (threadIdx.x == 0) { s_abort = 0; tma_prefetch_desc(&R->ta); tma_prefetch_desc(&R->ta2); tma_prefetch_desc(&R->tc); }
+  AgPolicy pol(a, R, cta);
+  gemm_pair_persistent<TP_BN, AG_STAGES, false, false>(smem_raw, &R->tb, pol, a.K, cta >> 1, a.ctas_per_rank >> 1, R->status, &s_abort);
 }
 
 // ------------------------------------------------------------------ host
 // The workspace is used in four quarters: [kernel: gemm_rs, ag_gemm][parity of that kernel's call count].
 static long long tp_quarter(long long tp_bytes) { return tp_bytes / 4 / 1024 * 1024; }
 static long long tp_need_per_call(int which, int nranks, int M, int N, int K) {
-  if (which == 0) return (long long)nranks * ((long long)M / nranks / GEMM_BM) * (N / TP_BN) * (GEMM_BM * TP_BN * 2);     // [src][tile] bf16 tiles
+  if (which == 0) return (long long)nranks * ((long long)M / nranks / TP_BM) * (N / TP_BN) * (TP_BM * TP_BN * 2);     // [src][tile] bf16 tiles
   return (long long)M * K * 2;                                                                                              // [M][K] bf16
+}
+
+// Flags per row block: 16 parts of 8 K bytes spread a block over as many CTAs (a power of two; fewer where the flag area would not hold them).
+static int ag_parts(int M) {
+  int p = 16;
+  while (p > 1 && 2LL * (M / TP_BM) * p * 4 > (512 << 10)) p /= 2;
+  return p;
 }
 
 static int tp_common_checks(piccl_comm** cs, int n, int M, int N, int K, int which) {
@@ -247,8 +317,8 @@ static int tp_common_checks(piccl_comm** cs, int n, int M, int N, int K, int whi
   piccl_comm* c = cs[0];
   if (c->nranks > TP_MAX_RANKS) return fail(PICCL_UNSUPPORTED, "fused tensor-parallel kernels support up to %d ranks", TP_MAX_RANKS);
   for (int i = 0; i < n; i++) if (!cs[i]->connected || cs[i]->broken) return fail(PICCL_INVALID_USAGE, "communicator not usable");
-  if (M <= 0 || M % (GEMM_BM * c->nranks) || N % TP_BN || K % GEMM_BK || N <= 0 || K <= 0) return fail(PICCL_INVALID_ARGUMENT, "shape: M %% (128*ranks), N %% 256, K %% 64 must be 0");
-  const long long nflags = which == 0 ? 2LL * c->nranks * (M / c->nranks / GEMM_BM) * (N / TP_BN) : 2LL * c->nranks * (M / c->nranks / GEMM_BM);
+  if (M <= 0 || M % (TP_BM * c->nranks) || N % TP_BN || K % TP_BK || N <= 0 || K <= 0) return fail(PICCL_INVALID_ARGUMENT, "shape: M %% (128*ranks), N %% 256, K %% 64 must be 0");
+  const long long nflags = which == 0 ? 2LL * c->nranks * (M / c->nranks / TP_BM) * (N / TP_BN) : 2LL * c->nranks * (M / c->nranks / TP_BM) * ag_parts(M);
   if (nflags * 4 > (512 << 10)) return fail(PICCL_UNSUPPORTED, "too many tiles for the flag area");
   long long need = piccl_tp_workspace_bytes(which, c->nranks, M, N, K);
   if (tp_quarter(c->h_ctx.tp_bytes) < tp_need_per_call(which, c->nranks, M, N, K)) return fail(PICCL_INVALID_USAGE, "tensor-parallel workspace too small: %lld bytes needed, %lld configured (tp_bytes / PICCL_TP_MB)", need, c->h_ctx.tp_bytes);
@@ -259,7 +329,11 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
   int rc = tp_common_checks(cs, n, M, N, K, which); if (rc) return rc;
   piccl_comm* c0 = cs[0];
   const int nr = c0->nranks;
-  int prev = -1; cudaGetDevice(&prev); if (prev != c0->device) cudaSetDevice(c0->device);
+  struct Guard {
+    int prev = -1, dev;
+    explicit Guard(int d) : dev(d) { cudaGetDevice(&prev); if (prev != dev) cudaSetDevice(dev); }
+    ~Guard() { if (prev >= 0 && prev != dev) cudaSetDevice(prev); }
+  } guard(c0->device);
   TpArgs a; memset(&a, 0, sizeof a);
   a.n = nr; a.M = M; a.N = N; a.K = K;
   a.flag_off = c0->h_ctx.tp_flag_off + (which ? (512 << 10) : 0);   // the two kernels keep their flags apart
@@ -269,9 +343,24 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
   const long long quarter = tp_quarter(c0->h_ctx.tp_bytes);
   const unsigned next_epoch = (which ? c0->tp_epoch_ag : c0->tp_epoch_rs) + 1;
   a.data_off = c0->h_ctx.tp_data_off + (which ? 2 * quarter : 0) + (long long)(next_epoch & 1) * quarter;
-  a.ctas_per_rank = std::max(1, c0->sm_count / n);
-  a.n_feed = which ? std::min(std::max(1, env().tp_feeders), a.ctas_per_rank / 2) : 0;
-  if (nr == 1) a.n_feed = 0;
+  a.n_part = ag_parts(M);
+  const int smem_bytes = which ? PairSmem<TP_BN, AG_STAGES, AgPolicy::EXTRA_BYTES>::DYNAMIC : PairSmem<TP_BN, RS_STAGES>::DYNAMIC;
+  const int threads = which ? AG_THREADS : PAIR_THREADS;
+  auto fn = which ? ag_gemm_kernel : gemm_rs_kernel;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem_bytes; cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  if (!c0->tp_pairs[which]) {
+    // pairs that can be resident at once (a pair needs two SMs of one GPC): the persistent grid is never larger, the ranks wait for one another
+    if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return fail(PICCL_CUDA_ERROR, "cannot get %d bytes of shared memory", smem_bytes);
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(c0->sm_count / 2 * 2); cfg.attrs = at; cfg.numAttrs = 1;
+    int active = 0;
+    if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) { cudaGetLastError(); return fail(PICCL_CUDA_ERROR, "no room for a pair of CTAs with %d bytes of shared memory each", smem_bytes); }
+    c0->tp_pairs[which] = std::min(active, c0->sm_count / 2);
+  }
+  a.ctas_per_rank = 2 * (c0->tp_pairs[which] / n);
+  if (a.ctas_per_rank < 2) return fail(PICCL_UNSUPPORTED, "%d ranks do not fit on %d pairs of SMs", n, c0->tp_pairs[which]);
   bool ok = true;
   for (int i = 0; i < n && ok; i++) {
     piccl_comm* c = cs[i];
@@ -281,27 +370,22 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
     if (!c->d_tp_status) { if (cudaMalloc(&c->d_tp_status, sizeof(int)) != cudaSuccess) { ok = false; break; } cudaMemset(c->d_tp_status, 0, sizeof(int)); }
     R.status = c->d_tp_status;
     if (which == 0) {
-      ok &= make_tmap_bf16_k64(&R.ta, A[i], (uint64_t)M, (uint64_t)K, (uint64_t)K, GEMM_BM);
+      ok &= make_tmap_bf16_k64(&R.ta, A[i], (uint64_t)M, (uint64_t)K, (uint64_t)K, TP_BM);
       R.ta2 = R.ta;
       a.epoch = ++c->tp_epoch_rs;
     } else {
-      ok &= make_tmap_bf16_k64(&R.ta, A[i], (uint64_t)(M / nr), (uint64_t)K, (uint64_t)K, GEMM_BM);
-      ok &= make_tmap_bf16_k64(&R.ta2, c->heap + a.data_off, (uint64_t)M, (uint64_t)K, (uint64_t)K, GEMM_BM);
+      ok &= make_tmap_bf16_k64(&R.ta, A[i], (uint64_t)(M / nr), (uint64_t)K, (uint64_t)K, TP_BM);
+      ok &= make_tmap_bf16_k64(&R.ta2, c->heap + a.data_off, (uint64_t)M, (uint64_t)K, (uint64_t)K, TP_BM);
       a.epoch = ++c->tp_epoch_ag;
     }
-    ok &= make_tmap_bf16_k64(&R.tb, B[i], (uint64_t)N, (uint64_t)K, (uint64_t)K, TP_BN);
+    ok &= make_tmap_bf16_k64(&R.tb, B[i], (uint64_t)N, (uint64_t)K, (uint64_t)K, TP_BN / 2);
+    ok &= make_tmap_bf16_k64(&R.tc, out[i], (uint64_t)(which ? M : M / nr), (uint64_t)N, (uint64_t)N, 32);
   }
-  if (!ok) { if (prev != c0->device && prev >= 0) cudaSetDevice(prev); return fail(PICCL_CUDA_ERROR, "tensor map or status set-up failed"); }
-  const int smem_bytes = which ? GemmSmem<TP_BN, TP_STAGES>::DYNAMIC : GemmSmem<TP_BN, RS_STAGES, RS_STAGING>::DYNAMIC;
-  const void* fn = which ? (const void*)ag_gemm_kernel : (const void*)gemm_rs_kernel;
-  static bool attr[2] = {false, false};
-  if (!attr[which]) { if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return fail(PICCL_CUDA_ERROR, "cannot get %d bytes of shared memory", smem_bytes); attr[which] = true; }
-  void* args[] = {&a};
-  cudaError_t e;
+  if (!ok) return fail(PICCL_CUDA_ERROR, "tensor map or status set-up failed");
   // ranks wait for one another inside the kernel: several virtual ranks on one device must be co-resident
-  if (n > 1) e = cudaLaunchCooperativeKernel(fn, dim3(n * a.ctas_per_rank), dim3(GEMM_THREADS), args, smem_bytes, stream);
-  else e = cudaLaunchKernel(fn, dim3(a.ctas_per_rank), dim3(GEMM_THREADS), args, smem_bytes, stream);
-  if (prev != c0->device && prev >= 0) cudaSetDevice(prev);
+  at[0].id = cudaLaunchAttributeCooperative; at[0].val.cooperative = 1;
+  cfg.gridDim = dim3(n * a.ctas_per_rank); cfg.attrs = at; cfg.numAttrs = n > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, a);
   if (e != cudaSuccess) return fail(PICCL_CUDA_ERROR, "fused kernel launch failed: %s", cudaGetErrorString(e));
   for (int i = 0; i < n; i++) cs[i]->stats.launches++;
   return PICCL_OK;
