@@ -20,13 +20,17 @@
 //
 //   struct Policy {
 //     void begin() const;                                           // every thread, after the set-up (barriers, TMEM) and before global memory is touched
+//     void report(int role) const;                                  // status word: a wait of that role ran out
 //     int  num_tiles() const;
-//     void tile(int idx, int v, int& m_blk, int& n_blk) const;     // 128-row block of CTA v (< 0: none), block of TN columns
+//     void tile(int idx, int v, int& m_blk, int& n_blk);           // 128-row block of CTA v (< 0: none), block of TN columns; the calls below are about it
 //     void k_range(int idx, int num_kb, int& kb0, int& kb1) const; // k-blocks that this entry of the tile order sums, not empty
 //     const CUtensorMap* a_map(int m_blk, int& row0) const;        // tensor map and first row of A for it
+//     const CUtensorMap* b_map() const;                            // tensor map of B
 //     bool gate(int m_blk, volatile int* abort) const;             // producer: wait until the row block may be loaded
 //     void prefetch(const EpiCtx&, int m_blk, int n_blk);          // epilogue warps, before they wait for the accumulator
 //     bool epilogue(const EpiCtx&, int idx, int m_blk, int n_blk, volatile int* abort);  // called by all eight warps; false: gave up
+//     void finish(const EpiCtx&);                                   // epilogue warps, after their last tile
+//     static constexpr int NSTAGE;                                  // staging buffers per epilogue warp
 //     static constexpr int EXTRA_BYTES; void extra_warp(uint8_t* smem, int lane, volatile int* abort);           // all lanes of warp 10
 //   };
 // Every wait is bounded; a wait that runs out sets the status word (1 producer, 2 / 3 MMA issuer, 4 epilogue, 5 gate, 6 policy), every
@@ -38,15 +42,16 @@
 namespace sm100 {
 
 constexpr int PAIR_BM = 128, PAIR_BK = 64, PAIR_THREADS = 320, PAIR_EPI_WARPS = 8;
-constexpr int PAIR_STAGING = 4096;                                  // bytes of staging per epilogue warp: 32 rows of 64 bf16
+constexpr int PAIR_STAGING = 4096;                                  // bytes of a staging buffer of an epilogue warp: 32 rows of 64 bf16
 constexpr unsigned long long kPairWaitLimitNs = 4000000000ull;      // 4 s
 constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;      // clears the bit that tells the two CTAs of a pair apart in a shared::cluster address
 
-template <int TN, int STAGES, int EXTRA_BYTES = 0>
+// NSTAGE: staging buffers per epilogue warp
+template <int TN, int STAGES, int EXTRA_BYTES = 0, int NSTAGE = 1>
 struct PairSmem {
   static constexpr int A_BYTES = PAIR_BM * PAIR_BK * 2, B_BYTES = (TN / 2) * PAIR_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;
-  static constexpr int BAR_OFF = STAGING_OFF + PAIR_EPI_WARPS * PAIR_STAGING;
+  static constexpr int BAR_OFF = STAGING_OFF + PAIR_EPI_WARPS * PAIR_STAGING * NSTAGE;
   static constexpr int EXTRA_OFF = (BAR_OFF + (2 * STAGES + 4) * 8 + 16 + 127) / 128 * 128;
   static constexpr int TOTAL = EXTRA_OFF + EXTRA_BYTES;
   static constexpr int DYNAMIC = TOTAL + 1024;                      // slack for the 1024-byte alignment of the tiles
@@ -108,7 +113,7 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16_major(uint32_t M, uint32_
 // What an epilogue warp knows about itself and its accumulator.
 struct EpiCtx {
   uint32_t tmem;         // this warp's lanes, first column of the accumulator
-  uint8_t* staging;      // this warp's PAIR_STAGING bytes
+  uint8_t* staging;      // this warp's staging buffers
   int quarter, half, lane;
 };
 // 64 columns of this thread's row, starting at column col0 of the tile
@@ -143,9 +148,8 @@ __device__ __forceinline__ void epi_staging_free(const EpiCtx& e) {
 }
 
 template <int TN, int STAGES, bool A_MN, bool B_MN, class Policy>
-__device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CUtensorMap* tmap_b, Policy& pol, int K, int first_tile, int tile_stride,
-                                                     int* status, volatile int* s_abort) {
-  typedef PairSmem<TN, STAGES, Policy::EXTRA_BYTES> L;
+__device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, Policy& pol, int K, int first_tile, int tile_stride, volatile int* s_abort) {
+  typedef PairSmem<TN, STAGES, Policy::EXTRA_BYTES, Policy::NSTAGE> L;
   static_assert(!B_MN || TN >= 128, "an MN-major half of B is at least one box of 64 columns");
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
@@ -165,7 +169,6 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
     for (int s = 0; s < STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 2 * PAIR_EPI_WARPS); }
     fence_barrier_init();
-    tma_prefetch_desc(tmap_b);
   }
   if (warp == 1) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
   tc_fence_before();
@@ -180,13 +183,14 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
     int stage = 0; uint32_t phase = 0;
     for (int t = first_tile; t < num_tiles && !*s_abort; t += tile_stride) {
       int m_blk, n_blk; pol.tile(t, v, m_blk, n_blk);
-      if (!pol.gate(m_blk, s_abort)) { *s_abort = 1; if (issuer) atomicExch(status, 5); break; }
+      if (!pol.gate(m_blk, s_abort)) { *s_abort = 1; if (issuer) pol.report(5); break; }
       int row0; const CUtensorMap* ta = pol.a_map(m_blk, row0);
+      const CUtensorMap* tb = pol.b_map();
       const int col0 = n_blk * TN + v * (TN / 2);
       int kb0, kb1; pol.k_range(t, num_kb, kb0, kb1);
       bool ok = true;
       for (int kb = kb0; kb < kb1; kb++) {
-        if (!mbar_wait(&empty[stage], phase ^ 1, s_abort, kPairWaitLimitNs)) { if (issuer) atomicExch(status, 1); ok = false; break; }
+        if (!mbar_wait(&empty[stage], phase ^ 1, s_abort, kPairWaitLimitNs)) { if (issuer) pol.report(1); ok = false; break; }
         uint8_t* sa = smem + stage * L::STAGE_BYTES; uint8_t* sb = sa + L::A_BYTES;
         if (issuer) {
           if (v == 0) mbar_arrive_expect_tx(&full[stage], 2 * L::STAGE_BYTES);      // the bytes of both CTAs land on the leader's barrier
@@ -196,8 +200,8 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
           } else tma_load_2d_pair(sa, ta, kb * PAIR_BK, row0, &full[stage]);
           if (B_MN) {
 #pragma unroll
-            for (int i = 0; i < TN / 128; i++) tma_load_2d_pair(sb + i * 8192, tmap_b, col0 + i * 64, kb * PAIR_BK, &full[stage]);
-          } else tma_load_2d_pair(sb, tmap_b, kb * PAIR_BK, col0, &full[stage]);
+            for (int i = 0; i < TN / 128; i++) tma_load_2d_pair(sb + i * 8192, tb, col0 + i * 64, kb * PAIR_BK, &full[stage]);
+          } else tma_load_2d_pair(sb, tb, kb * PAIR_BK, col0, &full[stage]);
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -213,13 +217,13 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
       int stage = 0; uint32_t phase = 0; int local = 0;
       for (int t = first_tile; t < num_tiles && !*s_abort; t += tile_stride, local++) {
         const int acc = local & 1; const uint32_t acc_phase = (local >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, s_abort, kPairWaitLimitNs)) { if (issuer) atomicExch(status, 2); break; }
+        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, s_abort, kPairWaitLimitNs)) { if (issuer) pol.report(2); break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN;
         int kb0, kb1; pol.k_range(t, num_kb, kb0, kb1);
         bool ok = true;
         for (int kb = kb0; kb < kb1; kb++) {
-          if (!mbar_wait(&full[stage], phase, s_abort, kPairWaitLimitNs)) { if (issuer) atomicExch(status, 3); ok = false; break; }
+          if (!mbar_wait(&full[stage], phase, s_abort, kPairWaitLimitNs)) { if (issuer) pol.report(3); ok = false; break; }
           tc_fence_after();
           const uint64_t da = desc_advance(da0, stage * L::STAGE_BYTES), db = desc_advance(db0, stage * L::STAGE_BYTES);
           if (issuer) {
@@ -242,20 +246,21 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, const CU
   } else {
     EpiCtx e;
     e.quarter = warp & 3; e.half = (warp - 2) >> 2; e.lane = lane;
-    e.staging = smem + L::STAGING_OFF + (warp - 2) * PAIR_STAGING;
+    e.staging = smem + L::STAGING_OFF + (warp - 2) * PAIR_STAGING * Policy::NSTAGE;
     int local = 0;
     for (int t = first_tile; t < num_tiles; t += tile_stride, local++) {
       int m_blk, n_blk; pol.tile(t, v, m_blk, n_blk);
       const int acc = local & 1; const uint32_t acc_phase = (local >> 1) & 1;
       e.tmem = tmem_base + ((uint32_t)(e.quarter * 32) << 16) + acc * TN;
       pol.prefetch(e, m_blk, n_blk);
-      if (!mbar_wait(&tmem_full[acc], acc_phase, s_abort, kPairWaitLimitNs)) { atomicExch(status, 4); break; }
+      if (!mbar_wait(&tmem_full[acc], acc_phase, s_abort, kPairWaitLimitNs)) { pol.report(4); break; }
       tc_fence_after();
-      if (!pol.epilogue(e, t, m_blk, n_blk, s_abort)) { *s_abort = 1; atomicExch(status, 6); break; }
+      if (!pol.epilogue(e, t, m_blk, n_blk, s_abort)) { *s_abort = 1; pol.report(6); break; }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(&tmem_empty[acc]);      // this warp's part of the accumulator may be overwritten
     }
+    pol.finish(e);
   }
   // Neither CTA leaves while the other may still touch its shared memory or barriers, TMEM is freed after the last read of it.  The
   // arrival goes out before the wait for the stores' reads of the staging buffers, so the two latencies overlap.

@@ -39,6 +39,7 @@ struct PlainPolicy {
   int num_m, num_n;                                    // tiles of 256 rows, of TN columns
   __device__ PlainPolicy(const GemmArgs& g) : a(g), num_m((g.M + 2 * PAIR_BM - 1) / (2 * PAIR_BM)), num_n((g.N + TN - 1) / TN) {}
   __device__ void begin() const { pdl_begin(); }
+  __device__ void report(int role) const { atomicExch(a.status, role); }
   __device__ int num_tiles() const { return num_m * num_n * a.slices; }
   // Bands of 16 row tiles, inside a band column tiles outer / row tiles inner: the pairs that run together share a band of A
   // (about 30 MB at K = 3584) that stays in L2 while B streams through once per band.
@@ -55,9 +56,11 @@ struct PlainPolicy {
     kb0 = (int)((long long)num_kb * sl / a.slices); kb1 = (int)((long long)num_kb * (sl + 1) / a.slices);
   }
   __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = m_blk * PAIR_BM; return &a.ta; }
+  __device__ const CUtensorMap* b_map() const { return &a.tb; }
   __device__ bool gate(int, volatile int*) const { return true; }
 
-  static constexpr int EXTRA_BYTES = 0;
+  static constexpr int EXTRA_BYTES = 0, NSTAGE = 1;
+  __device__ void finish(const EpiCtx&) {}
   static constexpr bool AUX = EPI == EPI_RESIDUAL || EPI == EPI_GELU_GRAD;
   static constexpr int PIECES = TN / 64;               // 64-column pieces of the tile; the halves of the warps share them
   static constexpr int PER = PIECES >= 2 ? PIECES / 2 : 1;
@@ -186,9 +189,9 @@ template <int TN, int STAGES, bool A_MN, bool B_MN, int EPI, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) gemm_pair_kernel(const __grid_constant__ GemmArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int s_abort;
-  if (threadIdx.x == 0) { s_abort = 0; tma_prefetch_desc(&a.ta); tma_prefetch_desc(&a.tc); }
+  if (threadIdx.x == 0) { s_abort = 0; tma_prefetch_desc(&a.ta); tma_prefetch_desc(&a.tb); tma_prefetch_desc(&a.tc); }
   PlainPolicy<TN, EPI, SPLIT> pol(a);
-  gemm_pair_persistent<TN, STAGES, A_MN, B_MN>(smem_raw, &a.tb, pol, a.K, blockIdx.x >> 1, gridDim.x >> 1, a.status, &s_abort);
+  gemm_pair_persistent<TN, STAGES, A_MN, B_MN>(smem_raw, pol, a.K, blockIdx.x >> 1, gridDim.x >> 1, &s_abort);
 }
 
 // ------------------------------------------------------------------ host

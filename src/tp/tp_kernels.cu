@@ -30,7 +30,7 @@ namespace piccl {
 
 using namespace sm100;
 typedef __nv_bfloat16 bf16;
-constexpr int TP_BN = 256, RS_STAGES = 6, AG_STAGES = 5, TP_MAX_RANKS = 8;
+constexpr int TP_BN = 256, RS_STAGES = 5, AG_STAGES = 5, TP_MAX_RANKS = 8;
 constexpr int TP_BM = PAIR_BM, TP_BK = PAIR_BK;
 
 __device__ __forceinline__ unsigned ld_acquire_sys_u32(const unsigned* p) {
@@ -65,118 +65,167 @@ struct TpRank {
 };
 struct TpArgs {
   int n, M, N, K;            // gemm_rs: K = K_local, N full;  ag_gemm: N = N_local, K full
-  int ctas_per_rank, n_part; // ag_gemm: parts of a row block, each with a flag of its own
+  int nv;                    // (virtual) ranks of this launch: every pair works for all of them, see the policies
+  int n_part;                // ag_gemm: parts of a row block, each with a flag of its own
   unsigned epoch;
   long long flag_off, data_off;
   TpRank r[TP_MAX_RANKS];    // one entry per virtual rank of the launch
 };
 
 // ------------------------------------------------------------------ GEMM -> reduce-scatter
+// Several virtual ranks on one device: every pair of CTAs works for each of them in turn, so that at any time one rank's operands are in
+// L2.  (With a ninth of the pairs for each of eight ranks, eight working sets of 12 MB per wave thrashed it: 3.4 GB read from memory for
+// 0.6 GB of operands, and the power that took held the clocks down: 4.2 ms for 8192 x 8192 x 3584 in a steady loop.)
 struct RsPolicy {
-  const TpRank* R; int n, rank, mb_per_owner, num_n, parity; unsigned epoch;
-  long long flag_off, data_off; unsigned* s_arrived;
-  int row_pairs, tiles_per_owner, group;
-  int seq = 0;
-  static constexpr int EXTRA_BYTES = 0;
-  __device__ RsPolicy(const TpArgs& a, const TpRank* r, unsigned* arrived)
-      : R(r), n(a.n), rank(r->rank), mb_per_owner(a.M / a.n / TP_BM), num_n(a.N / TP_BN), parity((int)(a.epoch & 1)), epoch(a.epoch), flag_off(a.flag_off), data_off(a.data_off),
-        s_arrived(arrived), row_pairs((a.M / TP_BM + 1) / 2), tiles_per_owner(mb_per_owner * num_n), group(min(16, (mb_per_owner + 1) / 2)) {}
+  const TpArgs& a; const TpRank* R = nullptr; unsigned* s_arrived;
+  int n, rank = 0, mb_per_owner, num_n, parity, tiles_per_owner, rp_remote, rp_own;
+  unsigned* pending = nullptr;       // flag of the remote tile whose stores this warp has issued but not waited for, and the tile's slot in s_arrived
+  int pending_slot = 0, seq = 0;
+  static constexpr int EXTRA_BYTES = 0, NSTAGE = 2;
+  __device__ RsPolicy(const TpArgs& args, unsigned* arrived)
+      : a(args), s_arrived(arrived), n(args.n), mb_per_owner(args.M / args.n / TP_BM), num_n(args.N / TP_BN), parity((int)(args.epoch & 1)), tiles_per_owner(mb_per_owner * num_n),
+        rp_remote(((args.n - 1) * mb_per_owner + 1) / 2), rp_own((mb_per_owner + 1) / 2) {}
   __device__ void begin() const {}
-  __device__ int num_tiles() const { return row_pairs * num_n; }
-  // Row blocks in the order rank+1, rank+2, ..., myself last, two to a pair.  Panels of 16 column blocks (one panel of B stays in
-  // L2); inside a panel groups of row pairs (about one owner), inside a group rows fastest.  All ranks walk the panels in the same order, so the
-  // partials of my own tiles of a panel are on their way while I still compute the other owners' tiles of that panel.
-  // No cycle of waits: within a panel an own tile comes after every remote tile of its column, and what the remote tile that it
-  // waits for comes after are own tiles of earlier panels, or of earlier columns in the one group that holds both kinds.
-  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) const {
-    constexpr int PN = 16;
-    const int per_panel = PN * row_pairs, panel = idx / per_panel;
-    int within = idx % per_panel;
-    const int cols = min(PN, num_n - panel * PN);             // last panel may be narrower
-    const int g = within / (group * cols); within %= group * cols;
-    const int rows = min(group, row_pairs - g * group);
-    const int i = 2 * (g * group + within % rows) + v;        // position in the order of row blocks
-    n_blk = panel * PN + within / rows;
-    m_blk = i < n * mb_per_owner ? (rank + 1 + i / mb_per_owner) % n * mb_per_owner + i % mb_per_owner : -1;
+  __device__ void report(int role) const { for (int i = 0; i < a.nv; i++) atomicExch(a.r[i].status, role); }
+  __device__ int num_tiles() const { return a.nv * (rp_remote + rp_own) * num_n; }
+  // Panels of 16 column blocks (one panel of B stays in L2); inside a panel first the row blocks of other owners, in the order rank+1,
+  // rank+2, ..., for every rank of the launch, then the own ones; two blocks to a pair, bands of 16 pairs, inside a band rows fastest.
+  // All ranks walk the panels in the same order, so the partials of my own tiles of a panel are on their way while I still compute
+  // the other owners' tiles of that panel; and as a panel's own tiles come after all its remote ones, waits never form a cycle.
+  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) {
+    constexpr int PN = 16, BAND = 16;
+    const int per_panel = PN * a.nv * (rp_remote + rp_own), panel = idx / per_panel, cols = min(PN, num_n - panel * PN);      // the last panel may be narrower
+    int w = idx % per_panel;
+    const int remote = a.nv * rp_remote * cols;
+    const bool own = w >= remote;
+    if (own) w -= remote;
+    const int rp = own ? rp_own : rp_remote, vr = w / (rp * cols);
+    w %= rp * cols;
+    R = &a.r[vr]; rank = R->rank;
+    const int band = w / (BAND * cols), rows = min(BAND, rp - band * BAND);
+    w %= BAND * cols;
+    const int i = 2 * (band * BAND + w % rows) + v;
+    n_blk = panel * PN + w / rows;
+    if (own) m_blk = i < mb_per_owner ? rank * mb_per_owner + i : -1;
+    else m_blk = i < (n - 1) * mb_per_owner ? (rank + 1 + i / mb_per_owner) % n * mb_per_owner + i % mb_per_owner : -1;
   }
   __device__ void k_range(int, int num_kb, int& kb0, int& kb1) const { kb0 = 0; kb1 = num_kb; }
   __device__ const CUtensorMap* a_map(int m_blk, int& row0) const { row0 = max(m_blk, 0) * TP_BM; return &R->ta; }
+  __device__ const CUtensorMap* b_map() const { return &R->tb; }
   __device__ bool gate(int, volatile int*) const { return true; }
   __device__ int tile_id(int m_blk, int n_blk) const { return (m_blk % mb_per_owner) + n_blk * mb_per_owner; }
   __device__ unsigned* flag_ptr(int owner, int src, int t) const {
-    return reinterpret_cast<unsigned*>(R->heap[owner] + flag_off) + ((size_t)(parity * n + src) * tiles_per_owner + t);
+    return reinterpret_cast<unsigned*>(R->heap[owner] + a.flag_off) + ((size_t)(parity * n + src) * tiles_per_owner + t);
   }
   // A tile travels as pieces of 32 rows x 64 columns: 4 KiB each, the 16-byte words of a row 512 bytes apart, so that both the
   // staging stores of the writer and the loads of the reader take consecutive words.  data_off: this call's half of the region.
   __device__ char* piece(int owner, int src, int t, const EpiCtx& e, int pc) const {
-    return R->heap[owner] + data_off + ((size_t)src * tiles_per_owner + t) * (size_t)(TP_BM * TP_BN * 2) + (e.quarter * 4 + pc) * PAIR_STAGING;
+    return R->heap[owner] + a.data_off + ((size_t)src * tiles_per_owner + t) * (size_t)(TP_BM * TP_BN * 2) + (e.quarter * 4 + pc) * PAIR_STAGING;
   }
   __device__ void prefetch(const EpiCtx&, int, int) {}
+  // Lane 0: this warp's stores for the pending tile have been performed (at most KEEP newer groups may be in flight); the last of the eight warps
+  // of the tile tells the owner.
+  template <int KEEP> __device__ void announce() {
+    if (!pending) return;
+    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(KEEP) : "memory");
+    asm volatile("fence.proxy.async;" ::: "memory");
+    unsigned before;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_u32(&s_arrived[pending_slot])) : "memory");
+    if (before == PAIR_EPI_WARPS - 1) {
+      s_arrived[pending_slot] = 0;                       // used again four tiles on, when every warp has left this one
+      st_release_sys_u32(pending, a.epoch);
+    }
+    pending = nullptr;
+  }
+  __device__ void finish(const EpiCtx& e) { if (e.lane == 0) announce<0>(); }
   __device__ bool epilogue(const EpiCtx& e, int, int m_blk, int n_blk, volatile int* abort_flag) {
-    const int slot = seq++ & 1;
-    if (m_blk < 0) return true;
-    const int owner = m_blk / mb_per_owner, t = tile_id(m_blk, n_blk);
+    const int slot = seq++ & 3;
+    const int owner = m_blk < 0 ? -1 : m_blk / mb_per_owner, t = m_blk < 0 ? 0 : tile_id(m_blk, n_blk);
+    if (m_blk < 0 || owner == rank) {                    // nothing is held back where this warp may wait, or has nothing to store
+      if (e.lane == 0) announce<0>();
+      __syncwarp();
+      if (m_blk < 0) return true;
+    }
     if (owner != rank) {
-#pragma unroll 1
-      for (int pc = e.half * 2; pc < e.half * 2 + 2; pc++) {
+      // The two pieces of this warp go out from a staging buffer each; the flag of a tile is raised in the epilogue of the next one, when its
+      // stores have long been performed (waiting for them here made short K wait: 8192 x 8192 x 1024 among eight ranks 1.6 ms).
+#pragma unroll
+      for (int p = 0; p < 2; p++) {
+        const int pc = e.half * 2 + p;
+        uint8_t* const st = e.staging + p * PAIR_STAGING;
         float v[64];
         epi_load64(e, pc * 64, v);
-        epi_staging_free(e);
+        // this buffer's last store was two groups ago
+        if (e.lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
           for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(v[8 * j + 2 * q], v[8 * j + 2 * q + 1]);
-          *reinterpret_cast<uint4*>(e.staging + j * 512 + e.lane * 16) = o;
+          *reinterpret_cast<uint4*>(st + j * 512 + e.lane * 16) = o;
         }
         fence_proxy_async();                             // these stores must be visible to the bulk-copy engine
         __syncwarp();
-        if (e.lane == 0) { bulk_store(piece(owner, rank, t, e, pc), e.staging, PAIR_STAGING); bulk_commit(); }
+        if (e.lane == 0) { bulk_store(piece(owner, rank, t, e, pc), st, PAIR_STAGING); bulk_commit(); }
       }
-      if (e.lane == 0) {
-        bulk_wait_all();                                 // data written; the last of the eight warps tells the owner
-        asm volatile("fence.proxy.async;" ::: "memory");
-        __threadfence_system();
-        if (atomicAdd(&s_arrived[slot], 1u) == PAIR_EPI_WARPS - 1) {
-          s_arrived[slot] = 0;                           // used again two tiles on, after every warp has left this one
-          __threadfence_system();
-          st_release_sys_u32(flag_ptr(owner, rank, t), epoch);
-        }
-      }
+      if (e.lane == 0) { announce<2>(); pending = flag_ptr(owner, rank, t); pending_slot = slot; }
       __syncwarp();
       return true;
     }
     // own tile: all other ranks' partials of this tile must have landed
-    const bool ok = e.lane >= n || e.lane == rank || wait_flag(flag_ptr(rank, e.lane, t), epoch, abort_flag);
+    const bool ok = e.lane >= n || e.lane == rank || wait_flag(flag_ptr(rank, e.lane, t), a.epoch, abort_flag);
     if (!__all_sync(0xffffffffu, ok)) return false;
 #pragma unroll 1
     for (int pc = e.half * 2; pc < e.half * 2 + 2; pc++) {
-      float sum[64];
-#pragma unroll
-      for (int i = 0; i < 64; i++) sum[i] = 0.f;
+      epi_staging_free(e);
 #pragma unroll 1
-      for (int src = 0; src < n; src++) {                // rank order: the same result whatever the arrival order
-        if (src == rank) {
-          float v[64];
-          epi_load64(e, pc * 64, v);
+      for (int h = 0; h < 2; h++) {                      // 32 columns; the words of four partials are in flight at a time
+        float sum[32];
 #pragma unroll
-          for (int i = 0; i < 64; i++) sum[i] += v[i];
-        } else {
-          const char* p = piece(rank, src, t, e, pc) + e.lane * 16;
-          uint4 w[8];
+        for (int i = 0; i < 32; i++) sum[i] = 0.f;
+        auto add_own = [&]() {
+          uint32_t r[32];
+          tmem_ld_32x32(e.tmem + pc * 64 + h * 32, r);
+          tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 8; j++)
-            asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[j].x), "=r"(w[j].y), "=r"(w[j].z), "=r"(w[j].w) : "l"(p + j * 512) : "memory");
+          for (int i = 0; i < 32; i++) sum[i] += __uint_as_float(r[i]);
+        };
 #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&w[j]);
+        for (int b = 0; b < TP_MAX_RANKS - 1; b += 4) {  // rank order: the same result whatever the arrival order
+          uint4 w[4][4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) { float2 f = __bfloat1622float2(b2[q]); sum[8 * j + 2 * q] += f.x; sum[8 * j + 2 * q + 1] += f.y; }
+          for (int i = 0; i < 4; i++) {
+            if (b + i < n - 1) {
+              const char* p = piece(rank, b + i < rank ? b + i : b + i + 1, t, e, pc) + h * 2048 + e.lane * 16;
+#pragma unroll
+              for (int j = 0; j < 4; j++)
+                asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[i][j].x), "=r"(w[i][j].y), "=r"(w[i][j].z), "=r"(w[i][j].w) : "l"(p + j * 512) : "memory");
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            if (b + i == rank) add_own();
+            if (b + i < n - 1) {
+#pragma unroll
+              for (int j = 0; j < 4; j++) {
+                const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&w[i][j]);
+#pragma unroll
+                for (int q = 0; q < 4; q++) { float2 f = __bfloat1622float2(b2[q]); sum[8 * j + 2 * q] += f.x; sum[8 * j + 2 * q + 1] += f.y; }
+              }
+            }
           }
         }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+          for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(sum[8 * j + 2 * q], sum[8 * j + 2 * q + 1]);
+          *reinterpret_cast<uint4*>(e.staging + e.lane * 128 + (((h * 4 + j) ^ (e.lane & 7)) << 4)) = o;      // as epi_stage_row lays a row out
+        }
       }
-      epi_staging_free(e);
-      epi_stage_row(e, sum);
+      fence_proxy_async();
+      __syncwarp();
       epi_ship(e, &R->tc, n_blk * TP_BN + pc * 64, (m_blk % mb_per_owner) * TP_BM + e.quarter * 32);
     }
     return true;
@@ -186,27 +235,41 @@ struct RsPolicy {
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) gemm_rs_kernel(const __grid_constant__ TpArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int s_abort;
-  __shared__ unsigned s_arrived[2];
-  const int vr = blockIdx.x / a.ctas_per_rank, cta = blockIdx.x % a.ctas_per_rank;
-  const TpRank* R = &a.r[vr];
-  if (threadIdx.x == 0) { s_abort = 0; s_arrived[0] = 0; s_arrived[1] = 0; tma_prefetch_desc(&R->ta); tma_prefetch_desc(&R->tc); }
-  RsPolicy pol(a, R, s_arrived);
-  gemm_pair_persistent<TP_BN, RS_STAGES, false, false>(smem_raw, &R->tb, pol, a.K, cta >> 1, a.ctas_per_rank >> 1, R->status, &s_abort);
+  __shared__ unsigned s_arrived[4];
+  if (threadIdx.x == 0) { s_abort = 0; for (int i = 0; i < 4; i++) s_arrived[i] = 0; }
+  RsPolicy pol(a, s_arrived);
+  gemm_pair_persistent<TP_BN, RS_STAGES, false, false>(smem_raw, pol, a.K, blockIdx.x >> 1, gridDim.x >> 1, &s_abort);
 }
 
 // ------------------------------------------------------------------ all-gather -> GEMM
 constexpr int FEED_PIECE = 4096, FEED_STAGES = 8, FEED_AHEAD = 5;
 struct AgPolicy {
-  const TpArgs& a; const TpRank* R; int cta, rank, mb_per_shard, num_n, parity;
-  static constexpr int EXTRA_BYTES = FEED_STAGES * FEED_PIECE + FEED_STAGES * 8;
-  __device__ AgPolicy(const TpArgs& args, const TpRank* r, int c)
-      : a(args), R(r), cta(c), rank(r->rank), mb_per_shard(args.M / args.n / TP_BM), num_n(args.N / TP_BN), parity((int)(args.epoch & 1)) {}
+  const TpArgs& a; const TpRank* R = nullptr; int rank = 0, mb_per_shard, num_n, parity;
+  static constexpr int NSTAGE = 1, EXTRA_BYTES = FEED_STAGES * FEED_PIECE + FEED_STAGES * 8;
+  __device__ AgPolicy(const TpArgs& args) : a(args), mb_per_shard(args.M / args.n / TP_BM), num_n(args.N / TP_BN), parity((int)(args.epoch & 1)) {}
   __device__ void begin() const {}
-  __device__ int num_tiles() const { return (a.M / TP_BM + 1) / 2 * num_n; }
-  // row blocks of the own shard first, then rank+1, ..., two to a pair
-  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) const {
-    const int i = 2 * (idx / num_n) + v;
-    n_blk = idx % num_n;
+  __device__ void report(int role) const { for (int i = 0; i < a.nv; i++) atomicExch(a.r[i].status, role); }
+  __device__ int num_tiles() const { return a.nv * ((a.M / TP_BM + 1) / 2) * num_n; }
+  // Row blocks of the own shard first, then rank+1, ..., two to a pair; chunks of pairs, inside a chunk rows fastest (bands of 16).  The
+  // first chunk is the own shard, of every rank of the launch; after that a chunk is about a shard, so that little has to have arrived before it
+  // starts, or, with several ranks on the device, 16 pairs: their own shards gave the feeding time enough, and B is read less often.
+  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) {
+    constexpr int BAND = 16;
+    const int rp = (a.M / TP_BM + 1) / 2, own = (mb_per_shard + 1) / 2, chunk = a.nv > 1 ? BAND : own;
+    int base = 0, rows = own, w = idx;
+    const int first = a.nv * own * num_n;
+    if (w >= first) {
+      w -= first;
+      const int c = w / (a.nv * chunk * num_n);
+      w %= a.nv * chunk * num_n;
+      base = own + c * chunk; rows = min(chunk, rp - base);
+    }
+    R = &a.r[w / (rows * num_n)]; rank = R->rank;
+    w %= rows * num_n;
+    const int band = w / (BAND * num_n), in_band = min(BAND, rows - band * BAND);
+    w %= BAND * num_n;
+    const int i = 2 * (base + band * BAND + w % in_band) + v;
+    n_blk = w / in_band;
     m_blk = i < a.n * mb_per_shard ? (rank + i / mb_per_shard) % a.n * mb_per_shard + i % mb_per_shard : -1;
   }
   __device__ void k_range(int, int num_kb, int& kb0, int& kb1) const { kb0 = 0; kb1 = num_kb; }
@@ -215,19 +278,21 @@ struct AgPolicy {
     if (m_blk / mb_per_shard == rank) { row0 = (m_blk % mb_per_shard) * TP_BM; return &R->ta; }
     row0 = m_blk * TP_BM; return &R->ta2;               // ta2 covers this call's half of the region
   }
-  __device__ unsigned* flags(int dest, int src, int mb) const {
-    return reinterpret_cast<unsigned*>(R->heap[dest] + a.flag_off) + ((size_t)(parity * a.n + src) * mb_per_shard + mb) * a.n_part;
+  __device__ const CUtensorMap* b_map() const { return &R->tb; }
+  __device__ unsigned* flags(const TpRank* r, int dest, int src, int mb) const {
+    return reinterpret_cast<unsigned*>(r->heap[dest] + a.flag_off) + ((size_t)(parity * a.n + src) * mb_per_shard + mb) * a.n_part;
   }
   __device__ bool gate(int m_blk, volatile int* abort_flag) const {
     if (m_blk < 0 || m_blk / mb_per_shard == rank) return true;
     const int lane = threadIdx.x & 31;
-    const unsigned* f = flags(rank, m_blk / mb_per_shard, m_blk % mb_per_shard);
+    const unsigned* f = flags(R, rank, m_blk / mb_per_shard, m_blk % mb_per_shard);
     const bool ok = lane >= a.n_part || wait_flag(f + lane, a.epoch, abort_flag);
     const bool all = __all_sync(0xffffffffu, ok);
     asm volatile("fence.proxy.async;" ::: "memory");    // the rows arrived before the flags; TMA reads them through the async proxy
     return all;
   }
   __device__ void prefetch(const EpiCtx&, int, int) {}
+  __device__ void finish(const EpiCtx&) {}
   __device__ bool epilogue(const EpiCtx& e, int, int m_blk, int n_blk, volatile int*) {
     if (m_blk < 0) return true;
 #pragma unroll 1
@@ -249,13 +314,15 @@ struct AgPolicy {
     fence_barrier_init();
     uint32_t phase = 0;                                  // bit s: the parity the next wait on stage s looks for
     const size_t block_bytes = (size_t)TP_BM * a.K * 2, part_bytes = block_bytes / a.n_part;
-    const int per_dest = mb_per_shard * a.n_part, units = (a.n - 1) * per_dest, np = (int)((part_bytes + FEED_PIECE - 1) / FEED_PIECE);
+    const int per_dest = mb_per_shard * a.n_part, units = (a.n - 1) * a.nv * per_dest, np = (int)((part_bytes + FEED_PIECE - 1) / FEED_PIECE);
     bool ok = true;
-    for (int u = cta; u < units && ok; u += a.ctas_per_rank) {
-      const int dest = (rank - 1 - u / per_dest + a.n) % a.n, mb = u % per_dest / a.n_part, part = u % a.n_part;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const int step = u / per_dest, mb = u % per_dest / a.n_part, part = u % a.n_part;
+      const TpRank* r = &a.r[step % a.nv];
+      const int from = r->rank, dest = (from - 1 - step / a.nv + a.n) % a.n;
       const size_t off = (size_t)mb * block_bytes + (size_t)part * part_bytes;
-      const char* src = reinterpret_cast<const char*>(R->a_shard) + off;
-      char* dst = R->heap[dest] + a.data_off + (size_t)rank * (a.M / a.n) * a.K * 2 + off;
+      const char* src = reinterpret_cast<const char*>(r->a_shard) + off;
+      char* dst = r->heap[dest] + a.data_off + (size_t)from * (a.M / a.n) * a.K * 2 + off;
       int issued = 0;
       for (int i = 0; i < np + FEED_AHEAD; i++) {
         if (i < np && ok) {
@@ -280,9 +347,9 @@ struct AgPolicy {
       }
       bulk_wait_all();                                   // the writes are performed; then tell the reader
       asm volatile("fence.proxy.async;" ::: "memory");
-      if (ok) st_release_sys_u32(flags(dest, rank, mb) + part, a.epoch);
+      if (ok) st_release_sys_u32(flags(r, dest, from, mb) + part, a.epoch);
     }
-    if (!ok) { *abort_flag = 1; atomicExch(R->status, 7); }
+    if (!ok) { *abort_flag = 1; report(7); }
   }
 };
 
@@ -290,11 +357,9 @@ constexpr int AG_THREADS = PAIR_THREADS + 32;
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(AG_THREADS, 1) ag_gemm_kernel(const __grid_constant__ TpArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int s_abort;
-  const int vr = blockIdx.x / a.ctas_per_rank, cta = blockIdx.x % a.ctas_per_rank;
-  const TpRank* R = &a.r[vr];
-  if (threadIdx.x == 0) { s_abort = 0; tma_prefetch_desc(&R->ta); tma_prefetch_desc(&R->ta2); tma_prefetch_desc(&R->tc); }
-  AgPolicy pol(a, R, cta);
-  gemm_pair_persistent<TP_BN, AG_STAGES, false, false>(smem_raw, &R->tb, pol, a.K, cta >> 1, a.ctas_per_rank >> 1, R->status, &s_abort);
+  if (threadIdx.x == 0) s_abort = 0;
+  AgPolicy pol(a);
+  gemm_pair_persistent<TP_BN, AG_STAGES, false, false>(smem_raw, pol, a.K, blockIdx.x >> 1, gridDim.x >> 1, &s_abort);
 }
 
 // ------------------------------------------------------------------ host
@@ -344,7 +409,7 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
   const unsigned next_epoch = (which ? c0->tp_epoch_ag : c0->tp_epoch_rs) + 1;
   a.data_off = c0->h_ctx.tp_data_off + (which ? 2 * quarter : 0) + (long long)(next_epoch & 1) * quarter;
   a.n_part = ag_parts(M);
-  const int smem_bytes = which ? PairSmem<TP_BN, AG_STAGES, AgPolicy::EXTRA_BYTES>::DYNAMIC : PairSmem<TP_BN, RS_STAGES>::DYNAMIC;
+  const int smem_bytes = which ? PairSmem<TP_BN, AG_STAGES, AgPolicy::EXTRA_BYTES>::DYNAMIC : PairSmem<TP_BN, RS_STAGES, RsPolicy::EXTRA_BYTES, RsPolicy::NSTAGE>::DYNAMIC;
   const int threads = which ? AG_THREADS : PAIR_THREADS;
   auto fn = which ? ag_gemm_kernel : gemm_rs_kernel;
   cudaLaunchConfig_t cfg = {};
@@ -359,8 +424,7 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
     if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) { cudaGetLastError(); return fail(PICCL_CUDA_ERROR, "no room for a pair of CTAs with %d bytes of shared memory each", smem_bytes); }
     c0->tp_pairs[which] = std::min(active, c0->sm_count / 2);
   }
-  a.ctas_per_rank = 2 * (c0->tp_pairs[which] / n);
-  if (a.ctas_per_rank < 2) return fail(PICCL_UNSUPPORTED, "%d ranks do not fit on %d pairs of SMs", n, c0->tp_pairs[which]);
+  a.nv = n;
   bool ok = true;
   for (int i = 0; i < n && ok; i++) {
     piccl_comm* c = cs[i];
@@ -382,9 +446,9 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
     ok &= make_tmap_bf16_k64(&R.tc, out[i], (uint64_t)(which ? M : M / nr), (uint64_t)N, (uint64_t)N, 32);
   }
   if (!ok) return fail(PICCL_CUDA_ERROR, "tensor map or status set-up failed");
-  // ranks wait for one another inside the kernel: several virtual ranks on one device must be co-resident
+  // ranks wait for one another inside the kernel: with several virtual ranks on one device all CTAs must be resident at once
   at[0].id = cudaLaunchAttributeCooperative; at[0].val.cooperative = 1;
-  cfg.gridDim = dim3(n * a.ctas_per_rank); cfg.attrs = at; cfg.numAttrs = n > 1 ? 1 : 0;
+  cfg.gridDim = dim3(2 * c0->tp_pairs[which]); cfg.attrs = at; cfg.numAttrs = n > 1 ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, a);
   if (e != cudaSuccess) return fail(PICCL_CUDA_ERROR, "fused kernel launch failed: %s", cudaGetErrorString(e));
   for (int i = 0; i < n; i++) cs[i]->stats.launches++;

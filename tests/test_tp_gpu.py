@@ -106,3 +106,33 @@ def test_workspace_is_checked():
     with pytest.raises(N.PicclError):
         tp.gemm_rs_group(g, a, b, o)
     g.close()
+
+
+@pytest.mark.parametrize("n,M,N,K", [(1, 128, 256, 64), (2, 256, 256, 64), (3, 384, 512, 128), (4, 1536, 256, 64), (8, 1024, 512, 64), (8, 3072, 256, 192), (2, 512, 256 * 17, 64), (1, 128 * 35, 256, 64)])
+def test_odd_row_blocks_and_panel_edges(n, M, N, K):
+    """One, or an odd number of, 128-row blocks per rank (half of a pair has no block), more column blocks than a panel, more row pairs than a band, K of one
+    k-block.  A result of either kernel is an fp32 sum rounded to bf16 (2^-9), a partial of the reduce-scatter is rounded too: error norm below 4e-3 of the result's."""
+    from piccl_b200.parallel import tp
+    g = _group(n, "gemm_rs", M, N, K)
+    As, Bs = [_bf(M, K, seed=10 + r) for r in range(n)], [_bf(N, K, seed=20 + r, scale=0.1) for r in range(n)]
+    outs = [torch.full((M // n, N), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(n)]
+    for rep in range(3):
+        tp.gemm_rs_group(g, As, Bs, outs)
+    torch.cuda.synchronize()
+    assert all(tp.tp_status(h) == 0 for h in g._hs)
+    ref = sum(As[r].double() @ Bs[r].double().t() for r in range(n))
+    got = torch.cat(outs).double()
+    assert (got - ref).norm() <= 4e-3 * ref.norm()
+    g.close()
+    g = _group(n, "ag_gemm", M, N, K)
+    shards = [_bf(M // n, K, seed=30 + r) for r in range(n)]
+    outs = [torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(n)]
+    for rep in range(3):
+        tp.ag_gemm_group(g, shards, Bs, outs)
+    torch.cuda.synchronize()
+    assert all(tp.tp_status(h) == 0 for h in g._hs)
+    full = torch.cat(shards).double()
+    for r in range(n):
+        ref = full @ Bs[r].double().t()
+        assert (outs[r].double() - ref).norm() <= 4e-3 * ref.norm()
+    g.close()
