@@ -56,6 +56,7 @@ struct KernelArgs {
   int elem_size;
   int avg;                                // 1: scale original contributions by `scale`
   float scale;
+  long long seg_bytes;                    // bytes of a FIFO segment, at most the slot size; the same on every rank
   unsigned long long timeout_ns;
   LaunchRank r[kMaxVRanks];
 };
@@ -103,6 +104,8 @@ typedef void (*ExecKernelFn)(KernelArgs);
 // [dtype][op 0..3]; filled by the exec_inst_*.cu translation units.
 ExecKernelFn exec_kernel_for(int dtype, int op);
 ExecKernelFn exec_copy_kernel();
+ExecKernelFn exec_shift_kernel_for(int dtype, int op);   // operands that are not 16-byte aligned
+ExecKernelFn exec_shift_copy_kernel();
 ExecKernelFn exec_defer_kernel_for(int dtype, int op);   // counter updates held back until the CTA is about to block (PICCL_EXEC_DEFER=1)
 ExecKernelFn exec_defer_copy_kernel();
 ExecKernelFn exec_ll_kernel_for(int dtype, int op);   // low-latency variant (exec_ll.cuh)

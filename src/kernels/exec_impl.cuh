@@ -45,6 +45,7 @@ __device__ __forceinline__ uint4 ld_local(const void* p) { return *reinterpret_c
 __device__ __forceinline__ void st_vec(void* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
 
 // ---------------------------------------------------------------- element-wise maths
+constexpr int OP_COPY = 4;            // collectives that only move data: no action has two operands
 template <int OP, typename A> __device__ __forceinline__ A red(A x, A y) {
   if (OP == 0) return x + y;
   if (OP == 1) return x * y;
@@ -208,19 +209,120 @@ __device__ __noinline__ void reduce_copy_dispatch(int nsrc, const char* const* s
   constexpr int N = Pack<T>::N;
   // 16-byte packs in flight per thread: 8 when only moving data; for reductions bounded by the accumulator registers
   constexpr int UR = (sizeof(typename AccOf<T>::type) * N * 4 <= 128) ? 4 : 2;
-  if (nsrc == 1 && !do_scale) {
+  if (OP == OP_COPY || (nsrc == 1 && !do_scale)) {
     if (ndst == 1) copy_vec<8, 1>(src[0], local_src == 0, 1, dst, 0, npack);
     else if (ndst == 2) copy_vec<8, 2>(src[0], local_src == 0, 2, dst, 0, npack);
     else copy_vec<4, 0>(src[0], local_src == 0, ndst, dst, 0, npack);
     return;
   }
-  if (nsrc == 1 && ndst == 1) reduce_copy_vec<T, OP, UR, 1, 1>(1, src, local_src, 1, dst, 0, npack, do_scale, scale);
+  if constexpr (OP == OP_COPY) return;
+  else if (nsrc == 1 && ndst == 1) reduce_copy_vec<T, OP, UR, 1, 1>(1, src, local_src, 1, dst, 0, npack, do_scale, scale);
   else if (nsrc == 2 && ndst == 1) reduce_copy_vec<T, OP, UR, 2, 1>(2, src, local_src, 1, dst, 0, npack, do_scale, scale);
   else if (nsrc == 2 && ndst == 2) reduce_copy_vec<T, OP, UR, 2, 2>(2, src, local_src, 2, dst, 0, npack, do_scale, scale);
   else reduce_copy_vec<T, OP, (UR > 2 ? 2 : UR), 0, 0>(nsrc, src, local_src, ndst, dst, 0, npack, do_scale, scale);
 }
 
-// Element-wise path: unaligned user buffers and the last, partial pack of an action.
+// ---- user buffers that are not 16-byte aligned (a block of an all-gather or reduce-scatter whose length is odd, a view into a buffer)
+// bytes [s, s + 16) of the 32 bytes lo, hi
+__device__ __forceinline__ uint4 shift_pair(const uint4& lo, const uint4& hi, int s) {
+  uint32_t e[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  if (s & 8) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) e[i] = e[i + 2];
+  }
+  if (s & 4) {
+#pragma unroll
+    for (int i = 0; i < 5; i++) e[i] = e[i + 1];
+  }
+  const int b = (s & 3) * 8;
+  return make_uint4(__funnelshift_r(e[0], e[1], b), __funnelshift_r(e[1], e[2], b), __funnelshift_r(e[2], e[3], b), __funnelshift_r(e[3], e[4], b));
+}
+// bytes [from, to) of v to p + [from, to), p 16-byte aligned
+static __device__ __noinline__ void store_part(char* p, const uint4 v, int from, int to) {
+  union { uint4 v; unsigned char b[16]; } u; u.v = v;
+  for (int i = from; i < to; i++) reinterpret_cast<unsigned char*>(p)[i] = u.b[i];
+}
+// The same movement where the local operand (source index local_src) or dst[0] is at any byte address: an unaligned source is read as the
+// two aligned words around each pack (the second one is the neighbour's first and hits L1), an unaligned destination is written as aligned
+// words too, put together from a lane's pack and the one before it.  Only the two ends of the run of packs that a warp
+// writes (kRun blocks of 512 bytes) go out in bytes.  (An element at a time, the path before, moved 1 MiB blocks of a
+// four-rank all-gather in 171 us.)
+// An aligned word that is read may reach up to 15 bytes beyond the operand's ends; it never leaves the 16-byte granule of a byte that
+// belongs to the operand, and allocations are whole granules.
+constexpr int kRun = 4;
+template <typename T, int OP>
+__device__ __noinline__ void reduce_copy_shift(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst, int local_dst, long long npack, bool do_scale, float scale) {
+  typedef typename AccOf<T>::type A;
+  constexpr int N = Pack<T>::N;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int sm = local_src >= 0 ? (int)(reinterpret_cast<uintptr_t>(src[local_src]) & 15) : 0;
+  const int dm = local_dst >= 0 ? (int)(reinterpret_cast<uintptr_t>(dst[local_dst]) & 15) : 0;
+  for (long long run = (long long)warp * (32 * kRun); run < npack; run += (long long)nwarp * (32 * kRun)) {
+    uint4 o[kRun];
+#pragma unroll
+    for (int u = 0; u < kRun; u++) o[u] = make_uint4(0, 0, 0, 0);
+    if (OP == OP_COPY || (nsrc == 1 && !do_scale)) {
+      uint4 lo[kRun], hi[kRun];
+#pragma unroll
+      for (int u = 0; u < kRun; u++) {
+        const long long p = run + u * 32 + lane;
+        if (p < npack) {
+          const char* q = src[0] + p * 16;
+          if (local_src == 0) { lo[u] = ld_local(q - sm); if (sm) hi[u] = ld_local(q - sm + 16); }
+          else lo[u] = ld_slot(q);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kRun; u++) o[u] = sm && local_src == 0 ? shift_pair(lo[u], hi[u], sm) : lo[u];
+    } else {
+#pragma unroll
+      for (int u = 0; u < kRun; u++) {
+        const long long p = run + u * 32 + lane;
+        if (p < npack) {
+          A acc[N];
+          for (int s = 0; s < nsrc; s++) {
+            const char* q = src[s] + p * 16;
+            uint4 v;
+            if (s == local_src) { v = ld_local(q - sm); if (sm) v = shift_pair(v, ld_local(q - sm + 16), sm); }
+            else v = ld_slot(q);
+            A x[N]; Pack<T>::up(v, x);
+            const bool sc = do_scale && s == local_src;
+#pragma unroll
+            for (int e = 0; e < N; e++) { const A y = sc ? scale_val<A>(x[e], scale) : x[e]; acc[e] = s == 0 ? y : red<OP, A>(acc[e], y); }
+          }
+          o[u] = Pack<T>::down(acc);
+        }
+      }
+    }
+    for (int d = 0; d < ndst; d++) {
+      if (d != local_dst || dm == 0) {
+#pragma unroll
+        for (int u = 0; u < kRun; u++) { const long long p = run + u * 32 + lane; if (p < npack) st_vec(dst[d] + p * 16, o[u]); }
+        continue;
+      }
+      uint4 last = make_uint4(0, 0, 0, 0);             // the pack before lane 0's
+#pragma unroll
+      for (int u = 0; u < kRun; u++) {
+        const long long p = run + u * 32 + lane;
+        uint4 prev;
+        prev.x = __shfl_up_sync(0xffffffffu, o[u].x, 1); prev.y = __shfl_up_sync(0xffffffffu, o[u].y, 1);
+        prev.z = __shfl_up_sync(0xffffffffu, o[u].z, 1); prev.w = __shfl_up_sync(0xffffffffu, o[u].w, 1);
+        if (lane == 0) prev = last;
+        last.x = __shfl_sync(0xffffffffu, o[u].x, 31); last.y = __shfl_sync(0xffffffffu, o[u].y, 31);
+        last.z = __shfl_sync(0xffffffffu, o[u].z, 31); last.w = __shfl_sync(0xffffffffu, o[u].w, 31);
+        if (p < npack) {
+          char* const w = dst[d] + p * 16 - dm;        // aligned word: the last dm bytes of the pack before, then this pack's first 16 - dm
+          const uint4 v = shift_pair(prev, o[u], 16 - dm);
+          if (u == 0 && lane == 0) store_part(w, v, dm, 16);
+          else st_vec(w, v);
+          if (p == npack - 1 || (u == kRun - 1 && lane == 31)) store_part(w + 16, shift_pair(o[u], o[u], 16 - dm), 0, dm);
+        }
+      }
+    }
+  }
+}
+
+// Element-wise path: the last, partial pack of an action (and unaligned buffers in the deferring variant).
 template <typename T, int OP>
 __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
                                                  long long first, long long nelem, bool do_scale, float scale) {
@@ -248,7 +350,9 @@ constexpr int kSliceCache = 192;      // actions whose CTA slice is precomputed 
 // and publishes all of them together, with the fences of the owning threads running side by side, at the first point
 // where the CTA is about to block (one probe of the flags it needs; somebody may be waiting for what was held back) and at
 // the end of the kernel.  Nothing is ever held back across a wait, so progress is as in the plain variant.
-template <typename T, int OP, bool DEFER>
+// SHIFT = true: for calls with operands that are not 16-byte aligned (a kernel of its own: the mere presence of that path cost the aligned one
+// 15 % in registers).
+template <typename T, int OP, bool DEFER, bool SHIFT = false>
 __global__ void __launch_bounds__(kMaxBlock, 1) exec_kernel(const KernelArgs ka) {
   const int vr = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta;
   const LaunchRank& L = ka.r[vr];
@@ -269,11 +373,11 @@ __global__ void __launch_bounds__(kMaxBlock, 1) exec_kernel(const KernelArgs ka)
   if (tid < nranks) { s_heap[tid] = ctx->heap[tid]; my_sent = ctx->sent[tid * max_cta + cta]; my_rcvd = ctx->rcvd[tid * max_cta + cta]; }
   if (tid == 0) { s_fail = 0; s_maxseg = 0; }
   __syncthreads();
-  const long long seg_elems = (slot_bytes / 16) * (esz >= 16 ? 1 : 16 / esz);
+  const long long seg_bytes = ka.seg_bytes, seg_elems = (seg_bytes / 16) * (esz >= 16 ? 1 : 16 / esz);
   {
     int m = 0;
     for (int ai = tid; ai < L.n_actions; ai += blockDim.x) {
-      const Slice sl = slice_of(L.actions[ai].count, esz, cta, ka.n_cta, slot_bytes);
+      const Slice sl = slice_of(L.actions[ai].count, esz, cta, ka.n_cta, seg_bytes);
       if (ai < kSliceCache) { s_lo[ai] = sl.lo; s_hi[ai] = sl.hi; }
       m = max(m, sl.nseg);
     }
@@ -298,7 +402,7 @@ __global__ void __launch_bounds__(kMaxBlock, 1) exec_kernel(const KernelArgs ka)
     for (int ai = 0; ai < L.n_actions; ai++) {
       long long sl_lo, sl_hi;
       if (ai < kSliceCache) { sl_lo = s_lo[ai]; sl_hi = s_hi[ai]; }
-      else { const Slice sl = slice_of(L.actions[ai].count, esz, cta, ka.n_cta, slot_bytes); sl_lo = sl.lo; sl_hi = sl.hi; }
+      else { const Slice sl = slice_of(L.actions[ai].count, esz, cta, ka.n_cta, seg_bytes); sl_lo = sl.lo; sl_hi = sl.hi; }
       const long long lo = sl_lo + (long long)seg * seg_elems;
       if (lo >= sl_hi) continue;
       const long long hi = (lo + seg_elems < sl_hi) ? lo + seg_elems : sl_hi;
@@ -373,8 +477,9 @@ __global__ void __launch_bounds__(kMaxBlock, 1) exec_kernel(const KernelArgs ka)
 
       // ---- one pass over the segment
       constexpr int N = Pack<T>::N;
-      long long nfull = aligned ? len / N : 0;
-      if (nfull) reduce_copy_dispatch<T, OP>(nsrc, src, local_src, ndst, dst, nfull, do_scale, ka.scale);
+      const long long nfull = (aligned || SHIFT) ? len / N : 0;
+      if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(nsrc, src, local_src, ndst, dst, ac.dst_buf != BUF_NONE ? 0 : -1, nfull, do_scale, ka.scale); }
+      else if (nfull) reduce_copy_dispatch<T, OP>(nsrc, src, local_src, ndst, dst, nfull, do_scale, ka.scale);
       if (nfull * N < len) reduce_copy_elem<T, OP>(nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale, ka.scale);
       __syncthreads();
 
@@ -386,13 +491,15 @@ __global__ void __launch_bounds__(kMaxBlock, 1) exec_kernel(const KernelArgs ka)
         }
         pending = true;
       } else if (tid < nranks) {
+        // the slots are read (their packs went through registers before the barrier), so a plain store frees them: a release would wait
+        // for the acknowledgement of everything the CTA stored
+        for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == tid) {
+          my_rcvd++;
+          *reinterpret_cast<volatile unsigned long long*>(s_heap[tid] + head_off + (long long)(rank * max_cta + cta) * kFlagStride) = my_rcvd;
+        }
         for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == tid) {
           my_sent++;
           st_release_sys(reinterpret_cast<unsigned long long*>(s_heap[tid] + tail_off + (long long)(rank * max_cta + cta) * kFlagStride), my_sent);
-        }
-        for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == tid) {
-          my_rcvd++;
-          st_release_sys(reinterpret_cast<unsigned long long*>(s_heap[tid] + head_off + (long long)(rank * max_cta + cta) * kFlagStride), my_rcvd);
         }
       }
     }

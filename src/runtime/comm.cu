@@ -351,6 +351,7 @@ static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, co
         return fail(PICCL_INTERNAL_ERROR, "program check failed (%s %s, rank %d): %s", coll_name(a.coll), algo_name(a.algo), c->rank, why);
     }
     ProgEntry e;
+    for (const Action& ac : p.actions) e.offsets_aligned &= (ac.src_off * a.elem_size) % 16 == 0 && (ac.dst_off * a.elem_size) % 16 == 0;
     int rc = upload_program(c, p, stream, e); if (rc) return rc;
     it = c->cache.emplace(k, e).first;
   } else {
@@ -606,6 +607,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     KernelArgs ka; memset(&ka, 0, sizeof ka);
     ka.n_vrank = n; ka.elem_size = esz; ka.avg = avg ? 1 : 0; ka.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
     int n_cta = 0;
+    bool aligned = true;
     for (int i = 0; i < n && rc == PICCL_OK; i++) {
       piccl_comm* c = comms[i]; const CallDesc& d = calls[i];
       std::lock_guard<std::mutex> l(c->mu);
@@ -628,9 +630,10 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
           n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
           if (n > 1) n_cta = std::min(n_cta, std::max(1, c->sm_count / n));
         }
-        ka.n_cta = n_cta; ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
+        ka.n_cta = n_cta; ka.seg_bytes = c->h_ctx.slot_bytes; ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
       }
       ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
+      aligned &= pe->offsets_aligned && ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(r)) & 15) == 0;
       c->stats.launches++;
     }
     if (rc) break;
@@ -642,8 +645,10 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     void* args[] = {&ka};
     cudaError_t e;
     const int block = use_llf ? kLLBlock : c0->cfg.block_size;
-    if (n > 1) e = cudaLaunchCooperativeKernel((const void*)fn, dim3(n * n_cta), dim3(block), args, 0, stream);
-    else e = cudaLaunchKernel((const void*)fn, dim3(n_cta), dim3(block), args, 0, stream);
+    // which kernel a rank runs is its own business: both speak the same protocol
+    const ExecKernelFn f = (aligned || use_llf || defer) ? fn : reducing ? exec_shift_kernel_for(d0.dtype, op) : exec_shift_copy_kernel();
+    if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n * n_cta), dim3(block), args, 0, stream);
+    else e = cudaLaunchKernel((const void*)f, dim3(n_cta), dim3(block), args, 0, stream);
     if (e != cudaSuccess) rc = fail(PICCL_CUDA_ERROR, "executor launch failed: %s", cudaGetErrorString(e));
     trace_end(c0, tr, stream);
   }
@@ -700,7 +705,7 @@ int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream) {
   int rc = upload_program(c, p, (cudaStream_t)stream, e); if (rc) return rc;
   c->cache.emplace(ProgKey{-1, 0, 0, 0, 1, 0, (long long)c->cache.size(), 0}, e);
   KernelArgs ka; memset(&ka, 0, sizeof ka);
-  ka.n_vrank = 1; ka.n_cta = 1; ka.elem_size = 1; ka.scale = 1.f; ka.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
+  ka.n_vrank = 1; ka.n_cta = 1; ka.elem_size = 1; ka.seg_bytes = c->h_ctx.slot_bytes; ka.scale = 1.f; ka.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
   ka.r[0].ctx = c->d_ctx; ka.r[0].actions = e.dev; ka.r[0].n_actions = 1;
   void* args[] = {&ka};
   CUDA_TRY(cudaLaunchKernel((const void*)exec_copy_kernel(), dim3(1), dim3(c->cfg.block_size), args, 0, (cudaStream_t)stream));

@@ -329,3 +329,35 @@ def test_low_latency_lines_spread_over_ctas(count, coll, algo):
                 ref = ref[r * count:(r + 1) * count] if coll == "reduce_scatter" else ref
                 assert torch.allclose(outs[r], ref, atol=7 * 8 * 2.0 ** -24, rtol=0)
     g.close()
+
+
+@pytest.mark.parametrize("dtype,offset", [(torch.uint8, 3), (torch.bfloat16, 1), (torch.float32, 3), (torch.float64, 1), (torch.bfloat16, 0)])
+@pytest.mark.parametrize("coll,algo", [("allgather", "RING"), ("allgather", "PRD"), ("broadcast", "RING"), ("reduce_scatter", "RING"), ("reduce_scatter", "PRD"), ("allreduce", "RING"),
+                                       ("allreduce", "PRM"), ("reduce", "RING"), ("allreduce", "DIRECT")])
+def test_operands_at_any_address(groups, coll, algo, dtype, offset):
+    """Messages too large for the low-latency path with operands that are not 16-byte aligned (a view that starts `offset` elements into its buffer, blocks of
+    an odd length): every byte of the result, and the bytes around it untouched.  Whole numbers and byte moves are exact; values are small integers, so sums are too."""
+    n, g = 4, groups(4)
+    count = 70001 * (4 if dtype == torch.uint8 else 1)
+    n_in, n_out = count * (n if coll == "reduce_scatter" else 1), count * (n if coll == "allgather" else 1)
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    high = 30 if dtype == torch.uint8 else 9
+    xs = [torch.randint(0, high, (n_in + 8,), generator=gen, device="cuda").to(dtype)[offset:offset + n_in] for _ in range(n)]
+    bufs = [torch.full((n_out + 40,), 77, device="cuda").to(dtype) for _ in range(n)]
+    outs = [b[16 + offset:16 + offset + n_out] for b in bufs]
+    g.run(coll, xs, outs, count, op="sum", root=1, algo=algo, k=2)
+    _check_ok(g)
+    total = torch.stack([x.double() for x in xs]).sum(0)
+    for r in range(n):
+        if coll == "allgather":
+            want = torch.cat(xs)
+        elif coll == "broadcast":
+            want = xs[1]
+        elif coll == "reduce_scatter":
+            want = total[r * count:(r + 1) * count].to(dtype)
+        elif coll == "reduce" and r != 1:
+            want = torch.full_like(outs[r], 77)
+        else:
+            want = total.to(dtype)
+        assert torch.equal(outs[r], want), f"rank {r}"
+        assert torch.all(bufs[r][:16 + offset] == 77) and torch.all(bufs[r][16 + offset + n_out:] == 77), f"rank {r} wrote outside its buffer"
