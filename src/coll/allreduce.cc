@@ -54,15 +54,18 @@ static Program ar_recursive(const CollArgs& a, const Resolved& rs, int rank, boo
   Buf cur = BUF_IN;
   if (!followers.empty()) { b.act(BUF_IN, 0, BUF_OUT, 0, a.count, followers, {}); cur = BUF_OUT; }
   if (core < n) b.next_step();
+  // One action per step: all partners' values + mine, in rank order, to the partners of the next step (after the last one to the followers) while
+  // the sum is stored, so it is never read back to be sent.
   for (size_t s = 0; s < rs.radices.size(); s++) {
     std::vector<int> peers = step_peers(rank, (int)s, rs.radices, core, permuted);
-    b.act(cur, 0, BUF_NONE, 0, a.count, {}, peers);        // my current value to every partner
-    b.act(cur, 0, BUF_OUT, 0, a.count, peers, {});         // all partners' values + mine, in rank order
+    if (s == 0) b.act(cur, 0, BUF_NONE, 0, a.count, {}, peers);
+    std::vector<int> next = s + 1 < rs.radices.size() ? step_peers(rank, (int)s + 1, rs.radices, core, permuted) : followers;
+    b.act(cur, 0, BUF_OUT, 0, a.count, peers, next);
     cur = BUF_OUT;
     b.next_step();
   }
   if (cur == BUF_IN && !a.in_place) b.act(BUF_IN, 0, BUF_OUT, 0, a.count, {}, {});
-  if (!followers.empty()) { b.act(BUF_OUT, 0, BUF_NONE, 0, a.count, {}, followers); b.next_step(); }
+  if (!followers.empty()) { if (rs.radices.empty()) b.act(BUF_OUT, 0, BUF_NONE, 0, a.count, {}, followers); b.next_step(); }
   return b.finish();
 }
 

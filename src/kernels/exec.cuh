@@ -21,7 +21,8 @@ namespace piccl {
 
 constexpr int kFlagStride = 128;          // bytes between two counters
 constexpr int kMaxVRanks = 8;             // virtual ranks one launch can carry (single-GPU emulation)
-constexpr int kMaxBlock = 512;
+constexpr int kMaxBlock = 512;             // threads of an executor CTA that move data
+constexpr int kCtlThreads = 64;            // and two warps more: waiter and publisher
 constexpr int kLLFifoCta = 16, kLLFifoSlots = 8, kLLFifoSlotBytes = 8192;   // low-latency FIFO: CTAs, ring depth, bytes per slot (half of it payload)
 
 struct RankCtx {
@@ -56,7 +57,10 @@ struct KernelArgs {
   int elem_size;
   int avg;                                // 1: scale original contributions by `scale`
   float scale;
-  long long seg_bytes;                    // bytes of a FIFO segment, at most the slot size; the same on every rank
+  // How a channel's FIFO memory (nslot * slot_bytes of the communicator) is cut up for this call; the same on every rank.  All entries of earlier calls
+  // are consumed, so the cut may differ from call to call where no rank can be a call ahead (one launch for all ranks).
+  long long seg_bytes;                    // bytes of a segment and of its slot
+  int nslot, window;                      // slots; segments that are walked together, at most half the slots
   unsigned long long timeout_ns;
   LaunchRank r[kMaxVRanks];
 };
@@ -106,8 +110,6 @@ ExecKernelFn exec_kernel_for(int dtype, int op);
 ExecKernelFn exec_copy_kernel();
 ExecKernelFn exec_shift_kernel_for(int dtype, int op);   // operands that are not 16-byte aligned
 ExecKernelFn exec_shift_copy_kernel();
-ExecKernelFn exec_defer_kernel_for(int dtype, int op);   // counter updates held back until the CTA is about to block (PICCL_EXEC_DEFER=1)
-ExecKernelFn exec_defer_copy_kernel();
 ExecKernelFn exec_ll_kernel_for(int dtype, int op);   // low-latency variant (exec_ll.cuh)
 ExecKernelFn exec_ll_copy_kernel();
 

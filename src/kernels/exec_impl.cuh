@@ -1,17 +1,25 @@
 // The fused collective executor: ONE kernel runs a whole collective.  Each CTA
-// owns a fixed slice of every action; for each FIFO segment it walks the
-// action program, and every action is a single pass
+// owns a fixed slice of every action; for each window of FIFO segments it walks
+// the action program, and every (action, segment) is a step, a single pass
 //     wait (bounded) -> load local + incoming slots -> reduce in registers ->
 //     store local + peers' slots -> publish counters
 // so reduction (reference: src/kernels/reduce_kernel.cu, one launch per step)
 // and block placement (reference: src/kernels/permutation_kernel.cu) never
 // exist as separate passes, and no ncclSend/ncclRecv is issued.
 //
+// Roles inside a CTA: one warp waits (credits and data of the next steps, up to
+// kStepDepth ahead), all warps but two move data, one warp publishes (a release
+// store waits for the acknowledgement of everything the CTA stored, a microsecond
+// and more).  They meet through named barriers per step, so the chain
+//     peer's stores -> its release -> my poll -> my loads
+// of one step overlaps the data movement of others.  With one group of threads doing all of it in
+// turn a 64 KiB step took 10 us, 3 of them for the data.
+//
 // Peer traffic is plain 16-byte stores into the peer's mapped heap (NVLink /
-// NVSwitch P2P); ordering is fence.acq_rel.sys + st.release.sys on the
-// producer and ld.acquire.sys on the consumer.  Every wait has a time limit;
-// on expiry the CTA records where it gave up, raises the abort flag that all
-// other waits poll, and the kernel returns.
+// NVSwitch P2P); ordering is st.release.sys on the producer and ld.acquire.sys
+// on the consumer.  Every wait has a time limit; on expiry the CTA records
+// where it gave up, raises the abort flag that all other waits poll, and the
+// kernel returns.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -95,12 +103,12 @@ template <> __device__ __forceinline__ double scale_val<double>(double v, float 
 // ---------------------------------------------------------------- bounded wait
 struct WaitCtx { RankCtx* ctx; unsigned long long timeout_ns; int cta, action, segment; };
 
-// Returns false if the wait was given up (time limit or abort raised elsewhere).
-static __device__ __noinline__ bool wait_counter(const unsigned long long* flag, unsigned long long want, const WaitCtx& w, int code, int peer) {
+// Returns false if the wait was given up (time limit or abort raised elsewhere).  `seen` (optional): the value last read.
+static __device__ __noinline__ bool wait_counter(const unsigned long long* flag, unsigned long long want, const WaitCtx& w, int code, int peer, unsigned long long* seen = nullptr) {
   unsigned long long t0 = 0, have = 0;
   for (unsigned spins = 1;; spins++) {
     have = ld_acquire_sys(flag);
-    if (have >= want) return true;
+    if (have >= want) { if (seen) *seen = have; return true; }
     if ((spins & 31u) == 0) {
       if (*(volatile int*)w.ctx->abort_flag) return false;
       unsigned long long now = globaltimer_ns();
@@ -121,105 +129,93 @@ static __device__ __noinline__ bool wait_counter(const unsigned long long* flag,
 }
 
 // ---------------------------------------------------------------- data movement
-// value = reduce(src[0..NSRC)) -> dst[0..NDST); `local_src` (index or -1) is the
-// user-buffer operand (plain loads, optional scaling); the other sources are FIFO slots.
-// NSRC / NDST > 0: compile-time operand counts (pointers stay in registers, loops unroll);
-// 0: run-time counts (generic path for wide radices).
-// Both loops run an unpredicated main part (all U packs of a thread in range) and finish the
-// remainder one pack at a time, which keeps the register count of the main part low.
-template <int U, int NDST>
-__device__ __forceinline__ void copy_vec(const char* src, bool src_local, int ndst_rt, char* const* dst, long long first, long long npack) {
-  const int ndst = NDST ? NDST : ndst_rt;
-  const long long nt = blockDim.x;
-  // whole super-blocks of nt * U packs; the rest is done one pack per thread at a time
-  const long long done = (U == 1) ? npack : first + ((npack - first) / (nt * U)) * (nt * U);
-  for (long long base = first + threadIdx.x; base < done; base += nt * U) {
-    uint4 v[U];
-    const char* sp = src + base * 16;
-#pragma unroll
-    for (int u = 0; u < U; u++) v[u] = src_local ? ld_local(sp + u * nt * 16) : ld_slot(sp + u * nt * 16);
-#pragma unroll
-    for (int d = 0; d < (NDST ? NDST : kMaxActionPeers + 1); d++) {
-      if (d < ndst) {
-        char* dp = dst[d] + base * 16;
-#pragma unroll
-        for (int u = 0; u < U; u++) st_vec(dp + u * nt * 16, v[u]);
-      }
-    }
-  }
-  if (U > 1 && done < npack) copy_vec<1, NDST>(src, src_local, ndst_rt, dst, done, npack);
-}
+__device__ __forceinline__ int data_threads() { return (int)blockDim.x - kCtlThreads; }
 
-template <typename T, int OP, int U, int NSRC, int NDST>
-__device__ __forceinline__ void reduce_copy_vec(int nsrc_rt, const char* const* src, int local_src, int ndst_rt, char* const* dst,
-                                                long long first, long long npack, bool do_scale, float scale) {
-  typedef typename AccOf<T>::type A;
-  constexpr int N = Pack<T>::N;
-  const int nsrc = NSRC ? NSRC : nsrc_rt, ndst = NDST ? NDST : ndst_rt;
-  const long long nt = blockDim.x;
-  const long long done = (U == 1) ? npack : first + ((npack - first) / (nt * U)) * (nt * U);
-  for (long long base = first + threadIdx.x; base < done; base += nt * U) {
-    A acc[U][N];
-    {
-      const char* sp = src[0] + base * 16;
+// value = reduce(src[0..nsrc)) -> dst[0..ndst), everything 16-byte aligned; `scaled`: index of the operand that is scaled first (avg), or -1.
+// The operands' packs stay as they were loaded until they are combined, so a thread has NSRC * U loads of 16 bytes in flight and no array of
+// accumulators; offsets are 32-bit (a segment is at most a slot).  Whatever U is, pack p is thread p % (data threads)'s, so a step may read what an earlier one
+// wrote.  The last round is as wide as the others instead of being finished a pack at a time, which took up to U - 1 further round trips: what lies
+// beyond the end loads the last pack again (loads under a condition made the compiler spill).  The slots' packs may
+// have been written by another GPU and the local operand is read once: all loads go past L1.
+template <typename T, int OP, int NSRC, bool SCALE>
+__device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, int scaled, float scale) {      // v[s * stride]: operand s
+  if constexpr (OP == OP_COPY) return v[0];
+  else {
+    typedef typename AccOf<T>::type A;
+    constexpr int N = Pack<T>::N;
+    if (NSRC == 1 && !SCALE) return v[0];
+    A acc[N];
+    Pack<T>::up(v[0], acc);
+    if (SCALE && scaled == 0) {
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        uint4 v = (local_src == 0) ? ld_local(sp + u * nt * 16) : ld_slot(sp + u * nt * 16);
-        Pack<T>::up(v, acc[u]);
-        if (do_scale && local_src == 0) {
-#pragma unroll
-          for (int e = 0; e < N; e++) acc[u][e] = scale_val<A>(acc[u][e], scale);
-        }
-      }
+      for (int e = 0; e < N; e++) acc[e] = scale_val<A>(acc[e], scale);
     }
 #pragma unroll
-    for (int s = 1; s < (NSRC ? NSRC : kMaxActionPeers + 1); s++) {
+    for (int s = 1; s < NSRC; s++) {
       if (s < nsrc) {
-        uint4 v[U];
-        const char* sp = src[s] + base * 16;
+        A x[N]; Pack<T>::up(v[s * stride], x);
+        if (SCALE && scaled == s) {
 #pragma unroll
-        for (int u = 0; u < U; u++) v[u] = (local_src == s) ? ld_local(sp + u * nt * 16) : ld_slot(sp + u * nt * 16);
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          A x[N]; Pack<T>::up(v[u], x);
-#pragma unroll
-          for (int e = 0; e < N; e++) {
-            A xv = (do_scale && local_src == s) ? scale_val<A>(x[e], scale) : x[e];
-            acc[u][e] = red<OP, A>(acc[u][e], xv);
-          }
+          for (int e = 0; e < N; e++) x[e] = scale_val<A>(x[e], scale);
         }
+#pragma unroll
+        for (int e = 0; e < N; e++) acc[e] = red<OP, A>(acc[e], x[e]);
       }
     }
-#pragma unroll
-    for (int d = 0; d < (NDST ? NDST : kMaxActionPeers + 1); d++) {
-      if (d < ndst) {
-        char* dp = dst[d] + base * 16;
-#pragma unroll
-        for (int u = 0; u < U; u++) st_vec(dp + u * nt * 16, Pack<T>::down(acc[u]));
-      }
-    }
+    return Pack<T>::down(acc);
   }
-  if (U > 1 && done < npack) reduce_copy_vec<T, OP, 1, NSRC, NDST>(nsrc_rt, src, local_src, ndst_rt, dst, done, npack, do_scale, scale);
 }
-
-// Picks the instantiation for the common operand counts of ring / pairwise schedules.
-template <typename T, int OP>
-__device__ __noinline__ void reduce_copy_dispatch(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
-                                                     long long npack, bool do_scale, float scale) {
-  constexpr int N = Pack<T>::N;
-  // 16-byte packs in flight per thread: 8 when only moving data; for reductions bounded by the accumulator registers
-  constexpr int UR = (sizeof(typename AccOf<T>::type) * N * 4 <= 128) ? 4 : 2;
-  if (OP == OP_COPY || (nsrc == 1 && !do_scale)) {
-    if (ndst == 1) copy_vec<8, 1>(src[0], local_src == 0, 1, dst, 0, npack);
-    else if (ndst == 2) copy_vec<8, 2>(src[0], local_src == 0, 2, dst, 0, npack);
-    else copy_vec<4, 0>(src[0], local_src == 0, ndst, dst, 0, npack);
-    return;
+template <typename T, int OP, int NSRC, int NDST, int U, bool EXACT, bool SCALE = false>      // EXACT: nsrc == NSRC, else the first operand stands in for what is missing; NDST 0: any number, read from the table each time
+__device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char* const* dst, int ndst, int n, int scaled, float scale) {
+  const int nsrc = EXACT ? NSRC : nsrc_rt, nt = data_threads(), tid = threadIdx.x;
+  const char* sp[NSRC]; char* dp[NDST ? NDST : 1];
+#pragma unroll
+  for (int s = 0; s < NSRC; s++) sp[s] = src[EXACT || s < nsrc ? s : 0];
+#pragma unroll
+  for (int d = 0; d < NDST; d++) dp[d] = dst[d];
+  auto put = [&](int off, const uint4& o) {
+#pragma unroll
+    for (int d = 0; d < NDST; d++) st_vec(dp[d] + off, o);
+    if (NDST == 0) for (int d = 0; d < ndst; d++) st_vec(dst[d] + off, o);
+  };
+  int p = tid;
+  for (; p + (U - 1) * nt < n; p += U * nt) {
+    uint4 v[NSRC][U];
+#pragma unroll
+    for (int s = 0; s < NSRC; s++)
+#pragma unroll
+      for (int u = 0; u < U; u++) v[s][u] = ld_slot(sp[s] + (p + u * nt) * 16);
+#pragma unroll
+    for (int u = 0; u < U; u++) put((p + u * nt) * 16, combine<T, OP, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
   }
-  if constexpr (OP == OP_COPY) return;
-  else if (nsrc == 1 && ndst == 1) reduce_copy_vec<T, OP, UR, 1, 1>(1, src, local_src, 1, dst, 0, npack, do_scale, scale);
-  else if (nsrc == 2 && ndst == 1) reduce_copy_vec<T, OP, UR, 2, 1>(2, src, local_src, 1, dst, 0, npack, do_scale, scale);
-  else if (nsrc == 2 && ndst == 2) reduce_copy_vec<T, OP, UR, 2, 2>(2, src, local_src, 2, dst, 0, npack, do_scale, scale);
-  else reduce_copy_vec<T, OP, (UR > 2 ? 2 : UR), 0, 0>(nsrc, src, local_src, ndst, dst, 0, npack, do_scale, scale);
+  if (U > 1 && p < n) {
+    uint4 v[NSRC][U];
+#pragma unroll
+    for (int s = 0; s < NSRC; s++)
+#pragma unroll
+      for (int u = 0; u < U - 1; u++) v[s][u] = ld_slot(sp[s] + min(p + u * nt, n - 1) * 16);
+#pragma unroll
+    for (int u = 0; u < U - 1; u++) if (p + u * nt < n) put((p + u * nt) * 16, combine<T, OP, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
+  }
+}
+template <typename T, int OP>
+__device__ __forceinline__ void move_aligned(const char* const* src, int nsrc, char* const* dst, int ndst, int n, int scaled, float scale) {
+  if (OP == OP_COPY || (nsrc == 1 && scaled < 0)) {
+    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(src, 1, dst, 1, n, -1, scale);
+    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(src, 1, dst, 2, n, -1, scale);
+    else stream<T, OP, 1, 0, 4, true>(src, 1, dst, ndst, n, -1, scale);
+  } else if constexpr (OP != OP_COPY) {
+    if (scaled >= 0) {
+      if (nsrc <= 2) stream<T, OP, 2, 0, 4, false, true>(src, nsrc, dst, ndst, n, scaled, scale);
+      else stream<T, OP, kMaxActionPeers + 1, 0, 1, false, true>(src, nsrc, dst, ndst, n, scaled, scale);
+    }
+    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(src, 2, dst, 1, n, -1, scale);
+    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(src, 2, dst, 2, n, -1, scale);
+    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(src, 4, dst, ndst, n, -1, scale);
+    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(src, nsrc, dst, ndst, n, -1, scale);
+    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(src, nsrc, dst, ndst, n, -1, scale);
+    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(src, nsrc, dst, ndst, n, -1, scale);
+  }
 }
 
 // ---- user buffers that are not 16-byte aligned (a block of an all-gather or reduce-scatter whose length is odd, a view into a buffer)
@@ -243,7 +239,7 @@ static __device__ __noinline__ void store_part(char* p, const uint4 v, int from,
   for (int i = from; i < to; i++) reinterpret_cast<unsigned char*>(p)[i] = u.b[i];
 }
 // The same movement where the local operand (source index local_src) or dst[0] is at any byte address: an unaligned source is read as the
-// two aligned words around each pack (the second one is the neighbour's first and hits L1), an unaligned destination is written as aligned
+// two aligned words around each pack (the second one is the neighbour's first and hits L2), an unaligned destination is written as aligned
 // words too, put together from a lane's pack and the one before it.  Only the two ends of the run of packs that a warp
 // writes (kRun blocks of 512 bytes) go out in bytes.  (An element at a time, the path before, moved 1 MiB blocks of a
 // four-rank all-gather in 171 us.)
@@ -254,45 +250,41 @@ template <typename T, int OP>
 __device__ __noinline__ void reduce_copy_shift(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst, int local_dst, long long npack, bool do_scale, float scale) {
   typedef typename AccOf<T>::type A;
   constexpr int N = Pack<T>::N;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = data_threads() >> 5;
   const int sm = local_src >= 0 ? (int)(reinterpret_cast<uintptr_t>(src[local_src]) & 15) : 0;
   const int dm = local_dst >= 0 ? (int)(reinterpret_cast<uintptr_t>(dst[local_dst]) & 15) : 0;
   for (long long run = (long long)warp * (32 * kRun); run < npack; run += (long long)nwarp * (32 * kRun)) {
     uint4 o[kRun];
-#pragma unroll
-    for (int u = 0; u < kRun; u++) o[u] = make_uint4(0, 0, 0, 0);
     if (OP == OP_COPY || (nsrc == 1 && !do_scale)) {
       uint4 lo[kRun], hi[kRun];
 #pragma unroll
-      for (int u = 0; u < kRun; u++) {
-        const long long p = run + u * 32 + lane;
-        if (p < npack) {
-          const char* q = src[0] + p * 16;
-          if (local_src == 0) { lo[u] = ld_local(q - sm); if (sm) hi[u] = ld_local(q - sm + 16); }
-          else lo[u] = ld_slot(q);
-        }
+      for (int u = 0; u < kRun; u++) {                 // beyond the end: the last pack again (a load under a condition makes the compiler spill)
+        const char* q = src[0] + min(run + u * 32 + lane, npack - 1) * 16 - sm;      // sm is 0 for a slot
+        lo[u] = ld_slot(q); hi[u] = ld_slot(q + (sm ? 16 : 0));
       }
 #pragma unroll
-      for (int u = 0; u < kRun; u++) o[u] = sm && local_src == 0 ? shift_pair(lo[u], hi[u], sm) : lo[u];
+      for (int u = 0; u < kRun; u++) o[u] = sm ? shift_pair(lo[u], hi[u], sm) : lo[u];
     } else {
+      A acc[kRun][N];
+#pragma unroll 1
+      for (int s = 0; s < nsrc; s++) {
+        const int m = s == local_src ? sm : 0;
+        uint4 lo[kRun], hi[kRun];
 #pragma unroll
-      for (int u = 0; u < kRun; u++) {
-        const long long p = run + u * 32 + lane;
-        if (p < npack) {
-          A acc[N];
-          for (int s = 0; s < nsrc; s++) {
-            const char* q = src[s] + p * 16;
-            uint4 v;
-            if (s == local_src) { v = ld_local(q - sm); if (sm) v = shift_pair(v, ld_local(q - sm + 16), sm); }
-            else v = ld_slot(q);
-            A x[N]; Pack<T>::up(v, x);
-            const bool sc = do_scale && s == local_src;
+        for (int u = 0; u < kRun; u++) {
+          const char* q = src[s] + min(run + u * 32 + lane, npack - 1) * 16 - m;
+          lo[u] = ld_slot(q); hi[u] = ld_slot(q + (m ? 16 : 0));
+        }
+        const bool sc = do_scale && s == local_src;
 #pragma unroll
-            for (int e = 0; e < N; e++) { const A y = sc ? scale_val<A>(x[e], scale) : x[e]; acc[e] = s == 0 ? y : red<OP, A>(acc[e], y); }
-          }
-          o[u] = Pack<T>::down(acc);
+        for (int u = 0; u < kRun; u++) {
+          A x[N]; Pack<T>::up(m ? shift_pair(lo[u], hi[u], m) : lo[u], x);
+#pragma unroll
+          for (int e = 0; e < N; e++) { const A y = sc ? scale_val<A>(x[e], scale) : x[e]; acc[u][e] = s == 0 ? y : red<OP, A>(acc[u][e], y); }
         }
       }
+#pragma unroll
+      for (int u = 0; u < kRun; u++) o[u] = Pack<T>::down(acc[u]);
     }
     for (int d = 0; d < ndst; d++) {
       if (d != local_dst || dm == 0) {
@@ -327,7 +319,7 @@ template <typename T, int OP>
 __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
                                                  long long first, long long nelem, bool do_scale, float scale) {
   typedef typename AccOf<T>::type A;
-  for (long long i = first + threadIdx.x; i < nelem; i += blockDim.x) {
+  for (long long i = first + threadIdx.x; i < nelem; i += data_threads()) {
     A acc = A();
     for (int s = 0; s < nsrc; s++) {
       const T* p = reinterpret_cast<const T*>(src[s]) + i;
@@ -342,43 +334,49 @@ __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, 
 }
 
 // ---------------------------------------------------------------- the kernel
-constexpr int kSliceCache = 192;      // actions whose CTA slice is precomputed in shared memory (the low-latency executor: the actions themselves)
+constexpr int kSliceCache = 192;      // actions kept in shared memory, with the CTA's slice of each
 
-// DEFER = true (PICCL_EXEC_DEFER=1) postpones the counter updates that end an action: a release store to another GPU waits
-// for the action's data to be acknowledged (a round trip through the switch), and a chain of independent actions, such as the
-// n-1 sends that open a DIRECT all-reduce, pays that once per action.  The deferred variant only bumps its private counters
-// and publishes all of them together, with the fences of the owning threads running side by side, at the first point
-// where the CTA is about to block (one probe of the flags it needs; somebody may be waiting for what was held back) and at
-// the end of the kernel.  Nothing is ever held back across a wait, so progress is as in the plain variant.
+constexpr int kStepDepth = 4;         // steps the waiter may be ahead of the publisher
+struct StepDesc {
+  const char* src[kMaxActionPeers + 1];      // operands in rank order: receive peers below me, my own buffer, receive peers above me
+  char* dst[kMaxActionPeers + 1];            // local destination first, then the send peers
+  long long len;                             // elements
+  int action, nsrc, ndst, local_src, local_dst, flags;
+};
+enum : int { STEP_SCALE = 1, STEP_ALIGNED = 2, STEP_LOCAL_DEP = 4, STEP_FAIL = 8, STEP_END = 16 };
+__device__ __forceinline__ void bar_sync_n(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive_n(int id, int n) { __threadfence_block(); asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
 // SHIFT = true: for calls with operands that are not 16-byte aligned (a kernel of its own: the mere presence of that path cost the aligned one
 // 15 % in registers).
-template <typename T, int OP, bool DEFER, bool SHIFT = false>
-__global__ void __launch_bounds__(kMaxBlock, 1) exec_kernel(const KernelArgs ka) {
+template <typename T, int OP, bool SHIFT>
+__global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const KernelArgs ka) {
   const int vr = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta;
   const LaunchRank& L = ka.r[vr];
   RankCtx* __restrict__ ctx = L.ctx;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, ndata = data_threads();
   constexpr int esz = (int)sizeof(T);
 
-  __shared__ int s_send_slot[kMaxRanks], s_recv_slot[kMaxRanks];
+  __shared__ StepDesc s_step[kStepDepth];
   __shared__ char* s_heap[kMaxRanks];
   __shared__ long long s_lo[kSliceCache], s_hi[kSliceCache];
-  __shared__ int s_fail, s_maxseg;
+  __shared__ Action s_act[kSliceCache];
+  __shared__ int s_maxseg;
+  __shared__ volatile int s_published;             // steps whose descriptor may be used again
 
   // everything read from the context more than once is fetched once, in parallel
-  const int rank = ctx->rank, nranks = ctx->nranks, max_cta = ctx->max_cta, nslot = ctx->nslot;
-  const long long slot_bytes = ctx->slot_bytes, tail_off = ctx->tail_off, head_off = ctx->head_off, fifo_off = ctx->fifo_off, scratch_off = ctx->scratch_off;
-  // thread p (< nranks) owns the two counters of the connections with peer p
-  unsigned long long my_sent = 0, my_rcvd = 0;
-  if (tid < nranks) { s_heap[tid] = ctx->heap[tid]; my_sent = ctx->sent[tid * max_cta + cta]; my_rcvd = ctx->rcvd[tid * max_cta + cta]; }
-  if (tid == 0) { s_fail = 0; s_maxseg = 0; }
+  const int rank = ctx->rank, nranks = ctx->nranks, max_cta = ctx->max_cta;
+  const long long tail_off = ctx->tail_off, head_off = ctx->head_off, fifo_off = ctx->fifo_off, scratch_off = ctx->scratch_off, chan_bytes = ctx->nslot * ctx->slot_bytes;
+  if (tid < nranks) s_heap[tid] = ctx->heap[tid];
+  if (tid == 0) { s_maxseg = 0; s_published = 0; }
   __syncthreads();
   const long long seg_bytes = ka.seg_bytes, seg_elems = (seg_bytes / 16) * (esz >= 16 ? 1 : 16 / esz);
   {
     int m = 0;
     for (int ai = tid; ai < L.n_actions; ai += blockDim.x) {
-      const Slice sl = slice_of(L.actions[ai].count, esz, cta, ka.n_cta, seg_bytes);
-      if (ai < kSliceCache) { s_lo[ai] = sl.lo; s_hi[ai] = sl.hi; }
+      const Action a = L.actions[ai];
+      const Slice sl = slice_of(a.count, esz, cta, ka.n_cta, seg_bytes);
+      if (ai < kSliceCache) { s_lo[ai] = sl.lo; s_hi[ai] = sl.hi; s_act[ai] = a; }
       m = max(m, sl.nseg);
     }
     if (m) atomicMax(&s_maxseg, m);
@@ -386,127 +384,139 @@ __global__ void __launch_bounds__(kMaxBlock, 1) exec_kernel(const KernelArgs ka)
   __syncthreads();
   const int maxseg = s_maxseg;
   char* const my_heap = s_heap[rank];
-  WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta;
-  bool failed = false;
-  // DEFER: what peer `tid` has been told so far, and whether any update is held back (the same value in every thread)
-  unsigned long long pub_sent = my_sent, pub_rcvd = my_rcvd;
-  bool pending = false;
-  auto flush = [&]() {
-    if (tid < nranks) {
-      if (pub_sent != my_sent) { st_release_sys(reinterpret_cast<unsigned long long*>(s_heap[tid] + tail_off + (long long)(rank * max_cta + cta) * kFlagStride), my_sent); pub_sent = my_sent; }
-      if (pub_rcvd != my_rcvd) { st_release_sys(reinterpret_cast<unsigned long long*>(s_heap[tid] + head_off + (long long)(rank * max_cta + cta) * kFlagStride), my_rcvd); pub_rcvd = my_rcvd; }
-    }
-  };
+  // barriers: 1 .. kStepDepth a step's descriptor is ready (waiter arrives, data warps wait), then as many for its data being moved (data warps
+  // arrive, publisher waits), then one among the data warps
+  constexpr int kReady = 1, kDone = 1 + kStepDepth, kData = 1 + 2 * kStepDepth;
 
-  for (int seg = 0; seg < maxseg && !failed; seg++) {
-    for (int ai = 0; ai < L.n_actions; ai++) {
-      long long sl_lo, sl_hi;
-      if (ai < kSliceCache) { sl_lo = s_lo[ai]; sl_hi = s_hi[ai]; }
-      else { const Slice sl = slice_of(L.actions[ai].count, esz, cta, ka.n_cta, seg_bytes); sl_lo = sl.lo; sl_hi = sl.hi; }
-      const long long lo = sl_lo + (long long)seg * seg_elems;
-      if (lo >= sl_hi) continue;
-      const long long hi = (lo + seg_elems < sl_hi) ? lo + seg_elems : sl_hi;
-      const long long len = hi - lo;
-      const Action ac = L.actions[ai];
-
-      if (DEFER && pending) {
-        // one probe of everything this action waits for; if anything is missing, tell the peers what was held back first
-        bool block = false;
-        if (tid < nranks) {
-          for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == tid && my_sent + 1 > (unsigned long long)nslot)
-            block |= ld_acquire_sys(reinterpret_cast<const unsigned long long*>(my_heap + head_off + (long long)(tid * max_cta + cta) * kFlagStride)) < my_sent + 1 - nslot;
-          for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == tid)
-            block |= ld_acquire_sys(reinterpret_cast<const unsigned long long*>(my_heap + tail_off + (long long)(tid * max_cta + cta) * kFlagStride)) < my_rcvd + 1;
-        }
-        if (__syncthreads_or(block)) { flush(); pending = false; }
+  if (tid < ndata) {                               // ---------------- data warps
+    for (int k = 0;; k++) {
+      const int d = k % kStepDepth;
+      bar_sync_n(kReady + d, ndata + 32);
+      const StepDesc& st = s_step[d];
+      const int flags = st.flags;
+      if (!(flags & (STEP_END | STEP_FAIL))) {
+        // an operand that earlier steps wrote: its elements were written by the threads that read them now, or by their warp; the barrier makes it plain
+        if (flags & STEP_LOCAL_DEP) bar_sync_n(kData, ndata);
+        const char* const* const src = st.src; char* const* const dst = st.dst;
+        const long long len = st.len;
+        const int nsrc = st.nsrc, ndst = st.ndst, local_src = st.local_src;
+        const bool do_scale = flags & STEP_SCALE;
+        constexpr int N = Pack<T>::N;
+        const long long nfull = (SHIFT || (flags & STEP_ALIGNED)) ? len / N : 0;
+        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(nsrc, src, local_src, ndst, dst, st.local_dst, nfull, do_scale, ka.scale); }
+        else if (nfull) move_aligned<T, OP>(src, nsrc, dst, ndst, (int)nfull, do_scale ? local_src : -1, ka.scale);
+        if (nfull * N < len) reduce_copy_elem<T, OP>(nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale, ka.scale);
       }
-      // ---- wait: credit on every send connection, data on every receive connection
-      if (tid < nranks) {
-        bool ok = true;
-        w.action = ai; w.segment = seg;
-        for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == tid) {
-          s_send_slot[tid] = (int)(my_sent % (unsigned)nslot);
-          if (my_sent + 1 > (unsigned long long)nslot)
-            ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + head_off + (long long)(tid * max_cta + cta) * kFlagStride),
-                              my_sent + 1 - nslot, w, 1, tid);
-        }
-        for (int j = 0; j < ac.n_recv && ok; j++) if (ac.recv_peer[j] == tid) {
-          s_recv_slot[tid] = (int)(my_rcvd % (unsigned)nslot);
-          ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + tail_off + (long long)(tid * max_cta + cta) * kFlagStride),
-                            my_rcvd + 1, w, 2, tid);
-        }
-        if (!ok) s_fail = 1;
-      }
-      __syncthreads();
-      if (s_fail) { failed = true; break; }
-
-      // ---- operands, in rank order: receive peers below me, my own buffer, receive peers above me
-      const char* src[kMaxActionPeers + 1]; char* dst[kMaxActionPeers + 1];
-      int nsrc = 0, ndst = 0, local_src = -1;
-      bool aligned = true;
-      const bool has_src = ac.src_buf != BUF_NONE;
-#pragma unroll
-      for (int j = 0; j <= kMaxActionPeers; j++) {
-        if (j <= ac.n_recv) {
-          if (j == ac.self_pos && has_src) {
-            const char* base = ac.src_buf == BUF_IN ? (const char*)L.in : ac.src_buf == BUF_OUT ? (const char*)L.out : my_heap + scratch_off;
-            src[nsrc] = base + (ac.src_off + lo) * esz;
-            aligned &= ((reinterpret_cast<uintptr_t>(src[nsrc]) & 15) == 0);
-            local_src = nsrc++;
-          }
-          if (j < ac.n_recv) {
-            const int p = ac.recv_peer[j];
-            src[nsrc++] = my_heap + fifo_off + ((long long)(p * max_cta + cta) * nslot + s_recv_slot[p]) * slot_bytes;
-          }
-        }
-      }
-      if (ac.dst_buf != BUF_NONE) {
-        char* base = ac.dst_buf == BUF_OUT ? (char*)L.out : my_heap + scratch_off;
-        dst[ndst] = base + (ac.dst_off + lo) * esz;
-        aligned &= ((reinterpret_cast<uintptr_t>(dst[ndst]) & 15) == 0);
-        ndst++;
-      }
-#pragma unroll
-      for (int j = 0; j < kMaxActionPeers; j++) {
-        if (j < ac.n_send) {
-          const int p = ac.send_peer[j];
-          dst[ndst++] = s_heap[p] + fifo_off + ((long long)(rank * max_cta + cta) * nslot + s_send_slot[p]) * slot_bytes;
-        }
-      }
-      const bool do_scale = ka.avg && (ac.flags & ACT_SCALE_SRC) && local_src >= 0;
-
-      // ---- one pass over the segment
-      constexpr int N = Pack<T>::N;
-      const long long nfull = (aligned || SHIFT) ? len / N : 0;
-      if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(nsrc, src, local_src, ndst, dst, ac.dst_buf != BUF_NONE ? 0 : -1, nfull, do_scale, ka.scale); }
-      else if (nfull) reduce_copy_dispatch<T, OP>(nsrc, src, local_src, ndst, dst, nfull, do_scale, ka.scale);
-      if (nfull * N < len) reduce_copy_elem<T, OP>(nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale, ka.scale);
-      __syncthreads();
-
-      // ---- publish: the data to the consumers, the freed slot to the producers
-      if (DEFER) {
-        if (tid < nranks) {
-          for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == tid) my_sent++;
-          for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == tid) my_rcvd++;
-        }
-        pending = true;
-      } else if (tid < nranks) {
-        // the slots are read (their packs went through registers before the barrier), so a plain store frees them: a release would wait
-        // for the acknowledgement of everything the CTA stored
-        for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == tid) {
-          my_rcvd++;
-          *reinterpret_cast<volatile unsigned long long*>(s_heap[tid] + head_off + (long long)(rank * max_cta + cta) * kFlagStride) = my_rcvd;
-        }
-        for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == tid) {
-          my_sent++;
-          st_release_sys(reinterpret_cast<unsigned long long*>(s_heap[tid] + tail_off + (long long)(rank * max_cta + cta) * kFlagStride), my_sent);
-        }
-      }
+      bar_arrive_n(kDone + d, ndata + 32);
+      if (flags & (STEP_END | STEP_FAIL)) return;
     }
   }
-  if (DEFER && pending && !failed) flush();
-  if (tid < nranks) { ctx->sent[tid * max_cta + cta] = my_sent; ctx->rcvd[tid * max_cta + cta] = my_rcvd; }
-}
 
+  // waiter and publisher: lane l has the connections with peers l and l + 32, and counts their entries on its own
+  unsigned long long sent[2] = {0, 0}, rcvd[2] = {0, 0};
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int p = lane + 32 * q;
+    if (p < nranks) { sent[q] = ctx->sent[p * max_cta + cta]; rcvd[q] = ctx->rcvd[p * max_cta + cta]; }
+  }
+  const unsigned nslot = (unsigned)ka.nslot;
+  const long long mine = (long long)(rank * max_cta + cta) * kFlagStride;      // my counters in a peer's heap
+
+  if (tid < ndata + 32) {                          // ---------------- waiter
+    WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta;
+    unsigned long long seen_head[2] = {0, 0};      // what a peer had consumed when last looked: no need to look again while that is credit enough
+    int k = 0;
+    bool failed = false;
+    // the descriptor of step k - kStepDepth has served; the publisher waits for nobody but the data warps, which wait for nothing beyond this warp
+    auto free_desc = [&]() {
+      unsigned long long t0 = 0;
+      for (unsigned spins = 1; s_published < k - kStepDepth + 1; spins++) {
+        if ((spins & 1023u) == 0) {
+          const unsigned long long now = globaltimer_ns();
+          if (t0 == 0) t0 = now;
+          else if (now - t0 > ka.timeout_ns) { *(volatile int*)ctx->abort_flag = 1; return; }
+        }
+      }
+      __threadfence_block();
+    };
+    for (int seg0 = 0; seg0 < maxseg && !failed; seg0 += ka.window) {
+      for (int ai = 0; ai < L.n_actions && !failed; ai++) {
+        const Action& ac = ai < kSliceCache ? s_act[ai] : L.actions[ai];
+        long long sl_lo, sl_hi;
+        if (ai < kSliceCache) { sl_lo = s_lo[ai]; sl_hi = s_hi[ai]; }
+        else { const Slice sl = slice_of(ac.count, esz, cta, ka.n_cta, seg_bytes); sl_lo = sl.lo; sl_hi = sl.hi; }
+        const bool has_src = ac.src_buf != BUF_NONE, has_dst = ac.dst_buf != BUF_NONE;
+        for (int seg = seg0; seg < seg0 + ka.window; seg++) {
+          const long long lo = sl_lo + (long long)seg * seg_elems;
+          if (lo >= sl_hi) break;
+          free_desc();
+          StepDesc& st = s_step[k % kStepDepth];
+          bool ok = true;
+          w.action = ai; w.segment = seg;
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            const int p = lane + 32 * q;
+            const long long theirs = (long long)(p * max_cta + cta) * kFlagStride;      // peer p's counters in my heap
+            for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) {
+              st.dst[j + has_dst] = s_heap[p] + fifo_off + (long long)(rank * max_cta + cta) * chan_bytes + (long long)(sent[q] % nslot) * seg_bytes;
+              if (++sent[q] > seen_head[q] + nslot && ok)
+                ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + head_off + theirs), sent[q] - nslot, w, 1, p, &seen_head[q]);
+            }
+            for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) {
+              st.src[j + (has_src && j >= ac.self_pos)] = my_heap + fifo_off + (long long)(p * max_cta + cta) * chan_bytes + (long long)(rcvd[q] % nslot) * seg_bytes;
+              ++rcvd[q];
+              if (ok) ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + tail_off + theirs), rcvd[q], w, 2, p);
+            }
+          }
+          ok = __all_sync(0xffffffffu, ok);
+          if (lane == 0) {
+            const char* lsrc = nullptr; char* ldst = nullptr;
+            if (has_src) { lsrc = (ac.src_buf == BUF_IN ? (const char*)L.in : ac.src_buf == BUF_OUT ? (const char*)L.out : my_heap + scratch_off) + (ac.src_off + lo) * esz; st.src[ac.self_pos] = lsrc; }
+            if (has_dst) { ldst = (ac.dst_buf == BUF_OUT ? (char*)L.out : my_heap + scratch_off) + (ac.dst_off + lo) * esz; st.dst[0] = ldst; }
+            st.len = (lo + seg_elems < sl_hi ? lo + seg_elems : sl_hi) - lo;
+            st.action = ai; st.nsrc = ac.n_recv + has_src; st.ndst = ac.n_send + has_dst; st.local_src = has_src ? ac.self_pos : -1; st.local_dst = has_dst ? 0 : -1;
+            st.flags = (ka.avg && (ac.flags & ACT_SCALE_SRC) && has_src ? STEP_SCALE : 0) | (((reinterpret_cast<uintptr_t>(lsrc) | reinterpret_cast<uintptr_t>(ldst)) & 15) == 0 ? STEP_ALIGNED : 0) |
+                       (has_src && ac.src_buf != BUF_IN ? STEP_LOCAL_DEP : 0) | (ok ? 0 : STEP_FAIL);
+          }
+          __syncwarp();
+          bar_arrive_n(kReady + k % kStepDepth, ndata + 32);
+          k++;
+          if (!ok) { failed = true; break; }
+        }
+        if (failed) break;
+      }
+    }
+    if (!failed) {
+      free_desc();
+      if (lane == 0) s_step[k % kStepDepth].flags = STEP_END;
+      __syncwarp();
+      bar_arrive_n(kReady + k % kStepDepth, ndata + 32);
+    }
+    return;
+  }
+
+  for (int k = 0;; k++) {                          // ---------------- publisher: the data to the consumers, the freed slots to the producers
+    const int d = k % kStepDepth;
+    bar_sync_n(kDone + d, ndata + 32);
+    const int flags = s_step[d].flags, ai = s_step[d].action;
+    if (flags & (STEP_END | STEP_FAIL)) break;
+    const Action& ac = ai < kSliceCache ? s_act[ai] : L.actions[ai];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int p = lane + 32 * q;
+      // the slots are read (their packs went through registers before the barrier), so a plain store frees them: a release would wait for the
+      // acknowledgement of everything the CTA stored
+      for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) *reinterpret_cast<volatile unsigned long long*>(s_heap[p] + head_off + mine) = ++rcvd[q];
+      for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) st_release_sys(reinterpret_cast<unsigned long long*>(s_heap[p] + tail_off + mine), ++sent[q]);
+    }
+    __syncwarp();
+    if (lane == 0) { __threadfence_block(); s_published = k + 1; }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int p = lane + 32 * q;
+    if (p < nranks) { ctx->sent[p * max_cta + cta] = sent[q]; ctx->rcvd[p * max_cta + cta] = rcvd[q]; }
+  }
+}
 
 }  // namespace piccl

@@ -375,7 +375,9 @@ static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
   if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) bytes /= std::max(1, a.nranks);
   if (a.algo == ALGO_DIRECT && a.coll != COLL_ALLGATHER && a.coll != COLL_REDUCE_SCATTER) bytes /= std::max(1, a.coll == COLL_ALLREDUCE ? a.nranks : a.nranks - 1);
   const Env& e = env();
-  long long n = (bytes + 32767) / 32768;
+  // (virtual ranks on one device, whose steps cost less than a way over NVLink: 280 KB among eight ranks 42 us at 32 KiB a CTA, 35 at 16)
+  const long long per = n_vrank > 1 ? 16384 : 32768;
+  long long n = (bytes + per - 1) / per;
   if (e.min_grid_set || e.max_grid_set) {
     long long g = a.count / std::max(1, c->cfg.block_size);
     n = std::max<long long>(e.min_grid_set ? e.min_grid : 1, std::min<long long>(e.max_grid_set ? e.max_grid : g, g));
@@ -383,6 +385,27 @@ static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
   n = std::max<long long>(1, std::min<long long>(n, c->cfg.max_cta));
   if (n_vrank > 1) n = std::min<long long>(n, std::max(1, c->sm_count / n_vrank));
   return (int)n;
+}
+
+// threads of an executor CTA: the configured block moves data, two more warps wait and publish
+static int exec_block(const piccl_comm* c) { return c->cfg.block_size + kCtlThreads; }
+
+// Segments of the executor.  Two are walked together where there are slots for it (the protocol needs two slots per segment of a window): the way from a
+// peer's stores to my loads then hides behind the other one.  One launch for all ranks: segments of at most 128 KiB, a quarter of the default
+// slot, so that what is on its way between ranks stays in L2 (512 KiB slots of 144 CTAs are 300 MB).  Measured with 512 threads, 8 x 64 MiB all-reduce on the
+// ring: 408 us with 128 KiB, 463 with 64 or 256 KiB, 446 with the slots as they are; at least 32 KiB, a round of four packs a thread, and
+// a message is cut into two where it can be.  Ranks in launches of their own keep the communicator's slots: they may be a call apart.
+static void cut_fifo(const piccl_comm* c, int n_vrank, int n_cta, const CollArgs& a, KernelArgs* ka) {
+  const RankCtx& x = c->h_ctx;
+  ka->seg_bytes = x.slot_bytes; ka->nslot = x.nslot; ka->window = x.nslot >= 4 ? 2 : 1;
+  if (n_vrank != c->nranks || n_vrank < 2) return;
+  const long long chan = x.nslot * x.slot_bytes, round = (long long)c->cfg.block_size * 64;
+  long long slice = a.count * a.elem_size;
+  if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) slice /= c->nranks;
+  slice = (slice + n_cta - 1) / n_cta;
+  const long long seg = std::min<long long>(round_up((slice + 1) / 2, round), std::max<long long>(round, 131072 / round * round));
+  ka->nslot = 4; ka->window = 2;
+  ka->seg_bytes = std::max<long long>(16, std::min<long long>(seg, chan / 4 / 16 * 16));
 }
 
 static bool fault_now(piccl_comm* c) {
@@ -465,10 +488,8 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
   const long long count = reducing ? (long long)d0.count : (long long)d0.count * esz_real;
   // small messages of every collective run the low-latency variant of the executor (flags inside the data lines)
   const bool use_llf = c0->llf_max_bytes > 0 && (long long)d0.count * esz_real <= c0->llf_max_bytes;
-  const bool defer = env().exec_defer != 0;
   ExecKernelFn fn = use_llf ? (reducing ? exec_ll_kernel_for(d0.dtype, op) : exec_ll_copy_kernel())
-                   : defer ? (reducing ? exec_defer_kernel_for(d0.dtype, op) : exec_defer_copy_kernel())
-                           : (reducing ? exec_kernel_for(d0.dtype, op) : exec_copy_kernel());
+                   : (reducing ? exec_kernel_for(d0.dtype, op) : exec_copy_kernel());
   if (!fn) return fail(PICCL_INTERNAL_ERROR, "no kernel for dtype %d op %d", d0.dtype, op);
 
   // small exchange-type all-reduces take the low-latency kernel (flags travel inside the data lines)
@@ -630,7 +651,8 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
           n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
           if (n > 1) n_cta = std::min(n_cta, std::max(1, c->sm_count / n));
         }
-        ka.n_cta = n_cta; ka.seg_bytes = c->h_ctx.slot_bytes; ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
+        ka.n_cta = n_cta; if (!use_llf) cut_fifo(c, n, n_cta, a, &ka);
+        ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
       }
       ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
       aligned &= pe->offsets_aligned && ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(r)) & 15) == 0;
@@ -644,9 +666,9 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     TraceRec* tr = trace_begin(c0, d0.coll, d0.algo, d0.k, cur * esz, n_cta, stream);
     void* args[] = {&ka};
     cudaError_t e;
-    const int block = use_llf ? kLLBlock : c0->cfg.block_size;
+    const int block = use_llf ? kLLBlock : exec_block(c0);
     // which kernel a rank runs is its own business: both speak the same protocol
-    const ExecKernelFn f = (aligned || use_llf || defer) ? fn : reducing ? exec_shift_kernel_for(d0.dtype, op) : exec_shift_copy_kernel();
+    const ExecKernelFn f = (aligned || use_llf) ? fn : reducing ? exec_shift_kernel_for(d0.dtype, op) : exec_shift_copy_kernel();
     if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n * n_cta), dim3(block), args, 0, stream);
     else e = cudaLaunchKernel((const void*)f, dim3(n_cta), dim3(block), args, 0, stream);
     if (e != cudaSuccess) rc = fail(PICCL_CUDA_ERROR, "executor launch failed: %s", cudaGetErrorString(e));
@@ -705,10 +727,10 @@ int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream) {
   int rc = upload_program(c, p, (cudaStream_t)stream, e); if (rc) return rc;
   c->cache.emplace(ProgKey{-1, 0, 0, 0, 1, 0, (long long)c->cache.size(), 0}, e);
   KernelArgs ka; memset(&ka, 0, sizeof ka);
-  ka.n_vrank = 1; ka.n_cta = 1; ka.elem_size = 1; ka.seg_bytes = c->h_ctx.slot_bytes; ka.scale = 1.f; ka.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
+  ka.n_vrank = 1; ka.n_cta = 1; ka.elem_size = 1; ka.seg_bytes = c->h_ctx.slot_bytes; ka.nslot = c->h_ctx.nslot; ka.window = 1; ka.scale = 1.f; ka.timeout_ns = (unsigned long long)timeout_ms * 1000000ull;
   ka.r[0].ctx = c->d_ctx; ka.r[0].actions = e.dev; ka.r[0].n_actions = 1;
   void* args[] = {&ka};
-  CUDA_TRY(cudaLaunchKernel((const void*)exec_copy_kernel(), dim3(1), dim3(c->cfg.block_size), args, 0, (cudaStream_t)stream));
+  CUDA_TRY(cudaLaunchKernel((const void*)exec_copy_kernel(), dim3(1), dim3(exec_block(c)), args, 0, (cudaStream_t)stream));
   return PICCL_OK;
 }
 

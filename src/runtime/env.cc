@@ -41,7 +41,6 @@ static void load() {
   e.llf_kb = env_int("PICCL_LLF_KB", 64);        // largest message (any collective) on the low-latency executor; 0 turns it off
   e.llx_kb = env_int("PICCL_LLX_KB", 64);        // largest block per rank of an all-gather / reduce-scatter taken by the one-exchange low-latency kernel
   e.tp_mb = env_int("PICCL_TP_MB", 0);           // heap space for the fused tensor-parallel kernels (0: none)
-  e.exec_defer = env_int("PICCL_EXEC_DEFER", 0);
   e.nvls = env_int("PICCL_NVLS", 1);            // 0: no NVLink multicast window (algorithm NVLS then runs the peer-to-peer schedules)
   e.nvls_chunk_kb = env_int("PICCL_NVLS_CHUNK_KB", 256);   // largest chunk = one part of a CTA's slot
   e.nvls_depth = env_int("PICCL_NVLS_DEPTH", 5);           // parts per slot (2 .. 8): chunks a CTA has in flight in its stages

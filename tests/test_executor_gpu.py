@@ -361,3 +361,29 @@ def test_operands_at_any_address(groups, coll, algo, dtype, offset):
             want = total.to(dtype)
         assert torch.equal(outs[r], want), f"rank {r}"
         assert torch.all(bufs[r][:16 + offset] == 77) and torch.all(bufs[r][16 + offset + n_out:] == 77), f"rank {r} wrote outside its buffer"
+
+
+@pytest.mark.parametrize("n,algo,k", [(2, "RING", 0), (3, "PRM", 3), (4, "PRD", 2), (4, "PRM", 4), (6, "PRM", 6), (7, "DIRECT", 0), (8, "PRM", 8), (8, "K_RING", 4), (8, "PRM", 2)])
+def test_rounds_segments_and_windows(n, algo, k):
+    """Default geometry (512 threads that move data, 128 KiB segments, two to a window): lengths around a round of four 16-byte packs per thread, around a segment, an odd
+    number of segments, and a partial pack; two to eight operands per step.  Whole numbers: exact."""
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    ctas = min(64, 148 // n)
+    g = LoopbackGroup(n, config=make_config(scratch_bytes=1 << 20, timeout_ms=5000))
+    parts = n if algo == "K_RING" or algo == "RING" or algo == "DIRECT" else 1
+    for per_cta in (8192, 8192 - 4, 8192 + 4, 3 * 32768 + 1):        # int32 elements of a CTA's slice
+        count = per_cta * ctas * parts - 3
+        xs = [torch.randint(-1000, 1001, (count,), generator=torch.Generator(device="cuda").manual_seed(r), dtype=torch.int32, device="cuda") for r in range(n)]
+        outs = [torch.empty_like(x) for x in xs]
+        want = torch.stack(xs).sum(0, dtype=torch.int32)
+        for rep in range(2):
+            g.run("allreduce", xs, outs, count, op="sum", algo=algo, k=k)
+        _check_ok(g)
+        for o in outs:
+            assert torch.equal(o, want), (n, algo, per_cta)
+        g.run("allreduce", xs, xs, count, op="max", algo=algo, k=k)      # in place
+        ref = xs[0].clone()
+        _check_ok(g)
+        for x in xs[1:]:
+            assert torch.equal(x, ref)
+    g.close()
