@@ -108,7 +108,9 @@ def model_lib() -> C.CDLL:
             vp, i, ll = C.c_void_p, C.c_int, C.c_longlong
             l.piccl_gpt2_create.argtypes, l.piccl_gpt2_create.restype = [vp], vp
             l.piccl_gpt2_destroy.argtypes = [vp]
-            l.piccl_gpt2_run.argtypes = [vp, vp, vp, i, i, vp, i, i, vp, C.POINTER(ll)]
+            l.piccl_gpt2_run.argtypes = [vp, vp, vp, i, i, vp, i, i, i, vp, C.POINTER(ll)]
+            l.piccl_gpt2_arena.argtypes, l.piccl_gpt2_arena.restype = [vp], vp
+            l.piccl_gpt2_capture_stream.argtypes, l.piccl_gpt2_capture_stream.restype = [vp], vp
             l.piccl_gpt2_error.restype = C.c_char_p
             _libs["model"] = l
         return _libs["model"]

@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 import weakref
 from dataclasses import dataclass
 from typing import Callable, Optional
@@ -32,6 +33,7 @@ from .. import ops
 from ..ops import gemm
 
 _READY = C.CFUNCTYPE(None, C.c_longlong)
+_MAX_GRAPHS = 8
 
 
 class _Desc(C.Structure):       # the native step's description of a model (src/model/gpt2_step.cc)
@@ -106,6 +108,10 @@ class GPT2:
         self._run_ends = torch.tensor([e // 8 for _, e, _ in self.groups], dtype=torch.int32, device=self.device)
         self._ticket = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._handle = None
+        self._arena = None
+        self._graphs: dict = {}      # captured steps, at most _MAX_GRAPHS, which share the memory of their attention outputs
+        self._graph_pool = None
+        self._seen: dict = {}        # how often a step was issued call by call; -1: it cannot be captured
         self._counts = (C.c_longlong * 4)()
 
     # ------------------------------------------------------------------ setup
@@ -140,15 +146,83 @@ class GPT2:
                          on_grads_ready: Optional[Callable[[int], None]] = None, loss_only: bool = False) -> torch.Tensor:
         """One training micro-step: returns the mean loss (fp32, on device) and leaves the
         gradients in `flat_g`.  `on_grads_ready(end)` is called whenever flat_g[:end] is final."""
+        loss, shared = self._step(idx, targets, on_grads_ready, loss_only)
+        return loss.clone() if shared else loss
+
+    def _step(self, idx, targets, on_grads_ready=None, loss_only=False):
+        """(loss, whether the tensor is overwritten by the next step)
+
+        A step that comes a third time with the same shape on the same input buffers (a trainer's, which it fills anew for each batch) is captured
+        into a CUDA graph and replayed from then on: issued call by call, the launches bound every model of a few hundred columns, and a replay
+        also runs the weight gradients on a second stream.  While a capture is open another thread's device-wide synchronisation would fail: there is none
+        in a program of several threads.  Inputs elsewhere, a step that reports finished gradients, and one inside somebody else's capture run as before."""
         B, S = idx.shape
         idx = idx.reshape(-1).contiguous()
         targets = targets.reshape(-1).contiguous()
         if idx.dtype != torch.int64 or targets.dtype != torch.int64 or targets.numel() != B * S or S > self.cfg.seq_len:
             raise ValueError("token ids and targets are int64 tensors of one shape, at most seq_len long")
+        if on_grads_ready is not None and not loss_only:
+            return self._issue(idx, targets, B, S, loss_only, 0, on_grads_ready), False
+        key = (idx.data_ptr(), targets.data_ptr(), B, S, loss_only, gemm.backend_code())
+        seen = self._seen.get(key, 0)
+        if seen == -1 or torch.cuda.is_current_stream_capturing():
+            return self._issue(idx, targets, B, S, loss_only, 0), False
+        arena = N.model_lib().piccl_gpt2_arena(self._native())
+        if arena != self._arena:                 # a larger shape moved the activations: what was captured before points to the old ones
+            self._arena = arena
+            self._graphs.clear()
+        entry = self._graphs.get(key)
+        if entry is None and seen >= 2 and len(self._graphs) < _MAX_GRAPHS and threading.active_count() == 1:
+            entry = self._capture(idx, targets, B, S, loss_only)
+            if entry is not None:
+                self._graphs[key] = entry
+            else:
+                self._seen[key] = -1             # a part of this step cannot be captured: issued call by call from now on
+        elif entry is None:
+            if len(self._seen) > 4096:
+                self._seen.clear()
+            self._seen[key] = min(seen + 1, 2)
+        if entry is None:                        # the call before the capture runs what will be captured: libraries set themselves up for it
+            return self._issue(idx, targets, B, S, loss_only, int(seen == 1)), False
+        graph, loss, counts = entry
+        graph.replay()
+        ops._bump(counts[0])
+        gemm.count(counts[1], counts[2])
+        return loss, True
+
+    def _capture(self, idx, targets, B, S, loss_only):
+        if not self._graphs:                     # a pool that no graph uses any more cannot be taken up again
+            self._graph_pool = torch.cuda.graph_pool_handle()
+        graph, cur = torch.cuda.CUDAGraph(), torch.cuda.current_stream()
+        stream = torch.cuda.ExternalStream(N.model_lib().piccl_gpt2_capture_stream(self._native()), device=self.device)
+        launched, products = ops.launch_count(), gemm.counts()
+        stream.wait_stream(cur)
+        ok = False
+        with torch.cuda.stream(stream):
+            graph.capture_begin(pool=self._graph_pool, capture_error_mode="thread_local")
+            try:
+                loss = self._issue(idx, targets, B, S, loss_only, 1)
+                ok = True
+            except RuntimeError:
+                pass
+            try:
+                graph.capture_end()
+            except RuntimeError:
+                ok = False
+        cur.wait_stream(stream)
+        after = gemm.counts()
+        counts = (ops.launch_count() - launched, after["tcgen05"] - products["tcgen05"], after["cublas"] - products["cublas"])
+        ops._bump(-counts[0])                    # the capture itself ran nothing
+        gemm.count(-counts[1], -counts[2])
+        if not ok or N.model_lib().piccl_gpt2_arena(self._native()) != self._arena:
+            return None
+        return graph, loss, counts
+
+    def _issue(self, idx, targets, B, S, loss_only, captured, on_grads_ready=None) -> torch.Tensor:
         loss = torch.empty((), dtype=torch.float32, device=self.device)
         raised: list = []
         cb = None
-        if on_grads_ready is not None and not loss_only:
+        if on_grads_ready is not None:
             def ready(end):
                 try:
                     if not raised:
@@ -156,7 +230,7 @@ class GPT2:
                 except BaseException as e:      # an exception may not unwind through the native frames: raised again below
                     raised.append(e)
             cb = _READY(ready)
-        rc = N.model_lib().piccl_gpt2_run(self._native(), idx.data_ptr(), targets.data_ptr(), B, S, loss.data_ptr(), int(not loss_only), gemm.backend_code(),
+        rc = N.model_lib().piccl_gpt2_run(self._native(), idx.data_ptr(), targets.data_ptr(), B, S, loss.data_ptr(), int(not loss_only), gemm.backend_code(), captured,
                                           C.cast(cb, C.c_void_p) if cb is not None else None, self._counts)
         ops._bump(self._counts[0])
         gemm.count(self._counts[1], self._counts[2])

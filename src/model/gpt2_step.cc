@@ -4,16 +4,24 @@
 // 256 columns took 1.4 ms for 0.3 ms of kernels, eight layers of 768 columns 4.5 ms for 2.7 ms.  Here a launch of this framework's
 // own kernels is a plain call (2 to 3 us); attention goes through ATen's fused kernels without autograd.
 //
+// A step of the same shape on the same input buffers is captured into a CUDA graph by the caller (models/gpt2.py).  Its weight gradients and
+// column sums, which nothing in the backward pass waits for, can then go to a second stream: small ones fill the SMs that the chain of
+// input gradients leaves idle, and in a graph the events between the streams cost no host time.
+//
 // The gradient buffer is laid out in the order in which the backward pass finishes it; `ready(end)` tells the caller that elements
 // [0, end) are final, which is where bucketed all-reduces start (the overlap that the reference gets from torch DDP).
 // Bias, gamma and beta gradients are column sums of tensors that some kernel holds in registers: each leaves partial rows in fp32,
 // one launch per layer folds the partial rows of all eight vectors.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime.h>
 #include <c10/core/GradMode.h>
 #include <torch/csrc/autograd/autograd.h>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 #include "../ops/piccl_ops.h"
@@ -40,16 +48,47 @@ struct Saved { at::Tensor q, k, v, out, lse, cq, ck, seed, offset; c10::SymInt m
 
 constexpr size_t kSplitBytes = (size_t)40 << 20;
 
+// The streams that steps are captured on.  They are nobody else's, unlike those of PyTorch's pool: cuBLAS's workspace, which belongs to a
+// stream, is written by every replay.  Streams of a model that is gone serve the next one, and so does that workspace.
+struct Streams { cudaStream_t main = nullptr, side = nullptr; int device = -1; };
+std::mutex g_streams_mutex;
+std::vector<Streams> g_streams;
+
+bool take_streams(Streams& st) {
+  const int device = at::cuda::current_device();
+  std::lock_guard<std::mutex> lock(g_streams_mutex);
+  for (auto it = g_streams.begin(); it != g_streams.end(); ++it)
+    if (it->device == device) { st = *it; g_streams.erase(it); return true; }
+  int low, high;
+  if (cudaDeviceGetStreamPriorityRange(&low, &high) != cudaSuccess || cudaStreamCreateWithPriority(&st.main, cudaStreamNonBlocking, std::max(high, low - 1)) != cudaSuccess) return false;
+  if (cudaStreamCreateWithPriority(&st.side, cudaStreamNonBlocking, low) != cudaSuccess) { cudaStreamDestroy(st.main); st.main = nullptr; return false; }
+  st.device = device;
+  return true;
+}
+void give_back(const Streams& st) {
+  std::lock_guard<std::mutex> lock(g_streams_mutex);
+  g_streams.push_back(st);
+}
+
+
 struct Model {
   Desc d;
   std::vector<long long> off;
   at::Tensor arena;         // activations and workspace, grown to the largest shape so far
   at::Tensor stage, owner;  // fp32 table of embedding gradients (all zero between calls), one row of the batch per token id
   at::Tensor split;         // workspace of the products that split K
-  void* ws = nullptr;
+  void* ws[2] = {nullptr, nullptr};      // of the main and the second stream
+  Streams streams;
+  cudaEvent_t ev_fork = nullptr, ev_layer[2] = {nullptr, nullptr};
   std::vector<Saved> saved;
   long long launches = 0, cublas = 0, tcgen05 = 0;
+  bool captured = false;
   int backend = 0;          // 0: by size, 1: this framework's GEMM, 2: cuBLAS
+
+  ~Model() {
+    for (cudaEvent_t e : {ev_fork, ev_layer[0], ev_layer[1]}) if (e) cudaEventDestroy(e);
+    if (streams.side) give_back(streams);
+  }
 
   b16* p(int l, int which) const { return d.p + off[4 + l * PER_LAYER + which]; }
   b16* g(int l, int which) const { return d.g + off[4 + l * PER_LAYER + which]; }
@@ -74,8 +113,9 @@ struct Carve {
 
 struct Layer { b16 *ln1, *qkv, *x2, *ln2, *h, *gl, *x3; float *mean1, *rstd1, *mean2, *rstd2; };
 struct Buffers {
-  b16 *x0, *a, *pr, *logits, *dln, *dxa, *dxb, *dg, *dln2, *datt, *dqkv, *dln1;
-  float *loss_rows, *parts;
+  b16 *x0, *a, *pr, *logits, *dln, *dln2, *datt, *dln1;
+  b16 *dxa[3], *dxb[2], *dg[2], *dqkv[2];      // taken in turn by the layers: weight gradients may still read those of the layer above
+  float *loss_rows, *parts[2];
   std::vector<Layer> layer;         // L + 1: the last one holds the input of the head
 };
 
@@ -93,8 +133,9 @@ void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, Bu
   }
   b.logits = c.get<b16>(T * d.Vp); b.loss_rows = c.get<float>(T);
   if (!train) return;
-  b.dln = c.get<b16>(T * C); b.dxa = c.get<b16>(T * C); b.dxb = c.get<b16>(T * C); b.dg = c.get<b16>(T * 4 * C); b.dln2 = c.get<b16>(T * C);
-  b.datt = c.get<b16>(T * C); b.dqkv = c.get<b16>(T * 3 * C); b.dln1 = c.get<b16>(T * C); b.parts = c.get<float>(part_floats);
+  for (b16*& x : b.dxa) x = c.get<b16>(T * C);
+  for (int q = 0; q < 2; q++) { b.dxb[q] = c.get<b16>(T * C); b.dg[q] = c.get<b16>(T * 4 * C); b.dqkv[q] = c.get<b16>(T * 3 * C); }
+  b.dln = c.get<b16>(T * C); b.dln2 = c.get<b16>(T * C); b.datt = c.get<b16>(T * C); b.dln1 = c.get<b16>(T * C); for (float*& x : b.parts) x = c.get<float>(part_floats);
 }
 
 at::Tensor view(b16* p, at::IntArrayRef sizes, at::IntArrayRef strides = {}) {
@@ -105,20 +146,21 @@ at::Tensor view(b16* p, at::IntArrayRef sizes, at::IntArrayRef strides = {}) {
 }
 
 // C[M, N] = A op B, bf16 row-major: layout NT A [M,K] B [N,K], NN A [M,K] B [K,N], TN A [K,M] B [K,N]
-// Plain products of more than 2 GFLOP go to cuBLAS unless the "tcgen05" backend is asked for: it has more tile shapes to fit ragged sizes
+// Plain products of more than some GFLOP go to cuBLAS unless the "tcgen05" backend is asked for: it has more tile shapes to fit ragged sizes
 // to the chip, and under the power cap it draws less for the same tile (GPT-2 medium step 23.5 ms with it, 24.7 without; 8 layers of
-// 768 columns on 3 x 777 tokens 2.97 / 3.10 ms).  Below, the launch counts: this framework's kernel costs a third of the host time and
-// overlaps its set-up with the kernel before it (2 layers of 256 columns 342 us, 500 with cuBLAS).
-constexpr double kOwnProductFlops = 2e9;
-int product(Model& m, int layout, b16* A, b16* B, b16* C, const b16* bias, int M, int N, int K, void* s) {
-  if (m.backend == 2 || (m.backend == 0 && 2.0 * M * N * K > kOwnProductFlops)) {
+// 768 columns on 3 x 777 tokens 2.97 / 3.10 ms).  Below, the launch counts: issued call by call this framework's kernel costs a third of
+// the host time (2 layers of 256 columns 342 us, 500 with cuBLAS); replayed from a graph it does not, and the line lies lower (the same
+// step 236 us at 2 GFLOP, 217 at 0.1; 12 layers of 512 columns on 4 x 512 tokens 1985 us, 1857).
+constexpr double kOwnProductFlops = 2e9, kOwnProductFlopsReplayed = 1e8;
+int product(Model& m, int layout, b16* A, b16* B, b16* C, const b16* bias, int M, int N, int K, void* s, int which_ws = 0) {
+  if (m.backend == 2 || (m.backend == 0 && 2.0 * M * N * K > (m.captured ? kOwnProductFlopsReplayed : kOwnProductFlops))) {
     at::Tensor out = view(C, {M, N});
     at::Tensor a = layout == TN ? view(A, {K, M}).t() : view(A, {M, K}), b = layout == NT ? view(B, {N, K}).t() : view(B, {K, N});
     if (bias) at::addmm_out(out, view(const_cast<b16*>(bias), {N}), a, b); else at::mm_out(out, a, b);
     m.cublas++;
     return 0;
   }
-  TRY(piccl_ops_gemm(layout, EPI_BIAS, A, B, C, nullptr, bias, nullptr, nullptr, m.ws, kSplitBytes, M, N, K, s));
+  TRY(piccl_ops_gemm(layout, EPI_BIAS, A, B, C, nullptr, bias, nullptr, nullptr, m.ws[which_ws], kSplitBytes, M, N, K, s));
   m.tcgen05++;
   return 0;
 }
@@ -157,7 +199,8 @@ void attention_grad(const Saved& sv, b16* dout, int B, int S, int H, int D, at::
 int run(Model& m, const long long* idx, const long long* tgt, int B, int S, float* loss, bool train, ReadyFn ready) {
   const Desc& d = m.d;
   const int T = B * S, C = d.C, L = d.L, H = d.H, D = C / H;
-  void* s = at::cuda::getCurrentCUDAStream().stream();
+  const cudaStream_t main_stream = at::cuda::getCurrentCUDAStream().stream();
+  void* s = main_stream;
   c10::NoGradGuard no_grad;
   const auto opt = at::TensorOptions().device(at::kCUDA, at::cuda::current_device());
 
@@ -171,7 +214,13 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   Carve c{static_cast<char*>(m.arena.data_ptr())};
   carve(c, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
   b16 *const lnf_g = d.p + m.off[0], *const lnf_b = d.p + m.off[1], *const wpe = d.p + m.off[2], *const wte = d.p + m.off[3];
-  if (!m.split.defined()) { m.split = at::empty({(int64_t)kSplitBytes}, opt.dtype(at::kByte)); m.split.narrow(0, 0, 64 << 10).zero_(); m.ws = m.split.data_ptr(); }
+  if (!m.split.defined()) {
+    m.split = at::empty({2, (int64_t)kSplitBytes}, opt.dtype(at::kByte));
+    m.split.narrow(1, 0, 64 << 10).zero_();
+    for (int q = 0; q < 2; q++) m.ws[q] = m.split.select(0, q).data_ptr();
+    if (!take_streams(m.streams)) { g_error = "cudaStreamCreate failed"; return -1001; }
+    for (cudaEvent_t* e : {&m.ev_fork, &m.ev_layer[0], &m.ev_layer[1]}) if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) { g_error = "cudaEventCreate failed"; return -1001; }
+  }
   if ((int)m.saved.size() < L) m.saved.resize(L);
 
   // ---------------- forward
@@ -207,55 +256,87 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
 
   // ---------------- backward (logits now hold d loss / d logits)
   b16 *const g_lnf_g = d.g + m.off[0], *const g_lnf_b = d.g + m.off[1], *const g_wpe = d.g + m.off[2], *const g_wte = d.g + m.off[3];
-  float *const ws2 = b.parts, *const ws1 = ws2 + 3 * row, *const ws_fc = ws1 + 3 * row, *const ws_qkv = ws_fc + fc_floats;
+  // Captured, the weight gradients and column sums of small models run beside the chain of input gradients.  Above 4 Mi elements of the
+  // residual stream a product fills the chip by itself, and a block of another kernel on one SM costs it a wave (8192 x 1024: 22.5 ms with
+  // weight gradients on the second stream, 23.3 with the column sums there as well, 22.4 with neither; 4096 x 768: 5.13 ms and 5.26).
+  const bool fork = m.captured && (long)T * C <= (4 << 20);
+  auto to_side = [&] {                // what comes next on the second stream sees all that the main one has done
+    cudaEventRecord(m.ev_fork, main_stream);
+    cudaStreamWaitEvent(m.streams.side, m.ev_fork, 0);
+  };
+  auto finish = [&](const piccl_finish_job* jobs, int n, int q) -> int {
+    if (!fork) { TRY(piccl_ops_finish_parts(jobs, n, s)); return 0; }
+    to_side();
+    TRY(piccl_ops_finish_parts(jobs, n, m.streams.side));
+    cudaEventRecord(m.ev_layer[q], m.streams.side);
+    return 0;
+  };
   auto done = [&](const b16* last_of, size_t n) { if (ready) ready((long long)(last_of - d.g) + (long long)n); };
-  DO(product(m, TN, b.logits, f.ln1, g_wte, nullptr, d.Vp, C, T, s));
+  // G[M, N] = A[T, M]^T B[T, N], on the second stream once the main one has come this far
+  auto weight_grad = [&](b16* A, b16* B, b16* G, int M, int N) -> int {
+    if (!fork) return product(m, TN, A, B, G, nullptr, M, N, T, s);
+    to_side();
+    c10::cuda::CUDAStreamGuard guard(c10::cuda::getStreamFromExternal(m.streams.side, m.streams.device));
+    return product(m, TN, A, B, G, nullptr, M, N, T, m.streams.side, 1);
+  };
+  DO(weight_grad(b.logits, f.ln1, g_wte, d.Vp, C));
   DO(product(m, NN, b.logits, wte, b.dln, nullptr, T, C, d.Vp, s));
-  TRY(piccl_ops_ln_bwd(b.dln, xin, lnf_g, f.mean1, f.rstd1, nullptr, b.dxa, ws1, 1, T, C, s));
+  b16* dx = b.dxa[L % 3];             // gradient of the residual stream above the layer at hand
   {
+    float* const ws1 = b.parts[L & 1] + 3 * row;
+    TRY(piccl_ops_ln_bwd(b.dln, xin, lnf_g, f.mean1, f.rstd1, nullptr, dx, ws1, 1, T, C, s));
     const piccl_finish_job jobs[3] = {{ws1, g_lnf_g, n_ln, C, 0, 0}, {ws1 + row, g_lnf_b, n_ln, C, 0, 0}, {ws1 + 2 * row, m.g(L - 1, B_PROJ), n_ln, C, 0, 0}};
-    TRY(piccl_ops_finish_parts(jobs, 3, s));
+    DO(finish(jobs, 3, L & 1));
   }
   done(g_lnf_b, C);
   for (int l = L - 1; l >= 0; l--) {
     Layer& y = b.layer[l];
+    const int q = l & 1;
+    b16 *const dg = b.dg[q], *const dxb = b.dxb[q], *const dqkv = b.dqkv[q], *const dx_below = b.dxa[l % 3];
+    float *const ws2 = b.parts[q], *const ws1 = ws2 + 3 * row, *const ws_fc = ws1 + 3 * row, *const ws_qkv = ws_fc + fc_floats;
+    if (fork && l + 2 <= L) cudaStreamWaitEvent(main_stream, m.ev_layer[q], 0);      // layer l + 2 is done with the buffers that this one writes
     // x3 = x2 + gelu(ln2 Wfc + bfc) Wproj + bproj
-    DO(product(m, TN, b.dxa, y.gl, m.g(l, W_PROJ), nullptr, C, 4 * C, T, s));
+    DO(weight_grad(dx, y.gl, m.g(l, W_PROJ), C, 4 * C));
     int n_fc = n_fc_own;
     if (m.backend == 2) {
       n_fc = n_fc_sep;
-      DO(product(m, NN, b.dxa, m.p(l, W_PROJ), b.dg, nullptr, T, 4 * C, C, s));
-      TRY(piccl_ops_gelu_bwd(b.dg, y.h, b.dg, ws_fc, T, 4 * C, s));
+      DO(product(m, NN, dx, m.p(l, W_PROJ), dg, nullptr, T, 4 * C, C, s));
+      TRY(piccl_ops_gelu_bwd(dg, y.h, dg, ws_fc, T, 4 * C, s));
     } else {
-      TRY(piccl_ops_gemm(NN, EPI_GELU_GRAD, b.dxa, m.p(l, W_PROJ), b.dg, nullptr, nullptr, y.h, ws_fc, nullptr, 0, T, 4 * C, C, s));
+      TRY(piccl_ops_gemm(NN, EPI_GELU_GRAD, dx, m.p(l, W_PROJ), dg, nullptr, nullptr, y.h, ws_fc, nullptr, 0, T, 4 * C, C, s));
       m.tcgen05++;
     }
-    DO(product(m, TN, b.dg, y.ln2, m.g(l, W_FC), nullptr, 4 * C, C, T, s));
-    DO(product(m, NN, b.dg, m.p(l, W_FC), b.dln2, nullptr, T, C, 4 * C, s));
-    TRY(piccl_ops_ln_bwd(b.dln2, y.x2, m.p(l, LN2_G), y.mean2, y.rstd2, b.dxa, b.dxb, ws2, 1, T, C, s));
+    DO(weight_grad(dg, y.ln2, m.g(l, W_FC), 4 * C, C));
+    DO(product(m, NN, dg, m.p(l, W_FC), b.dln2, nullptr, T, C, 4 * C, s));
+    TRY(piccl_ops_ln_bwd(b.dln2, y.x2, m.p(l, LN2_G), y.mean2, y.rstd2, dx, dxb, ws2, 1, T, C, s));
     // x2 = xin + attention Wo + bo
-    DO(product(m, TN, b.dxb, static_cast<b16*>(att[l].data_ptr()), m.g(l, W_O), nullptr, C, C, T, s));
-    DO(product(m, NN, b.dxb, m.p(l, W_O), b.datt, nullptr, T, C, C, s));
+    DO(weight_grad(dxb, static_cast<b16*>(att[l].data_ptr()), m.g(l, W_O), C, C));
+    DO(product(m, NN, dxb, m.p(l, W_O), b.datt, nullptr, T, C, C, s));
     at::Tensor dq[3];
     attention_grad(m.saved[l], b.datt, B, S, H, D, dq);
     const void* ptr[3]; long long st[9];
     for (int i = 0; i < 3; i++) { ptr[i] = dq[i].data_ptr(); for (int j = 0; j < 3; j++) st[3 * i + j] = dq[i].stride(j); }
-    TRY(piccl_ops_qkv_grad(ptr, st, b.dqkv, ws_qkv, B, S, H, D, s));
-    DO(product(m, TN, b.dqkv, y.ln1, m.g(l, W_QKV), nullptr, 3 * C, C, T, s));
-    DO(product(m, NN, b.dqkv, m.p(l, W_QKV), b.dln1, nullptr, T, C, 3 * C, s));
-    TRY(piccl_ops_ln_bwd(b.dln1, l ? b.layer[l - 1].x3 : b.x0, m.p(l, LN1_G), y.mean1, y.rstd1, b.dxb, b.dxa, ws1, l > 0, T, C, s));
+    TRY(piccl_ops_qkv_grad(ptr, st, dqkv, ws_qkv, B, S, H, D, s));
+    DO(weight_grad(dqkv, y.ln1, m.g(l, W_QKV), 3 * C, C));
+    DO(product(m, NN, dqkv, m.p(l, W_QKV), b.dln1, nullptr, T, C, 3 * C, s));
+    TRY(piccl_ops_ln_bwd(b.dln1, l ? b.layer[l - 1].x3 : b.x0, m.p(l, LN1_G), y.mean1, y.rstd1, dxb, dx_below, ws1, l > 0, T, C, s));
     const piccl_finish_job jobs[8] = {{ws2, m.g(l, LN2_G), n_ln, C, 0, 0}, {ws2 + row, m.g(l, LN2_B), n_ln, C, 0, 0}, {ws2 + 2 * row, m.g(l, B_O), n_ln, C, 0, 0},
                                       {ws_fc, m.g(l, B_FC), n_fc, 4 * C, 0, 0}, {ws_qkv, m.g(l, B_QKV), n_qkv, 3 * C, 0, 0}, {ws1, m.g(l, LN1_G), n_ln, C, 0, 0},
                                       {ws1 + row, m.g(l, LN1_B), n_ln, C, 0, 0}, {ws1 + 2 * row, l ? m.g(l - 1, B_PROJ) : nullptr, n_ln, C, 0, 0}};
-    TRY(piccl_ops_finish_parts(jobs, l ? 8 : 7, s));
+    DO(finish(jobs, l ? 8 : 7, q));
+    dx = dx_below;
     done(m.g(l, B_PROJ), C);
     m.saved[l] = Saved();
-    att[l] = at::Tensor();
+    if (!fork) att[l] = at::Tensor();  // the second stream may still read it
   }
-  TRY(piccl_ops_wpe_bwd(b.dxa, g_wpe, B, S, C, 0, s));
+  TRY(piccl_ops_wpe_bwd(dx, g_wpe, B, S, C, 0, s));
   done(g_wpe, (size_t)d.seq_len * C);
   if (!m.stage.defined()) { m.stage = at::zeros({d.Vp, C}, opt.dtype(at::kFloat)); m.owner = at::zeros({d.Vp}, opt.dtype(at::kInt)); }
-  TRY(piccl_ops_wte_bwd_rows(idx, b.dxa, m.stage.data_ptr<float>(), m.owner.data_ptr<int>(), g_wte, T, C, s));
+  if (fork) {
+    cudaEventRecord(m.ev_fork, m.streams.side);
+    cudaStreamWaitEvent(main_stream, m.ev_fork, 0);
+  }
+  TRY(piccl_ops_wte_bwd_rows(idx, dx, m.stage.data_ptr<float>(), m.owner.data_ptr<int>(), g_wte, T, C, s));
   m.launches++;                       // two kernels
   done(g_wte, (size_t)d.Vp * C);
   return 0;
@@ -273,18 +354,23 @@ void* piccl_gpt2_create(const void* desc) {
 }
 void piccl_gpt2_destroy(void* h) { delete static_cast<Model*>(h); }
 
-// idx / tgt: int64 [B * S] on the device; loss: one float on the device.  counts[4] (optional): launches of this framework's kernels,
+// idx / tgt: int64 [B * S] on the device; loss: one float on the device; captured: the call is captured into a graph.  counts[4] (optional): launches of this framework's kernels,
 // products on tcgen05, products on cuBLAS since the last call.  0, or an error code whose text piccl_gpt2_error() holds.
-int piccl_gpt2_run(void* h, const long long* idx, const long long* tgt, int B, int S, float* loss, int train, int backend, ReadyFn ready, long long* counts) {
+int piccl_gpt2_run(void* h, const long long* idx, const long long* tgt, int B, int S, float* loss, int train, int backend, int captured, ReadyFn ready, long long* counts) {
   Model& m = *static_cast<Model*>(h);
   m.launches = m.cublas = m.tcgen05 = 0;
   m.backend = backend;
+  m.captured = captured != 0;
   int rc;
   try { rc = run(m, idx, tgt, B, S, loss, train != 0, ready); }
   catch (const std::exception& e) { g_error = e.what(); rc = -1000; }
   if (counts) { counts[0] = m.launches; counts[1] = m.tcgen05; counts[2] = m.cublas; }
   return rc;
 }
+// The stream on which a step is captured (nullptr before the first step).
+void* piccl_gpt2_capture_stream(void* h) { return static_cast<Model*>(h)->streams.main; }
+// Where the activations are: a graph captured earlier is of no use once this has changed.
+const void* piccl_gpt2_arena(void* h) { const Model& m = *static_cast<Model*>(h); return m.arena.defined() ? m.arena.data_ptr() : nullptr; }
 const char* piccl_gpt2_error(void) { return g_error.c_str(); }
 
 }  // extern "C"

@@ -54,3 +54,36 @@ def test_training_reduces_loss_and_ready_ranges_are_monotonic():
         m.optimizer_step(lr=1e-3)
     assert ends == sorted(ends) and ends[-1] == m.n_params
     assert losses[-1] < losses[0] - 0.5, losses
+
+
+@pytest.mark.parametrize("layers,d_model,shapes", [
+    (1, 256, [(4, 128)]),
+    (5, 256, [(3, 77), (4, 128), (3, 77)]),       # layers take the gradient buffers in turn; a larger batch moves the activations; back to the first one
+    (3, 512, [(8, 512)]),                         # products of both back ends
+])
+def test_replayed_steps_equal_issued_ones(layers, d_model, shapes):
+    from piccl_b200.models.gpt2 import GPT2, GPT2Config
+    cfg = GPT2Config(vocab_size=1000, seq_len=512, n_layer=layers, n_head=d_model // 64, d_model=d_model)
+    replayed, issued = GPT2(cfg, seed=2), GPT2(cfg, seed=2)
+    gen = torch.Generator().manual_seed(5)
+    for B, S in shapes:
+        a, b = torch.empty(B, S, dtype=torch.int64, device="cuda"), torch.empty(B, S, dtype=torch.int64, device="cuda")
+        for step in range(6):
+            tok = torch.randint(0, cfg.vocab_size, (B, S + 1), generator=gen)
+            a.copy_(tok[:, :-1]); b.copy_(tok[:, 1:])
+            replayed.flat_g.fill_(float("nan")); issued.flat_g.fill_(float("nan"))
+            got = replayed.forward_backward(a, b)
+            want = issued.forward_backward(a, b, on_grads_ready=lambda end: None)       # reports gradients: always issued call by call
+            assert abs(float(got) - float(want)) <= 1e-5 * float(want)
+            n = torch.isnan(issued.flat_g)
+            assert torch.equal(torch.isnan(replayed.flat_g), n)
+            # the same kernels on the same operands: only sums by atomics (attention, embedding) come in another order, at worst another
+            # rounding to bf16 (2^-8) of an element in each of the two halves of a layer
+            g, w = replayed.flat_g[~n].double(), issued.flat_g[~n].double()
+            assert float((g - w).norm()) <= 2 ** -7 * float(w.norm()), step
+            want = issued._issue(a.reshape(-1), b.reshape(-1), B, S, True, 0)
+            assert abs(float(replayed.loss(a, b)) - float(want)) <= 1e-5 * float(want)
+            replayed.flat_g[n] = 0.0                  # positions that no token had
+            replayed.optimizer_step(lr=1e-4 * (step + 1))
+            issued.flat_p.copy_(replayed.flat_p)
+    assert replayed._graphs, "nothing was captured"
