@@ -209,74 +209,107 @@ __global__ void __launch_bounds__(512) ce_fwd_bwd_kernel(bf16* __restrict__ logi
   }
 }
 
-// The same with the row kept in shared memory between its passes (maximum, sum of exponentials, gradient): logits are read from memory
-// once, where the kernel above reads them twice (8192 x 50304: 567 -> 300 us; read + write at the copy rate: 252 us).  The passes of
-// the blocks that share an SM overlap: one loads its row while the other computes.  GRAD = false leaves the logits as they are.
+// What a thread has seen of a row so far: maximum and sum of exp(x - maximum).
+struct OnlineSum {
+  float m = -INFINITY, s = 0.f;
+  static constexpr float kLog2e = 1.4426950408889634f;
+  __device__ __forceinline__ void add(const f32x2 x2, float mb, f32x2& a) {
+    float x, y; unpack2(fma2(x2, both2(kLog2e), both2(mb)), x, y);
+    a = add2(a, pack2(ex2_approx(x), ex2_approx(y)));
+  }
+  template <int N> __device__ __forceinline__ void packs(const bf16x8 (&p)[N]) {
+    __nv_bfloat162 q = p[0].v[0];
+#pragma unroll
+    for (int u = 0; u < N; u++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) q = __hmax2(q, p[u].v[e]);
+    const float top = fmaxf(__low2float(q), __high2float(q));
+    if (top > m) { s *= ex2_approx((m - top) * kLog2e); m = top; }               // at first 0 * exp(-inf)
+    const float mb = m == -INFINITY ? 0.f : -m * kLog2e;
+    f32x2 a[2] = {both2(0.f), both2(0.f)};
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+      float v[8]; unpack8(p[u], v);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) add(pack2(v[e], v[e + 1]), mb, a[(e >> 1) & 1]);
+    }
+    float x, y; unpack2(add2(a[0], a[1]), x, y);
+    s += x + y;
+  }
+  // all threads of a block of W warps: the whole row's m and s
+  template <int W> __device__ __forceinline__ void block(float2 (&sh)[W]) {
+    const float wm = warp_max(m);
+    const float ws = warp_sum(wm == -INFINITY ? 0.f : s * ex2_approx((m - wm) * kLog2e));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_float2(wm, ws);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const float2 w = lane < W ? sh[lane] : make_float2(-INFINITY, 0.f);
+    m = warp_max(w.x);
+    s = warp_sum(w.x == -INFINITY ? 0.f : w.y * ex2_approx((w.x - m) * kLog2e));
+  }
+};
+// columns from V on are padding
+__device__ __forceinline__ bf16x8 mask_padding(bf16x8 p, int col, int V) {
+  float v[8]; unpack8(p, v);
+#pragma unroll
+  for (int e = 0; e < 8; e++) if (col + e >= V) v[e] = -INFINITY;
+  return pack8(v);
+}
+// exp(x - m) / s * gs of a pack; lb = -(m + log s) in base 2
+__device__ __forceinline__ bf16x8 ce_gradient(const bf16x8& p, float lb, float gs) {
+  float v[8]; unpack8(p, v);
+#pragma unroll
+  for (int e = 0; e < 8; e += 2) {
+    float x, y; unpack2(fma2(pack2(v[e], v[e + 1]), both2(OnlineSum::kLog2e), both2(lb)), x, y);
+    unpack2(mul2(pack2(ex2_approx(x), ex2_approx(y)), both2(gs)), v[e], v[e + 1]);
+  }
+  return pack8(v);
+}
+// the target's column has gs less
+__device__ __forceinline__ bf16 ce_gradient_target(float x, float lb, float gs) { return __float2bfloat16_rn(ex2_approx(fmaf(x, OnlineSum::kLog2e, lb)) * gs - gs); }
+
+// The same in one pass over memory: the sum of exponentials is taken while the row comes in, relative to the thread's maximum so far, and
+// the gradient needs the row once more, from shared memory.  GRAD = false leaves the logits as they are and keeps nothing.
+// Two blocks share an SM: one loads while the other computes.  8192 x 50304: 364 us with the gradient, 183 without (386 and 219 with a pass
+// of its own for the sum; the copy rate allows 252 and 126, the special-function units 183 and 92).  One block per SM with the next row
+// on its way to a second buffer was slower, 492 us.
 template <bool GRAD>
-__global__ void __launch_bounds__(512) ce_row_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss, int V, int Vp, float gscale) {
+__global__ void __launch_bounds__(512, 2) ce_row_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss, int V, int Vp, float gscale) {
   pdl_begin();
   extern __shared__ __align__(16) unsigned char ce_smem[];
   bf16x8* const row_s = reinterpret_cast<bf16x8*>(ce_smem);
-  __shared__ float sh[16];
-  const int row = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ float2 sh[16];
+  const int row = blockIdx.x, tid = threadIdx.x;
   bf16x8* lp = reinterpret_cast<bf16x8*>(logits + (size_t)row * Vp);
   const int n8 = Vp / 8, full8 = V / 8;               // packs [full8, n8) hold padding columns
-  const float kLog2e = 1.4426950408889634f;
   const long long t = targets[row];
-  float m = -INFINITY;
+  const bool valid = t >= 0 && t < V;
+  const bool owner = valid ? (int)(t >> 3) % 512 == tid : tid == 0;      // has the target's pack
+  const float xt = valid && owner ? __bfloat162float(reinterpret_cast<const bf16*>(lp)[t]) : 0.f;
+  OnlineSum o;
   int i = tid;
   for (; i + 3 * 512 < full8; i += 4 * 512) {
     bf16x8 p[4];
 #pragma unroll
     for (int u = 0; u < 4; u++) p[u] = lp[i + u * 512];
+    if (GRAD) {
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      row_s[i + u * 512] = p[u];
-      float v[8]; unpack8(p[u], v);
-#pragma unroll
-      for (int e = 0; e < 8; e++) m = fmaxf(m, v[e]);
+      for (int u = 0; u < 4; u++) row_s[i + u * 512] = p[u];
     }
+    o.packs(p);
   }
   for (; i < n8; i += 512) {
-    const bf16x8 p = lp[i];
-    float v[8]; unpack8(p, v);
-#pragma unroll
-    for (int e = 0; e < 8; e++) { if (i * 8 + e >= V) v[e] = -INFINITY; m = fmaxf(m, v[e]); }
-    row_s[i] = pack8(v);
+    const bf16x8 p[1] = {i < full8 ? lp[i] : mask_padding(lp[i], i * 8, V)};
+    if (GRAD) row_s[i] = p[0];
+    o.packs(p);
   }
-  m = warp_max(m);
-  if (lane == 0) sh[warp] = m;
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < 16; w++) m = fmaxf(m, sh[w]);
-  const float mb = -m * kLog2e;
-  float s = 0.f;
-  for (i = tid; i < n8; i += 512) {
-    float v[8]; unpack8(row_s[i], v);
-#pragma unroll
-    for (int e = 0; e < 8; e++) s += ex2_approx(fmaf(v[e], kLog2e, mb));      // padding: exp(-inf) = 0
-  }
-  s = warp_sum(s);
-  __syncthreads();
-  if (lane == 0) sh[warp] = s;
-  __syncthreads();
-  s = 0.f;
-#pragma unroll
-  for (int w = 0; w < 16; w++) s += sh[w];
-  const bool valid = t >= 0 && t < V;
-  if (tid == 0) loss[row] = valid ? (logf(s) + m - __bfloat162float(reinterpret_cast<const bf16*>(row_s)[t])) : 0.f;
+  o.block(sh);
+  if (owner) loss[row] = valid ? logf(o.s) + o.m - xt : 0.f;
   if (!GRAD) return;
-  const float lb = mb - log2f(s), gs = valid ? gscale : 0.f;
-  for (i = tid; i < n8; i += 512) {
-    float v[8]; unpack8(row_s[i], v);
-#pragma unroll
-    for (int e = 0; e < 8; e++) v[e] = ex2_approx(fmaf(v[e], kLog2e, lb)) * gs;
-    if (valid && (t >> 3) == i) {
-#pragma unroll
-      for (int e = 0; e < 8; e++) if (e == (int)(t & 7)) v[e] -= gscale;
-    }
-    lp[i] = pack8(v);
-  }
+  const float lb = -o.m * OnlineSum::kLog2e - log2f(o.s);
+#pragma unroll 1       // stores in bursts of four cost a quarter of the time
+  for (i = tid; i < n8; i += 512) lp[i] = ce_gradient(row_s[i], lb, valid ? gscale : 0.f);
+  if (valid && owner) reinterpret_cast<bf16*>(lp)[t] = ce_gradient_target(xt, lb, gscale);
 }
 
 // out[0] = mean of x[0..n), one block
@@ -506,18 +539,18 @@ int piccl_ops_colsum(const void* x, void* out, float* workspace, int rows, int C
 // grad = 0: losses only, the logits stay as they are.
 int piccl_ops_ce(void* logits, const long long* targets, float* loss, int rows, int V, int Vp, float gscale, int grad, void* stream) {
   if (Vp % 8 || V > Vp) return -1;
-  const int smem = Vp * 2;
-  if (smem <= 220 * 1024) {                           // a row fits one SM (two up to 56 Ki columns); beyond, or without it, the two-pass kernel
+  const int smem = Vp * 2, most = 220 * 1024;        // a row fits one SM (two up to 56 Ki columns); beyond, the gradient takes the two-pass kernel
+  cudaStream_t s = (cudaStream_t)stream;
+  if (!grad) launch_pdl(ce_row_kernel<false>, rows, 512, 0, s, (bf16*)logits, targets, loss, V, Vp, gscale);
+  else if (smem <= most) {
     static bool ready[64] = {false};
     int dev = 0; cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !ready[dev]) {
-      if (cudaFuncSetAttribute(ce_row_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess ||
-          cudaFuncSetAttribute(ce_row_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return -4;
+      if (cudaFuncSetAttribute(ce_row_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return -4;
       ready[dev] = true;
     }
-    if (grad) launch_pdl(ce_row_kernel<true>, rows, 512, smem, (cudaStream_t)stream, (bf16*)logits, targets, loss, V, Vp, gscale);
-    else launch_pdl(ce_row_kernel<false>, rows, 512, smem, (cudaStream_t)stream, (bf16*)logits, targets, loss, V, Vp, gscale);
-  } else launch_pdl(ce_fwd_bwd_kernel, rows, 512, 0, (cudaStream_t)stream, (bf16*)logits, targets, loss, V, Vp, gscale);
+    launch_pdl(ce_row_kernel<true>, rows, 512, smem, s, (bf16*)logits, targets, loss, V, Vp, gscale);
+  } else launch_pdl(ce_fwd_bwd_kernel, rows, 512, 0, s, (bf16*)logits, targets, loss, V, Vp, gscale);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 int piccl_ops_ce_fwd_bwd(void* logits, const long long* targets, float* loss, int rows, int V, int Vp, float gscale, void* stream) {

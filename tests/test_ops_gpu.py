@@ -110,3 +110,54 @@ def test_embedding_forward_backward():
     ops.wte_bwd(idx, dx, stage, dwte)
     ref_g = torch.zeros(V, C, device="cuda").index_add_(0, idx, dx.float())
     assert torch.allclose(dwte.float(), ref_g, atol=5e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("C,rows", [(256, 1), (256, 6001), (512, 3700), (768, 3001), (1024, 5), (1024, 3001), (2048, 1800)])
+def test_layernorm_rows_in_several_rounds(C, rows):
+    # more rows than the resident warps (forward) and groups (backward) have at once: rows are prefetched, the last round is partial
+    from piccl_b200 import ops
+    x, res, gamma, beta = _bf(rows, C, seed=1), _bf(rows, C, seed=2), _bf(C, seed=3) * 0.1 + 1, _bf(C, seed=4) * 0.1
+    y, s, mean, rstd = torch.empty_like(x), torch.empty_like(x), torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda")
+    for r in (res, None):
+        ops.layernorm_fwd(x, r, gamma, beta, s, y, mean, rstd)
+        xin = (x.float() + r.float()).to(torch.bfloat16) if r is not None else x
+        assert torch.equal(s, xin)
+        xr, gr, br = xin.double().requires_grad_(), gamma.double().requires_grad_(), beta.double().requires_grad_()
+        yr = F.layer_norm(xr, (C,), gr, br, 1e-5)
+        assert torch.all((y.double() - yr).abs() <= 2 ** -8 * yr.abs() + 1e-4)          # one rounding to bf16, fp32 sums
+    if C > 1024:
+        return
+    dy = _bf(rows, C, seed=5)
+    dx, dg, db = torch.empty_like(x), torch.empty_like(gamma), torch.empty_like(beta)
+    ops.layernorm_bwd(dy, x, gamma, mean, rstd, None, dx, dg, db)
+    yr.backward(dy.double())
+    for got, want in ((dx, xr.grad), (dg, gr.grad), (db, br.grad)):
+        assert torch.all((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-3 * want.abs().max())
+
+
+@pytest.mark.parametrize("rows,V,Vp", [(3, 5, 8), (40, 1000, 1024), (5, 16400, 16512), (9, 50257, 50304), (2, 120001, 120064)])
+def test_cross_entropy_online(rows, V, Vp):
+    # vocabularies below and beyond a block's round of 16384 columns and beyond what shared memory holds; logits that rise along the row
+    # raise the running maximum all the time
+    from ctypes import c_float, c_void_p
+    from piccl_b200 import _native as N
+    logits = _bf(rows, Vp, scale=3.0, seed=1)
+    logits[0] += torch.linspace(-20, 20, Vp, device="cuda").to(torch.bfloat16)
+    logits[1, : V // 2] = float("-inf")
+    tgt = torch.randint(V // 2, V, (rows,), generator=torch.Generator().manual_seed(2)).cuda()
+    tgt[-1] = -100                                          # no target: no loss, no gradient
+    ref_in = logits[:, :V].double().requires_grad_()
+    ref = F.cross_entropy(ref_in, tgt, reduction="none")
+    ref.sum().backward()
+    for grad in (0, 1):
+        loss, lg = torch.empty(rows, device="cuda"), logits.clone()
+        rc = N.ops_lib().piccl_ops_ce(c_void_p(lg.data_ptr()), c_void_p(tgt.data_ptr()), c_void_p(loss.data_ptr()), rows, V, Vp, c_float(0.5), grad, c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        # exponents up to 2^7 carry fp32 rounding of 2^-17; the sum and the logarithm add less
+        assert torch.all((loss.double() - ref.detach()).abs() <= 1e-4)
+        if not grad:
+            assert torch.equal(lg, logits)
+            continue
+        want = 0.5 * ref_in.grad
+        assert torch.all((lg[:, :V].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5)
+        assert lg[:, V:].abs().sum() == 0
