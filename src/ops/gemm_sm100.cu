@@ -254,8 +254,10 @@ static int device_ready(int dev) {
   return 0;
 }
 
-// Tile width and slices of K: waves of the persistent grid times the clocks of a tile.  A k-step of 16 takes 136 / 68 / 51 clocks at
-// 256 / 128 / 64 columns (measured; the MMA alone needs TN / 2), which favours wide tiles until they no longer fill the pairs.
+// Tile width and slices of K: waves of the persistent grid times the clocks of a tile.  A k-step of 16 takes 136 / 84 / 70 clocks at
+// 256 / 128 / 64 columns: the MMA alone needs TN / 2, and with all pairs busy narrow tiles ask more of the L2 than it gives (8192 x 4096 x
+// 1024: 50 / 67 / 98 us; alone on the chip 68 and 51 clocks).  Over 48 shapes of 128 to 8192 rows the width taken is 1 % behind the best
+// of the three on average, 11 % at worst (3 % and 24 % when the rule had the clocks of a chip that is otherwise idle).
 // K is split where the tiles of a deep product leave pairs idle (weight gradients, few rows): a slice then writes its accumulator and
 // the last one reads the others' (about 30 clocks a column and slice: 1024 x 1024 x 8192 gains, 23.1 -> 18.7 us, 3072 x 1024 x 8192 does not).  A slice keeps at least 8 k-blocks.
 constexpr size_t kTicketBytes = 64 * 1024;
@@ -266,7 +268,7 @@ static Variant* choose(int layout, int epi, int M, int N, int K, int pairs, size
   for (auto& v : g_variants) {
     if (v.layout != layout || v.epi != epi) continue;
     const long tiles = (long)((M + 255) / 256) * ((N + v.tn - 1) / v.tn);
-    const double step = v.tn == 256 ? 136 : v.tn == 128 ? 68 : 51;
+    const double step = v.tn == 256 ? 136 : v.tn == 128 ? 84 : 70;
     for (int s = v.split ? 2 : 1; s <= (v.split ? 16 : 1) && (s == 1 || kb / s >= 8); s++) {
       if (s > 1 && (split_bytes(tiles, s, v.tn) > ws_bytes || tiles * 64 > (long)kTicketBytes)) break;
       const double cost = (double)((tiles * s + pairs - 1) / pairs) * (step * 4 * ((kb + s - 1) / s) + 10.0 * v.tn) + (s > 1 ? 30.0 * v.tn * (s + 1) : 0);
