@@ -269,7 +269,7 @@ def run_piccl(args):
         st = comm.stats()
         comm_stats = {"allreduce_calls": int(st.calls[1]), "in_switch_calls": int(st.nvls_calls), "kernel_launches": int(st.launches)}
     algo_name = trainer.averager.algo
-    launch_mode = "CUDA graph replay" if trainer.use_graph else "eager"
+    launch_mode = "CUDA graph replay" if trainer.use_graph else "forward and backward replayed from a CUDA graph, AdamW launched" if world == 1 else "eager"
     gemm_counts = None
     if rank == 0:
         from piccl_b200.ops import gemm
