@@ -7,9 +7,11 @@
 namespace piccl_ops {
 
 // y = LN(x + res) * gamma + beta ; sum_out = x + res (optional)
-// Memory bound: up to 4 tensors of rows * C bf16.  The grid is what the chip holds at once; a warp loads its next row before it works on the
-// one it has, so that 4 KiB per warp are always on their way at C = 1024 (16 to 20 warps an SM: more than the 44 KB that
-// cover the latency).  8192 x 1024: 18.6 -> 17.3 us without the L2, 10.3 at the copy rate of a long copy.
+// Up to 4 tensors of rows * C bf16.  The grid is what the chip holds at once; a warp loads its next row before it works on the one it has, so
+// that 4 KiB per warp are always on their way at C = 1024 (20 warps an SM: more than the 44 KB that cover the latency).  gamma and beta come
+// from shared memory and the arithmetic runs on pairs: reading them from the L1 again for each row and with
+// an instruction per element the kernel was bound by its load queue and by issue (32768 x 1024: 56.4 us, now 44.5, 41.1 at the copy rate;
+// 8192 x 1024: 17.2 us, now 14.1 without the L2).
 constexpr int ln_fwd_blocks(int V) { return V == 1 ? 10 : V == 2 ? 6 : V <= 4 ? 5 : V <= 6 ? 4 : 3; }      // of 4 warps per SM
 template <int V, bool RES>   // V 16-byte vectors per lane: C = 256 * V
 __global__ void __launch_bounds__(128, ln_fwd_blocks(V)) ln_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, const bf16* __restrict__ gamma,
@@ -19,7 +21,7 @@ __global__ void __launch_bounds__(128, ln_fwd_blocks(V)) ln_fwd_kernel(const bf1
   constexpr int C = 256 * V;
   const int lane = threadIdx.x & 31, step = gridDim.x * 4;
   int row = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (row >= rows) return;
+  __shared__ bf16x8 sg[V * 32], sb[V * 32];
   bf16x8 px[V], pr[V];
   auto load = [&](int r) {
 #pragma unroll
@@ -28,17 +30,19 @@ __global__ void __launch_bounds__(128, ln_fwd_blocks(V)) ln_fwd_kernel(const bf1
       if (RES) pr[i] = reinterpret_cast<const bf16x8*>(res)[(size_t)r * (C / 8) + lane + 32 * i];
     }
   };
-  load(row);
+  if (row < rows) load(row);
+  for (int i = threadIdx.x; i < V * 32; i += 128) { sg[i] = reinterpret_cast<const bf16x8*>(gamma)[i]; sb[i] = reinterpret_cast<const bf16x8*>(beta)[i]; }
+  __syncthreads();
   for (; row < rows; row += step) {
-    float v[V][8];
+    f32x2 v[V][4];
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < V; i++) {
       unpack8(px[i], v[i]);
       if (RES) {
-        float r[8]; unpack8(pr[i], r);
+        f32x2 r[4]; unpack8(pr[i], r);
 #pragma unroll
-        for (int e = 0; e < 8; e++) v[i][e] += r[e];
+        for (int e = 0; e < 4; e++) v[i][e] = add2(v[i][e], r[e]);
       }
       if (sum_out) {
         const bf16x8 p = pack8(v[i]);
@@ -46,25 +50,26 @@ __global__ void __launch_bounds__(128, ln_fwd_blocks(V)) ln_fwd_kernel(const bf1
         unpack8(p, v[i]);          // normalise exactly what was stored
       }
 #pragma unroll
-      for (int e = 0; e < 8; e++) s += v[i][e];
+      for (int e = 0; e < 4; e++) { float a, b; unpack2(v[i][e], a, b); s += a; s += b; }
     }
     if (row + step < rows) load(row + step);
     const float mu = warp_sum(s) / C;
+    const f32x2 neg_mu = both2(-mu);
     float q = 0.f;
 #pragma unroll
     for (int i = 0; i < V; i++)
 #pragma unroll
-      for (int e = 0; e < 8; e++) { const float d = v[i][e] - mu; q += d * d; }
+      for (int e = 0; e < 4; e++) { v[i][e] = add2(v[i][e], neg_mu); float a, b; unpack2(v[i][e], a, b); q = fmaf(a, a, q); q = fmaf(b, b, q); }
     const float rs = rsqrtf(warp_sum(q) / C + eps);
+    const f32x2 rs2 = both2(rs);
     if (lane == 0) { mean[row] = mu; rstd[row] = rs; }
 #pragma unroll
     for (int i = 0; i < V; i++) {
-      float g[8], b[8], o[8];
-      unpack8(reinterpret_cast<const bf16x8*>(gamma)[lane + 32 * i], g);
-      unpack8(reinterpret_cast<const bf16x8*>(beta)[lane + 32 * i], b);
+      f32x2 g[4], b[4];
+      unpack8(sg[lane + 32 * i], g); unpack8(sb[lane + 32 * i], b);
 #pragma unroll
-      for (int e = 0; e < 8; e++) o[e] = (v[i][e] - mu) * rs * g[e] + b[e];
-      reinterpret_cast<bf16x8*>(y)[(size_t)row * (C / 8) + lane + 32 * i] = pack8(o);
+      for (int e = 0; e < 4; e++) v[i][e] = fma2(mul2(v[i][e], rs2), g[e], b[e]);
+      reinterpret_cast<bf16x8*>(y)[(size_t)row * (C / 8) + lane + 32 * i] = pack8(v[i]);
     }
   }
 }
@@ -72,24 +77,27 @@ __global__ void __launch_bounds__(128, ln_fwd_blocks(V)) ln_fwd_kernel(const bf1
 // dx = LN-backward(dy) + dres ; per-block partial column sums in fp32: part[0] = dgamma, part[1] = dbeta and, with_dsum, part[2] = sum
 // of the dx written (dx is the gradient that enters the layer before, whose bias gradient is exactly that sum: the kernel that
 // has the rows in registers adds them up, so nobody reads dx again for it).
-// Memory bound: 4 tensors of rows * C bf16.  A row is spread over V warps (8 columns a thread), so the three accumulators cost 24
+// 4 tensors of rows * C bf16.  A row is spread over V warps (8 columns a thread), so the three accumulators cost 24
 // registers instead of the 96 of a warp per row at C = 1024, and R rows are in flight per group; G groups of V warps make a
 // block of about 8 warps.  The grid is what the chip holds at once: each block leaves one partial row per vector.  The next rows are loaded
-// while those at hand wait for their sums (8192 x 1024: 19.7 -> 17.6 us without the L2, 10.3 at the copy rate of a long copy).
+// while those at hand wait for their sums, the arithmetic runs on pairs and the four sums of two rows are reduced together: 2 instructions
+// in 3 had been shuffles, conversions and single additions (32768 x 1024: 58.1 -> 55.4 us, 41.1 at the copy rate; 8192 x 1024: 16.7 us).
+// What is left is the wait for the sums, with 16 warps an SM.
 template <int V, int G, int R, bool RES>   // C = 256 * V
 __global__ void __launch_bounds__(32 * V * G, 2) ln_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ xin, const bf16* __restrict__ gamma,
                                                                const float* __restrict__ mean, const float* __restrict__ rstd, const bf16* __restrict__ dres,
                                                                bf16* __restrict__ dx, float* __restrict__ part, int rows, int with_dsum) {
   pdl_begin();
   constexpr int C = 256 * V;
-  __shared__ float red[2][G][V][2 * R];
+  static_assert(R == 2, "four sums are reduced together");
+  __shared__ float4 red[2][G][V];
   __shared__ float sh[G][C];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = warp / V, wv = warp % V;
   const int c8 = wv * 32 + lane;
-  float ga[8], dg[8], db[8], ds[8];
+  f32x2 ga[4], dg[4], db[4], ds[4];
   unpack8(reinterpret_cast<const bf16x8*>(gamma)[c8], ga);
 #pragma unroll
-  for (int e = 0; e < 8; e++) { dg[e] = 0.f; db[e] = 0.f; ds[e] = 0.f; }
+  for (int e = 0; e < 4; e++) { dg[e] = both2(0.f); db[e] = both2(0.f); ds[e] = both2(0.f); }
   int buf = 0;
   bf16x8 ny[R], nx[R], nr[R];                          // the rows to come: loaded while those before them are worked on
   float nmu[R], nrs[R];
@@ -108,60 +116,67 @@ __global__ void __launch_bounds__(32 * V * G, 2) ln_bwd_kernel(const bf16* __res
   int r0 = (blockIdx.x * G + g) * R;
   if (r0 < rows) load(r0);
   for (; r0 < rows; r0 += step, buf ^= 1) {
-    bf16x8 py[R], px[R], pr[R];
-    float mu[R], rs[R];
+    f32x2 t[R][4], xh[R][4];                           // dy * gamma and the normalised input
+    bf16x8 pr[R];
+    float s[2 * R], rs[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) { py[r] = ny[r]; px[r] = nx[r]; if (RES) pr[r] = nr[r]; mu[r] = nmu[r]; rs[r] = nrs[r]; }
+    for (int r = 0; r < R; r++) {
+      const bool in = r0 + r < rows;
+      f32x2 y[4];
+      unpack8(nx[r], xh[r]); unpack8(ny[r], y);
+      if (RES) pr[r] = nr[r];
+      rs[r] = nrs[r];
+      const f32x2 neg_mu = both2(-nmu[r]), rs2 = both2(rs[r]);
+      f32x2 s1 = both2(0.f), s2 = both2(0.f);
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        if (!in) y[e] = both2(0.f);                    // a row beyond the last one adds nothing
+        xh[r][e] = mul2(add2(xh[r][e], neg_mu), rs2);
+        t[r][e] = mul2(y[e], ga[e]);
+        dg[e] = fma2(y[e], xh[r][e], dg[e]);
+        db[e] = add2(db[e], y[e]);
+        s1 = add2(s1, t[r][e]);
+        s2 = fma2(t[r][e], xh[r][e], s2);
+      }
+      s[2 * r] = sum2(s1); s[2 * r + 1] = sum2(s2);
+    }
     if (r0 + step < rows) load(r0 + step);
-    float s[2 * R];
+    // the four sums over the warp together: each exchange halves what a lane still has to add, lanes 8 i to 8 i + 7 end up with sum i
+    const bool hi = lane & 16, odd = lane & 8;
+    float a = hi ? s[2] : s[0], b = hi ? s[3] : s[1];
+    a += __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 16);
+    b += __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 16);
+    float c = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      s[2 * r] = 0.f; s[2 * r + 1] = 0.f;
-      if (r0 + r < rows) {
-        float x[8], y[8];
-        unpack8(px[r], x); unpack8(py[r], y);
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-          const float xh = (x[e] - mu[r]) * rs[r], t = y[e] * ga[e];
-          dg[e] += y[e] * xh; db[e] += y[e];
-          s[2 * r] += t; s[2 * r + 1] += t * xh;
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 2 * R; i++) s[i] = warp_sum(s[i]);
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if (V > 1) {
-      if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < 2 * R; i++) red[buf][g][wv][i] = s[i];
-      }
+      if ((lane & 7) == 0) reinterpret_cast<float*>(&red[buf][g][wv])[lane >> 3] = c;
       asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(32 * V) : "memory");      // the other buffer is free: its readers have passed this barrier
+      float4 w = red[buf][g][0];
 #pragma unroll
-      for (int i = 0; i < 2 * R; i++) {
-        s[i] = 0.f;
+      for (int i = 1; i < V; i++) { const float4 u = red[buf][g][i]; w.x += u.x; w.y += u.y; w.z += u.z; w.w += u.w; }
+      s[0] = w.x; s[1] = w.y; s[2] = w.z; s[3] = w.w;
+    } else {
 #pragma unroll
-        for (int w = 0; w < V; w++) s[i] += red[buf][g][w][i];
-      }
+      for (int i = 0; i < 4; i++) s[i] = __shfl_sync(0xffffffffu, c, 8 * i);
     }
 #pragma unroll
     for (int r = 0; r < R; r++) {
       if (r0 + r < rows) {
-        const float s1 = s[2 * r] * (1.f / C), s2 = s[2 * r + 1] * (1.f / C);
-        float x[8], y[8], o[8];
-        unpack8(px[r], x); unpack8(py[r], y);
+        const f32x2 neg_s1 = both2(s[2 * r] * (-1.f / C)), neg_s2 = both2(s[2 * r + 1] * (-1.f / C)), rs2 = both2(rs[r]);
+        f32x2 o[4];
         if (RES) unpack8(pr[r], o);
-        else {
 #pragma unroll
-          for (int e = 0; e < 8; e++) o[e] = 0.f;
+        for (int e = 0; e < 4; e++) {
+          const f32x2 d = fma2(xh[r][e], neg_s2, add2(t[r][e], neg_s1));
+          o[e] = RES ? fma2(d, rs2, o[e]) : mul2(d, rs2);
         }
-#pragma unroll
-        for (int e = 0; e < 8; e++) o[e] += rs[r] * (y[e] * ga[e] - s1 - (x[e] - mu[r]) * rs[r] * s2);
         const bf16x8 p = pack8(o);
         reinterpret_cast<bf16x8*>(dx)[(size_t)(r0 + r) * (C / 8) + c8] = p;
         if (with_dsum) {
           unpack8(p, o);
 #pragma unroll
-          for (int e = 0; e < 8; e++) ds[e] += o[e];
+          for (int e = 0; e < 4; e++) ds[e] = add2(ds[e], o[e]);
         }
       }
     }
@@ -171,7 +186,7 @@ __global__ void __launch_bounds__(32 * V * G, 2) ln_bwd_kernel(const bf16* __res
   for (int vec = 0; vec < 3; vec++) {
     if (vec == 2 && !with_dsum) break;
 #pragma unroll
-    for (int e = 0; e < 8; e++) sh[g][c8 * 8 + e] = vec == 0 ? dg[e] : vec == 1 ? db[e] : ds[e];
+    for (int e = 0; e < 4; e++) unpack2(vec == 0 ? dg[e] : vec == 1 ? db[e] : ds[e], sh[g][c8 * 8 + 2 * e], sh[g][c8 * 8 + 2 * e + 1]);
     __syncthreads();
     float* dst = part + ((size_t)vec * gridDim.x + blockIdx.x) * C;
     for (int c = threadIdx.x; c < C; c += 32 * V * G) {

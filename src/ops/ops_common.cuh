@@ -60,6 +60,17 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ f32x2 both2(float a) { return pack2(a, a); }
+__device__ __forceinline__ float sum2(f32x2 v) { float a, b; unpack2(v, a, b); return a + b; }
+__device__ __forceinline__ void unpack8(const bf16x8& p, f32x2 (&f)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) { const float2 t = __bfloat1622float2(p.v[i]); f[i] = pack2(t.x, t.y); }
+}
+__device__ __forceinline__ bf16x8 pack8(const f32x2 (&f)[4]) {
+  bf16x8 p;
+#pragma unroll
+  for (int i = 0; i < 4; i++) { float a, b; unpack2(f[i], a, b); p.v[i] = __floats2bfloat162_rn(a, b); }
+  return p;
+}
 
 __device__ __forceinline__ f32x2 gelu_sigmoid2(f32x2 x, f32x2 xx) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f, c = -2.f * k0 * 1.4426950408889634f;
