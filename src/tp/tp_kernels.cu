@@ -138,6 +138,14 @@ struct RsPolicy {
     pending = nullptr;
   }
   __device__ void finish(const EpiCtx& e) { if (e.lane == 0) announce<0>(); }
+  // Buffer p of the warp, free to be written: every tile with a result, own or remote, sends its first piece from buffer 0 and its second
+  // from buffer 1, one group each, so the last store out of buffer p is two groups old whatever kind of tile came before.
+  __device__ EpiCtx staging_turn(EpiCtx e, int p) const {
+    if (e.lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+    __syncwarp();
+    e.staging += p * PAIR_STAGING;
+    return e;
+  }
   __device__ bool epilogue(const EpiCtx& e, int, int m_blk, int n_blk, volatile int* abort_flag) {
     const int slot = seq++ & 3;
     const int owner = m_blk < 0 ? -1 : m_blk / mb_per_owner, t = m_blk < 0 ? 0 : tile_id(m_blk, n_blk);
@@ -152,12 +160,9 @@ struct RsPolicy {
 #pragma unroll
       for (int p = 0; p < 2; p++) {
         const int pc = e.half * 2 + p;
-        uint8_t* const st = e.staging + p * PAIR_STAGING;
         float v[64];
         epi_load64(e, pc * 64, v);
-        // this buffer's last store was two groups ago
-        if (e.lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        __syncwarp();
+        uint8_t* const st = staging_turn(e, p).staging;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
@@ -177,8 +182,9 @@ struct RsPolicy {
     const bool ok = e.lane >= n || e.lane == rank || wait_flag(flag_ptr(rank, e.lane, t), a.epoch, abort_flag);
     if (!__all_sync(0xffffffffu, ok)) return false;
 #pragma unroll 1
-    for (int pc = e.half * 2; pc < e.half * 2 + 2; pc++) {
-      epi_staging_free(e);
+    for (int p = 0; p < 2; p++) {
+      const int pc = e.half * 2 + p;
+      const EpiCtx b = staging_turn(e, p);
 #pragma unroll 1
       for (int h = 0; h < 2; h++) {                      // 32 columns; the words of four partials are in flight at a time
         float sum[32];
@@ -192,12 +198,12 @@ struct RsPolicy {
           for (int i = 0; i < 32; i++) sum[i] += __uint_as_float(r[i]);
         };
 #pragma unroll
-        for (int b = 0; b < TP_MAX_RANKS - 1; b += 4) {  // rank order: the same result whatever the arrival order
+        for (int q0 = 0; q0 < TP_MAX_RANKS - 1; q0 += 4) {  // rank order: the same result whatever the arrival order
           uint4 w[4][4];
 #pragma unroll
           for (int i = 0; i < 4; i++) {
-            if (b + i < n - 1) {
-              const char* p = piece(rank, b + i < rank ? b + i : b + i + 1, t, e, pc) + h * 2048 + e.lane * 16;
+            if (q0 + i < n - 1) {
+              const char* p = piece(rank, q0 + i < rank ? q0 + i : q0 + i + 1, t, e, pc) + h * 2048 + e.lane * 16;
 #pragma unroll
               for (int j = 0; j < 4; j++)
                 asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[i][j].x), "=r"(w[i][j].y), "=r"(w[i][j].z), "=r"(w[i][j].w) : "l"(p + j * 512) : "memory");
@@ -205,8 +211,8 @@ struct RsPolicy {
           }
 #pragma unroll
           for (int i = 0; i < 4; i++) {
-            if (b + i == rank) add_own();
-            if (b + i < n - 1) {
+            if (q0 + i == rank) add_own();
+            if (q0 + i < n - 1) {
 #pragma unroll
               for (int j = 0; j < 4; j++) {
                 const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&w[i][j]);
@@ -221,12 +227,12 @@ struct RsPolicy {
           uint4 o; __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
           for (int q = 0; q < 4; q++) o2[q] = __floats2bfloat162_rn(sum[8 * j + 2 * q], sum[8 * j + 2 * q + 1]);
-          *reinterpret_cast<uint4*>(e.staging + e.lane * 128 + (((h * 4 + j) ^ (e.lane & 7)) << 4)) = o;      // as epi_stage_row lays a row out
+          *reinterpret_cast<uint4*>(b.staging + e.lane * 128 + (((h * 4 + j) ^ (e.lane & 7)) << 4)) = o;      // as epi_stage_row lays a row out
         }
       }
       fence_proxy_async();
       __syncwarp();
-      epi_ship(e, &R->tc, n_blk * TP_BN + pc * 64, (m_blk % mb_per_owner) * TP_BM + e.quarter * 32);
+      epi_ship(b, &R->tc, n_blk * TP_BN + pc * 64, (m_blk % mb_per_owner) * TP_BM + e.quarter * 32);
     }
     return true;
   }

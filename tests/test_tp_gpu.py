@@ -136,3 +136,25 @@ def test_odd_row_blocks_and_panel_edges(n, M, N, K):
         ref = full @ Bs[r].double().t()
         assert (outs[r].double() - ref).norm() <= 4e-3 * ref.norm()
     g.close()
+
+
+@pytest.mark.parametrize("n,M,N", [(2, 4096, 8192), (2, 2048, 16384), (8, 8192, 8192)])
+def test_own_tiles_followed_by_remote_ones(n, M, N):
+    """More than one panel of 16 column blocks and several tiles per pair and panel: a warp's own tile is followed by another owner's, and both go through its
+    staging buffers.  One k-block, so that the next accumulator is ready at once.  Operands of -1, 0, 1: partials are whole numbers up to 64 and sums up to
+    512, of which bf16 holds those up to 256 exactly and rounds the others once; every element is compared."""
+    from piccl_b200.parallel import tp
+    K = 64
+    g = _group(n, "gemm_rs", M, N, K)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    As, Bs = [[torch.randint(-1, 2, (rows, K), generator=gen, device="cuda").bfloat16() for _ in range(n)] for rows in (M, N)]
+    want = sum(a.float() @ b.float().t() for a, b in zip(As, Bs)).bfloat16()
+    outs = [torch.empty((M // n, N), device="cuda", dtype=torch.bfloat16) for _ in range(n)]
+    for rep in range(8):
+        for o in outs:
+            o.fill_(float("nan"))
+        tp.gemm_rs_group(g, As, Bs, outs)
+        torch.cuda.synchronize()
+        assert all(tp.tp_status(h) == 0 for h in g._hs)
+        assert torch.equal(torch.cat(outs), want), rep
+    g.close()
