@@ -133,7 +133,7 @@ def embed_fwd(idx, wte, wpe, out, seq: int):
 
 
 def wpe_bwd(dx, dwpe, batch: int, seq: int, accumulate: bool = False):
-    _chk(N.ops_lib().piccl_ops_wpe_bwd(_p(dx), _p(dwpe), batch, seq, dx.shape[1], int(accumulate), C.c_void_p(_s())), "wpe_bwd")
+    _chk(N.ops_lib().piccl_ops_wpe_bwd(_p(dx), _p(dwpe), batch, seq, seq, dx.shape[1], int(accumulate), C.c_void_p(_s())), "wpe_bwd")
     _bump()
 
 

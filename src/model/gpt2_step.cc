@@ -329,7 +329,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
     m.saved[l] = Saved();
     if (!fork) att[l] = at::Tensor();  // the second stream may still read it
   }
-  TRY(piccl_ops_wpe_bwd(dx, g_wpe, B, S, C, 0, s));
+  TRY(piccl_ops_wpe_bwd(dx, g_wpe, B, S, d.seq_len, C, 0, s));
   done(g_wpe, (size_t)d.seq_len * C);
   if (!m.stage.defined()) { m.stage = at::zeros({d.Vp, C}, opt.dtype(at::kFloat)); m.owner = at::zeros({d.Vp}, opt.dtype(at::kInt)); }
   if (fork) {

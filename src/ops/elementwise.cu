@@ -418,10 +418,12 @@ __global__ void __launch_bounds__(128) embed_fwd_kernel(const long long* __restr
   }
 }
 
-// dwpe[s, :] += sum over batch of dx[b*S + s, :]   (one block per position; deterministic)
+// dwpe[s, :] (+)= sum over batch of dx[b*S + s, :]   (one block per row of the table; deterministic).  Positions from S on, which no token
+// of this batch had, get the empty sum.
 __global__ void __launch_bounds__(128) wpe_bwd_kernel(const bf16* __restrict__ dx, bf16* __restrict__ dwpe, int B, int S, int C8, int accumulate) {
   pdl_begin();
   int s = blockIdx.x;
+  if (s >= S) B = 0;
   for (int i = threadIdx.x; i < C8; i += blockDim.x) {
     float acc[8];
 #pragma unroll
@@ -589,9 +591,10 @@ int piccl_ops_embed_fwd(const long long* idx, const void* wte, const void* wpe, 
   launch_pdl(embed_fwd_kernel, rows, 128, 0, (cudaStream_t)stream, idx, (const bf16*)wte, (const bf16*)wpe, (bf16*)out, rows, S, C / 8);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
-int piccl_ops_wpe_bwd(const void* dx, void* dwpe, int B, int S, int C, int accumulate, void* stream) {
-  if (C % 8) return -1;
-  launch_pdl(wpe_bwd_kernel, S, 128, 0, (cudaStream_t)stream, (const bf16*)dx, (bf16*)dwpe, B, S, C / 8, accumulate);
+// rows: rows of dwpe that are written, S or more
+int piccl_ops_wpe_bwd(const void* dx, void* dwpe, int B, int S, int rows, int C, int accumulate, void* stream) {
+  if (C % 8 || rows < S) return -1;
+  launch_pdl(wpe_bwd_kernel, rows, 128, 0, (cudaStream_t)stream, (const bf16*)dx, (bf16*)dwpe, B, S, C / 8, accumulate);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // stage: fp32 [V, C], zeroed by the caller

@@ -75,15 +75,14 @@ def test_replayed_steps_equal_issued_ones(layers, d_model, shapes):
             got = replayed.forward_backward(a, b)
             want = issued.forward_backward(a, b, on_grads_ready=lambda end: None)       # reports gradients: always issued call by call
             assert abs(float(got) - float(want)) <= 1e-5 * float(want)
-            n = torch.isnan(issued.flat_g)
-            assert torch.equal(torch.isnan(replayed.flat_g), n)
+            for m in (replayed, issued):              # every element is written, also for positions that no token had
+                assert not torch.isnan(m.flat_g).any() and not m.g["wpe"][S:].any()
             # the same kernels on the same operands: only sums by atomics (attention, embedding) come in another order, at worst another
             # rounding to bf16 (2^-8) of an element in each of the two halves of a layer
-            g, w = replayed.flat_g[~n].double(), issued.flat_g[~n].double()
+            g, w = replayed.flat_g.double(), issued.flat_g.double()
             assert float((g - w).norm()) <= 2 ** -7 * float(w.norm()), step
             want = issued._issue(a.reshape(-1), b.reshape(-1), B, S, True, 0)
             assert abs(float(replayed.loss(a, b)) - float(want)) <= 1e-5 * float(want)
-            replayed.flat_g[n] = 0.0                  # positions that no token had
             replayed.optimizer_step(lr=1e-4 * (step + 1))
             issued.flat_p.copy_(replayed.flat_p)
     assert replayed._graphs, "nothing was captured"
