@@ -75,6 +75,8 @@ struct Model {
   Desc d;
   std::vector<long long> off;
   at::Tensor arena;         // activations and workspace, grown to the largest shape so far
+  bool in_callers_graph = false;       // the caller captured launches that use this arena into a graph of its own
+  std::vector<at::Tensor> kept;        // such arenas, outgrown since: that graph may be replayed as long as the model lives
   at::Tensor stage, owner;  // fp32 table of embedding gradients (all zero between calls), one row of the batch per token id
   at::Tensor split;         // workspace of the products that split K
   void* ws[2] = {nullptr, nullptr};      // of the main and the second stream
@@ -196,6 +198,11 @@ void attention_grad(const Saved& sv, b16* dout, int B, int S, int H, int D, at::
   for (auto& t : d) if (t.stride(3) != 1) t = t.contiguous();
 }
 
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
 int run(Model& m, const long long* idx, const long long* tgt, int B, int S, float* loss, bool train, ReadyFn ready) {
   const Desc& d = m.d;
   const int T = B * S, C = d.C, L = d.L, H = d.H, D = C / H;
@@ -210,7 +217,13 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   Buffers b;
   Carve count{nullptr};
   carve(count, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
-  if (!m.arena.defined() || (size_t)m.arena.numel() < count.used) { m.arena = at::Tensor(); m.arena = at::empty({(int64_t)count.used}, opt.dtype(at::kByte)); }
+  if (!m.arena.defined() || (size_t)m.arena.numel() < count.used) {
+    if (m.in_callers_graph) m.kept.push_back(m.arena);
+    m.in_callers_graph = false;
+    m.arena = at::Tensor(); m.arena = at::empty({(int64_t)count.used}, opt.dtype(at::kByte));
+  }
+  // (captures of the model's own steps come with m.captured; models/gpt2.py drops those graphs when the arena moves)
+  m.in_callers_graph |= !m.captured && capturing(main_stream);
   Carve c{static_cast<char*>(m.arena.data_ptr())};
   carve(c, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
   b16 *const lnf_g = d.p + m.off[0], *const lnf_b = d.p + m.off[1], *const wpe = d.p + m.off[2], *const wte = d.p + m.off[3];
