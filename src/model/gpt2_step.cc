@@ -79,6 +79,7 @@ struct Model {
   std::vector<at::Tensor> kept;        // such arenas, outgrown since: that graph may be replayed as long as the model lives
   at::Tensor stage, owner;  // fp32 table of embedding gradients (all zero between calls), one row of the batch per token id
   at::Tensor split;         // workspace of the products that split K
+  bool split_zero = false, stage_zero = false;      // their zeros have been written, not only captured
   void* ws[2] = {nullptr, nullptr};      // of the main and the second stream
   Streams streams;
   cudaEvent_t ev_fork = nullptr, ev_layer[2] = {nullptr, nullptr};
@@ -223,16 +224,20 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
     m.arena = at::Tensor(); m.arena = at::empty({(int64_t)count.used}, opt.dtype(at::kByte));
   }
   // (captures of the model's own steps come with m.captured; models/gpt2.py drops those graphs when the arena moves)
-  m.in_callers_graph |= !m.captured && capturing(main_stream);
+  const bool in_capture = capturing(main_stream);
+  m.in_callers_graph |= !m.captured && in_capture;
   Carve c{static_cast<char*>(m.arena.data_ptr())};
   carve(c, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
   b16 *const lnf_g = d.p + m.off[0], *const lnf_b = d.p + m.off[1], *const wpe = d.p + m.off[2], *const wte = d.p + m.off[3];
   if (!m.split.defined()) {
     m.split = at::empty({2, (int64_t)kSplitBytes}, opt.dtype(at::kByte));
-    m.split.narrow(1, 0, 64 << 10).zero_();
     for (int q = 0; q < 2; q++) m.ws[q] = m.split.select(0, q).data_ptr();
     if (!take_streams(m.streams)) { g_error = "cudaStreamCreate failed"; return -1001; }
     for (cudaEvent_t* e : {&m.ev_fork, &m.ev_layer[0], &m.ev_layer[1]}) if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) { g_error = "cudaEventCreate failed"; return -1001; }
+  }
+  if (!m.split_zero) {                // in a capture the zeros come with every replay, and the next call writes them again
+    m.split.narrow(1, 0, 64 << 10).zero_();
+    m.split_zero = !in_capture;
   }
   if ((int)m.saved.size() < L) m.saved.resize(L);
 
@@ -344,7 +349,11 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   }
   TRY(piccl_ops_wpe_bwd(dx, g_wpe, B, S, d.seq_len, C, 0, s));
   done(g_wpe, (size_t)d.seq_len * C);
-  if (!m.stage.defined()) { m.stage = at::zeros({d.Vp, C}, opt.dtype(at::kFloat)); m.owner = at::zeros({d.Vp}, opt.dtype(at::kInt)); }
+  if (!m.stage.defined()) { m.stage = at::empty({d.Vp, C}, opt.dtype(at::kFloat)); m.owner = at::empty({d.Vp}, opt.dtype(at::kInt)); }
+  if (!m.stage_zero) {
+    m.stage.zero_();
+    m.stage_zero = !in_capture;
+  }
   if (fork) {
     cudaEventRecord(m.ev_fork, m.streams.side);
     cudaStreamWaitEvent(main_stream, m.ev_fork, 0);

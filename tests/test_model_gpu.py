@@ -112,3 +112,30 @@ def test_whole_step_graph_outlives_a_larger_evaluation():
             others = [torch.full((3 << 20,), 77, dtype=torch.uint8, device="cuda") for _ in range(32)]      # what the allocator has free among its large blocks
     torch.cuda.synchronize()
     assert all(bool((t == 77).all()) for t in others)
+
+
+def test_first_step_inside_a_callers_capture():
+    """A model whose very first step is captured by its user: steps issued before the first replay, and replays after them, start from zeroed workspaces."""
+    from piccl_b200.models.gpt2 import GPT2, GPT2Config
+    cfg = GPT2Config(vocab_size=1000, seq_len=128, n_layer=2, n_head=4, d_model=256)
+    tok = torch.randint(0, cfg.vocab_size, (8, cfg.seq_len + 1), generator=torch.Generator().manual_seed(8))
+    x, y = tok[:, :-1].contiguous().cuda(), tok[:, 1:].contiguous().cuda()
+    known = GPT2(cfg, seed=5)
+    want = known.forward_backward(x, y)                            # also sets the libraries up
+    fill = [torch.full((64 << 20,), 0x55, dtype=torch.uint8, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    del fill                                                       # what the allocator hands out now is not zero
+    model, graph = GPT2(cfg, seed=5), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        loss = model.forward_backward(x, y)
+    for issued in (True, False, False, True):
+        model.flat_g.fill_(float("nan"))
+        if issued:
+            loss2 = model.forward_backward(x, y)
+        else:
+            graph.replay()
+            loss2 = loss
+        assert abs(float(loss2) - float(want)) <= 1e-5 * float(want)
+        for name, g in known.g.items():                            # the same kernels; sums by atomics may round differently
+            d = (model.g[name].double() - g.double()).norm()
+            assert float(d) <= 2 ** -7 * float(g.double().norm()), (issued, name)
