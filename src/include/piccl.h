@@ -111,6 +111,8 @@ int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const voi
  * The *_group variants run several communicators of this process (virtual ranks on one device) as a
  * single cooperative launch. */
 long long piccl_tp_workspace_bytes(int which /*0 gemm_rs, 1 ag_gemm*/, int nranks, int M, int N, int K);
+/* Bytes [begin, end) of the 1 MiB flag area that a call of this shape uses, by the parity of the kernel's call count. */
+int piccl_tp_flag_range(int which, int nranks, int M, int N, int parity, long long* begin, long long* end);
 int piccl_gemm_rs(piccl_comm_t* c, const void* A, const void* B, void* out, int M, int N, int K_local, void* stream);
 int piccl_ag_gemm(piccl_comm_t* c, const void* A_shard, const void* B, void* out, int M, int N_local, int K, void* stream);
 int piccl_gemm_rs_group(piccl_comm_t** comms, int n, const void* const* A, const void* const* B, void* const* out, int M, int N, int K_local, void* stream);

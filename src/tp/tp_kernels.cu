@@ -52,6 +52,13 @@ __device__ __forceinline__ bool wait_flag(const unsigned* flag, unsigned epoch, 
   }
 }
 
+// The flag area of a rank's heap: half of it for each kernel, half of that for each parity of the kernel's call count, whatever the shape.  A
+// rank that is one call ahead, with another shape, then never writes a flag that a peer still waits for: waits look for
+// equality, so a flag of the next call in its place would be waited out.
+constexpr long long TP_FLAG_KERNEL = 512 << 10, TP_FLAG_CALL = TP_FLAG_KERNEL / 2;
+// bytes from the start of a kernel's half: flag t of the `per_src` that source rank src raises
+__host__ __device__ inline long long tp_flag_at(int parity, int src, long long per_src, long long t) { return parity * TP_FLAG_CALL + (src * per_src + t) * 4; }
+
 struct TpRank {
   CUtensorMap ta;            // gemm_rs: A [M, K_local];   ag_gemm: local shard [M/n, K]
   CUtensorMap ta2;           // ag_gemm: gathered buffer [2*M, K] in this rank's heap
@@ -115,7 +122,7 @@ struct RsPolicy {
   __device__ bool gate(int, volatile int*) const { return true; }
   __device__ int tile_id(int m_blk, int n_blk) const { return (m_blk % mb_per_owner) + n_blk * mb_per_owner; }
   __device__ unsigned* flag_ptr(int owner, int src, int t) const {
-    return reinterpret_cast<unsigned*>(R->heap[owner] + a.flag_off) + ((size_t)(parity * n + src) * tiles_per_owner + t);
+    return reinterpret_cast<unsigned*>(R->heap[owner] + a.flag_off + tp_flag_at(parity, src, tiles_per_owner, t));
   }
   // A tile travels as pieces of 32 rows x 64 columns: 4 KiB each, the 16-byte words of a row 512 bytes apart, so that both the
   // staging stores of the writer and the loads of the reader take consecutive words.  data_off: this call's half of the region.
@@ -286,7 +293,7 @@ struct AgPolicy {
   }
   __device__ const CUtensorMap* b_map() const { return &R->tb; }
   __device__ unsigned* flags(const TpRank* r, int dest, int src, int mb) const {
-    return reinterpret_cast<unsigned*>(r->heap[dest] + a.flag_off) + ((size_t)(parity * a.n + src) * mb_per_shard + mb) * a.n_part;
+    return reinterpret_cast<unsigned*>(r->heap[dest] + a.flag_off + tp_flag_at(parity, src, (long long)mb_per_shard * a.n_part, (long long)mb * a.n_part));
   }
   __device__ bool gate(int m_blk, volatile int* abort_flag) const {
     if (m_blk < 0 || m_blk / mb_per_shard == rank) return true;
@@ -379,8 +386,12 @@ static long long tp_need_per_call(int which, int nranks, int M, int N, int K) {
 // Flags per row block: 16 parts of 8 K bytes spread a block over as many CTAs (a power of two; fewer where the flag area would not hold them).
 static int ag_parts(int M) {
   int p = 16;
-  while (p > 1 && 2LL * (M / TP_BM) * p * 4 > (512 << 10)) p /= 2;
+  while (p > 1 && (M / TP_BM) * 4LL * p > TP_FLAG_CALL) p /= 2;
   return p;
+}
+static long long tp_flags_per_src(int which, int nranks, int M, int N) {
+  const long long blocks = M / nranks / TP_BM;
+  return which == 0 ? blocks * (N / TP_BN) : blocks * ag_parts(M);
 }
 
 static int tp_common_checks(piccl_comm** cs, int n, int M, int N, int K, int which) {
@@ -389,8 +400,7 @@ static int tp_common_checks(piccl_comm** cs, int n, int M, int N, int K, int whi
   if (c->nranks > TP_MAX_RANKS) return fail(PICCL_UNSUPPORTED, "fused tensor-parallel kernels support up to %d ranks", TP_MAX_RANKS);
   for (int i = 0; i < n; i++) if (!cs[i]->connected || cs[i]->broken) return fail(PICCL_INVALID_USAGE, "communicator not usable");
   if (M <= 0 || M % (TP_BM * c->nranks) || N % TP_BN || K % TP_BK || N <= 0 || K <= 0) return fail(PICCL_INVALID_ARGUMENT, "shape: M %% (128*ranks), N %% 256, K %% 64 must be 0");
-  const long long nflags = which == 0 ? 2LL * c->nranks * (M / c->nranks / TP_BM) * (N / TP_BN) : 2LL * c->nranks * (M / c->nranks / TP_BM) * ag_parts(M);
-  if (nflags * 4 > (512 << 10)) return fail(PICCL_UNSUPPORTED, "too many tiles for the flag area");
+  if (c->nranks * tp_flags_per_src(which, c->nranks, M, N) * 4 > TP_FLAG_CALL) return fail(PICCL_UNSUPPORTED, "too many tiles for the flag area");
   long long need = piccl_tp_workspace_bytes(which, c->nranks, M, N, K);
   if (tp_quarter(c->h_ctx.tp_bytes) < tp_need_per_call(which, c->nranks, M, N, K)) return fail(PICCL_INVALID_USAGE, "tensor-parallel workspace too small: %lld bytes needed, %lld configured (tp_bytes / PICCL_TP_MB)", need, c->h_ctx.tp_bytes);
   return PICCL_OK;
@@ -407,9 +417,9 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
   } guard(c0->device);
   TpArgs a; memset(&a, 0, sizeof a);
   a.n = nr; a.M = M; a.N = N; a.K = K;
-  a.flag_off = c0->h_ctx.tp_flag_off + (which ? (512 << 10) : 0);   // the two kernels keep their flags apart
+  a.flag_off = c0->h_ctx.tp_flag_off + (which ? TP_FLAG_KERNEL : 0);   // the two kernels keep their flags apart
   // ... and their payload: each kernel owns one half of the workspace, and each call one half of that, chosen by the parity of
-  // the kernel's own call count.  The strides do not depend on the shape: a rank that is one call ahead (the other kernel, or
+  // the kernel's own call count.  Neither these places nor the flags' depend on the shape: a rank that is one call ahead (the other kernel, or
   // the same kernel with another shape) never writes where a peer still reads the call before.
   const long long quarter = tp_quarter(c0->h_ctx.tp_bytes);
   const unsigned next_epoch = (which ? c0->tp_epoch_ag : c0->tp_epoch_rs) + 1;
@@ -470,6 +480,13 @@ extern "C" {
 long long piccl_tp_workspace_bytes(int which, int nranks, int M, int N, int K) {
   // four quarters (two kernels x two calls in flight), each large enough for one call of this shape
   return 4 * ((tp_need_per_call(which, nranks, M, N, K) + 1023) / 1024 * 1024);
+}
+int piccl_tp_flag_range(int which, int nranks, int M, int N, int parity, long long* begin, long long* end) {
+  if (which < 0 || which > 1 || nranks < 1 || nranks > TP_MAX_RANKS || M <= 0 || M % (TP_BM * nranks) || N <= 0 || N % TP_BN || parity < 0 || parity > 1) return fail(PICCL_INVALID_ARGUMENT, "no such call");
+  const long long per_src = tp_flags_per_src(which, nranks, M, N), base = which ? TP_FLAG_KERNEL : 0;
+  if (nranks * per_src * 4 > TP_FLAG_CALL) return fail(PICCL_UNSUPPORTED, "too many tiles for the flag area");
+  *begin = base + tp_flag_at(parity, 0, per_src, 0); *end = base + tp_flag_at(parity, nranks - 1, per_src, per_src - 1) + 4;
+  return PICCL_OK;
 }
 int piccl_gemm_rs(piccl_comm_t* c, const void* A, const void* B, void* out, int M, int N, int K_local, void* stream) {
   if (!c) return fail(PICCL_INVALID_ARGUMENT, "null communicator");

@@ -120,3 +120,29 @@ def test_rank_that_never_joins_is_reported_within_the_time_limit():
     assert results[1] == "left"
     assert results[0].startswith("error after"), results
     assert float(results[0].split()[2].rstrip("s:")) < 30
+
+
+def test_tensor_parallel_flags_of_neighbouring_calls_do_not_overlap():
+    """A rank may be one call ahead of a peer, of another shape or of the other kernel: no flag of the one call lies where the other's do."""
+    import ctypes as C
+    import itertools
+    from piccl_b200 import _native as N
+    lib = N.lib()
+
+    def flags(which, n, M, cols, parity):
+        lo, hi = C.c_longlong(), C.c_longlong()
+        rc = lib.piccl_tp_flag_range(which, n, M, cols, parity, C.byref(lo), C.byref(hi))
+        return (lo.value, hi.value) if rc == 0 else None
+
+    for n in range(1, 9):
+        shapes = [(128 * n * b, 256 * c) for b in (1, 2, 3, 8, 16, 61) for c in (1, 5, 32, 128)]
+        calls = {s: [[flags(w, n, *s, p) for p in (0, 1)] for w in (0, 1)] for s in shapes}
+        usable = [(s, w) for s in shapes for w in (0, 1) if calls[s][w][0] is not None]
+        assert len(usable) > len(shapes)
+        for (s, w), (t, v) in itertools.product(usable, usable):
+            for p, q in itertools.product((0, 1), (0, 1)):
+                if (w, p) == (v, q):
+                    continue
+                a, b = calls[s][w][p], calls[t][v][q]
+                assert 0 <= a[0] < a[1] <= 1 << 20
+                assert a[1] <= b[0] or b[1] <= a[0], (n, s, w, p, t, v, q)
