@@ -209,12 +209,13 @@ __global__ void __launch_bounds__(512) ce_fwd_bwd_kernel(bf16* __restrict__ logi
   }
 }
 
-// What a thread has seen of a row so far: maximum and sum of exp(x - maximum).
+// What a thread has seen of a row so far: maximum and sum of exp(x - maximum).  The maximum is taken off before the value is scaled to base 2:
+// one fma of both would round maximum * log2(e), and the sum would be off by that (3e-5 at logits around 400).
 struct OnlineSum {
   float m = -INFINITY, s = 0.f;
   static constexpr float kLog2e = 1.4426950408889634f;
-  __device__ __forceinline__ void add(const f32x2 x2, float mb, f32x2& a) {
-    float x, y; unpack2(fma2(x2, both2(kLog2e), both2(mb)), x, y);
+  __device__ __forceinline__ void add(const f32x2 x2, float neg_m, f32x2& a) {
+    float x, y; unpack2(mul2(add2(x2, both2(neg_m)), both2(kLog2e)), x, y);
     a = add2(a, pack2(ex2_approx(x), ex2_approx(y)));
   }
   template <int N> __device__ __forceinline__ void packs(const bf16x8 (&p)[N]) {
@@ -225,13 +226,13 @@ struct OnlineSum {
       for (int e = 0; e < 4; e++) q = __hmax2(q, p[u].v[e]);
     const float top = fmaxf(__low2float(q), __high2float(q));
     if (top > m) { s *= ex2_approx((m - top) * kLog2e); m = top; }               // at first 0 * exp(-inf)
-    const float mb = m == -INFINITY ? 0.f : -m * kLog2e;
+    const float neg_m = m == -INFINITY ? 0.f : -m;
     f32x2 a[2] = {both2(0.f), both2(0.f)};
 #pragma unroll
     for (int u = 0; u < N; u++) {
       float v[8]; unpack8(p[u], v);
 #pragma unroll
-      for (int e = 0; e < 8; e += 2) add(pack2(v[e], v[e + 1]), mb, a[(e >> 1) & 1]);
+      for (int e = 0; e < 8; e += 2) add(pack2(v[e], v[e + 1]), neg_m, a[(e >> 1) & 1]);
     }
     float x, y; unpack2(add2(a[0], a[1]), x, y);
     s += x + y;
@@ -255,18 +256,18 @@ __device__ __forceinline__ bf16x8 mask_padding(bf16x8 p, int col, int V) {
   for (int e = 0; e < 8; e++) if (col + e >= V) v[e] = -INFINITY;
   return pack8(v);
 }
-// exp(x - m) / s * gs of a pack; lb = -(m + log s) in base 2
-__device__ __forceinline__ bf16x8 ce_gradient(const bf16x8& p, float lb, float gs) {
+// exp(x - m) / s * gs of a pack; ls = -log2 s
+__device__ __forceinline__ bf16x8 ce_gradient(const bf16x8& p, float neg_m, float ls, float gs) {
   float v[8]; unpack8(p, v);
 #pragma unroll
   for (int e = 0; e < 8; e += 2) {
-    float x, y; unpack2(fma2(pack2(v[e], v[e + 1]), both2(OnlineSum::kLog2e), both2(lb)), x, y);
+    float x, y; unpack2(fma2(add2(pack2(v[e], v[e + 1]), both2(neg_m)), both2(OnlineSum::kLog2e), both2(ls)), x, y);
     unpack2(mul2(pack2(ex2_approx(x), ex2_approx(y)), both2(gs)), v[e], v[e + 1]);
   }
   return pack8(v);
 }
 // the target's column has gs less
-__device__ __forceinline__ bf16 ce_gradient_target(float x, float lb, float gs) { return __float2bfloat16_rn(ex2_approx(fmaf(x, OnlineSum::kLog2e, lb)) * gs - gs); }
+__device__ __forceinline__ bf16 ce_gradient_target(float x, float neg_m, float ls, float gs) { return __float2bfloat16_rn(ex2_approx(fmaf(x + neg_m, OnlineSum::kLog2e, ls)) * gs - gs); }
 
 // The same in one pass over memory: the sum of exponentials is taken while the row comes in, relative to the thread's maximum so far, and
 // the gradient needs the row once more, from shared memory.  GRAD = false leaves the logits as they are and keeps nothing.
@@ -304,12 +305,12 @@ __global__ void __launch_bounds__(512, 2) ce_row_kernel(bf16* __restrict__ logit
     o.packs(p);
   }
   o.block(sh);
-  if (owner) loss[row] = valid ? logf(o.s) + o.m - xt : 0.f;
+  if (owner) loss[row] = valid ? logf(o.s) + (o.m - xt) : 0.f;
   if (!GRAD) return;
-  const float lb = -o.m * OnlineSum::kLog2e - log2f(o.s);
+  const float ls = -log2f(o.s);
 #pragma unroll 1       // stores in bursts of four cost a quarter of the time
-  for (i = tid; i < n8; i += 512) lp[i] = ce_gradient(row_s[i], lb, valid ? gscale : 0.f);
-  if (valid && owner) reinterpret_cast<bf16*>(lp)[t] = ce_gradient_target(xt, lb, gscale);
+  for (i = tid; i < n8; i += 512) lp[i] = ce_gradient(row_s[i], -o.m, ls, valid ? gscale : 0.f);
+  if (valid && owner) reinterpret_cast<bf16*>(lp)[t] = ce_gradient_target(xt, -o.m, ls, gscale);
 }
 
 // out[0] = mean of x[0..n), one block

@@ -161,3 +161,24 @@ def test_cross_entropy_online(rows, V, Vp):
         want = 0.5 * ref_in.grad
         assert torch.all((lg[:, :V].double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5)
         assert lg[:, V:].abs().sum() == 0
+
+
+@pytest.mark.parametrize("offset", [0.0, 100.0, -400.0, 1000.0])
+def test_cross_entropy_does_not_depend_on_an_offset(offset):
+    """A common offset of the logits costs no precision: differences of bf16 values are exact in fp32.  Left are the roundings of the exponents (|x - max| log2 e <= 60,
+    weighted by the probabilities: below 2^-20), of the exponentials and their sum (2^-22, some 20 additions), of a logarithm up to 11 and of a loss up to 64 (2^-19)."""
+    from ctypes import c_float, c_void_p
+    from piccl_b200 import _native as N
+    rows, V, Vp = 512, 5003, 5120
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    logits = (torch.randn(rows, Vp, generator=gen, device="cuda") * 4 + offset).bfloat16()
+    tgt = torch.randint(0, V, (rows,), generator=gen, device="cuda")
+    ref_in = logits[:, :V].double().requires_grad_()
+    ref = F.cross_entropy(ref_in, tgt, reduction="none")
+    ref.sum().backward()
+    for grad in (0, 1):
+        loss, lg = torch.empty(rows, device="cuda"), logits.clone()
+        rc = N.ops_lib().piccl_ops_ce(c_void_p(lg.data_ptr()), c_void_p(tgt.data_ptr()), c_void_p(loss.data_ptr()), rows, V, Vp, c_float(1.0), grad, c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        assert float((loss.double() - ref.detach()).abs().max()) <= 6e-6
+    assert float((lg[:, :V].double() - ref_in.grad).norm()) <= 2 ** -9 * float(ref_in.grad.norm())
