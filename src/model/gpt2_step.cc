@@ -334,12 +334,22 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
     attention_grad(m.saved[l], b.datt, B, S, H, D, dq);
     const void* ptr[3]; long long st[9];
     for (int i = 0; i < 3; i++) { ptr[i] = dq[i].data_ptr(); for (int j = 0; j < 3; j++) st[3 * i + j] = dq[i].stride(j); }
-    TRY(piccl_ops_qkv_grad(ptr, st, dqkv, ws_qkv, B, S, H, D, s));
+    int n_q = n_qkv;
+    bool words = D % 8 == 0;          // rows of a head are whole 16-byte words
+    for (int i = 0; i < 3; i++) words &= (reinterpret_cast<uintptr_t>(ptr[i]) % 16 | (st[3 * i] | st[3 * i + 1] | st[3 * i + 2]) % 8) == 0;
+    if (words) TRY(piccl_ops_qkv_grad(ptr, st, dqkv, ws_qkv, B, S, H, D, s));
+    else {                            // heads of 4 columns, say: packed by ATen, the column sums from the packed rows
+      const at::Tensor packed = view(dqkv, {B, S, 3, H, D});
+      for (int i = 0; i < 3; i++) packed.select(2, i).copy_(dq[i].transpose(1, 2));
+      const int per = (T + n_qkv - 1) / n_qkv;
+      n_q = (T + per - 1) / per;
+      TRY(piccl_ops_colsum(dqkv, nullptr, ws_qkv, T, 3 * C, per, 0, s));
+    }
     DO(weight_grad(dqkv, y.ln1, m.g(l, W_QKV), 3 * C, C));
     DO(product(m, NN, dqkv, m.p(l, W_QKV), b.dln1, nullptr, T, C, 3 * C, s));
     TRY(piccl_ops_ln_bwd(b.dln1, l ? b.layer[l - 1].x3 : b.x0, m.p(l, LN1_G), y.mean1, y.rstd1, dxb, dx_below, ws1, l > 0, T, C, s));
     const piccl_finish_job jobs[8] = {{ws2, m.g(l, LN2_G), n_ln, C, 0, 0}, {ws2 + row, m.g(l, LN2_B), n_ln, C, 0, 0}, {ws2 + 2 * row, m.g(l, B_O), n_ln, C, 0, 0},
-                                      {ws_fc, m.g(l, B_FC), n_fc, 4 * C, 0, 0}, {ws_qkv, m.g(l, B_QKV), n_qkv, 3 * C, 0, 0}, {ws1, m.g(l, LN1_G), n_ln, C, 0, 0},
+                                      {ws_fc, m.g(l, B_FC), n_fc, 4 * C, 0, 0}, {ws_qkv, m.g(l, B_QKV), n_q, 3 * C, 0, 0}, {ws1, m.g(l, LN1_G), n_ln, C, 0, 0},
                                       {ws1 + row, m.g(l, LN1_B), n_ln, C, 0, 0}, {ws1 + 2 * row, l ? m.g(l - 1, B_PROJ) : nullptr, n_ln, C, 0, 0}};
     DO(finish(jobs, l ? 8 : 7, q));
     dx = dx_below;

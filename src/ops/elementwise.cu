@@ -530,12 +530,13 @@ int piccl_ops_finish_parts(const void* jobs, int n, void* stream) {
   launch_pdl(finish_parts_kernel, dim3((c + 31) / 32, n), 512, 0, (cudaStream_t)stream, a);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
-// workspace: ceil(rows / rows_per_block) * C floats
+// workspace: ceil(rows / rows_per_block) * C floats; out null: the partial rows are left there
 int piccl_ops_colsum(const void* x, void* out, float* workspace, int rows, int C, int rows_per_block, int accumulate, void* stream) {
   if (C % 8) return -1;
   int nparts = (rows + rows_per_block - 1) / rows_per_block;
   launch_pdl(colsum_kernel, dim3((C + 255) / 256, nparts), 256, 0, (cudaStream_t)stream, (const bf16*)x, workspace, rows, C, rows_per_block);
   PICCL_OPS_CHECK_LAUNCH();
+  if (!out) return 0;
   const FinishJob j{workspace, (bf16*)out, nparts, C, accumulate, 0};
   return piccl_ops_finish_parts(&j, 1, stream);
 }

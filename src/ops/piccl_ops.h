@@ -11,6 +11,7 @@ int piccl_ops_ln_bwd(const void* dy, const void* xin, const void* gamma, const f
 int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, void* pre, const void* bias, const void* aux, float* part, void* ws, size_t ws_bytes, int M, int N, int K, void* stream);
 int piccl_ops_bias_gelu_fwd(const void* h, const void* bias, void* h_out, void* g, long long rows, int C, void* stream);
 int piccl_ops_gelu_bwd(const void* dg, const void* h, void* dh, float* part, long long rows, int C, void* stream);
+int piccl_ops_colsum(const void* x, void* out, float* workspace, int rows, int C, int rows_per_block, int accumulate, void* stream);
 int piccl_ops_col_parts(long long rows, int C);
 int piccl_ops_qkv_grad(const void* const* g, const long long* strides, void* dqkv, float* part, int B, int S, int H, int D, void* stream);
 struct piccl_finish_job { const float* part; void* out; int nparts, C, accumulate, pad; };
