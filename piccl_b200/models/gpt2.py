@@ -161,6 +161,8 @@ class GPT2:
         targets = targets.reshape(-1).contiguous()
         if idx.dtype != torch.int64 or targets.dtype != torch.int64 or targets.numel() != B * S or S > self.cfg.seq_len:
             raise ValueError("token ids and targets are int64 tensors of one shape, at most seq_len long")
+        if self.cfg.d_model % self.cfg.n_head:      # the native step would take heads of d_model // n_head columns
+            raise RuntimeError(f"{self.cfg.d_model} columns are not {self.cfg.n_head} heads of one width")
         if on_grads_ready is not None and not loss_only:
             return self._issue(idx, targets, B, S, loss_only, 0, on_grads_ready), False
         key = (idx.data_ptr(), targets.data_ptr(), B, S, loss_only, gemm.backend_code())

@@ -146,3 +146,12 @@ def test_tensor_parallel_flags_of_neighbouring_calls_do_not_overlap():
                 a, b = calls[s][w][p], calls[t][v][q]
                 assert 0 <= a[0] < a[1] <= 1 << 20
                 assert a[1] <= b[0] or b[1] <= a[0], (n, s, w, p, t, v, q)
+
+
+def test_heads_of_unequal_width_are_refused():
+    from piccl_b200.models.gpt2 import GPT2, GPT2Config
+    model = GPT2(GPT2Config(vocab_size=100, seq_len=16, n_layer=1, n_head=30, d_model=256), device="cpu")
+    idx = torch.zeros(2, 16, dtype=torch.int64)
+    for run in (model.loss, model.forward_backward, lambda a, b: model.forward_backward(a, b, on_grads_ready=lambda end: None)):
+        with pytest.raises(RuntimeError, match="heads"):
+            run(idx, idx)
