@@ -178,7 +178,7 @@ class LoopbackGroup(_CommBase):
 
     def run(self, coll: str, send: Sequence[torch.Tensor], recv: Sequence[Optional[torch.Tensor]], count: int, op: str = "sum",
             root: int = 0, algo="RING", k: int = -1, stream=None):
-        rc = self._lib.piccl_group_collective(self.handles(), self.nranks, N.COLL[coll], self.table(send), self.table(recv), count, _dt(send[0]), N.OP[op], root, _algo(algo), k,
+        rc = self._lib.piccl_group_collective(self.handles(), self.nranks, N.COLL[coll], self._pack(*[t.data_ptr() for t in send]), self.table(recv), count, _dt(send[0]), N.OP[op], root, _algo(algo), k,
                                               _stream_ptr(stream))
         if rc:
             N.check(rc, f"piccl_group_collective({coll})")
@@ -190,7 +190,7 @@ class LoopbackGroup(_CommBase):
             self._comms = self._pack(*[h.value for h in self._hs])
         return self._comms
 
-    def table(self, tensors: Sequence[Optional[torch.Tensor]]) -> bytes:
+    def table(self, tensors: Sequence[Optional[torch.Tensor]]) -> bytes:      # None: a rank that receives nothing
         return self._pack(*[0 if t is None else t.data_ptr() for t in tensors])
 
     def status(self, rank: int = 0) -> N.Status:

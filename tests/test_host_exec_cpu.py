@@ -155,3 +155,28 @@ def test_heads_of_unequal_width_are_refused():
     for run in (model.loss, model.forward_backward, lambda a, b: model.forward_backward(a, b, on_grads_ready=lambda end: None)):
         with pytest.raises(RuntimeError, match="heads"):
             run(idx, idx)
+
+
+def test_a_group_call_without_an_operand_is_refused():
+    """A rank that receives nothing may have no receive buffer; every rank has something to send, and a missing tensor must not become a null pointer."""
+    import struct
+    from piccl_b200.parallel.comm import LoopbackGroup
+
+    class Stream:
+        cuda_stream = 0
+
+    class Recorder:
+        calls = 0
+
+        def piccl_group_collective(self, *args):
+            self.calls += 1
+            return 0
+
+    g = LoopbackGroup.__new__(LoopbackGroup)
+    g._lib, g.nranks, g._hs, g._comms, g._pack = Recorder(), 2, [], b"", struct.Struct("2Q").pack
+    a, b, stream = torch.ones(4), torch.ones(4), Stream()
+    g.run("reduce", [a, b], [a, None], 4, stream=stream)
+    assert g._lib.calls == 1
+    with pytest.raises(AttributeError):
+        g.run("reduce", [a, None], [a, b], 4, stream=stream)
+    assert g._lib.calls == 1
