@@ -84,7 +84,10 @@ def bias_gelu_fwd(h, bias, h_out, g):
 
 
 def gelu_bwd(dg, h, dh):
-    rows, Cc = h.shape
+    # element by element: any shape will do, as long as the kernel gets rows of whole 16-byte words
+    n = h.numel()
+    Cc = h.shape[1] if h.dim() == 2 and h.shape[1] % 8 == 0 else min(n & -n, 2048) or 8
+    rows = n // Cc
     _chk(N.ops_lib().piccl_ops_gelu_bwd(_p(dg), _p(h), _p(dh), C.c_void_p(0), C.c_longlong(rows), Cc, C.c_void_p(_s())), "gelu_bwd")
     _bump()
 

@@ -182,3 +182,20 @@ def test_cross_entropy_does_not_depend_on_an_offset(offset):
         assert rc == 0
         assert float((loss.double() - ref.detach()).abs().max()) <= 6e-6
     assert float((lg[:, :V].double() - ref_in.grad).norm()) <= 2 ** -9 * float(ref_in.grad.norm())
+
+
+@pytest.mark.parametrize("shape", [(4096,), (8,), (4, 8, 64), (16, 12), (3, 40), (0,), (0, 16), (5, 3, 24), (1, 4104)])
+def test_gelu_backward_of_any_shape(shape):
+    """Vectors, batches of matrices and rows that are no multiple of 16 bytes, in place too; one rounding to bf16 of a value that is exact to a few fp32 roundings."""
+    from piccl_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    h, dg = (torch.randn(shape, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    x = h.double().requires_grad_()
+    F.gelu(x, approximate="tanh").backward(dg.double())
+    dh = torch.empty_like(h)
+    ops.gelu_bwd(dg, h, dh)
+    assert torch.all((dh.double() - x.grad).abs() <= 2 ** -8 * x.grad.abs() + 2e-6 * dg.double().abs())
+    ops.gelu_bwd(dg, h, dg)
+    assert torch.equal(dg, dh)
+    with pytest.raises(RuntimeError):
+        ops.gelu_bwd(torch.ones(12, device="cuda").bfloat16(), torch.ones(12, device="cuda").bfloat16(), torch.ones(12, device="cuda").bfloat16())
