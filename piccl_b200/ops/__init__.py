@@ -66,8 +66,9 @@ class _FinishJob(C.Structure):
     _fields_ = [("part", C.c_void_p), ("out", C.c_void_p), ("nparts", C.c_int), ("C", C.c_int), ("accumulate", C.c_int), ("pad", C.c_int)]
 
 
-def layernorm_bwd(dy, xin, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate: bool = False):
-    """dx = dLN(dy) + dres; dgamma / dbeta (bf16) written or accumulated."""
+def layernorm_bwd(dy, xin, gamma, mean, rstd, dres, dx, dgamma, dbeta, accumulate: bool = False, rows_per_block: int = 32):
+    """dx = dLN(dy) + dres; dgamma / dbeta (bf16) written or accumulated.  `rows_per_block` is taken for callers that pass it: the kernel's
+    persistent grid splits the rows by itself."""
     rows, Cc = dy.shape
     n = N.ops_lib().piccl_ops_ln_bwd_parts(rows, Cc)
     ws = _workspace(2 * max(n, 1) * Cc, dy.device)

@@ -199,3 +199,16 @@ def test_gelu_backward_of_any_shape(shape):
     assert torch.equal(dg, dh)
     with pytest.raises(RuntimeError):
         ops.gelu_bwd(torch.ones(12, device="cuda").bfloat16(), torch.ones(12, device="cuda").bfloat16(), torch.ones(12, device="cuda").bfloat16())
+
+
+def test_layernorm_backward_takes_a_row_split():
+    from piccl_b200 import ops
+    rows, C = 70, 512
+    x, dy, gamma = _bf(rows, C, seed=1), _bf(rows, C, seed=2), _bf(C, seed=3)
+    mean, rstd = x.float().mean(1), (x.float().var(1, unbiased=False) + 1e-5).rsqrt()
+    got = []
+    for split in ((), (False, 16)):
+        out = [torch.empty_like(x), torch.empty_like(gamma), torch.empty_like(gamma)]
+        ops.layernorm_bwd(dy, x, gamma, mean, rstd, None, *out, *split)
+        got.append(out)
+    assert all(torch.equal(a, b) for a, b in zip(*got))
