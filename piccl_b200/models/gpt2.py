@@ -244,8 +244,15 @@ class GPT2:
 
     # ------------------------------------------------------------------ optimizer
     def optimizer_step(self, lr: float = 3e-4, betas=(0.9, 0.95), eps: float = 1e-8, weight_decay: float = 0.1) -> None:
-        """Fused AdamW over the flat buffers in one launch; the step number lives on the device so that it can be replayed."""
+        """Fused AdamW over the flat buffers in one launch (one per run of parameters in models of more than some 500 layers); the step number lives
+        on the device so that it can be replayed."""
         self.step_count += 1
+        if len(self.groups) > ops.MAX_ADAMW_RUNS:
+            self.step_dev.add_(1)
+            for b, e, decay in self.groups:
+                ops.adamw_devstep(self.flat_p[b:e], self.master[b:e], self.m[b:e], self.v[b:e], self.flat_g[b:e], lr, betas[0], betas[1], eps, weight_decay if decay else 0.0,
+                                  self.step_dev)
+            return
         ops.adamw_runs(self.flat_p, self.master, self.m, self.v, self.flat_g, self._run_ends, 0 if self.groups[0][2] else 1, lr, betas[0], betas[1], eps, weight_decay,
                        self.step_dev, self._ticket)
 

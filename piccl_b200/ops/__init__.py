@@ -122,6 +122,9 @@ def adamw_devstep(p, master, m, v, g, lr: float, b1: float, b2: float, eps: floa
     _bump()
 
 
+MAX_ADAMW_RUNS = 1024      # runs that the kernel keeps in shared memory (kMaxRuns)
+
+
 def adamw_runs(p, master, m, v, g, ends, decay_parity: int, lr: float, b1: float, b2: float, eps: float, wd: float, step_dev, ticket):
     """AdamW over flat buffers in one launch: run i ends before pack `ends[i]` of 8 elements (device int32), runs of parity `decay_parity` decay;
     `step_dev` (device int32, steps done so far) is advanced by the launch, `ticket` is a device int32 that holds zero."""

@@ -159,3 +159,28 @@ def test_narrow_heads(n_head, seq):
             for name, rg in ((f"h{l}.w_qkv", ref.h[l].attn["c_attn"].weight.grad), (f"h{l}.b_qkv", ref.h[l].attn["c_attn"].bias.grad), (f"h{l}.w_o", ref.h[l].attn["c_proj"].weight.grad)):
                 assert (mine.g[name].float() - rg).norm() <= 2e-2 * rg.norm(), (step, name)
     assert mine._graphs
+
+
+def test_optimizer_beyond_the_runs_of_one_launch(monkeypatch):
+    """Models with more runs of decaying and other parameters than one launch takes: a launch per run, the same update up to the rounding of a few fp32 operations."""
+    from piccl_b200 import ops
+    from piccl_b200.models.gpt2 import GPT2, GPT2Config
+    cfg = GPT2Config(vocab_size=500, seq_len=32, n_layer=1, n_head=4, d_model=256)
+    one, many = GPT2(cfg, seed=1), GPT2(cfg, seed=1)
+    for step in range(3):
+        g = torch.randn(one.n_params, generator=torch.Generator(device="cuda").manual_seed(step), device="cuda").bfloat16()
+        for m in (one, many):
+            m.flat_g.copy_(g)
+        one.optimizer_step(lr=1e-2)
+        with monkeypatch.context() as mp:
+            mp.setattr(ops, "MAX_ADAMW_RUNS", 2)
+            assert len(many.groups) > 2
+            many.optimizer_step(lr=1e-2)
+        assert int(one.step_dev) == int(many.step_dev) == step + 1
+        for a, b in ((one.master, many.master), (one.m, many.m), (one.v, many.v)):
+            assert torch.allclose(a, b, rtol=1e-5, atol=1e-7)
+    # and the native call refuses what does not fit
+    ends = torch.arange(1, ops.MAX_ADAMW_RUNS + 2, dtype=torch.int32, device="cuda")
+    p, f = torch.zeros(8 * ends.numel(), device="cuda", dtype=torch.bfloat16), [torch.zeros(8 * ends.numel(), device="cuda") for _ in range(3)]
+    with pytest.raises(RuntimeError):
+        ops.adamw_runs(p, *f, p, ends, 0, 1e-3, 0.9, 0.95, 1e-8, 0.1, one.step_dev, one._ticket)
