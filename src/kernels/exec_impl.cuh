@@ -34,8 +34,8 @@ __device__ __forceinline__ unsigned long long ld_acquire_sys(const unsigned long
   asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_sys(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void st_relaxed_sys(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ void fence_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -501,13 +501,13 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
     const int flags = s_step[d].flags, ai = s_step[d].action;
     if (flags & (STEP_END | STEP_FAIL)) break;
     const Action& ac = ai < kSliceCache ? s_act[ai] : L.actions[ai];
+    // one fence for both: what the data warps stored comes before the consumers' counters, what they read before the producers'
+    fence_sys();
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int p = lane + 32 * q;
-      // the slots are read (their packs went through registers before the barrier), so a plain store frees them: a release would wait for the
-      // acknowledgement of everything the CTA stored
-      for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) *reinterpret_cast<volatile unsigned long long*>(s_heap[p] + head_off + mine) = ++rcvd[q];
-      for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) st_release_sys(reinterpret_cast<unsigned long long*>(s_heap[p] + tail_off + mine), ++sent[q]);
+      for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) st_relaxed_sys(reinterpret_cast<unsigned long long*>(s_heap[p] + tail_off + mine), ++sent[q]);
+      for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) st_relaxed_sys(reinterpret_cast<unsigned long long*>(s_heap[p] + head_off + mine), ++rcvd[q]);
     }
     __syncwarp();
     if (lane == 0) { __threadfence_block(); s_published = k + 1; }
