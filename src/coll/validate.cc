@@ -1,6 +1,6 @@
 // CPU data-flow executor: runs the programs of all ranks against each other
-// exactly as the device kernel would (same CTA slicing, same per-step segment
-// interleaving, bounded FIFOs) and compares the buffers with a serial
+// in the order of the device kernel (same CTA slicing, same windows of segments,
+// bounded FIFOs) and compares the buffers with a serial
 // reduction.  The reference has no such check (it relies on the external OSU
 // validation flag, README.md:40-44).
 #include <cmath>
@@ -18,7 +18,7 @@ template <class T> T apply(int op, T a, T b) {
   switch (op) { case 0: return a + b; case 1: return a * b; case 2: return a > b ? a : b; default: return a < b ? a : b; }
 }
 
-struct Cursor { int seg = 0, maxseg = 0; size_t act = 0; bool done = false; };
+struct Cursor { int seg0 = 0, seg = 0, maxseg = 0; size_t act = 0; bool done = false; };      // window seg0, segment seg of it
 
 struct Sizes { int64_t in_elems, out_elems; };
 Sizes buffer_sizes(const CollArgs& a) {
@@ -31,8 +31,9 @@ Sizes buffer_sizes(const CollArgs& a) {
 }
 
 template <class T>
-ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer) {
+ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer, int window) {
   ValidateResult res;
+  if (window <= 0) window = window_of(fifo_cap);
   int n = a.nranks;
   int64_t st = a.block_stride ? a.block_stride : a.count;
   Sizes sz = buffer_sizes(a);
@@ -77,8 +78,8 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
     struct Entry { std::vector<T> data; int64_t n; };
     std::vector<std::deque<Entry>> fifo((size_t)n * n);   // [src*n+dst]
     std::vector<Cursor> cur(n);
-    // Deferred publishing (the executor's DEFER variant): a push is visible to the consumer, and a pop to the producer, only
-    // once the rank that made it has published it, which it does when it is about to block and when its program ends.
+    // Deferred publishing: a push is visible to the consumer, and a pop to the producer, only once the rank that made it has published it, at the
+    // latest when it is about to block and when its program ends (the executor's publisher is a warp of its own and may be that late).
     std::vector<int64_t> pushed((size_t)n * n, 0), popped((size_t)n * n, 0), pub_push((size_t)n * n, 0), pub_pop((size_t)n * n, 0);
     auto flush = [&](int r) {
       bool any = false;
@@ -89,7 +90,7 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
       }
       return any;
     };
-    // device order: outer loop over segments, inner loop over all actions of the program
+    // device order: for each window of segments, for each action of the program, for each segment of the window
     for (int r = 0; r < n; r++) {
       for (auto& ac : progs[r].actions) cur[r].maxseg = std::max(cur[r].maxseg, slice_of(ac.count, a.elem_size, cta, n_cta, slot_bytes).nseg);
       cur[r].done = cur[r].maxseg == 0;
@@ -158,8 +159,9 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
             }
           }
           if (!advance) break;
-          c.act++;
-          if (c.act >= p.actions.size()) { c.act = 0; c.seg++; if (c.seg >= c.maxseg) { c.done = true; progress = true; if (defer) flush(r); } }
+          if (++c.seg < c.seg0 + window) continue;
+          if (++c.act >= p.actions.size()) { c.act = 0; c.seg0 += window; if (c.seg0 >= c.maxseg) { c.done = true; progress = true; if (defer) flush(r); } }
+          c.seg = c.seg0;
         }
       }
     }
@@ -225,13 +227,13 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
 
 }  // namespace
 
-ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish) {
-  if (integer) return run<int32_t>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish);
-  return run<float>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish);
+ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish, int window) {
+  if (integer) return run<int32_t>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window);
+  return run<float>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window);
 }
 
-ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish) {
-  return run<float>(a, 0, false, fifo_cap, (int64_t)(256 * 1024) / a.elem_size, n_cta, defer_publish);
+ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish, int window) {
+  return run<float>(a, 0, false, fifo_cap, (int64_t)(256 * 1024) / a.elem_size, n_cta, defer_publish, window);
 }
 
 }  // namespace piccl

@@ -6,7 +6,7 @@
 // directed rank pair and CTA), so a program is correct iff, for every
 // connection, the k-th entry pushed by the sender is the k-th entry popped by
 // the receiver.  The validator (validate.cc) checks exactly that, with bounded
-// FIFO capacity, on real data.
+// FIFO capacity and in the executor's order of segments and actions, on real data.
 //
 // Reference parity: the schedules reproduce the send/recv patterns of
 // src/coll/{allgather,allreduce,broadcast,reduce,reduce_scatter}.c of the
@@ -127,12 +127,14 @@ struct ValidateResult {
 // seed 0; int32 in [-1000,1000] when integer=true) with FIFOs of `fifo_cap`
 // entries and segments of `seg_elems` elements, and compares with a serial
 // reduction.  op: 0 sum, 1 prod, 2 max, 3 min.
-// defer_publish models the executor variant that holds its counter updates back until it is about to block (exec_impl.cuh).
-ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish = false);
+// defer_publish: counters are published as late as can be, when the rank is about to block.  The executor's publisher works behind the warps that
+// wait and move data; what terminates when it is this late terminates whenever it comes.
+// window: segments that are walked together (0: as many as the executor walks with a FIFO of fifo_cap entries).
+ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish = false, int window = 0);
 
 // Symbolic check for sizes too large to materialise: coverage of every output
 // element and FIFO order, no data.
-ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish = false);
+ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish = false, int window = 0);
 
 // ---- dumps ----
 // Transfers in the reference's schedule XML format

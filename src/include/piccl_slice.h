@@ -30,4 +30,8 @@ PICCL_HD Slice slice_of(int64_t count, int elem_size, int cta, int n_cta, int64_
   return s;
 }
 
+// Segments that the executor walks together: for each window of segments, for each action, for each segment of the window.  Two where the FIFO has
+// slots for it: every segment of a window may have an entry in flight and one that the next action sends before it is consumed.
+PICCL_HD int window_of(int nslot) { return nslot >= 4 ? 2 : 1; }
+
 }  // namespace piccl

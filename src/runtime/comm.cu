@@ -8,6 +8,7 @@
 // whatever the caller has (real NCCL in the preload shim, torch.distributed
 // in the Python package, a pipe in the benchmark).
 #include "comm.h"
+#include "../include/piccl_slice.h"
 #include "nvls.h"
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
@@ -397,14 +398,14 @@ static int exec_block(const piccl_comm* c) { return c->cfg.block_size + kCtlThre
 // a message is cut into two where it can be.  Ranks in launches of their own keep the communicator's slots: they may be a call apart.
 static void cut_fifo(const piccl_comm* c, int n_vrank, int n_cta, const CollArgs& a, KernelArgs* ka) {
   const RankCtx& x = c->h_ctx;
-  ka->seg_bytes = x.slot_bytes; ka->nslot = x.nslot; ka->window = x.nslot >= 4 ? 2 : 1;
+  ka->seg_bytes = x.slot_bytes; ka->nslot = x.nslot; ka->window = window_of(x.nslot);
   if (n_vrank != c->nranks || n_vrank < 2) return;
   const long long chan = x.nslot * x.slot_bytes, round = (long long)c->cfg.block_size * 64;
   long long slice = a.count * a.elem_size;
   if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) slice /= c->nranks;
   slice = (slice + n_cta - 1) / n_cta;
   const long long seg = std::min<long long>(round_up((slice + 1) / 2, round), std::max<long long>(round, 131072 / round * round));
-  ka->nslot = 4; ka->window = 2;
+  ka->nslot = 4; ka->window = window_of(4);
   ka->seg_bytes = std::max<long long>(16, std::min<long long>(seg, chan / 4 / 16 * 16));
 }
 

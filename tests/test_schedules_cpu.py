@@ -23,12 +23,30 @@ def test_all_rank_counts_and_radices(coll, algo):
 
 @pytest.mark.parametrize("algo", ALGOS)
 def test_deferred_counter_updates_never_deadlock(algo):
-    """The executor variant that publishes its FIFO counters only when it is about to block (exec_impl.cuh, DEFER):
+    """The executor publishes its FIFO counters behind the data it moves (exec_impl.cuh).  Published as late as can be, when the rank is about to block:
     every schedule still terminates with the right data, also with the smallest FIFO."""
     for coll in COLLS:
         for n, k, in_place in itertools.product([2, 3, 4, 6, 8, 9, 16], [-1, 2, 4, 8], [False, True]):
             v = S.validate(coll, algo, n, 257, k=k, root=n - 1, in_place=in_place, n_cta=2, seg_elems=32, fifo_cap=2, deferred=True)
             assert v.ok, f"{coll} {algo} n={n} k={k} in_place={in_place}: {v.error}"
+
+
+@pytest.mark.parametrize("coll", COLLS)
+@pytest.mark.parametrize("algo", ALGOS)
+def test_windows_of_segments_never_deadlock(coll, algo):
+    """The executor's order with the FIFOs it uses: one segment at a time below four slots, windows of two from there on; one, an odd and an even number of
+    segments, counters published at once and as late as can be."""
+    for n, k, in_place in itertools.product([2, 3, 4, 6, 7, 8, 9, 16], [-1, 2, 4, 8], [False, True]):
+        for fifo, count, deferred in itertools.product([3, 4, 5], [30, 32 * 2 * 3 * n, 257], [False, True]):
+            v = S.validate(coll, algo, n, count, k=k, root=n - 1, in_place=in_place, n_cta=2, seg_elems=32, fifo_cap=fifo, deferred=deferred)
+            assert v.ok, f"{coll} {algo} n={n} k={k} in_place={in_place} fifo={fifo} count={count} deferred={deferred}: {v.error}"
+
+
+def test_a_window_needs_its_slots():
+    """Two segments to a window with one slot for each: a rank that receives and forwards waits for a slot that only its own later step frees."""
+    assert S.validate("allreduce", "RING", 4, 2048, n_cta=1, seg_elems=32, fifo_cap=4, window=2).ok
+    v = S.validate("allreduce", "RING", 4, 2048, n_cta=1, seg_elems=32, fifo_cap=2, window=2)
+    assert not v.ok and "deadlock" in v.error
 
 
 @pytest.mark.parametrize("op", ["sum", "prod", "max", "min"])
