@@ -376,8 +376,9 @@ static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
   if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) bytes /= std::max(1, a.nranks);
   if (a.algo == ALGO_DIRECT && a.coll != COLL_ALLGATHER && a.coll != COLL_REDUCE_SCATTER) bytes /= std::max(1, a.coll == COLL_ALLREDUCE ? a.nranks : a.nranks - 1);
   const Env& e = env();
-  // (virtual ranks on one device, whose steps cost less than a way over NVLink: 280 KB among eight ranks 42 us at 32 KiB a CTA, 35 at 16)
-  const long long per = n_vrank > 1 ? 16384 : 32768;
+  // (all ranks in one launch, whose steps cost less than a way over NVLink: 280 KB among eight ranks 42 us at 32 KiB a CTA, 35 at 16.  Part of the ranks
+  // in one launch: the others may be in launches of other sizes and have to come to the same number)
+  const long long per = n_vrank > 1 && n_vrank == c->nranks ? 16384 : 32768;
   long long n = (bytes + per - 1) / per;
   if (e.min_grid_set || e.max_grid_set) {
     long long g = a.count / std::max(1, c->cfg.block_size);
