@@ -1,7 +1,5 @@
-"""CTA-pair GEMM (src/ops2/gemm_sm100_2cta.cu, `tcgen05.mma.cta_group::2`) against a PyTorch fp32 reference.
-The kernel has not run on a GPU yet, so the test only runs when PICCL_TEST_PAIR_GEMM=1 asks for it; every wait in the kernel
-is bounded and a wait that ran out is reported through the status word."""
-import os
+"""The GEMM on CTA pairs (src/include/sm100_gemm_pair.cuh, `tcgen05.mma.cta_group::2`) at whole tiles, one to many per pair, against a PyTorch
+fp32 reference; every wait in the kernel is bounded and a wait that ran out is reported through the status word."""
 import sys
 from pathlib import Path
 
@@ -9,7 +7,7 @@ import pytest
 import torch
 
 sys.path.insert(0, str(Path(__file__).resolve().parent.parent))
-pytestmark = [pytest.mark.gpu, pytest.mark.skipif(os.environ.get("PICCL_TEST_PAIR_GEMM") != "1", reason="set PICCL_TEST_PAIR_GEMM=1 to run the CTA-pair GEMM")]
+pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,N,K,with_bias", [(256, 256, 64, False), (256, 256, 512, True), (512, 768, 1024, False), (8192, 1024, 1024, True), (2048, 4096, 3584, False)])

@@ -78,10 +78,12 @@ def test_replayed_steps_equal_issued_ones(layers, d_model, shapes):
             assert abs(float(got) - float(want)) <= 1e-5 * float(want)
             for m in (replayed, issued):              # every element is written, also for positions that no token had
                 assert not torch.isnan(m.flat_g).any() and not m.g["wpe"][S:].any()
-            # the same kernels on the same operands: only sums by atomics (attention, embedding) come in another order, at worst another
-            # rounding to bf16 (2^-8) of an element in each of the two halves of a layer
-            g, w = replayed.flat_g.double(), issued.flat_g.double()
-            assert float((g - w).norm()) <= 2 ** -7 * float(w.norm()), step
+            # every gradient by itself: those of gains and biases are a small part of the whole, and a wait that is missing between the streams may spoil
+            # one of them alone.  The sums are the same up to the order of a few (attention and embedding by atomics, products of another back end): at
+            # worst another rounding to bf16 (2^-8) of an element in each of the two halves of a layer
+            for name, w in issued.g.items():
+                d = (replayed.g[name].double() - w.double()).norm()
+                assert float(d) <= 2 ** -7 * float(w.double().norm()), (step, name)
             want = issued._issue(a.reshape(-1), b.reshape(-1), B, S, True, 0)
             assert abs(float(replayed.loss(a, b)) - float(want)) <= 1e-5 * float(want)
             replayed.optimizer_step(lr=1e-4 * (step + 1))
