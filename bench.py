@@ -221,6 +221,11 @@ def run_collectives(world: int):
 
 
 # ------------------------------------------------------------------------------------------------ our arm
+def replay_share(replayed: int, steps: int) -> str:
+    """How the steps of a region, warm-up included, were launched."""
+    return f"{replayed} of {steps} steps replayed from a CUDA graph, the others issued call by call" if replayed else "issued call by call"
+
+
 def run_piccl(args):
     import torch
     rank, world, local = dist_env()
@@ -258,10 +263,12 @@ def run_piccl(args):
         return trainer.step(a, b)
 
     sampler = ClockSampler(local).start() if rank == 0 else None
-    l0 = trainer.kernel_launches()
+    l0, r0 = trainer.kernel_launches(), trainer.replayed_steps()
     ms_dev, _, last = timed_region(step_dev, args.steps, args.warmup, world)
     launches = (trainer.kernel_launches() - l0) // max(1, args.steps + args.warmup) * args.steps
+    r1 = trainer.replayed_steps()
     ms_e2e, wall_e2e, last_loss = timed_region(step_e2e, args.steps, max(1, args.warmup // 2), world)
+    launch_mode = f"device-timed: {replay_share(r1 - r0, args.steps + args.warmup)}; end to end: {replay_share(trainer.replayed_steps() - r1, args.steps + max(1, args.warmup // 2))}"
     clocks = sampler.stop() if sampler else None
     h2d = 2 * args.micro_batch * cfg.seq_len * 8
     comm_stats = None
@@ -269,7 +276,6 @@ def run_piccl(args):
         st = comm.stats()
         comm_stats = {"allreduce_calls": int(st.calls[1]), "in_switch_calls": int(st.nvls_calls), "kernel_launches": int(st.launches)}
     algo_name = trainer.averager.algo
-    launch_mode = "CUDA graph replay" if trainer.use_graph else "forward and backward replayed from a CUDA graph, AdamW launched" if world == 1 else "eager"
     gemm_counts = None
     if rank == 0:
         from piccl_b200.ops import gemm

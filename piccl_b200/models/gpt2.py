@@ -111,6 +111,7 @@ class GPT2:
         self._arena = None
         self._graphs: dict = {}      # captured steps, at most _MAX_GRAPHS, which share the memory of their attention outputs
         self._graph_pool = None
+        self.replays = 0             # steps replayed so far
         self._seen: dict = {}        # how often a step was issued call by call; -1: it cannot be captured
         self._counts = (C.c_longlong * 4)()
 
@@ -188,6 +189,7 @@ class GPT2:
             return self._issue(idx, targets, B, S, loss_only, int(seen == 1)), False
         graph, loss, counts = entry
         graph.replay()
+        self.replays += 1
         ops._bump(counts[0])
         gemm.count(counts[1], counts[2])
         return loss, True

@@ -36,8 +36,8 @@ class DataParallelTrainer:
         self._tgt = None
         # CUDA graph of the whole step (forward, backward with overlapped bucket reductions, AdamW): after two eager steps
         # the launches are captured once and replayed, which removes the per-launch host cost (about a thousand launches).
-        # Off unless asked for (PICCL_TRAIN_GRAPH=1 or use_graph=True), on one GPU and on several alike, so that step times at
-        # different GPU counts compare the same launch mode.
+        # Off unless asked for (PICCL_TRAIN_GRAPH=1 or use_graph=True).  Without it a step that averages gradients is issued call by call, and
+        # one on a single GPU may replay its forward and backward pass (GPT2._step): replayed_steps() tells what happened.
         env_graph = os.environ.get("PICCL_TRAIN_GRAPH")
         default_graph = env_graph == "1"
         self.use_graph = default_graph if use_graph is None else use_graph
@@ -100,6 +100,10 @@ class DataParallelTrainer:
         self._loss_host.copy_(loss.reshape(1), non_blocking=True)
         torch.cuda.current_stream().synchronize()
         return float(self._loss_host[0])
+
+    def replayed_steps(self) -> int:
+        """Steps so far whose forward and backward pass, or all of whose launches (`use_graph`), came from a CUDA graph."""
+        return self._replayed + self.model.replays
 
     def kernel_launches(self) -> int:
         """Launches of this framework's own kernels so far (model kernels + collective executor); a replayed step

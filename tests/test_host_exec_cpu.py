@@ -180,3 +180,9 @@ def test_a_group_call_without_an_operand_is_refused():
     with pytest.raises(AttributeError):
         g.run("reduce", [a, None], [a, b], 4, stream=stream)
     assert g._lib.calls == 1
+
+
+def test_bench_names_the_launch_mode_from_what_happened():
+    import bench
+    assert bench.replay_share(0, 23) == "issued call by call"
+    assert bench.replay_share(21, 23).startswith("21 of 23 steps replayed")
