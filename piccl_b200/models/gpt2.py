@@ -40,6 +40,16 @@ class _Desc(C.Structure):       # the native step's description of a model (src/
     _fields_ = [(n, C.c_int) for n in ("L", "C", "H", "V", "Vp", "seq_len")] + [("eps", C.c_float), ("pad", C.c_int), ("p", C.c_void_p), ("g", C.c_void_p), ("off", C.c_void_p)]
 
 
+# What a program may switch between two steps and attention or the library products look at in each call: a step captured under one setting is not
+# replayed under another.  (The functions behind the torch.backends properties, which take three times as long: half a microsecond.)
+_SETTINGS = [getattr(torch._C, f"_get_{n}") for n in ("cudnn_sdp_enabled", "flash_sdp_enabled", "mem_efficient_sdp_enabled", "math_sdp_enabled", "deterministic_algorithms",
+                                                      "cublas_allow_bf16_reduced_precision_reduction")]
+
+
+def _library_settings() -> tuple:
+    return tuple([f() for f in _SETTINGS])
+
+
 @dataclass
 class GPT2Config:
     vocab_size: int = 50257
@@ -166,7 +176,7 @@ class GPT2:
             raise RuntimeError(f"{self.cfg.d_model} columns are not {self.cfg.n_head} heads of one width")
         if on_grads_ready is not None and not loss_only:
             return self._issue(idx, targets, B, S, loss_only, 0, on_grads_ready), False
-        key = (idx.data_ptr(), targets.data_ptr(), B, S, loss_only, gemm.backend_code())
+        key = (idx.data_ptr(), targets.data_ptr(), B, S, loss_only, gemm.backend_code(), _library_settings())
         seen = self._seen.get(key, 0)
         if seen == -1 or torch.cuda.is_current_stream_capturing():
             return self._issue(idx, targets, B, S, loss_only, 0), False

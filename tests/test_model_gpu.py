@@ -186,3 +186,26 @@ def test_optimizer_beyond_the_runs_of_one_launch(monkeypatch):
     p, f = torch.zeros(8 * ends.numel(), device="cuda", dtype=torch.bfloat16), [torch.zeros(8 * ends.numel(), device="cuda") for _ in range(3)]
     with pytest.raises(RuntimeError):
         ops.adamw_runs(p, *f, p, ends, 0, 1e-3, 0.9, 0.95, 1e-8, 0.1, one.step_dev, one._ticket)
+
+
+def test_a_captured_step_is_not_replayed_under_other_library_settings():
+    """Attention back ends (a context manager) and deterministic algorithms are looked up in each call; a graph holds what was chosen at its capture."""
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    from piccl_b200.models.gpt2 import GPT2, GPT2Config
+    cfg = GPT2Config.tiny()
+    m = GPT2(cfg, seed=1)
+    tok = torch.randint(0, cfg.vocab_size, (2, cfg.seq_len + 1), generator=torch.Generator().manual_seed(0)).cuda()
+    a, b = tok[:, :-1].contiguous(), tok[:, 1:].contiguous()
+    for _ in range(4):
+        want = float(m.forward_backward(a, b))
+    assert m.replays == 2
+    with sdpa_kernel(SDPBackend.MATH):
+        assert abs(float(m.forward_backward(a, b)) - want) <= 1e-3 * want
+    assert m.replays == 2
+    torch.use_deterministic_algorithms(True, warn_only=True)
+    try:
+        assert abs(float(m.forward_backward(a, b)) - want) <= 1e-3 * want
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert m.replays == 2
+    assert float(m.forward_backward(a, b)) == want and m.replays == 3
