@@ -1,11 +1,13 @@
 """Matrix products of the model: y = x W^T (+ bias), dx = dy W, dW = dy^T x.
 
-Back ends, chosen once per process (`set_backend`):
-  "auto"     (default) the better one for the product at hand: this framework's kernel for small products and
-             wherever its epilogue saves a pass (GELU and its derivative), cuBLAS for large plain ones
+Back ends, chosen once per process (`set_backend`), of the native training step (src/model/gpt2_step.cc) and of the functions below:
+  "auto"     (default) this framework's kernel wherever its epilogue saves a pass (GELU and its derivative); of the plain
+             products the step gives it the small ones, by their operations, and cuBLAS the large; the functions below
+             leave all plain products to cuBLAS
   "tcgen05"  this framework's sm_100a kernel (src/ops/gemm_sm100.cu: TMA -> shared memory ->
-             tcgen05.mma with TMEM accumulators) for every product of the training step
-  "cublas"   cuBLAS through torch.mm / torch.addmm for all three
+             tcgen05.mma with TMEM accumulators) for every product that it supports
+  "cublas"   cuBLAS
+The step issues its products itself and reports their number through `count`; the functions are for programs that put a model together from Python.
 """
 from __future__ import annotations
 
@@ -43,8 +45,8 @@ def count(tcgen05: int, cublas: int) -> None:
 
 
 def _own_kernel_ok(x, w, out, fused_epilogue: bool = False) -> bool:
-    """"auto": the tcgen05 kernel where its fused epilogue saves a pass over the activations (GELU and its derivative);
-    plain products stay on cuBLAS.  "tcgen05": wherever supported."""
+    """"auto": the tcgen05 kernel where its fused epilogue saves a pass over the activations (GELU); plain products stay on cuBLAS.
+    "tcgen05": wherever supported."""
     if _backend == "cublas" or (_backend == "auto" and not fused_epilogue):
         return False
     from . import gemm_sm100

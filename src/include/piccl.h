@@ -104,7 +104,7 @@ int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const voi
 
 /* ---- fused tensor-parallel kernels (tcgen05 GEMM + peer-memory collective in one kernel) ----
  * All operands bf16, row-major, contiguous, 16-byte aligned.  The communicator needs tp_bytes >=
- * piccl_tp_workspace_bytes(...).  M % (128 * nranks) == 0, N % 256 == 0 (N_local % 128), K % 64 == 0.
+ * piccl_tp_workspace_bytes(...).  M % (128 * nranks) == 0, N % 256 == 0 (N_local too), K % 64 == 0.
  *
  * piccl_gemm_rs:  out[M/n, N] = rows [rank*M/n, (rank+1)*M/n) of  sum_r A_r[M, K_local] * B_r[N, K_local]^T
  * piccl_ag_gemm:  out[M, N_local] = concat_r(A_r[M/n, K]) * B[N_local, K]^T

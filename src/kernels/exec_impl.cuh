@@ -49,7 +49,6 @@ __device__ __forceinline__ uint4 ld_slot(const void* p) {
   asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ uint4 ld_local(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ void st_vec(void* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
 
 // ---------------------------------------------------------------- element-wise maths
@@ -241,8 +240,8 @@ static __device__ __noinline__ void store_part(char* p, const uint4 v, int from,
 // The same movement where the local operand (source index local_src) or dst[0] is at any byte address: an unaligned source is read as the
 // two aligned words around each pack (the second one is the neighbour's first and hits L2), an unaligned destination is written as aligned
 // words too, put together from a lane's pack and the one before it.  Only the two ends of the run of packs that a warp
-// writes (kRun blocks of 512 bytes) go out in bytes.  (An element at a time, the path before, moved 1 MiB blocks of a
-// four-rank all-gather in 171 us.)
+// writes (kRun blocks of 512 bytes) go out in bytes.  (1 MiB blocks at odd
+// addresses, all-gather of four ranks: 30 us; an element at a time 171.)
 // An aligned word that is read may reach up to 15 bytes beyond the operand's ends; it never leaves the 16-byte granule of a byte that
 // belongs to the operand, and allocations are whole granules.
 constexpr int kRun = 4;
@@ -314,7 +313,7 @@ __device__ __noinline__ void reduce_copy_shift(int nsrc, const char* const* src,
   }
 }
 
-// Element-wise path: the last, partial pack of an action (and unaligned buffers in the deferring variant).
+// Element-wise path: the last, partial pack of an action.
 template <typename T, int OP>
 __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
                                                  long long first, long long nelem, bool do_scale, float scale) {

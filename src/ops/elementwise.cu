@@ -363,8 +363,8 @@ __global__ void __launch_bounds__(256) adamw_kernel(bf16* __restrict__ p, float*
   }
 }
 
-// AdamW over all parameters in one launch: run g of the flat buffers ends before pack ends[g] (8 elements), odd runs of `first_decay`
-// parity decay.  The step number is the device's own (*step holds the steps done so far); the last block to finish advances it.
+// AdamW over all parameters in one launch: run g of the flat buffers ends before pack ends[g] (8 elements), runs of parity
+// `decay_parity` decay.  The step number is the device's own (*step holds the steps done so far); the last block to finish advances it.
 constexpr int kMaxRuns = 1024;
 __global__ void __launch_bounds__(256) adamw_runs_kernel(bf16* __restrict__ p, float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
                                                          const bf16* __restrict__ g, const int* __restrict__ ends, int nruns, int decay_parity, size_t n8,
