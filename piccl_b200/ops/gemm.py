@@ -44,18 +44,18 @@ def count(tcgen05: int, cublas: int) -> None:
     _counts["cublas"] += cublas
 
 
-def _own_kernel_ok(x, w, out, fused_epilogue: bool = False) -> bool:
+def _own_kernel_ok(x, w, out, *others, fused_epilogue: bool = False) -> bool:
     """"auto": the tcgen05 kernel where its fused epilogue saves a pass over the activations (GELU); plain products stay on cuBLAS.
-    "tcgen05": wherever supported."""
+    "tcgen05": wherever supported.  The kernel needs operands that start on a 16-byte boundary."""
     if _backend == "cublas" or (_backend == "auto" and not fused_epilogue):
         return False
     from . import gemm_sm100
-    return gemm_sm100.available() and gemm_sm100.supports(x, w, out)
+    return gemm_sm100.available() and gemm_sm100.supports(x, w, out) and all(t is None or t.data_ptr() % 16 == 0 for t in (x, w, out, *others))
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias, out: torch.Tensor) -> torch.Tensor:
     """out[M, N] = x[M, K] @ w[N, K]^T + bias[N]"""
-    if _own_kernel_ok(x, w, out):
+    if _own_kernel_ok(x, w, out, bias):
         from . import gemm_sm100
         gemm_sm100.gemm(gemm_sm100.NT, gemm_sm100.BIAS, x, w, out, bias=bias)
         _counts["tcgen05"] += 1
@@ -68,7 +68,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias, out: torch.Tensor) -> torch.T
 
 def linear_gelu(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor, h_out, g_out: torch.Tensor) -> None:
     """h_out = x @ w^T + bias (None: not wanted);  g_out = gelu_tanh(h_out)   — one kernel where the tcgen05 GEMM is usable."""
-    if _own_kernel_ok(x, w, g_out, fused_epilogue=True):
+    if _own_kernel_ok(x, w, g_out, bias, h_out, fused_epilogue=True):
         from . import gemm_sm100
         gemm_sm100.gemm(gemm_sm100.NT, gemm_sm100.GELU, x, w, g_out, bias=bias, pre=h_out)
         _counts["tcgen05"] += 1

@@ -492,6 +492,7 @@ extern "C" {
 
 int piccl_ops_bias_gelu_fwd(const void* h, const void* bias, void* h_out, void* g, long long rows, int C, void* stream) {
   if (C % 8) return -1;
+  if ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(h_out) | reinterpret_cast<uintptr_t>(g)) & 15) return -2;      // 16-byte words
   size_t n8 = (size_t)rows * C / 8;
   launch_pdl(bias_gelu_fwd_kernel, grid_for(n8, 256), 256, 0, (cudaStream_t)stream, (const bf16*)h, (const bf16*)bias, (bf16*)h_out, (bf16*)g, n8, C / 8);
   PICCL_OPS_CHECK_LAUNCH(); return 0;

@@ -101,3 +101,39 @@ def test_gemm_layouts_epilogues_and_edges(M, N, K, layout, epilogue):
         assert (part.double().sum(0) - out.double().sum(0)).norm() <= 1e-5 * out.double().abs().sum(0).norm()      # fp32 sums of M values
     assert (out.double() - ref).norm() <= 4e-3 * ref.norm()
     assert torch.isnan(guard[M]).all()
+
+
+@pytest.mark.parametrize("backend", ["auto", "tcgen05", "cublas"])
+@pytest.mark.parametrize("which", ["none", "x", "w", "bias", "h", "out"])
+def test_products_of_views_at_any_address(backend, which):
+    """An operand or result that starts 2 bytes beyond a 16-byte boundary, at a ragged shape: cuBLAS takes what the kernel cannot.  Bias and GELU by a kernel of their own
+    read 16-byte words: there such a view is refused."""
+    from piccl_b200.ops import gemm
+
+    def t(name, *shape, scale=1.0):
+        n = 1
+        for s in shape:
+            n *= s
+        buf = _bf(n + 8, seed=len(name) + shape[0], scale=scale)
+        off = 1 if name == which else 0
+        return buf[off:off + n].view(shape)
+
+    M, N, K = 200, 72, 40
+    x, w, bias = t("x", M, K), t("w", N, K, scale=0.05), t("bias", N)
+    h, out = t("h", M, N), t("out", M, N)
+    ref = x.double() @ w.double().t() + bias.double()
+    saved = gemm.backend()
+    try:
+        gemm.set_backend(backend)
+        gemm.linear(x, w, bias, out)
+        assert (out.double() - ref).norm() <= 4e-3 * ref.norm()            # one rounding to bf16
+        if which in ("bias", "h", "out"):
+            with pytest.raises(RuntimeError):
+                gemm.linear_gelu(x, w, bias, h, out)
+            return
+        gemm.linear_gelu(x, w, bias, h, out)
+        assert (h.double() - ref).norm() <= 8e-3 * ref.norm()              # cuBLAS rounds before the bias is added: two
+        want = F.gelu(h.double(), approximate="tanh")
+        assert (out.double() - want).norm() <= 4e-3 * want.norm()
+    finally:
+        gemm.set_backend(saved)
