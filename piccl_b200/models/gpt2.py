@@ -219,10 +219,11 @@ class GPT2:
                 ok = True
             except RuntimeError:
                 pass
-            try:
-                graph.capture_end()
-            except RuntimeError:
-                ok = False
+            finally:                             # also when an interrupt comes here: the stream must not stay in capture
+                try:
+                    graph.capture_end()
+                except RuntimeError:
+                    ok = False
         cur.wait_stream(stream)
         after = gemm.counts()
         counts = (ops.launch_count() - launched, after["tcgen05"] - products["tcgen05"], after["cublas"] - products["cublas"])

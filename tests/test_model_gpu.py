@@ -209,3 +209,26 @@ def test_a_captured_step_is_not_replayed_under_other_library_settings():
         torch.use_deterministic_algorithms(False)
     assert m.replays == 2
     assert float(m.forward_backward(a, b)) == want and m.replays == 3
+
+
+def test_an_interrupt_during_a_capture_leaves_the_model_usable():
+    from piccl_b200.models.gpt2 import GPT2, GPT2Config
+    cfg = GPT2Config.tiny()
+    m = GPT2(cfg, seed=1)
+    tok = torch.randint(0, cfg.vocab_size, (2, cfg.seq_len + 1), generator=torch.Generator().manual_seed(0)).cuda()
+    a, b = tok[:, :-1].contiguous(), tok[:, 1:].contiguous()
+    want = [float(m.forward_backward(a, b)) for _ in range(2)][-1]
+    issue = m._issue
+
+    def interrupted(*args):
+        issue(*args)
+        raise KeyboardInterrupt
+
+    m._issue = interrupted
+    with pytest.raises(KeyboardInterrupt):
+        m.forward_backward(a, b)
+    m._issue = issue
+    for _ in range(3):
+        assert float(m.forward_backward(a, b)) == want
+    torch.cuda.synchronize()
+    assert m.replays == 3
