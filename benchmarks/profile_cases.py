@@ -1,6 +1,7 @@
 """Small, self-terminating workloads for ncu captures (one kernel, a few launches, well under a few GB):
 
     python benchmarks/profile_cases.py exec      # fused collective executor: 2 virtual ranks, ring all-reduce of 256 MiB fp32
+    python benchmarks/profile_cases.py exec8     # the same among 8 virtual ranks, 32 MiB fp32 each
     python benchmarks/profile_cases.py exec_ll   # low-latency all-reduce, 8 virtual ranks, 16 KiB
     python benchmarks/profile_cases.py gemm      # tcgen05 GEMM 8192 x 8192 x 3584 bf16
     python benchmarks/profile_cases.py direct    # DIRECT all-reduce, 8 virtual ranks, 16 MiB fp32
@@ -25,15 +26,20 @@ import torch
 sys.path.insert(0, str(Path(__file__).resolve().parent.parent))
 
 
-def case_exec(ll: bool = False):
+def _group8():
+    """Eight ranks with FIFOs of 128 KiB slots for the 18 CTAs that each gets: 1.2 GiB of heaps for FIFOs and low-latency slots instead of 10."""
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    return LoopbackGroup(8, config=make_config(max_cta=18, nslot=4, slot_bytes=128 << 10, scratch_bytes=1 << 20))
+
+
+def case_exec(ranks: int = 2, count: int = 64 << 20, algo: str = "RING"):
     from piccl_b200.parallel.comm import LoopbackGroup
-    n = 8 if ll else 2
-    count = 4096 if ll else 64 << 20
-    g = LoopbackGroup(n)
+    n = ranks
+    g = LoopbackGroup(n) if n == 2 else _group8()
     xs = [torch.ones(count, device="cuda") for _ in range(n)]
     outs = [torch.empty_like(x) for x in xs]
     for _ in range(4):
-        g.run("allreduce", xs, outs, count, algo="PRD" if ll else "RING")
+        g.run("allreduce", xs, outs, count, algo=algo)
     torch.cuda.synchronize()
     assert g.status().aborted == 0
     g.close()
@@ -92,9 +98,8 @@ def case_nvls():
 
 
 def case_llf():
-    from piccl_b200.parallel.comm import LoopbackGroup
     n, count = 8, 4096
-    g = LoopbackGroup(n)
+    g = _group8()
     xs = [torch.full((count,), float(r), device="cuda") for r in range(n)]
     outs = [torch.empty(n * count, device="cuda") for _ in range(n)]
     for _ in range(4):
@@ -170,5 +175,5 @@ def case_ce():
 
 if __name__ == "__main__":
     which = sys.argv[1] if len(sys.argv) > 1 else "exec"
-    {"exec": case_exec, "exec_ll": lambda: case_exec(True), "gemm": case_gemm, "direct": case_direct, "tp": case_tp, "ln": case_ln, "ce": case_ce, "nvls": case_nvls, "llf": case_llf, "ag_gemm": case_ag_gemm, "elementwise": case_elementwise}[which]()
+    {"exec": case_exec, "exec8": lambda: case_exec(8, 8 << 20), "exec_ll": lambda: case_exec(8, 4096, "PRD"), "gemm": case_gemm, "direct": case_direct, "tp": case_tp, "ln": case_ln, "ce": case_ce, "nvls": case_nvls, "llf": case_llf, "ag_gemm": case_ag_gemm, "elementwise": case_elementwise}[which]()
     print(f"profile case {which} done")

@@ -8,16 +8,16 @@
 // exist as separate passes, and no ncclSend/ncclRecv is issued.
 //
 // Roles inside a CTA: one warp waits (credits and data of the next steps, up to
-// kStepDepth ahead), all warps but two move data, one warp publishes (a release
-// store waits for the acknowledgement of everything the CTA stored, a microsecond
-// and more).  They meet through named barriers per step, so the chain
+// kStepDepth ahead), all warps but two move data, one warp publishes (its fence
+// waits for the acknowledgement of everything the CTA stored, a microsecond and
+// more).  They meet through named barriers per step, so the chain
 //     peer's stores -> its release -> my poll -> my loads
 // of one step overlaps the data movement of others.  With one group of threads doing all of it in
 // turn a 64 KiB step took 10 us, 3 of them for the data.
 //
 // Peer traffic is plain 16-byte stores into the peer's mapped heap (NVLink /
-// NVSwitch P2P); ordering is st.release.sys on the producer and ld.acquire.sys
-// on the consumer.  Every wait has a time limit; on expiry the CTA records
+// NVSwitch P2P); ordering is a fence and a relaxed store on the producer and
+// ld.acquire.sys on the consumer, and the same way back for the slots that are free.  Every wait has a time limit; on expiry the CTA records
 // where it gave up, raises the abort flag that all other waits poll, and the
 // kernel returns.
 #pragma once
@@ -500,7 +500,9 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
     const int flags = s_step[d].flags, ai = s_step[d].action;
     if (flags & (STEP_END | STEP_FAIL)) break;
     const Action& ac = ai < kSliceCache ? s_act[ai] : L.actions[ai];
-    // one fence for both: what the data warps stored comes before the consumers' counters, what they read before the producers'
+    // One fence for both: what the data warps stored comes before the consumers' counters, what they read before the producers'.  It waits for the
+    // acknowledgement of everything the CTA stored, so a credit costs up to a microsecond at the end of a call: 1 MiB blocks of an all-gather 31.6 us, 29.9
+    // with plain stores for the heads, which nothing orders behind the reads.  A release per counter took 38.0, a warp of its own for the heads 32.5.
     fence_sys();
 #pragma unroll
     for (int q = 0; q < 2; q++) {
