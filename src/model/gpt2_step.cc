@@ -150,10 +150,10 @@ at::Tensor view(b16* p, at::IntArrayRef sizes, at::IntArrayRef strides = {}) {
 
 // C[M, N] = A op B, bf16 row-major: layout NT A [M,K] B [N,K], NN A [M,K] B [K,N], TN A [K,M] B [K,N]
 // Plain products of more than some GFLOP go to cuBLAS unless the "tcgen05" backend is asked for: it has more tile shapes to fit ragged sizes
-// to the chip, and under the power cap it draws less for the same tile (GPT-2 medium step 23.5 ms with it, 24.7 without; 8 layers of
-// 768 columns on 3 x 777 tokens 2.97 / 3.10 ms).  Below, the launch counts: issued call by call this framework's kernel costs a third of
+// to the chip (GPT-2 medium step 23.5 ms with it, 24.7 without; 8 layers of 768 columns on 3 x 777 tokens 2.97 / 3.10 ms).  Below, the launch counts: issued call by call this framework's kernel costs a third of
 // the host time (2 layers of 256 columns 342 us, 500 with cuBLAS); replayed from a graph it does not, and the line lies lower (the same
-// step 236 us at 2 GFLOP, 217 at 0.1; 12 layers of 512 columns on 4 x 512 tokens 1985 us, 1857).
+// step 236 us at 2 GFLOP, 217 at 0.1; 12 layers of 512 columns on 4 x 512 tokens 1985 us, 1857).  So a product between the two lines runs on one back end issued and on the other replayed: the sums are the same up to
+// their order.
 constexpr double kOwnProductFlops = 2e9, kOwnProductFlopsReplayed = 1e8;
 int product(Model& m, int layout, b16* A, b16* B, b16* C, const b16* bias, int M, int N, int K, void* s, int which_ws = 0) {
   if (m.backend == 2 || (m.backend == 0 && 2.0 * M * N * K > (m.captured ? kOwnProductFlopsReplayed : kOwnProductFlops))) {

@@ -271,7 +271,7 @@ __device__ __forceinline__ bf16 ce_gradient_target(float x, float neg_m, float l
 
 // The same in one pass over memory: the sum of exponentials is taken while the row comes in, relative to the thread's maximum so far, and
 // the gradient needs the row once more, from shared memory.  GRAD = false leaves the logits as they are and keeps nothing.
-// Two blocks share an SM: one loads while the other computes.  8192 x 50304: 364 us with the gradient, 183 without (386 and 219 with a pass
+// Two blocks share an SM: one loads while the other computes.  8192 x 50304: 364 us with the gradient, 183 without (372 and 193 from a cold L2; 386 and 219 with a pass
 // of its own for the sum; the copy rate allows 252 and 126, the special-function units 183 and 92).  One block per SM with the next row
 // on its way to a second buffer was slower, 492 us.
 template <bool GRAD>
