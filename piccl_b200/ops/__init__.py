@@ -109,6 +109,20 @@ def cross_entropy_fwd_bwd(logits, targets, loss_rows, vocab: int, gscale: float)
     _bump()
 
 
+def attention_fwd(qkv, out, lse, batch: int):
+    """Causal attention of packed rows [batch * S, 3 * heads * 64] -> [batch * S, heads * 64]; lse: batch * heads * (S rounded up to 128) floats, or None."""
+    rows, Cc = out.shape
+    _chk(N.ops_lib().piccl_ops_attn_fwd(_p(qkv), _p(out), _p(lse), batch, rows // batch, Cc // 64, C.c_void_p(_s())), "attn_fwd")
+    _bump()
+
+
+def attention_bwd(qkv, out, dout, lse, delta, dqkv, part, batch: int):
+    """dqkv, the gradient of the packed rows, and in part its partial column sums: one row per batch entry and 128 positions.  delta: scratch like lse."""
+    rows, Cc = out.shape
+    _chk(N.ops_lib().piccl_ops_attn_bwd(_p(qkv), _p(out), _p(dout), _p(lse), _p(delta), _p(dqkv), _p(part), batch, rows // batch, Cc // 64, C.c_void_p(_s())), "attn_bwd")
+    _bump(2)
+
+
 def adamw(p, master, m, v, g, lr: float, b1: float, b2: float, eps: float, wd: float, step: int, gscale: float = 1.0):
     _chk(N.ops_lib().piccl_ops_adamw(_p(p), _p(master), _p(m), _p(v), _p(g), C.c_longlong(p.numel()), C.c_float(lr), C.c_float(b1), C.c_float(b2),
                                      C.c_float(eps), C.c_float(wd), step, C.c_float(gscale), C.c_void_p(_s())), "adamw")

@@ -2,7 +2,8 @@
 //
 // Why native: the step is a few dozen launches per layer, and issued from Python each cost about 15 us of host time: two layers of
 // 256 columns took 1.4 ms for 0.3 ms of kernels, eight layers of 768 columns 4.5 ms for 2.7 ms.  Here a launch of this framework's
-// own kernels is a plain call (2 to 3 us); attention goes through ATen's fused kernels without autograd.
+// own kernels is a plain call (2 to 3 us); attention of heads of 64 columns is one of them, of other heads it goes through ATen's fused kernels
+// without autograd.
 //
 // A step of the same shape on the same input buffers is captured into a CUDA graph by the caller (models/gpt2.py).  Its weight gradients and
 // column sums, which nothing in the backward pass waits for, can then go to a second stream: small ones fill the SMs that the chain of
@@ -114,15 +115,16 @@ struct Carve {
   }
 };
 
-struct Layer { b16 *ln1, *qkv, *x2, *ln2, *h, *gl, *x3; float *mean1, *rstd1, *mean2, *rstd2; };
+struct Layer { b16 *ln1, *qkv, *att, *x2, *ln2, *h, *gl, *x3; float *mean1, *rstd1, *mean2, *rstd2, *lse; };
 struct Buffers {
   b16 *x0, *a, *pr, *logits, *dln, *dln2, *datt, *dln1;
   b16 *dxa[3], *dxb[2], *dg[2], *dqkv[2];      // taken in turn by the layers: weight gradients may still read those of the layer above
-  float *loss_rows, *parts[2];
+  float *loss_rows, *parts[2], *delta;
   std::vector<Layer> layer;         // L + 1: the last one holds the input of the head
 };
 
-void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, Buffers& b) {
+// lse_floats: of the attention kernels' row sums, 0 where attention is ATen's
+void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, size_t lse_floats, Buffers& b) {
   const size_t C = d.C;
   b.x0 = c.get<b16>(T * C); b.a = c.get<b16>(T * C); b.pr = c.get<b16>(T * C);
   b.layer.resize(d.L + 1);
@@ -132,12 +134,14 @@ void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, Bu
     y.ln1 = c.get<b16>(T * C); y.mean1 = c.get<float>(T); y.rstd1 = c.get<float>(T);
     if (train && l == d.L) continue;
     y.qkv = c.get<b16>(T * 3 * C); y.x2 = c.get<b16>(T * C); y.ln2 = c.get<b16>(T * C); y.mean2 = c.get<float>(T); y.rstd2 = c.get<float>(T);
+    y.att = lse_floats ? c.get<b16>(T * C) : nullptr; y.lse = lse_floats && train ? c.get<float>(lse_floats) : nullptr;
     y.h = train ? c.get<b16>(T * 4 * C) : nullptr; y.gl = c.get<b16>(T * 4 * C); y.x3 = c.get<b16>(T * C);
   }
   b.logits = c.get<b16>(T * d.Vp); b.loss_rows = c.get<float>(T);
   if (!train) return;
   for (b16*& x : b.dxa) x = c.get<b16>(T * C);
   for (int q = 0; q < 2; q++) { b.dxb[q] = c.get<b16>(T * C); b.dg[q] = c.get<b16>(T * 4 * C); b.dqkv[q] = c.get<b16>(T * 3 * C); }
+  b.delta = c.get<float>(lse_floats);
   b.dln = c.get<b16>(T * C); b.dln2 = c.get<b16>(T * C); b.datt = c.get<b16>(T * C); b.dln1 = c.get<b16>(T * C); for (float*& x : b.parts) x = c.get<float>(part_floats);
 }
 
@@ -169,12 +173,19 @@ int product(Model& m, int layout, b16* A, b16* B, b16* C, const b16* bias, int M
 }
 #define DO(expr) do { const int rc_ = (expr); if (rc_ != 0) return rc_; } while (0)
 
+// What scaled_dot_product_attention would pick for q, k, v within packed rows.
+int64_t sdp_choice(b16* qkv, int B, int S, int H, int D) {
+  const int64_t C = (int64_t)H * D, sizes[4] = {B, H, S, D}, strides[4] = {(int64_t)S * 3 * C, D, 3 * C, 1};
+  return at::_fused_sdp_choice(view(qkv, sizes, strides), view(qkv + C, sizes, strides), view(qkv + 2 * C, sizes, strides), {}, 0.0, true);
+}
+constexpr int64_t kCudnnAttention = 3;       // sdp::SDPBackend::cudnn_attention
+
 // Causal attention of qkv [B * S, 3 C]; the [B, S, H, D] output is contiguous.
 at::Tensor attention(Saved& sv, b16* qkv, int B, int S, int H, int D, bool train) {
   const int64_t C = (int64_t)H * D, sizes[4] = {B, H, S, D}, strides[4] = {(int64_t)S * 3 * C, D, 3 * C, 1};
   sv.q = view(qkv, sizes, strides); sv.k = view(qkv + C, sizes, strides); sv.v = view(qkv + 2 * C, sizes, strides);
   // the kernel that scaled_dot_product_attention would pick: cuDNN's is called without autograd, any other through it
-  sv.direct = at::_fused_sdp_choice(sv.q, sv.k, sv.v, {}, 0.0, true) == 3 /* sdp::SDPBackend::cudnn_attention */;
+  sv.direct = at::_fused_sdp_choice(sv.q, sv.k, sv.v, {}, 0.0, true) == kCudnnAttention;
   if (sv.direct) {
     auto r = at::_scaled_dot_product_cudnn_attention(sv.q, sv.k, sv.v, {}, train, 0.0, true, false);
     sv.out = std::get<0>(r); sv.lse = std::get<1>(r); sv.cq = std::get<2>(r); sv.ck = std::get<3>(r); sv.mq = std::get<4>(r); sv.mk = std::get<5>(r);
@@ -214,10 +225,15 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
 
   // partial rows of the column sums: dgamma, dbeta and bias gradient of both LayerNorms, the MLP's and the attention's bias gradients
   const int n_ln = piccl_ops_ln_bwd_parts(T, C), n_qkv = piccl_ops_col_parts(T, 3 * C), n_fc_own = (T + 31) / 32, n_fc_sep = piccl_ops_col_parts(T, 4 * C);
-  const size_t row = (size_t)n_ln * C, fc_floats = (size_t)std::max(n_fc_own, n_fc_sep) * 4 * C;
+  // Heads of 64 columns: this framework's kernels, where PyTorch would take cuDNN's (a program that asks for another back end gets that one).
+  // (Any address will do for the question.)
+  const bool own_attention = D == 64 && sdp_choice(d.p, B, S, H, D) == kCudnnAttention;
+  const int n_att = own_attention ? piccl_ops_attn_parts(B, S) : 0;
+  const size_t row = (size_t)n_ln * C, fc_floats = (size_t)std::max(n_fc_own, n_fc_sep) * 4 * C, part_floats = 6 * row + fc_floats + (size_t)std::max(n_qkv, n_att) * 3 * C;
+  const size_t lse_floats = own_attention ? (size_t)B * H * piccl_ops_attn_rows(S) : 0;
   Buffers b;
   Carve count{nullptr};
-  carve(count, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
+  carve(count, d, T, train, part_floats, lse_floats, b);
   if (!m.arena.defined() || (size_t)m.arena.numel() < count.used) {
     if (m.in_callers_graph) m.kept.push_back(m.arena);
     m.in_callers_graph = false;
@@ -227,7 +243,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   const bool in_capture = capturing(main_stream);
   m.in_callers_graph |= !m.captured && in_capture;
   Carve c{static_cast<char*>(m.arena.data_ptr())};
-  carve(c, d, T, train, 6 * row + fc_floats + (size_t)n_qkv * 3 * C, b);
+  carve(c, d, T, train, part_floats, lse_floats, b);
   b16 *const lnf_g = d.p + m.off[0], *const lnf_b = d.p + m.off[1], *const wpe = d.p + m.off[2], *const wte = d.p + m.off[3];
   if (!m.split.defined()) {
     m.split = at::empty({2, (int64_t)kSplitBytes}, opt.dtype(at::kByte));
@@ -249,8 +265,9 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   for (int l = 0; l < L; l++) {
     Layer& y = b.layer[l]; Layer& z = b.layer[l + 1];
     DO(product(m, NT, y.ln1, m.p(l, W_QKV), y.qkv, m.p(l, B_QKV), T, 3 * C, C, s));
-    att[l] = attention(m.saved[l], y.qkv, B, S, H, D, train);
-    DO(product(m, NT, static_cast<b16*>(att[l].data_ptr()), m.p(l, W_O), b.a, m.p(l, B_O), T, C, C, s));
+    if (own_attention) TRY(piccl_ops_attn_fwd(y.qkv, y.att, y.lse, B, S, H, s));
+    else { att[l] = attention(m.saved[l], y.qkv, B, S, H, D, train); y.att = static_cast<b16*>(att[l].data_ptr()); }
+    DO(product(m, NT, y.att, m.p(l, W_O), b.a, m.p(l, B_O), T, C, C, s));
     if (!train) { m.saved[l] = Saved(); att[l] = at::Tensor(); }
     TRY(piccl_ops_ln_fwd(b.a, xin, m.p(l, LN2_G), m.p(l, LN2_B), y.x2, y.ln2, y.mean2, y.rstd2, T, C, d.eps, s));
     if (m.backend == 2) {
@@ -328,22 +345,28 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
     DO(product(m, NN, dg, m.p(l, W_FC), b.dln2, nullptr, T, C, 4 * C, s));
     TRY(piccl_ops_ln_bwd(b.dln2, y.x2, m.p(l, LN2_G), y.mean2, y.rstd2, dx, dxb, ws2, 1, T, C, s));
     // x2 = xin + attention Wo + bo
-    DO(weight_grad(dxb, static_cast<b16*>(att[l].data_ptr()), m.g(l, W_O), C, C));
+    DO(weight_grad(dxb, y.att, m.g(l, W_O), C, C));
     DO(product(m, NN, dxb, m.p(l, W_O), b.datt, nullptr, T, C, C, s));
-    at::Tensor dq[3];
-    attention_grad(m.saved[l], b.datt, B, S, H, D, dq);
-    const void* ptr[3]; long long st[9];
-    for (int i = 0; i < 3; i++) { ptr[i] = dq[i].data_ptr(); for (int j = 0; j < 3; j++) st[3 * i + j] = dq[i].stride(j); }
     int n_q = n_qkv;
-    bool words = D % 8 == 0;          // rows of a head are whole 16-byte words
-    for (int i = 0; i < 3; i++) words &= (reinterpret_cast<uintptr_t>(ptr[i]) % 16 | (st[3 * i] | st[3 * i + 1] | st[3 * i + 2]) % 8) == 0;
-    if (words) TRY(piccl_ops_qkv_grad(ptr, st, dqkv, ws_qkv, B, S, H, D, s));
-    else {                            // heads of 4 columns, say: packed by ATen, the column sums from the packed rows
-      const at::Tensor packed = view(dqkv, {B, S, 3, H, D});
-      for (int i = 0; i < 3; i++) packed.select(2, i).copy_(dq[i].transpose(1, 2));
-      const int per = (T + n_qkv - 1) / n_qkv;
-      n_q = (T + per - 1) / per;
-      TRY(piccl_ops_colsum(dqkv, nullptr, ws_qkv, T, 3 * C, per, 0, s));
+    if (own_attention) {
+      n_q = n_att;
+      TRY(piccl_ops_attn_bwd(y.qkv, y.att, b.datt, y.lse, b.delta, dqkv, ws_qkv, B, S, H, s));
+      m.launches++;                   // two kernels
+    } else {
+      at::Tensor dq[3];
+      attention_grad(m.saved[l], b.datt, B, S, H, D, dq);
+      const void* ptr[3]; long long st[9];
+      for (int i = 0; i < 3; i++) { ptr[i] = dq[i].data_ptr(); for (int j = 0; j < 3; j++) st[3 * i + j] = dq[i].stride(j); }
+      bool words = D % 8 == 0;          // rows of a head are whole 16-byte words
+      for (int i = 0; i < 3; i++) words &= (reinterpret_cast<uintptr_t>(ptr[i]) % 16 | (st[3 * i] | st[3 * i + 1] | st[3 * i + 2]) % 8) == 0;
+      if (words) TRY(piccl_ops_qkv_grad(ptr, st, dqkv, ws_qkv, B, S, H, D, s));
+      else {                            // heads of 4 columns, say: packed by ATen, the column sums from the packed rows
+        const at::Tensor packed = view(dqkv, {B, S, 3, H, D});
+        for (int i = 0; i < 3; i++) packed.select(2, i).copy_(dq[i].transpose(1, 2));
+        const int per = (T + n_qkv - 1) / n_qkv;
+        n_q = (T + per - 1) / per;
+        TRY(piccl_ops_colsum(dqkv, nullptr, ws_qkv, T, 3 * C, per, 0, s));
+      }
     }
     DO(weight_grad(dqkv, y.ln1, m.g(l, W_QKV), 3 * C, C));
     DO(product(m, NN, dqkv, m.p(l, W_QKV), b.dln1, nullptr, T, C, 3 * C, s));
