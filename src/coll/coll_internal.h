@@ -32,7 +32,25 @@ struct Builder {
     prog.actions.push_back(a);
   }
   void next_step() { step++; }
-  Program finish() { prog.nsteps = step; return prog; }
+  Program finish() {
+    prog.nsteps = step;
+    // Which elements of the local buffers come up again: from the last action to the first, the ranges that later ones read.  (A range that is read in
+    // parts counts as read; in-place calls see the two buffers as one, an element there is read before it is written.)
+    struct Range { Buf buf; int64_t lo, hi; };
+    std::vector<Range> later;
+    auto again = [&](uint8_t buf, int64_t off, int64_t n) {
+      for (const Range& r : later) if (r.buf == buf && off < r.hi && r.lo < off + n) return true;
+      return false;
+    };
+    for (size_t i = prog.actions.size(); i-- > 0;) {
+      Action& a = prog.actions[i];
+      if (a.dst_buf != BUF_NONE && !again(a.dst_buf, a.dst_off, a.count)) a.flags |= ACT_DST_DONE;
+      if (a.src_buf == BUF_NONE) continue;
+      if (!again(a.src_buf, a.src_off, a.count)) a.flags |= ACT_SRC_DONE;
+      later.push_back({(Buf)a.src_buf, a.src_off, a.src_off + a.count});
+    }
+    return prog;
+  }
 };
 
 // Tree shapes for broadcast / reduce (root-relative virtual ranks).

@@ -41,6 +41,8 @@ constexpr int kMaxRanks = 64;
 
 // Flags of an action.
 constexpr uint8_t ACT_SCALE_SRC = 1;  // local source is an original contribution (pre-scaled for avg)
+constexpr uint8_t ACT_SRC_DONE = 2;   // no later action reads the local operand's elements again
+constexpr uint8_t ACT_DST_DONE = 4;   // no later action reads what this one stores locally
 
 // One unit of work, executed by every CTA on its slice of [0,count).
 // Fixed 48-byte layout shared with the device code.

@@ -49,6 +49,22 @@ __device__ __forceinline__ uint4 ld_slot(const void* p) {
   asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+// The same, and stores, with the priority that the line gets in L2: one that is done with goes first, so that the FIFO's slots, which another rank reads
+// next, stay.
+__device__ __forceinline__ unsigned long long l2_policy(bool first) {
+  unsigned long long p;
+  if (first) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  else asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint4 ld_hint(const void* p, unsigned long long policy) {
+  uint4 v;
+  asm volatile("ld.relaxed.sys.global.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_hint(void* p, const uint4& v, unsigned long long policy) {
+  asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1,%2,%3,%4}, %5;" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void st_vec(void* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
 
 // ---------------------------------------------------------------- element-wise maths
@@ -164,17 +180,26 @@ __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, i
     return Pack<T>::down(acc);
   }
 }
+struct L2Hints { bool src_done, dst_done; int local_src, local_dst; };
 template <typename T, int OP, int NSRC, int NDST, int U, bool EXACT, bool SCALE = false>      // EXACT: nsrc == NSRC, else the first operand stands in for what is missing; NDST 0: any number, read from the table each time
-__device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char* const* dst, int ndst, int n, int scaled, float scale) {
+__device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
+  constexpr bool HINT_SRC = NSRC <= 2;                   // (more sources leave no registers for their policies)
   const int nsrc = EXACT ? NSRC : nsrc_rt, nt = data_threads(), tid = threadIdx.x;
   const char* sp[NSRC]; char* dp[NDST ? NDST : 1];
 #pragma unroll
   for (int s = 0; s < NSRC; s++) sp[s] = src[EXACT || s < nsrc ? s : 0];
 #pragma unroll
   for (int d = 0; d < NDST; d++) dp[d] = dst[d];
+  unsigned long long ps[HINT_SRC ? NSRC : 1], pd[NDST ? NDST : 1];
+  const unsigned long long normal = l2_policy(false);
+#pragma unroll
+  for (int s = 0; s < NSRC; s++) if (HINT_SRC) ps[s] = h.src_done && s == h.local_src ? l2_policy(true) : normal;
+#pragma unroll
+  for (int d = 0; d < NDST; d++) pd[d] = h.dst_done && d == h.local_dst ? l2_policy(true) : normal;
+  auto get = [&](int s, int off) { if constexpr (HINT_SRC) return ld_hint(sp[s] + off, ps[s]); else return ld_slot(sp[s] + off); };
   auto put = [&](int off, const uint4& o) {
 #pragma unroll
-    for (int d = 0; d < NDST; d++) st_vec(dp[d] + off, o);
+    for (int d = 0; d < NDST; d++) st_hint(dp[d] + off, o, pd[d]);
     if (NDST == 0) for (int d = 0; d < ndst; d++) st_vec(dst[d] + off, o);
   };
   int p = tid;
@@ -183,7 +208,7 @@ __device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char
 #pragma unroll
     for (int s = 0; s < NSRC; s++)
 #pragma unroll
-      for (int u = 0; u < U; u++) v[s][u] = ld_slot(sp[s] + (p + u * nt) * 16);
+      for (int u = 0; u < U; u++) v[s][u] = get(s, (p + u * nt) * 16);
 #pragma unroll
     for (int u = 0; u < U; u++) put((p + u * nt) * 16, combine<T, OP, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
   }
@@ -192,38 +217,38 @@ __device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char
 #pragma unroll
     for (int s = 0; s < NSRC; s++)
 #pragma unroll
-      for (int u = 0; u < U - 1; u++) v[s][u] = ld_slot(sp[s] + min(p + u * nt, n - 1) * 16);
+      for (int u = 0; u < U - 1; u++) v[s][u] = get(s, min(p + u * nt, n - 1) * 16);
 #pragma unroll
     for (int u = 0; u < U - 1; u++) if (p + u * nt < n) put((p + u * nt) * 16, combine<T, OP, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
   }
 }
 template <typename T, int OP>
-__device__ __forceinline__ void move_aligned(const char* const* src, int nsrc, char* const* dst, int ndst, int n, int scaled, float scale) {
+__device__ __forceinline__ void move_aligned(const char* const* src, int nsrc, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
   if (OP == OP_COPY || (nsrc == 1 && scaled < 0)) {
-    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(src, 1, dst, 1, n, -1, scale);
-    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(src, 1, dst, 2, n, -1, scale);
-    else stream<T, OP, 1, 0, 4, true>(src, 1, dst, ndst, n, -1, scale);
+    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(src, 1, dst, 1, n, -1, scale, h);
+    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(src, 1, dst, 2, n, -1, scale, h);
+    else stream<T, OP, 1, 0, 4, true>(src, 1, dst, ndst, n, -1, scale, h);
   } else if constexpr (OP != OP_COPY) {
     // Scaled operands (avg, which is a sum) have loops of their own too: in the general one a lone operand was loaded twice and the destinations read
     // from the table for each pack (25 MiB of bf16 averaged among four ranks: 155 us, now 136).
     if (scaled >= 0) {
       if constexpr (OP == 0) {
         if (nsrc == 1) {
-          if (ndst == 1) stream<T, OP, 1, 1, 8, true, true>(src, 1, dst, 1, n, 0, scale);
-          else stream<T, OP, 1, 0, 4, true, true>(src, 1, dst, ndst, n, 0, scale);
+          if (ndst == 1) stream<T, OP, 1, 1, 8, true, true>(src, 1, dst, 1, n, 0, scale, h);
+          else stream<T, OP, 1, 0, 4, true, true>(src, 1, dst, ndst, n, 0, scale, h);
         }
-        else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true, true>(src, 2, dst, 1, n, scaled, scale);
-        else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true, true>(src, 2, dst, 2, n, scaled, scale);
-        else if (nsrc <= 4) stream<T, OP, 4, 0, 2, false, true>(src, nsrc, dst, ndst, n, scaled, scale);
-        else stream<T, OP, kMaxActionPeers + 1, 0, 1, false, true>(src, nsrc, dst, ndst, n, scaled, scale);
+        else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true, true>(src, 2, dst, 1, n, scaled, scale, h);
+        else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true, true>(src, 2, dst, 2, n, scaled, scale, h);
+        else if (nsrc <= 4) stream<T, OP, 4, 0, 2, false, true>(src, nsrc, dst, ndst, n, scaled, scale, h);
+        else stream<T, OP, kMaxActionPeers + 1, 0, 1, false, true>(src, nsrc, dst, ndst, n, scaled, scale, h);
       }
     }
-    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(src, 2, dst, 1, n, -1, scale);
-    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(src, 2, dst, 2, n, -1, scale);
-    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(src, 4, dst, ndst, n, -1, scale);
-    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(src, nsrc, dst, ndst, n, -1, scale);
-    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(src, nsrc, dst, ndst, n, -1, scale);
-    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(src, nsrc, dst, ndst, n, -1, scale);
+    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(src, 2, dst, 1, n, -1, scale, h);
+    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(src, 2, dst, 2, n, -1, scale, h);
+    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(src, 4, dst, ndst, n, -1, scale, h);
+    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(src, nsrc, dst, ndst, n, -1, scale, h);
+    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(src, nsrc, dst, ndst, n, -1, scale, h);
+    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(src, nsrc, dst, ndst, n, -1, scale, h);
   }
 }
 
@@ -352,7 +377,7 @@ struct StepDesc {
   long long len;                             // elements
   int action, nsrc, ndst, local_src, local_dst, flags;
 };
-enum : int { STEP_SCALE = 1, STEP_ALIGNED = 2, STEP_LOCAL_DEP = 4, STEP_FAIL = 8, STEP_END = 16 };
+enum : int { STEP_SCALE = 1, STEP_ALIGNED = 2, STEP_LOCAL_DEP = 4, STEP_FAIL = 8, STEP_END = 16, STEP_SRC_DONE = 32, STEP_DST_DONE = 64 };
 __device__ __forceinline__ void bar_sync_n(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive_n(int id, int n) { __threadfence_block(); asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
@@ -413,7 +438,7 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
         constexpr int N = Pack<T>::N;
         const long long nfull = (SHIFT || (flags & STEP_ALIGNED)) ? len / N : 0;
         if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(nsrc, src, local_src, ndst, dst, st.local_dst, nfull, do_scale, ka.scale); }
-        else if (nfull) move_aligned<T, OP>(src, nsrc, dst, ndst, (int)nfull, do_scale ? local_src : -1, ka.scale);
+        else if (nfull) move_aligned<T, OP>(src, nsrc, dst, ndst, (int)nfull, do_scale ? local_src : -1, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
         if (nfull * N < len) reduce_copy_elem<T, OP>(nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale, ka.scale);
       }
       bar_arrive_n(kDone + d, ndata + 32);
@@ -485,7 +510,7 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
             st.len = (lo + seg_elems < sl_hi ? lo + seg_elems : sl_hi) - lo;
             st.action = ai; st.nsrc = ac.n_recv + has_src; st.ndst = ac.n_send + has_dst; st.local_src = has_src ? ac.self_pos : -1; st.local_dst = has_dst ? 0 : -1;
             st.flags = (ka.avg && (ac.flags & ACT_SCALE_SRC) && has_src ? STEP_SCALE : 0) | (((reinterpret_cast<uintptr_t>(lsrc) | reinterpret_cast<uintptr_t>(ldst)) & 15) == 0 ? STEP_ALIGNED : 0) |
-                       (has_src && ac.src_buf != BUF_IN ? STEP_LOCAL_DEP : 0) | (ok ? 0 : STEP_FAIL);
+                       (has_src && ac.src_buf != BUF_IN ? STEP_LOCAL_DEP : 0) | (ka.last_first && (ac.flags & ACT_SRC_DONE) ? STEP_SRC_DONE : 0) | (ka.last_first && (ac.flags & ACT_DST_DONE) ? STEP_DST_DONE : 0) | (ok ? 0 : STEP_FAIL);
           }
           __syncwarp();
           bar_arrive_n(kReady + k % kStepDepth, ndata + 32);

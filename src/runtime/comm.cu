@@ -392,6 +392,23 @@ static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
 // threads of an executor CTA: the configured block moves data, two more warps wait and publish
 static int exec_block(const piccl_comm* c) { return c->cfg.block_size + kCtlThreads; }
 
+// Do the caller's buffers of a launch of n ranks, read and written, crowd what is on its way between ranks out of L2?  Then the executor asks L2 to let go of
+// the caller's lines first, each with its last use (exec_impl.cuh: stream).  us without and with: all-reduce on the ring 8 x 4 MiB (64 MiB touched) 75 / 80,
+// 8 x 8 94 / 96, 8 x 16 119 / 117, 8 x 64 408 / 369, recursive doubling 4 x 16 (128 MiB) 92 / 90, 4 x 25 138 / 134; all-gather 4 x 2 MiB (40 MiB) 30.3 / 30.2, 4 x 4 41.0 / 38.8,
+// 4 x 16 117 / 105; reduce-scatter 2 x 8 MiB (48 MiB) 19.9 / 21.1, 2 x 16 33.9 / 31.8, 8 x 8 221 / 204; broadcast 4 x 8 MiB (40 MiB) 43.8 / 43.4, 4 x 16 56.5 / 54.8;
+// reduce 4 x 16 MiB 53.3 / 50.5.  (Of an all-reduce more stays in L2 from one
+// call to the next: its line lies higher.)
+static bool crowds_l2(const CollArgs& a, int n) {
+  const long long one = (long long)a.count * a.elem_size;
+  long long bytes = 0, line = 72ll << 20;
+  switch (a.coll) {
+    case COLL_ALLREDUCE: bytes = 2 * n * one; line = 128ll << 20; break;
+    case COLL_ALLGATHER: case COLL_REDUCE_SCATTER: bytes = n * (1 + a.nranks) * one; break;
+    default: bytes = (n + 1) * one; break;
+  }
+  return bytes > line;
+}
+
 // Segments of the executor.  Two are walked together where there are slots for it (the protocol needs two slots per segment of a window): the way from a
 // peer's stores to my loads then hides behind the other one.  One launch for all ranks: segments of at most 128 KiB, a quarter of the default
 // slot, so that what is on its way between ranks stays in L2 (512 KiB slots of 144 CTAs are 300 MB).  Measured with 512 threads, 8 x 64 MiB all-reduce on the
@@ -654,6 +671,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
           if (n > 1) n_cta = std::min(n_cta, std::max(1, c->sm_count / n));
         }
         ka.n_cta = n_cta; if (!use_llf) cut_fifo(c, n, n_cta, a, &ka);
+        ka.last_first = crowds_l2(a, n);
         ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
       }
       ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;

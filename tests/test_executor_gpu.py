@@ -104,6 +104,51 @@ def test_allreduce_avg(groups):
         assert torch.allclose(outs[1], _ref_reduce(xs, "avg"), atol=1e-5)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,algo,k", [(2, "RING", -1), (4, "PRD", 2), (8, "K_RING", 4), (3, "PRM", 3), (4, "PRM", 4), (8, "PRM", 8), (6, "RM", 3), (5, "DIRECT", -1)])
+def test_averaged_operands(groups, n, algo, k, dtype):
+    """Scaled operands alone and beside one, up to three and up to seven others, to one and several destinations; lengths around a round of the loops.
+    Each of at most three partial sums is rounded to the type once, and so is the scaled operand."""
+    eps = 2.0 ** (-24 if dtype == torch.float32 else -9)
+    for count in (1, 9, 4096 * 8 + 3, 100003):
+        g = groups(n)
+        xs = _inputs(n, count, dtype, seed=count)
+        outs = [torch.empty_like(x) for x in xs]
+        g.run("allreduce", xs, outs, count, op="avg", algo=algo, k=k)
+        _check_ok(g)
+        for o in outs:
+            assert (o.double() - torch.stack(xs).double().mean(0)).abs().max() <= 2 * n * eps
+
+
+@pytest.mark.parametrize("coll,n,count,dtype,algo,k", [("allreduce", 4, (17 << 20) + 5, torch.bfloat16, "PRD", 2), ("allreduce", 8, (5 << 20) + 3, torch.float32, "RING", -1),
+                                                       ("allgather", 4, 4 << 20, torch.int32, "RING", -1), ("reduce_scatter", 2, 5 << 20, torch.float32, "AUTO", -1),
+                                                       ("broadcast", 3, (6 << 20) + 1, torch.float32, "RING", -1), ("reduce", 4, (5 << 20) + 7, torch.int32, "AUTO", -1)])
+def test_buffers_larger_than_the_cache(coll, n, count, dtype, algo, k):
+    """Calls whose buffers crowd L2, where loads and stores carry a priority: twice on the same buffers, the second time with other values."""
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    g = LoopbackGroup(n, config=make_config(timeout_ms=5000))
+    try:
+        outs = [torch.zeros(count * n if coll == "allgather" else count, dtype=dtype, device="cuda") for _ in range(n)]
+        xs = None
+        for seed in (1, 2):
+            new = _inputs(n, count * n if coll == "reduce_scatter" else count, dtype, seed=seed)
+            xs = new if xs is None else [x.copy_(y) for x, y in zip(xs, new)]
+            g.run(coll, xs, outs, count, op="sum", root=0, algo=algo, k=k)
+            _check_ok(g)
+            total = torch.stack(xs).double().sum(0) if coll not in ("allgather", "broadcast") else None
+            for r, o in enumerate(outs):
+                if coll == "reduce" and r:
+                    continue
+                want = torch.cat(xs) if coll == "allgather" else xs[0] if coll == "broadcast" else total[r * count:(r + 1) * count] if coll == "reduce_scatter" else total
+                if dtype == torch.int32 or total is None:
+                    assert torch.equal(o.double(), want.double())
+                else:
+                    assert (o.double() - want).abs().max() <= n * n * 2.0 ** (-24 if dtype == torch.float32 else -9)
+    finally:
+        g.close()
+
+
+
 @pytest.mark.parametrize("n", [2, 4, 8])
 @pytest.mark.parametrize("algo", ALGOS)
 def test_allgather(groups, n, algo):
