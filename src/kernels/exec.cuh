@@ -60,6 +60,7 @@ struct KernelArgs {
   // How a channel's FIFO memory (nslot * slot_bytes of the communicator) is cut up for this call; the same on every rank.  All entries of earlier calls
   // are consumed, so the cut may differ from call to call where no rank can be a call ahead (one launch for all ranks).
   long long seg_bytes;                    // bytes of a segment and of its slot
+  int one_gpu;                            // 1: every rank's heap is on this GPU: counters and fences need no scope beyond it
   int last_first;                         // 1: what is used for the last time leaves L2 first
   int nslot, window;                      // slots; segments that are walked together, at most half the slots
   unsigned long long timeout_ns;

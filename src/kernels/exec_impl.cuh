@@ -17,7 +17,7 @@
 //
 // Peer traffic is plain 16-byte stores into the peer's mapped heap (NVLink /
 // NVSwitch P2P); ordering is a fence and a relaxed store on the producer and
-// ld.acquire.sys on the consumer, and the same way back for the slots that are free.  Every wait has a time limit; on expiry the CTA records
+// an acquiring load on the consumer, and the same way back for the slots that are free.  Every wait has a time limit; on expiry the CTA records
 // where it gave up, raises the abort flag that all other waits poll, and the
 // kernel returns.
 #pragma once
@@ -29,15 +29,23 @@
 namespace piccl {
 
 // ---------------------------------------------------------------- memory primitives
-__device__ __forceinline__ unsigned long long ld_acquire_sys(const unsigned long long* p) {
+// Counters and fences, for ranks on several GPUs or all on one.  At system scope every fence also waits on the way to the host and the peers: with all
+// ranks on one GPU all-reduce 8 x 4 MiB on the ring took 79 us, at GPU scope 56; all-gather 8 x 2 MiB 94 / 72, 4 x 1 MiB at odd addresses 35.6 / 28.5, all-reduce
+// 8 x 64 MiB 370 / 360 (on a machine where that way was short 60 / 56, 76 / 72, 29.5 / 28.5 and 367 / 360).
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p, bool one_gpu) {
   unsigned long long v;
-  asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  if (one_gpu) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  else asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_relaxed_sys(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v, bool one_gpu) {
+  if (one_gpu) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+  else asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ void fence_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
+__device__ __forceinline__ void fence_ranks(bool one_gpu) {
+  if (one_gpu) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  else asm volatile("fence.acq_rel.sys;" ::: "memory");
+}
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -59,7 +67,7 @@ __device__ __forceinline__ unsigned long long l2_policy(bool first) {
 }
 __device__ __forceinline__ uint4 ld_hint(const void* p, unsigned long long policy) {
   uint4 v;
-  asm volatile("ld.relaxed.sys.global.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy) : "memory");
+  asm volatile("ld.relaxed.gpu.global.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy) : "memory");
   return v;
 }
 __device__ __forceinline__ void st_hint(void* p, const uint4& v, unsigned long long policy) {
@@ -116,13 +124,13 @@ template <> __device__ __forceinline__ float scale_val<float>(float v, float s) 
 template <> __device__ __forceinline__ double scale_val<double>(double v, float s) { return v * (double)s; }
 
 // ---------------------------------------------------------------- bounded wait
-struct WaitCtx { RankCtx* ctx; unsigned long long timeout_ns; int cta, action, segment; };
+struct WaitCtx { RankCtx* ctx; unsigned long long timeout_ns; int cta, action, segment; bool one_gpu; };
 
 // Returns false if the wait was given up (time limit or abort raised elsewhere).  `seen` (optional): the value last read.
 static __device__ __noinline__ bool wait_counter(const unsigned long long* flag, unsigned long long want, const WaitCtx& w, int code, int peer, unsigned long long* seen = nullptr) {
   unsigned long long t0 = 0, have = 0;
   for (unsigned spins = 1;; spins++) {
-    have = ld_acquire_sys(flag);
+    have = ld_acquire(flag, w.one_gpu);
     if (have >= want) { if (seen) *seen = have; return true; }
     if ((spins & 31u) == 0) {
       if (*(volatile int*)w.ctx->abort_flag) return false;
@@ -457,7 +465,7 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   const long long mine = (long long)(rank * max_cta + cta) * kFlagStride;      // my counters in a peer's heap
 
   if (tid < ndata + 32) {                          // ---------------- waiter
-    WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta;
+    WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta; w.one_gpu = ka.one_gpu;
     unsigned long long seen_head[2] = {0, 0};      // what a peer had consumed when last looked: no need to look again while that is credit enough
     int k = 0;
     bool failed = false;
@@ -538,12 +546,12 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
     // One fence for both: what the data warps stored comes before the consumers' counters, what they read before the producers'.  It waits for the
     // acknowledgement of everything the CTA stored, so a credit costs up to a microsecond at the end of a call: 1 MiB blocks of an all-gather 31.6 us, 29.9
     // with plain stores for the heads, which nothing orders behind the reads.  A release per counter took 38.0, a warp of its own for the heads 32.5.
-    fence_sys();
+    fence_ranks(ka.one_gpu);
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int p = lane + 32 * q;
-      for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) st_relaxed_sys(reinterpret_cast<unsigned long long*>(s_heap[p] + tail_off + mine), ++sent[q]);
-      for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) st_relaxed_sys(reinterpret_cast<unsigned long long*>(s_heap[p] + head_off + mine), ++rcvd[q]);
+      for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[p] + tail_off + mine), ++sent[q], ka.one_gpu);
+      for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[p] + head_off + mine), ++rcvd[q], ka.one_gpu);
     }
     __syncwarp();
     if (lane == 0) { __threadfence_block(); s_published = k + 1; }

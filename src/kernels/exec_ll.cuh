@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
   __syncthreads();
   const int maxseg = s_maxseg;
   char* const my_heap = s_heap[rank];
-  WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta;
+  WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta; w.one_gpu = false;
   bool failed = false;
   unsigned long long t0 = 0;
 

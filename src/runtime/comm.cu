@@ -672,8 +672,10 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
         }
         ka.n_cta = n_cta; if (!use_llf) cut_fifo(c, n, n_cta, a, &ka);
         ka.last_first = crowds_l2(a, n);
+        ka.one_gpu = n == c->nranks;
         ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
       }
+      ka.one_gpu &= c->device == c0->device;
       ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
       aligned &= pe->offsets_aligned && ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(r)) & 15) == 0;
       c->stats.launches++;
