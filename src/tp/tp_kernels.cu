@@ -33,17 +33,22 @@ typedef __nv_bfloat16 bf16;
 constexpr int TP_BN = 256, RS_STAGES = 5, AG_STAGES = 5, TP_MAX_RANKS = 8;
 constexpr int TP_BM = PAIR_BM, TP_BK = PAIR_BK;
 
-__device__ __forceinline__ unsigned ld_acquire_sys_u32(const unsigned* p) {
-  unsigned v; asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v;
+// Flags, for ranks on several GPUs or (one_gpu) all of them in one launch.
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p, bool one_gpu) {
+  unsigned v;
+  if (one_gpu) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  else asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
-__device__ __forceinline__ void st_release_sys_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v, bool one_gpu) {
+  if (one_gpu) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  else asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // Bounded wait until *flag == epoch.
-__device__ __forceinline__ bool wait_flag(const unsigned* flag, unsigned epoch, volatile int* abort_flag) {
+__device__ __forceinline__ bool wait_flag(const unsigned* flag, unsigned epoch, bool one_gpu, volatile int* abort_flag) {
   unsigned long long t0 = 0;
   for (unsigned it = 1;; it++) {
-    if (ld_acquire_sys_u32(flag) == epoch) return true;
+    if (ld_acquire_u32(flag, one_gpu) == epoch) return true;
     if ((it & 63u) == 0) {
       if (*abort_flag) return false;
       unsigned long long now = gtime_ns();
@@ -75,6 +80,7 @@ struct TpArgs {
   int nv;                    // (virtual) ranks of this launch: every pair works for all of them, see the policies
   int n_part;                // ag_gemm: parts of a row block, each with a flag of its own
   unsigned epoch;
+  int one_gpu;               // all ranks in this launch: flags need no scope beyond the GPU
   long long flag_off, data_off;
   TpRank r[TP_MAX_RANKS];    // one entry per virtual rank of the launch
 };
@@ -140,7 +146,7 @@ struct RsPolicy {
     asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_u32(&s_arrived[pending_slot])) : "memory");
     if (before == PAIR_EPI_WARPS - 1) {
       s_arrived[pending_slot] = 0;                       // used again four tiles on, when every warp has left this one
-      st_release_sys_u32(pending, a.epoch);
+      st_release_u32(pending, a.epoch, a.one_gpu);
     }
     pending = nullptr;
   }
@@ -186,7 +192,7 @@ struct RsPolicy {
       return true;
     }
     // own tile: all other ranks' partials of this tile must have landed
-    const bool ok = e.lane >= n || e.lane == rank || wait_flag(flag_ptr(rank, e.lane, t), a.epoch, abort_flag);
+    const bool ok = e.lane >= n || e.lane == rank || wait_flag(flag_ptr(rank, e.lane, t), a.epoch, a.one_gpu, abort_flag);
     if (!__all_sync(0xffffffffu, ok)) return false;
 #pragma unroll 1
     for (int p = 0; p < 2; p++) {
@@ -299,7 +305,7 @@ struct AgPolicy {
     if (m_blk < 0 || m_blk / mb_per_shard == rank) return true;
     const int lane = threadIdx.x & 31;
     const unsigned* f = flags(R, rank, m_blk / mb_per_shard, m_blk % mb_per_shard);
-    const bool ok = lane >= a.n_part || wait_flag(f + lane, a.epoch, abort_flag);
+    const bool ok = lane >= a.n_part || wait_flag(f + lane, a.epoch, a.one_gpu, abort_flag);
     const bool all = __all_sync(0xffffffffu, ok);
     asm volatile("fence.proxy.async;" ::: "memory");    // the rows arrived before the flags; TMA reads them through the async proxy
     return all;
@@ -360,7 +366,7 @@ struct AgPolicy {
       }
       bulk_wait_all();                                   // the writes are performed; then tell the reader
       asm volatile("fence.proxy.async;" ::: "memory");
-      if (ok) st_release_sys_u32(flags(r, dest, from, mb) + part, a.epoch);
+      if (ok) st_release_u32(flags(r, dest, from, mb) + part, a.epoch, a.one_gpu);
     }
     if (!ok) { *abort_flag = 1; report(7); }
   }
@@ -440,11 +446,12 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
     if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) { cudaGetLastError(); return fail(PICCL_CUDA_ERROR, "no room for a pair of CTAs with %d bytes of shared memory each", smem_bytes); }
     c0->tp_pairs[which] = std::min(active, c0->sm_count / 2);
   }
-  a.nv = n;
+  a.nv = n; a.one_gpu = n == nr;
   bool ok = true;
   for (int i = 0; i < n && ok; i++) {
     piccl_comm* c = cs[i];
     TpRank& R = a.r[i];
+    a.one_gpu &= c->device == c0->device;
     R.rank = c->rank; R.out = (bf16*)out[i]; R.a_shard = (const bf16*)A[i];
     for (int p = 0; p < nr; p++) R.heap[p] = c->h_ctx.heap[p];
     if (!c->d_tp_status) { if (cudaMalloc(&c->d_tp_status, sizeof(int)) != cudaSuccess) { ok = false; break; } cudaMemset(c->d_tp_status, 0, sizeof(int)); }
