@@ -61,19 +61,23 @@ struct AttnCtx {
   __device__ bool wait(uint64_t* bar, uint32_t parity) const { return mbar_wait(bar, parity, abort, kAttnWaitLimitNs); }
 };
 
-// rows: warps that hold rows and arrive together; ready: arrivals that make the tile's own operands complete
-__device__ __forceinline__ void attn_begin(AttnCtx& c, uint8_t* raw, int* s_abort, uint32_t* s_tmem, int warp, int rows, int ready) {
+// rows: warps that hold rows and arrive together; ready: arrivals that make the tile's own operands complete.  first(): the loads that need nothing but the
+// barriers; the loading warp starts them while TMEM is allocated and the CTA assembles (a thousand clocks).
+template <class F>
+__device__ __forceinline__ void attn_begin(AttnCtx& c, uint8_t* raw, int* s_abort, uint32_t* s_tmem, int warp, int rows, int ready, const F& first) {
   c.smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   uint64_t* b = reinterpret_cast<uint64_t*>(c.smem + AttnSmem::BARS);
   c.full = b; c.empty = b + AT_STAGES; b += 2 * AT_STAGES;
   c.ready = b; c.s_full = b + 1; c.p_full = b + 3; c.acc_done = b + 5; c.dp_full = b + 7; c.ds_full = b + 8; c.sums = b + 9; c.own = b + 11;
   c.abort = s_abort;
-  if (threadIdx.x == 0) {
+  if (warp == AT_LOAD && elect_one()) {
     *s_abort = 0;
     for (int i = 0; i < AT_STAGES; i++) { mbar_init(&c.full[i], 1); mbar_init(&c.empty[i], 1); }
     for (int i = 0; i < 2; i++) { mbar_init(&c.s_full[i], 1); mbar_init(&c.p_full[i], rows); mbar_init(&c.acc_done[i], 1); mbar_init(&c.sums[i], 4); }
     mbar_init(c.ready, ready); mbar_init(c.dp_full, 1); mbar_init(c.ds_full, rows); mbar_init(c.own, 1);
     fence_barrier_init();
+    pdl_begin();
+    first(c);
   }
   if (warp == AT_MMA) tmem_alloc_cta(s_tmem, AT_TMEM);
   tc_fence_before();
@@ -165,27 +169,33 @@ __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t da, uint64_t db, uin
 }
 
 // The tiles of the steps, through a ring of STAGES: columns x0 of map 0 and x1 of map 1, rows 64 * (first + j), and those rows of r0 and r1.
-template <int STAGES>
-__device__ __forceinline__ bool attn_produce(const AttnCtx& c, const CUtensorMap* m0, int x0, const CUtensorMap* m1, int x1, int first, int steps, int b, const float* r0, const float* r1) {
-  const bool issuer = elect_one();
-  for (int j = 0; j < steps; j++) {
-    const int st = j % STAGES;
-    if (!c.wait(&c.empty[st], ((j / STAGES) & 1) ^ 1)) return false;
-    if (issuer) {
-      uint8_t* s = c.smem + st * AttnSmem::STAGE;
-      mbar_arrive_expect_tx(&c.full[st], AttnSmem::STAGE + (r0 ? 2 * AT_STEP * 4 : 0));
-      tma_load_3d(s, m0, x0, (first + j) * AT_STEP, b, &c.full[st]);
-      tma_load_3d(s + AT_TILE, m1, x1, (first + j) * AT_STEP, b, &c.full[st]);
-      if (r0) {
-        uint8_t* q = c.smem + AttnSmem::ROWS + st * 2 * AT_STEP * 4;
-        bulk_load(q, r0 + (first + j) * AT_STEP, AT_STEP * 4, &c.full[st]);
-        bulk_load(q + AT_STEP * 4, r1 + (first + j) * AT_STEP, AT_STEP * 4, &c.full[st]);
-      }
+struct AttnSteps {
+  const CUtensorMap *m0, *m1;
+  int x0, x1, first, steps, b;
+  const float *r0, *r1;
+  __device__ __forceinline__ void load(const AttnCtx& c, int j, int st) const {      // one thread
+    uint8_t* s = c.smem + st * AttnSmem::STAGE;
+    mbar_arrive_expect_tx(&c.full[st], AttnSmem::STAGE + (r0 ? 2 * AT_STEP * 4 : 0));
+    tma_load_3d(s, m0, x0, (first + j) * AT_STEP, b, &c.full[st]);
+    tma_load_3d(s + AT_TILE, m1, x1, (first + j) * AT_STEP, b, &c.full[st]);
+    if (r0) {
+      uint8_t* q = c.smem + AttnSmem::ROWS + st * 2 * AT_STEP * 4;
+      bulk_load(q, r0 + (first + j) * AT_STEP, AT_STEP * 4, &c.full[st]);
+      bulk_load(q + AT_STEP * 4, r1 + (first + j) * AT_STEP, AT_STEP * 4, &c.full[st]);
     }
-    __syncwarp();
   }
-  return true;
-}
+  template <int STAGES> __device__ __forceinline__ void begin(const AttnCtx& c) const { for (int j = 0; j < STAGES && j < steps; j++) load(c, j, j); }      // one thread
+  template <int STAGES> __device__ __forceinline__ bool rest(const AttnCtx& c) const {
+    const bool issuer = elect_one();
+    for (int j = STAGES; j < steps; j++) {
+      const int st = j % STAGES;
+      if (!c.wait(&c.empty[st], ((j / STAGES) & 1) ^ 1)) return false;
+      if (issuer) load(c, j, st);
+      __syncwarp();
+    }
+    return true;
+  }
+};
 // 128 rows of a matrix -> 16 KiB of shared memory
 __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, int x, int row0, int b, uint64_t* bar) {
   for (int i = 0; i < 2; i++) tma_load_3d(dst + i * AT_TILE, m, x, row0 + i * AT_STEP, b, bar);
@@ -202,18 +212,20 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_fwd_kernel(const __grid_co
   __shared__ int s_abort;
   __shared__ uint32_t s_tmem;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  AttnCtx c;
-  attn_begin(c, smem_raw, &s_abort, &s_tmem, warp, 4, 1);
   const int heads = a.B * a.H, tile = a.tiles - 1 - blockIdx.x / heads, bh = blockIdx.x % heads, b = bh / a.H, h = bh % a.H, C = a.H * AT_D, q0 = tile * AT_ROWS;
   const int steps = (min(a.S, q0 + AT_ROWS) + AT_STEP - 1) / AT_STEP;
   constexpr uint32_t T_O = 0, T_S = 128;
+  const AttnSteps keys{&a.qkv, &a.qkv, C + h * AT_D, 2 * C + h * AT_D, 0, steps, b, nullptr, nullptr};
+  AttnCtx c;
+  attn_begin(c, smem_raw, &s_abort, &s_tmem, warp, 4, 1, [&](const AttnCtx& c) {
+    mbar_arrive_expect_tx(c.ready, 2 * AT_TILE);
+    load_tile(c.smem + AttnSmem::OWN, &a.qkv, h * AT_D, q0, b, c.ready);
+    keys.begin<AT_STAGES>(c);
+  });
   bool ok = true;
 
-  if (warp == AT_LOAD) {
-    if (elect_one()) { mbar_arrive_expect_tx(c.ready, 2 * AT_TILE); load_tile(c.smem + AttnSmem::OWN, &a.qkv, h * AT_D, q0, b, c.ready); }
-    __syncwarp();
-    ok = attn_produce<AT_STAGES>(c, &a.qkv, C + h * AT_D, &a.qkv, 2 * C + h * AT_D, 0, steps, b, nullptr, nullptr);
-  } else if (warp == AT_MMA) {
+  if (warp == AT_LOAD) ok = keys.rest<AT_STAGES>(c);
+  else if (warp == AT_MMA) {
     const bool issuer = elect_one();
     const uint64_t dq = make_smem_desc_k128(c.smem + AttnSmem::OWN), dk0 = make_smem_desc_k128(c.smem), dv0 = make_smem_desc_mn128(c.smem + AT_TILE);
     auto scores = [&](int j) {
@@ -336,23 +348,23 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_dq_kernel(const __grid_con
   __shared__ int s_abort;
   __shared__ uint32_t s_tmem;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  AttnCtx c;
-  attn_begin(c, smem_raw, &s_abort, &s_tmem, warp, 8, 8);
   const int heads = a.B * a.H, tile = a.tiles - 1 - blockIdx.x / heads, bh = blockIdx.x % heads, b = bh / a.H, h = bh % a.H, C = a.H * AT_D, q0 = tile * AT_ROWS;
   const int steps = (min(a.S, q0 + AT_ROWS) + AT_STEP - 1) / AT_STEP;
   constexpr int STAGES = AT_STAGES - 1;                  // the last stage's place has the tile of the output
-  uint8_t* const own = c.smem + AttnSmem::OWN;           // Q, then dO
   constexpr uint32_t T_Q = 0, T_DO = 32, T_DQ = 64, T_S = 128, T_DP = 192;
+  const AttnSteps keys{&a.qkv, &a.qkv, C + h * AT_D, 2 * C + h * AT_D, 0, steps, b, nullptr, nullptr};
+  AttnCtx c;
+  attn_begin(c, smem_raw, &s_abort, &s_tmem, warp, 8, 8, [&](const AttnCtx& c) {
+    uint8_t* const t = c.smem + AttnSmem::OWN;
+    mbar_arrive_expect_tx(c.own, 6 * AT_TILE);
+    load_tile(t, &a.qkv, h * AT_D, q0, b, c.own); load_tile(t + 2 * AT_TILE, &a.dout, h * AT_D, q0, b, c.own); load_tile(c.smem + STAGES * AttnSmem::STAGE, &a.out, h * AT_D, q0, b, c.own);
+    keys.begin<STAGES>(c);
+  });
+  uint8_t* const own = c.smem + AttnSmem::OWN;           // Q, then dO
   bool ok = true;
 
-  if (warp == AT_LOAD) {
-    if (elect_one()) {
-      mbar_arrive_expect_tx(c.own, 6 * AT_TILE);
-      load_tile(own, &a.qkv, h * AT_D, q0, b, c.own); load_tile(own + 2 * AT_TILE, &a.dout, h * AT_D, q0, b, c.own); load_tile(c.smem + STAGES * AttnSmem::STAGE, &a.out, h * AT_D, q0, b, c.own);
-    }
-    __syncwarp();
-    ok = attn_produce<STAGES>(c, &a.qkv, C + h * AT_D, &a.qkv, 2 * C + h * AT_D, 0, steps, b, nullptr, nullptr);
-  } else if (warp == AT_MMA) {
+  if (warp == AT_LOAD) ok = keys.rest<STAGES>(c);
+  else if (warp == AT_MMA) {
     const bool issuer = elect_one();
     const uint64_t dk0 = make_smem_desc_k128(c.smem), dv0 = make_smem_desc_k128(c.smem + AT_TILE), dkn0 = make_smem_desc_mn128(c.smem);
     auto scores = [&](int j) {
@@ -465,23 +477,23 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_dkv_kernel(const __grid_co
   __shared__ int s_abort;
   __shared__ uint32_t s_tmem;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  AttnCtx c;
-  attn_begin(c, smem_raw, &s_abort, &s_tmem, warp, 8, 1);
   const int heads = a.B * a.H, tile = blockIdx.x / heads, bh = blockIdx.x % heads, b = bh / a.H, h = bh % a.H, C = a.H * AT_D, k0 = tile * AT_ROWS;
   const int first = k0 / AT_STEP, steps = (a.S + AT_STEP - 1) / AT_STEP - first;
   constexpr uint32_t T_DK = 0, T_DV = 64, T_S = 128, T_DP = 192;
+  const size_t at = (size_t)bh * a.tiles * AT_ROWS;
+  const AttnSteps queries{&a.qkv, &a.dout, h * AT_D, h * AT_D, first, steps, b, a.lse + at, a.delta + at};
+  AttnCtx c;
+  attn_begin(c, smem_raw, &s_abort, &s_tmem, warp, 8, 1, [&](const AttnCtx& c) {
+    uint8_t* const t = c.smem + AttnSmem::OWN;
+    mbar_arrive_expect_tx(c.ready, 4 * AT_TILE);
+    load_tile(t, &a.qkv, C + h * AT_D, k0, b, c.ready); load_tile(t + 2 * AT_TILE, &a.qkv, 2 * C + h * AT_D, k0, b, c.ready);
+    queries.begin<AT_STAGES>(c);
+  });
   uint8_t* const own = c.smem + AttnSmem::OWN;           // K, then V: 128 rows each
   bool ok = true;
 
-  if (warp == AT_LOAD) {
-    if (elect_one()) {
-      mbar_arrive_expect_tx(c.ready, 4 * AT_TILE);
-      load_tile(own, &a.qkv, C + h * AT_D, k0, b, c.ready); load_tile(own + 2 * AT_TILE, &a.qkv, 2 * C + h * AT_D, k0, b, c.ready);
-    }
-    __syncwarp();
-    const size_t at = (size_t)bh * a.tiles * AT_ROWS;
-    ok = attn_produce<AT_STAGES>(c, &a.qkv, h * AT_D, &a.dout, h * AT_D, first, steps, b, a.lse + at, a.delta + at);
-  } else if (warp == AT_MMA) {
+  if (warp == AT_LOAD) ok = queries.rest<AT_STAGES>(c);
+  else if (warp == AT_MMA) {
     const bool issuer = elect_one();
     const uint64_t k_own = make_smem_desc_k128(own), v_own = make_smem_desc_k128(own + 2 * AT_TILE);
     const uint64_t dq0 = make_smem_desc_k128(c.smem), do0 = make_smem_desc_k128(c.smem + AT_TILE), dqn0 = make_smem_desc_mn128(c.smem), don0 = make_smem_desc_mn128(c.smem + AT_TILE);
