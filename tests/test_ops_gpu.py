@@ -212,3 +212,24 @@ def test_layernorm_backward_takes_a_row_split():
         ops.layernorm_bwd(dy, x, gamma, mean, rstd, None, *out, *split)
         got.append(out)
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def test_partial_rows_of_any_width_and_alignment():
+    """Vectors folded together whose rows are not whole pairs, or begin in the middle of one, beside one that is read in pairs; up to more rows than are in flight."""
+    import ctypes as C
+    from piccl_b200 import _native as N
+    from piccl_b200.ops import _FinishJob, _s
+    g = torch.Generator(device="cuda").manual_seed(3)
+    jobs, want, outs, keep = [], [], [], []
+    for n, Cc, shift, acc in [(1, 1, 0, 0), (33, 77, 0, 1), (16, 64, 1, 0), (160, 66, 0, 1), (161, 130, 0, 0), (500, 63, 1, 0)]:
+        flat = torch.randn(n * Cc + shift, generator=g, device="cuda")
+        part = flat[shift:].view(n, Cc)
+        out = torch.randn(Cc, generator=g, device="cuda").bfloat16()
+        want.append(part.double().sum(0) + (out.double() if acc else 0))
+        outs.append(out)
+        keep.append(flat)
+        jobs.append((part.data_ptr(), out.data_ptr(), n, Cc, acc, 0))
+    assert N.ops_lib().piccl_ops_finish_parts((_FinishJob * len(jobs))(*jobs), len(jobs), C.c_void_p(_s())) == 0
+    for w, o, f in zip(want, outs, keep):
+        # one rounding to bf16 of the sum, and of each of the fp32 additions
+        assert ((o.double() - w).abs() <= 2.0 ** -8 * w.abs() + f.numel() * 2.0 ** -24 * f.abs().max()).all()
