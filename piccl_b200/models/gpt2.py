@@ -12,8 +12,9 @@ flat fp32 buffers and are updated by one fused kernel per parameter group.
 The step itself is native (src/model/gpt2_step.cc): residual-add + LayerNorm
 (forward / backward), GEMMs with fused GELU, bias gradients, embedding, softmax cross
 entropy with in-place gradient and AdamW are this framework's CUDA kernels (src/ops);
-so is attention of heads of 64 columns (other widths, and other back ends that the
-program asks PyTorch for, go through PyTorch's fused kernels).
+for heads of 64 columns so are the backward pass of attention and its forward pass in an
+evaluation (the rest, and other back ends that the program asks PyTorch for, goes
+through PyTorch's fused kernels).
 
 The reference has no model code at all; this module exists for the end-to-end
 data-parallel benchmark (GPT-2 medium under bucketed gradient all-reduce).

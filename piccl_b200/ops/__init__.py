@@ -110,16 +110,18 @@ def cross_entropy_fwd_bwd(logits, targets, loss_rows, vocab: int, gscale: float)
 
 
 def attention_fwd(qkv, out, lse, batch: int):
-    """Causal attention of packed rows [batch * S, 3 * heads * 64] -> [batch * S, heads * 64]; lse: batch * heads * (S rounded up to 128) floats, or None."""
+    """Causal attention of packed rows [batch * S, 3 * heads * 64] -> [batch * S, heads * 64]; lse: [batch * heads, S] floats, the logarithm of each row's sum of
+    exponentials, or None."""
     rows, Cc = out.shape
     _chk(N.ops_lib().piccl_ops_attn_fwd(_p(qkv), _p(out), _p(lse), batch, rows // batch, Cc // 64, C.c_void_p(_s())), "attn_fwd")
     _bump()
 
 
-def attention_bwd(qkv, out, dout, lse, delta, dqkv, part, batch: int):
-    """dqkv, the gradient of the packed rows, and in part its partial column sums: one row per batch entry and 128 positions.  delta: scratch like lse."""
+def attention_bwd(qkv, out, dout, lse, scratch, dqkv, part, batch: int):
+    """dqkv, the gradient of the packed rows, and in part its partial column sums: one row per batch entry and 128 positions.
+    scratch: 2 * batch * heads * (S rounded up to 128) floats."""
     rows, Cc = out.shape
-    _chk(N.ops_lib().piccl_ops_attn_bwd(_p(qkv), _p(out), _p(dout), _p(lse), _p(delta), _p(dqkv), _p(part), batch, rows // batch, Cc // 64, C.c_void_p(_s())), "attn_bwd")
+    _chk(N.ops_lib().piccl_ops_attn_bwd(_p(qkv), _p(out), _p(dout), _p(lse), _p(scratch), _p(dqkv), _p(part), batch, rows // batch, Cc // 64, C.c_void_p(_s())), "attn_bwd")
     _bump(2)
 
 

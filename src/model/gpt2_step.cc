@@ -2,8 +2,8 @@
 //
 // Why native: the step is a few dozen launches per layer, and issued from Python each cost about 15 us of host time: two layers of
 // 256 columns took 1.4 ms for 0.3 ms of kernels, eight layers of 768 columns 4.5 ms for 2.7 ms.  Here a launch of this framework's
-// own kernels is a plain call (2 to 3 us); attention of heads of 64 columns is one of them, of other heads it goes through ATen's fused kernels
-// without autograd.
+// own kernels is a plain call (2 to 3 us); attention goes through ATen's fused kernels without autograd, but for heads of 64 columns the way back, and
+// the forward pass of an evaluation, are this framework's.
 //
 // A step of the same shape on the same input buffers is captured into a CUDA graph by the caller (models/gpt2.py).  Its weight gradients and
 // column sums, which nothing in the backward pass waits for, can then go to a second stream: small ones fill the SMs that the chain of
@@ -115,16 +115,16 @@ struct Carve {
   }
 };
 
-struct Layer { b16 *ln1, *qkv, *att, *x2, *ln2, *h, *gl, *x3; float *mean1, *rstd1, *mean2, *rstd2, *lse; };
+struct Layer { b16 *ln1, *qkv, *att, *x2, *ln2, *h, *gl, *x3; float *mean1, *rstd1, *mean2, *rstd2; };
 struct Buffers {
   b16 *x0, *a, *pr, *logits, *dln, *dln2, *datt, *dln1;
   b16 *dxa[3], *dxb[2], *dg[2], *dqkv[2];      // taken in turn by the layers: weight gradients may still read those of the layer above
-  float *loss_rows, *parts[2], *delta;
+  float *loss_rows, *parts[2], *row_sums;
   std::vector<Layer> layer;         // L + 1: the last one holds the input of the head
 };
 
-// lse_floats: of the attention kernels' row sums, 0 where attention is ATen's
-void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, size_t lse_floats, Buffers& b) {
+// row_floats: scratch of the attention kernels, 0 where attention is ATen's
+void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, size_t row_floats, Buffers& b) {
   const size_t C = d.C;
   b.x0 = c.get<b16>(T * C); b.a = c.get<b16>(T * C); b.pr = c.get<b16>(T * C);
   b.layer.resize(d.L + 1);
@@ -134,14 +134,14 @@ void carve(Carve& c, const Desc& d, size_t T, bool train, size_t part_floats, si
     y.ln1 = c.get<b16>(T * C); y.mean1 = c.get<float>(T); y.rstd1 = c.get<float>(T);
     if (train && l == d.L) continue;
     y.qkv = c.get<b16>(T * 3 * C); y.x2 = c.get<b16>(T * C); y.ln2 = c.get<b16>(T * C); y.mean2 = c.get<float>(T); y.rstd2 = c.get<float>(T);
-    y.att = lse_floats ? c.get<b16>(T * C) : nullptr; y.lse = lse_floats && train ? c.get<float>(lse_floats) : nullptr;
+    y.att = row_floats && !train ? c.get<b16>(T * C) : nullptr;
     y.h = train ? c.get<b16>(T * 4 * C) : nullptr; y.gl = c.get<b16>(T * 4 * C); y.x3 = c.get<b16>(T * C);
   }
   b.logits = c.get<b16>(T * d.Vp); b.loss_rows = c.get<float>(T);
   if (!train) return;
   for (b16*& x : b.dxa) x = c.get<b16>(T * C);
   for (int q = 0; q < 2; q++) { b.dxb[q] = c.get<b16>(T * C); b.dg[q] = c.get<b16>(T * 4 * C); b.dqkv[q] = c.get<b16>(T * 3 * C); }
-  b.delta = c.get<float>(lse_floats);
+  b.row_sums = c.get<float>(row_floats);
   b.dln = c.get<b16>(T * C); b.dln2 = c.get<b16>(T * C); b.datt = c.get<b16>(T * C); b.dln1 = c.get<b16>(T * C); for (float*& x : b.parts) x = c.get<float>(part_floats);
 }
 
@@ -225,15 +225,17 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
 
   // partial rows of the column sums: dgamma, dbeta and bias gradient of both LayerNorms, the MLP's and the attention's bias gradients
   const int n_ln = piccl_ops_ln_bwd_parts(T, C), n_qkv = piccl_ops_col_parts(T, 3 * C), n_fc_own = (T + 31) / 32, n_fc_sep = piccl_ops_col_parts(T, 4 * C);
-  // Heads of 64 columns: this framework's kernels, where PyTorch would take cuDNN's (a program that asks for another back end gets that one).
-  // (Any address will do for the question.)
+  // Heads of 64 columns: this framework's kernels, where PyTorch would take cuDNN's (a program that asks for another back end gets that one; any address will do
+  // for the question).  A training step keeps cuDNN's forward kernel, whose sums of exponentials the way back takes as they are: the two forward kernels are equally
+  // exact and fast (2.0e-3 off fp64; 8 x 1024 tokens 40 us, own 41), but another order of its sums rolls the rounding of every activation above it anew, and gradients
+  // of one step then differ by 0.95 % from those that this model has had, with the own way back alone by 0.48 % (8 layers of 768 columns).
   const bool own_attention = D == 64 && sdp_choice(d.p, B, S, H, D) == kCudnnAttention;
   const int n_att = own_attention ? piccl_ops_attn_parts(B, S) : 0;
   const size_t row = (size_t)n_ln * C, fc_floats = (size_t)std::max(n_fc_own, n_fc_sep) * 4 * C, part_floats = 6 * row + fc_floats + (size_t)std::max(n_qkv, n_att) * 3 * C;
-  const size_t lse_floats = own_attention ? (size_t)B * H * piccl_ops_attn_rows(S) : 0;
+  const size_t row_floats = own_attention ? (size_t)2 * B * H * piccl_ops_attn_rows(S) : 0;
   Buffers b;
   Carve count{nullptr};
-  carve(count, d, T, train, part_floats, lse_floats, b);
+  carve(count, d, T, train, part_floats, row_floats, b);
   if (!m.arena.defined() || (size_t)m.arena.numel() < count.used) {
     if (m.in_callers_graph) m.kept.push_back(m.arena);
     m.in_callers_graph = false;
@@ -243,7 +245,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   const bool in_capture = capturing(main_stream);
   m.in_callers_graph |= !m.captured && in_capture;
   Carve c{static_cast<char*>(m.arena.data_ptr())};
-  carve(c, d, T, train, part_floats, lse_floats, b);
+  carve(c, d, T, train, part_floats, row_floats, b);
   b16 *const lnf_g = d.p + m.off[0], *const lnf_b = d.p + m.off[1], *const wpe = d.p + m.off[2], *const wte = d.p + m.off[3];
   if (!m.split.defined()) {
     m.split = at::empty({2, (int64_t)kSplitBytes}, opt.dtype(at::kByte));
@@ -265,7 +267,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   for (int l = 0; l < L; l++) {
     Layer& y = b.layer[l]; Layer& z = b.layer[l + 1];
     DO(product(m, NT, y.ln1, m.p(l, W_QKV), y.qkv, m.p(l, B_QKV), T, 3 * C, C, s));
-    if (own_attention) TRY(piccl_ops_attn_fwd(y.qkv, y.att, y.lse, B, S, H, s));
+    if (own_attention && !train) TRY(piccl_ops_attn_fwd(y.qkv, y.att, nullptr, B, S, H, s));
     else { att[l] = attention(m.saved[l], y.qkv, B, S, H, D, train); y.att = static_cast<b16*>(att[l].data_ptr()); }
     DO(product(m, NT, y.att, m.p(l, W_O), b.a, m.p(l, B_O), T, C, C, s));
     if (!train) { m.saved[l] = Saved(); att[l] = at::Tensor(); }
@@ -350,7 +352,8 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
     int n_q = n_qkv;
     if (own_attention) {
       n_q = n_att;
-      TRY(piccl_ops_attn_bwd(y.qkv, y.att, b.datt, y.lse, b.delta, dqkv, ws_qkv, B, S, H, s));
+      const at::Tensor lse = m.saved[l].lse.contiguous();      // [B, H, S]
+      TRY(piccl_ops_attn_bwd(y.qkv, y.att, b.datt, lse.data_ptr<float>(), b.row_sums, dqkv, ws_qkv, B, S, H, s));
       m.launches++;                   // two kernels
     } else {
       at::Tensor dq[3];

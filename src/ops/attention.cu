@@ -16,9 +16,9 @@
 // 512 clocks of an SM's special-function units (16 results a clock) and 256 / 384 / 640 of its tensor cores (forward, dQ, dK and dV; the last
 // reads K and V from shared memory for every step); what is measured is 1070 / 1100 / 1550, most of it the way from one product through
 // the threads to the next and the start and end of a CTA.  (A third of the exponentials as polynomials on the fma units changed nothing.)
-// 8 x 1024 tokens, 16 heads, within a training step of GPT-2 medium: forward 41 us, backward 112, where cuDNN's kernels with the conversion of dQ, the sum o * do, and the
-// packing and column sums of the gradient took 40 and 123; 4 x 128 tokens,
-// 4 heads, alone and with events around each: 10 and 15 us, cuDNN 11 and 27.
+// 8 x 1024 tokens, 16 heads, within a training step of GPT-2 medium: backward 112 us, where cuDNN's kernel with the sum o * do, the conversion of dQ and the
+// packing and column sums of the gradient took 123 in five launches; forward 41, cuDNN 40.  Back to back on a stream: 8 x 1024 tokens 35 and 95, 3 x 777 with 12 heads 13.7 and 36.3,
+// 4 x 128 with 4 heads 4.5 and 9.9.
 // Blocks are ordered by falling length of their walk.
 #include <cstring>
 #include <mutex>
@@ -36,7 +36,8 @@ constexpr unsigned long long kAttnWaitLimitNs = 4000000000ull;
 
 struct AttnArgs {
   CUtensorMap qkv, out, dout, result;   // 64 rows of the packed rows, of the output and its gradient; 32 rows of the result
-  float *lse, *delta, *part;            // [B * H][tiles * 128] minus log2 of the row's sum of exponentials (-inf beyond S), minus the sum of o * do; [B * tiles][3 H D]
+  const float* lse_in;                  // [B * H][S] logarithm of the row's sum of exponentials
+  float *lse_out, *lse, *delta, *part;  // the same; [B * H][tiles * 128] minus that to base 2 (-inf beyond S), minus the sum of o * do; [B * tiles][3 H D]
   int B, S, H, tiles;
   int* status;
 };
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_fwd_kernel(const __grid_co
       const float2 w = other[r];
       const float top = fmaxf(m, w.x);                   // finite: key 0 is in a step of group 0
       const float f0 = ex2_approx((m - top) * kAttnLog2), f1 = w.x == -INFINITY ? 0.f : ex2_approx((w.x - top) * kAttnLog2), sum = l * f0 + w.y * f1, inv = 1.f / sum;
-      if (a.lse) a.lse[(size_t)bh * a.tiles * AT_ROWS + row] = row < a.S ? -fmaf(top, kAttnLog2, log2f(sum)) : -INFINITY;
+      if (a.lse_out && row < a.S) a.lse_out[(size_t)bh * a.S + row] = fmaf(top, kAttnScale, logf(sum));
       uint8_t* const piece = c.smem + AttnSmem::OWN + warp * 4096;      // Q has been read for the last time
 #pragma unroll
       for (int q = 0; q < 2; q++) {
@@ -401,7 +402,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_dq_kernel(const __grid_con
     const int g = warp >> 2, r = (warp & 3) * 32 + lane, row = q0 + r;
     const uint32_t lanes = c.tmem + ((uint32_t)((warp & 3) * 32) << 16), ts = lanes + T_S + 32 * g, tdp = lanes + T_DP + 32 * g;
     const size_t pad = (size_t)bh * a.tiles * AT_ROWS + row;
-    const f32x2 n2 = both2(a.lse[pad]);
+    const float minus_lse = row < a.S ? a.lse_in[(size_t)bh * a.S + row] * -1.4426950408889634f : -INFINITY;
+    const f32x2 n2 = both2(minus_lse);
     float* const rows = reinterpret_cast<float*>(c.smem + AttnSmem::ROWS);
     ok = c.wait(c.own, 0);
     {
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_dq_kernel(const __grid_con
           d = fmaf(u.x, v.x, d); d = fmaf(u.y, v.y, d);
         }
         rows[r] = -d;
-        a.delta[pad] = -d;
+        a.delta[pad] = -d; a.lse[pad] = minus_lse;
       }
       tmem_st_wait();
       if (ok) warp_arrive(c.ready, lane);
@@ -609,26 +611,26 @@ using namespace piccl_ops;
 extern "C" {
 
 // Causal attention of packed rows qkv [B * S, 3 * H * 64] -> out [B * S, H * 64], all bf16, contiguous, 16-byte aligned.
-// lse (null: not wanted): B * H * piccl_ops_attn_rows(S) floats for the backward pass, minus log2 of each row's sum of exponentials, -inf beyond S.
+// lse (null: not wanted): B * H * S floats, the logarithm of the sum of exponentials of each row's scaled scores.
 int piccl_ops_attn_rows(int S) { return (S + AT_ROWS - 1) / AT_ROWS * AT_ROWS; }
 int piccl_ops_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, void* stream) {
   if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return -2;
   AttnArgs a;
   const int rc = attn_args(a, qkv, B, S, H); if (rc) return rc;
   if (!make_tmap_bf16_rows(&a.result, out, B, S, (uint64_t)H * AT_D, 32)) return -3;
-  a.out = a.dout = a.qkv; a.lse = lse;
+  a.out = a.dout = a.qkv; a.lse_out = lse;
   return launch_pdl(attn_fwd_kernel, B * H * a.tiles, AT_THREADS, AttnSmem::DYNAMIC, (cudaStream_t)stream, a) == cudaSuccess ? 0 : -5;
 }
-// dqkv: gradient of qkv; part: [piccl_ops_attn_parts(B, S)][3 * H * 64] floats, its partial column sums; delta: as many floats as lse, scratch.
+// lse: as above, from whichever kernel computed out.  dqkv: gradient of qkv; part: [piccl_ops_attn_parts(B, S)][3 * H * 64] floats, its partial column sums; scratch: 2 * B * H *
+// piccl_ops_attn_rows(S) floats, 16-byte aligned.
 int piccl_ops_attn_parts(int B, int S) { return B * ((S + AT_ROWS - 1) / AT_ROWS); }
-int piccl_ops_attn_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv, float* part, int B, int S, int H, void* stream) {
-  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dqkv) | reinterpret_cast<uintptr_t>(lse) |
-       reinterpret_cast<uintptr_t>(delta)) & 15) return -2;
+int piccl_ops_attn_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* scratch, void* dqkv, float* part, int B, int S, int H, void* stream) {
+  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dqkv) | reinterpret_cast<uintptr_t>(scratch)) & 15) return -2;
   AttnArgs a;
   const int rc = attn_args(a, qkv, B, S, H); if (rc) return rc;
   if (!make_tmap_bf16_rows(&a.out, out, B, S, (uint64_t)H * AT_D, AT_STEP) || !make_tmap_bf16_rows(&a.dout, dout, B, S, (uint64_t)H * AT_D, AT_STEP) ||
       !make_tmap_bf16_rows(&a.result, dqkv, B, S, 3ull * H * AT_D, 32)) return -3;
-  a.lse = const_cast<float*>(lse); a.delta = delta; a.part = part;
+  a.lse_in = lse; a.lse = scratch; a.delta = scratch + (size_t)B * H * a.tiles * AT_ROWS; a.part = part;
   const int grid = B * H * a.tiles;
   if (launch_pdl(attn_dq_kernel, grid, AT_THREADS, AttnSmem::DYNAMIC, (cudaStream_t)stream, a) != cudaSuccess) return -5;
   return launch_pdl(attn_dkv_kernel, grid, AT_THREADS, AttnSmem::DYNAMIC, (cudaStream_t)stream, a) == cudaSuccess ? 0 : -5;

@@ -23,7 +23,7 @@ int piccl_ops_wte_bwd_rows(const long long* idx, const void* dx, float* stage, i
 int piccl_ops_attn_rows(int S);
 int piccl_ops_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, void* stream);
 int piccl_ops_attn_parts(int B, int S);
-int piccl_ops_attn_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv, float* part, int B, int S, int H, void* stream);
+int piccl_ops_attn_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* scratch, void* dqkv, float* part, int B, int S, int H, void* stream);
 #ifdef __cplusplus
 }
 #endif
