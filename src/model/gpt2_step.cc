@@ -350,7 +350,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
     DO(weight_grad(dxb, y.att, m.g(l, W_O), C, C));
     DO(product(m, NN, dxb, m.p(l, W_O), b.datt, nullptr, T, C, C, s));
     int n_q = n_qkv;
-    if (own_attention) {
+    if (own_attention && m.saved[l].direct) {
       n_q = n_att;
       const at::Tensor lse = m.saved[l].lse.contiguous();      // [B, H, S]
       TRY(piccl_ops_attn_bwd(y.qkv, y.att, b.datt, lse.data_ptr<float>(), b.row_sums, dqkv, ws_qkv, B, S, H, s));
