@@ -581,17 +581,15 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_dkv_kernel(const __grid_co
   attn_end(c, warp, lane);
 }
 
-static int* g_attn_status[64] = {nullptr};
-static std::mutex g_attn_mu;
+// (nothing but attributes: the first call may lie inside a stream capture)
 static int attn_ready(int dev) {
-  std::lock_guard<std::mutex> l(g_attn_mu);
-  if (g_attn_status[dev]) return 0;
+  static std::mutex mu;
+  static bool ready[64] = {false};
+  std::lock_guard<std::mutex> l(mu);
+  if (ready[dev]) return 0;
   for (const void* f : {(const void*)attn_fwd_kernel, (const void*)attn_dq_kernel, (const void*)attn_dkv_kernel})
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem::DYNAMIC) != cudaSuccess) return -4;
-  int* p = nullptr;
-  if (cudaMalloc(&p, sizeof(int)) != cudaSuccess) return -7;
-  cudaMemset(p, 0, sizeof(int));
-  g_attn_status[dev] = p;
+  ready[dev] = true;
   return 0;
 }
 static int attn_args(AttnArgs& a, const void* qkv, int B, int S, int H) {
@@ -600,7 +598,8 @@ static int attn_args(AttnArgs& a, const void* qkv, int B, int S, int H) {
   if (dev < 0 || dev >= 64) return -6;
   const int rc = attn_ready(dev); if (rc) return rc;
   memset(&a, 0, sizeof a);
-  a.B = B; a.S = S; a.H = H; a.tiles = (S + AT_ROWS - 1) / AT_ROWS; a.status = g_attn_status[dev];
+  a.B = B; a.S = S; a.H = H; a.tiles = (S + AT_ROWS - 1) / AT_ROWS; a.status = status_word(STATUS_ATTENTION);
+  if (!a.status) return -7;
   return make_tmap_bf16_rows(&a.qkv, qkv, B, S, 3ull * H * AT_D, AT_STEP) ? 0 : -3;
 }
 
@@ -636,11 +635,6 @@ int piccl_ops_attn_bwd(const void* qkv, const void* out, const void* dout, const
   return launch_pdl(attn_dkv_kernel, grid, AT_THREADS, AttnSmem::DYNAMIC, (cudaStream_t)stream, a) == cudaSuccess ? 0 : -5;
 }
 // Non-zero if an attention kernel on the current device gave up on a wait (10 / 20 / 30 + warp).  Synchronises.
-int piccl_ops_attn_status(void) {
-  int dev = 0; cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !g_attn_status[dev]) return 0;
-  int v = 0; cudaMemcpy(&v, g_attn_status[dev], sizeof v, cudaMemcpyDeviceToHost);
-  return v;
-}
+int piccl_ops_attn_status(void) { return read_status(STATUS_ATTENTION); }
 
 }  // extern "C"

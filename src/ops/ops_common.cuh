@@ -26,6 +26,11 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Status word of the current device (status.cu); null if there is no device.
+enum StatusKind { STATUS_ATTENTION, kStatusKinds };
+int* status_word(StatusKind kind);
+int read_status(StatusKind kind);         // synchronises
+
 struct alignas(16) bf16x8 { __nv_bfloat162 v[4]; };
 
 __device__ __forceinline__ void unpack8(const bf16x8& p, float (&f)[8]) {

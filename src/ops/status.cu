@@ -1,0 +1,34 @@
+// Status words of the kernels whose waits are bounded: 0, or the role that gave up.  One of each kind per device, in the library's image: nothing is allocated at a
+// kernel's first use, which may lie inside a caller's stream capture (an allocation or a copy on the default stream there ends the capture).
+#include <atomic>
+#include "ops_common.cuh"
+
+namespace piccl_ops {
+
+__device__ int g_status_words[kStatusKinds];
+
+int* status_word(StatusKind kind) {
+  static std::atomic<int*> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  int* p = known[dev].load(std::memory_order_acquire);
+  if (!p) {                           // may load the module: a capture in the default mode would refuse that
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* a = nullptr;
+    const cudaError_t e = cudaGetSymbolAddress(&a, g_status_words);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    p = static_cast<int*>(a);
+    known[dev].store(p, std::memory_order_release);
+  }
+  return p + kind;
+}
+int read_status(StatusKind kind) {
+  const int* p = status_word(kind);
+  int v = 0;
+  if (p) cudaMemcpy(&v, p, sizeof v, cudaMemcpyDeviceToHost);
+  return v;
+}
+
+}  // namespace piccl_ops

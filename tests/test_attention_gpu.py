@@ -85,3 +85,37 @@ def test_what_is_not_a_number_stays_so():
         seen = torch.isfinite(out.float()).all(1)
         assert not seen[key:].any(), key
         assert not torch.isfinite(dqkv[key:, :64].float()).all(1).any(), key
+
+
+def test_first_use_may_lie_inside_a_callers_capture():
+    """In a process whose libraries and other kernels are set up, the first step (evaluation) with heads of 64 columns is captured by its caller."""
+    import subprocess
+    code = """
+import sys, torch
+from piccl_b200.models.gpt2 import GPT2, GPT2Config
+from piccl_b200 import _native as N
+evaluation = sys.argv[1] == "eval"
+def model(heads):
+    return GPT2(GPT2Config(vocab_size=1000, seq_len=128, n_layer=2, n_head=heads, d_model=256), seed=1)
+tok = torch.randint(0, 1000, (4, 129), generator=torch.Generator().manual_seed(0)).cuda()
+x, y = tok[:, :-1].contiguous(), tok[:, 1:].contiguous()
+other = model(2)                           # heads of 128 columns: the same products and launches, attention through PyTorch
+other.loss(x, y); other.forward_backward(x, y)
+q = torch.randn(4, 4, 128, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+torch.nn.functional.scaled_dot_product_attention(q, q, q, is_causal=True).sum().backward()
+torch.cuda.synchronize()
+m, g = model(4), torch.cuda.CUDAGraph()
+run = m.loss if evaluation else m.forward_backward
+with torch.cuda.graph(g):
+    loss = run(x, y)
+m.flat_g.fill_(float("nan"))
+g.replay()
+got, grads = float(loss), m.flat_g.clone()
+assert abs(float(run(x, y)) - got) <= 1e-5 * got
+if not evaluation:                          # the products of a replay may be another back end's
+    assert float((m.flat_g.double() - grads.double()).norm()) <= 2 ** -7 * float(grads.double().norm())
+assert N.ops_lib().piccl_ops_attn_status() == 0
+"""
+    for what in ("eval", "train"):
+        r = subprocess.run([sys.executable, "-c", code, what], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, (what, r.stderr[-2000:])
