@@ -225,11 +225,11 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
 
   // partial rows of the column sums: dgamma, dbeta and bias gradient of both LayerNorms, the MLP's and the attention's bias gradients
   const int n_ln = piccl_ops_ln_bwd_parts(T, C), n_qkv = piccl_ops_col_parts(T, 3 * C), n_fc_own = (T + 31) / 32, n_fc_sep = piccl_ops_col_parts(T, 4 * C);
-  // Heads of 64 columns: this framework's kernels, where PyTorch would take cuDNN's (a program that asks for another back end gets that one; any address will do
-  // for the question).  A training step keeps cuDNN's forward kernel, whose sums of exponentials the way back takes as they are: the two forward kernels are equally
+  // Heads of 64 columns: this framework's kernels, where they are the faster ones and PyTorch would take cuDNN's (a program that asks for another back end gets that one; any
+  // address will do for the question).  A training step keeps cuDNN's forward kernel, whose sums of exponentials the way back takes as they are: the two forward kernels are equally
   // exact and fast (2.0e-3 off fp64; 8 x 1024 tokens 40 us, own 41), but another order of its sums rolls the rounding of every activation above it anew, and gradients
   // of one step then differ by 0.95 % from those that this model has had, with the own way back alone by 0.48 % (8 layers of 768 columns).
-  const bool own_attention = D == 64 && sdp_choice(d.p, B, S, H, D) == kCudnnAttention;
+  const bool own_attention = D == 64 && piccl_ops_attn_pays(train, B, S, H, at::cuda::getCurrentDeviceProperties()->multiProcessorCount) && sdp_choice(d.p, B, S, H, D) == kCudnnAttention;
   const int n_att = own_attention ? piccl_ops_attn_parts(B, S) : 0;
   const size_t row = (size_t)n_ln * C, fc_floats = (size_t)std::max(n_fc_own, n_fc_sep) * 4 * C, part_floats = 6 * row + fc_floats + (size_t)std::max(n_qkv, n_att) * 3 * C;
   const size_t row_floats = own_attention ? (size_t)2 * B * H * piccl_ops_attn_rows(S) : 0;

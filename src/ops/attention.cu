@@ -634,6 +634,19 @@ int piccl_ops_attn_bwd(const void* qkv, const void* out, const void* dout, const
   if (launch_pdl(attn_dq_kernel, grid, AT_THREADS, AttnSmem::DYNAMIC, (cudaStream_t)stream, a) != cudaSuccess) return -5;
   return launch_pdl(attn_dkv_kernel, grid, AT_THREADS, AttnSmem::DYNAMIC, (cudaStream_t)stream, a) == cudaSuccess ? 0 : -5;
 }
+// Is this kernel (backward: both) at least as fast as cuDNN's, with the packing and the column sums that come with that one?  Measured alone at 1 to 64 batch entries times heads, time of
+// this against that in percent; n: tiles of 128 rows, of which a chip of 148 SMs holds 296 at once.  One tile's walk grows with S: where all tiles are resident together the longest walk
+// is the whole time and cuDNN's shorter step wins, where they take turns the early ends of the short walks are filled.  cuDNN has no tail to mask where S is a multiple of 128.
+//   backward  S 512 -3 to -31, 640 +2 to -22, 777 -5 to -37, 1000 +2 to -34 | 896 n 7 +9, 224 +11, 308 -10, 448 -23; 1024 n 32 +11, 224 +19, 320 -8, 384 -18;
+//             1536 n 240 +33, 336 +3, 384 -9; 2048 n 256 +46, 384 0, 448 -8; 3072 n 288 +60, 432 0, 480 -4; 4096 n 256 +73, 512 +1, 1024 -2; 8192 n 256 +94, 1024 +6
+//   forward   S 33 +1 to -5, 128 -13 to -29, 512 -9 to -31, 1024 -1 to -28 | 1536 n 144 -19, 288 +7, 384 -1, 768 -7; 1600 -2 to -29;
+//             2048 n 192 -13, 288 +9, 1024 -1; 4096 n 128 -18, 384 +11, 1024 +4; 8192 n 128 -17, 512 +15
+int piccl_ops_attn_pays(int backward, int B, int S, int H, int sms) {
+  const long long n = (long long)B * H * ((S + AT_ROWS - 1) / AT_ROWS), slots = 2ll * sms;
+  const bool ragged = S % AT_ROWS != 0;
+  if (backward) return S <= 640 || (ragged && S < 1024) || (S <= 3584 && n >= slots + S / 20);
+  return S <= 1024 || 3 * n <= 4ll * sms || (S <= 1600 && (ragged || n > slots + 16));
+}
 // Non-zero if an attention kernel on the current device gave up on a wait (10 / 20 / 30 + warp).  Synchronises.
 int piccl_ops_attn_status(void) { return read_status(STATUS_ATTENTION); }
 

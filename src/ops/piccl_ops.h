@@ -20,6 +20,7 @@ int piccl_ops_ce(void* logits, const long long* targets, float* loss, int rows, 
 int piccl_ops_mean(const float* x, float* out, int n, void* stream);
 int piccl_ops_wpe_bwd(const void* dx, void* dwpe, int B, int S, int rows, int C, int accumulate, void* stream);
 int piccl_ops_wte_bwd_rows(const long long* idx, const void* dx, float* stage, int* owner, void* dwte, int rows, int C, void* stream);
+int piccl_ops_attn_pays(int backward, int B, int S, int H, int sms);
 int piccl_ops_attn_rows(int S);
 int piccl_ops_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, void* stream);
 int piccl_ops_attn_parts(int B, int S);
