@@ -158,7 +158,8 @@ class GPT2:
     def forward_backward(self, idx: torch.Tensor, targets: torch.Tensor,
                          on_grads_ready: Optional[Callable[[int], None]] = None, loss_only: bool = False) -> torch.Tensor:
         """One training micro-step: returns the mean loss (fp32, on device) and leaves the
-        gradients in `flat_g`.  `on_grads_ready(end)` is called whenever flat_g[:end] is final."""
+        gradients in `flat_g`.  `on_grads_ready(end)` is called whenever flat_g[:end] is final.
+        The loss is not a number where a kernel on this device gave up on a bounded wait (the gradients are void then): ops.raise_if_a_wait_ran_out() tells."""
         loss, shared = self._step(idx, targets, on_grads_ready, loss_only)
         return loss.clone() if shared else loss
 

@@ -43,6 +43,15 @@ def _chk(rc: int, name: str) -> None:
         raise RuntimeError(f"{name} failed (code {rc})")
 
 
+def raise_if_a_wait_ran_out() -> None:
+    """Raises if a GEMM or attention kernel on the current device gave up on a bounded wait since the last such report: what it should have written is void, and
+    so are results computed from it.  Losses of GPT2 are not a number from then on until it is reported here.  Synchronises."""
+    words = (C.c_int * 2)()
+    _chk(N.ops_lib().piccl_ops_status(words, 1), "status")
+    if any(words):
+        raise RuntimeError("a kernel gave up on a wait: " + ", ".join(f"{n} (role {w})" for n, w in zip(("GEMM", "attention"), words) if w))
+
+
 _ws: dict = {}
 
 

@@ -5,7 +5,8 @@
 
 `step` copies the batch from (pinned) host memory, runs forward, backward with
 bucketed gradient averaging overlapped on a second stream, the fused AdamW
-update, and reads the loss back.  `step_device` is the same without the two host
+update, and reads the loss back; it raises if a kernel of the step gave up on a
+bounded wait (the weights are void then).  `step_device` is the same without the two host
 transfers.
 """
 from __future__ import annotations
@@ -99,7 +100,10 @@ class DataParallelTrainer:
         loss = self.step_device(self._idx, self._tgt)
         self._loss_host.copy_(loss.reshape(1), non_blocking=True)
         torch.cuda.current_stream().synchronize()
-        return float(self._loss_host[0])
+        loss = float(self._loss_host[0])
+        if loss != loss:
+            ops.raise_if_a_wait_ran_out()
+        return loss
 
     def replayed_steps(self) -> int:
         """Steps so far whose forward and backward pass, or all of whose launches (`use_graph`), came from a CUDA graph."""

@@ -288,8 +288,8 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   Layer& f = b.layer[L];
   DO(product(m, NT, f.ln1, wte, b.logits, nullptr, T, d.Vp, C, s));
   TRY(piccl_ops_ce(b.logits, tgt, b.loss_rows, T, d.V, d.Vp, 1.0f / (float)T, train, s));
-  TRY(piccl_ops_mean(b.loss_rows, loss, T, s));
-  if (!train) return 0;
+  // The loss comes last, since it also tells whether a kernel of the pass gave up on a wait: its products or gradients are left over from another layer or step then.
+  if (!train) { TRY(piccl_ops_pass_loss(b.loss_rows, loss, T, s)); return 0; }
 
   // ---------------- backward (logits now hold d loss / d logits)
   b16 *const g_lnf_g = d.g + m.off[0], *const g_lnf_b = d.g + m.off[1], *const g_wpe = d.g + m.off[2], *const g_wte = d.g + m.off[3];
@@ -397,6 +397,7 @@ int run(Model& m, const long long* idx, const long long* tgt, int B, int S, floa
   TRY(piccl_ops_wte_bwd_rows(idx, dx, m.stage.data_ptr<float>(), m.owner.data_ptr<int>(), g_wte, T, C, s));
   m.launches++;                       // two kernels
   done(g_wte, (size_t)d.Vp * C);
+  TRY(piccl_ops_pass_loss(b.loss_rows, loss, T, s));
   return 0;
 }
 

@@ -324,9 +324,11 @@ __global__ void __launch_bounds__(512, 2) ce_row_kernel(bf16* __restrict__ logit
   if (valid && owner) reinterpret_cast<bf16*>(lp)[t] = ce_gradient_target(xt, -o.m, ls, gscale);
 }
 
-// out[0] = mean of x[0..n), one block
-__global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ x, float* __restrict__ out, int n) {
+// out[0] = mean of x[0..n), one block; not a number where a word of `status` (optional) is set
+__global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ x, float* __restrict__ out, int n, const int* status) {
   pdl_begin();
+  int failed = 0;
+  if (status && threadIdx.x == 0) for (int i = 0; i < kStatusKinds; i++) failed |= status[i];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += 1024) s += x[i];
   __shared__ float sh[32];
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ x,
   __syncthreads();
   if (threadIdx.x < 32) {
     s = warp_sum(sh[threadIdx.x]);
-    if (threadIdx.x == 0) out[0] = s / (float)n;
+    if (threadIdx.x == 0) out[0] = failed ? __int_as_float(0x7fffffff) : s / (float)n;
   }
 }
 
@@ -574,7 +576,15 @@ int piccl_ops_ce_fwd_bwd(void* logits, const long long* targets, float* loss, in
 }
 int piccl_ops_mean(const float* x, float* out, int n, void* stream) {
   if (n < 1) return -1;
-  launch_pdl(mean_kernel, 1, 1024, 0, (cudaStream_t)stream, x, out, n);
+  launch_pdl(mean_kernel, 1, 1024, 0, (cudaStream_t)stream, x, out, n, nullptr);
+  PICCL_OPS_CHECK_LAUNCH(); return 0;
+}
+// The same at the end of a pass: not a number where a wait of a GEMM or attention kernel on this device ran out, in this pass or an earlier one (piccl_ops_status tells which).
+int piccl_ops_pass_loss(const float* rows, float* loss, int n, void* stream) {
+  if (n < 1) return -1;
+  const int* status = status_word(STATUS_GEMM);
+  if (!status) return -7;
+  launch_pdl(mean_kernel, 1, 1024, 0, (cudaStream_t)stream, rows, loss, n, status);
   PICCL_OPS_CHECK_LAUNCH(); return 0;
 }
 // One AdamW step over flat buffers of n elements that alternate between decaying and non-decaying runs: ends[i] (device) is the end of

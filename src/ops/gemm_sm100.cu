@@ -201,7 +201,6 @@ struct MapKey {
 };
 static std::mutex g_mu;
 static std::map<MapKey, CUtensorMap> g_maps;
-static int* g_status[64] = {nullptr};
 static int g_pairs[64] = {0};
 
 // box rows x 64 columns of a row-major [rows, cols] matrix
@@ -233,10 +232,6 @@ static Variant g_variants[] = {
 // Prepares the device state; pairs that can be resident at once (a pair needs two SMs of one GPC): the persistent grid is never larger.
 static int device_ready(int dev) {
   std::lock_guard<std::mutex> l(g_mu);
-  if (!g_status[dev]) {
-    if (cudaMalloc(&g_status[dev], sizeof(int)) != cudaSuccess) return -7;
-    cudaMemset(g_status[dev], 0, sizeof(int));
-  }
   if (!g_pairs[dev]) {
     Variant& v = g_variants[0];
     if (cudaFuncSetAttribute((const void*)v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem) != cudaSuccess) return -4;
@@ -310,7 +305,8 @@ int piccl_ops_gemm(int layout, int epi, const void* A, const void* B, void* C, v
   if (pre) { if (!get_map(pre, M, N, 32, &a.tpre)) return -3; } else a.tpre = a.tc;
   a.bias = (const bf16*)bias; a.aux = (const bf16*)aux; a.part = part;
   a.slices = slices; a.ticket = (unsigned*)ws; a.split = (float4*)((char*)ws + kTicketBytes);
-  a.M = M; a.N = N; a.K = K; a.status = g_status[dev];
+  a.M = M; a.N = N; a.K = K; a.status = status_word(STATUS_GEMM);
+  if (!a.status) return -7;
   const long tiles = (long)((M + 255) / 256) * ((N + v->tn - 1) / v->tn) * slices;
   const int pairs = (int)(tiles < g_pairs[dev] ? tiles : g_pairs[dev]);
   return launch_pdl(v->fn, dim3(2 * pairs), dim3(PAIR_THREADS), v->smem, (cudaStream_t)stream, a) == cudaSuccess ? 0 : -5;
@@ -328,12 +324,6 @@ int piccl_ops_gemm_bf16_nt(const void* A, const void* B, void* C, const void* bi
   return piccl_ops_gemm_bf16_nt_ex(A, B, C, nullptr, bias, M, N, K, gelu, stream);
 }
 // Non-zero if a GEMM on the current device gave up on a wait (1 producer, 2/3 MMA issuer, 4 epilogue).  Synchronises.
-int piccl_ops_gemm_status(void) {
-  using namespace piccl_ops;
-  int dev = 0; cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !g_status[dev]) return 0;
-  int v = 0; cudaMemcpy(&v, g_status[dev], sizeof v, cudaMemcpyDeviceToHost);
-  return v;
-}
+int piccl_ops_gemm_status(void) { return piccl_ops::read_status(piccl_ops::STATUS_GEMM); }
 
 }  // extern "C"

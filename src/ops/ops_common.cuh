@@ -27,7 +27,7 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
 }
 
 // Status word of the current device (status.cu); null if there is no device.
-enum StatusKind { STATUS_ATTENTION, kStatusKinds };
+enum StatusKind { STATUS_GEMM, STATUS_ATTENTION, kStatusKinds };
 int* status_word(StatusKind kind);
 int read_status(StatusKind kind);         // synchronises
 

@@ -18,6 +18,7 @@ struct piccl_finish_job { const float* part; void* out; int nparts, C, accumulat
 int piccl_ops_finish_parts(const void* jobs, int n, void* stream);
 int piccl_ops_ce(void* logits, const long long* targets, float* loss, int rows, int V, int Vp, float gscale, int grad, void* stream);
 int piccl_ops_mean(const float* x, float* out, int n, void* stream);
+int piccl_ops_pass_loss(const float* rows, float* loss, int n, void* stream);
 int piccl_ops_wpe_bwd(const void* dx, void* dwpe, int B, int S, int rows, int C, int accumulate, void* stream);
 int piccl_ops_wte_bwd_rows(const long long* idx, const void* dx, float* stage, int* owner, void* dwte, int rows, int C, void* stream);
 int piccl_ops_attn_pays(int backward, int B, int S, int H, int sms);

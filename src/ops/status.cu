@@ -32,3 +32,24 @@ int read_status(StatusKind kind) {
 }
 
 }  // namespace piccl_ops
+
+extern "C" {
+
+// The words of the current device, out[0] GEMM, out[1] attention; clear: zero from now on.  A word stays set until it is cleared here.  Synchronises.
+int piccl_ops_status(int* out, int clear) {
+  int* p = piccl_ops::status_word(piccl_ops::STATUS_GEMM);
+  if (!p) return -7;
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e == cudaSuccess) e = cudaMemcpy(out, p, piccl_ops::kStatusKinds * sizeof(int), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess && clear) e = cudaMemset(p, 0, piccl_ops::kStatusKinds * sizeof(int));
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  return (int)e;
+}
+// Sets a word as a kernel that gave up would, for tests of what reads it.
+int piccl_ops_test_set_status(int kind, int value) {
+  if (kind < 0 || kind >= piccl_ops::kStatusKinds) return -1;
+  int* p = piccl_ops::status_word((piccl_ops::StatusKind)kind);
+  return p ? (int)cudaMemcpy(p, &value, sizeof value, cudaMemcpyHostToDevice) : -7;
+}
+
+}  // extern "C"

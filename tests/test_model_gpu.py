@@ -279,3 +279,27 @@ def test_attention_on_both_sides_of_its_rule(B, S, n_head, own):
         other_eval, plain_eval = run(True)
     assert abs(other - loss) < 2e-3 and abs(other_eval - evaluated) < 2e-3
     assert launches - plain == layers * own and eval_launches - plain_eval == layers * fwd
+
+
+@pytest.mark.parametrize("kind,name", [(0, "GEMM"), (1, "attention")])
+def test_a_wait_that_ran_out_is_reported(kind, name):
+    """The status word that a kernel sets when it gives up (set here from the host): the loss of a step or an evaluation is not a number, issued, replayed and in a graph of the whole step,
+    the trainer raises, and once reported all is as before."""
+    from piccl_b200 import _native as N, ops
+    from piccl_b200.models.gpt2 import GPT2Config
+    from piccl_b200.train import DataParallelTrainer
+    cfg = GPT2Config.tiny()
+    tok = torch.randint(0, cfg.vocab_size, (2, cfg.seq_len + 1), generator=torch.Generator().manual_seed(0))
+    x, y = tok[:, :-1].contiguous().pin_memory(), tok[:, 1:].contiguous().pin_memory()
+    xd, yd = x.cuda(), y.cuda()
+    for use_graph in (False, True):
+        t = DataParallelTrainer(cfg, seed=4, use_graph=use_graph)
+        for step in range(6):
+            assert t.step(x, y) > 0
+            assert N.ops_lib().piccl_ops_test_set_status(kind, 11) == 0
+            assert torch.isnan(t.model.loss(xd, yd)) and torch.isnan(t.model.loss(xd, yd))      # stays until it is reported
+            with pytest.raises(RuntimeError, match=name):
+                t.step(x, y)
+            ops.raise_if_a_wait_ran_out()                  # nothing more to report
+            assert t.step(x, y) > 0 and float(t.model.loss(xd, yd)) > 0
+        assert t.replayed_steps() > 0
