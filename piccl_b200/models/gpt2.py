@@ -49,7 +49,7 @@ _SETTINGS = [getattr(torch._C, f"_get_{n}") for n in ("cudnn_sdp_enabled", "flas
 
 
 def _library_settings() -> tuple:
-    return tuple([f() for f in _SETTINGS])
+    return tuple([f() for f in _SETTINGS] + torch._C._get_sdp_priority_order())      # (the order in which attention's back ends are tried)
 
 
 @dataclass

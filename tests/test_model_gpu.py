@@ -211,6 +211,27 @@ def test_a_captured_step_is_not_replayed_under_other_library_settings():
     assert float(m.forward_backward(a, b)) == want and m.replays == 3
 
 
+def test_a_captured_step_is_not_replayed_under_another_order_of_back_ends():
+    """The same attention back ends enabled, but another one first."""
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    from piccl_b200.models.gpt2 import GPT2, GPT2Config
+    cfg = GPT2Config.tiny()
+    m = GPT2(cfg, seed=1)
+    tok = torch.randint(0, cfg.vocab_size, (2, cfg.seq_len + 1), generator=torch.Generator().manual_seed(0)).cuda()
+    a, b = tok[:, :-1].contiguous(), tok[:, 1:].contiguous()
+    orders = [SDPBackend.CUDNN_ATTENTION, SDPBackend.EFFICIENT_ATTENTION], [SDPBackend.EFFICIENT_ATTENTION, SDPBackend.CUDNN_ATTENTION]
+    with sdpa_kernel(orders[0], set_priority=True):
+        for _ in range(4):
+            want = float(m.forward_backward(a, b))
+        grads = m.flat_g.clone()
+    assert m.replays == 2
+    with sdpa_kernel(orders[1], set_priority=True):
+        assert abs(float(m.forward_backward(a, b)) - want) <= 1e-3 * want
+    assert m.replays == 2 and not torch.equal(m.flat_g, grads)
+    with sdpa_kernel(orders[0], set_priority=True):
+        assert float(m.forward_backward(a, b)) == want and m.replays == 3
+
+
 def test_an_interrupt_during_a_capture_leaves_the_model_usable():
     from piccl_b200.models.gpt2 import GPT2, GPT2Config
     cfg = GPT2Config.tiny()
