@@ -118,19 +118,41 @@ def cross_entropy_fwd_bwd(logits, targets, loss_rows, vocab: int, gscale: float)
     _bump()
 
 
+def _attention_operands(batch: int, qkv, out, rows_like=(), floats=()) -> tuple[int, int]:
+    """(positions, heads) of packed rows; everything that the kernels do not look at: shapes, types, layout and device."""
+    if out.dim() != 2 or out.shape[1] == 0 or out.shape[1] % 64 or batch <= 0 or out.shape[0] == 0 or out.shape[0] % batch:
+        raise ValueError(f"attention: {tuple(out.shape)} is not [{batch} * positions, heads * 64]")
+    rows, Cc = out.shape
+    for t, width in ((qkv, 3 * Cc), (out, Cc), *rows_like):
+        if t.numel() != rows * width or t.dtype != torch.bfloat16 or not t.is_contiguous():
+            raise ValueError(f"attention: contiguous bf16 [{rows}, {width}] wanted, got {t.dtype} {tuple(t.shape)}")
+    S = rows // batch
+    heads, pad = Cc // 64, (S + 127) // 128 * 128
+    for t, n in ((t, f(S, heads, pad)) for t, f in floats if t is not None):
+        if t.numel() < n or t.dtype != torch.float32 or not t.is_contiguous():
+            raise ValueError(f"attention: {n} contiguous floats wanted, got {t.dtype} {tuple(t.shape)}")
+    for t in (qkv, out, *(t for t, _ in rows_like), *(t for t, _ in floats if t is not None)):
+        if not t.is_cuda or t.device != qkv.device:
+            raise ValueError("attention: tensors of one CUDA device wanted")
+    return S, heads
+
+
 def attention_fwd(qkv, out, lse, batch: int):
     """Causal attention of packed rows [batch * S, 3 * heads * 64] -> [batch * S, heads * 64]; lse: [batch * heads, S] floats, the logarithm of each row's sum of
-    exponentials, or None."""
-    rows, Cc = out.shape
-    _chk(N.ops_lib().piccl_ops_attn_fwd(_p(qkv), _p(out), _p(lse), batch, rows // batch, Cc // 64, C.c_void_p(_s())), "attn_fwd")
+    exponentials, which attention_bwd takes, or None."""
+    S, heads = _attention_operands(batch, qkv, out, floats=[(lse, lambda S, h, pad: batch * h * S)])
+    _chk(N.ops_lib().piccl_ops_attn_fwd(_p(qkv), _p(out), _p(lse), batch, S, heads, C.c_void_p(_s())), "attn_fwd")
     _bump()
 
 
 def attention_bwd(qkv, out, dout, lse, scratch, dqkv, part, batch: int):
     """dqkv, the gradient of the packed rows, and in part its partial column sums: one row per batch entry and 128 positions.
-    scratch: 2 * batch * heads * (S rounded up to 128) floats."""
-    rows, Cc = out.shape
-    _chk(N.ops_lib().piccl_ops_attn_bwd(_p(qkv), _p(out), _p(dout), _p(lse), _p(scratch), _p(dqkv), _p(part), batch, rows // batch, Cc // 64, C.c_void_p(_s())), "attn_bwd")
+    lse as attention_fwd leaves it; scratch: 2 * batch * heads * (S rounded up to 128) floats."""
+    if lse is None or scratch is None or part is None:
+        raise ValueError("attention: the backward pass takes lse, scratch and part")
+    S, heads = _attention_operands(batch, qkv, out, [(dout, out.shape[-1]), (dqkv, 3 * out.shape[-1])],
+                                   [(lse, lambda S, h, pad: batch * h * S), (scratch, lambda S, h, pad: 2 * batch * h * pad), (part, lambda S, h, pad: batch * (pad // 128) * 3 * h * 64)])
+    _chk(N.ops_lib().piccl_ops_attn_bwd(_p(qkv), _p(out), _p(dout), _p(lse), _p(scratch), _p(dqkv), _p(part), batch, S, heads, C.c_void_p(_s())), "attn_bwd")
     _bump(2)
 
 

@@ -613,7 +613,7 @@ extern "C" {
 // lse (null: not wanted): B * H * S floats, the logarithm of the sum of exponentials of each row's scaled scores.
 int piccl_ops_attn_rows(int S) { return (S + AT_ROWS - 1) / AT_ROWS * AT_ROWS; }
 int piccl_ops_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, void* stream) {
-  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return -2;
+  if (!qkv || !out || ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) || (reinterpret_cast<uintptr_t>(lse) & 3)) return -2;
   AttnArgs a;
   const int rc = attn_args(a, qkv, B, S, H); if (rc) return rc;
   if (!make_tmap_bf16_rows(&a.result, out, B, S, (uint64_t)H * AT_D, 32)) return -3;
@@ -624,7 +624,8 @@ int piccl_ops_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int
 // piccl_ops_attn_rows(S) floats, 16-byte aligned.
 int piccl_ops_attn_parts(int B, int S) { return B * ((S + AT_ROWS - 1) / AT_ROWS); }
 int piccl_ops_attn_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* scratch, void* dqkv, float* part, int B, int S, int H, void* stream) {
-  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dqkv) | reinterpret_cast<uintptr_t>(scratch)) & 15) return -2;
+  for (const void* p : {qkv, out, dout, (const void*)dqkv, (const void*)scratch}) if (!p || (reinterpret_cast<uintptr_t>(p) & 15)) return -2;
+  for (const void* p : {(const void*)lse, (const void*)part}) if (!p || (reinterpret_cast<uintptr_t>(p) & 3)) return -2;
   AttnArgs a;
   const int rc = attn_args(a, qkv, B, S, H); if (rc) return rc;
   if (!make_tmap_bf16_rows(&a.out, out, B, S, (uint64_t)H * AT_D, AT_STEP) || !make_tmap_bf16_rows(&a.dout, dout, B, S, (uint64_t)H * AT_D, AT_STEP) ||
