@@ -122,6 +122,7 @@ int piccl_tp_status(piccl_comm_t* c);   /* 0, or the role that gave up on a wait
 /* Test hook: launches the executor with one action that waits for data nobody
  * sends.  The wait runs into its time limit, the kernel returns and the status
  * reports it; the communicator is unusable afterwards. */
+int piccl_test_last_first(int coll, int nranks, int in_launch, int one_device, long long bytes);
 int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream);
 
 /* ---- schedule layer (CPU only) ---- */

@@ -397,8 +397,9 @@ static int exec_block(const piccl_comm* c) { return c->cfg.block_size + kCtlThre
 // 8 x 8 94 / 96, 8 x 16 119 / 117, 8 x 64 408 / 369, recursive doubling 4 x 16 (128 MiB) 92 / 90, 4 x 25 138 / 134; all-gather 4 x 2 MiB (40 MiB) 30.3 / 30.2, 4 x 4 41.0 / 38.8,
 // 4 x 16 117 / 105; reduce-scatter 2 x 8 MiB (48 MiB) 19.9 / 21.1, 2 x 16 33.9 / 31.8, 8 x 8 221 / 204; broadcast 4 x 8 MiB (40 MiB) 43.8 / 43.4, 4 x 16 56.5 / 54.8;
 // reduce 4 x 16 MiB 53.3 / 50.5.  (Of an all-reduce more stays in L2 from one
-// call to the next: its line lies higher.)
-static bool crowds_l2(const CollArgs& a, int n) {
+// call to the next: its line lies higher.)  All of this is of launches that carry every rank on one GPU: elsewhere the slots are filled by other GPUs, and nothing leaves first.
+static bool crowds_l2(const CollArgs& a, int n, bool one_gpu) {
+  if (!one_gpu) return false;
   const long long one = (long long)a.count * a.elem_size;
   long long bytes = 0, line = 72ll << 20;
   switch (a.coll) {
@@ -648,6 +649,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     ka.n_vrank = n; ka.elem_size = esz; ka.avg = avg ? 1 : 0; ka.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
     int n_cta = 0;
     bool aligned = true;
+    CollArgs priorities_of;
     for (int i = 0; i < n && rc == PICCL_OK; i++) {
       piccl_comm* c = comms[i]; const CallDesc& d = calls[i];
       std::lock_guard<std::mutex> l(c->mu);
@@ -671,7 +673,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
           if (n > 1) n_cta = std::min(n_cta, std::max(1, c->sm_count / n));
         }
         ka.n_cta = n_cta; if (!use_llf) cut_fifo(c, n, n_cta, a, &ka);
-        ka.last_first = crowds_l2(a, n);
+        priorities_of = a;
         ka.one_gpu = n == c->nranks;
         ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
       }
@@ -681,6 +683,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       c->stats.launches++;
     }
     if (rc) break;
+    ka.last_first = crowds_l2(priorities_of, n, ka.one_gpu);
     bool skip = false;
     for (int i = 0; i < n; i++) skip |= fault_now(comms[i]);
     for (int i = 0; i < n; i++) comms[i]->call_index++;
@@ -738,6 +741,11 @@ int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const voi
   return run(comms, ncomms, d, (cudaStream_t)stream);
 }
 
+// Whether the executor asks L2 to let go of the caller's lines first, for blocks of `bytes` in a launch of `in_launch` of `nranks` ranks (as crowds_l2 above has it).
+int piccl_test_last_first(int coll, int nranks, int in_launch, int one_device, long long bytes) {
+  CollArgs a; a.coll = (Coll)coll; a.nranks = nranks; a.count = bytes; a.elem_size = 1;
+  return crowds_l2(a, in_launch, one_device && in_launch == nranks);
+}
 int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream) {
   if (!c || !c->connected) return fail(PICCL_INVALID_USAGE, "communicator is not connected");
   DevGuard g(c->device);

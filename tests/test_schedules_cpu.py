@@ -177,3 +177,16 @@ def test_xml_transfer_counts():
     assert count(coll="allreduce", algo="PRM", nranks=n, count=64, k=8) == n * (n - 1)
     assert count(coll="broadcast", algo="RING", nranks=n, count=64) == n - 1
     assert count(coll="reduce", algo="PRD", nranks=n, count=64) == n - 1
+
+
+def test_cache_priorities_are_for_launches_that_carry_every_rank():
+    """The executor's evict-first priorities were measured with all ranks on one GPU, where the FIFO's slots and the caller's buffers share its cache."""
+    from piccl_b200 import _native as N
+    f = N.lib().piccl_test_last_first
+    for coll in N.COLL.values():
+        for n in (2, 4, 8):
+            assert f(coll, n, n, 1, 1 << 30), (coll, n)
+            assert not f(coll, n, 1, 1, 1 << 30), (coll, n)             # one rank per launch, whether or not its GPU has others
+            assert not f(coll, n, n, 0, 1 << 30), (coll, n)
+            assert not f(coll, n, n // 2, 1, 1 << 30) or n // 2 == n, (coll, n)
+            assert not f(coll, n, n, 1, 1 << 16), (coll, n)
