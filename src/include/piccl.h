@@ -119,10 +119,13 @@ int piccl_gemm_rs_group(piccl_comm_t** comms, int n, const void* const* A, const
 int piccl_ag_gemm_group(piccl_comm_t** comms, int n, const void* const* A_shard, const void* const* B, void* const* out, int M, int N_local, int K, void* stream);
 int piccl_tp_status(piccl_comm_t* c);   /* 0, or the role that gave up on a wait; synchronises */
 
+/* Test hook: the executor's L2 priorities (1 operands, 2 results) for blocks of
+ * `bytes` in a launch of `in_launch` of `nranks` ranks. */
+int piccl_test_leave_first(int coll, int nranks, int in_launch, int one_device, long long bytes);
+
 /* Test hook: launches the executor with one action that waits for data nobody
  * sends.  The wait runs into its time limit, the kernel returns and the status
  * reports it; the communicator is unusable afterwards. */
-int piccl_test_last_first(int coll, int nranks, int in_launch, int one_device, long long bytes);
 int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream);
 
 /* ---- schedule layer (CPU only) ---- */

@@ -61,7 +61,7 @@ struct KernelArgs {
   // are consumed, so the cut may differ from call to call where no rank can be a call ahead (one launch for all ranks).
   long long seg_bytes;                    // bytes of a segment and of its slot
   int one_gpu;                            // 1: every rank's heap is on this GPU: counters and fences need no scope beyond it
-  int last_first;                         // 1: what is used for the last time leaves L2 first
+  int leave_first;                        // with their last use leave L2 first: operands (1), results (2)
   int nslot, window;                      // slots; segments that are walked together, at most half the slots
   unsigned long long timeout_ns;
   LaunchRank r[kMaxVRanks];

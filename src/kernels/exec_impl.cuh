@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
             st.len = (lo + seg_elems < sl_hi ? lo + seg_elems : sl_hi) - lo;
             st.action = ai; st.nsrc = ac.n_recv + has_src; st.ndst = ac.n_send + has_dst; st.local_src = has_src ? ac.self_pos : -1; st.local_dst = has_dst ? 0 : -1;
             st.flags = (ka.avg && (ac.flags & ACT_SCALE_SRC) && has_src ? STEP_SCALE : 0) | (((reinterpret_cast<uintptr_t>(lsrc) | reinterpret_cast<uintptr_t>(ldst)) & 15) == 0 ? STEP_ALIGNED : 0) |
-                       (has_src && ac.src_buf != BUF_IN ? STEP_LOCAL_DEP : 0) | (ka.last_first && (ac.flags & ACT_SRC_DONE) ? STEP_SRC_DONE : 0) | (ka.last_first && (ac.flags & ACT_DST_DONE) ? STEP_DST_DONE : 0) | (ok ? 0 : STEP_FAIL);
+                       (has_src && ac.src_buf != BUF_IN ? STEP_LOCAL_DEP : 0) | ((ka.leave_first & 1) && (ac.flags & ACT_SRC_DONE) ? STEP_SRC_DONE : 0) | ((ka.leave_first & 2) && (ac.flags & ACT_DST_DONE) ? STEP_DST_DONE : 0) | (ok ? 0 : STEP_FAIL);
           }
           __syncwarp();
           bar_arrive_n(kReady + k % kStepDepth, ndata + 32);

@@ -392,22 +392,29 @@ static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
 // threads of an executor CTA: the configured block moves data, two more warps wait and publish
 static int exec_block(const piccl_comm* c) { return c->cfg.block_size + kCtlThreads; }
 
-// Do the caller's buffers of a launch of n ranks, read and written, crowd what is on its way between ranks out of L2?  Then the executor asks L2 to let go of
-// the caller's lines first, each with its last use (exec_impl.cuh: stream).  us without and with: all-reduce on the ring 8 x 4 MiB (64 MiB touched) 75 / 80,
-// 8 x 8 94 / 96, 8 x 16 119 / 117, 8 x 64 408 / 369, recursive doubling 4 x 16 (128 MiB) 92 / 90, 4 x 25 138 / 134; all-gather 4 x 2 MiB (40 MiB) 30.3 / 30.2, 4 x 4 41.0 / 38.8,
-// 4 x 16 117 / 105; reduce-scatter 2 x 8 MiB (48 MiB) 19.9 / 21.1, 2 x 16 33.9 / 31.8, 8 x 8 221 / 204; broadcast 4 x 8 MiB (40 MiB) 43.8 / 43.4, 4 x 16 56.5 / 54.8;
-// reduce 4 x 16 MiB 53.3 / 50.5.  (Of an all-reduce more stays in L2 from one
-// call to the next: its line lies higher.)  All of this is of launches that carry every rank on one GPU: elsewhere the slots are filled by other GPUs, and nothing leaves first.
-static bool crowds_l2(const CollArgs& a, int n, bool one_gpu) {
-  if (!one_gpu) return false;
-  const long long one = (long long)a.count * a.elem_size;
-  long long bytes = 0, line = 72ll << 20;
+// Do the caller's buffers of a launch of n ranks, read and written, crowd what is on its way between ranks out of L2 (126 MB)?  Then the executor asks L2 to let go of
+// the caller's lines first, each with its last use (exec_impl.cuh: stream): of operands (1) and of results (2).
+// Operands, us without and with: all-reduce on the ring 8 x 16 MiB 109.7 / 108.1, 8 x 32 209 / 200.6, 8 x 64 407 / 392, recursive doubling 4 x 17 93.1 / 89.2; reduce-scatter
+// 2 x 16 MiB 33.2 / 31.5, 8 x 8 216 / 202.5, 8 x 16 418 / 392; reduce 4 x 16 49.5 / 47.9; below their lines no gain or a loss (all-reduce 8 x 4 MiB 75 / 80, reduce-scatter 2 x 8 19.9 / 21.1).
+// (Of an all-reduce more stays in L2 from one call to the next: its line lies higher.)  A reader of the operands after the call loses nothing (reduce-scatter 2 x 16 47.8 / 46.7).
+// Results are read by whoever called, and those that L2 could keep are worth more there.  Call, and call with a kernel that scales the results in place, without and with:
+// reduce-scatter 2 x 32 MiB (64 MiB of results) 56.3 / 55.1, but 72.5 / 77.7; broadcast 4 x 16 (64) 50 / 50, 68.4 / 72.6; all-gather 4 x 4 (64) 35.5 / 34.3, 51.9 / 54.0, 2 x 26 (104)
+// 48.5 / 45.3, 76.5 / 80.5; all-reduce 2 x 40 (80) 59.4 / 54.9, 81.9 / 84.3, 8 x 12 (96) 97.2 / 97.3, 126 / 128.  So results leave first only where they do not fit in any case: all-gather 4 x 8 (128)
+// 61.2 / 55.7, 99.6 / 96.6, 4 x 16 (256) 115 / 102, 195 / 186; reduce-scatter 2 x 64 (128) 102.8 / 99.3, 141.5 / 141.6; broadcast 8 x 32 (256) 157.8 / 153.2, 239.6 / 235.8; all-reduce
+// 8 x 32 (256) 200.6 / 193, 281 / 274.6, 8 x 64 392 / 369.5, 551 / 529.  An all-reduce passes over them again for each step, and gains from 100 MiB on: recursive doubling 4 x 25 131 / 128.5, 162.9 / 161.
+// All of this is of launches that carry every rank on one GPU: elsewhere the slots are filled by other GPUs, and nothing leaves first.
+static int leave_first(const CollArgs& a, int n, bool one_gpu) {
+  if (!one_gpu) return 0;
+  const long long one = (long long)a.count * a.elem_size, MiB = 1 << 20;
+  long long bytes = 0, line = 72 * MiB, results = n * one, results_line = 120 * MiB;
   switch (a.coll) {
-    case COLL_ALLREDUCE: bytes = 2 * n * one; line = 128ll << 20; break;
-    case COLL_ALLGATHER: case COLL_REDUCE_SCATTER: bytes = n * (1 + a.nranks) * one; break;
+    case COLL_ALLREDUCE: bytes = 2 * n * one; line = 128 * MiB; results_line = 98 * MiB; break;
+    case COLL_ALLGATHER: bytes = n * (1 + a.nranks) * one; results = n * a.nranks * one; break;
+    case COLL_REDUCE_SCATTER: bytes = n * (1 + a.nranks) * one; break;
+    case COLL_REDUCE: bytes = (n + 1) * one; results = one; break;
     default: bytes = (n + 1) * one; break;
   }
-  return bytes > line;
+  return bytes <= line ? 0 : results > results_line ? 3 : 1;
 }
 
 // Segments of the executor.  Two are walked together where there are slots for it (the protocol needs two slots per segment of a window): the way from a
@@ -683,7 +690,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       c->stats.launches++;
     }
     if (rc) break;
-    ka.last_first = crowds_l2(priorities_of, n, ka.one_gpu);
+    ka.leave_first = leave_first(priorities_of, n, ka.one_gpu);
     bool skip = false;
     for (int i = 0; i < n; i++) skip |= fault_now(comms[i]);
     for (int i = 0; i < n; i++) comms[i]->call_index++;
@@ -741,10 +748,10 @@ int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const voi
   return run(comms, ncomms, d, (cudaStream_t)stream);
 }
 
-// Whether the executor asks L2 to let go of the caller's lines first, for blocks of `bytes` in a launch of `in_launch` of `nranks` ranks (as crowds_l2 above has it).
-int piccl_test_last_first(int coll, int nranks, int in_launch, int one_device, long long bytes) {
+// Which of the caller's lines the executor asks L2 to let go of first (1 operands, 2 results), for blocks of `bytes` in a launch of `in_launch` of `nranks` ranks.
+int piccl_test_leave_first(int coll, int nranks, int in_launch, int one_device, long long bytes) {
   CollArgs a; a.coll = (Coll)coll; a.nranks = nranks; a.count = bytes; a.elem_size = 1;
-  return crowds_l2(a, in_launch, one_device && in_launch == nranks);
+  return leave_first(a, in_launch, one_device && in_launch == nranks);
 }
 int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream) {
   if (!c || !c->connected) return fail(PICCL_INVALID_USAGE, "communicator is not connected");

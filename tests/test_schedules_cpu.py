@@ -182,7 +182,7 @@ def test_xml_transfer_counts():
 def test_cache_priorities_are_for_launches_that_carry_every_rank():
     """The executor's evict-first priorities were measured with all ranks on one GPU, where the FIFO's slots and the caller's buffers share its cache."""
     from piccl_b200 import _native as N
-    f = N.lib().piccl_test_last_first
+    f = N.lib().piccl_test_leave_first
     for coll in N.COLL.values():
         for n in (2, 4, 8):
             assert f(coll, n, n, 1, 1 << 30), (coll, n)
@@ -190,3 +190,13 @@ def test_cache_priorities_are_for_launches_that_carry_every_rank():
             assert not f(coll, n, n, 0, 1 << 30), (coll, n)
             assert not f(coll, n, n // 2, 1, 1 << 30) or n // 2 == n, (coll, n)
             assert not f(coll, n, n, 1, 1 << 16), (coll, n)
+
+
+def test_results_that_the_cache_can_keep_stay_there():
+    """Results of 64 MiB in all are worth more to their reader in the cache than to the call; those beyond its 126 MB leave first, and operands from lower lines on."""
+    from piccl_b200 import _native as N
+    f, MiB = N.lib().piccl_test_leave_first, 1 << 20
+    for coll, n, block, want in [("reduce_scatter", 2, 32, 1), ("broadcast", 4, 16, 1), ("allgather", 4, 4, 1), ("allgather", 2, 26, 1), ("allreduce", 2, 40, 1),
+                                 ("allreduce", 8, 12, 1), ("reduce", 4, 32, 1), ("allgather", 4, 8, 3), ("reduce_scatter", 2, 64, 3), ("broadcast", 8, 32, 3), ("allreduce", 4, 25, 3),
+                                 ("allreduce", 8, 64, 3), ("reduce", 2, 128, 3), ("allreduce", 8, 8, 0), ("allgather", 8, 1, 0), ("reduce_scatter", 2, 8, 0), ("broadcast", 8, 8, 0)]:
+        assert f(N.COLL[coll], n, n, 1, block * MiB) == want, (coll, n, block)
