@@ -74,14 +74,16 @@ def test_rows_of_one_batch_entry_do_not_see_another():
 
 
 def test_what_is_not_a_number_stays_so():
-    """A key that is not a number, on any column of a step, spoils the rows that see it and no row before it."""
+    """A key that is not a number, on any column of a step, spoils the rows that see it; the output of no row before it (dQ's product multiplies the hidden keys of a step by zero)."""
     B, S, H = 1, 200, 1
     gen = torch.Generator(device="cuda").manual_seed(0)
     dout = torch.randn(B * S, H * 64, generator=gen, device="cuda").bfloat16()
     for key in range(8):
         qkv = torch.randn(B * S, 3 * H * 64, generator=gen, device="cuda").bfloat16()
+        clean = _run(qkv, dout, B, S, H)
         qkv[key, 64:128] = float("nan")
-        out, _, dqkv, _ = _run(qkv, dout, B, S, H)
+        out, lse, dqkv, _ = _run(qkv, dout, B, S, H)
+        assert torch.equal(out[:key], clean[0][:key]) and torch.equal(lse[:, :key], clean[1][:, :key]), key
         seen = torch.isfinite(out.float()).all(1)
         assert not seen[key:].any(), key
         assert not torch.isfinite(dqkv[key:, :64].float()).all(1).any(), key

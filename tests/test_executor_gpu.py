@@ -107,8 +107,8 @@ def test_allreduce_avg(groups):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("n,algo,k", [(2, "RING", -1), (4, "PRD", 2), (8, "K_RING", 4), (3, "PRM", 3), (4, "PRM", 4), (8, "PRM", 8), (6, "RM", 3), (5, "DIRECT", -1)])
 def test_averaged_operands(groups, n, algo, k, dtype):
-    """Scaled operands alone and beside one, up to three and up to seven others, to one and several destinations; lengths around a round of the loops.
-    Each of at most three partial sums is rounded to the type once, and so is the scaled operand."""
+    """Scaled operands alone and beside one, up to three and up to seven others, in small slots: the low-latency kernels, unaligned offsets and the ends of the aligned loops
+    (their full rounds: test_averaged_rounds_of_the_default_geometry).  Each of at most three partial sums is rounded to the type once, and so is the scaled operand."""
     eps = 2.0 ** (-24 if dtype == torch.float32 else -9)
     for count in (1, 9, 4096 * 8 + 3, 100003):
         g = groups(n)
@@ -431,4 +431,31 @@ def test_rounds_segments_and_windows(n, algo, k):
         _check_ok(g)
         for x in xs:
             assert torch.equal(x, want), (n, algo, per_cta)
+    g.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n,algo,k", [(2, "RING", -1), (8, "RING", -1), (4, "PRD", 2), (3, "PRM", 3), (4, "PRM", 4), (8, "PRM", 8), (8, "K_RING", 4), (5, "DIRECT", -1)])
+def test_averaged_rounds_of_the_default_geometry(n, algo, k, dtype):
+    """Default geometry (512 threads that move data): CTA slices of whole 16-byte packs, so that every offset is aligned, above the low-latency kernels' sizes and around full rounds of
+    one, two, four and eight packs a thread (4096 packs are 1 of 8, 2 of 4 ...), with a segment more and a partial segment.  The scaled operand alone to one destination and to several, beside
+    one (to one and two destinations), two and three, four and seven others.  Values and averages of 2, 4 and 8 ranks are multiples of 1 / 64 up to one: exact in each type."""
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    ctas, per_pack = min(64, 148 // n), 16 // torch.tensor([], dtype=dtype).element_size()
+    parts = n if algo in ("RING", "K_RING", "DIRECT") else 1
+    g = LoopbackGroup(n, config=make_config(scratch_bytes=1 << 20, timeout_ms=5000))
+    for packs in (4097, 8191, 8192, 12289):
+        count = packs * per_pack * ctas * parts
+        xs = [torch.randint(-8, 9, (count,), generator=torch.Generator(device="cuda").manual_seed(packs + r), device="cuda").to(dtype) / 8 for r in range(n)]
+        outs = [torch.full_like(x, float("nan")) for x in xs]
+        want = sum(x.double() for x in xs) / n
+        for rep in range(2):
+            g.run("allreduce", xs, outs, count, op="avg", algo=algo, k=k)
+        _check_ok(g)
+        bound = 0.0 if n in (2, 4, 8) else 2 * n * 2.0 ** -{torch.float32: 24, torch.bfloat16: 9, torch.float16: 11}[dtype]
+        for o in outs:
+            assert (o.double() - want).abs().max() <= bound, (packs, o.dtype)
+        g.run("allreduce", xs, xs, count, op="avg", algo=algo, k=k)      # in place
+        _check_ok(g)
+        assert all(torch.equal(x, o) for x, o in zip(xs, outs))
     g.close()
