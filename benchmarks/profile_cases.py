@@ -11,6 +11,7 @@
     python benchmarks/profile_cases.py nvls      # in-switch all-reduce kernel with the switch emulated: 4 virtual ranks, 64 MiB bf16 each
     python benchmarks/profile_cases.py llf       # low-latency executor: all-gather of 16 KiB per rank, 8 virtual ranks
     python benchmarks/profile_cases.py ag_gemm   # fused all-gather -> GEMM, 2 virtual ranks, 4096 x 2048 x 4096
+    python benchmarks/profile_cases.py attention # causal attention forward and backward, 8 x 1024 tokens, 16 heads of 64 columns
     python benchmarks/profile_cases.py elementwise  # AdamW on 128 Mi parameters, bias + GELU forward / backward on 8192 x 4096, embedding 8192 x 1024, column sum
 
 Typical capture (after the same command has exited 0 without ncu):
@@ -148,6 +149,20 @@ def case_elementwise():
     assert torch.isfinite(cs.float()).all() and float(master.abs().max()) > 0
 
 
+def case_attention():
+    from piccl_b200 import _native as N
+    from piccl_b200 import ops
+    B, S, H = 8, 1024, 16
+    qkv, dout = torch.randn(B * S, 3 * H * 64, device="cuda").bfloat16(), torch.randn(B * S, H * 64, device="cuda").bfloat16()
+    out, dqkv, lse = torch.empty_like(dout), torch.empty_like(qkv), torch.empty(B * H, S, device="cuda")
+    scratch, part = torch.empty(2 * B * H * S, device="cuda"), torch.empty(B * S // 128, 3 * H * 64, device="cuda")
+    for _ in range(4):
+        ops.attention_fwd(qkv, out, lse, B)
+        ops.attention_bwd(qkv, out, dout, lse, scratch, dqkv, part, B)
+    torch.cuda.synchronize()
+    assert N.ops_lib().piccl_ops_attn_status() == 0 and torch.isfinite(dqkv.float()).all()
+
+
 def case_ln():
     from piccl_b200 import ops
     T, C = 8192 * 4, 1024
@@ -175,5 +190,5 @@ def case_ce():
 
 if __name__ == "__main__":
     which = sys.argv[1] if len(sys.argv) > 1 else "exec"
-    {"exec": case_exec, "exec8": lambda: case_exec(8, 8 << 20), "exec_ll": lambda: case_exec(8, 4096, "PRD"), "gemm": case_gemm, "direct": case_direct, "tp": case_tp, "ln": case_ln, "ce": case_ce, "nvls": case_nvls, "llf": case_llf, "ag_gemm": case_ag_gemm, "elementwise": case_elementwise}[which]()
+    {"exec": case_exec, "exec8": lambda: case_exec(8, 8 << 20), "exec_ll": lambda: case_exec(8, 4096, "PRD"), "gemm": case_gemm, "direct": case_direct, "tp": case_tp, "ln": case_ln, "ce": case_ce, "nvls": case_nvls, "llf": case_llf, "ag_gemm": case_ag_gemm, "attention": case_attention, "elementwise": case_elementwise}[which]()
     print(f"profile case {which} done")
