@@ -2,7 +2,7 @@
 
   piccl_b200/lib/piccl.so        collectives library + NCCL-ABI preload shim + fused TP kernels
   piccl_b200/lib/libpiccl_ops.so model kernels (tcgen05 GEMM, layer norm, cross entropy, AdamW, ...)
-  piccl_b200/lib/libpiccl_model.so native training step (launches the kernels of libpiccl_ops.so; attention's forward pass through ATen)
+  piccl_b200/lib/libpiccl_model.so native training step (launches the kernels of libpiccl_ops.so; attention partly through ATen)
   piccl_b200/lib/piccl_sched     schedule dump / validation command line tool
   piccl_b200/lib/coll_bench      OSU-style collective benchmark (fork per GPU, no MPI)
   piccl_b200/lib/loggp_bench     PRTT measurements between two GPUs (input of tools/loggp_param)
@@ -53,7 +53,7 @@ def targets() -> dict[str, dict]:
             "src": _sources("ops/*.cu", "ops/*.cc"),
             "link": ["-shared", "-cudart", "static", "-ldl", "-lpthread", "-lrt"],
         },
-        # the training step: calls libpiccl_ops.so and, for attention's forward pass, ATen
+        # the training step: calls libpiccl_ops.so and, for a part of attention, ATen
         "libpiccl_model.so": {
             "src": _sources("model/*.cc"),
             "flags": [f"-I{p}" for p in (TORCH / "include", TORCH / "include" / "torch" / "csrc" / "api" / "include")],

@@ -13,8 +13,8 @@ The step itself is native (src/model/gpt2_step.cc): residual-add + LayerNorm
 (forward / backward), GEMMs with fused GELU, bias gradients, embedding, softmax cross
 entropy with in-place gradient and AdamW are this framework's CUDA kernels (src/ops);
 for heads of 64 columns so are the backward pass of attention and its forward pass in an
-evaluation (the rest, and other back ends that the program asks PyTorch for, goes
-through PyTorch's fused kernels).
+evaluation, at the sizes where they are the faster kernels (the rest, and other back ends
+that the program asks PyTorch for, goes through PyTorch's fused kernels).
 
 The reference has no model code at all; this module exists for the end-to-end
 data-parallel benchmark (GPT-2 medium under bucketed gradient all-reduce).

@@ -188,6 +188,7 @@ __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, i
     return Pack<T>::down(acc);
   }
 }
+// (Only the aligned loops take these: at odd addresses, with more than two operands, or with destinations read from the table (NDST 0), lines keep the normal priority.)
 struct L2Hints { bool src_done, dst_done; int local_src, local_dst; };
 template <typename T, int OP, int NSRC, int NDST, int U, bool EXACT, bool SCALE = false>      // EXACT: nsrc == NSRC, else the first operand stands in for what is missing; NDST 0: any number, read from the table each time
 __device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
@@ -544,8 +545,8 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
     if (flags & (STEP_END | STEP_FAIL)) break;
     const Action& ac = ai < kSliceCache ? s_act[ai] : L.actions[ai];
     // One fence for both: what the data warps stored comes before the consumers' counters, what they read before the producers'.  It waits for the
-    // acknowledgement of everything the CTA stored, so a credit costs up to a microsecond at the end of a call: 1 MiB blocks of an all-gather 31.6 us, 29.9
-    // with plain stores for the heads, which nothing orders behind the reads.  A release per counter took 38.0, a warp of its own for the heads 32.5.
+    // acknowledgement of everything the CTA stored, so a credit costs up to a microsecond at the end of a call: 1 MiB blocks of an all-gather, with system scope, 31.6 us, 29.9
+    // with plain stores for the heads, which nothing orders behind the reads.  A release per counter took 38.0, a warp of its own for the heads 32.5.  (With GPU scope the call takes 28.7; the others were not timed again.)
     fence_ranks(ka.one_gpu);
 #pragma unroll
     for (int q = 0; q < 2; q++) {

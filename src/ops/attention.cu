@@ -207,7 +207,7 @@ constexpr uint32_t kIdescK = make_idesc_bf16_major(AT_ROWS, AT_STEP, false, fals
 // ------------------------------------------------------------------ forward
 // The two groups of four warps take the steps in turn, each with a maximum, a sum and an accumulator of its own; they are put together at the end.
 // TMEM columns: O 0 and 64, S 128 and 192 (P of a step lies over its S).  A row's maximum is raised only when the new one is more than 2^8
-// above it: until then the sums stay within range, and the accumulator is scaled a few times a row instead of at every step.
+// above it (the conditional rescaling of FlashAttention-4): until then the sums stay within range, and the accumulator is scaled a few times a row instead of at every step.
 __global__ void __launch_bounds__(AT_THREADS, 2) attn_fwd_kernel(const __grid_constant__ AttnArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ int s_abort;
