@@ -126,6 +126,9 @@ class GPT2:
         self.replays = 0             # steps replayed so far
         self._seen: dict = {}        # how often a step was issued call by call; -1: it cannot be captured
         self._counts = (C.c_longlong * 4)()
+        if self.device.type == "cuda":       # PyTorch settles its order of attention's back ends when it is first asked for one; captured steps are known by that order too
+            q = torch.empty(1, 1, 8, 64, dtype=torch.bfloat16, device=self.device)
+            torch._fused_sdp_choice(q, q, q, None, 0.0, True)
 
     # ------------------------------------------------------------------ setup
     def _init_weights(self, seed: int) -> None:

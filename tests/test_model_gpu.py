@@ -232,6 +232,17 @@ def test_a_captured_step_is_not_replayed_under_another_order_of_back_ends():
         assert float(m.forward_backward(a, b)) == want and m.replays == 3
 
 
+def test_the_first_model_of_a_process_is_captured_at_its_third_step():
+    """In a process that has not asked PyTorch for an attention back end before."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    code = ("import torch\nfrom piccl_b200.models.gpt2 import GPT2, GPT2Config\nm = GPT2(GPT2Config.tiny(), seed=1)\nx = torch.zeros(2, 128, dtype=torch.int64, device='cuda')\n"
+            "for _ in range(4): m.forward_backward(x, x)\nassert m.replays == 2, m.replays")
+    r = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_an_interrupt_during_a_capture_leaves_the_model_usable():
     from piccl_b200.models.gpt2 import GPT2, GPT2Config
     cfg = GPT2Config.tiny()
