@@ -31,13 +31,18 @@ Sizes buffer_sizes(const CollArgs& a) {
 }
 
 template <class T>
-ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer, int window) {
+ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer, int window, bool share) {
   ValidateResult res;
   if (window <= 0) window = window_of(fifo_cap);
   int n = a.nranks;
   int64_t st = a.block_stride ? a.block_stride : a.count;
   Sizes sz = buffer_sizes(a);
   std::vector<Program> progs; for (int r = 0; r < n; r++) progs.push_back(compile(a, r));
+  std::vector<std::vector<SharedOps>> shared;
+  if (a.in_place && a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) share = false;      // sums over a send buffer that another rank may still read
+  if (share && !share_operands(progs, shared)) share = false;
+  size_t most_actions = 1;
+  for (auto& p : progs) most_actions = std::max(most_actions, p.actions.size());
   int64_t slot_bytes = std::max<int64_t>(16, seg_elems_req * a.elem_size / 16 * 16);
 
   const int64_t guard = with_data ? 8 : 0;
@@ -80,9 +85,13 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
     std::vector<Cursor> cur(n);
     // Deferred publishing: a push is visible to the consumer, and a pop to the producer, only once the rank that made it has published it, at the
     // latest when it is about to block and when its program ends (the executor's publisher is a warp of its own and may be that late).
+    // Progress: where in the walk a rank has come to (its last finished step), as the executor's progress counters tell it.
+    std::vector<int64_t> passed(n, 0), pub_passed(n, 0);
+    std::vector<std::vector<std::vector<T>>> kept(n, std::vector<std::vector<T>>(window));
     std::vector<int64_t> pushed((size_t)n * n, 0), popped((size_t)n * n, 0), pub_push((size_t)n * n, 0), pub_pop((size_t)n * n, 0);
     auto flush = [&](int r) {
-      bool any = false;
+      bool any = pub_passed[r] != passed[r];
+      pub_passed[r] = passed[r];
       for (int o = 0; o < n; o++) {
         size_t out_c = (size_t)r * n + o, in_c = (size_t)o * n + r;
         if (pub_push[out_c] != pushed[out_c]) { pub_push[out_c] = pushed[out_c]; any = true; }
@@ -117,6 +126,11 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
               if ((defer ? pushed[cn] - pub_pop[cn] : (int64_t)fifo[cn].size()) >= fifo_cap) ready = false;
             }
             for (int i = 0; i < ac.n_recv; i++) {
+              if (ac.recv_peer[i] == kSharedPeer) {
+                const SharedOps& x = shared[r][c.act];
+                if (x.after[i] >= 0 && x.from[i] != r && (defer ? pub_passed[x.from[i]] : passed[x.from[i]]) < step_position(c.seg0, c.seg, (size_t)x.after[i], most_actions, window)) ready = false;
+                continue;
+              }
               size_t cn = (size_t)ac.recv_peer[i] * n + r;
               if (defer ? pub_push[cn] - popped[cn] <= 0 : fifo[cn].empty()) ready = false;
             }
@@ -126,24 +140,35 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
               std::vector<T> val;
               if (with_data) {
                 val.resize(len);
-                const T* src = ac.src_buf == BUF_IN ? in[r] : ac.src_buf == BUF_OUT ? out[r] : ac.src_buf == BUF_SCRATCH ? scratch[r].data() : nullptr;
-                int64_t src_lim = ac.src_buf == BUF_IN ? sz.in_elems : ac.src_buf == BUF_OUT ? sz.out_elems : p.scratch_elems;
+                auto base = [&](int o, uint8_t buf) -> const T* { return buf == BUF_IN ? in[o] : buf == BUF_OUT ? out[o] : buf == BUF_SCRATCH ? scratch[o].data() : nullptr; };
+                auto limit = [&](int o, uint8_t buf) { return buf == BUF_IN ? sz.in_elems : buf == BUF_OUT ? sz.out_elems : progs[o].scratch_elems; };
+                const T* src = base(r, ac.src_buf);
+                const int64_t src_lim = limit(r, ac.src_buf);
+                const std::vector<T> again = kept[r][c.seg - c.seg0];
+                if (ac.src_buf == BUF_KEPT && (int64_t)again.size() != len) { res.error = "no kept value"; return res; }
                 if (src && ac.src_off + hi > src_lim) { res.error = "source range out of bounds"; return res; }
                 // rank order: recv peers below me, me, recv peers above me
                 bool first = true; int pos = 0;
                 auto fold = [&](const T* x) { for (int64_t i = 0; i < len; i++) val[i] = first ? x[i] : apply<T>(op, val[i], x[i]); first = false; };
                 for (int i = 0; i <= ac.n_recv; i++) {
                   if (i == ac.self_pos && src) fold(src + ac.src_off + lo);
-                  if (i < ac.n_recv) {
+                  if (i == ac.self_pos && ac.src_buf == BUF_KEPT) fold(again.data());
+                  if (i < ac.n_recv && ac.recv_peer[i] == kSharedPeer) {
+                    const SharedOps& x = shared[r][c.act];
+                    if (x.off[i] < 0 || x.off[i] + hi > limit(x.from[i], x.buf[i])) { res.error = "shared range out of bounds"; return res; }
+                    fold(base(x.from[i], x.buf[i]) + x.off[i] + lo);
+                  } else if (i < ac.n_recv) {
                     Entry& e = fifo[(size_t)ac.recv_peer[i] * n + r].front();
                     if (e.n != len) { res.error = "fifo entry size mismatch"; return res; }
                     fold(e.data.data()); pos++;
                   }
                 }
               } else {
-                for (int i = 0; i < ac.n_recv; i++) if (fifo[(size_t)ac.recv_peer[i] * n + r].front().n != len) { res.error = "fifo entry size mismatch"; return res; }
+                for (int i = 0; i < ac.n_recv; i++) if (ac.recv_peer[i] != kSharedPeer && fifo[(size_t)ac.recv_peer[i] * n + r].front().n != len) { res.error = "fifo entry size mismatch"; return res; }
               }
-              for (int i = 0; i < ac.n_recv; i++) { fifo[(size_t)ac.recv_peer[i] * n + r].pop_front(); popped[(size_t)ac.recv_peer[i] * n + r]++; }
+              if (ac.keep) kept[r][c.seg - c.seg0] = val;
+              passed[r] = step_position(c.seg0, c.seg, c.act, most_actions, window);
+              for (int i = 0; i < ac.n_recv; i++) if (ac.recv_peer[i] != kSharedPeer) { fifo[(size_t)ac.recv_peer[i] * n + r].pop_front(); popped[(size_t)ac.recv_peer[i] * n + r]++; }
               if (ac.dst_buf != BUF_NONE) {
                 int64_t lim = ac.dst_buf == BUF_OUT ? sz.out_elems : p.scratch_elems;
                 if (ac.dst_buf == BUF_IN || ac.dst_off + hi > lim || ac.dst_off + lo < 0) { res.error = "destination range out of bounds"; return res; }
@@ -227,13 +252,13 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
 
 }  // namespace
 
-ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish, int window) {
-  if (integer) return run<int32_t>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window);
-  return run<float>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window);
+ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish, int window, bool share) {
+  if (integer) return run<int32_t>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, share);
+  return run<float>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, share);
 }
 
-ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish, int window) {
-  return run<float>(a, 0, false, fifo_cap, (int64_t)(256 * 1024) / a.elem_size, n_cta, defer_publish, window);
+ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish, int window, bool share) {
+  return run<float>(a, 0, false, fifo_cap, (int64_t)(256 * 1024) / a.elem_size, n_cta, defer_publish, window, share);
 }
 
 }  // namespace piccl

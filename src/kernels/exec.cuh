@@ -1,10 +1,11 @@
 // Device-side data structures of the fused collective executor and the
 // layout of the per-rank symmetric heap.
 //
-//   heap = [ tail counters | head counters | scratch | FIFO slots ]
+//   heap = [ tail counters | head counters | progress counters | ... | scratch | FIFO slots ]
 //
 // tail[src][cta]  (in the receiver's heap, written by `src`): entries `src` has pushed
 // head[dst][cta]  (in the sender's heap, written by `dst`):   entries `dst` has consumed
+// progress[cta]   (in the rank's own heap):               steps it has published, where ranks read each other's buffers (one launch on one GPU)
 // slot(src, cta, i) (in the receiver's heap): payload of entry number e with e % nslot == i
 //
 // All counters only ever grow, over the whole life of the communicator, so a
@@ -28,7 +29,7 @@ constexpr int kLLFifoCta = 16, kLLFifoSlots = 8, kLLFifoSlotBytes = 8192;   // l
 struct RankCtx {
   int rank, nranks, max_cta, nslot;
   long long slot_bytes;
-  long long tail_off, head_off, ll_off, scratch_off, fifo_off, heap_bytes;
+  long long tail_off, head_off, prog_off, ll_off, scratch_off, fifo_off, heap_bytes;
   long long ll_slot_bytes;                // bytes of one low-latency slot (2 x the largest payload)
   long long scratch_bytes;
   long long llf_off, llf_head_off;                // low-latency FIFO of the executor: lines and head counters
@@ -45,6 +46,7 @@ struct RankCtx {
 struct LaunchRank {
   RankCtx* ctx;
   const Action* actions;
+  const SharedOps* shared;                // of the actions, where ranks read each other's buffers; else null
   int n_actions;
   int pad;
   const void* in;
@@ -62,6 +64,11 @@ struct KernelArgs {
   long long seg_bytes;                    // bytes of a segment and of its slot
   int one_gpu;                            // 1: every rank's heap is on this GPU: counters and fences need no scope beyond it
   int leave_first;                        // with their last use leave L2 first: operands (1), results (2)
+  // Ranks that read each other's buffers (prog_total != 0): r[i] is rank i.  Each raises a progress counter per CTA, from call to call by `prog_total`; within a call to what
+  // step_position says of the step it has published.
+  uint8_t working[kMaxVRanks];            // the ranks that have anything to do, and the launch's CTAs
+  int prog_actions;                       // most actions of any rank
+  long long prog_total;
   int nslot, window;                      // slots; segments that are walked together, at most half the slots
   unsigned long long timeout_ns;
   LaunchRank r[kMaxVRanks];

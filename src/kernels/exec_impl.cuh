@@ -123,6 +123,17 @@ template <typename A> __device__ __forceinline__ A scale_val(A v, float s) { ret
 template <> __device__ __forceinline__ float scale_val<float>(float v, float s) { return v * s; }
 template <> __device__ __forceinline__ double scale_val<double>(double v, float s) { return v * (double)s; }
 
+// Operands to scale (avg): bit s, operand s is an original contribution; bit 8 + s, of another rank, which would have put it into a slot: it is rounded to the
+// element type as it would be there, so that a call's result does not depend on how its operands came.
+constexpr int kRoundedShift = 8;
+template <typename T, typename A> __device__ __forceinline__ A scale_operand(A v, int scaled, int s, float scale) {
+  if (scaled >> s & 1) {
+    v = scale_val<A>(v, scale);
+    if (scaled >> (s + kRoundedShift) & 1) v = Cvt<T>::up(Cvt<T>::down(v));
+  }
+  return v;
+}
+
 // ---------------------------------------------------------------- bounded wait
 struct WaitCtx { RankCtx* ctx; unsigned long long timeout_ns; int cta, action, segment; bool one_gpu; };
 
@@ -154,7 +165,7 @@ static __device__ __noinline__ bool wait_counter(const unsigned long long* flag,
 // ---------------------------------------------------------------- data movement
 __device__ __forceinline__ int data_threads() { return (int)blockDim.x - kCtlThreads; }
 
-// value = reduce(src[0..nsrc)) -> dst[0..ndst), everything 16-byte aligned; `scaled`: index of the operand that is scaled first (avg), or -1.
+// value = reduce(src[0..nsrc)) -> dst[0..ndst), everything 16-byte aligned; `scaled`: see scale_operand.
 // The operands' packs stay as they were loaded until they are combined, so a thread has NSRC * U loads of 16 bytes in flight and no array of
 // accumulators; offsets are 32-bit (a segment is at most a slot).  Whatever U is, pack p is thread p % (data threads)'s, so a step may read what an earlier one
 // wrote.  The last round is as wide as the others instead of being finished a pack at a time, which took up to U - 1 further round trips: what lies
@@ -169,17 +180,17 @@ __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, i
     if (NSRC == 1 && !SCALE) return v[0];
     A acc[N];
     Pack<T>::up(v[0], acc);
-    if (SCALE && scaled == 0) {
+    if (SCALE) {
 #pragma unroll
-      for (int e = 0; e < N; e++) acc[e] = scale_val<A>(acc[e], scale);
+      for (int e = 0; e < N; e++) acc[e] = scale_operand<T, A>(acc[e], scaled, 0, scale);
     }
 #pragma unroll
     for (int s = 1; s < NSRC; s++) {
       if (s < nsrc) {
         A x[N]; Pack<T>::up(v[s * stride], x);
-        if (SCALE && scaled == s) {
+        if (SCALE) {
 #pragma unroll
-          for (int e = 0; e < N; e++) x[e] = scale_val<A>(x[e], scale);
+          for (int e = 0; e < N; e++) x[e] = scale_operand<T, A>(x[e], scaled, s, scale);
         }
 #pragma unroll
         for (int e = 0; e < N; e++) acc[e] = red<OP, A>(acc[e], x[e]);
@@ -233,18 +244,18 @@ __device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char
 }
 template <typename T, int OP>
 __device__ __forceinline__ void move_aligned(const char* const* src, int nsrc, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
-  if (OP == OP_COPY || (nsrc == 1 && scaled < 0)) {
-    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(src, 1, dst, 1, n, -1, scale, h);
-    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(src, 1, dst, 2, n, -1, scale, h);
-    else stream<T, OP, 1, 0, 4, true>(src, 1, dst, ndst, n, -1, scale, h);
+  if (OP == OP_COPY || (nsrc == 1 && !scaled)) {
+    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(src, 1, dst, 1, n, 0, scale, h);
+    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(src, 1, dst, 2, n, 0, scale, h);
+    else stream<T, OP, 1, 0, 4, true>(src, 1, dst, ndst, n, 0, scale, h);
   } else if constexpr (OP != OP_COPY) {
     // Scaled operands (avg, which is a sum) have loops of their own too: in the general one a lone operand was loaded twice and the destinations read
     // from the table for each pack (25 MiB of bf16 averaged among four ranks: 155 us, now 136).
-    if (scaled >= 0) {
+    if (scaled) {
       if constexpr (OP == 0) {
         if (nsrc == 1) {
-          if (ndst == 1) stream<T, OP, 1, 1, 8, true, true>(src, 1, dst, 1, n, 0, scale, h);
-          else stream<T, OP, 1, 0, 4, true, true>(src, 1, dst, ndst, n, 0, scale, h);
+          if (ndst == 1) stream<T, OP, 1, 1, 8, true, true>(src, 1, dst, 1, n, 1, scale, h);
+          else stream<T, OP, 1, 0, 4, true, true>(src, 1, dst, ndst, n, 1, scale, h);
         }
         else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true, true>(src, 2, dst, 1, n, scaled, scale, h);
         else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true, true>(src, 2, dst, 2, n, scaled, scale, h);
@@ -252,12 +263,12 @@ __device__ __forceinline__ void move_aligned(const char* const* src, int nsrc, c
         else stream<T, OP, kMaxActionPeers + 1, 0, 1, false, true>(src, nsrc, dst, ndst, n, scaled, scale, h);
       }
     }
-    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(src, 2, dst, 1, n, -1, scale, h);
-    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(src, 2, dst, 2, n, -1, scale, h);
-    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(src, 4, dst, ndst, n, -1, scale, h);
-    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(src, nsrc, dst, ndst, n, -1, scale, h);
-    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(src, nsrc, dst, ndst, n, -1, scale, h);
-    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(src, nsrc, dst, ndst, n, -1, scale, h);
+    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(src, 2, dst, 1, n, 0, scale, h);
+    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(src, 2, dst, 2, n, 0, scale, h);
+    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(src, 4, dst, ndst, n, 0, scale, h);
+    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(src, nsrc, dst, ndst, n, 0, scale, h);
+    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(src, nsrc, dst, ndst, n, 0, scale, h);
+    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(src, nsrc, dst, ndst, n, 0, scale, h);
   }
 }
 
@@ -281,86 +292,155 @@ static __device__ __noinline__ void store_part(char* p, const uint4 v, int from,
   union { uint4 v; unsigned char b[16]; } u; u.v = v;
   for (int i = from; i < to; i++) reinterpret_cast<unsigned char*>(p)[i] = u.b[i];
 }
-// The same movement where the local operand (source index local_src) or dst[0] is at any byte address: an unaligned source is read as the
-// two aligned words around each pack (the second one is the neighbour's first and hits L2), an unaligned destination is written as aligned
+// The same movement where sources or the local destination (dst[local_dst]) are at any byte address: an unaligned source is read as the
+// two aligned words around each pack, an unaligned destination is written as aligned
 // words too, put together from a lane's pack and the one before it.  Only the two ends of the run of packs that a warp
-// writes (kRun blocks of 512 bytes) go out in bytes.  (1 MiB blocks at odd
+// writes (2 to 8 blocks of 512 bytes) go out in bytes.  (1 MiB blocks at odd
 // addresses, all-gather of four ranks: 30 us; an element at a time 171.)
 // An aligned word that is read may reach up to 15 bytes beyond the operand's ends; it never leaves the 16-byte granule of a byte that
 // belongs to the operand, and allocations are whole granules.
-constexpr int kRun = 4;
-template <typename T, int OP>
-__device__ __noinline__ void reduce_copy_shift(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst, int local_dst, long long npack, bool do_scale, float scale) {
+// The words of a run of packs that one warp moves: w[u] is lane's word of block u, and, for an operand that is off by m bytes, `last` the word after the run.  A pack's second
+// word is the next lane's first one (of its block, or of the run), so it comes by shuffle: loaded again past L1, an operand
+// costs the L2 twice its bytes (us: reduce-scatter of 8 x 2 MB of bf16 at odd addresses 119, now 104, 4 x 0.85 MB averaged 27.2 and 24.7; all-gather of 4 x 1 MiB 18.4 either way).
+__device__ __forceinline__ int address_mod(const void* p) { return (int)(reinterpret_cast<uintptr_t>(p) & 15); }      // 0 for a slot
+template <int RUN> struct RunWords { uint4 w[RUN], last; };
+template <int RUN>
+__device__ __forceinline__ void load_run(RunWords<RUN>& r, const char* src, int m, long long run, int lane, long long npack) {
+  const char* const base = src - m;
+  const long long top = m ? npack : npack - 1;         // beyond the end: the last word again (a load under a condition makes the compiler spill)
+#pragma unroll
+  for (int u = 0; u < RUN; u++) r.w[u] = ld_slot(base + min(run + u * 32 + lane, top) * 16);
+  r.last = m ? ld_slot(base + min(run + RUN * 32, top) * 16) : r.w[0];
+}
+template <int RUN>
+__device__ __forceinline__ uint4 run_pack(const RunWords<RUN>& r, int u, int m, int lane) {
+  if (m == 0) return r.w[u];
+  const uint4 mine = r.w[u], over = u + 1 < RUN ? r.w[u + 1 < RUN ? u + 1 : u] : r.last;
+  // lane 0 offers the first word of the next block, which lane 31 needs; the others their own
+  const uint4 offer = lane == 0 ? over : mine;
+  const int from = (lane + 1) & 31;
+  uint4 hi;
+  hi.x = __shfl_sync(0xffffffffu, offer.x, from); hi.y = __shfl_sync(0xffffffffu, offer.y, from);
+  hi.z = __shfl_sync(0xffffffffu, offer.z, from); hi.w = __shfl_sync(0xffffffffu, offer.w, from);
+  return shift_pair(mine, hi, m);
+}
+// Packs o[] of a run to every destination.
+template <int RUN>
+__device__ __forceinline__ void store_run(const uint4 (&o)[RUN], int ndst, char* const* dst, int local_dst, int dm, long long run, int lane, long long npack) {
+  for (int d = 0; d < ndst; d++) {
+    if (d != local_dst || dm == 0) {
+#pragma unroll
+      for (int u = 0; u < RUN; u++) { const long long p = run + u * 32 + lane; if (p < npack) st_vec(dst[d] + p * 16, o[u]); }
+      continue;
+    }
+#pragma unroll
+    for (int u = 0; u < RUN; u++) {
+      const long long p = run + u * 32 + lane;
+      // the pack before: lane 31 offers the block's before, which lane 0 needs
+      const uint4 offer = lane == 31 && u > 0 ? o[u > 0 ? u - 1 : 0] : o[u];
+      const int from = (lane + 31) & 31;
+      uint4 prev;
+      prev.x = __shfl_sync(0xffffffffu, offer.x, from); prev.y = __shfl_sync(0xffffffffu, offer.y, from);
+      prev.z = __shfl_sync(0xffffffffu, offer.z, from); prev.w = __shfl_sync(0xffffffffu, offer.w, from);
+      if (p < npack) {
+        char* const w = dst[d] + p * 16 - dm;        // aligned word: the last dm bytes of the pack before, then this pack's first 16 - dm
+        const uint4 v = shift_pair(prev, o[u], 16 - dm);
+        if (u == 0 && lane == 0) store_part(w, v, dm, 16);
+        else st_vec(w, v);
+        if (p == npack - 1 || (u == RUN - 1 && lane == 31)) store_part(w + 16, shift_pair(o[u], o[u], 16 - dm), 0, dm);
+      }
+    }
+  }
+}
+template <typename T, int OP, int RUN>
+__device__ __noinline__ void copy_shift(const char* src, int ndst, char* const* dst, int local_dst, long long npack) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = data_threads() >> 5;
+  char* one[1] = {dst[0]};
+  int dm = local_dst >= 0 ? address_mod(dst[local_dst]) : 0;
+  if (ndst == 1 && dm) {                               // (a shift for the source and one for the destination: all-gather of 4 x 1 MiB 20.5 us)  One destination: its whole words, for which one shift will do, and the bytes at both ends
+    const int head = 16 - dm;
+    if (warp == nwarp - 1 && lane < 16) {
+      const long long at = lane < head ? lane : npack * 16 - 16 + lane;      // (the last dm bytes are the words' remainder)
+      one[0][at] = *reinterpret_cast<const volatile char*>(src + at);
+    }
+    src += head; one[0] += head; npack -= 1; dm = 0; dst = one;
+  }
+  const int m = address_mod(src);
+  for (long long run = (long long)warp * (32 * RUN); run < npack; run += (long long)nwarp * (32 * RUN)) {
+    RunWords<RUN> r;
+    load_run(r, src, m, run, lane, npack);
+    uint4 o[RUN];
+#pragma unroll
+    for (int u = 0; u < RUN; u++) o[u] = run_pack(r, u, m, lane);
+    store_run<RUN>(o, ndst, dst, local_dst, dm, run, lane, npack);
+  }
+}
+template <typename T, int OP, int RUN>
+__device__ __noinline__ void reduce_shift(int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
   typedef typename AccOf<T>::type A;
   constexpr int N = Pack<T>::N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = data_threads() >> 5;
-  const int sm = local_src >= 0 ? (int)(reinterpret_cast<uintptr_t>(src[local_src]) & 15) : 0;
-  const int dm = local_dst >= 0 ? (int)(reinterpret_cast<uintptr_t>(dst[local_dst]) & 15) : 0;
-  for (long long run = (long long)warp * (32 * kRun); run < npack; run += (long long)nwarp * (32 * kRun)) {
-    uint4 o[kRun];
-    if (OP == OP_COPY || (nsrc == 1 && !do_scale)) {
-      uint4 lo[kRun], hi[kRun];
+  const int dm = local_dst >= 0 ? address_mod(dst[local_dst]) : 0;
+  for (long long run = (long long)warp * (32 * RUN); run < npack; run += (long long)nwarp * (32 * RUN)) {
+    A acc[RUN][N];
+    auto operand = [&](const RunWords<RUN>& r, int u, int s, int m, A (&x)[N]) {
+      Pack<T>::up(run_pack(r, u, m, lane), x);
+      if (scaled >> s & 1) {
 #pragma unroll
-      for (int u = 0; u < kRun; u++) {                 // beyond the end: the last pack again (a load under a condition makes the compiler spill)
-        const char* q = src[0] + min(run + u * 32 + lane, npack - 1) * 16 - sm;      // sm is 0 for a slot
-        lo[u] = ld_slot(q); hi[u] = ld_slot(q + (sm ? 16 : 0));
+        for (int e = 0; e < N; e++) x[e] = scale_operand<T, A>(x[e], scaled, s, scale);
       }
+    };
+    {                                                // two operands' loads in flight, beside no accumulators yet
+      const int second = min(1, nsrc - 1), m = address_mod(src[0]), m2 = address_mod(src[second]);
+      RunWords<RUN> r, r2;
+      load_run(r, src[0], m, run, lane, npack);
+      load_run(r2, src[second], m2, run, lane, npack);
 #pragma unroll
-      for (int u = 0; u < kRun; u++) o[u] = sm ? shift_pair(lo[u], hi[u], sm) : lo[u];
-    } else {
-      A acc[kRun][N];
+      for (int u = 0; u < RUN; u++) {
+        operand(r, u, 0, m, acc[u]);
+        if (nsrc > 1) {
+          A x[N]; operand(r2, u, 1, m2, x);
+#pragma unroll
+          for (int e = 0; e < N; e++) acc[u][e] = red<OP, A>(acc[u][e], x[e]);
+        }
+      }
+    }
 #pragma unroll 1
-      for (int s = 0; s < nsrc; s++) {
-        const int m = s == local_src ? sm : 0;
-        uint4 lo[kRun], hi[kRun];
+    for (int s = 2; s < nsrc; s++) {
+      const int m = address_mod(src[s]);
+      RunWords<RUN> r;
+      load_run(r, src[s], m, run, lane, npack);
 #pragma unroll
-        for (int u = 0; u < kRun; u++) {
-          const char* q = src[s] + min(run + u * 32 + lane, npack - 1) * 16 - m;
-          lo[u] = ld_slot(q); hi[u] = ld_slot(q + (m ? 16 : 0));
-        }
-        const bool sc = do_scale && s == local_src;
+      for (int u = 0; u < RUN; u++) {
+        A x[N]; operand(r, u, s, m, x);
 #pragma unroll
-        for (int u = 0; u < kRun; u++) {
-          A x[N]; Pack<T>::up(m ? shift_pair(lo[u], hi[u], m) : lo[u], x);
-#pragma unroll
-          for (int e = 0; e < N; e++) { const A y = sc ? scale_val<A>(x[e], scale) : x[e]; acc[u][e] = s == 0 ? y : red<OP, A>(acc[u][e], y); }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kRun; u++) o[u] = Pack<T>::down(acc[u]);
-    }
-    for (int d = 0; d < ndst; d++) {
-      if (d != local_dst || dm == 0) {
-#pragma unroll
-        for (int u = 0; u < kRun; u++) { const long long p = run + u * 32 + lane; if (p < npack) st_vec(dst[d] + p * 16, o[u]); }
-        continue;
-      }
-      uint4 last = make_uint4(0, 0, 0, 0);             // the pack before lane 0's
-#pragma unroll
-      for (int u = 0; u < kRun; u++) {
-        const long long p = run + u * 32 + lane;
-        uint4 prev;
-        prev.x = __shfl_up_sync(0xffffffffu, o[u].x, 1); prev.y = __shfl_up_sync(0xffffffffu, o[u].y, 1);
-        prev.z = __shfl_up_sync(0xffffffffu, o[u].z, 1); prev.w = __shfl_up_sync(0xffffffffu, o[u].w, 1);
-        if (lane == 0) prev = last;
-        last.x = __shfl_sync(0xffffffffu, o[u].x, 31); last.y = __shfl_sync(0xffffffffu, o[u].y, 31);
-        last.z = __shfl_sync(0xffffffffu, o[u].z, 31); last.w = __shfl_sync(0xffffffffu, o[u].w, 31);
-        if (p < npack) {
-          char* const w = dst[d] + p * 16 - dm;        // aligned word: the last dm bytes of the pack before, then this pack's first 16 - dm
-          const uint4 v = shift_pair(prev, o[u], 16 - dm);
-          if (u == 0 && lane == 0) store_part(w, v, dm, 16);
-          else st_vec(w, v);
-          if (p == npack - 1 || (u == kRun - 1 && lane == 31)) store_part(w + 16, shift_pair(o[u], o[u], 16 - dm), 0, dm);
-        }
+        for (int e = 0; e < N; e++) acc[u][e] = red<OP, A>(acc[u][e], x[e]);
       }
     }
+    uint4 o[RUN];
+#pragma unroll
+    for (int u = 0; u < RUN; u++) o[u] = Pack<T>::down(acc[u]);
+    store_run<RUN>(o, ndst, dst, local_dst, dm, run, lane, npack);
+  }
+}
+// A warp takes runs of 2, 4 or 8 blocks (sums: 2 or 4): as few rounds as can be, and then over as many warps.
+template <typename T, int OP>
+__device__ __forceinline__ void reduce_copy_shift(int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
+  const long long blocks = (npack + data_threads() - 1) / data_threads();      // per warp
+  if (OP == OP_COPY || (nsrc == 1 && !scaled)) {
+    if (blocks > 4) copy_shift<T, OP, 8>(src[0], ndst, dst, local_dst, npack);
+    else if (blocks > 2) copy_shift<T, OP, 4>(src[0], ndst, dst, local_dst, npack);
+    else copy_shift<T, OP, 2>(src[0], ndst, dst, local_dst, npack);
+  } else if constexpr (OP != OP_COPY) {
+    if (blocks > 2) reduce_shift<T, OP, 4>(nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
+    else reduce_shift<T, OP, 2>(nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
   }
 }
 
 // Element-wise path: the last, partial pack of an action.
 template <typename T, int OP>
 __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
-                                                 long long first, long long nelem, bool do_scale, float scale) {
+                                                 long long first, long long nelem, int scaled, float scale) {
   typedef typename AccOf<T>::type A;
   for (long long i = first + threadIdx.x; i < nelem; i += data_threads()) {
     A acc = A();
@@ -368,7 +448,7 @@ __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, 
       const T* p = reinterpret_cast<const T*>(src[s]) + i;
       T raw = (local_src == s) ? *p : *reinterpret_cast<const volatile T*>(p);
       A x = Cvt<T>::up(raw);
-      if (do_scale && local_src == s) x = scale_val<A>(x, scale);
+      x = scale_operand<T, A>(x, scaled, s, scale);
       acc = (s == 0) ? x : red<OP, A>(acc, x);
     }
     T o = Cvt<T>::down(acc);
@@ -377,6 +457,7 @@ __device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, 
 }
 
 // ---------------------------------------------------------------- the kernel
+constexpr int kSharedCache = 64;       // and their operands in other ranks' buffers
 constexpr int kSliceCache = 192;      // actions kept in shared memory, with the CTA's slice of each
 
 constexpr int kStepDepth = 4;         // steps the waiter may be ahead of the publisher
@@ -384,9 +465,11 @@ struct StepDesc {
   const char* src[kMaxActionPeers + 1];      // operands in rank order: receive peers below me, my own buffer, receive peers above me
   char* dst[kMaxActionPeers + 1];            // local destination first, then the send peers
   long long len;                             // elements
+  long long position;                        // in the rank's walk (step_position)
   int action, nsrc, ndst, local_src, local_dst, flags;
+  int scaled;                                // operands to scale (scale_operand)
 };
-enum : int { STEP_SCALE = 1, STEP_ALIGNED = 2, STEP_LOCAL_DEP = 4, STEP_FAIL = 8, STEP_END = 16, STEP_SRC_DONE = 32, STEP_DST_DONE = 64 };
+enum : int { STEP_ALIGNED = 2, STEP_LOCAL_DEP = 4, STEP_FAIL = 8, STEP_END = 16, STEP_SRC_DONE = 32, STEP_DST_DONE = 64 };
 __device__ __forceinline__ void bar_sync_n(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive_n(int id, int n) { __threadfence_block(); asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
@@ -394,7 +477,7 @@ __device__ __forceinline__ void bar_arrive_n(int id, int n) { __threadfence_bloc
 // 15 % in registers).
 template <typename T, int OP, bool SHIFT>
 __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const KernelArgs ka) {
-  const int vr = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta;
+  const int launched = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta, vr = ka.working[launched];
   const LaunchRank& L = ka.r[vr];
   RankCtx* __restrict__ ctx = L.ctx;
   const int tid = threadIdx.x, lane = tid & 31, ndata = data_threads();
@@ -406,11 +489,14 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   __shared__ Action s_act[kSliceCache];
   __shared__ int s_maxseg;
   __shared__ volatile int s_published;             // steps whose descriptor may be used again
+  __shared__ SharedOps s_shared[kSharedCache];
+  __shared__ const char *s_in[kMaxVRanks], *s_out[kMaxVRanks], *s_kept[2];      // all ranks' buffers; the slots of a window's entries that this rank reads again
 
   // everything read from the context more than once is fetched once, in parallel
   const int rank = ctx->rank, nranks = ctx->nranks, max_cta = ctx->max_cta;
-  const long long tail_off = ctx->tail_off, head_off = ctx->head_off, fifo_off = ctx->fifo_off, scratch_off = ctx->scratch_off, chan_bytes = ctx->nslot * ctx->slot_bytes;
+  const long long tail_off = ctx->tail_off, head_off = ctx->head_off, fifo_off = ctx->fifo_off, scratch_off = ctx->scratch_off, prog_off = ctx->prog_off, chan_bytes = ctx->nslot * ctx->slot_bytes;
   if (tid < nranks) s_heap[tid] = ctx->heap[tid];
+  if (tid < ka.n_vrank) { s_in[tid] = (const char*)ka.r[tid].in; s_out[tid] = (const char*)ka.r[tid].out; }
   if (tid == 0) { s_maxseg = 0; s_published = 0; }
   __syncthreads();
   const long long seg_bytes = ka.seg_bytes, seg_elems = (seg_bytes / 16) * (esz >= 16 ? 1 : 16 / esz);
@@ -420,6 +506,7 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
       const Action a = L.actions[ai];
       const Slice sl = slice_of(a.count, esz, cta, ka.n_cta, seg_bytes);
       if (ai < kSliceCache) { s_lo[ai] = sl.lo; s_hi[ai] = sl.hi; s_act[ai] = a; }
+      if (L.shared && ai < kSharedCache) s_shared[ai] = L.shared[ai];
       m = max(m, sl.nseg);
     }
     if (m) atomicMax(&s_maxseg, m);
@@ -443,12 +530,12 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
         const char* const* const src = st.src; char* const* const dst = st.dst;
         const long long len = st.len;
         const int nsrc = st.nsrc, ndst = st.ndst, local_src = st.local_src;
-        const bool do_scale = flags & STEP_SCALE;
+        const int scaled = st.scaled;
         constexpr int N = Pack<T>::N;
         const long long nfull = (SHIFT || (flags & STEP_ALIGNED)) ? len / N : 0;
-        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(nsrc, src, local_src, ndst, dst, st.local_dst, nfull, do_scale, ka.scale); }
-        else if (nfull) move_aligned<T, OP>(src, nsrc, dst, ndst, (int)nfull, do_scale ? local_src : -1, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
-        if (nfull * N < len) reduce_copy_elem<T, OP>(nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale, ka.scale);
+        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(nsrc, src, ndst, dst, st.local_dst, nfull, scaled, ka.scale); }
+        else if (nfull) move_aligned<T, OP>(src, nsrc, dst, ndst, (int)nfull, scaled, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
+        if (nfull * N < len) reduce_copy_elem<T, OP>(nsrc, src, local_src, ndst, dst, nfull * N, len, scaled, ka.scale);
       }
       bar_arrive_n(kDone + d, ndata + 32);
       if (flags & (STEP_END | STEP_FAIL)) return;
@@ -464,9 +551,13 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   }
   const unsigned nslot = (unsigned)ka.nslot;
   const long long mine = (long long)(rank * max_cta + cta) * kFlagStride;      // my counters in a peer's heap
+  // progress of this CTA of every rank: all were raised by the same calls, so mine, which only I write, says where the others' began
+  const long long my_prog = prog_off + (long long)cta * kFlagStride;
+  const unsigned long long prog0 = ka.prog_total ? *reinterpret_cast<const unsigned long long*>(my_heap + my_prog) : 0;
 
   if (tid < ndata + 32) {                          // ---------------- waiter
     WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta; w.one_gpu = ka.one_gpu;
+    unsigned long long seen_prog = 0;              // of rank `lane`
     unsigned long long seen_head[2] = {0, 0};      // what a peer had consumed when last looked: no need to look again while that is credit enough
     int k = 0;
     bool failed = false;
@@ -496,12 +587,17 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
           StepDesc& st = s_step[k % kStepDepth];
           bool ok = true;
           w.action = ai; w.segment = seg;
+          const char* const kept = ac.src_buf == BUF_KEPT ? s_kept[seg - seg0] : nullptr;
+          if (ac.keep) __syncwarp();               // (before the same step puts another one there)
+          bool aligned = true, dep = has_src && ac.src_buf != BUF_IN;      // dep: an operand that earlier steps of this CTA wrote
+          int scaled = 0;
 #pragma unroll
           for (int q = 0; q < 2; q++) {
             const int p = lane + 32 * q;
             const long long theirs = (long long)(p * max_cta + cta) * kFlagStride;      // peer p's counters in my heap
             for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) {
               st.dst[j + has_dst] = s_heap[p] + fifo_off + (long long)(rank * max_cta + cta) * chan_bytes + (long long)(sent[q] % nslot) * seg_bytes;
+              if (ac.keep && j == 0) s_kept[seg - seg0] = st.dst[j + has_dst];
               if (++sent[q] > seen_head[q] + nslot && ok)
                 ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + head_off + theirs), sent[q] - nslot, w, 1, p, &seen_head[q]);
             }
@@ -511,15 +607,34 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
               if (ok) ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + tail_off + theirs), rcvd[q], w, 2, p);
             }
           }
+          if (L.shared) {                          // operands in the buffers of rank `lane`
+            const SharedOps& x = ai < kSharedCache ? s_shared[ai] : L.shared[ai];
+            for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == kSharedPeer && x.from[j] == lane) {
+              const int at = j + (has_src && j >= ac.self_pos);
+              const char* const from = (x.buf[j] == BUF_IN ? s_in[lane] : x.buf[j] == BUF_OUT ? s_out[lane] : s_heap[lane] + scratch_off) + (x.off[j] + lo) * esz;
+              st.src[at] = from;
+              aligned &= (reinterpret_cast<uintptr_t>(from) & 15) == 0;
+              dep |= lane == rank && x.after[j] >= 0;
+              if (x.scaled >> j & 1) scaled |= (lane == rank ? 1 : 1 | 1 << kRoundedShift) << at;
+              const unsigned long long want = prog0 + (unsigned long long)step_position(seg0, seg, x.after[j], ka.prog_actions, ka.window);
+              if (x.after[j] >= 0 && lane != rank && want > seen_prog && ok)
+                ok = wait_counter(reinterpret_cast<const unsigned long long*>(s_heap[lane] + my_prog), want, w, 2, lane, &seen_prog);
+            }
+            aligned = __all_sync(0xffffffffu, aligned); dep = __any_sync(0xffffffffu, dep);
+            scaled = __reduce_or_sync(0xffffffffu, scaled);
+          }
           ok = __all_sync(0xffffffffu, ok);
           if (lane == 0) {
             const char* lsrc = nullptr; char* ldst = nullptr;
-            if (has_src) { lsrc = (ac.src_buf == BUF_IN ? (const char*)L.in : ac.src_buf == BUF_OUT ? (const char*)L.out : my_heap + scratch_off) + (ac.src_off + lo) * esz; st.src[ac.self_pos] = lsrc; }
+            if (has_src) { lsrc = kept ? kept : (ac.src_buf == BUF_IN ? (const char*)L.in : ac.src_buf == BUF_OUT ? (const char*)L.out : my_heap + scratch_off) + (ac.src_off + lo) * esz; st.src[ac.self_pos] = lsrc; }
             if (has_dst) { ldst = (ac.dst_buf == BUF_OUT ? (char*)L.out : my_heap + scratch_off) + (ac.dst_off + lo) * esz; st.dst[0] = ldst; }
             st.len = (lo + seg_elems < sl_hi ? lo + seg_elems : sl_hi) - lo;
             st.action = ai; st.nsrc = ac.n_recv + has_src; st.ndst = ac.n_send + has_dst; st.local_src = has_src ? ac.self_pos : -1; st.local_dst = has_dst ? 0 : -1;
-            st.flags = (ka.avg && (ac.flags & ACT_SCALE_SRC) && has_src ? STEP_SCALE : 0) | (((reinterpret_cast<uintptr_t>(lsrc) | reinterpret_cast<uintptr_t>(ldst)) & 15) == 0 ? STEP_ALIGNED : 0) |
-                       (has_src && ac.src_buf != BUF_IN ? STEP_LOCAL_DEP : 0) | ((ka.leave_first & 1) && (ac.flags & ACT_SRC_DONE) ? STEP_SRC_DONE : 0) | ((ka.leave_first & 2) && (ac.flags & ACT_DST_DONE) ? STEP_DST_DONE : 0) | (ok ? 0 : STEP_FAIL);
+            if ((ac.flags & ACT_SCALE_SRC) && has_src) scaled |= 1 << ac.self_pos;
+            st.scaled = ka.avg ? scaled : 0;
+            st.position = step_position(seg0, seg, ai, ka.prog_actions, ka.window);
+            st.flags = ((aligned ? (reinterpret_cast<uintptr_t>(lsrc) | reinterpret_cast<uintptr_t>(ldst)) & 15 : 1) == 0 ? STEP_ALIGNED : 0) |
+                       (dep ? STEP_LOCAL_DEP : 0) | ((ka.leave_first & 1) && (ac.flags & ACT_SRC_DONE) ? STEP_SRC_DONE : 0) | ((ka.leave_first & 2) && (ac.flags & ACT_DST_DONE) ? STEP_DST_DONE : 0) | (ok ? 0 : STEP_FAIL);
           }
           __syncwarp();
           bar_arrive_n(kReady + k % kStepDepth, ndata + 32);
@@ -554,6 +669,7 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
       for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[p] + tail_off + mine), ++sent[q], ka.one_gpu);
       for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[p] + head_off + mine), ++rcvd[q], ka.one_gpu);
     }
+    if (ka.prog_total && lane == 0) st_relaxed(reinterpret_cast<unsigned long long*>(my_heap + my_prog), prog0 + (unsigned long long)s_step[d].position, ka.one_gpu);
     __syncwarp();
     if (lane == 0) { __threadfence_block(); s_published = k + 1; }
   }
@@ -561,6 +677,11 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   for (int q = 0; q < 2; q++) {
     const int p = lane + 32 * q;
     if (p < nranks) { ctx->sent[p * max_cta + cta] = sent[q]; ctx->rcvd[p * max_cta + cta] = rcvd[q]; }
+  }
+  if (ka.prog_total) {                               // the first rank also counts for those that have nothing to do
+    bool raise = lane == rank;
+    if (launched == 0 && lane < ka.n_vrank) raise |= ka.r[lane].n_actions == 0;
+    if (raise) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[lane] + my_prog), prog0 + (unsigned long long)ka.prog_total, ka.one_gpu);
   }
 }
 

@@ -96,7 +96,7 @@ int piccl_comm_create(int rank, int nranks, int device, const piccl_config_t* us
   if (cfg.tp_bytes <= 0) cfg.tp_bytes = (long long)e.tp_mb << 20;
   c->cfg.tp_bytes = cfg.tp_bytes;
   const long long tp_flags = cfg.tp_bytes > 0 ? (1 << 20) : 0;
-  x.tail_off = 0; x.head_off = flags; x.ll_off = 2 * flags; x.tp_flag_off = x.ll_off + ll_bytes;
+  x.tail_off = 0; x.head_off = flags; x.prog_off = 2 * flags; x.ll_off = x.prog_off + round_up((long long)cfg.max_cta * kFlagStride, 4096); x.tp_flag_off = x.ll_off + ll_bytes;
   // low-latency FIFO of the executor (all collectives, small messages): head counters, then the lines
   x.llf_head_off = x.tp_flag_off + tp_flags;
   x.llf_off = x.llf_head_off + round_up((long long)nranks * kLLFifoCta * kFlagStride, 4096);
@@ -284,8 +284,11 @@ int piccl_comm_nranks(piccl_comm_t* c) { return c ? c->nranks : -1; }
 // ------------------------------------------------------------------ program cache
 namespace piccl {
 
-static int upload_program(piccl_comm* c, const Program& p, cudaStream_t stream, ProgEntry& e) {
-  size_t bytes = std::max<size_t>(p.actions.size(), 1) * sizeof(Action);
+struct CallDesc { Coll coll; const void* send; void* recv; size_t count; int dtype, op, root; Algo algo; int k; };
+
+static int upload_program(piccl_comm* c, const Program& p, cudaStream_t stream, ProgEntry& e, const std::vector<SharedOps>* shared = nullptr) {
+  const size_t act_bytes = p.actions.size() * sizeof(Action), sh_bytes = shared ? shared->size() * sizeof(SharedOps) : 0;
+  size_t bytes = std::max<size_t>(act_bytes + sh_bytes, sizeof(Action));
   bytes = (bytes + 255) / 256 * 256;
   if (c->chunks.empty() || c->chunks.back().used + bytes > c->chunks.back().cap) {
     ProgChunk ch; ch.cap = std::max<size_t>(1 << 20, bytes); ch.used = 0;
@@ -295,10 +298,12 @@ static int upload_program(piccl_comm* c, const Program& p, cudaStream_t stream, 
     c->chunks.push_back(ch);
   }
   ProgChunk& ch = c->chunks.back();
-  memcpy(ch.host + ch.used, p.actions.data(), p.actions.size() * sizeof(Action));
+  memcpy(ch.host + ch.used, p.actions.data(), act_bytes);
+  if (sh_bytes) memcpy(ch.host + ch.used + act_bytes, shared->data(), sh_bytes);
   e.dev = reinterpret_cast<const Action*>(ch.dev + ch.used);
-  e.n_actions = (int)p.actions.size(); e.scratch_elems = p.scratch_elems; e.origin = stream; e.synced = false;
-  if (!p.actions.empty()) CUDA_TRY(cudaMemcpyAsync(ch.dev + ch.used, ch.host + ch.used, p.actions.size() * sizeof(Action), cudaMemcpyHostToDevice, stream));
+  if (sh_bytes) e.dev_shared = reinterpret_cast<const SharedOps*>(ch.dev + ch.used + act_bytes);
+  e.n_actions = (int)p.actions.size(); for (const Action& ac : p.actions) e.most = std::max<long long>(e.most, ac.count); e.scratch_elems = p.scratch_elems; e.origin = stream; e.synced = false;
+  if (!p.actions.empty()) CUDA_TRY(cudaMemcpyAsync(ch.dev + ch.used, ch.host + ch.used, act_bytes + sh_bytes, cudaMemcpyHostToDevice, stream));
   CUDA_TRY(cudaEventCreateWithFlags(&e.ready, cudaEventDisableTiming));
   CUDA_TRY(cudaEventRecord(e.ready, stream));
   ch.used += bytes;
@@ -325,8 +330,14 @@ static const char* check_program(const Program& p, const CollArgs& a, long long 
   return nullptr;
 }
 
-static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, const ProgEntry** out) {
-  ProgKey k{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, a.block_stride};
+// The programs of all ranks of a launch that read each other's buffers, compiled when the first of them is not in its cache.
+struct GroupPrograms { bool made = false; std::vector<Program> progs; std::vector<std::vector<SharedOps>> shared; };
+
+static ProgKey key_of(const CollArgs& a, bool shared) { return ProgKey{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, a.block_stride, shared ? 1 : 0}; }
+
+// group: the program as share_operands makes it; the other one is kept beside it, for a captured call whose buffers overlap.
+static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, const ProgEntry** out, GroupPrograms* group = nullptr) {
+  const ProgKey k = key_of(a, group != nullptr);
   auto it = c->cache.find(k);
   if (it == c->cache.end()) {
     // A new program needs device and pinned memory and an upload on the caller's stream: not inside a stream capture (an
@@ -345,33 +356,74 @@ static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, co
       c->stats.fallbacks++;
       return fail(PICCL_UNSUPPORTED, "program cache full (%zu MiB for %zu distinct calls)", held >> 20, c->cache.size());
     }
-    c->stats.program_cache_misses++;
-    Program p = compile(a, c->rank);
-    if (env().debug) {
+    if (group) {
+      const ProgEntry* plain = nullptr;
+      if (int rc = get_program(c, a, stream, &plain)) return rc;
+      if (!group->made) {
+        group->made = true;
+        for (int r = 0; r < a.nranks; r++) group->progs.push_back(compile(a, r));
+        if (!share_operands(group->progs, group->shared)) group->shared.clear();
+      }
+    } else c->stats.program_cache_misses++;
+    Program p = group ? std::move(group->progs[c->rank]) : compile(a, c->rank);
+    if (env().debug && !group) {
       if (const char* why = check_program(p, a, c->h_ctx.scratch_bytes / std::max(1, a.elem_size)))
         return fail(PICCL_INTERNAL_ERROR, "program check failed (%s %s, rank %d): %s", coll_name(a.coll), algo_name(a.algo), c->rank, why);
     }
     ProgEntry e;
     for (const Action& ac : p.actions) e.offsets_aligned &= (ac.src_off * a.elem_size) % 16 == 0 && (ac.dst_off * a.elem_size) % 16 == 0;
-    int rc = upload_program(c, p, stream, e); if (rc) return rc;
+    const std::vector<SharedOps>* sh = group && !group->shared.empty() ? &group->shared[c->rank] : nullptr;
+    if (sh) for (size_t i = 0; i < sh->size(); i++) for (int j = 0; j < p.actions[i].n_recv; j++) e.offsets_aligned &= (*sh)[i].off[j] * a.elem_size % 16 == 0;
+    int rc = upload_program(c, p, stream, e, sh); if (rc) return rc;
     it = c->cache.emplace(k, e).first;
   } else {
     c->stats.program_cache_hits++;
     ProgEntry& e = it->second;
     if (!e.synced) {
-      if (e.origin != stream) CUDA_TRY(cudaStreamWaitEvent(stream, e.ready, 0));
+      // Asked first, and in the relaxed mode: a stream in capture cannot wait for an upload outside it, and a question in the global mode would end the capture.
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
       if (cudaEventQuery(e.ready) == cudaSuccess) e.synced = true; else cudaGetLastError();
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (!e.synced && e.origin != stream) CUDA_TRY(cudaStreamWaitEvent(stream, e.ready, 0));
     }
   }
   *out = &it->second;
   return PICCL_OK;
 }
 
+// May the ranks of this launch read each other's buffers (share.cc)?  All of them in one launch on one GPU; no receive buffer may overlap another rank's buffers, or,
+// but for an all-gather or broadcast in place, which never write what others read, its own send buffer: a rank could overwrite what another is still to read.
+static bool may_share(piccl_comm** comms, int n, const CallDesc* calls, long long bytes) {
+  const CallDesc& d0 = calls[0];
+  if (n != comms[0]->nranks || n < 2) return false;
+  struct Span { const char *lo, *hi; } in[kMaxVRanks], out[kMaxVRanks];
+  auto meet = [](const Span& a, const Span& b) { return a.lo < b.hi && b.lo < a.hi; };
+  const long long blocks_in = d0.coll == COLL_REDUCE_SCATTER ? n : 1, blocks_out = d0.coll == COLL_ALLGATHER ? n : 1;
+  const bool moves = d0.coll == COLL_ALLGATHER || d0.coll == COLL_BROADCAST;
+  int in_place = 0;
+  for (int i = 0; i < n; i++) {
+    if (comms[i]->rank != i || comms[i]->slots_only) return false;
+    const char *s = (const char*)calls[i].send, *r = (const char*)calls[i].recv;
+    const bool reads = d0.coll != COLL_BROADCAST || i == d0.root, writes = d0.coll != COLL_REDUCE || i == d0.root;
+    in[i] = {s, s + (reads ? blocks_in * bytes : 0)}; out[i] = {r, r + (writes ? blocks_out * bytes : 0)};
+    in_place += moves && s == r + (d0.coll == COLL_ALLGATHER ? i * bytes : 0);
+  }
+  if (in_place != 0 && in_place != n) return false;
+  for (int i = 0; i < n; i++)
+    for (int j = 0; j < n; j++) {
+      if (i < j && meet(out[i], out[j])) return false;
+      if (meet(out[i], in[j]) && !(i == j && in_place)) return false;
+    }
+  return true;
+}
+
 // CTAs for one collective: enough to fill NVLink for large messages, one for tiny ones.
 // All ranks compute the same number from the same arguments.  The reference's grid formula
 // grid = clamp(count / block, MIN, MAX) (src/kernels/permutation_kernel.cu:76-77) is kept when
 // PICCL_MIN/MAX_GRID_SIZE are set; the result is capped by the FIFO channel count.
-static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
+// n_working of the n_vrank ranks of the launch have CTAs.
+static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_working, int n_vrank) {
   long long bytes = a.count * a.elem_size;
   if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) bytes /= std::max(1, a.nranks);
   if (a.algo == ALGO_DIRECT && a.coll != COLL_ALLGATHER && a.coll != COLL_REDUCE_SCATTER) bytes /= std::max(1, a.coll == COLL_ALLREDUCE ? a.nranks : a.nranks - 1);
@@ -385,7 +437,7 @@ static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
     n = std::max<long long>(e.min_grid_set ? e.min_grid : 1, std::min<long long>(e.max_grid_set ? e.max_grid : g, g));
   }
   n = std::max<long long>(1, std::min<long long>(n, c->cfg.max_cta));
-  if (n_vrank > 1) n = std::min<long long>(n, std::max(1, c->sm_count / n_vrank));
+  if (n_vrank > 1) n = std::min<long long>(n, std::max(1, c->sm_count / n_working));
   return (int)n;
 }
 
@@ -485,8 +537,6 @@ static bool ll_plan(piccl_comm** comms, int n, Algo algo, int k, LLArgs* out) {
   if (p.usable) *out = p.args;
   return p.usable;
 }
-
-struct CallDesc { Coll coll; const void* send; void* recv; size_t count; int dtype, op, root; Algo algo; int k; };
 
 // Runs one collective over `n` communicators of this process (n == 1: the normal case).
 static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t stream) {
@@ -648,15 +698,19 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     }
   }
 
+  bool share = !use_llf && may_share(comms, n, calls, (long long)d0.count * esz_real);
   nvtxRangePushA(coll_name(d0.coll));
   int rc = PICCL_OK;
   for (long long done = 0; done < count && rc == PICCL_OK; done += slab) {
     long long cur = std::min(slab, count - done);
     KernelArgs ka; memset(&ka, 0, sizeof ka);
-    ka.n_vrank = n; ka.elem_size = esz; ka.avg = avg ? 1 : 0; ka.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
+    ka.n_vrank = n; ka.elem_size = esz; ka.one_gpu = n == c0->nranks; ka.avg = avg ? 1 : 0; ka.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
     int n_cta = 0;
     bool aligned = true;
-    CollArgs priorities_of;
+    CollArgs first;
+    GroupPrograms group;
+    long long most = 0;
+    bool any_shared = false;
     for (int i = 0; i < n && rc == PICCL_OK; i++) {
       piccl_comm* c = comms[i]; const CallDesc& d = calls[i];
       std::lock_guard<std::mutex> l(c->mu);
@@ -669,28 +723,35 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       }
       if (d.coll == COLL_REDUCE && c->rank != d.root) a.in_place = false;
       const ProgEntry* pe = nullptr;
-      rc = get_program(c, a, stream, &pe); if (rc) break;
-      if (i == 0) {
-        n_cta = choose_cta(c, a, n);
-        if (use_llf) {   // a line (8 bytes) per thread and action while there are CTAs, then several; a segment holds 4 KiB
-          long long ab = a.count * a.elem_size;
-          if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) ab /= std::max(1, a.nranks);
-          if (a.algo == ALGO_DIRECT && a.coll != COLL_ALLGATHER && a.coll != COLL_REDUCE_SCATTER) ab /= std::max(1, a.coll == COLL_ALLREDUCE ? a.nranks : a.nranks - 1);
-          n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
-          if (n > 1) n_cta = std::min(n_cta, std::max(1, c->sm_count / n));
-        }
-        ka.n_cta = n_cta; if (!use_llf) cut_fifo(c, n, n_cta, a, &ka);
-        priorities_of = a;
-        ka.one_gpu = n == c->nranks;
-        ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
-      }
+      if (i == 0 && share && cap_state != cudaStreamCaptureStatusNone) share = c->cache.count(key_of(a, true)) != 0;      // (a capture replays what was built before it)
+      rc = get_program(c, a, stream, &pe, share ? &group : nullptr); if (rc) break;
+      if (i == 0) first = a;
       ka.one_gpu &= c->device == c0->device;
-      ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
+      ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].shared = pe->dev_shared; any_shared |= pe->dev_shared != nullptr; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
+      ka.prog_actions = std::max(ka.prog_actions, pe->n_actions); most = std::max(most, pe->most);
       aligned &= pe->offsets_aligned && ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(r)) & 15) == 0;
       c->stats.launches++;
     }
     if (rc) break;
-    ka.leave_first = leave_first(priorities_of, n, ka.one_gpu);
+    // Ranks with nothing to do, whose operands others read (the leaves of a tree), leave their SMs to those that have.
+    int n_working = 0;
+    for (int i = 0; i < n; i++) if (ka.r[i].n_actions > 0 || !any_shared) ka.working[n_working++] = (uint8_t)i;
+    if (n_working == 0) ka.working[n_working++] = 0;
+    n_cta = choose_cta(c0, first, n_working, n);
+    if (use_llf) {   // a line (8 bytes) per thread and action while there are CTAs, then several; a segment holds 4 KiB
+      long long ab = first.count * first.elem_size;
+      if (first.coll == COLL_ALLREDUCE && (first.algo == ALGO_RING || first.algo == ALGO_K_RING)) ab /= std::max(1, first.nranks);
+      if (first.algo == ALGO_DIRECT && first.coll != COLL_ALLGATHER && first.coll != COLL_REDUCE_SCATTER) ab /= std::max(1, first.coll == COLL_ALLREDUCE ? first.nranks : first.nranks - 1);
+      n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
+      if (n > 1) n_cta = std::min(n_cta, std::max(1, c0->sm_count / n));
+    }
+    ka.n_cta = n_cta; if (!use_llf) cut_fifo(c0, n, n_cta, first, &ka);
+    ka.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
+    if (any_shared) {          // the widest slice is CTA 0's
+      const long long segs = slice_of(most, esz, 0, n_cta, ka.seg_bytes).nseg;
+      ka.prog_total = round_up(segs, ka.window) * ka.prog_actions + 1;
+    }
+    ka.leave_first = leave_first(first, n, ka.one_gpu);
     bool skip = false;
     for (int i = 0; i < n; i++) skip |= fault_now(comms[i]);
     for (int i = 0; i < n; i++) comms[i]->call_index++;
@@ -701,7 +762,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     const int block = use_llf ? kLLBlock : exec_block(c0);
     // which kernel a rank runs is its own business: both speak the same protocol
     const ExecKernelFn f = (aligned || use_llf) ? fn : reducing ? exec_shift_kernel_for(d0.dtype, op) : exec_shift_copy_kernel();
-    if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n * n_cta), dim3(block), args, 0, stream);
+    if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n_working * n_cta), dim3(block), args, 0, stream);
     else e = cudaLaunchKernel((const void*)f, dim3(n_cta), dim3(block), args, 0, stream);
     if (e != cudaSuccess) rc = fail(PICCL_CUDA_ERROR, "executor launch failed: %s", cudaGetErrorString(e));
     trace_end(c0, tr, stream);
@@ -752,6 +813,12 @@ int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const voi
 int piccl_test_leave_first(int coll, int nranks, int in_launch, int one_device, long long bytes) {
   CollArgs a; a.coll = (Coll)coll; a.nranks = nranks; a.count = bytes; a.elem_size = 1;
   return leave_first(a, in_launch, one_device && in_launch == nranks);
+}
+// on != 0: ranks of one launch do not read each other's buffers, everything that crosses goes through the slots as it does between GPUs.
+int piccl_test_slots_only(piccl_comm_t* c, int on) {
+  if (!c) return fail(PICCL_INVALID_ARGUMENT, "null communicator");
+  c->slots_only = on != 0;
+  return PICCL_OK;
 }
 int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream) {
   if (!c || !c->connected) return fail(PICCL_INVALID_USAGE, "communicator is not connected");

@@ -459,3 +459,44 @@ def test_averaged_rounds_of_the_default_geometry(n, algo, k, dtype):
         _check_ok(g)
         assert all(torch.equal(x, o) for x, o in zip(xs, outs))
     g.close()
+
+
+@pytest.mark.parametrize("dtype,offset", [(torch.float32, 0), (torch.bfloat16, 0), (torch.bfloat16, 1)])
+@pytest.mark.parametrize("coll", ["allreduce", "allgather", "reduce_scatter", "broadcast", "reduce"])
+def test_reading_each_others_buffers_changes_nothing(coll, dtype, offset):
+    """Every algorithm on three and eight ranks, with the ranks reading each other's buffers and with everything through the slots, in turn on one communicator, from a captured graph too,
+    and with a receive buffer that is another rank's send buffer (slots, whatever was asked for).  Operands and hops are rounded alike: bit for bit the same."""
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    for n in (3, 8):
+        g = LoopbackGroup(n, config=make_config(scratch_bytes=1 << 20, timeout_ms=5000))
+        count = 40013 if coll in ("allgather", "reduce_scatter") else 180013 * n      # (above the sizes that other kernels take outside a capture)
+        n_in, n_out = count * (n if coll == "reduce_scatter" else 1), count * (n if coll == "allgather" else 1)
+        xs = [x[offset:] for x in _inputs(n, n_in + offset, dtype, seed=3)]
+        op = "sum" if coll in ("allgather", "broadcast") else "avg"
+        for algo in ALGOS:
+            outs = [[torch.full((n_out + offset,), 7.0, device="cuda", dtype=dtype)[offset:] for _ in range(n)] for _ in range(3)]
+            for variant, slots in enumerate((1, 0)):
+                for h in g._hs:
+                    g._lib.piccl_test_slots_only(h, slots)
+                for _ in range(2):
+                    g.run(coll, xs, outs[variant], count, op=op, root=1, algo=algo, k=4)
+            _check_ok(g)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                g.run(coll, xs, outs[2], count, op=op, root=1, algo=algo, k=4)
+            for _ in range(2):
+                graph.replay()
+            _check_ok(g)
+            for r in range(n):
+                assert torch.equal(outs[0][r], outs[1][r]) and torch.equal(outs[0][r], outs[2][r]), (coll, algo, n, r)
+            if n_in == n_out and coll != "broadcast":       # rank 0 receives into rank 1's send buffer (the ring's sums contain what they overwrite)
+                ys = [x.clone() for x in xs]
+                zs = [ys[1]] + [torch.full_like(x, 7.0) for x in xs[1:]]
+                if coll == "reduce":
+                    zs[1], zs[0] = ys[2], zs[1]
+                g.run(coll, ys, zs, count, op=op, root=1, algo="RING")
+                _check_ok(g)
+                g.run(coll, xs, outs[0], count, op=op, root=1, algo="RING")
+                _check_ok(g)
+                assert torch.equal(zs[1], outs[0][1])
+        g.close()

@@ -200,3 +200,27 @@ def test_results_that_the_cache_can_keep_stay_there():
                                  ("allreduce", 8, 12, 1), ("reduce", 4, 32, 1), ("allgather", 4, 8, 3), ("reduce_scatter", 2, 64, 3), ("broadcast", 8, 32, 3), ("allreduce", 4, 25, 3),
                                  ("allreduce", 8, 64, 3), ("reduce", 2, 128, 3), ("allreduce", 8, 8, 0), ("allgather", 8, 1, 0), ("reduce_scatter", 2, 8, 0), ("broadcast", 8, 8, 0)]:
         assert f(N.COLL[coll], n, n, 1, block * MiB) == want, (coll, n, block)
+
+
+@pytest.mark.parametrize("coll", COLLS)
+@pytest.mark.parametrize("algo", ALGOS)
+def test_programs_that_read_each_others_buffers(coll, algo):
+    """All ranks in one launch: values that are only handed on are read at their origin (share.cc).  Same data, no deadlock, also with progress and counters
+    published as late as can be; in place, and with block strides wider than a block."""
+    for n, k, in_place in itertools.product(range(2, 9), [-1, 2, 3, 4, 8], [False, True]):
+        for fifo, count, deferred in itertools.product([2, 4], [5, 30, 32 * 2 * 3 * n, 257], [False, True]):
+            v = S.validate(coll, algo, n, count, k=k, root=n - 1, in_place=in_place, n_cta=2, seg_elems=32, fifo_cap=fifo, deferred=deferred, shared=True)
+            assert v.ok, f"{coll} {algo} n={n} k={k} in_place={in_place} fifo={fifo} count={count} deferred={deferred}: {v.error}"
+        if coll in ("allgather", "reduce_scatter"):
+            assert S.validate(coll, algo, n, 100, k=k, stride=130, n_cta=2, seg_elems=32, shared=True).ok
+
+
+def test_what_is_handed_on_takes_no_slot():
+    """Entries that are left: none where data only moves, the n - 1 hops of each share's partial sums on the ring, one exchange of sums among four ranks doubling."""
+    def entries(coll, algo, n, **kw):
+        return S.validate(coll, algo, n, 1024, n_cta=1, seg_elems=1024, shared=True, **kw).fifo_entries
+    assert all(entries(c, a, 8, k=2) == 0 for c in ("allgather", "broadcast") for a in ALGOS)
+    assert entries("allreduce", "RING", 8) == 8 * 6 and entries("allreduce", "PRD", 4) == 4 and entries("allreduce", "DIRECT", 8) == 0
+    assert entries("reduce_scatter", "RING", 2) == 0
+    in_place = S.validate("allreduce", "RING", 8, 1024, n_cta=1, seg_elems=1024, in_place=True, shared=True).fifo_entries
+    assert in_place == S.validate("allreduce", "RING", 8, 1024, n_cta=1, seg_elems=1024, in_place=True).fifo_entries
