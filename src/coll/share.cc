@@ -173,4 +173,14 @@ bool share_operands(std::vector<Program>& progs, std::vector<std::vector<SharedO
   return true;
 }
 
+bool nothing_waits(const std::vector<Program>& progs, const std::vector<std::vector<SharedOps>>& shared) {
+  for (size_t r = 0; r < progs.size(); r++)
+    for (size_t i = 0; i < progs[r].actions.size(); i++) {
+      const Action& a = progs[r].actions[i];
+      if (a.dst_buf != BUF_OUT || a.n_send || (a.src_buf != BUF_NONE && a.src_buf != BUF_IN)) return false;
+      for (int j = 0; j < a.n_recv; j++) if (a.recv_peer[j] != kSharedPeer || shared[r][i].after[j] >= 0 || shared[r][i].buf[j] == BUF_SCRATCH) return false;
+    }
+  return true;
+}
+
 }  // namespace piccl

@@ -117,6 +117,8 @@ Program compile(const CollArgs& a, int rank);
 // of rank r.  The caller vouches that no rank's receive buffer overlaps another rank's buffers or its own send buffer (in place: all-gather and broadcast only).
 // false: the programs are as they were.
 bool share_operands(std::vector<Program>& progs, std::vector<std::vector<SharedOps>>& shared);
+// Does no action of these programs wait for another, of any rank?
+bool nothing_waits(const std::vector<Program>& progs, const std::vector<std::vector<SharedOps>>& shared);
 
 // Chunking used by allreduce: chunk c covers [displ(c), displ(c)+cnt(c)); chunk
 // starts are multiples of 16 bytes; tail chunks may be short or empty.

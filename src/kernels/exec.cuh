@@ -23,6 +23,7 @@ namespace piccl {
 constexpr int kFlagStride = 128;          // bytes between two counters
 constexpr int kMaxVRanks = 8;             // virtual ranks one launch can carry (single-GPU emulation)
 constexpr int kMaxBlock = 512;             // threads of an executor CTA that move data
+constexpr int kFlatBlock = 256;            // threads of a block of a call in which nothing waits
 constexpr int kCtlThreads = 64;            // and two warps more: waiter and publisher
 constexpr int kLLFifoCta = 16, kLLFifoSlots = 8, kLLFifoSlotBytes = 8192;   // low-latency FIFO: CTAs, ring depth, bytes per slot (half of it payload)
 
@@ -119,6 +120,8 @@ ExecKernelFn exec_kernel_for(int dtype, int op);
 ExecKernelFn exec_copy_kernel();
 ExecKernelFn exec_shift_kernel_for(int dtype, int op);   // operands that are not 16-byte aligned
 ExecKernelFn exec_shift_copy_kernel();
+ExecKernelFn exec_flat_kernel_for(int dtype, int op, bool shift);   // calls in which nothing waits (exec_flat.cuh)
+ExecKernelFn exec_flat_copy_kernel(bool shift);
 ExecKernelFn exec_ll_kernel_for(int dtype, int op);   // low-latency variant (exec_ll.cuh)
 ExecKernelFn exec_ll_copy_kernel();
 

@@ -163,11 +163,10 @@ static __device__ __noinline__ bool wait_counter(const unsigned long long* flag,
 }
 
 // ---------------------------------------------------------------- data movement
-__device__ __forceinline__ int data_threads() { return (int)blockDim.x - kCtlThreads; }
-
+// (nt: the block's threads, from thread 0, that move data)
 // value = reduce(src[0..nsrc)) -> dst[0..ndst), everything 16-byte aligned; `scaled`: see scale_operand.
 // The operands' packs stay as they were loaded until they are combined, so a thread has NSRC * U loads of 16 bytes in flight and no array of
-// accumulators; offsets are 32-bit (a segment is at most a slot).  Whatever U is, pack p is thread p % (data threads)'s, so a step may read what an earlier one
+// accumulators; offsets are 32-bit (a segment is at most a slot).  Whatever U is, pack p is thread p % nt's, so a step may read what an earlier one
 // wrote.  The last round is as wide as the others instead of being finished a pack at a time, which took up to U - 1 further round trips: what lies
 // beyond the end loads the last pack again (loads under a condition made the compiler spill).  The slots' packs may
 // have been written by another GPU and the local operand is read once: all loads go past L1.
@@ -202,9 +201,9 @@ __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, i
 // (Only the aligned loops take these: at odd addresses, with more than two operands, or with destinations read from the table (NDST 0), lines keep the normal priority.)
 struct L2Hints { bool src_done, dst_done; int local_src, local_dst; };
 template <typename T, int OP, int NSRC, int NDST, int U, bool EXACT, bool SCALE = false>      // EXACT: nsrc == NSRC, else the first operand stands in for what is missing; NDST 0: any number, read from the table each time
-__device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
+__device__ __forceinline__ void stream(int nt, const char* const* src, int nsrc_rt, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
   constexpr bool HINT_SRC = NSRC <= 2;                   // (more sources leave no registers for their policies)
-  const int nsrc = EXACT ? NSRC : nsrc_rt, nt = data_threads(), tid = threadIdx.x;
+  const int nsrc = EXACT ? NSRC : nsrc_rt, tid = threadIdx.x;
   const char* sp[NSRC]; char* dp[NDST ? NDST : 1];
 #pragma unroll
   for (int s = 0; s < NSRC; s++) sp[s] = src[EXACT || s < nsrc ? s : 0];
@@ -243,32 +242,32 @@ __device__ __forceinline__ void stream(const char* const* src, int nsrc_rt, char
   }
 }
 template <typename T, int OP>
-__device__ __forceinline__ void move_aligned(const char* const* src, int nsrc, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
+__device__ __forceinline__ void move_aligned(int nt, const char* const* src, int nsrc, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
   if (OP == OP_COPY || (nsrc == 1 && !scaled)) {
-    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(src, 1, dst, 1, n, 0, scale, h);
-    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(src, 1, dst, 2, n, 0, scale, h);
-    else stream<T, OP, 1, 0, 4, true>(src, 1, dst, ndst, n, 0, scale, h);
+    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(nt, src, 1, dst, 1, n, 0, scale, h);
+    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(nt, src, 1, dst, 2, n, 0, scale, h);
+    else stream<T, OP, 1, 0, 4, true>(nt, src, 1, dst, ndst, n, 0, scale, h);
   } else if constexpr (OP != OP_COPY) {
     // Scaled operands (avg, which is a sum) have loops of their own too: in the general one a lone operand was loaded twice and the destinations read
     // from the table for each pack (25 MiB of bf16 averaged among four ranks: 155 us, now 136).
     if (scaled) {
       if constexpr (OP == 0) {
         if (nsrc == 1) {
-          if (ndst == 1) stream<T, OP, 1, 1, 8, true, true>(src, 1, dst, 1, n, 1, scale, h);
-          else stream<T, OP, 1, 0, 4, true, true>(src, 1, dst, ndst, n, 1, scale, h);
+          if (ndst == 1) stream<T, OP, 1, 1, 8, true, true>(nt, src, 1, dst, 1, n, 1, scale, h);
+          else stream<T, OP, 1, 0, 4, true, true>(nt, src, 1, dst, ndst, n, 1, scale, h);
         }
-        else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true, true>(src, 2, dst, 1, n, scaled, scale, h);
-        else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true, true>(src, 2, dst, 2, n, scaled, scale, h);
-        else if (nsrc <= 4) stream<T, OP, 4, 0, 2, false, true>(src, nsrc, dst, ndst, n, scaled, scale, h);
-        else stream<T, OP, kMaxActionPeers + 1, 0, 1, false, true>(src, nsrc, dst, ndst, n, scaled, scale, h);
+        else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true, true>(nt, src, 2, dst, 1, n, scaled, scale, h);
+        else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true, true>(nt, src, 2, dst, 2, n, scaled, scale, h);
+        else if (nsrc <= 4) stream<T, OP, 4, 0, 2, false, true>(nt, src, nsrc, dst, ndst, n, scaled, scale, h);
+        else stream<T, OP, kMaxActionPeers + 1, 0, 1, false, true>(nt, src, nsrc, dst, ndst, n, scaled, scale, h);
       }
     }
-    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(src, 2, dst, 1, n, 0, scale, h);
-    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(src, 2, dst, 2, n, 0, scale, h);
-    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(src, 4, dst, ndst, n, 0, scale, h);
-    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(src, nsrc, dst, ndst, n, 0, scale, h);
-    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(src, nsrc, dst, ndst, n, 0, scale, h);
-    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(src, nsrc, dst, ndst, n, 0, scale, h);
+    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(nt, src, 2, dst, 1, n, 0, scale, h);
+    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(nt, src, 2, dst, 2, n, 0, scale, h);
+    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(nt, src, 4, dst, ndst, n, 0, scale, h);
+    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
+    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
+    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
   }
 }
 
@@ -353,8 +352,8 @@ __device__ __forceinline__ void store_run(const uint4 (&o)[RUN], int ndst, char*
   }
 }
 template <typename T, int OP, int RUN>
-__device__ __noinline__ void copy_shift(const char* src, int ndst, char* const* dst, int local_dst, long long npack) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = data_threads() >> 5;
+__device__ __noinline__ void copy_shift(int nt, const char* src, int ndst, char* const* dst, int local_dst, long long npack) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = nt >> 5;
   char* one[1] = {dst[0]};
   int dm = local_dst >= 0 ? address_mod(dst[local_dst]) : 0;
   if (ndst == 1 && dm) {                               // (a shift for the source and one for the destination: all-gather of 4 x 1 MiB 20.5 us)  One destination: its whole words, for which one shift will do, and the bytes at both ends
@@ -376,10 +375,10 @@ __device__ __noinline__ void copy_shift(const char* src, int ndst, char* const* 
   }
 }
 template <typename T, int OP, int RUN>
-__device__ __noinline__ void reduce_shift(int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
+__device__ __noinline__ void reduce_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
   typedef typename AccOf<T>::type A;
   constexpr int N = Pack<T>::N;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = data_threads() >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = nt >> 5;
   const int dm = local_dst >= 0 ? address_mod(dst[local_dst]) : 0;
   for (long long run = (long long)warp * (32 * RUN); run < npack; run += (long long)nwarp * (32 * RUN)) {
     A acc[RUN][N];
@@ -425,24 +424,24 @@ __device__ __noinline__ void reduce_shift(int nsrc, const char* const* src, int 
 }
 // A warp takes runs of 2, 4 or 8 blocks (sums: 2 or 4): as few rounds as can be, and then over as many warps.
 template <typename T, int OP>
-__device__ __forceinline__ void reduce_copy_shift(int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
-  const long long blocks = (npack + data_threads() - 1) / data_threads();      // per warp
+__device__ __forceinline__ void reduce_copy_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
+  const long long blocks = (npack + nt - 1) / nt;      // per warp
   if (OP == OP_COPY || (nsrc == 1 && !scaled)) {
-    if (blocks > 4) copy_shift<T, OP, 8>(src[0], ndst, dst, local_dst, npack);
-    else if (blocks > 2) copy_shift<T, OP, 4>(src[0], ndst, dst, local_dst, npack);
-    else copy_shift<T, OP, 2>(src[0], ndst, dst, local_dst, npack);
+    if (blocks > 4) copy_shift<T, OP, 8>(nt, src[0], ndst, dst, local_dst, npack);
+    else if (blocks > 2) copy_shift<T, OP, 4>(nt, src[0], ndst, dst, local_dst, npack);
+    else copy_shift<T, OP, 2>(nt, src[0], ndst, dst, local_dst, npack);
   } else if constexpr (OP != OP_COPY) {
-    if (blocks > 2) reduce_shift<T, OP, 4>(nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
-    else reduce_shift<T, OP, 2>(nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
+    if (blocks > 2) reduce_shift<T, OP, 4>(nt, nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
+    else reduce_shift<T, OP, 2>(nt, nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
   }
 }
 
 // Element-wise path: the last, partial pack of an action.
 template <typename T, int OP>
-__device__ __noinline__ void reduce_copy_elem(int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
+__device__ __noinline__ void reduce_copy_elem(int nt, int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
                                                  long long first, long long nelem, int scaled, float scale) {
   typedef typename AccOf<T>::type A;
-  for (long long i = first + threadIdx.x; i < nelem; i += data_threads()) {
+  for (long long i = first + threadIdx.x; i < nelem; i += nt) {
     A acc = A();
     for (int s = 0; s < nsrc; s++) {
       const T* p = reinterpret_cast<const T*>(src[s]) + i;
@@ -480,7 +479,7 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   const int launched = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta, vr = ka.working[launched];
   const LaunchRank& L = ka.r[vr];
   RankCtx* __restrict__ ctx = L.ctx;
-  const int tid = threadIdx.x, lane = tid & 31, ndata = data_threads();
+  const int tid = threadIdx.x, lane = tid & 31, ndata = (int)blockDim.x - kCtlThreads;
   constexpr int esz = (int)sizeof(T);
 
   __shared__ StepDesc s_step[kStepDepth];
@@ -533,9 +532,9 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
         const int scaled = st.scaled;
         constexpr int N = Pack<T>::N;
         const long long nfull = (SHIFT || (flags & STEP_ALIGNED)) ? len / N : 0;
-        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(nsrc, src, ndst, dst, st.local_dst, nfull, scaled, ka.scale); }
-        else if (nfull) move_aligned<T, OP>(src, nsrc, dst, ndst, (int)nfull, scaled, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
-        if (nfull * N < len) reduce_copy_elem<T, OP>(nsrc, src, local_src, ndst, dst, nfull * N, len, scaled, ka.scale);
+        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(ndata, nsrc, src, ndst, dst, st.local_dst, nfull, scaled, ka.scale); }
+        else if (nfull) move_aligned<T, OP>(ndata, src, nsrc, dst, ndst, (int)nfull, scaled, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
+        if (nfull * N < len) reduce_copy_elem<T, OP>(ndata, nsrc, src, local_src, ndst, dst, nfull * N, len, scaled, ka.scale);
       }
       bar_arrive_n(kDone + d, ndata + 32);
       if (flags & (STEP_END | STEP_FAIL)) return;

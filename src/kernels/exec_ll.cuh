@@ -9,6 +9,7 @@
 // and the region is zero at start, so stale lines can never look complete.
 #pragma once
 #include "exec_impl.cuh"
+#include "exec_flat.cuh"
 
 namespace piccl {
 
@@ -167,5 +168,7 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
   namespace piccl {                                                                                \
   ExecKernelFn exec_table_##DT[4] = {exec_kernel<T, 0, false>, exec_kernel<T, 1, false>, exec_kernel<T, 2, false>, exec_kernel<T, 3, false>}; \
   ExecKernelFn exec_shift_table_##DT[4] = {exec_kernel<T, 0, true>, exec_kernel<T, 1, true>, exec_kernel<T, 2, true>, exec_kernel<T, 3, true>}; \
+  ExecKernelFn exec_flat_table_##DT[8] = {exec_flat_kernel<T, 0, false>, exec_flat_kernel<T, 1, false>, exec_flat_kernel<T, 2, false>, exec_flat_kernel<T, 3, false>,              \
+                                          exec_flat_kernel<T, 0, true>, exec_flat_kernel<T, 1, true>, exec_flat_kernel<T, 2, true>, exec_flat_kernel<T, 3, true>};               \
   ExecKernelFn exec_ll_table_##DT[4] = {exec_ll_kernel<T, 0>, exec_ll_kernel<T, 1>, exec_ll_kernel<T, 2>, exec_ll_kernel<T, 3>}; \
   }

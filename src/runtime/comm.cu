@@ -331,7 +331,7 @@ static const char* check_program(const Program& p, const CollArgs& a, long long 
 }
 
 // The programs of all ranks of a launch that read each other's buffers, compiled when the first of them is not in its cache.
-struct GroupPrograms { bool made = false; std::vector<Program> progs; std::vector<std::vector<SharedOps>> shared; };
+struct GroupPrograms { bool made = false, flat = false; std::vector<Program> progs; std::vector<std::vector<SharedOps>> shared; };
 
 static ProgKey key_of(const CollArgs& a, bool shared) { return ProgKey{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, a.block_stride, shared ? 1 : 0}; }
 
@@ -363,6 +363,7 @@ static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, co
         group->made = true;
         for (int r = 0; r < a.nranks; r++) group->progs.push_back(compile(a, r));
         if (!share_operands(group->progs, group->shared)) group->shared.clear();
+        else group->flat = nothing_waits(group->progs, group->shared);
       }
     } else c->stats.program_cache_misses++;
     Program p = group ? std::move(group->progs[c->rank]) : compile(a, c->rank);
@@ -372,6 +373,7 @@ static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, co
     }
     ProgEntry e;
     for (const Action& ac : p.actions) e.offsets_aligned &= (ac.src_off * a.elem_size) % 16 == 0 && (ac.dst_off * a.elem_size) % 16 == 0;
+    e.flat = group && group->flat;
     const std::vector<SharedOps>* sh = group && !group->shared.empty() ? &group->shared[c->rank] : nullptr;
     if (sh) for (size_t i = 0; i < sh->size(); i++) for (int j = 0; j < p.actions[i].n_recv; j++) e.offsets_aligned &= (*sh)[i].off[j] * a.elem_size % 16 == 0;
     int rc = upload_program(c, p, stream, e, sh); if (rc) return rc;
@@ -485,6 +487,23 @@ static void cut_fifo(const piccl_comm* c, int n_vrank, int n_cta, const CollArgs
   const long long seg = std::min<long long>(round_up((slice + 1) / 2, round), std::max<long long>(round, 131072 / round * round));
   ka->nslot = 4; ka->window = window_of(4);
   ka->seg_bytes = std::max<long long>(16, std::min<long long>(seg, chan / 4 / 16 * 16));
+}
+
+// Slices to an action where nothing waits: blocks of 4 KiB, one 16-byte pack a thread, while there are SMs for more of them, and no larger than 64 KiB, so that
+// the last wave is short.  us, executor (which reads at the origin too) and this: all-gather 4 x 1 MiB at odd addresses 18.4 / 10.4, 8 x 8 MiB 147 / 97.5, 4 x 16 MiB 81 / 55, 4 x 4 KiB 12.3 / 6.6;
+// broadcast 8 x 16 MiB 41 / 26.7; reduce-scatter 2 x 32 MiB 41 / 33; all-reduce in one exchange 4 x 32 MiB 83 / 52, 2 x 4 MB 11.3 / 6.1.
+static int flat_slices(const piccl_comm* c, long long bytes, long long actions, long long* slice_bytes) {
+  const long long even = (actions * bytes / (12LL * c->sm_count) + 4095) / 4096 * 4096;
+  *slice_bytes = std::max<long long>(4096, std::min<long long>(65536, even));
+  return (int)std::max<long long>(1, (bytes + *slice_bytes - 1) / *slice_bytes);
+}
+static cudaError_t launch_flat(ExecKernelFn f, long long blocks, void** args, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::max<long long>(1, blocks)); cfg.blockDim = dim3(kFlatBlock); cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, (const void*)f, args);
 }
 
 static bool fault_now(piccl_comm* c) {
@@ -698,7 +717,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     }
   }
 
-  bool share = !use_llf && may_share(comms, n, calls, (long long)d0.count * esz_real);
+  bool share = may_share(comms, n, calls, (long long)d0.count * esz_real);
   nvtxRangePushA(coll_name(d0.coll));
   int rc = PICCL_OK;
   for (long long done = 0; done < count && rc == PICCL_OK; done += slab) {
@@ -706,11 +725,12 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     KernelArgs ka; memset(&ka, 0, sizeof ka);
     ka.n_vrank = n; ka.elem_size = esz; ka.one_gpu = n == c0->nranks; ka.avg = avg ? 1 : 0; ka.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
     int n_cta = 0;
+    long long n_blocks = 0;
     bool aligned = true;
     CollArgs first;
     GroupPrograms group;
     long long most = 0;
-    bool any_shared = false;
+    bool any_shared = false, flat = false;
     for (int i = 0; i < n && rc == PICCL_OK; i++) {
       piccl_comm* c = comms[i]; const CallDesc& d = calls[i];
       std::lock_guard<std::mutex> l(c->mu);
@@ -725,6 +745,11 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       const ProgEntry* pe = nullptr;
       if (i == 0 && share && cap_state != cudaStreamCaptureStatusNone) share = c->cache.count(key_of(a, true)) != 0;      // (a capture replays what was built before it)
       rc = get_program(c, a, stream, &pe, share ? &group : nullptr); if (rc) break;
+      if (i == 0) flat = pe->flat;
+      if (use_llf && share && !flat) {                // (what waits for something does so in the lines of the low-latency variant)
+        share = false;
+        rc = get_program(c, a, stream, &pe); if (rc) break;
+      }
       if (i == 0) first = a;
       ka.one_gpu &= c->device == c0->device;
       ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].shared = pe->dev_shared; any_shared |= pe->dev_shared != nullptr; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
@@ -745,9 +770,10 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
       if (n > 1) n_cta = std::min(n_cta, std::max(1, c0->sm_count / n));
     }
-    ka.n_cta = n_cta; if (!use_llf) cut_fifo(c0, n, n_cta, first, &ka);
+    if (flat) { long long a = 0; for (int i = 0; i < n; i++) a += ka.r[i].n_actions; n_cta = flat_slices(c0, most * esz, a, &ka.seg_bytes); n_blocks = a * n_cta; }
+    ka.n_cta = n_cta; if (!use_llf && !flat) cut_fifo(c0, n, n_cta, first, &ka);
     ka.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
-    if (any_shared) {          // the widest slice is CTA 0's
+    if (any_shared && !flat) { // the widest slice is CTA 0's
       const long long segs = slice_of(most, esz, 0, n_cta, ka.seg_bytes).nseg;
       ka.prog_total = round_up(segs, ka.window) * ka.prog_actions + 1;
     }
@@ -762,7 +788,8 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     const int block = use_llf ? kLLBlock : exec_block(c0);
     // which kernel a rank runs is its own business: both speak the same protocol
     const ExecKernelFn f = (aligned || use_llf) ? fn : reducing ? exec_shift_kernel_for(d0.dtype, op) : exec_shift_copy_kernel();
-    if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n_working * n_cta), dim3(block), args, 0, stream);
+    if (flat) e = launch_flat(reducing ? exec_flat_kernel_for(d0.dtype, op, !aligned) : exec_flat_copy_kernel(!aligned), n_blocks, args, stream);
+    else if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n_working * n_cta), dim3(block), args, 0, stream);
     else e = cudaLaunchKernel((const void*)f, dim3(n_cta), dim3(block), args, 0, stream);
     if (e != cudaSuccess) rc = fail(PICCL_CUDA_ERROR, "executor launch failed: %s", cudaGetErrorString(e));
     trace_end(c0, tr, stream);

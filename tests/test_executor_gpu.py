@@ -500,3 +500,36 @@ def test_reading_each_others_buffers_changes_nothing(coll, dtype, offset):
                 _check_ok(g)
                 assert torch.equal(zs[1], outs[0][1])
         g.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.float64])
+@pytest.mark.parametrize("coll,n,algo,op", [("allgather", 3, "RING", "sum"), ("broadcast", 8, "PRD", "sum"), ("reduce", 2, "RING", "max"), ("reduce_scatter", 4, "DIRECT", "sum"), ("allreduce", 5, "PRM", "avg"),
+                                            ("allreduce", 8, "DIRECT", "min")])
+def test_calls_in_which_nothing_waits(coll, n, algo, op, dtype):
+    """Blocks of 4 KiB to 64 KiB: one element, a pack and its neighbours, a block and its neighbours, several blocks, a message whose blocks are larger; operands and results
+    3 elements into their buffers too.  Small whole numbers: exact but for fifths, whose sum of five rounded operands errs by half a unit each and once more."""
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    if op == "avg" and dtype == torch.uint8:
+        pytest.skip("integers are not averaged")
+    g = LoopbackGroup(n, config=make_config(scratch_bytes=1 << 20, timeout_ms=5000))
+    esz = torch.tensor([], dtype=dtype).element_size()
+    big = 1200001 if coll in ("allgather", "reduce_scatter") else 4200001
+    for nbytes, off in itertools.product([esz, 16, 16 + esz, 4096 - esz, 4096, 4096 + esz, 5 * 4096 + 8, big // esz * esz], [0, 3]):
+        count = max(1, nbytes // esz)
+        n_in, n_out = count * (n if coll == "reduce_scatter" else 1), count * (n if coll == "allgather" else 1)
+        gen = torch.Generator(device="cuda").manual_seed(nbytes)
+        xs = [torch.randint(0, 9, (n_in + off,), generator=gen, device="cuda").to(dtype)[off:] for _ in range(n)]
+        bufs = [torch.full((n_out + off + 8,), 77, device="cuda").to(dtype) for _ in range(n)]
+        outs = [b[off:off + n_out] for b in bufs]
+        g.run(coll, xs, outs, count, op=op, root=1, algo=algo, k=8)
+        _check_ok(g)
+        st = torch.stack([x.double() for x in xs])
+        total = st.max(0).values if op == "max" else st.min(0).values if op == "min" else st.mean(0) if op == "avg" else st.sum(0)
+        for r in range(n):
+            want = torch.cat(xs) if coll == "allgather" else xs[1] if coll == "broadcast" else total[r * count:(r + 1) * count] if coll == "reduce_scatter" else total
+            if coll == "reduce" and r != 1:
+                want = torch.full_like(outs[r], 77)
+            bound = 0.0 if op != "avg" else 2 * n * 2.0 ** -{torch.float32: 24, torch.bfloat16: 9, torch.float64: 24}[dtype] * 8       # (1 / 5 is an fp32 factor)
+            assert (outs[r].double() - want.double()).abs().max() <= bound, (count, off, r)
+            assert torch.all(bufs[r][:off] == 77) and torch.all(bufs[r][off + n_out:] == 77), (count, off, r)
+    g.close()
