@@ -183,4 +183,72 @@ bool nothing_waits(const std::vector<Program>& progs, const std::vector<std::vec
   return true;
 }
 
+// The same for the low-latency variant, whose entries carry their own flags and which has no progress counters: what stands in a buffer before the call is read there, and
+// every other value goes from the action that makes it straight to all that use it, instead of being handed on.
+bool share_lines(std::vector<Program>& progs, std::vector<std::vector<SharedOps>>& shared) {
+  const int n = (int)progs.size();
+  Tracer t(progs);
+  if (n < 2 || n > kMaxActionPeers + 1 || !t.match()) return false;
+  // the action that makes the value which action i of rank r sends
+  auto maker = [&](int r, int i) {
+    Ref at{r, i};
+    for (;;) {
+      const Action& a = progs[at.rank].actions[at.act];
+      if (a.n_recv == 1 && a.src_buf == BUF_NONE) at = t.producer[at.rank][at.act][0];
+      else if (a.n_recv == 0 && a.src_buf != BUF_IN) {
+        const int w = t.writer(at.rank, 0, at.act, a.src_buf, a.src_off, a.count);
+        if (w < 0 || progs[at.rank].actions[w].dst_off != a.src_off || progs[at.rank].actions[w].count != a.count) return at;
+        at.act = w;
+      } else return at;
+    }
+  };
+  std::vector<Program> next = progs;
+  shared.assign(n, {});
+  for (int r = 0; r < n; r++) { shared[r].resize(progs[r].actions.size()); for (Action& a : next[r].actions) a.n_send = 0; }
+  bool any = false;
+  std::vector<std::vector<std::vector<Ref>>> from(n);         // the entries that are left, by who takes them
+  for (int r = 0; r < n; r++) {
+    from[r].resize(progs[r].actions.size());
+    for (size_t i = 0; i < progs[r].actions.size(); i++)
+      for (int j = 0; j < progs[r].actions[i].n_recv; j++) {
+        const Ref p = t.producer[r][i][j];
+        const Origin o = t.origin(p.rank, p.act);
+        if (o.ok && o.after < 0) {
+          next[r].actions[i].recv_peer[j] = kSharedPeer;
+          SharedOps& x = shared[r][i];
+          x.buf[j] = o.buf; x.from[j] = (uint8_t)o.rank; x.off[j] = o.off; x.after[j] = -1;
+          if (o.scaled) x.scaled |= (uint8_t)(1u << j);
+          any = true;
+          continue;
+        }
+        const Ref m = maker(p.rank, p.act);
+        Action& a = next[m.rank].actions[m.act];
+        if (m.rank == r || a.n_send == kMaxActionPeers) return false;
+        for (int q = 0; q < a.n_send; q++) if (a.send_peer[q] == r) return false;
+        a.send_peer[a.n_send++] = (uint8_t)r;
+        next[r].actions[i].recv_peer[j] = (uint8_t)m.rank;
+        from[r][i].push_back(m);
+        any |= m.rank != p.rank || m.act != p.act;
+      }
+  }
+  if (!any) return false;
+  // entries of a connection are taken in the order in which they are sent, still
+  for (int s = 0; s < n; s++)
+    for (int d = 0; d < n; d++) {
+      int last = -1;
+      for (size_t i = 0; i < from[d].size(); i++) for (const Ref& m : from[d][i]) if (m.rank == s) { if (m.act <= last) return false; last = m.act; }
+    }
+  for (int r = 0; r < n; r++) {
+    std::vector<Action> kept;
+    std::vector<SharedOps> ops;
+    for (size_t i = 0; i < next[r].actions.size(); i++) {
+      if (next[r].actions[i].dst_buf == BUF_NONE && next[r].actions[i].n_send == 0) continue;
+      kept.push_back(next[r].actions[i]); ops.push_back(shared[r][i]);
+    }
+    next[r].actions = std::move(kept); shared[r] = std::move(ops);
+  }
+  progs = std::move(next);
+  return true;
+}
+
 }  // namespace piccl

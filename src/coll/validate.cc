@@ -31,7 +31,7 @@ Sizes buffer_sizes(const CollArgs& a) {
 }
 
 template <class T>
-ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer, int window, bool share) {
+ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer, int window, int share) {
   ValidateResult res;
   if (window <= 0) window = window_of(fifo_cap);
   int n = a.nranks;
@@ -39,8 +39,8 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
   Sizes sz = buffer_sizes(a);
   std::vector<Program> progs; for (int r = 0; r < n; r++) progs.push_back(compile(a, r));
   std::vector<std::vector<SharedOps>> shared;
-  if (a.in_place && a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) share = false;      // sums over a send buffer that another rank may still read
-  if (share && !share_operands(progs, shared)) share = false;
+  if (a.in_place && a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) share = 0;      // sums over a send buffer that another rank may still read
+  if (share && !(share == 2 ? share_lines(progs, shared) : share_operands(progs, shared))) share = 0;
   size_t most_actions = 1;
   for (auto& p : progs) most_actions = std::max(most_actions, p.actions.size());
   int64_t slot_bytes = std::max<int64_t>(16, seg_elems_req * a.elem_size / 16 * 16);
@@ -252,12 +252,12 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
 
 }  // namespace
 
-ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish, int window, bool share) {
+ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish, int window, int share) {
   if (integer) return run<int32_t>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, share);
   return run<float>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, share);
 }
 
-ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish, int window, bool share) {
+ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish, int window, int share) {
   return run<float>(a, 0, false, fifo_cap, (int64_t)(256 * 1024) / a.elem_size, n_cta, defer_publish, window, share);
 }
 

@@ -117,6 +117,7 @@ Program compile(const CollArgs& a, int rank);
 // of rank r.  The caller vouches that no rank's receive buffer overlaps another rank's buffers or its own send buffer (in place: all-gather and broadcast only).
 // false: the programs are as they were.
 bool share_operands(std::vector<Program>& progs, std::vector<std::vector<SharedOps>>& shared);
+bool share_lines(std::vector<Program>& progs, std::vector<std::vector<SharedOps>>& shared);      // for the low-latency variant
 // Does no action of these programs wait for another, of any rank?
 bool nothing_waits(const std::vector<Program>& progs, const std::vector<std::vector<SharedOps>>& shared);
 
@@ -150,13 +151,13 @@ struct ValidateResult {
 // reduction.  op: 0 sum, 1 prod, 2 max, 3 min.
 // defer_publish: counters are published as late as can be, when the rank is about to block.  The executor's publisher works behind the warps that
 // wait and move data; what terminates when it is this late terminates whenever it comes.
-// share: the programs as share_operands leaves them.
+// share: the programs as share_operands (1) or share_lines (2) leaves them.
 // window: segments that are walked together (0: as many as the executor walks with a FIFO of fifo_cap entries).
-ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish = false, int window = 0, bool share = false);
+ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish = false, int window = 0, int share = 0);
 
 // Symbolic check for sizes too large to materialise: coverage of every output
 // element and FIFO order, no data.
-ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish = false, int window = 0, bool share = false);
+ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish = false, int window = 0, int share = 0);
 
 // ---- dumps ----
 // Transfers in the reference's schedule XML format

@@ -331,13 +331,13 @@ static const char* check_program(const Program& p, const CollArgs& a, long long 
 }
 
 // The programs of all ranks of a launch that read each other's buffers, compiled when the first of them is not in its cache.
-struct GroupPrograms { bool made = false, flat = false; std::vector<Program> progs; std::vector<std::vector<SharedOps>> shared; };
+struct GroupPrograms { bool lines = false, made = false, flat = false; std::vector<Program> progs; std::vector<std::vector<SharedOps>> shared; };
 
-static ProgKey key_of(const CollArgs& a, bool shared) { return ProgKey{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, a.block_stride, shared ? 1 : 0}; }
+static ProgKey key_of(const CollArgs& a, int shared) { return ProgKey{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, a.block_stride, shared}; }
 
-// group: the program as share_operands makes it; the other one is kept beside it, for a captured call whose buffers overlap.
+// group: the program as share_operands or share_lines makes it; the other one is kept beside it, for a captured call whose buffers overlap.
 static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, const ProgEntry** out, GroupPrograms* group = nullptr) {
-  const ProgKey k = key_of(a, group != nullptr);
+  const ProgKey k = key_of(a, !group ? 0 : group->lines ? 2 : 1);
   auto it = c->cache.find(k);
   if (it == c->cache.end()) {
     // A new program needs device and pinned memory and an upload on the caller's stream: not inside a stream capture (an
@@ -362,7 +362,7 @@ static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, co
       if (!group->made) {
         group->made = true;
         for (int r = 0; r < a.nranks; r++) group->progs.push_back(compile(a, r));
-        if (!share_operands(group->progs, group->shared)) group->shared.clear();
+        if (!(group->lines ? share_lines(group->progs, group->shared) : share_operands(group->progs, group->shared))) group->shared.clear();
         else group->flat = nothing_waits(group->progs, group->shared);
       }
     } else c->stats.program_cache_misses++;
@@ -729,6 +729,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     bool aligned = true;
     CollArgs first;
     GroupPrograms group;
+    group.lines = use_llf;
     long long most = 0;
     bool any_shared = false, flat = false;
     for (int i = 0; i < n && rc == PICCL_OK; i++) {
@@ -743,13 +744,9 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       }
       if (d.coll == COLL_REDUCE && c->rank != d.root) a.in_place = false;
       const ProgEntry* pe = nullptr;
-      if (i == 0 && share && cap_state != cudaStreamCaptureStatusNone) share = c->cache.count(key_of(a, true)) != 0;      // (a capture replays what was built before it)
+      if (i == 0 && share && cap_state != cudaStreamCaptureStatusNone) share = c->cache.count(key_of(a, use_llf ? 2 : 1)) != 0;      // (a capture replays what was built before it)
       rc = get_program(c, a, stream, &pe, share ? &group : nullptr); if (rc) break;
       if (i == 0) flat = pe->flat;
-      if (use_llf && share && !flat) {                // (what waits for something does so in the lines of the low-latency variant)
-        share = false;
-        rc = get_program(c, a, stream, &pe); if (rc) break;
-      }
       if (i == 0) first = a;
       ka.one_gpu &= c->device == c0->device;
       ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].shared = pe->dev_shared; any_shared |= pe->dev_shared != nullptr; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
@@ -768,12 +765,12 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       if (first.coll == COLL_ALLREDUCE && (first.algo == ALGO_RING || first.algo == ALGO_K_RING)) ab /= std::max(1, first.nranks);
       if (first.algo == ALGO_DIRECT && first.coll != COLL_ALLGATHER && first.coll != COLL_REDUCE_SCATTER) ab /= std::max(1, first.coll == COLL_ALLREDUCE ? first.nranks : first.nranks - 1);
       n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
-      if (n > 1) n_cta = std::min(n_cta, std::max(1, c0->sm_count / n));
+      if (n > 1) n_cta = std::min(n_cta, std::max(1, c0->sm_count / n_working));
     }
     if (flat) { long long a = 0; for (int i = 0; i < n; i++) a += ka.r[i].n_actions; n_cta = flat_slices(c0, most * esz, a, &ka.seg_bytes); n_blocks = a * n_cta; }
     ka.n_cta = n_cta; if (!use_llf && !flat) cut_fifo(c0, n, n_cta, first, &ka);
     ka.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
-    if (any_shared && !flat) { // the widest slice is CTA 0's
+    if (any_shared && !flat && !use_llf) { // the widest slice is CTA 0's
       const long long segs = slice_of(most, esz, 0, n_cta, ka.seg_bytes).nseg;
       ka.prog_total = round_up(segs, ka.window) * ka.prog_actions + 1;
     }

@@ -21,7 +21,7 @@ struct HandleBlob {
 };
 
 struct ProgKey {
-  int coll, algo, k, root, elem_size, in_place; long long count, stride; int shared = 0 /* ranks read each other's buffers */;
+  int coll, algo, k, root, elem_size, in_place; long long count, stride; int shared = 0 /* ranks read each other's buffers: 1, 2 in the low-latency variant */;
   bool operator==(const ProgKey& o) const {
     return coll == o.coll && algo == o.algo && k == o.k && root == o.root && elem_size == o.elem_size && in_place == o.in_place && count == o.count && stride == o.stride && shared == o.shared;
   }

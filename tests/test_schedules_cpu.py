@@ -211,8 +211,11 @@ def test_programs_that_read_each_others_buffers(coll, algo):
         for fifo, count, deferred in itertools.product([2, 4], [5, 30, 32 * 2 * 3 * n, 257], [False, True]):
             v = S.validate(coll, algo, n, count, k=k, root=n - 1, in_place=in_place, n_cta=2, seg_elems=32, fifo_cap=fifo, deferred=deferred, shared=True)
             assert v.ok, f"{coll} {algo} n={n} k={k} in_place={in_place} fifo={fifo} count={count} deferred={deferred}: {v.error}"
+        for fifo, count, deferred in itertools.product([4, 8], [5, 32 * 2 * 3 * n, 257], [False, True]):
+            v = S.validate(coll, algo, n, count, k=k, root=n - 1, in_place=in_place, n_cta=2, seg_elems=32, fifo_cap=fifo, deferred=deferred, window=1, shared=2)
+            assert v.ok, f"lines: {coll} {algo} n={n} k={k} in_place={in_place} fifo={fifo} count={count} deferred={deferred}: {v.error}"
         if coll in ("allgather", "reduce_scatter"):
-            assert S.validate(coll, algo, n, 100, k=k, stride=130, n_cta=2, seg_elems=32, shared=True).ok
+            assert all(S.validate(coll, algo, n, 100, k=k, stride=130, n_cta=2, seg_elems=32, shared=sh).ok for sh in (1, 2))
 
 
 def test_what_is_handed_on_takes_no_slot():
