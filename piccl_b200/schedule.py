@@ -71,16 +71,16 @@ class Validation:
 
 def validate(coll, algo, nranks: int, count: int, k: int = -1, root: int = 0, elem_size: int = 4, in_place: bool = False,
              op: str = "sum", integer: bool = False, fifo_cap: int = 2, seg_elems: int = 64, n_cta: int = 2,
-             stride: int = 0, symbolic: bool = False, deferred: bool = False, window: int = 0, shared: int = 0) -> Validation:
+             stride: int = 0, symbolic: bool = False, deferred: bool = False, window: int = 0, flow: bool = False) -> Validation:
     """Runs all ranks' programs against each other on the CPU (see src/coll/validate.cc).
     `deferred`: FIFO counters are published as late as can be (the executor's publisher works behind its other warps); `window`: segments walked
-    together, 0 as the executor does with a FIFO of `fifo_cap` entries; `shared`: the programs of ranks that read each other's buffers (1 or
-    True), and those of the low-latency variant (2)."""
+    together, 0 as the executor does with a FIFO of `fifo_cap` entries; `flow`: the call's data flow (src/coll/flow.cc) in place
+    of its programs."""
     l = N.lib()
     ent, depth, err, sent = C.c_longlong(), C.c_int(), C.c_double(), C.c_longlong()
     msg = C.create_string_buffer(512)
     rc = l.piccl_sched_validate(_coll(coll), _algo(algo), k, nranks, root, count, stride, elem_size, int(in_place), N.OP[op], int(integer),
-                                fifo_cap, seg_elems, n_cta, int(symbolic) | (2 if deferred else 0) | int(shared) << 2 | window << 8, C.byref(ent), C.byref(depth), C.byref(err), C.byref(sent), msg, 512)
+                                fifo_cap, seg_elems, n_cta, int(symbolic) | (2 if deferred else 0) | (4 if flow else 0) | window << 8, C.byref(ent), C.byref(depth), C.byref(err), C.byref(sent), msg, 512)
     return Validation(rc == 0, msg.value.decode(), ent.value, depth.value, err.value, sent.value)
 
 

@@ -37,11 +37,11 @@ int piccl_sched_validate(int coll, int algo, int k, int n, int root, long long c
                          int op, int integer, int fifo_cap, long long seg_elems, int n_cta, int symbolic,
                          long long* fifo_entries, int* max_depth, double* max_err, long long* bytes_sent, char* err, int err_cap) {
   CollArgs a = mk(coll, algo, k, n, root, count, stride, esz, in_place);
-  // `symbolic`: bit 0 = no data (coverage and FIFO order only), bit 1 = deferred publishing of the counters, bits 2 and 3 = programs of ranks that read each other's buffers (1, 2: of the low-latency variant), from bit 8 on: segments to a window (0: the executor's choice)
+  // `symbolic`: bit 0 = no data (coverage and FIFO order only), bit 1 = deferred publishing of the counters, bit 2 = the call's data flow in place of its programs, from bit 8 on: segments to a window (0: the executor's choice)
   const bool defer = (symbolic & 2) != 0;
-  const int share = symbolic >> 2 & 3;
+  const bool flow = (symbolic & 4) != 0;
   const int window = symbolic >> 8;
-  ValidateResult v = (symbolic & 1) ? validate_symbolic(a, fifo_cap, n_cta, defer, window, share) : validate(a, op, integer != 0, fifo_cap, seg_elems, n_cta, defer, window, share);
+  ValidateResult v = (symbolic & 1) ? validate_symbolic(a, fifo_cap, n_cta, defer, window) : validate(a, op, integer != 0, fifo_cap, seg_elems, n_cta, defer, window, flow);
   if (fifo_entries) *fifo_entries = v.fifo_entries;
   if (max_depth) *max_depth = v.max_fifo_depth;
   if (max_err) *max_err = v.max_abs_err;

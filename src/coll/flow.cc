@@ -1,0 +1,184 @@
+// What a collective computes, without the way it takes: for launches that carry all ranks on one GPU, where every rank's buffers are equally near.
+//
+// A program says which operands are combined where, in which order, and through which slots the values travel.  Between GPUs that way is the point; on one GPU it is
+// several passes over memory for each hop.  `data_flow` follows the entries of all ranks' programs back and keeps what they compute: each element of a
+// receive buffer as an expression over the send buffers, with the operands of each action in its order and each partial result rounded to the element type where it would
+// have been put into a slot, so that the results are bit for bit those of the programs.  A sum that one rank makes and others receive, or that several ranks make alike, is
+// computed once and stored in all their buffers.  Nothing in such a call waits (kernels/exec_flow.cuh).
+//
+// us through the slots and this, one B200: all-reduce 4 x 25 MiB averaged by recursive doubling 131 / 43, 8 x 64 MiB on the ring 353 / 189, 8 x 280 KB 45 / 7.4, 8 x 4 KB 37 / 7.2; all-gather 4 x 1 MiB at
+// odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34; broadcast 8 x 16 MiB 110 / 27; reduce 8 x 16 MiB in two rings 120 / 69.
+#include <algorithm>
+#include <map>
+#include "coll_internal.h"
+
+namespace piccl {
+
+namespace {
+
+struct Ref { int rank = -1, act = -1; bool operator<(const Ref& o) const { return rank != o.rank ? rank < o.rank : act < o.act; } };
+
+struct Flow {
+  const std::vector<Program>& progs;
+  std::vector<std::vector<std::vector<Ref>>> producer;      // [rank][action][receive operand]
+  FlowOp op;                                                // the expression being built
+  bool ok = true;
+  explicit Flow(const std::vector<Program>& p) : progs(p), producer(p.size()) {}
+
+  // the k-th entry pushed on a connection is the k-th one popped; false: the programs do not fit together
+  bool match() {
+    const int n = (int)progs.size();
+    std::vector<std::vector<int>> pushed((size_t)n * n);
+    std::vector<size_t> popped((size_t)n * n, 0);
+    for (int s = 0; s < n; s++) {
+      producer[s].resize(progs[s].actions.size());
+      for (size_t i = 0; i < progs[s].actions.size(); i++)
+        for (int j = 0; j < progs[s].actions[i].n_send; j++) pushed[(size_t)s * n + progs[s].actions[i].send_peer[j]].push_back((int)i);
+    }
+    for (int d = 0; d < n; d++)
+      for (size_t i = 0; i < progs[d].actions.size(); i++) {
+        const Action& a = progs[d].actions[i];
+        for (int j = 0; j < a.n_recv; j++) {
+          const size_t c = (size_t)a.recv_peer[j] * n + d;
+          if (popped[c] >= pushed[c].size()) return false;
+          const int act = pushed[c][popped[c]++];
+          if (progs[a.recv_peer[j]].actions[act].count != a.count) return false;
+          producer[d][i].push_back({(int)a.recv_peer[j], act});
+        }
+      }
+    for (size_t c = 0; c < pushed.size(); c++) if (popped[c] != pushed[c].size()) return false;
+    return true;
+  }
+  // the last action of rank s in [begin, end) that stores any of the range (-1: none), and whether it stores exactly that
+  int writer(int s, int begin, int end, uint8_t buf, int64_t off, int64_t n, bool* exact) const {
+    for (int i = end; i-- > begin;) {
+      const Action& a = progs[s].actions[i];
+      if (a.dst_buf != buf || a.dst_off >= off + n || off >= a.dst_off + a.count) continue;
+      *exact = a.dst_off == off && a.count == n;
+      return i;
+    }
+    return -1;
+  }
+  // where the value of an action that only hands on (one operand) comes from: the action that makes it, or one whose operand is a buffer's elements
+  Ref maker(Ref at) {
+    for (;;) {
+      const Action& a = progs[at.rank].actions[at.act];
+      if (a.n_recv == 1 && a.src_buf == BUF_NONE) { at = producer[at.rank][at.act][0]; continue; }
+      if (a.n_recv == 0 && a.src_buf != BUF_IN) {
+        bool exact = false;
+        const int w = writer(at.rank, 0, at.act, a.src_buf, a.src_off, a.count, &exact);
+        if (w >= 0 && exact) { at.act = w; continue; }
+        if (w >= 0 || a.src_buf != BUF_OUT) ok = false;
+      }
+      return at;
+    }
+  }
+  void leaf(int rank, uint8_t buf, int64_t off, bool scaled, bool rounded, int level, bool first) {
+    if (op.n_leaf == kFlowLeaves) { ok = false; return; }
+    const int i = op.n_leaf++;
+    op.leaf_rank[i] = (uint8_t)rank; op.leaf_buf[i] = buf; op.leaf_off[i] = off;
+    op.place[i] = (uint8_t)(level | (first ? 4 : 0));
+    if (scaled) op.scaled |= (uint8_t)(1u << i);
+    // (one half, quarter or eighth of an element is itself an element but where it is too small for one: not rounding it there loses nothing, and all ranks' averages are the same)
+    if (scaled && rounded && (progs.size() & (progs.size() - 1)) != 0) op.rounded |= (uint8_t)(1u << i);
+  }
+  void event(bool merge) {                                  // after the last leaf
+    uint8_t& p = op.place[op.n_leaf - 1];
+    const int k = p >> 3 & 3;
+    if (k == 3) { ok = false; return; }
+    p = (uint8_t)((p & ~0x18) | (k + 1) << 3 | (merge ? 0x20 << k : 0));
+    op.nested = 1;
+  }
+  // The operands of the action that makes `at`, folded into accumulator `level`.
+  void fold(Ref at, int level) {
+    if (!ok) return;
+    if (level >= kFlowLevels) { ok = false; return; }
+    const Action& a = progs[at.rank].actions[at.act];
+    struct Operand { Ref from; bool own; };                 // own: the rank's elements of the send buffer
+    std::vector<Operand> operands;
+    for (int j = 0; j <= a.n_recv && ok; j++) {
+      if (j == a.self_pos && a.src_buf == BUF_IN) operands.push_back({at, true});
+      else if (j == a.self_pos && a.src_buf != BUF_NONE) {
+        bool exact = false;
+        const int w = writer(at.rank, 0, at.act, a.src_buf, a.src_off, a.count, &exact);
+        if (w < 0 || !exact) { ok = false; return; }
+        operands.push_back({maker({at.rank, w}), false});
+      }
+      if (j < a.n_recv) operands.push_back({maker(producer[at.rank][at.act][j]), false});
+    }
+    if (!ok) return;
+    auto simple = [&](const Operand& o) { return o.own || progs[o.from.rank].actions[o.from.act].n_recv == 0; };
+    bool first = true;
+    auto emit = [&](const Operand& o, bool before) {
+      if (!ok) return;
+      const Action& b = progs[o.from.rank].actions[o.from.act];
+      if (o.own) leaf(at.rank, BUF_IN, a.src_off, (a.flags & ACT_SCALE_SRC) != 0, false, level, first);
+      else if (simple(o)) leaf(o.from.rank, b.src_buf, b.src_off, (b.flags & ACT_SCALE_SRC) && b.src_buf == BUF_IN, true, level, first);
+      else if (first) { fold(o.from, level); if (ok) event(false); }
+      else { fold(o.from, level + 1); if (ok) event(true); }
+      if (ok && before) op.before |= (uint8_t)(1u << (op.n_leaf - 1));
+      first = false;
+    };
+    // a result behind a leaf: the result first, the leaf as its left operand (a ring's hops would need an accumulator each)
+    const bool turned = operands.size() >= 2 && simple(operands[0]) && !simple(operands[1]);
+    if (turned) { emit(operands[1], false); emit(operands[0], true); }
+    for (size_t q = turned ? 2 : 0; q < operands.size(); q++) emit(operands[q], false);
+  }
+};
+
+}  // namespace
+
+bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops) {
+  const int n = (int)progs.size();
+  ops.clear();
+  Flow f(progs);
+  if (n < 2 || n > kFlowLeaves || !f.match()) return false;
+  std::map<Ref, int> made;                                  // the operation of what an action makes
+  auto alike = [](const FlowOp& a, const FlowOp& b) {
+    if (a.count != b.count || a.n_leaf != b.n_leaf || a.nested != b.nested || a.scaled != b.scaled || a.rounded != b.rounded || a.before != b.before) return false;
+    for (int i = 0; i < a.n_leaf; i++) if (a.leaf_rank[i] != b.leaf_rank[i] || a.leaf_buf[i] != b.leaf_buf[i] || a.leaf_off[i] != b.leaf_off[i] || a.place[i] != b.place[i]) return false;
+    return true;
+  };
+  for (int r = 0; r < n; r++)
+    for (size_t i = 0; i < progs[r].actions.size(); i++) {
+      const Action& a = progs[r].actions[i];
+      if (a.dst_buf != BUF_OUT) continue;
+      bool exact = false;
+      if (f.writer(r, (int)i + 1, (int)progs[r].actions.size(), a.dst_buf, a.dst_off, a.count, &exact) >= 0) { if (!exact) return false; continue; }      // stored for a later step only
+      const Ref m = f.maker({r, (int)i});
+      if (!f.ok) return false;
+      const Action& b = progs[m.rank].actions[m.act];
+      f.op = FlowOp();
+      f.op.count = a.count;
+      int at = -1;
+      if (b.n_recv == 0) {
+        // A copy has one destination: the operand comes from the cache again for the next (all-gather 8 x 8 MiB 97.5 us, 107 with eight destinations; 4 x 1 MiB at odd addresses, where a
+        // copy to one place is shifted once, 10.4 and 15.2).  The maker's own copy of a scaled operand is the value that others receive.
+        f.leaf(m.rank, b.src_buf, b.src_off, (b.flags & ACT_SCALE_SRC) && b.src_buf == BUF_IN, false, 0, true);
+      } else {
+        const auto it = made.find(m);
+        if (it != made.end()) at = it->second;
+        else {
+          f.fold(m, 0);
+          for (size_t q = 0; q < ops.size() && f.ok && at < 0; q++) if (ops[q].n_leaf > 1 && alike(ops[q], f.op)) at = (int)q;
+        }
+      }
+      if (!f.ok) return false;
+      if (at < 0 || ops[at].n_dst == kFlowLeaves) { at = (int)ops.size(); ops.push_back(f.op); }
+      if (b.n_recv != 0) made[m] = at;
+      FlowOp& op = ops[at];
+      op.dst_rank[op.n_dst] = (uint8_t)r; op.dst_off[op.n_dst++] = a.dst_off;
+    }
+  // Elements of a buffer that no other operation reads may leave the cache with their use.
+  for (size_t i = 0; i < ops.size(); i++) {
+    bool again = false;
+    for (size_t q = 0; q < ops.size() && !again; q++)
+      for (int l = 0; l < ops[i].n_leaf && q != i && !again; l++)
+        for (int k = 0; k < ops[q].n_leaf; k++)
+          again |= ops[q].leaf_rank[k] == ops[i].leaf_rank[l] && ops[q].leaf_buf[k] == ops[i].leaf_buf[l] && ops[q].leaf_off[k] < ops[i].leaf_off[l] + ops[i].count && ops[i].leaf_off[l] < ops[q].leaf_off[k] + ops[q].count;
+    ops[i].once = !again;
+  }
+  return !ops.empty();
+}
+
+}  // namespace piccl

@@ -31,18 +31,13 @@ Sizes buffer_sizes(const CollArgs& a) {
 }
 
 template <class T>
-ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer, int window, int share) {
+ValidateResult run(const CollArgs& a, int op_, bool with_data, int fifo_cap, int64_t seg_elems_req, int n_cta, bool defer, int window, bool flow) {
   ValidateResult res;
   if (window <= 0) window = window_of(fifo_cap);
   int n = a.nranks;
   int64_t st = a.block_stride ? a.block_stride : a.count;
   Sizes sz = buffer_sizes(a);
   std::vector<Program> progs; for (int r = 0; r < n; r++) progs.push_back(compile(a, r));
-  std::vector<std::vector<SharedOps>> shared;
-  if (a.in_place && a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) share = 0;      // sums over a send buffer that another rank may still read
-  if (share && !(share == 2 ? share_lines(progs, shared) : share_operands(progs, shared))) share = 0;
-  size_t most_actions = 1;
-  for (auto& p : progs) most_actions = std::max(most_actions, p.actions.size());
   int64_t slot_bytes = std::max<int64_t>(16, seg_elems_req * a.elem_size / 16 * 16);
 
   const int64_t guard = with_data ? 8 : 0;
@@ -66,7 +61,7 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
       for (int64_t i = 0; i < sz.in_elems; i++) {
         T v;
         if (std::is_floating_point<T>::value) v = (T)fd(gen); else v = (T)id(gen);
-        if (op == 1) v = std::is_floating_point<T>::value ? (T)(1.0 + 0.01 * (double)v) : (T)((i + r) % 3 == 0 ? 2 : 1);
+        if (op_ == 1) v = std::is_floating_point<T>::value ? (T)(1.0 + 0.01 * (double)v) : (T)((i + r) % 3 == 0 ? 2 : 1);
         in[r][i] = v;
       }
       in_copy[r].assign(in[r], in[r] + sz.in_elems);
@@ -78,6 +73,30 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
   // symbolic coverage: count of writes per OUT pack is too big for 1 GiB; track per (rank) intervals
   std::vector<std::vector<std::pair<int64_t, int64_t>>> cover(n);
 
+  std::vector<FlowOp> ops;
+  if (flow) {
+    if (!with_data || (a.in_place && a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) || !data_flow(progs, ops)) { res.error = "no data flow"; return res; }
+    for (const FlowOp& op : ops) {
+      for (int i = 0; i < op.n_leaf; i++) if (op.leaf_off[i] < 0 || op.leaf_off[i] + op.count > (op.leaf_buf[i] == BUF_IN ? sz.in_elems : sz.out_elems)) { res.error = "leaf out of bounds"; return res; }
+      for (int i = 0; i < op.n_dst; i++) if (op.dst_off[i] < 0 || op.dst_off[i] + op.count > sz.out_elems) { res.error = "destination range out of bounds"; return res; }
+      for (int64_t e = 0; e < op.count; e++) {
+        T acc[kFlowLevels] = {};
+        int level = 0;
+        for (int i = 0; i < op.n_leaf; i++) {
+          const T* b = op.leaf_buf[i] == BUF_IN ? in[op.leaf_rank[i]] : out[op.leaf_rank[i]];
+          const T x = b[op.leaf_off[i] + e];
+          level = op.place[i] & 3;
+          acc[level] = op.place[i] & 4 ? x : op.before >> i & 1 ? apply<T>(op_, x, acc[level]) : apply<T>(op_, acc[level], x);
+          for (int k = 0; k < (op.place[i] >> 3 & 3); k++) if (op.place[i] >> (5 + k) & 1) { level--; acc[level] = apply<T>(op_, acc[level], acc[level + 1]); }
+        }
+        if (level != 0) { res.error = "accumulators left"; return res; }
+        for (int i = 0; i < op.n_dst; i++) out[op.dst_rank[i]][op.dst_off[i] + e] = acc[0];
+      }
+      for (int i = 0; i < op.n_dst; i++) cover[op.dst_rank[i]].push_back({op.dst_off[i], op.dst_off[i] + op.count});
+    }
+    n_cta = 0;                    // (no entries)
+  }
+
   int64_t entries = 0; int maxdepth = 0; std::vector<int64_t> sent_bytes(n, 0);
   for (int cta = 0; cta < n_cta; cta++) {
     struct Entry { std::vector<T> data; int64_t n; };
@@ -85,13 +104,9 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
     std::vector<Cursor> cur(n);
     // Deferred publishing: a push is visible to the consumer, and a pop to the producer, only once the rank that made it has published it, at the
     // latest when it is about to block and when its program ends (the executor's publisher is a warp of its own and may be that late).
-    // Progress: where in the walk a rank has come to (its last finished step), as the executor's progress counters tell it.
-    std::vector<int64_t> passed(n, 0), pub_passed(n, 0);
-    std::vector<std::vector<std::vector<T>>> kept(n, std::vector<std::vector<T>>(window));
     std::vector<int64_t> pushed((size_t)n * n, 0), popped((size_t)n * n, 0), pub_push((size_t)n * n, 0), pub_pop((size_t)n * n, 0);
     auto flush = [&](int r) {
-      bool any = pub_passed[r] != passed[r];
-      pub_passed[r] = passed[r];
+      bool any = false;
       for (int o = 0; o < n; o++) {
         size_t out_c = (size_t)r * n + o, in_c = (size_t)o * n + r;
         if (pub_push[out_c] != pushed[out_c]) { pub_push[out_c] = pushed[out_c]; any = true; }
@@ -126,11 +141,6 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
               if ((defer ? pushed[cn] - pub_pop[cn] : (int64_t)fifo[cn].size()) >= fifo_cap) ready = false;
             }
             for (int i = 0; i < ac.n_recv; i++) {
-              if (ac.recv_peer[i] == kSharedPeer) {
-                const SharedOps& x = shared[r][c.act];
-                if (x.after[i] >= 0 && x.from[i] != r && (defer ? pub_passed[x.from[i]] : passed[x.from[i]]) < step_position(c.seg0, c.seg, (size_t)x.after[i], most_actions, window)) ready = false;
-                continue;
-              }
               size_t cn = (size_t)ac.recv_peer[i] * n + r;
               if (defer ? pub_push[cn] - popped[cn] <= 0 : fifo[cn].empty()) ready = false;
             }
@@ -140,35 +150,24 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
               std::vector<T> val;
               if (with_data) {
                 val.resize(len);
-                auto base = [&](int o, uint8_t buf) -> const T* { return buf == BUF_IN ? in[o] : buf == BUF_OUT ? out[o] : buf == BUF_SCRATCH ? scratch[o].data() : nullptr; };
-                auto limit = [&](int o, uint8_t buf) { return buf == BUF_IN ? sz.in_elems : buf == BUF_OUT ? sz.out_elems : progs[o].scratch_elems; };
-                const T* src = base(r, ac.src_buf);
-                const int64_t src_lim = limit(r, ac.src_buf);
-                const std::vector<T> again = kept[r][c.seg - c.seg0];
-                if (ac.src_buf == BUF_KEPT && (int64_t)again.size() != len) { res.error = "no kept value"; return res; }
+                const T* src = ac.src_buf == BUF_IN ? in[r] : ac.src_buf == BUF_OUT ? out[r] : ac.src_buf == BUF_SCRATCH ? scratch[r].data() : nullptr;
+                int64_t src_lim = ac.src_buf == BUF_IN ? sz.in_elems : ac.src_buf == BUF_OUT ? sz.out_elems : p.scratch_elems;
                 if (src && ac.src_off + hi > src_lim) { res.error = "source range out of bounds"; return res; }
                 // rank order: recv peers below me, me, recv peers above me
                 bool first = true; int pos = 0;
-                auto fold = [&](const T* x) { for (int64_t i = 0; i < len; i++) val[i] = first ? x[i] : apply<T>(op, val[i], x[i]); first = false; };
+                auto fold = [&](const T* x) { for (int64_t i = 0; i < len; i++) val[i] = first ? x[i] : apply<T>(op_, val[i], x[i]); first = false; };
                 for (int i = 0; i <= ac.n_recv; i++) {
                   if (i == ac.self_pos && src) fold(src + ac.src_off + lo);
-                  if (i == ac.self_pos && ac.src_buf == BUF_KEPT) fold(again.data());
-                  if (i < ac.n_recv && ac.recv_peer[i] == kSharedPeer) {
-                    const SharedOps& x = shared[r][c.act];
-                    if (x.off[i] < 0 || x.off[i] + hi > limit(x.from[i], x.buf[i])) { res.error = "shared range out of bounds"; return res; }
-                    fold(base(x.from[i], x.buf[i]) + x.off[i] + lo);
-                  } else if (i < ac.n_recv) {
+                  if (i < ac.n_recv) {
                     Entry& e = fifo[(size_t)ac.recv_peer[i] * n + r].front();
                     if (e.n != len) { res.error = "fifo entry size mismatch"; return res; }
                     fold(e.data.data()); pos++;
                   }
                 }
               } else {
-                for (int i = 0; i < ac.n_recv; i++) if (ac.recv_peer[i] != kSharedPeer && fifo[(size_t)ac.recv_peer[i] * n + r].front().n != len) { res.error = "fifo entry size mismatch"; return res; }
+                for (int i = 0; i < ac.n_recv; i++) if (fifo[(size_t)ac.recv_peer[i] * n + r].front().n != len) { res.error = "fifo entry size mismatch"; return res; }
               }
-              if (ac.keep) kept[r][c.seg - c.seg0] = val;
-              passed[r] = step_position(c.seg0, c.seg, c.act, most_actions, window);
-              for (int i = 0; i < ac.n_recv; i++) if (ac.recv_peer[i] != kSharedPeer) { fifo[(size_t)ac.recv_peer[i] * n + r].pop_front(); popped[(size_t)ac.recv_peer[i] * n + r]++; }
+              for (int i = 0; i < ac.n_recv; i++) { fifo[(size_t)ac.recv_peer[i] * n + r].pop_front(); popped[(size_t)ac.recv_peer[i] * n + r]++; }
               if (ac.dst_buf != BUF_NONE) {
                 int64_t lim = ac.dst_buf == BUF_OUT ? sz.out_elems : p.scratch_elems;
                 if (ac.dst_buf == BUF_IN || ac.dst_off + hi > lim || ac.dst_off + lo < 0) { res.error = "destination range out of bounds"; return res; }
@@ -217,7 +216,7 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
 
   // data check
   double maxerr = 0;
-  auto expect_reduce = [&](int64_t idx_in) { T v = in_copy[0][idx_in]; for (int r = 1; r < n; r++) v = apply<T>(op, v, in_copy[r][idx_in]); return v; };
+  auto expect_reduce = [&](int64_t idx_in) { T v = in_copy[0][idx_in]; for (int r = 1; r < n; r++) v = apply<T>(op_, v, in_copy[r][idx_in]); return v; };
   auto check = [&](int r, int64_t oi, T want, double tol) {
     double e = std::fabs((double)out[r][oi] - (double)want);
     maxerr = std::max(maxerr, e);
@@ -252,13 +251,13 @@ ValidateResult run(const CollArgs& a, int op, bool with_data, int fifo_cap, int6
 
 }  // namespace
 
-ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish, int window, int share) {
-  if (integer) return run<int32_t>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, share);
-  return run<float>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, share);
+ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish, int window, bool flow) {
+  if (integer) return run<int32_t>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, flow);
+  return run<float>(a, op, true, fifo_cap, seg_elems, n_cta, defer_publish, window, flow);
 }
 
-ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish, int window, int share) {
-  return run<float>(a, 0, false, fifo_cap, (int64_t)(256 * 1024) / a.elem_size, n_cta, defer_publish, window, share);
+ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish, int window) {
+  return run<float>(a, 0, false, fifo_cap, (int64_t)(256 * 1024) / a.elem_size, n_cta, defer_publish, window, false);
 }
 
 }  // namespace piccl

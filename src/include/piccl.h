@@ -99,8 +99,8 @@ int piccl_broadcast(piccl_comm_t* c, const void* send, void* recv, size_t count,
 /* Runs one collective over several communicators of THIS process that live on
  * the same device (virtual ranks) as a single cooperative kernel launch.  Used
  * to exercise the multi-rank protocol on one GPU.  With all ranks in the launch,
- * and buffers that do not overlap, what is only handed on is read at its origin
- * instead of crossing hop by hop through the slots. */
+ * and buffers that do not overlap, what the ranks' programs compute is computed
+ * straight from the send buffers, bit for bit the same. */
 int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const void* const* send, void* const* recv,
                            size_t count, int dtype, int op, int root, int algo, int k, void* stream);
 
@@ -125,8 +125,8 @@ int piccl_tp_status(piccl_comm_t* c);   /* 0, or the role that gave up on a wait
  * `bytes` in a launch of `in_launch` of `nranks` ranks. */
 int piccl_test_leave_first(int coll, int nranks, int in_launch, int one_device, long long bytes);
 
-/* Test hook: ranks of one launch do not read each other's buffers but use the
- * slots for everything, as ranks on several GPUs do. */
+/* Test hook: a launch that carries all ranks runs their programs, through the
+ * slots, as ranks on several GPUs do, and not the call's data flow. */
 int piccl_test_slots_only(piccl_comm_t* c, int on);
 
 /* Test hook: launches the executor with one action that waits for data nobody

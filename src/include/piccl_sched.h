@@ -34,7 +34,7 @@ enum Coll : int { COLL_ALLGATHER = 0, COLL_ALLREDUCE = 1, COLL_BROADCAST = 2, CO
 // has no multicast window.
 enum Algo : int { ALGO_DEFAULT_NCCL = 0, ALGO_RING = 1, ALGO_K_RING = 2, ALGO_RD = 3, ALGO_RM = 4, ALGO_PRD = 5, ALGO_PRM = 6, ALGO_AUTO = 7, ALGO_DIRECT = 8, ALGO_NVLS = 9 };
 
-enum Buf : uint8_t { BUF_NONE = 0, BUF_IN = 1, BUF_OUT = 2, BUF_SCRATCH = 3, BUF_KEPT = 4 /* the entry that the last action with `keep` sent */ };
+enum Buf : uint8_t { BUF_NONE = 0, BUF_IN = 1, BUF_OUT = 2, BUF_SCRATCH = 3 };
 
 constexpr int kMaxActionPeers = 7;   // k-1 for the largest supported radix (8)
 constexpr int kMaxRanks = 64;
@@ -54,7 +54,7 @@ struct Action {
   uint8_t self_pos = 0;         // position of the local operand among the recv peers (rank order)
   uint8_t flags = 0;
   uint8_t step = 0;             // schedule step the action belongs to (informational)
-  uint8_t keep = 0;             // 1: a later action reads the value again from the slot of send_peer[0] (share_operands)
+  uint8_t pad = 0;
   uint8_t recv_peer[kMaxActionPeers + 1] = {0};
   uint8_t send_peer[kMaxActionPeers + 1] = {0};
   int64_t src_off = 0;          // element offsets into the local buffers
@@ -63,17 +63,24 @@ struct Action {
 };
 static_assert(sizeof(Action) == 48, "Action layout is shared with device code");
 
-// Operands that an action reads where another rank holds them, in place of an entry of a FIFO (receive operands whose peer is kSharedPeer).
-constexpr uint8_t kSharedPeer = 0xff;
-struct SharedOps {
-  uint8_t buf[kMaxActionPeers + 1] = {0};       // of rank from[j]
-  uint8_t from[kMaxActionPeers + 1] = {0};
-  int32_t after[kMaxActionPeers + 1] = {0};     // that rank's action which stores the elements; -1: they are there before the call
-  int64_t off[kMaxActionPeers + 1] = {0};
-  uint8_t scaled = 0;                           // bit j: operand j is an original contribution (pre-scaled for avg)
-  uint8_t pad[7] = {0};
+// One operation of a call whose ranks all run in one launch on one GPU (flow.cc): an expression over elements of the ranks' buffers, stored in one or more receive buffers.
+// Leaves are folded in their order into accumulators that stand for actions that wait for their operands: place[i] bits 0-1 the accumulator, bit 2 set: it begins with
+// this leaf, bits 3-4 how many results are complete behind it, from bit 5 one bit for each of these: 0, rounded to the element type where it is; 1, rounded
+// and folded into the accumulator below, which is the one in use from then on.
+constexpr int kFlowLeaves = 8, kFlowLevels = 4;
+struct FlowOp {
+  int64_t count = 0;
+  int64_t leaf_off[kFlowLeaves] = {0};
+  int64_t dst_off[kFlowLeaves] = {0};
+  uint8_t leaf_rank[kFlowLeaves] = {0}, leaf_buf[kFlowLeaves] = {0}, place[kFlowLeaves] = {0}, dst_rank[kFlowLeaves] = {0};
+  uint8_t n_leaf = 0, n_dst = 0;
+  uint8_t nested = 0;            // 1: some results are rounded before the last one
+  uint8_t scaled = 0, rounded = 0;      // bit i: leaf i is an original contribution (pre-scaled for avg), which is rounded once scaled
+  uint8_t once = 0;              // 1: no other operation reads the leaves
+  uint8_t before = 0;            // bit i: leaf i is the left operand of what it is folded into
+  uint8_t pad[1] = {0};
 };
-static_assert(sizeof(SharedOps) == 120, "SharedOps layout is shared with device code");
+static_assert(sizeof(FlowOp) == 176, "FlowOp layout is shared with device code");
 
 struct Program {
   int rank = 0, nranks = 0;
@@ -113,13 +120,9 @@ Resolved resolve(Coll coll, Algo algo, int k, int nranks);
 // to RING shapes through resolve()).
 Program compile(const CollArgs& a, int rank);
 
-// The programs of ALL ranks of a launch on one GPU, changed so that values which are only handed on are read at their origin (share.cc); shared[r][i]: of action i
-// of rank r.  The caller vouches that no rank's receive buffer overlaps another rank's buffers or its own send buffer (in place: all-gather and broadcast only).
-// false: the programs are as they were.
-bool share_operands(std::vector<Program>& progs, std::vector<std::vector<SharedOps>>& shared);
-bool share_lines(std::vector<Program>& progs, std::vector<std::vector<SharedOps>>& shared);      // for the low-latency variant
-// Does no action of these programs wait for another, of any rank?
-bool nothing_waits(const std::vector<Program>& progs, const std::vector<std::vector<SharedOps>>& shared);
+// The operations of a call, from the programs of ALL its ranks.  The caller vouches that no rank's receive buffer overlaps another rank's buffers or its own send
+// buffer (in place: all-gather and broadcast only).  false: they have no such form.
+bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops);
 
 // Chunking used by allreduce: chunk c covers [displ(c), displ(c)+cnt(c)); chunk
 // starts are multiples of 16 bytes; tail chunks may be short or empty.
@@ -151,13 +154,13 @@ struct ValidateResult {
 // reduction.  op: 0 sum, 1 prod, 2 max, 3 min.
 // defer_publish: counters are published as late as can be, when the rank is about to block.  The executor's publisher works behind the warps that
 // wait and move data; what terminates when it is this late terminates whenever it comes.
-// share: the programs as share_operands (1) or share_lines (2) leaves them.
+// flow: what data_flow makes of the programs is run instead of them; an error where it does not take them.
 // window: segments that are walked together (0: as many as the executor walks with a FIFO of fifo_cap entries).
-ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish = false, int window = 0, int share = 0);
+ValidateResult validate(const CollArgs& a, int op, bool integer, int fifo_cap, int64_t seg_elems, int n_cta, bool defer_publish = false, int window = 0, bool flow = false);
 
 // Symbolic check for sizes too large to materialise: coverage of every output
 // element and FIFO order, no data.
-ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish = false, int window = 0, int share = 0);
+ValidateResult validate_symbolic(const CollArgs& a, int fifo_cap, int n_cta, bool defer_publish = false, int window = 0);
 
 // ---- dumps ----
 // Transfers in the reference's schedule XML format

@@ -34,10 +34,4 @@ PICCL_HD Slice slice_of(int64_t count, int elem_size, int cta, int n_cta, int64_
 // slots for it: every segment of a window may have an entry in flight and one that the next action sends before it is consumed.
 PICCL_HD int window_of(int nslot) { return nslot >= 4 ? 2 : 1; }
 
-// A step's place in a rank's walk, counted from 1: segment `seg` of window [seg0, seg0 + window), action `act`, where no rank of the launch has more than
-// `most_actions`.  (Places of segments that an action does not have are left out, so that a reader knows a producer's place from its own.)
-PICCL_HD int64_t step_position(int64_t seg0, int64_t seg, int64_t act, int64_t most_actions, int window) {
-  return seg0 * most_actions + act * window + (seg - seg0) + 1;
-}
-
 }  // namespace piccl

@@ -1,11 +1,10 @@
 // Device-side data structures of the fused collective executor and the
 // layout of the per-rank symmetric heap.
 //
-//   heap = [ tail counters | head counters | progress counters | ... | scratch | FIFO slots ]
+//   heap = [ tail counters | head counters | scratch | FIFO slots ]
 //
 // tail[src][cta]  (in the receiver's heap, written by `src`): entries `src` has pushed
 // head[dst][cta]  (in the sender's heap, written by `dst`):   entries `dst` has consumed
-// progress[cta]   (in the rank's own heap):               steps it has published, where ranks read each other's buffers (one launch on one GPU)
 // slot(src, cta, i) (in the receiver's heap): payload of entry number e with e % nslot == i
 //
 // All counters only ever grow, over the whole life of the communicator, so a
@@ -23,14 +22,14 @@ namespace piccl {
 constexpr int kFlagStride = 128;          // bytes between two counters
 constexpr int kMaxVRanks = 8;             // virtual ranks one launch can carry (single-GPU emulation)
 constexpr int kMaxBlock = 512;             // threads of an executor CTA that move data
-constexpr int kFlatBlock = 256;            // threads of a block of a call in which nothing waits
+constexpr int kFlowBlock = 256;            // threads of a block that runs a slice of an operation (exec_flow.cuh)
 constexpr int kCtlThreads = 64;            // and two warps more: waiter and publisher
 constexpr int kLLFifoCta = 16, kLLFifoSlots = 8, kLLFifoSlotBytes = 8192;   // low-latency FIFO: CTAs, ring depth, bytes per slot (half of it payload)
 
 struct RankCtx {
   int rank, nranks, max_cta, nslot;
   long long slot_bytes;
-  long long tail_off, head_off, prog_off, ll_off, scratch_off, fifo_off, heap_bytes;
+  long long tail_off, head_off, ll_off, scratch_off, fifo_off, heap_bytes;
   long long ll_slot_bytes;                // bytes of one low-latency slot (2 x the largest payload)
   long long scratch_bytes;
   long long llf_off, llf_head_off;                // low-latency FIFO of the executor: lines and head counters
@@ -47,7 +46,6 @@ struct RankCtx {
 struct LaunchRank {
   RankCtx* ctx;
   const Action* actions;
-  const SharedOps* shared;                // of the actions, where ranks read each other's buffers; else null
   int n_actions;
   int pad;
   const void* in;
@@ -65,15 +63,25 @@ struct KernelArgs {
   long long seg_bytes;                    // bytes of a segment and of its slot
   int one_gpu;                            // 1: every rank's heap is on this GPU: counters and fences need no scope beyond it
   int leave_first;                        // with their last use leave L2 first: operands (1), results (2)
-  // Ranks that read each other's buffers (prog_total != 0): r[i] is rank i.  Each raises a progress counter per CTA, from call to call by `prog_total`; within a call to what
-  // step_position says of the step it has published.
-  uint8_t working[kMaxVRanks];            // the ranks that have anything to do, and the launch's CTAs
-  int prog_actions;                       // most actions of any rank
-  long long prog_total;
   int nslot, window;                      // slots; segments that are walked together, at most half the slots
   unsigned long long timeout_ns;
   LaunchRank r[kMaxVRanks];
 };
+
+// ---- all ranks in one launch on one GPU (exec_flow.cuh)
+struct FlowArgs {
+  int n_ops, n_slices;                    // grid: n_ops x n_slices blocks
+  int avg;
+  float scale;
+  int leave_first;                        // as above
+  long long slice_bytes;
+  const FlowOp* ops;
+  const void* in[kMaxVRanks];
+  void* out[kMaxVRanks];
+};
+typedef void (*FlowKernelFn)(FlowArgs);
+FlowKernelFn exec_flow_kernel_for(int dtype, int op, bool shift);      // shift: operands that are not 16-byte aligned
+FlowKernelFn exec_flow_copy_kernel(bool shift);
 
 // ---- low-latency all-reduce (ll_allreduce.cu)
 constexpr int kLLMaxSteps = 6;
@@ -120,8 +128,6 @@ ExecKernelFn exec_kernel_for(int dtype, int op);
 ExecKernelFn exec_copy_kernel();
 ExecKernelFn exec_shift_kernel_for(int dtype, int op);   // operands that are not 16-byte aligned
 ExecKernelFn exec_shift_copy_kernel();
-ExecKernelFn exec_flat_kernel_for(int dtype, int op, bool shift);   // calls in which nothing waits (exec_flat.cuh)
-ExecKernelFn exec_flat_copy_kernel(bool shift);
 ExecKernelFn exec_ll_kernel_for(int dtype, int op);   // low-latency variant (exec_ll.cuh)
 ExecKernelFn exec_ll_copy_kernel();
 

@@ -200,7 +200,8 @@ __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, i
 }
 // (Only the aligned loops take these: at odd addresses, with more than two operands, or with destinations read from the table (NDST 0), lines keep the normal priority.)
 struct L2Hints { bool src_done, dst_done; int local_src, local_dst; };
-template <typename T, int OP, int NSRC, int NDST, int U, bool EXACT, bool SCALE = false>      // EXACT: nsrc == NSRC, else the first operand stands in for what is missing; NDST 0: any number, read from the table each time
+// FLOW: all operands and results are the caller's (exec_flow.cuh).
+template <typename T, int OP, bool FLOW, int NSRC, int NDST, int U, bool EXACT, bool SCALE = false>      // EXACT: nsrc == NSRC, else the first operand stands in for what is missing; NDST 0: any number, read from the table each time
 __device__ __forceinline__ void stream(int nt, const char* const* src, int nsrc_rt, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
   constexpr bool HINT_SRC = NSRC <= 2;                   // (more sources leave no registers for their policies)
   const int nsrc = EXACT ? NSRC : nsrc_rt, tid = threadIdx.x;
@@ -212,14 +213,17 @@ __device__ __forceinline__ void stream(int nt, const char* const* src, int nsrc_
   unsigned long long ps[HINT_SRC ? NSRC : 1], pd[NDST ? NDST : 1];
   const unsigned long long normal = l2_policy(false);
 #pragma unroll
-  for (int s = 0; s < NSRC; s++) if (HINT_SRC) ps[s] = h.src_done && s == h.local_src ? l2_policy(true) : normal;
+  for (int s = 0; s < NSRC; s++) if (HINT_SRC) ps[s] = h.src_done && (FLOW || s == h.local_src) ? l2_policy(true) : normal;
 #pragma unroll
-  for (int d = 0; d < NDST; d++) pd[d] = h.dst_done && d == h.local_dst ? l2_policy(true) : normal;
+  for (int d = 0; d < NDST; d++) pd[d] = h.dst_done && (FLOW || d == h.local_dst) ? l2_policy(true) : normal;
+  const unsigned long long every = FLOW && h.dst_done ? l2_policy(true) : normal;
   auto get = [&](int s, int off) { if constexpr (HINT_SRC) return ld_hint(sp[s] + off, ps[s]); else return ld_slot(sp[s] + off); };
   auto put = [&](int off, const uint4& o) {
 #pragma unroll
     for (int d = 0; d < NDST; d++) st_hint(dp[d] + off, o, pd[d]);
-    if (NDST == 0) for (int d = 0; d < ndst; d++) st_vec(dst[d] + off, o);
+    if (NDST == 0) {
+      for (int d = 0; d < ndst; d++) if constexpr (FLOW) st_hint(dst[d] + off, o, every); else st_vec(dst[d] + off, o);
+    }
   };
   int p = tid;
   for (; p + (U - 1) * nt < n; p += U * nt) {
@@ -241,33 +245,33 @@ __device__ __forceinline__ void stream(int nt, const char* const* src, int nsrc_
     for (int u = 0; u < U - 1; u++) if (p + u * nt < n) put((p + u * nt) * 16, combine<T, OP, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
   }
 }
-template <typename T, int OP>
+template <typename T, int OP, bool FLOW>
 __device__ __forceinline__ void move_aligned(int nt, const char* const* src, int nsrc, char* const* dst, int ndst, int n, int scaled, float scale, const L2Hints& h) {
   if (OP == OP_COPY || (nsrc == 1 && !scaled)) {
-    if (ndst == 1) stream<T, OP, 1, 1, 8, true>(nt, src, 1, dst, 1, n, 0, scale, h);
-    else if (ndst == 2) stream<T, OP, 1, 2, 8, true>(nt, src, 1, dst, 2, n, 0, scale, h);
-    else stream<T, OP, 1, 0, 4, true>(nt, src, 1, dst, ndst, n, 0, scale, h);
+    if (ndst == 1) stream<T, OP, FLOW, 1, 1, 8, true>(nt, src, 1, dst, 1, n, 0, scale, h);
+    else if (ndst == 2) stream<T, OP, FLOW, 1, 2, 8, true>(nt, src, 1, dst, 2, n, 0, scale, h);
+    else stream<T, OP, FLOW, 1, 0, 4, true>(nt, src, 1, dst, ndst, n, 0, scale, h);
   } else if constexpr (OP != OP_COPY) {
     // Scaled operands (avg, which is a sum) have loops of their own too: in the general one a lone operand was loaded twice and the destinations read
     // from the table for each pack (25 MiB of bf16 averaged among four ranks: 155 us, now 136).
     if (scaled) {
       if constexpr (OP == 0) {
         if (nsrc == 1) {
-          if (ndst == 1) stream<T, OP, 1, 1, 8, true, true>(nt, src, 1, dst, 1, n, 1, scale, h);
-          else stream<T, OP, 1, 0, 4, true, true>(nt, src, 1, dst, ndst, n, 1, scale, h);
+          if (ndst == 1) stream<T, OP, FLOW, 1, 1, 8, true, true>(nt, src, 1, dst, 1, n, 1, scale, h);
+          else stream<T, OP, FLOW, 1, 0, 4, true, true>(nt, src, 1, dst, ndst, n, 1, scale, h);
         }
-        else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true, true>(nt, src, 2, dst, 1, n, scaled, scale, h);
-        else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true, true>(nt, src, 2, dst, 2, n, scaled, scale, h);
-        else if (nsrc <= 4) stream<T, OP, 4, 0, 2, false, true>(nt, src, nsrc, dst, ndst, n, scaled, scale, h);
-        else stream<T, OP, kMaxActionPeers + 1, 0, 1, false, true>(nt, src, nsrc, dst, ndst, n, scaled, scale, h);
+        else if (nsrc == 2 && ndst == 1) stream<T, OP, FLOW, 2, 1, 4, true, true>(nt, src, 2, dst, 1, n, scaled, scale, h);
+        else if (nsrc == 2 && ndst == 2) stream<T, OP, FLOW, 2, 2, 4, true, true>(nt, src, 2, dst, 2, n, scaled, scale, h);
+        else if (nsrc <= 4) stream<T, OP, FLOW, 4, 0, 2, false, true>(nt, src, nsrc, dst, ndst, n, scaled, scale, h);
+        else stream<T, OP, FLOW, kMaxActionPeers + 1, 0, 1, false, true>(nt, src, nsrc, dst, ndst, n, scaled, scale, h);
       }
     }
-    else if (nsrc == 2 && ndst == 1) stream<T, OP, 2, 1, 4, true>(nt, src, 2, dst, 1, n, 0, scale, h);
-    else if (nsrc == 2 && ndst == 2) stream<T, OP, 2, 2, 4, true>(nt, src, 2, dst, 2, n, 0, scale, h);
-    else if (nsrc == 4) stream<T, OP, 4, 0, 2, true>(nt, src, 4, dst, ndst, n, 0, scale, h);
-    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, kMaxActionPeers + 1, 0, 1, true>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
-    else if (nsrc < 4) stream<T, OP, 4, 0, 2, false>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
-    else stream<T, OP, kMaxActionPeers + 1, 0, 1, false>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
+    else if (nsrc == 2 && ndst == 1) stream<T, OP, FLOW, 2, 1, 4, true>(nt, src, 2, dst, 1, n, 0, scale, h);
+    else if (nsrc == 2 && ndst == 2) stream<T, OP, FLOW, 2, 2, 4, true>(nt, src, 2, dst, 2, n, 0, scale, h);
+    else if (nsrc == 4) stream<T, OP, FLOW, 4, 0, 2, true>(nt, src, 4, dst, ndst, n, 0, scale, h);
+    else if (nsrc == kMaxActionPeers + 1) stream<T, OP, FLOW, kMaxActionPeers + 1, 0, 1, true>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
+    else if (nsrc < 4) stream<T, OP, FLOW, 4, 0, 2, false>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
+    else stream<T, OP, FLOW, kMaxActionPeers + 1, 0, 1, false>(nt, src, nsrc, dst, ndst, n, 0, scale, h);
   }
 }
 
@@ -291,7 +295,7 @@ static __device__ __noinline__ void store_part(char* p, const uint4 v, int from,
   union { uint4 v; unsigned char b[16]; } u; u.v = v;
   for (int i = from; i < to; i++) reinterpret_cast<unsigned char*>(p)[i] = u.b[i];
 }
-// The same movement where sources or the local destination (dst[local_dst]) are at any byte address: an unaligned source is read as the
+// The same movement where sources or destinations are at any byte address: an unaligned source is read as the
 // two aligned words around each pack, an unaligned destination is written as aligned
 // words too, put together from a lane's pack and the one before it.  Only the two ends of the run of packs that a warp
 // writes (2 to 8 blocks of 512 bytes) go out in bytes.  (1 MiB blocks at odd
@@ -325,9 +329,10 @@ __device__ __forceinline__ uint4 run_pack(const RunWords<RUN>& r, int u, int m, 
 }
 // Packs o[] of a run to every destination.
 template <int RUN>
-__device__ __forceinline__ void store_run(const uint4 (&o)[RUN], int ndst, char* const* dst, int local_dst, int dm, long long run, int lane, long long npack) {
+__device__ __forceinline__ void store_run(const uint4 (&o)[RUN], int ndst, char* const* dst, long long run, int lane, long long npack) {
   for (int d = 0; d < ndst; d++) {
-    if (d != local_dst || dm == 0) {
+    const int dm = address_mod(dst[d]);
+    if (dm == 0) {
 #pragma unroll
       for (int u = 0; u < RUN; u++) { const long long p = run + u * 32 + lane; if (p < npack) st_vec(dst[d] + p * 16, o[u]); }
       continue;
@@ -352,17 +357,16 @@ __device__ __forceinline__ void store_run(const uint4 (&o)[RUN], int ndst, char*
   }
 }
 template <typename T, int OP, int RUN>
-__device__ __noinline__ void copy_shift(int nt, const char* src, int ndst, char* const* dst, int local_dst, long long npack) {
+__device__ __noinline__ void copy_shift(int nt, const char* src, int ndst, char* const* dst, long long npack) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = nt >> 5;
   char* one[1] = {dst[0]};
-  int dm = local_dst >= 0 ? address_mod(dst[local_dst]) : 0;
-  if (ndst == 1 && dm) {                               // (a shift for the source and one for the destination: all-gather of 4 x 1 MiB 20.5 us)  One destination: its whole words, for which one shift will do, and the bytes at both ends
-    const int head = 16 - dm;
+  if (ndst == 1 && address_mod(dst[0])) {                               // (a shift for the source and one for the destination: all-gather of 4 x 1 MiB 20.5 us)  One destination: its whole words, for which one shift will do, and the bytes at both ends
+    const int head = 16 - address_mod(dst[0]);
     if (warp == nwarp - 1 && lane < 16) {
-      const long long at = lane < head ? lane : npack * 16 - 16 + lane;      // (the last dm bytes are the words' remainder)
+      const long long at = lane < head ? lane : npack * 16 - 16 + lane;      // (the last bytes are the words' remainder)
       one[0][at] = *reinterpret_cast<const volatile char*>(src + at);
     }
-    src += head; one[0] += head; npack -= 1; dm = 0; dst = one;
+    src += head; one[0] += head; npack -= 1; dst = one;
   }
   const int m = address_mod(src);
   for (long long run = (long long)warp * (32 * RUN); run < npack; run += (long long)nwarp * (32 * RUN)) {
@@ -371,15 +375,14 @@ __device__ __noinline__ void copy_shift(int nt, const char* src, int ndst, char*
     uint4 o[RUN];
 #pragma unroll
     for (int u = 0; u < RUN; u++) o[u] = run_pack(r, u, m, lane);
-    store_run<RUN>(o, ndst, dst, local_dst, dm, run, lane, npack);
+    store_run<RUN>(o, ndst, dst, run, lane, npack);
   }
 }
 template <typename T, int OP, int RUN>
-__device__ __noinline__ void reduce_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
+__device__ __noinline__ void reduce_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, long long npack, int scaled, float scale) {
   typedef typename AccOf<T>::type A;
   constexpr int N = Pack<T>::N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = nt >> 5;
-  const int dm = local_dst >= 0 ? address_mod(dst[local_dst]) : 0;
   for (long long run = (long long)warp * (32 * RUN); run < npack; run += (long long)nwarp * (32 * RUN)) {
     A acc[RUN][N];
     auto operand = [&](const RunWords<RUN>& r, int u, int s, int m, A (&x)[N]) {
@@ -419,20 +422,20 @@ __device__ __noinline__ void reduce_shift(int nt, int nsrc, const char* const* s
     uint4 o[RUN];
 #pragma unroll
     for (int u = 0; u < RUN; u++) o[u] = Pack<T>::down(acc[u]);
-    store_run<RUN>(o, ndst, dst, local_dst, dm, run, lane, npack);
+    store_run<RUN>(o, ndst, dst, run, lane, npack);
   }
 }
 // A warp takes runs of 2, 4 or 8 blocks (sums: 2 or 4): as few rounds as can be, and then over as many warps.
 template <typename T, int OP>
-__device__ __forceinline__ void reduce_copy_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, int local_dst, long long npack, int scaled, float scale) {
+__device__ __forceinline__ void reduce_copy_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, long long npack, int scaled, float scale) {
   const long long blocks = (npack + nt - 1) / nt;      // per warp
   if (OP == OP_COPY || (nsrc == 1 && !scaled)) {
-    if (blocks > 4) copy_shift<T, OP, 8>(nt, src[0], ndst, dst, local_dst, npack);
-    else if (blocks > 2) copy_shift<T, OP, 4>(nt, src[0], ndst, dst, local_dst, npack);
-    else copy_shift<T, OP, 2>(nt, src[0], ndst, dst, local_dst, npack);
+    if (blocks > 4) copy_shift<T, OP, 8>(nt, src[0], ndst, dst, npack);
+    else if (blocks > 2) copy_shift<T, OP, 4>(nt, src[0], ndst, dst, npack);
+    else copy_shift<T, OP, 2>(nt, src[0], ndst, dst, npack);
   } else if constexpr (OP != OP_COPY) {
-    if (blocks > 2) reduce_shift<T, OP, 4>(nt, nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
-    else reduce_shift<T, OP, 2>(nt, nsrc, src, ndst, dst, local_dst, npack, scaled, scale);
+    if (blocks > 2) reduce_shift<T, OP, 4>(nt, nsrc, src, ndst, dst, npack, scaled, scale);
+    else reduce_shift<T, OP, 2>(nt, nsrc, src, ndst, dst, npack, scaled, scale);
   }
 }
 
@@ -456,7 +459,6 @@ __device__ __noinline__ void reduce_copy_elem(int nt, int nsrc, const char* cons
 }
 
 // ---------------------------------------------------------------- the kernel
-constexpr int kSharedCache = 64;       // and their operands in other ranks' buffers
 constexpr int kSliceCache = 192;      // actions kept in shared memory, with the CTA's slice of each
 
 constexpr int kStepDepth = 4;         // steps the waiter may be ahead of the publisher
@@ -464,11 +466,9 @@ struct StepDesc {
   const char* src[kMaxActionPeers + 1];      // operands in rank order: receive peers below me, my own buffer, receive peers above me
   char* dst[kMaxActionPeers + 1];            // local destination first, then the send peers
   long long len;                             // elements
-  long long position;                        // in the rank's walk (step_position)
   int action, nsrc, ndst, local_src, local_dst, flags;
-  int scaled;                                // operands to scale (scale_operand)
 };
-enum : int { STEP_ALIGNED = 2, STEP_LOCAL_DEP = 4, STEP_FAIL = 8, STEP_END = 16, STEP_SRC_DONE = 32, STEP_DST_DONE = 64 };
+enum : int { STEP_SCALE = 1, STEP_ALIGNED = 2, STEP_LOCAL_DEP = 4, STEP_FAIL = 8, STEP_END = 16, STEP_SRC_DONE = 32, STEP_DST_DONE = 64 };
 __device__ __forceinline__ void bar_sync_n(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive_n(int id, int n) { __threadfence_block(); asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
@@ -476,7 +476,7 @@ __device__ __forceinline__ void bar_arrive_n(int id, int n) { __threadfence_bloc
 // 15 % in registers).
 template <typename T, int OP, bool SHIFT>
 __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const KernelArgs ka) {
-  const int launched = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta, vr = ka.working[launched];
+  const int vr = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta;
   const LaunchRank& L = ka.r[vr];
   RankCtx* __restrict__ ctx = L.ctx;
   const int tid = threadIdx.x, lane = tid & 31, ndata = (int)blockDim.x - kCtlThreads;
@@ -488,14 +488,11 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   __shared__ Action s_act[kSliceCache];
   __shared__ int s_maxseg;
   __shared__ volatile int s_published;             // steps whose descriptor may be used again
-  __shared__ SharedOps s_shared[kSharedCache];
-  __shared__ const char *s_in[kMaxVRanks], *s_out[kMaxVRanks], *s_kept[2];      // all ranks' buffers; the slots of a window's entries that this rank reads again
 
   // everything read from the context more than once is fetched once, in parallel
   const int rank = ctx->rank, nranks = ctx->nranks, max_cta = ctx->max_cta;
-  const long long tail_off = ctx->tail_off, head_off = ctx->head_off, fifo_off = ctx->fifo_off, scratch_off = ctx->scratch_off, prog_off = ctx->prog_off, chan_bytes = ctx->nslot * ctx->slot_bytes;
+  const long long tail_off = ctx->tail_off, head_off = ctx->head_off, fifo_off = ctx->fifo_off, scratch_off = ctx->scratch_off, chan_bytes = ctx->nslot * ctx->slot_bytes;
   if (tid < nranks) s_heap[tid] = ctx->heap[tid];
-  if (tid < ka.n_vrank) { s_in[tid] = (const char*)ka.r[tid].in; s_out[tid] = (const char*)ka.r[tid].out; }
   if (tid == 0) { s_maxseg = 0; s_published = 0; }
   __syncthreads();
   const long long seg_bytes = ka.seg_bytes, seg_elems = (seg_bytes / 16) * (esz >= 16 ? 1 : 16 / esz);
@@ -505,7 +502,6 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
       const Action a = L.actions[ai];
       const Slice sl = slice_of(a.count, esz, cta, ka.n_cta, seg_bytes);
       if (ai < kSliceCache) { s_lo[ai] = sl.lo; s_hi[ai] = sl.hi; s_act[ai] = a; }
-      if (L.shared && ai < kSharedCache) s_shared[ai] = L.shared[ai];
       m = max(m, sl.nseg);
     }
     if (m) atomicMax(&s_maxseg, m);
@@ -529,12 +525,12 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
         const char* const* const src = st.src; char* const* const dst = st.dst;
         const long long len = st.len;
         const int nsrc = st.nsrc, ndst = st.ndst, local_src = st.local_src;
-        const int scaled = st.scaled;
+        const bool do_scale = flags & STEP_SCALE;
         constexpr int N = Pack<T>::N;
         const long long nfull = (SHIFT || (flags & STEP_ALIGNED)) ? len / N : 0;
-        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(ndata, nsrc, src, ndst, dst, st.local_dst, nfull, scaled, ka.scale); }
-        else if (nfull) move_aligned<T, OP>(ndata, src, nsrc, dst, ndst, (int)nfull, scaled, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
-        if (nfull * N < len) reduce_copy_elem<T, OP>(ndata, nsrc, src, local_src, ndst, dst, nfull * N, len, scaled, ka.scale);
+        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(ndata, nsrc, src, ndst, dst, nfull, do_scale ? 1 << local_src : 0, ka.scale); }
+        else if (nfull) move_aligned<T, OP, false>(ndata, src, nsrc, dst, ndst, (int)nfull, do_scale ? 1 << local_src : 0, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
+        if (nfull * N < len) reduce_copy_elem<T, OP>(ndata, nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale ? 1 << local_src : 0, ka.scale);
       }
       bar_arrive_n(kDone + d, ndata + 32);
       if (flags & (STEP_END | STEP_FAIL)) return;
@@ -550,13 +546,9 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   }
   const unsigned nslot = (unsigned)ka.nslot;
   const long long mine = (long long)(rank * max_cta + cta) * kFlagStride;      // my counters in a peer's heap
-  // progress of this CTA of every rank: all were raised by the same calls, so mine, which only I write, says where the others' began
-  const long long my_prog = prog_off + (long long)cta * kFlagStride;
-  const unsigned long long prog0 = ka.prog_total ? *reinterpret_cast<const unsigned long long*>(my_heap + my_prog) : 0;
 
   if (tid < ndata + 32) {                          // ---------------- waiter
     WaitCtx w; w.ctx = ctx; w.timeout_ns = ka.timeout_ns; w.cta = cta; w.one_gpu = ka.one_gpu;
-    unsigned long long seen_prog = 0;              // of rank `lane`
     unsigned long long seen_head[2] = {0, 0};      // what a peer had consumed when last looked: no need to look again while that is credit enough
     int k = 0;
     bool failed = false;
@@ -586,17 +578,12 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
           StepDesc& st = s_step[k % kStepDepth];
           bool ok = true;
           w.action = ai; w.segment = seg;
-          const char* const kept = ac.src_buf == BUF_KEPT ? s_kept[seg - seg0] : nullptr;
-          if (ac.keep) __syncwarp();               // (before the same step puts another one there)
-          bool aligned = true, dep = has_src && ac.src_buf != BUF_IN;      // dep: an operand that earlier steps of this CTA wrote
-          int scaled = 0;
 #pragma unroll
           for (int q = 0; q < 2; q++) {
             const int p = lane + 32 * q;
             const long long theirs = (long long)(p * max_cta + cta) * kFlagStride;      // peer p's counters in my heap
             for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) {
               st.dst[j + has_dst] = s_heap[p] + fifo_off + (long long)(rank * max_cta + cta) * chan_bytes + (long long)(sent[q] % nslot) * seg_bytes;
-              if (ac.keep && j == 0) s_kept[seg - seg0] = st.dst[j + has_dst];
               if (++sent[q] > seen_head[q] + nslot && ok)
                 ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + head_off + theirs), sent[q] - nslot, w, 1, p, &seen_head[q]);
             }
@@ -606,34 +593,15 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
               if (ok) ok = wait_counter(reinterpret_cast<const unsigned long long*>(my_heap + tail_off + theirs), rcvd[q], w, 2, p);
             }
           }
-          if (L.shared) {                          // operands in the buffers of rank `lane`
-            const SharedOps& x = ai < kSharedCache ? s_shared[ai] : L.shared[ai];
-            for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == kSharedPeer && x.from[j] == lane) {
-              const int at = j + (has_src && j >= ac.self_pos);
-              const char* const from = (x.buf[j] == BUF_IN ? s_in[lane] : x.buf[j] == BUF_OUT ? s_out[lane] : s_heap[lane] + scratch_off) + (x.off[j] + lo) * esz;
-              st.src[at] = from;
-              aligned &= (reinterpret_cast<uintptr_t>(from) & 15) == 0;
-              dep |= lane == rank && x.after[j] >= 0;
-              if (x.scaled >> j & 1) scaled |= (lane == rank ? 1 : 1 | 1 << kRoundedShift) << at;
-              const unsigned long long want = prog0 + (unsigned long long)step_position(seg0, seg, x.after[j], ka.prog_actions, ka.window);
-              if (x.after[j] >= 0 && lane != rank && want > seen_prog && ok)
-                ok = wait_counter(reinterpret_cast<const unsigned long long*>(s_heap[lane] + my_prog), want, w, 2, lane, &seen_prog);
-            }
-            aligned = __all_sync(0xffffffffu, aligned); dep = __any_sync(0xffffffffu, dep);
-            scaled = __reduce_or_sync(0xffffffffu, scaled);
-          }
           ok = __all_sync(0xffffffffu, ok);
           if (lane == 0) {
             const char* lsrc = nullptr; char* ldst = nullptr;
-            if (has_src) { lsrc = kept ? kept : (ac.src_buf == BUF_IN ? (const char*)L.in : ac.src_buf == BUF_OUT ? (const char*)L.out : my_heap + scratch_off) + (ac.src_off + lo) * esz; st.src[ac.self_pos] = lsrc; }
+            if (has_src) { lsrc = (ac.src_buf == BUF_IN ? (const char*)L.in : ac.src_buf == BUF_OUT ? (const char*)L.out : my_heap + scratch_off) + (ac.src_off + lo) * esz; st.src[ac.self_pos] = lsrc; }
             if (has_dst) { ldst = (ac.dst_buf == BUF_OUT ? (char*)L.out : my_heap + scratch_off) + (ac.dst_off + lo) * esz; st.dst[0] = ldst; }
             st.len = (lo + seg_elems < sl_hi ? lo + seg_elems : sl_hi) - lo;
             st.action = ai; st.nsrc = ac.n_recv + has_src; st.ndst = ac.n_send + has_dst; st.local_src = has_src ? ac.self_pos : -1; st.local_dst = has_dst ? 0 : -1;
-            if ((ac.flags & ACT_SCALE_SRC) && has_src) scaled |= 1 << ac.self_pos;
-            st.scaled = ka.avg ? scaled : 0;
-            st.position = step_position(seg0, seg, ai, ka.prog_actions, ka.window);
-            st.flags = ((aligned ? (reinterpret_cast<uintptr_t>(lsrc) | reinterpret_cast<uintptr_t>(ldst)) & 15 : 1) == 0 ? STEP_ALIGNED : 0) |
-                       (dep ? STEP_LOCAL_DEP : 0) | ((ka.leave_first & 1) && (ac.flags & ACT_SRC_DONE) ? STEP_SRC_DONE : 0) | ((ka.leave_first & 2) && (ac.flags & ACT_DST_DONE) ? STEP_DST_DONE : 0) | (ok ? 0 : STEP_FAIL);
+            st.flags = (ka.avg && (ac.flags & ACT_SCALE_SRC) && has_src ? STEP_SCALE : 0) | (((reinterpret_cast<uintptr_t>(lsrc) | reinterpret_cast<uintptr_t>(ldst)) & 15) == 0 ? STEP_ALIGNED : 0) |
+                       (has_src && ac.src_buf != BUF_IN ? STEP_LOCAL_DEP : 0) | ((ka.leave_first & 1) && (ac.flags & ACT_SRC_DONE) ? STEP_SRC_DONE : 0) | ((ka.leave_first & 2) && (ac.flags & ACT_DST_DONE) ? STEP_DST_DONE : 0) | (ok ? 0 : STEP_FAIL);
           }
           __syncwarp();
           bar_arrive_n(kReady + k % kStepDepth, ndata + 32);
@@ -668,7 +636,6 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
       for (int j = 0; j < ac.n_send; j++) if (ac.send_peer[j] == p) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[p] + tail_off + mine), ++sent[q], ka.one_gpu);
       for (int j = 0; j < ac.n_recv; j++) if (ac.recv_peer[j] == p) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[p] + head_off + mine), ++rcvd[q], ka.one_gpu);
     }
-    if (ka.prog_total && lane == 0) st_relaxed(reinterpret_cast<unsigned long long*>(my_heap + my_prog), prog0 + (unsigned long long)s_step[d].position, ka.one_gpu);
     __syncwarp();
     if (lane == 0) { __threadfence_block(); s_published = k + 1; }
   }
@@ -676,11 +643,6 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
   for (int q = 0; q < 2; q++) {
     const int p = lane + 32 * q;
     if (p < nranks) { ctx->sent[p * max_cta + cta] = sent[q]; ctx->rcvd[p * max_cta + cta] = rcvd[q]; }
-  }
-  if (ka.prog_total) {                               // the first rank also counts for those that have nothing to do
-    bool raise = lane == rank;
-    if (launched == 0 && lane < ka.n_vrank) raise |= ka.r[lane].n_actions == 0;
-    if (raise) st_relaxed(reinterpret_cast<unsigned long long*>(s_heap[lane] + my_prog), prog0 + (unsigned long long)ka.prog_total, ka.one_gpu);
   }
 }
 

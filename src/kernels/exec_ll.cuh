@@ -9,7 +9,7 @@
 // and the region is zero at start, so stale lines can never look complete.
 #pragma once
 #include "exec_impl.cuh"
-#include "exec_flat.cuh"
+#include "exec_flow.cuh"
 
 namespace piccl {
 
@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
   typedef typename AccOf<T>::type A;
   constexpr int E = LLUnit<T>::E;
   constexpr int esz = (int)sizeof(T);
-  const int vr = ka.working[blockIdx.x / ka.n_cta], cta = blockIdx.x % ka.n_cta;
+  const int vr = blockIdx.x / ka.n_cta, cta = blockIdx.x % ka.n_cta;
   const LaunchRank& L = ka.r[vr];
   RankCtx* __restrict__ ctx = L.ctx;
   const int tid = threadIdx.x;
@@ -33,15 +33,12 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
   __shared__ long long s_lo[kSliceCache], s_hi[kSliceCache];
   __shared__ char* s_heap[kMaxRanks];
   __shared__ Action s_act[kSliceCache];
-  __shared__ SharedOps s_shared[kSharedCache];
-  __shared__ const char *s_in[kMaxVRanks], *s_out[kMaxVRanks];      // all ranks' buffers
   __shared__ int s_maxseg;
 
   const int rank = ctx->rank, nranks = ctx->nranks;
   const long long llf_off = ctx->llf_off, llf_head_off = ctx->llf_head_off, scratch_off = ctx->scratch_off;
   unsigned long long my_sent = 0, my_rcvd = 0, seen_head = 0;      // seen_head: what peer `tid` had consumed when last looked
   if (tid < nranks) { s_heap[tid] = ctx->heap[tid]; my_sent = ctx->sent_ll[tid * kLLFifoCta + cta]; my_rcvd = ctx->rcvd_ll[tid * kLLFifoCta + cta]; }
-  if (tid < ka.n_vrank) { s_in[tid] = (const char*)ka.r[tid].in; s_out[tid] = (const char*)ka.r[tid].out; }
   if (tid == 0) { s_maxseg = 0; s_credit[0] = s_credit[1] = 0; }
   __syncthreads();
   constexpr long long kPayload = kLLFifoSlotBytes / 2;
@@ -53,7 +50,6 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
       const Action a = L.actions[ai];
       const Slice sl = slice_of(a.count, esz, cta, ka.n_cta, kPayload);
       if (ai < kSliceCache) { s_act[ai] = a; s_lo[ai] = sl.lo; s_hi[ai] = sl.hi; }
-      if (L.shared && ai < kSharedCache) s_shared[ai] = L.shared[ai];
       m = max(m, sl.nseg);
     }
     if (m) atomicMax(&s_maxseg, m);
@@ -72,9 +68,9 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
     freed = false;
   };
 
-  // One barrier to an action: behind it all threads are done with the action before, whose slots are given back then, beside this action's polling.  With a second
-  // one after the data, slices worked out anew and the heads read for every entry, and values handed on hop by hop: all-reduce of 4 KiB on the ring, eight ranks 37.8 us, now 28.7, four 18.5
-  // and 14.4; reduce-scatter of 8 KiB blocks, four ranks, 12.3 and 10.3.  What is left is three microseconds a hop: a line's way through the L2 and the poll that sees it.
+  // One barrier to an action: behind it all threads are done with the action before, whose slots are given back then, beside this action's polling.  (With a second one after the
+  // data, slices worked out anew and the heads read for every entry, all through the slots: all-reduce of 4 KiB on the ring, eight ranks, 38.9 us, now 28.5, of 16 KiB among four 19.4
+  // and 14.4; all-gather of 16 KiB by PRM, eight ranks, 30.3 and 22.6; reduce-scatter of 8 KiB, four ranks, 12.4 and 10.8.)  What is left is a line's way through the L2 and the poll that sees it.
   bool over = false;                                   // given up, by all threads
   for (int seg = 0; seg < maxseg && !over; seg++) {
     for (int ai = 0; ai < L.n_actions; ai++) {
@@ -117,7 +113,6 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
       const T* lsrc = nullptr; T* ldst = nullptr;
       if (has_src) lsrc = reinterpret_cast<const T*>(ac.src_buf == BUF_IN ? (const char*)L.in : ac.src_buf == BUF_OUT ? (const char*)L.out : my_heap + scratch_off) + ac.src_off + lo;
       if (ac.dst_buf != BUF_NONE) ldst = reinterpret_cast<T*>(ac.dst_buf == BUF_OUT ? (char*)L.out : my_heap + scratch_off) + ac.dst_off + lo;
-      const SharedOps* const x = L.shared ? (ai < kSharedCache ? s_shared + ai : L.shared + ai) : nullptr;
       const int do_scale = ka.avg && (ac.flags & ACT_SCALE_SRC) && has_src ? 1 : 0;
       const long long nunits = (len + E - 1) / E;
       // a unit of a buffer, in one load where it is whole and stands at a multiple of its size
@@ -146,15 +141,6 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
           }
           if (j == ac.n_recv) break;
           const int p = ac.recv_peer[j];
-          if (p == kSharedPeer) {                      // in rank x->from[j]'s buffer since before the call
-            const T* const from = reinterpret_cast<const T*>(x->buf[j] == BUF_IN ? s_in[x->from[j]] : s_out[x->from[j]]) + x->off[j] + lo;
-            A v[E];
-            load_unit(from, u, (reinterpret_cast<uintptr_t>(from) & 7) == 0, ka.avg && (x->scaled >> j & 1) ? (x->from[j] == rank ? 1 : 1 | 1 << kRoundedShift) : 0, v);
-#pragma unroll
-            for (int e = 0; e < E; e++) acc[e] = have ? red<OP, A>(acc[e], v[e]) : v[e];
-            have = true;
-            continue;
-          }
           const unsigned seq = s_recv_seq[p];
           const char* src = my_heap + llf_off + ((long long)(p * kLLFifoCta + cta) * kLLFifoSlots + (seq - 1) % kLLFifoSlots) * kLLFifoSlotBytes + u * 16;
           uint4 line;
@@ -210,7 +196,7 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
   namespace piccl {                                                                                \
   ExecKernelFn exec_table_##DT[4] = {exec_kernel<T, 0, false>, exec_kernel<T, 1, false>, exec_kernel<T, 2, false>, exec_kernel<T, 3, false>}; \
   ExecKernelFn exec_shift_table_##DT[4] = {exec_kernel<T, 0, true>, exec_kernel<T, 1, true>, exec_kernel<T, 2, true>, exec_kernel<T, 3, true>}; \
-  ExecKernelFn exec_flat_table_##DT[8] = {exec_flat_kernel<T, 0, false>, exec_flat_kernel<T, 1, false>, exec_flat_kernel<T, 2, false>, exec_flat_kernel<T, 3, false>,              \
-                                          exec_flat_kernel<T, 0, true>, exec_flat_kernel<T, 1, true>, exec_flat_kernel<T, 2, true>, exec_flat_kernel<T, 3, true>};               \
+  FlowKernelFn exec_flow_table_##DT[8] = {exec_flow_kernel<T, 0, false>, exec_flow_kernel<T, 1, false>, exec_flow_kernel<T, 2, false>, exec_flow_kernel<T, 3, false>,              \
+                                          exec_flow_kernel<T, 0, true>, exec_flow_kernel<T, 1, true>, exec_flow_kernel<T, 2, true>, exec_flow_kernel<T, 3, true>};               \
   ExecKernelFn exec_ll_table_##DT[4] = {exec_ll_kernel<T, 0>, exec_ll_kernel<T, 1>, exec_ll_kernel<T, 2>, exec_ll_kernel<T, 3>}; \
   }

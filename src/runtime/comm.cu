@@ -96,7 +96,7 @@ int piccl_comm_create(int rank, int nranks, int device, const piccl_config_t* us
   if (cfg.tp_bytes <= 0) cfg.tp_bytes = (long long)e.tp_mb << 20;
   c->cfg.tp_bytes = cfg.tp_bytes;
   const long long tp_flags = cfg.tp_bytes > 0 ? (1 << 20) : 0;
-  x.tail_off = 0; x.head_off = flags; x.prog_off = 2 * flags; x.ll_off = x.prog_off + round_up((long long)cfg.max_cta * kFlagStride, 4096); x.tp_flag_off = x.ll_off + ll_bytes;
+  x.tail_off = 0; x.head_off = flags; x.ll_off = 2 * flags; x.tp_flag_off = x.ll_off + ll_bytes;
   // low-latency FIFO of the executor (all collectives, small messages): head counters, then the lines
   x.llf_head_off = x.tp_flag_off + tp_flags;
   x.llf_off = x.llf_head_off + round_up((long long)nranks * kLLFifoCta * kFlagStride, 4096);
@@ -286,9 +286,8 @@ namespace piccl {
 
 struct CallDesc { Coll coll; const void* send; void* recv; size_t count; int dtype, op, root; Algo algo; int k; };
 
-static int upload_program(piccl_comm* c, const Program& p, cudaStream_t stream, ProgEntry& e, const std::vector<SharedOps>* shared = nullptr) {
-  const size_t act_bytes = p.actions.size() * sizeof(Action), sh_bytes = shared ? shared->size() * sizeof(SharedOps) : 0;
-  size_t bytes = std::max<size_t>(act_bytes + sh_bytes, sizeof(Action));
+// `bytes` of `data` on the device; they stay as long as the communicator.
+static int upload(piccl_comm* c, const void* data, size_t data_bytes, size_t bytes, cudaStream_t stream, ProgEntry& e, const void** dev) {
   bytes = (bytes + 255) / 256 * 256;
   if (c->chunks.empty() || c->chunks.back().used + bytes > c->chunks.back().cap) {
     ProgChunk ch; ch.cap = std::max<size_t>(1 << 20, bytes); ch.used = 0;
@@ -298,15 +297,29 @@ static int upload_program(piccl_comm* c, const Program& p, cudaStream_t stream, 
     c->chunks.push_back(ch);
   }
   ProgChunk& ch = c->chunks.back();
-  memcpy(ch.host + ch.used, p.actions.data(), act_bytes);
-  if (sh_bytes) memcpy(ch.host + ch.used + act_bytes, shared->data(), sh_bytes);
-  e.dev = reinterpret_cast<const Action*>(ch.dev + ch.used);
-  if (sh_bytes) e.dev_shared = reinterpret_cast<const SharedOps*>(ch.dev + ch.used + act_bytes);
-  e.n_actions = (int)p.actions.size(); for (const Action& ac : p.actions) e.most = std::max<long long>(e.most, ac.count); e.scratch_elems = p.scratch_elems; e.origin = stream; e.synced = false;
-  if (!p.actions.empty()) CUDA_TRY(cudaMemcpyAsync(ch.dev + ch.used, ch.host + ch.used, act_bytes + sh_bytes, cudaMemcpyHostToDevice, stream));
+  memcpy(ch.host + ch.used, data, data_bytes);
+  *dev = ch.dev + ch.used; e.origin = stream; e.synced = false;
+  if (data_bytes) CUDA_TRY(cudaMemcpyAsync(ch.dev + ch.used, ch.host + ch.used, data_bytes, cudaMemcpyHostToDevice, stream));
   CUDA_TRY(cudaEventCreateWithFlags(&e.ready, cudaEventDisableTiming));
   CUDA_TRY(cudaEventRecord(e.ready, stream));
   ch.used += bytes;
+  return PICCL_OK;
+}
+static int upload_program(piccl_comm* c, const Program& p, cudaStream_t stream, ProgEntry& e) {
+  const void* dev = nullptr;
+  const int rc = upload(c, p.actions.data(), p.actions.size() * sizeof(Action), std::max<size_t>(p.actions.size(), 1) * sizeof(Action), stream, e, &dev);
+  e.dev = static_cast<const Action*>(dev); e.n_actions = (int)p.actions.size(); e.scratch_elems = p.scratch_elems;
+  return rc;
+}
+// The entry's upload is done, or `stream` waits for it.
+static int after_upload(ProgEntry& e, cudaStream_t stream) {
+  if (e.synced) return PICCL_OK;
+  // Asked first, and in the relaxed mode: a stream in capture cannot wait for an upload outside it, and a question in the global mode would end the capture.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (cudaEventQuery(e.ready) == cudaSuccess) e.synced = true; else cudaGetLastError();
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!e.synced && e.origin != stream) CUDA_TRY(cudaStreamWaitEvent(stream, e.ready, 0));
   return PICCL_OK;
 }
 
@@ -330,14 +343,8 @@ static const char* check_program(const Program& p, const CollArgs& a, long long 
   return nullptr;
 }
 
-// The programs of all ranks of a launch that read each other's buffers, compiled when the first of them is not in its cache.
-struct GroupPrograms { bool lines = false, made = false, flat = false; std::vector<Program> progs; std::vector<std::vector<SharedOps>> shared; };
-
-static ProgKey key_of(const CollArgs& a, int shared) { return ProgKey{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, a.block_stride, shared}; }
-
-// group: the program as share_operands or share_lines makes it; the other one is kept beside it, for a captured call whose buffers overlap.
-static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, const ProgEntry** out, GroupPrograms* group = nullptr) {
-  const ProgKey k = key_of(a, !group ? 0 : group->lines ? 2 : 1);
+static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, const ProgEntry** out) {
+  ProgKey k{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, a.block_stride};
   auto it = c->cache.find(k);
   if (it == c->cache.end()) {
     // A new program needs device and pinned memory and an upload on the caller's stream: not inside a stream capture (an
@@ -356,47 +363,27 @@ static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, co
       c->stats.fallbacks++;
       return fail(PICCL_UNSUPPORTED, "program cache full (%zu MiB for %zu distinct calls)", held >> 20, c->cache.size());
     }
-    if (group) {
-      const ProgEntry* plain = nullptr;
-      if (int rc = get_program(c, a, stream, &plain)) return rc;
-      if (!group->made) {
-        group->made = true;
-        for (int r = 0; r < a.nranks; r++) group->progs.push_back(compile(a, r));
-        if (!(group->lines ? share_lines(group->progs, group->shared) : share_operands(group->progs, group->shared))) group->shared.clear();
-        else group->flat = nothing_waits(group->progs, group->shared);
-      }
-    } else c->stats.program_cache_misses++;
-    Program p = group ? std::move(group->progs[c->rank]) : compile(a, c->rank);
-    if (env().debug && !group) {
+    c->stats.program_cache_misses++;
+    Program p = compile(a, c->rank);
+    if (env().debug) {
       if (const char* why = check_program(p, a, c->h_ctx.scratch_bytes / std::max(1, a.elem_size)))
         return fail(PICCL_INTERNAL_ERROR, "program check failed (%s %s, rank %d): %s", coll_name(a.coll), algo_name(a.algo), c->rank, why);
     }
     ProgEntry e;
     for (const Action& ac : p.actions) e.offsets_aligned &= (ac.src_off * a.elem_size) % 16 == 0 && (ac.dst_off * a.elem_size) % 16 == 0;
-    e.flat = group && group->flat;
-    const std::vector<SharedOps>* sh = group && !group->shared.empty() ? &group->shared[c->rank] : nullptr;
-    if (sh) for (size_t i = 0; i < sh->size(); i++) for (int j = 0; j < p.actions[i].n_recv; j++) e.offsets_aligned &= (*sh)[i].off[j] * a.elem_size % 16 == 0;
-    int rc = upload_program(c, p, stream, e, sh); if (rc) return rc;
+    int rc = upload_program(c, p, stream, e); if (rc) return rc;
     it = c->cache.emplace(k, e).first;
   } else {
     c->stats.program_cache_hits++;
-    ProgEntry& e = it->second;
-    if (!e.synced) {
-      // Asked first, and in the relaxed mode: a stream in capture cannot wait for an upload outside it, and a question in the global mode would end the capture.
-      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-      cudaThreadExchangeStreamCaptureMode(&mode);
-      if (cudaEventQuery(e.ready) == cudaSuccess) e.synced = true; else cudaGetLastError();
-      cudaThreadExchangeStreamCaptureMode(&mode);
-      if (!e.synced && e.origin != stream) CUDA_TRY(cudaStreamWaitEvent(stream, e.ready, 0));
-    }
+    if (int rc = after_upload(it->second, stream)) return rc;
   }
   *out = &it->second;
   return PICCL_OK;
 }
 
-// May the ranks of this launch read each other's buffers (share.cc)?  All of them in one launch on one GPU; no receive buffer may overlap another rank's buffers, or,
-// but for an all-gather or broadcast in place, which never write what others read, its own send buffer: a rank could overwrite what another is still to read.
-static bool may_share(piccl_comm** comms, int n, const CallDesc* calls, long long bytes) {
+// May this launch run the call's data flow (flow.cc) in place of the ranks' programs?  All ranks in one launch on one GPU; no receive buffer may overlap another rank's buffers, or,
+// but for an all-gather or broadcast in place, which never write what others read, its own send buffer: an operation could overwrite what another is still to read.
+static bool may_flow(piccl_comm** comms, int n, const CallDesc* calls, long long bytes) {
   const CallDesc& d0 = calls[0];
   if (n != comms[0]->nranks || n < 2) return false;
   struct Span { const char *lo, *hi; } in[kMaxVRanks], out[kMaxVRanks];
@@ -424,8 +411,7 @@ static bool may_share(piccl_comm** comms, int n, const CallDesc* calls, long lon
 // All ranks compute the same number from the same arguments.  The reference's grid formula
 // grid = clamp(count / block, MIN, MAX) (src/kernels/permutation_kernel.cu:76-77) is kept when
 // PICCL_MIN/MAX_GRID_SIZE are set; the result is capped by the FIFO channel count.
-// n_working of the n_vrank ranks of the launch have CTAs.
-static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_working, int n_vrank) {
+static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_vrank) {
   long long bytes = a.count * a.elem_size;
   if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) bytes /= std::max(1, a.nranks);
   if (a.algo == ALGO_DIRECT && a.coll != COLL_ALLGATHER && a.coll != COLL_REDUCE_SCATTER) bytes /= std::max(1, a.coll == COLL_ALLREDUCE ? a.nranks : a.nranks - 1);
@@ -439,7 +425,7 @@ static int choose_cta(const piccl_comm* c, const CollArgs& a, int n_working, int
     n = std::max<long long>(e.min_grid_set ? e.min_grid : 1, std::min<long long>(e.max_grid_set ? e.max_grid : g, g));
   }
   n = std::max<long long>(1, std::min<long long>(n, c->cfg.max_cta));
-  if (n_vrank > 1) n = std::min<long long>(n, std::max(1, c->sm_count / n_working));
+  if (n_vrank > 1) n = std::min<long long>(n, std::max(1, c->sm_count / n_vrank));
   return (int)n;
 }
 
@@ -487,23 +473,6 @@ static void cut_fifo(const piccl_comm* c, int n_vrank, int n_cta, const CollArgs
   const long long seg = std::min<long long>(round_up((slice + 1) / 2, round), std::max<long long>(round, 131072 / round * round));
   ka->nslot = 4; ka->window = window_of(4);
   ka->seg_bytes = std::max<long long>(16, std::min<long long>(seg, chan / 4 / 16 * 16));
-}
-
-// Slices to an action where nothing waits: blocks of 4 KiB, one 16-byte pack a thread, while there are SMs for more of them, and no larger than 64 KiB, so that
-// the last wave is short.  us, executor (which reads at the origin too) and this: all-gather 4 x 1 MiB at odd addresses 18.4 / 10.4, 8 x 8 MiB 147 / 97.5, 4 x 16 MiB 81 / 55, 4 x 4 KiB 12.3 / 6.6;
-// broadcast 8 x 16 MiB 41 / 26.7; reduce-scatter 2 x 32 MiB 41 / 33; all-reduce in one exchange 4 x 32 MiB 83 / 52, 2 x 4 MB 11.3 / 6.1.
-static int flat_slices(const piccl_comm* c, long long bytes, long long actions, long long* slice_bytes) {
-  const long long even = (actions * bytes / (12LL * c->sm_count) + 4095) / 4096 * 4096;
-  *slice_bytes = std::max<long long>(4096, std::min<long long>(65536, even));
-  return (int)std::max<long long>(1, (bytes + *slice_bytes - 1) / *slice_bytes);
-}
-static cudaError_t launch_flat(ExecKernelFn f, long long blocks, void** args, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)std::max<long long>(1, blocks)); cfg.blockDim = dim3(kFlatBlock); cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  return cudaLaunchKernelExC(&cfg, (const void*)f, args);
 }
 
 static bool fault_now(piccl_comm* c) {
@@ -555,6 +524,83 @@ static bool ll_plan(piccl_comm** comms, int n, Algo algo, int k, LLArgs* out) {
   c0->ll_plans.push_back(p);
   if (p.usable) *out = p.args;
   return p.usable;
+}
+
+// Slices to an operation: blocks of 4 KiB, one 16-byte pack a thread, while there are SMs for more of them, and no larger than 64 KiB, so that the last wave is short (figures in flow.cc).
+static int flow_slices(const piccl_comm* c, long long bytes, long long ops, long long* slice_bytes) {
+  const long long even = (ops * bytes / (12LL * c->sm_count) + 4095) / 4096 * 4096;
+  *slice_bytes = std::max<long long>(4096, std::min<long long>(65536, even));
+  return (int)std::max<long long>(1, (bytes + *slice_bytes - 1) / *slice_bytes);
+}
+
+// The call's data flow, all ranks in this launch.  PICCL_UNSUPPORTED: nothing was done, the ranks' programs are to run.
+static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long count, int esz, int op, bool avg, bool capturing, cudaStream_t stream) {
+  piccl_comm* c0 = comms[0];
+  const CallDesc& d0 = calls[0];
+  const bool reducing = d0.coll == COLL_ALLREDUCE || d0.coll == COLL_REDUCE || d0.coll == COLL_REDUCE_SCATTER;
+  CollArgs a; a.coll = d0.coll; a.algo = d0.algo; a.k = d0.k; a.nranks = n; a.root = d0.root; a.count = count; a.elem_size = esz;
+  a.in_place = !reducing && d0.send == d0.recv;              // (an all-gather's rank 0: its block is the buffer's first; may_flow: all ranks or none)
+  ProgKey k{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, 0};
+  k.flow = 1;
+  ProgEntry* e = nullptr;
+  {
+    std::lock_guard<std::mutex> l(c0->mu);
+    auto it = c0->cache.find(k);
+    if (it == c0->cache.end()) {
+      size_t held = 0;
+      for (const auto& ch : c0->chunks) held += ch.cap;
+      if (capturing || held > ((size_t)256 << 20)) return PICCL_UNSUPPORTED;      // (the programs' path says why)
+      std::vector<Program> progs;
+      for (int r = 0; r < n; r++) progs.push_back(compile(a, r));
+      std::vector<FlowOp> ops;
+      ProgEntry x;
+      if (data_flow(progs, ops)) {
+        for (const FlowOp& o : ops) {
+          x.most = std::max<long long>(x.most, o.count);
+          for (int i = 0; i < o.n_leaf; i++) x.offsets_aligned &= o.leaf_off[i] * esz % 16 == 0;
+          for (int i = 0; i < o.n_dst; i++) x.offsets_aligned &= o.dst_off[i] * esz % 16 == 0;
+        }
+        x.n_ops = (int)ops.size();
+      }
+      const void* dev = nullptr;
+      if (int rc = upload(c0, ops.data(), ops.size() * sizeof(FlowOp), std::max<size_t>(1, ops.size()) * sizeof(FlowOp), stream, x, &dev)) return rc;
+      x.ops = static_cast<const FlowOp*>(dev);
+      it = c0->cache.emplace(k, x).first;
+      for (int i = 0; i < n; i++) comms[i]->stats.program_cache_misses++;
+    } else {
+      if (int rc = after_upload(it->second, stream)) return rc;
+      for (int i = 0; i < n; i++) comms[i]->stats.program_cache_hits++;
+    }
+    e = &it->second;
+  }
+  if (e->n_ops == 0) return PICCL_UNSUPPORTED;
+  FlowArgs fa; memset(&fa, 0, sizeof fa);
+  fa.n_ops = e->n_ops; fa.avg = avg ? 1 : 0; fa.scale = avg ? 1.0f / (float)n : 1.0f; fa.ops = e->ops;
+  fa.leave_first = leave_first(a, n, true);
+  fa.n_slices = flow_slices(c0, e->most * esz, e->n_ops, &fa.slice_bytes);
+  bool aligned = e->offsets_aligned, skip = false;
+  for (int i = 0; i < n; i++) {
+    fa.in[i] = calls[i].send; fa.out[i] = calls[i].recv;
+    aligned &= ((reinterpret_cast<uintptr_t>(calls[i].send) | reinterpret_cast<uintptr_t>(calls[i].recv)) & 15) == 0;
+    std::lock_guard<std::mutex> l(comms[i]->mu);
+    comms[i]->stats.launches++;
+    skip |= fault_now(comms[i]); comms[i]->call_index++;
+  }
+  if (skip) return PICCL_OK;
+  TraceRec* tr = trace_begin(c0, d0.coll, d0.algo, d0.k, count * esz, fa.n_slices, stream);
+  nvtxRangePushA(coll_name(d0.coll));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((long long)fa.n_ops * fa.n_slices)); cfg.blockDim = dim3(kFlowBlock); cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  void* args[] = {&fa};
+  const cudaError_t err = cudaLaunchKernelExC(&cfg, (const void*)(reducing ? exec_flow_kernel_for(d0.dtype, op, !aligned) : exec_flow_copy_kernel(!aligned)), args);
+  nvtxRangePop();
+  trace_end(c0, tr, stream);
+  if (err != cudaSuccess) return fail(PICCL_CUDA_ERROR, "launch of a data flow failed: %s", cudaGetErrorString(err));
+  for (int i = 0; i < n; i++) { comms[i]->stats.calls[d0.coll]++; comms[i]->stats.bytes[d0.coll] += (unsigned long long)count * esz; }
+  return PICCL_OK;
 }
 
 // Runs one collective over `n` communicators of this process (n == 1: the normal case).
@@ -717,21 +763,20 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     }
   }
 
-  bool share = may_share(comms, n, calls, (long long)d0.count * esz_real);
+  if (may_flow(comms, n, calls, (long long)d0.count * esz_real)) {
+    const int flow = run_flow(comms, n, calls, count, esz, op, avg, cap_state != cudaStreamCaptureStatusNone, stream);
+    if (flow != PICCL_UNSUPPORTED) return flow;
+  }
+
   nvtxRangePushA(coll_name(d0.coll));
   int rc = PICCL_OK;
   for (long long done = 0; done < count && rc == PICCL_OK; done += slab) {
     long long cur = std::min(slab, count - done);
     KernelArgs ka; memset(&ka, 0, sizeof ka);
-    ka.n_vrank = n; ka.elem_size = esz; ka.one_gpu = n == c0->nranks; ka.avg = avg ? 1 : 0; ka.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
+    ka.n_vrank = n; ka.elem_size = esz; ka.avg = avg ? 1 : 0; ka.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
     int n_cta = 0;
-    long long n_blocks = 0;
     bool aligned = true;
-    CollArgs first;
-    GroupPrograms group;
-    group.lines = use_llf;
-    long long most = 0;
-    bool any_shared = false, flat = false;
+    CollArgs priorities_of;
     for (int i = 0; i < n && rc == PICCL_OK; i++) {
       piccl_comm* c = comms[i]; const CallDesc& d = calls[i];
       std::lock_guard<std::mutex> l(c->mu);
@@ -744,37 +789,28 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
       }
       if (d.coll == COLL_REDUCE && c->rank != d.root) a.in_place = false;
       const ProgEntry* pe = nullptr;
-      if (i == 0 && share && cap_state != cudaStreamCaptureStatusNone) share = c->cache.count(key_of(a, use_llf ? 2 : 1)) != 0;      // (a capture replays what was built before it)
-      rc = get_program(c, a, stream, &pe, share ? &group : nullptr); if (rc) break;
-      if (i == 0) flat = pe->flat;
-      if (i == 0) first = a;
+      rc = get_program(c, a, stream, &pe); if (rc) break;
+      if (i == 0) {
+        n_cta = choose_cta(c, a, n);
+        if (use_llf) {   // a line (8 bytes) per thread and action while there are CTAs, then several; a segment holds 4 KiB
+          long long ab = a.count * a.elem_size;
+          if (a.coll == COLL_ALLREDUCE && (a.algo == ALGO_RING || a.algo == ALGO_K_RING)) ab /= std::max(1, a.nranks);
+          if (a.algo == ALGO_DIRECT && a.coll != COLL_ALLGATHER && a.coll != COLL_REDUCE_SCATTER) ab /= std::max(1, a.coll == COLL_ALLREDUCE ? a.nranks : a.nranks - 1);
+          n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
+          if (n > 1) n_cta = std::min(n_cta, std::max(1, c->sm_count / n));
+        }
+        ka.n_cta = n_cta; if (!use_llf) cut_fifo(c, n, n_cta, a, &ka);
+        priorities_of = a;
+        ka.one_gpu = n == c->nranks;
+        ka.timeout_ns = (unsigned long long)c->cfg.timeout_ms * 1000000ull;
+      }
       ka.one_gpu &= c->device == c0->device;
-      ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].shared = pe->dev_shared; any_shared |= pe->dev_shared != nullptr; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
-      ka.prog_actions = std::max(ka.prog_actions, pe->n_actions); most = std::max(most, pe->most);
+      ka.r[i].ctx = c->d_ctx; ka.r[i].actions = pe->dev; ka.r[i].n_actions = pe->n_actions; ka.r[i].in = s; ka.r[i].out = r;
       aligned &= pe->offsets_aligned && ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(r)) & 15) == 0;
       c->stats.launches++;
     }
     if (rc) break;
-    // Ranks with nothing to do, whose operands others read (the leaves of a tree), leave their SMs to those that have.
-    int n_working = 0;
-    for (int i = 0; i < n; i++) if (ka.r[i].n_actions > 0 || !any_shared) ka.working[n_working++] = (uint8_t)i;
-    if (n_working == 0) ka.working[n_working++] = 0;
-    n_cta = choose_cta(c0, first, n_working, n);
-    if (use_llf) {   // a line (8 bytes) per thread and action while there are CTAs, then several; a segment holds 4 KiB
-      long long ab = first.count * first.elem_size;
-      if (first.coll == COLL_ALLREDUCE && (first.algo == ALGO_RING || first.algo == ALGO_K_RING)) ab /= std::max(1, first.nranks);
-      if (first.algo == ALGO_DIRECT && first.coll != COLL_ALLGATHER && first.coll != COLL_REDUCE_SCATTER) ab /= std::max(1, first.coll == COLL_ALLREDUCE ? first.nranks : first.nranks - 1);
-      n_cta = (int)std::max<long long>(1, std::min<long long>((ab + kLLBlock * 8 - 1) / (kLLBlock * 8), kLLFifoCta));
-      if (n > 1) n_cta = std::min(n_cta, std::max(1, c0->sm_count / n_working));
-    }
-    if (flat) { long long a = 0; for (int i = 0; i < n; i++) a += ka.r[i].n_actions; n_cta = flat_slices(c0, most * esz, a, &ka.seg_bytes); n_blocks = a * n_cta; }
-    ka.n_cta = n_cta; if (!use_llf && !flat) cut_fifo(c0, n, n_cta, first, &ka);
-    ka.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
-    if (any_shared && !flat && !use_llf) { // the widest slice is CTA 0's
-      const long long segs = slice_of(most, esz, 0, n_cta, ka.seg_bytes).nseg;
-      ka.prog_total = round_up(segs, ka.window) * ka.prog_actions + 1;
-    }
-    ka.leave_first = leave_first(first, n, ka.one_gpu);
+    ka.leave_first = leave_first(priorities_of, n, ka.one_gpu);
     bool skip = false;
     for (int i = 0; i < n; i++) skip |= fault_now(comms[i]);
     for (int i = 0; i < n; i++) comms[i]->call_index++;
@@ -785,8 +821,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     const int block = use_llf ? kLLBlock : exec_block(c0);
     // which kernel a rank runs is its own business: both speak the same protocol
     const ExecKernelFn f = (aligned || use_llf) ? fn : reducing ? exec_shift_kernel_for(d0.dtype, op) : exec_shift_copy_kernel();
-    if (flat) e = launch_flat(reducing ? exec_flat_kernel_for(d0.dtype, op, !aligned) : exec_flat_copy_kernel(!aligned), n_blocks, args, stream);
-    else if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n_working * n_cta), dim3(block), args, 0, stream);
+    if (n > 1) e = cudaLaunchCooperativeKernel((const void*)f, dim3(n * n_cta), dim3(block), args, 0, stream);
     else e = cudaLaunchKernel((const void*)f, dim3(n_cta), dim3(block), args, 0, stream);
     if (e != cudaSuccess) rc = fail(PICCL_CUDA_ERROR, "executor launch failed: %s", cudaGetErrorString(e));
     trace_end(c0, tr, stream);
@@ -838,7 +873,7 @@ int piccl_test_leave_first(int coll, int nranks, int in_launch, int one_device, 
   CollArgs a; a.coll = (Coll)coll; a.nranks = nranks; a.count = bytes; a.elem_size = 1;
   return leave_first(a, in_launch, one_device && in_launch == nranks);
 }
-// on != 0: ranks of one launch do not read each other's buffers, everything that crosses goes through the slots as it does between GPUs.
+// on != 0: everything that crosses goes through the slots as it does between GPUs, also where one launch carries all ranks.
 int piccl_test_slots_only(piccl_comm_t* c, int on) {
   if (!c) return fail(PICCL_INVALID_ARGUMENT, "null communicator");
   c->slots_only = on != 0;

@@ -21,20 +21,20 @@ struct HandleBlob {
 };
 
 struct ProgKey {
-  int coll, algo, k, root, elem_size, in_place; long long count, stride; int shared = 0 /* ranks read each other's buffers: 1, 2 in the low-latency variant */;
+  int coll, algo, k, root, elem_size, in_place; long long count, stride; int flow = 0 /* the call's data flow, kept by rank 0 */;
   bool operator==(const ProgKey& o) const {
-    return coll == o.coll && algo == o.algo && k == o.k && root == o.root && elem_size == o.elem_size && in_place == o.in_place && count == o.count && stride == o.stride && shared == o.shared;
+    return coll == o.coll && algo == o.algo && k == o.k && root == o.root && elem_size == o.elem_size && in_place == o.in_place && count == o.count && stride == o.stride && flow == o.flow;
   }
 };
 struct ProgKeyHash {
   size_t operator()(const ProgKey& k) const {
     unsigned long long h = 1469598103934665603ull;
     auto mix = [&](unsigned long long v) { h ^= v; h *= 1099511628211ull; };
-    mix(k.coll); mix(k.algo); mix((unsigned)k.k); mix(k.root); mix(k.elem_size); mix(k.in_place); mix((unsigned long long)k.count); mix((unsigned long long)k.stride); mix(k.shared);
+    mix(k.coll); mix(k.algo); mix((unsigned)k.k); mix(k.root); mix(k.elem_size); mix(k.in_place); mix((unsigned long long)k.count); mix((unsigned long long)k.stride); mix(k.flow);
     return (size_t)h;
   }
 };
-struct ProgEntry { const Action* dev = nullptr; const SharedOps* dev_shared = nullptr; int n_actions = 0; long long most = 0 /* elements of its largest action */; bool flat = false /* nothing in the call waits */; long long scratch_elems = 0; cudaEvent_t ready = nullptr; cudaStream_t origin = nullptr; bool synced = false, offsets_aligned = true /* all offsets into user buffers are multiples of 16 bytes */; };
+struct ProgEntry { const Action* dev = nullptr; int n_actions = 0; const FlowOp* ops = nullptr; int n_ops = 0; long long most = 0 /* elements of its largest operation */; long long scratch_elems = 0; cudaEvent_t ready = nullptr; cudaStream_t origin = nullptr; bool synced = false, offsets_aligned = true /* all offsets into user buffers are multiples of 16 bytes */; };
 struct ProgChunk { char* dev = nullptr; char* host = nullptr; size_t cap = 0, used = 0; };
 
 // What a low-latency all-reduce of one algorithm and radix looks like for the communicators of a launch: the arguments that do not
@@ -57,7 +57,7 @@ struct piccl_comm {
   long long llf_max_bytes = 0;         // largest message the low-latency executor takes (0: off)
   piccl_status_t* h_status = nullptr; piccl_status_t* d_status = nullptr;
   bool ipc_opened[piccl::kMaxRanks] = {false};
-  bool connected = false, broken = false, slots_only = false /* ranks of one launch do not read each other's buffers (tests) */;
+  bool connected = false, broken = false, slots_only = false /* everything goes through the ranks' slots, also where one launch carries all ranks (tests) */;
   unsigned long long call_index = 0;
   unsigned tp_epoch_rs = 0, tp_epoch_ag = 0;   // epochs of the fused tensor-parallel kernels
   int* d_tp_status = nullptr;

@@ -463,33 +463,37 @@ def test_averaged_rounds_of_the_default_geometry(n, algo, k, dtype):
 
 @pytest.mark.parametrize("dtype,offset", [(torch.float32, 0), (torch.bfloat16, 0), (torch.bfloat16, 1)])
 @pytest.mark.parametrize("coll", ["allreduce", "allgather", "reduce_scatter", "broadcast", "reduce"])
-def test_reading_each_others_buffers_changes_nothing(coll, dtype, offset):
-    """Every algorithm on three and eight ranks, with the ranks reading each other's buffers and with everything through the slots, in turn on one communicator, from a captured graph too,
-    and with a receive buffer that is another rank's send buffer (slots, whatever was asked for).  Operands and hops are rounded alike: bit for bit the same."""
+def test_data_flow_is_the_programs_bit_for_bit(coll, dtype, offset):
+    """Every algorithm on three, four and eight ranks: the ranks' programs through the slots and the call's data flow, in turn on one communicator, from a captured graph
+    too, and with a receive buffer that is another rank's send buffer (programs, whatever was asked for).  Operands are combined and rounded alike: the same bits, also of averages, and of
+    maxima of zeros of both signs and values that are not numbers."""
     from piccl_b200.parallel.comm import LoopbackGroup, make_config
-    for n in (3, 8):
+    for n, k in ((3, 2), (4, 2), (8, 2), (8, 4)):
         g = LoopbackGroup(n, config=make_config(scratch_bytes=1 << 20, timeout_ms=5000))
         count = 40013 if coll in ("allgather", "reduce_scatter") else 180013 * n      # (above the sizes that other kernels take outside a capture)
         n_in, n_out = count * (n if coll == "reduce_scatter" else 1), count * (n if coll == "allgather" else 1)
-        xs = [x[offset:] for x in _inputs(n, n_in + offset, dtype, seed=3)]
-        op = "sum" if coll in ("allgather", "broadcast") else "avg"
-        for algo in ALGOS:
+        ins = {"avg": [x[offset:] for x in _inputs(n, n_in + offset, dtype, seed=3)]}
+        odd = torch.tensor([0.0, -0.0, float("nan"), 1.0, -1.0, float("inf"), -float("inf")], device="cuda", dtype=dtype)
+        ins["max"] = [odd[torch.randint(0, 7, (n_in + offset,), generator=torch.Generator(device="cuda").manual_seed(r), device="cuda")][offset:] for r in range(n)]
+        for algo, op in itertools.product(ALGOS, ["avg", "max"] if coll in ("allreduce", "reduce_scatter", "reduce") else ["avg"]):
+            xs, op = ins[op], "sum" if coll in ("allgather", "broadcast") else op
             outs = [[torch.full((n_out + offset,), 7.0, device="cuda", dtype=dtype)[offset:] for _ in range(n)] for _ in range(3)]
             for variant, slots in enumerate((1, 0)):
                 for h in g._hs:
                     g._lib.piccl_test_slots_only(h, slots)
                 for _ in range(2):
-                    g.run(coll, xs, outs[variant], count, op=op, root=1, algo=algo, k=4)
+                    g.run(coll, xs, outs[variant], count, op=op, root=1, algo=algo, k=k)
             _check_ok(g)
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph):
-                g.run(coll, xs, outs[2], count, op=op, root=1, algo=algo, k=4)
+                g.run(coll, xs, outs[2], count, op=op, root=1, algo=algo, k=k)
             for _ in range(2):
                 graph.replay()
             _check_ok(g)
+            bits = lambda t: t.clone().view(torch.int16 if dtype == torch.bfloat16 else torch.int32)
             for r in range(n):
-                assert torch.equal(outs[0][r], outs[1][r]) and torch.equal(outs[0][r], outs[2][r]), (coll, algo, n, r)
-            if n_in == n_out and coll != "broadcast":       # rank 0 receives into rank 1's send buffer (the ring's sums contain what they overwrite)
+                assert torch.equal(bits(outs[0][r]), bits(outs[1][r])) and torch.equal(bits(outs[0][r]), bits(outs[2][r])), (coll, algo, op, n, k, r)
+            if n_in == n_out and coll != "broadcast" and op == "avg":       # rank 0 receives into rank 1's send buffer (the ring's sums contain what they overwrite)
                 ys = [x.clone() for x in xs]
                 zs = [ys[1]] + [torch.full_like(x, 7.0) for x in xs[1:]]
                 if coll == "reduce":
@@ -503,9 +507,9 @@ def test_reading_each_others_buffers_changes_nothing(coll, dtype, offset):
 
 
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.float64])
-@pytest.mark.parametrize("coll,n,algo,op", [("allgather", 3, "RING", "sum"), ("broadcast", 8, "PRD", "sum"), ("reduce", 2, "RING", "max"), ("reduce_scatter", 4, "DIRECT", "sum"), ("allreduce", 5, "PRM", "avg"),
+@pytest.mark.parametrize("coll,n,algo,op", [("allgather", 3, "RING", "sum"), ("broadcast", 8, "PRD", "sum"), ("reduce", 2, "RING", "max"), ("reduce_scatter", 4, "DIRECT", "sum"), ("allreduce", 5, "PRM", "avg"), ("allreduce", 4, "PRD", "sum"), ("reduce", 8, "K_RING", "max"),
                                             ("allreduce", 8, "DIRECT", "min")])
-def test_calls_in_which_nothing_waits(coll, n, algo, op, dtype):
+def test_slices_of_a_data_flow(coll, n, algo, op, dtype):
     """Blocks of 4 KiB to 64 KiB: one element, a pack and its neighbours, a block and its neighbours, several blocks, a message whose blocks are larger; operands and results
     3 elements into their buffers too.  Small whole numbers: exact but for fifths, whose sum of five rounded operands errs by half a unit each and once more."""
     from piccl_b200.parallel.comm import LoopbackGroup, make_config
