@@ -26,6 +26,8 @@
 //     void k_range(int idx, int num_kb, int& kb0, int& kb1) const; // k-blocks that this entry of the tile order sums, not empty
 //     const CUtensorMap* a_map(int m_blk, int& row0) const;        // tensor map and first row of A for it
 //     const CUtensorMap* b_map() const;                            // tensor map of B
+//     static constexpr bool K_RANKS = true; int kb_per_rank; const CUtensorMap* a_of(int p) const, *b_of(int p) const;      // optional: k-blocks [p, p + 1) * kb_per_rank come from
+//                                                                   // these maps, each from its column 0 (a_map still gives the row)
 //     bool gate(int m_blk, volatile int* abort) const;             // producer: wait until the row block may be loaded
 //     void prefetch(const EpiCtx&, int m_blk, int n_blk);          // epilogue warps, before they wait for the accumulator
 //     bool epilogue(const EpiCtx&, int idx, int m_blk, int n_blk, volatile int* abort);  // called by all eight warps; false: gave up
@@ -147,6 +149,9 @@ __device__ __forceinline__ void epi_staging_free(const EpiCtx& e) {
   __syncwarp();
 }
 
+template <class P, class = void> struct k_over_ranks { static constexpr bool value = false; };
+template <class P> struct k_over_ranks<P, decltype((void)P::K_RANKS)> { static constexpr bool value = P::K_RANKS; };
+
 template <int TN, int STAGES, bool A_MN, bool B_MN, class Policy>
 __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, Policy& pol, int K, int first_tile, int tile_stride, volatile int* s_abort) {
   typedef PairSmem<TN, STAGES, Policy::EXTRA_BYTES, Policy::NSTAGE> L;
@@ -192,16 +197,18 @@ __device__ __forceinline__ void gemm_pair_persistent(uint8_t* smem_raw, Policy& 
       for (int kb = kb0; kb < kb1; kb++) {
         if (!mbar_wait(&empty[stage], phase ^ 1, s_abort, kPairWaitLimitNs)) { if (issuer) pol.report(1); ok = false; break; }
         uint8_t* sa = smem + stage * L::STAGE_BYTES; uint8_t* sb = sa + L::A_BYTES;
+        int k0 = kb * PAIR_BK;
+        if constexpr (k_over_ranks<Policy>::value) { const int p = kb / pol.kb_per_rank; ta = pol.a_of(p); tb = pol.b_of(p); k0 = (kb - p * pol.kb_per_rank) * PAIR_BK; }
         if (issuer) {
           if (v == 0) mbar_arrive_expect_tx(&full[stage], 2 * L::STAGE_BYTES);      // the bytes of both CTAs land on the leader's barrier
           if (A_MN) {
 #pragma unroll
-            for (int i = 0; i < PAIR_BM / 64; i++) tma_load_2d_pair(sa + i * 8192, ta, row0 + i * 64, kb * PAIR_BK, &full[stage]);
-          } else tma_load_2d_pair(sa, ta, kb * PAIR_BK, row0, &full[stage]);
+            for (int i = 0; i < PAIR_BM / 64; i++) tma_load_2d_pair(sa + i * 8192, ta, row0 + i * 64, k0, &full[stage]);
+          } else tma_load_2d_pair(sa, ta, k0, row0, &full[stage]);
           if (B_MN) {
 #pragma unroll
-            for (int i = 0; i < TN / 128; i++) tma_load_2d_pair(sb + i * 8192, tb, col0 + i * 64, kb * PAIR_BK, &full[stage]);
-          } else tma_load_2d_pair(sb, tb, kb * PAIR_BK, col0, &full[stage]);
+            for (int i = 0; i < TN / 128; i++) tma_load_2d_pair(sb + i * 8192, tb, col0 + i * 64, k0, &full[stage]);
+          } else tma_load_2d_pair(sb, tb, k0, col0, &full[stage]);
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1; }

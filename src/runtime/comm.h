@@ -61,6 +61,7 @@ struct piccl_comm {
   unsigned long long call_index = 0;
   unsigned tp_epoch_rs = 0, tp_epoch_ag = 0;   // epochs of the fused tensor-parallel kernels
   int* d_tp_status = nullptr;
+  int tp_local_ready = 0;              // bit 3 * kernel + width: the kernel has its shared memory
   int tp_pairs[2] = {0, 0};            // CTA pairs of the tensor-parallel kernels that fit the device (0: not asked yet)
   void* persist = nullptr;             // state of the persistent launcher (runtime/persistent.cu)
   void* nvls = nullptr;                // multicast window of the in-switch all-reduce (runtime/nvls.cu)

@@ -381,6 +381,76 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(AG_THREADS, 1) ag_ge
   gemm_pair_persistent<TP_BN, AG_STAGES, false, false>(smem_raw, pol, a.K, blockIdx.x >> 1, gridDim.x >> 1, &s_abort);
 }
 
+// ------------------------------------------------------------------ all ranks in one launch on one GPU
+// There every rank's operands can be read where they are: nothing is pushed, flagged or waited for.  ag_gemm takes the rows of a shard from its owner; gemm_rs sums an owner's tile over
+// all ranks' k in the accumulator, where the partial tiles otherwise go through memory as bf16.  Without waits between CTAs the launch need not be cooperative, overlaps the end of the kernel
+// before, has no more CTAs than tiles, and takes narrow tiles where wide ones leave the chip idle.  Large products are bound by the power cap, small ones by the launch and one tile's k.
+// us, exchanging through the workspace and this: ag_gemm 2 x 4096 x 2048 x 4096 120 / 109, 2 x 512 x 768 x 1024 16.4 / 7.7, 4 x 3584 x 1280 x 1728 86.7 / 52.5, 8 x 8192 x 8192 x 4096 3439 / 3179;
+// gemm_rs 8 x 8192 x 8192 x 3584 3021 / 2931, 4 x 512 x 1280 x 384 18.5 / 9.5, 2 x 8192 x 8192 x 256 159 / 66, 8 x 8192 x 1024 x 4096 473 / 449.
+template <int TN, bool RS>
+struct LocalPolicy {
+  const TpArgs& a; const TpRank* R = nullptr; int rank = 0, mb_per_shard, blocks, rp, num_n, kb_per_rank;
+  static constexpr int EXTRA_BYTES = 0, NSTAGE = 1;
+  static constexpr bool K_RANKS = RS;
+  __device__ LocalPolicy(const TpArgs& args)
+      : a(args), mb_per_shard(args.M / args.n / TP_BM), blocks(RS ? mb_per_shard : args.M / TP_BM), rp((blocks + 1) / 2), num_n(args.N / TN), kb_per_rank(args.K / TP_BK) {}
+  __device__ void begin() const {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
+  __device__ void report(int role) const { for (int i = 0; i < a.nv; i++) atomicExch(a.r[i].status, role); }
+  __device__ int num_tiles() const { return a.nv * rp * num_n; }
+  // one rank after the other; bands of 16 pairs of row blocks, inside a band rows fastest
+  __device__ void tile(int idx, int v, int& m_blk, int& n_blk) {
+    constexpr int BAND = 16;
+    rank = idx / (rp * num_n);
+    R = &a.r[rank];
+    int w = idx % (rp * num_n);
+    const int band = w / (BAND * num_n), in_band = min(BAND, rp - band * BAND);
+    w %= BAND * num_n;
+    const int i = 2 * (band * BAND + w % in_band) + v;
+    n_blk = w / in_band;
+    m_blk = i < blocks ? i : -1;
+  }
+  __device__ void k_range(int, int num_kb, int& kb0, int& kb1) const { kb0 = 0; kb1 = num_kb; }
+  __device__ const CUtensorMap* a_map(int m_blk, int& row0) const {
+    const int m = max(m_blk, 0);
+    if (RS) { row0 = (rank * mb_per_shard + m) * TP_BM; return &R->ta; }
+    row0 = m % mb_per_shard * TP_BM; return &a.r[m / mb_per_shard].ta;
+  }
+  __device__ const CUtensorMap* b_map() const { return &R->tb; }
+  __device__ const CUtensorMap* a_of(int p) const { return &a.r[p].ta; }
+  __device__ const CUtensorMap* b_of(int p) const { return &a.r[p].tb; }
+  __device__ bool gate(int, volatile int*) const { return true; }
+  __device__ void prefetch(const EpiCtx&, int, int) {}
+  __device__ void finish(const EpiCtx&) {}
+  __device__ bool epilogue(const EpiCtx& e, int, int m_blk, int n_blk, volatile int*) {
+    constexpr int PIECES = TN / 128 > 0 ? TN / 128 : 1;      // of 64 columns, to each half of the warps; a tile of 64 columns is the first half's
+    if (m_blk < 0 || e.half * PIECES * 64 >= TN) return true;
+#pragma unroll 1
+    for (int pc = e.half * PIECES; pc < (e.half + 1) * PIECES; pc++) {
+      float v[64];
+      epi_load64(e, pc * 64, v);
+      epi_staging_free(e);
+      epi_stage_row(e, v);
+      epi_ship(e, &R->tc, n_blk * TN + pc * 64, m_blk * TP_BM + e.quarter * 32);
+    }
+    return true;
+  }
+};
+template <int TN, int STAGES, bool RS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) tp_local_kernel(const __grid_constant__ TpArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ int s_abort;
+  if (threadIdx.x == 0) s_abort = 0;
+  LocalPolicy<TN, RS> pol(a);
+  gemm_pair_persistent<TN, STAGES, false, false>(smem_raw, pol, RS ? a.n * a.K : a.K, blockIdx.x >> 1, gridDim.x >> 1, &s_abort);
+}
+struct LocalVariant { void (*fn)(TpArgs); int tn, smem; };
+static const LocalVariant kLocal[2][3] = {
+    {{tp_local_kernel<256, 6, true>, 256, PairSmem<256, 6>::DYNAMIC}, {tp_local_kernel<128, 8, true>, 128, PairSmem<128, 8>::DYNAMIC}, {tp_local_kernel<64, 9, true>, 64, PairSmem<64, 9>::DYNAMIC}},
+    {{tp_local_kernel<256, 6, false>, 256, PairSmem<256, 6>::DYNAMIC}, {tp_local_kernel<128, 8, false>, 128, PairSmem<128, 8>::DYNAMIC}, {tp_local_kernel<64, 9, false>, 64, PairSmem<64, 9>::DYNAMIC}}};
+
 // ------------------------------------------------------------------ host
 // The workspace is used in four quarters: [kernel: gemm_rs, ag_gemm][parity of that kernel's call count].
 static long long tp_quarter(long long tp_bytes) { return tp_bytes / 4 / 1024 * 1024; }
@@ -410,6 +480,30 @@ static int tp_common_checks(piccl_comm** cs, int n, int M, int N, int K, int whi
   long long need = piccl_tp_workspace_bytes(which, c->nranks, M, N, K);
   if (tp_quarter(c->h_ctx.tp_bytes) < tp_need_per_call(which, c->nranks, M, N, K)) return fail(PICCL_INVALID_USAGE, "tensor-parallel workspace too small: %lld bytes needed, %lld configured (tp_bytes / PICCL_TP_MB)", need, c->h_ctx.tp_bytes);
   return PICCL_OK;
+}
+
+// All ranks in this launch on one GPU, and no result over an operand?
+static bool tp_local(piccl_comm** cs, int n, const void* const* A, const void* const* B, void* const* out, int M, int N, int K, int which) {
+  if (n < 2 || n != cs[0]->nranks) return false;
+  const long long rows = M / n, a_bytes = (which ? rows : M) * 2LL * K, b_bytes = 2LL * N * K, o_bytes = (which ? M : rows) * 2LL * N;
+  auto meet = [](const void* x, long long nx, const void* y, long long ny) { return (const char*)x < (const char*)y + ny && (const char*)y < (const char*)x + nx; };
+  for (int i = 0; i < n; i++) {
+    if (cs[i]->rank != i || cs[i]->device != cs[0]->device || cs[i]->slots_only) return false;
+    for (int j = 0; j < n; j++) if (meet(out[i], o_bytes, A[j], a_bytes) || meet(out[i], o_bytes, B[j], b_bytes) || (i < j && meet(out[i], o_bytes, out[j], o_bytes))) return false;
+  }
+  return true;
+}
+// Tile width: waves of the persistent grid times the clocks of a tile, which are those of the plain GEMM (gemm_sm100.cu: choose).
+static int tp_local_width(int n, int M, int N, int K, int which, int pairs) {
+  const long long blocks = which ? M / TP_BM : M / n / TP_BM, kb = (which ? K : (long long)n * K) / TP_BK;
+  int best = 0; double best_cost = 0;
+  for (int v = 0; v < 3; v++) {
+    const int tn = kLocal[which][v].tn;
+    const long long tiles = n * ((blocks + 1) / 2) * (N / tn);
+    const double cost = (double)((tiles + pairs - 1) / pairs) * ((tn == 256 ? 136 : tn == 128 ? 84 : 70) * 4.0 * kb + 10.0 * tn);
+    if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
+  }
+  return best;
 }
 
 static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* const* B, void* const* out, int M, int N, int K, int which, cudaStream_t stream) {
@@ -448,6 +542,8 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
   }
   a.nv = n; a.one_gpu = n == nr;
   bool ok = true;
+  const bool local = tp_local(cs, n, A, B, out, M, N, K, which);
+  const LocalVariant& lv = kLocal[which][local ? tp_local_width(n, M, N, K, which, c0->tp_pairs[which]) : 0];
   for (int i = 0; i < n && ok; i++) {
     piccl_comm* c = cs[i];
     TpRank& R = a.r[i];
@@ -459,16 +555,30 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
     if (which == 0) {
       ok &= make_tmap_bf16_k64(&R.ta, A[i], (uint64_t)M, (uint64_t)K, (uint64_t)K, TP_BM);
       R.ta2 = R.ta;
-      a.epoch = ++c->tp_epoch_rs;
+      if (!local) a.epoch = ++c->tp_epoch_rs;
     } else {
       ok &= make_tmap_bf16_k64(&R.ta, A[i], (uint64_t)(M / nr), (uint64_t)K, (uint64_t)K, TP_BM);
-      ok &= make_tmap_bf16_k64(&R.ta2, c->heap + a.data_off, (uint64_t)M, (uint64_t)K, (uint64_t)K, TP_BM);
-      a.epoch = ++c->tp_epoch_ag;
+      if (!local) { ok &= make_tmap_bf16_k64(&R.ta2, c->heap + a.data_off, (uint64_t)M, (uint64_t)K, (uint64_t)K, TP_BM); a.epoch = ++c->tp_epoch_ag; }
     }
-    ok &= make_tmap_bf16_k64(&R.tb, B[i], (uint64_t)N, (uint64_t)K, (uint64_t)K, TP_BN / 2);
+    ok &= make_tmap_bf16_k64(&R.tb, B[i], (uint64_t)N, (uint64_t)K, (uint64_t)K, local ? lv.tn / 2 : TP_BN / 2);
     ok &= make_tmap_bf16_k64(&R.tc, out[i], (uint64_t)(which ? M : M / nr), (uint64_t)N, (uint64_t)N, 32);
   }
   if (!ok) return fail(PICCL_CUDA_ERROR, "tensor map or status set-up failed");
+  if (local) {
+    const int bit = 1 << (3 * which + (int)(&lv - kLocal[which]));
+    if (!(c0->tp_local_ready & bit)) {
+      if (cudaFuncSetAttribute((const void*)lv.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lv.smem) != cudaSuccess) return fail(PICCL_CUDA_ERROR, "cannot get %d bytes of shared memory", lv.smem);
+      c0->tp_local_ready |= bit;
+    }
+    const long long tiles = n * ((((which ? M : M / n) / TP_BM) + 1) / 2) * (long long)(N / lv.tn);
+    cfg.gridDim = dim3(2 * (unsigned)std::min<long long>(tiles, c0->tp_pairs[which])); cfg.blockDim = dim3(PAIR_THREADS); cfg.dynamicSmemBytes = lv.smem;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, lv.fn, a);
+    if (e != cudaSuccess) return fail(PICCL_CUDA_ERROR, "fused kernel launch failed: %s", cudaGetErrorString(e));
+    for (int i = 0; i < n; i++) cs[i]->stats.launches++;
+    return PICCL_OK;
+  }
   // ranks wait for one another inside the kernel: with several virtual ranks on one device all CTAs must be resident at once
   at[0].id = cudaLaunchAttributeCooperative; at[0].val.cooperative = 1;
   cfg.gridDim = dim3(2 * c0->tp_pairs[which]); cfg.attrs = at; cfg.numAttrs = n > 1 ? 1 : 0;
