@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 import threading
 from pathlib import Path
@@ -89,6 +90,21 @@ def lib() -> C.CDLL:
             _declare(l)
             _libs["piccl"] = l
         return _libs["piccl"]
+
+
+def fastcall():
+    """The module that calls the library with lists of tensors (src/python/fastcall.cc)."""
+    with _lock:
+        if "fastcall" not in _libs:
+            spec = importlib.util.spec_from_file_location("_fastcall", _ensure_built("_fastcall.so"))
+            _libs["fastcall"] = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(_libs["fastcall"])
+        return _libs["fastcall"]
+
+
+def address(function) -> int:
+    """Where a function of a library is."""
+    return C.cast(function, C.c_void_p).value
 
 
 def ops_lib() -> C.CDLL:

@@ -3,6 +3,7 @@
   piccl_b200/lib/piccl.so        collectives library + NCCL-ABI preload shim + fused TP kernels
   piccl_b200/lib/libpiccl_ops.so model kernels (tcgen05 GEMM, layer norm, cross entropy, AdamW, ...)
   piccl_b200/lib/libpiccl_model.so native training step (launches the kernels of libpiccl_ops.so; attention partly through ATen)
+  piccl_b200/lib/_fastcall.so    calls with lists of tensors for the Python front end
   piccl_b200/lib/piccl_sched     schedule dump / validation command line tool
   piccl_b200/lib/coll_bench      OSU-style collective benchmark (fork per GPU, no MPI)
   piccl_b200/lib/loggp_bench     PRTT measurements between two GPUs (input of tools/loggp_param)
@@ -21,6 +22,7 @@ import os
 import shlex
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -59,6 +61,11 @@ def targets() -> dict[str, dict]:
             "flags": [f"-I{p}" for p in (TORCH / "include", TORCH / "include" / "torch" / "csrc" / "api" / "include")],
             "link": ["-shared", "-cudart", "none", f"-L{OUT}", "-lpiccl_ops", f"-L{TORCH / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
                      "-Xlinker", "-rpath,$ORIGIN", "-Xlinker", f"-rpath,{TORCH / 'lib'}"],
+        },
+        "_fastcall.so": {
+            "src": _sources("python/*.cc"),
+            "flags": [f"-I{sysconfig.get_paths()['include']}"],
+            "link": ["-shared", "-cudart", "none"],
         },
         "piccl_sched": {
             "src": _sources("coll/*.cc", "tools/piccl_sched.cc"),

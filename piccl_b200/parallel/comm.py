@@ -152,7 +152,9 @@ class Communicator(_CommBase):
 
 
 class LoopbackGroup(_CommBase):
-    """`nranks` virtual ranks on one device; every collective is one cooperative launch."""
+    """`nranks` virtual ranks on one device; every collective is one launch."""
+
+    _collective = None           # the native call (src/python/fastcall.cc); without it, as with a stand-in for the library, the call goes through ctypes
 
     def __init__(self, nranks: int, device: Optional[int] = None, config: Optional[N.Config] = None):
         super().__init__()
@@ -162,6 +164,7 @@ class LoopbackGroup(_CommBase):
         self._hs = []
         self._comms = None
         self._pack = struct.Struct(f"{nranks}Q").pack
+        self._collective, self._entry = N.fastcall().collective, N.address(self._lib.piccl_group_collective)
         blobs = []
         for r in range(nranks):
             h = C.c_void_p()
@@ -178,20 +181,20 @@ class LoopbackGroup(_CommBase):
 
     def run(self, coll: str, send: Sequence[torch.Tensor], recv: Sequence[Optional[torch.Tensor]], count: int, op: str = "sum",
             root: int = 0, algo="RING", k: int = -1, stream=None):
-        rc = self._lib.piccl_group_collective(self.handles(), self.nranks, N.COLL[coll], self._pack(*[t.data_ptr() for t in send]), self.table(recv), count, _dt(send[0]), N.OP[op], root, _algo(algo), k,
-                                              _stream_ptr(stream))
+        if self._collective is not None:
+            rc = self._collective(self._entry, self.handles(), self.nranks, send, recv, count, N.COLL[coll], _dt(send[0]), N.OP[op], root, _algo(algo), k, _stream_ptr(stream))
+        else:
+            rc = self._lib.piccl_group_collective(self.handles(), self.nranks, N.COLL[coll], self._pack(*[t.data_ptr() for t in send]), self._pack(*[0 if t is None else t.data_ptr() for t in recv]), count,
+                                                  _dt(send[0]), N.OP[op], root, _algo(algo), k, _stream_ptr(stream))
         if rc:
             N.check(rc, f"piccl_group_collective({coll})")
 
-    # Small collectives are bound by the host path, so the tables of addresses that a call takes are packed as bytes, and the
-    # communicators' table is built once (an 8-rank call spent 12 of its 18 us in Python).
+    # Small collectives are bound by the host path: the tables of addresses are filled in native code, and the
+    # communicators' table is built once.
     def handles(self) -> bytes:
         if self._comms is None:
             self._comms = self._pack(*[h.value for h in self._hs])
         return self._comms
-
-    def table(self, tensors: Sequence[Optional[torch.Tensor]]) -> bytes:      # None: a rank that receives nothing
-        return self._pack(*[0 if t is None else t.data_ptr() for t in tensors])
 
     def status(self, rank: int = 0) -> N.Status:
         s = N.Status()

@@ -61,9 +61,21 @@ def tp_status(comm_or_handle) -> int:
     return int(_declare().piccl_tp_status(h))
 
 
+_entries: dict = {}
+
+
+def _entry(lib, fn_name: str) -> int:
+    at = _entries.get(fn_name)
+    if at is None:
+        at = _entries[fn_name] = N.address(getattr(lib, fn_name))
+    return at
+
+
 def _group(fn_name, g: LoopbackGroup, As, Bs, outs, M, N_, K, stream):
     lib = _declare()
-    N.check(getattr(lib, fn_name)(g.handles(), g.nranks, g.table(As), g.table(Bs), g.table(outs), M, N_, K, _stream_ptr(stream)), fn_name)
+    rc = N.fastcall().product(_entry(lib, fn_name), g.handles(), g.nranks, As, Bs, outs, M, N_, K, _stream_ptr(stream))
+    if rc:
+        N.check(rc, fn_name)
 
 
 def gemm_rs_group(g: LoopbackGroup, As, Bs, outs, stream=None):

@@ -634,12 +634,18 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
                    : (reducing ? exec_kernel_for(d0.dtype, op) : exec_copy_kernel());
   if (!fn) return fail(PICCL_INTERNAL_ERROR, "no kernel for dtype %d op %d", d0.dtype, op);
 
+  // All ranks in this launch: the call's data flow, where no way between the ranks is asked for by name.  Among eight ranks the low-latency kernels, which are cooperative launches, take 8.2 us for an
+  // all-reduce of 64 KiB and for an all-gather of 4 KiB blocks, the data flow 4.9.  At 1 KiB the all-reduce takes 5.9 and 5.1: up to 16 KiB (both ends of a launch, little more) an exchange asked
+  // for by its algorithm stays on the kernel that is made for it.
+  constexpr long long kOwnKernelBytes = 16384;
+  const bool flows = !env().launch_persistent && d0.algo != ALGO_NVLS && env().proto != 3 && may_flow(comms, n, calls, (long long)d0.count * esz_real);
   // small exchange-type all-reduces take the low-latency kernel (flags travel inside the data lines)
   // (not while the stream is being captured: the call epoch is a launch argument, a replay would reuse it)
   cudaStreamCaptureStatus cap_state = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap_state) != cudaSuccess) { cudaGetLastError(); cap_state = cudaStreamCaptureStatusNone; }
   if (cap_state == cudaStreamCaptureStatusNone && d0.coll == COLL_ALLREDUCE && c0->ll_max_bytes > 0 && (long long)d0.count * esz_real <= c0->ll_max_bytes &&
       (d0.algo == ALGO_RD || d0.algo == ALGO_RM || d0.algo == ALGO_PRD || d0.algo == ALGO_PRM)) {
+    if (flows && (long long)d0.count * esz_real > kOwnKernelBytes) { const int rc = run_flow(comms, n, calls, count, esz, op, avg, false, stream); if (rc != PICCL_UNSUPPORTED) return rc; }
     LLKernelFn lf = ll_kernel_for(d0.dtype, op);
     LLArgs la;
     if (lf && ll_plan(comms, n, d0.algo, d0.k, &la)) {
@@ -682,6 +688,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
   if (cap_state == cudaStreamCaptureStatusNone && (d0.coll == COLL_ALLGATHER || d0.coll == COLL_REDUCE_SCATTER) && c0->ll_max_bytes > 0 && c0->nranks >= 2 &&
       (long long)d0.count * esz_real <= std::min<long long>(c0->ll_max_bytes, (long long)env().llx_kb * 1024) &&
       (d0.algo == ALGO_DIRECT || ((d0.algo == ALGO_RM || d0.algo == ALGO_PRM) && d0.k >= c0->nranks))) {
+    if (flows) { const int rc = run_flow(comms, n, calls, count, esz, op, avg, false, stream); if (rc != PICCL_UNSUPPORTED) return rc; }
     LLXKernelFn xf = d0.coll == COLL_ALLGATHER ? llx_allgather_kernel() : llx_reduce_scatter_kernel_for(d0.dtype, op);
     LLXArgs xa; memset(&xa, 0, sizeof xa);
     xa.n_vrank = n; xa.avg = avg ? 1 : 0; xa.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
@@ -763,7 +770,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     }
   }
 
-  if (may_flow(comms, n, calls, (long long)d0.count * esz_real)) {
+  if (flows) {
     const int flow = run_flow(comms, n, calls, count, esz, op, avg, cap_state != cudaStreamCaptureStatusNone, stream);
     if (flow != PICCL_UNSUPPORTED) return flow;
   }
