@@ -400,8 +400,19 @@ struct LocalPolicy {
   }
   __device__ void report(int role) const { for (int i = 0; i < a.nv; i++) atomicExch(a.r[i].status, role); }
   __device__ int num_tiles() const { return a.nv * rp * num_n; }
-  // one rank after the other; bands of 16 pairs of row blocks, inside a band rows fastest
+  // ag_gemm: one rank after the other; bands of 16 pairs of row blocks, inside a band rows fastest.  gemm_rs: bands of 8 pairs across owners, so that a wave of the grid is about as many
+  // rows as columns: each wave reads all ranks' k of them.
   __device__ void tile(int idx, int v, int& m_blk, int& n_blk) {
+    if (RS) {
+      constexpr int BAND = 8;
+      const int band = idx / (BAND * num_n), in_band = min(BAND, a.nv * rp - band * BAND), w = idx % (BAND * num_n), pair = band * BAND + w % in_band;
+      n_blk = w / in_band;
+      rank = pair / rp;
+      R = &a.r[rank];
+      const int i = 2 * (pair % rp) + v;
+      m_blk = i < blocks ? i : -1;
+      return;
+    }
     constexpr int BAND = 16;
     rank = idx / (rp * num_n);
     R = &a.r[rank];
