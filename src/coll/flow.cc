@@ -6,8 +6,8 @@
 // have been put into a slot, so that the results are bit for bit those of the programs.  A sum that one rank makes and others receive, or that several ranks make alike, is
 // computed once and stored in all their buffers.  Nothing in such a call waits (kernels/exec_flow.cuh).
 //
-// us through the slots and this, one B200: all-reduce 4 x 25 MiB averaged by recursive doubling 131 / 43, 8 x 64 MiB on the ring 353 / 189, 8 x 280 KB 45 / 7.4, 8 x 4 KB 37 / 7.2; all-gather 4 x 1 MiB at
-// odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34; broadcast 8 x 16 MiB 110 / 27; reduce 8 x 16 MiB in two rings 120 / 69.
+// us through the slots and this, one B200: all-reduce 4 x 25 MiB averaged by recursive doubling 131 / 38, 8 x 64 MiB on the ring 353 / 188, 8 x 280 KB 45 / 4.8, 8 x 4 KB 37 / 4.7; all-gather 4 x 1 MiB at
+// odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34; broadcast 8 x 16 MiB 110 / 27; 8 x 8 MiB 196 / 98; reduce 8 x 16 MiB on the ring 92 / 28, in two rings 120 / 69.
 #include <algorithm>
 #include <map>
 #include "coll_internal.h"
@@ -169,6 +169,29 @@ bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops) {
       FlowOp& op = ops[at];
       op.dst_rank[op.n_dst] = (uint8_t)r; op.dst_off[op.n_dst++] = a.dst_off;
     }
+  // Shapes that the kernel has straight code for: one accumulator (rings), and even trees of 4 and 8 operands in pairs and fours (recursive algorithms).
+  auto even_tree = [](const FlowOp& op, int r0, int r1, int r2) {
+    if (op.n_leaf != r0 * r1 * r2 || op.before) return false;
+    for (int i = 0; i < op.n_leaf; i++) {
+      const int a = i % r0, b = i / r0 % r1, c = i / (r0 * r1);
+      // groups behind the first of their kind have an accumulator of their own, one up for each kind
+      const int level = (b > 0) + (c > 0);
+      int place = level | (a == 0 ? 4 : 0), done = 0;
+      if (a == r0 - 1) { place |= b > 0 ? 0x20 << done : 0; done++; }
+      if (a == r0 - 1 && b == r1 - 1 && r2 > 1) { place |= c > 0 ? 0x20 << done : 0; done++; }
+      if (op.place[i] != (place | done << 3)) return false;
+    }
+    return true;
+  };
+  for (FlowOp& op : ops) {
+    if (!op.nested) continue;
+    bool chain = true;
+    for (int i = 0; i < op.n_leaf; i++) chain &= (op.place[i] & 3) == 0;
+    if (chain) op.shape = FLOW_CHAIN;
+    else if (even_tree(op, 2, 2, 1) || even_tree(op, 2, 2, 2)) op.shape = 2 | 2 << 4;
+    else if (even_tree(op, 4, 2, 1)) op.shape = 4 | 2 << 4;
+    else if (even_tree(op, 2, 4, 1)) op.shape = 2 | 4 << 4;
+  }
   // Elements of a buffer that no other operation reads may leave the cache with their use.
   for (size_t i = 0; i < ops.size(); i++) {
     bool again = false;

@@ -78,8 +78,9 @@ struct FlowOp {
   uint8_t scaled = 0, rounded = 0;      // bit i: leaf i is an original contribution (pre-scaled for avg), which is rounded once scaled
   uint8_t once = 0;              // 1: no other operation reads the leaves
   uint8_t before = 0;            // bit i: leaf i is the left operand of what it is folded into
-  uint8_t pad[1] = {0};
+  uint8_t shape = 0;             // of a nested expression: 0 any, FLOW_CHAIN, or the radices of an even tree, innermost first: r0 | r1 << 4 (a third one is 2)
 };
+constexpr uint8_t FLOW_CHAIN = 1;      // one accumulator
 static_assert(sizeof(FlowOp) == 176, "FlowOp layout is shared with device code");
 
 struct Program {

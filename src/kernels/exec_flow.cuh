@@ -20,8 +20,13 @@ template <typename T, int OP, int LEVELS> struct FlowAcc {
     }
   }
   static __device__ __forceinline__ void fold(A (&s)[N], const A (&x)[N], bool first) {
+    if (first) {
 #pragma unroll
-    for (int e = 0; e < N; e++) s[e] = first ? x[e] : red<OP, A>(s[e], x[e]);
+      for (int e = 0; e < N; e++) s[e] = x[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < N; e++) s[e] = red<OP, A>(s[e], x[e]);
+    }
   }
   static __device__ __forceinline__ void fold_before(A (&s)[N], const A (&x)[N]) {
 #pragma unroll
@@ -57,6 +62,57 @@ template <typename T, int OP, int LEVELS> struct FlowAcc {
   }
 };
 
+// The shapes that most calls have, without a branch per leaf: the general form works as long as it waits (us, general and this: reduce-scatter 8 x 8 MiB on the ring 128 / 98, reduce 8 x 16 MiB
+// 38 / 28, all-reduce 4 x 25 MiB averaged by recursive doubling 43 / 38, maximum of 8 x 8 MB in fours and pairs 53 / 31).
+template <typename T, int OP> struct FlowEval {
+  typedef typename AccOf<T>::type A;
+  static constexpr int N = Pack<T>::N;
+  typedef FlowAcc<T, OP, 2> Acc;
+  static __device__ __forceinline__ void get(const uint4& v, int i, int scaled, float scale, A (&x)[N]) {
+    Pack<T>::up(v, x);
+    if (scaled >> i & 1) {
+#pragma unroll
+      for (int e = 0; e < N; e++) x[e] = scale_operand<T, A>(x[e], scaled, i, scale);
+    }
+  }
+  // one accumulator: a ring's hops
+  template <int LEAVES, class V> static __device__ __forceinline__ void chain(const V& v, const FlowOp& op, int scaled, float scale, A (&s)[N]) {
+    get(v(0), 0, scaled, scale, s);
+#pragma unroll
+    for (int i = 1; i < LEAVES; i++) {
+      if (i < op.n_leaf) {
+        A x[N];
+        get(v(i), i, scaled, scale, x);
+        if (OP >= 2 && (op.before >> i & 1)) Acc::fold_before(s, x); else Acc::fold(s, x, false);
+        if (op.place[i] >> 3 & 3) Acc::round(s);
+      }
+    }
+  }
+  template <int FIRST, int R0, int R1, int R2, class V> static __device__ __forceinline__ void tree(const V& v, int scaled, float scale, A (&s)[N]) {
+    if constexpr (R2 > 1) {
+      tree<FIRST, R0, R1, 1>(v, scaled, scale, s); Acc::round(s);
+      A x[N];
+      tree<FIRST + R0 * R1, R0, R1, 1>(v, scaled, scale, x); Acc::round(x);
+      Acc::fold(s, x, false);
+    } else if constexpr (R1 > 1) {
+      tree<FIRST, R0, 1, 1>(v, scaled, scale, s); Acc::round(s);
+#pragma unroll
+      for (int b = 1; b < R1; b++) {
+        A x[N];
+        if (b == 1) tree<FIRST + R0, R0, 1, 1>(v, scaled, scale, x);
+        else if (b == 2) tree<(R1 > 2 ? FIRST + 2 * R0 : 0), R0, 1, 1>(v, scaled, scale, x);
+        else tree<(R1 > 3 ? FIRST + 3 * R0 : 0), R0, 1, 1>(v, scaled, scale, x);
+        Acc::round(x);
+        Acc::fold(s, x, false);
+      }
+    } else {
+      get(v(FIRST), FIRST, scaled, scale, s);
+#pragma unroll
+      for (int a = 1; a < R0; a++) { A x[N]; get(v(FIRST + a), FIRST + a, scaled, scale, x); Acc::fold(s, x, false); }
+    }
+  }
+};
+
 // Packs of an operation with nested results; LEAVES: at least as many as it has.
 template <typename T, int OP, int LEAVES, int U>
 __device__ __forceinline__ void flow_tree(const FlowOp& op, const char* const* src, char* const* dst, int n, int scaled, float scale, bool dst_done) {
@@ -72,10 +128,21 @@ __device__ __forceinline__ void flow_tree(const FlowOp& op, const char* const* s
       for (int u = 0; u < U; u++) v[i][u] = ld_slot(sp[i] + (size_t)min(p + u * kFlowBlock, n - 1) * 16);
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      FlowAcc<T, OP, LEAVES <= 4 ? 2 : kFlowLevels> acc;
+      typedef FlowEval<T, OP> E;
+      typename E::A s[E::N];
+      auto leaf = [&](int i) -> const uint4& { return v[i][u]; };
+      if (op.shape == FLOW_CHAIN) E::template chain<LEAVES>(leaf, op, scaled, scale, s);
+      else if (op.shape == (2 | 2 << 4)) E::template tree<0, 2, 2, LEAVES / 4>(leaf, scaled, scale, s);
+      else if (LEAVES == 8 && op.shape == (4 | 2 << 4)) { if constexpr (LEAVES == 8) E::template tree<0, 4, 2, 1>(leaf, scaled, scale, s); }
+      else if (LEAVES == 8 && op.shape == (2 | 4 << 4)) { if constexpr (LEAVES == 8) E::template tree<0, 2, 4, 1>(leaf, scaled, scale, s); }
+      else {
+        FlowAcc<T, OP, LEAVES <= 4 ? 2 : kFlowLevels> acc;
 #pragma unroll
-      for (int i = 0; i < LEAVES; i++) if (i < op.n_leaf) acc.leaf(v[i][u], i, op.place[i], op.before >> i & 1, scaled, scale);
-      const uint4 o = Pack<T>::down(acc.s0);
+        for (int i = 0; i < LEAVES; i++) if (i < op.n_leaf) acc.leaf(v[i][u], i, op.place[i], op.before >> i & 1, scaled, scale);
+#pragma unroll
+        for (int e = 0; e < E::N; e++) s[e] = acc.s0[e];
+      }
+      const uint4 o = Pack<T>::down(s);
       if (p + u * kFlowBlock < n) for (int d = 0; d < op.n_dst; d++) st_hint(dst[d] + (size_t)(p + u * kFlowBlock) * 16, o, policy);
     }
   }
@@ -85,7 +152,7 @@ template <typename T, int OP>
 __device__ __noinline__ void flow_tree_shift(const FlowOp& op, const char* const* src, char* const* dst, long long npack, int scaled, float scale) {
   const int lane = threadIdx.x & 31;
   for (long long run = threadIdx.x & ~31; run < npack; run += kFlowBlock) {
-    FlowAcc<T, OP, kFlowLevels> acc;
+    FlowAcc<T, OP, kFlowLevels> acc;      // (the general form: what comes at odd addresses is bound by its shifts)
 #pragma unroll 1
     for (int i0 = 0; i0 < op.n_leaf; i0 += 4) {            // four leaves' loads in flight
       RunWords<1> r[4];
