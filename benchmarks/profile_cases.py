@@ -2,6 +2,7 @@
 
     python benchmarks/profile_cases.py exec      # fused collective executor: 2 virtual ranks, ring all-reduce of 256 MiB fp32
     python benchmarks/profile_cases.py exec8     # the same among 8 virtual ranks, 32 MiB fp32 each
+    python benchmarks/profile_cases.py flow      # data flow of a ring all-reduce, 8 virtual ranks, 32 MiB fp32 each
     python benchmarks/profile_cases.py exec_ll   # low-latency all-reduce, 8 virtual ranks, 16 KiB
     python benchmarks/profile_cases.py gemm      # tcgen05 GEMM 8192 x 8192 x 3584 bf16
     python benchmarks/profile_cases.py direct    # DIRECT all-reduce, 8 virtual ranks, 16 MiB fp32
@@ -30,19 +31,31 @@ sys.path.insert(0, str(Path(__file__).resolve().parent.parent))
 def _group8():
     """Eight ranks with FIFOs of 128 KiB slots for the 18 CTAs that each gets: 1.2 GiB of heaps for FIFOs and low-latency slots instead of 10."""
     from piccl_b200.parallel.comm import LoopbackGroup, make_config
-    return LoopbackGroup(8, config=make_config(max_cta=18, nslot=4, slot_bytes=128 << 10, scratch_bytes=1 << 20))
+    return LoopbackGroup(8, config=make_config(max_cta=18, nslot=4, slot_bytes=128 << 10, scratch_bytes=1 << 20)).slots_only()
 
 
 def case_exec(ranks: int = 2, count: int = 64 << 20, algo: str = "RING"):
     from piccl_b200.parallel.comm import LoopbackGroup
     n = ranks
-    g = LoopbackGroup(n) if n == 2 else _group8()
+    g = LoopbackGroup(n).slots_only() if n == 2 else _group8()
     xs = [torch.ones(count, device="cuda") for _ in range(n)]
     outs = [torch.empty_like(x) for x in xs]
     for _ in range(4):
         g.run("allreduce", xs, outs, count, algo=algo)
     torch.cuda.synchronize()
     assert g.status().aborted == 0
+    g.close()
+
+
+def case_flow():
+    n, count = 8, 8 << 20
+    g = _group8().slots_only(False)
+    xs = [torch.full((count,), float(r + 1), device="cuda") for r in range(n)]
+    outs = [torch.empty_like(x) for x in xs]
+    for _ in range(4):
+        g.run("allreduce", xs, outs, count, algo="RING")
+    torch.cuda.synchronize()
+    assert g.status().aborted == 0 and float(outs[3][12345]) == n * (n + 1) / 2
     g.close()
 
 
@@ -59,7 +72,7 @@ def case_gemm():
 def case_direct():
     from piccl_b200.parallel.comm import LoopbackGroup
     n, count = 8, 4 << 20
-    g = LoopbackGroup(n)
+    g = LoopbackGroup(n).slots_only()
     xs = [torch.full((count,), float(r + 1), device="cuda") for r in range(n)]
     outs = [torch.empty_like(x) for x in xs]
     for _ in range(4):
@@ -73,7 +86,7 @@ def case_tp():
     from piccl_b200.parallel import tp
     from piccl_b200.parallel.comm import LoopbackGroup, make_config
     n, M, N, K = 2, 4096, 4096, 2048
-    g = LoopbackGroup(n, config=make_config(tp_bytes=tp.workspace_bytes("gemm_rs", n, M, N, K)))
+    g = LoopbackGroup(n, config=make_config(tp_bytes=tp.workspace_bytes("gemm_rs", n, M, N, K))).slots_only()
     As = [torch.randn(M, K, device="cuda").to(torch.bfloat16) for _ in range(n)]
     Bs = [torch.randn(N, K, device="cuda").to(torch.bfloat16) for _ in range(n)]
     outs = [torch.empty(M // n, N, device="cuda", dtype=torch.bfloat16) for _ in range(n)]
@@ -114,7 +127,7 @@ def case_ag_gemm():
     from piccl_b200.parallel import tp
     from piccl_b200.parallel.comm import LoopbackGroup, make_config
     n, M, N, K = 2, 4096, 2048, 4096
-    g = LoopbackGroup(n, config=make_config(tp_bytes=tp.workspace_bytes("ag_gemm", n, M, N, K)))
+    g = LoopbackGroup(n, config=make_config(tp_bytes=tp.workspace_bytes("ag_gemm", n, M, N, K))).slots_only()
     As = [torch.randn(M // n, K, device="cuda").to(torch.bfloat16) for _ in range(n)]
     Bs = [torch.randn(N, K, device="cuda").to(torch.bfloat16) for _ in range(n)]
     outs = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(n)]
@@ -190,5 +203,5 @@ def case_ce():
 
 if __name__ == "__main__":
     which = sys.argv[1] if len(sys.argv) > 1 else "exec"
-    {"exec": case_exec, "exec8": lambda: case_exec(8, 8 << 20), "exec_ll": lambda: case_exec(8, 4096, "PRD"), "gemm": case_gemm, "direct": case_direct, "tp": case_tp, "ln": case_ln, "ce": case_ce, "nvls": case_nvls, "llf": case_llf, "ag_gemm": case_ag_gemm, "attention": case_attention, "elementwise": case_elementwise}[which]()
+    {"exec": case_exec, "flow": case_flow, "exec8": lambda: case_exec(8, 8 << 20), "exec_ll": lambda: case_exec(8, 4096, "PRD"), "gemm": case_gemm, "direct": case_direct, "tp": case_tp, "ln": case_ln, "ce": case_ce, "nvls": case_nvls, "llf": case_llf, "ag_gemm": case_ag_gemm, "attention": case_attention, "elementwise": case_elementwise}[which]()
     print(f"profile case {which} done")

@@ -3,8 +3,9 @@
 `Communicator` is one rank of a multi-process job (one process per GPU); the
 heap handles are exchanged through torch.distributed.  `LoopbackGroup` holds
 several virtual ranks on ONE device inside one process and runs each collective
-as a single cooperative kernel launch — the way to exercise the multi-rank
-protocol when only one GPU is at hand.
+as a single kernel launch: from what the call computes where buffers do not
+overlap, else as the ranks' programs, which `slots_only` asks for in any case — the
+way to exercise the multi-rank protocol when only one GPU is at hand.
 
 The collectives mirror the reference's intercepted entry points
 (src/piccl.c:29-173) but can also be called directly, with the algorithm and k
@@ -195,6 +196,12 @@ class LoopbackGroup(_CommBase):
         if self._comms is None:
             self._comms = self._pack(*[h.value for h in self._hs])
         return self._comms
+
+    def slots_only(self, on: bool = True) -> "LoopbackGroup":
+        """Everything that crosses goes through the ranks' slots and workspaces, as between GPUs, although one launch carries all ranks."""
+        for h in self._hs:
+            self._lib.piccl_test_slots_only(h, int(on))
+        return self
 
     def status(self, rank: int = 0) -> N.Status:
         s = N.Status()
