@@ -7,7 +7,7 @@
 // computed once and stored in all their buffers.  Nothing in such a call waits (kernels/exec_flow.cuh).
 //
 // us through the slots and this, one B200: all-reduce 4 x 25 MiB averaged by recursive doubling 131 / 38, 8 x 64 MiB on the ring 353 / 188, 8 x 280 KB 45 / 4.8, 8 x 4 KB 37 / 4.7; all-gather 4 x 1 MiB at
-// odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34; broadcast 8 x 16 MiB 110 / 27; 8 x 8 MiB 196 / 98; reduce 8 x 16 MiB on the ring 92 / 28, in two rings 120 / 69.
+// odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34; broadcast 8 x 16 MiB 110 / 27; 8 x 8 MiB 196 / 98; reduce 8 x 16 MiB on the ring 92 / 28, in two rings 120 / 56.
 #include <algorithm>
 #include <map>
 #include "coll_internal.h"

@@ -136,9 +136,13 @@ __device__ __forceinline__ void flow_tree(const FlowOp& op, const char* const* s
       else if (LEAVES == 8 && op.shape == (4 | 2 << 4)) { if constexpr (LEAVES == 8) E::template tree<0, 4, 2, 1>(leaf, scaled, scale, s); }
       else if (LEAVES == 8 && op.shape == (2 | 4 << 4)) { if constexpr (LEAVES == 8) E::template tree<0, 2, 4, 1>(leaf, scaled, scale, s); }
       else {
+        // a loop over an array in local memory: written out per leaf, the code is so long that a small call spends 5 us fetching it
         FlowAcc<T, OP, LEAVES <= 4 ? 2 : kFlowLevels> acc;
+        uint4 w[LEAVES];
 #pragma unroll
-        for (int i = 0; i < LEAVES; i++) if (i < op.n_leaf) acc.leaf(v[i][u], i, op.place[i], op.before >> i & 1, scaled, scale);
+        for (int i = 0; i < LEAVES; i++) w[i] = v[i][u];
+#pragma unroll 1
+        for (int i = 0; i < op.n_leaf; i++) acc.leaf(w[i], i, op.place[i], op.before >> i & 1, scaled, scale);
 #pragma unroll
         for (int e = 0; e < E::N; e++) s[e] = acc.s0[e];
       }
@@ -152,7 +156,7 @@ template <typename T, int OP>
 __device__ __noinline__ void flow_tree_shift(const FlowOp& op, const char* const* src, char* const* dst, long long npack, int scaled, float scale) {
   const int lane = threadIdx.x & 31;
   for (long long run = threadIdx.x & ~31; run < npack; run += kFlowBlock) {
-    FlowAcc<T, OP, kFlowLevels> acc;      // (the general form: what comes at odd addresses is bound by its shifts)
+    FlowAcc<T, OP, kFlowLevels> acc;      // (the general form: what comes at odd addresses is bound by its shifts; a loop over an array, as above, takes half as long again)
 #pragma unroll 1
     for (int i0 = 0; i0 < op.n_leaf; i0 += 4) {            // four leaves' loads in flight
       RunWords<1> r[4];
@@ -195,8 +199,12 @@ __global__ void __launch_bounds__(kFlowBlock, 3) exec_flow_kernel(const FlowArgs
       if (tid < len - nfull * N) {                         // the last, partial pack, an element a thread
         typedef typename AccOf<T>::type A;
         A s[kFlowLevels];
+        T raw[kFlowLeaves];
+#pragma unroll
+        for (int i = 0; i < kFlowLeaves; i++) if (i < op.n_leaf) raw[i] = *reinterpret_cast<const volatile T*>(reinterpret_cast<const T*>(s_src[i]) + nfull * N + tid);
+#pragma unroll 1
         for (int i = 0; i < op.n_leaf; i++) {
-          const A x = scale_operand<T, A>(Cvt<T>::up(*(reinterpret_cast<const T*>(s_src[i]) + nfull * N + tid)), scaled, i, fa.scale);
+          const A x = scale_operand<T, A>(Cvt<T>::up(raw[i]), scaled, i, fa.scale);
           int level = op.place[i] & 3, merges = op.place[i] >> 5;
           s[level] = op.place[i] & 4 ? x : op.before >> i & 1 ? red<OP, A>(x, s[level]) : red<OP, A>(s[level], x);
           for (int k = op.place[i] >> 3 & 3; k > 0; k--, merges >>= 1) {
