@@ -37,7 +37,7 @@ template <typename T, int OP, int LEVELS> struct FlowAcc {
     Pack<T>::up(v, x);
     if (scaled >> i & 1) {
 #pragma unroll
-      for (int e = 0; e < N; e++) x[e] = scale_operand<T, A>(x[e], scaled, i, scale);
+      for (int e = 0; e < N; e++) x[e] = scale_operand<T, true>(x[e], scaled, i, scale);
     }
     int level = place & 3;
     const bool first = place & 4;
@@ -72,7 +72,7 @@ template <typename T, int OP> struct FlowEval {
     Pack<T>::up(v, x);
     if (scaled >> i & 1) {
 #pragma unroll
-      for (int e = 0; e < N; e++) x[e] = scale_operand<T, A>(x[e], scaled, i, scale);
+      for (int e = 0; e < N; e++) x[e] = scale_operand<T, true>(x[e], scaled, i, scale);
     }
   }
   // one accumulator: a ring's hops
@@ -171,6 +171,26 @@ __device__ __noinline__ void flow_tree_shift(const FlowOp& op, const char* const
   }
 }
 
+// The last, partial pack of an operation without nested results.  All operands are on their way before the first is used: one after the other, eight cost six microseconds at the end of a call.
+template <typename T, int OP>
+__device__ __noinline__ void flow_elem(const FlowOp& op, const char* const* src, char* const* dst, long long first, long long nelem, int scaled, float scale) {
+  typedef typename AccOf<T>::type A;
+  for (long long i = first + threadIdx.x; i < nelem; i += kFlowBlock) {
+    T raw[kFlowLeaves];
+#pragma unroll
+    for (int s = 0; s < kFlowLeaves; s++) if (s < op.n_leaf) raw[s] = *reinterpret_cast<const volatile T*>(reinterpret_cast<const T*>(src[s]) + i);
+    A acc = A();
+#pragma unroll
+    for (int s = 0; s < kFlowLeaves; s++)
+      if (s < op.n_leaf) {
+        const A x = scale_operand<T, true>(Cvt<T>::up(raw[s]), scaled, s, scale);
+        acc = s == 0 ? x : red<OP, A>(acc, x);
+      }
+    const T o = Cvt<T>::down(acc);
+    for (int d = 0; d < op.n_dst; d++) reinterpret_cast<T*>(dst[d])[i] = o;
+  }
+}
+
 template <typename T, int OP, bool SHIFT>
 __global__ void __launch_bounds__(kFlowBlock, 3) exec_flow_kernel(const FlowArgs fa) {
   constexpr int esz = (int)sizeof(T), N = Pack<T>::N;
@@ -204,7 +224,7 @@ __global__ void __launch_bounds__(kFlowBlock, 3) exec_flow_kernel(const FlowArgs
         for (int i = 0; i < kFlowLeaves; i++) if (i < op.n_leaf) raw[i] = *reinterpret_cast<const volatile T*>(reinterpret_cast<const T*>(s_src[i]) + nfull * N + tid);
 #pragma unroll 1
         for (int i = 0; i < op.n_leaf; i++) {
-          const A x = scale_operand<T, A>(Cvt<T>::up(raw[i]), scaled, i, fa.scale);
+          const A x = scale_operand<T, true>(Cvt<T>::up(raw[i]), scaled, i, fa.scale);
           int level = op.place[i] & 3, merges = op.place[i] >> 5;
           s[level] = op.place[i] & 4 ? x : op.before >> i & 1 ? red<OP, A>(x, s[level]) : red<OP, A>(s[level], x);
           for (int k = op.place[i] >> 3 & 3; k > 0; k--, merges >>= 1) {
@@ -217,9 +237,9 @@ __global__ void __launch_bounds__(kFlowBlock, 3) exec_flow_kernel(const FlowArgs
     }
     return;
   }
-  if constexpr (SHIFT) { if (nfull) reduce_copy_shift<T, OP>(kFlowBlock, op.n_leaf, s_src, op.n_dst, s_dst, nfull, scaled, fa.scale); }
+  if constexpr (SHIFT) { if (nfull) reduce_copy_shift<T, OP, true>(kFlowBlock, op.n_leaf, s_src, op.n_dst, s_dst, nfull, scaled, fa.scale); }
   else if (nfull) move_aligned<T, OP, true>(kFlowBlock, s_src, op.n_leaf, s_dst, op.n_dst, (int)nfull, scaled, fa.scale, L2Hints{(fa.leave_first & 1) && op.once, dst_done, 0, 0});
-  if (nfull * N < len) reduce_copy_elem<T, OP>(kFlowBlock, op.n_leaf, s_src, -1, op.n_dst, s_dst, nfull * N, len, scaled, fa.scale);
+  if (nfull * N < len) flow_elem<T, OP>(op, s_src, s_dst, nfull * N, len, scaled, fa.scale);
 }
 
 }  // namespace piccl

@@ -124,12 +124,13 @@ template <> __device__ __forceinline__ float scale_val<float>(float v, float s) 
 template <> __device__ __forceinline__ double scale_val<double>(double v, float s) { return v * (double)s; }
 
 // Operands to scale (avg): bit s, operand s is an original contribution; bit 8 + s, of another rank, which would have put it into a slot: it is rounded to the
-// element type as it would be there, so that a call's result does not depend on how its operands came.
+// element type as it would be there, so that a call's result does not depend on how its operands came.  FLOW: only a data flow has such operands; in the executor, where the lone operand to scale is the
+// rank's own, the test for them cost the loops of 16-bit types a tenth, also those that scale nothing (reduce of 8 x 16 MiB of bf16 in two rings 120 us, with it 133; reduce-scatter of 8 x 8 MiB averaged on the ring 211 and 218).
 constexpr int kRoundedShift = 8;
-template <typename T, typename A> __device__ __forceinline__ A scale_operand(A v, int scaled, int s, float scale) {
+template <typename T, bool FLOW, typename A> __device__ __forceinline__ A scale_operand(A v, int scaled, int s, float scale) {
   if (scaled >> s & 1) {
     v = scale_val<A>(v, scale);
-    if (scaled >> (s + kRoundedShift) & 1) v = Cvt<T>::up(Cvt<T>::down(v));
+    if (FLOW && (scaled >> (s + kRoundedShift) & 1)) v = Cvt<T>::up(Cvt<T>::down(v));
   }
   return v;
 }
@@ -170,7 +171,7 @@ static __device__ __noinline__ bool wait_counter(const unsigned long long* flag,
 // wrote.  The last round is as wide as the others instead of being finished a pack at a time, which took up to U - 1 further round trips: what lies
 // beyond the end loads the last pack again (loads under a condition made the compiler spill).  The slots' packs may
 // have been written by another GPU and the local operand is read once: all loads go past L1.
-template <typename T, int OP, int NSRC, bool SCALE>
+template <typename T, int OP, bool FLOW, int NSRC, bool SCALE>
 __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, int scaled, float scale) {      // v[s * stride]: operand s
   if constexpr (OP == OP_COPY) return v[0];
   else {
@@ -181,7 +182,7 @@ __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, i
     Pack<T>::up(v[0], acc);
     if (SCALE) {
 #pragma unroll
-      for (int e = 0; e < N; e++) acc[e] = scale_operand<T, A>(acc[e], scaled, 0, scale);
+      for (int e = 0; e < N; e++) acc[e] = scale_operand<T, FLOW>(acc[e], scaled, 0, scale);
     }
 #pragma unroll
     for (int s = 1; s < NSRC; s++) {
@@ -189,7 +190,7 @@ __device__ __forceinline__ uint4 combine(const uint4* v, int stride, int nsrc, i
         A x[N]; Pack<T>::up(v[s * stride], x);
         if (SCALE) {
 #pragma unroll
-          for (int e = 0; e < N; e++) x[e] = scale_operand<T, A>(x[e], scaled, s, scale);
+          for (int e = 0; e < N; e++) x[e] = scale_operand<T, FLOW>(x[e], scaled, s, scale);
         }
 #pragma unroll
         for (int e = 0; e < N; e++) acc[e] = red<OP, A>(acc[e], x[e]);
@@ -233,7 +234,7 @@ __device__ __forceinline__ void stream(int nt, const char* const* src, int nsrc_
 #pragma unroll
       for (int u = 0; u < U; u++) v[s][u] = get(s, (p + u * nt) * 16);
 #pragma unroll
-    for (int u = 0; u < U; u++) put((p + u * nt) * 16, combine<T, OP, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
+    for (int u = 0; u < U; u++) put((p + u * nt) * 16, combine<T, OP, FLOW, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
   }
   if (U > 1 && p < n) {
     uint4 v[NSRC][U];
@@ -242,7 +243,7 @@ __device__ __forceinline__ void stream(int nt, const char* const* src, int nsrc_
 #pragma unroll
       for (int u = 0; u < U - 1; u++) v[s][u] = get(s, min(p + u * nt, n - 1) * 16);
 #pragma unroll
-    for (int u = 0; u < U - 1; u++) if (p + u * nt < n) put((p + u * nt) * 16, combine<T, OP, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
+    for (int u = 0; u < U - 1; u++) if (p + u * nt < n) put((p + u * nt) * 16, combine<T, OP, FLOW, NSRC, SCALE>(&v[0][u], U, nsrc, scaled, scale));
   }
 }
 template <typename T, int OP, bool FLOW>
@@ -378,7 +379,7 @@ __device__ __noinline__ void copy_shift(int nt, const char* src, int ndst, char*
     store_run<RUN>(o, ndst, dst, run, lane, npack);
   }
 }
-template <typename T, int OP, int RUN>
+template <typename T, int OP, bool FLOW, int RUN>
 __device__ __noinline__ void reduce_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, long long npack, int scaled, float scale) {
   typedef typename AccOf<T>::type A;
   constexpr int N = Pack<T>::N;
@@ -389,7 +390,7 @@ __device__ __noinline__ void reduce_shift(int nt, int nsrc, const char* const* s
       Pack<T>::up(run_pack(r, u, m, lane), x);
       if (scaled >> s & 1) {
 #pragma unroll
-        for (int e = 0; e < N; e++) x[e] = scale_operand<T, A>(x[e], scaled, s, scale);
+        for (int e = 0; e < N; e++) x[e] = scale_operand<T, FLOW>(x[e], scaled, s, scale);
       }
     };
     {                                                // two operands' loads in flight, beside no accumulators yet
@@ -426,7 +427,7 @@ __device__ __noinline__ void reduce_shift(int nt, int nsrc, const char* const* s
   }
 }
 // A warp takes runs of 2, 4 or 8 blocks (sums: 2 or 4): as few rounds as can be, and then over as many warps.
-template <typename T, int OP>
+template <typename T, int OP, bool FLOW>
 __device__ __forceinline__ void reduce_copy_shift(int nt, int nsrc, const char* const* src, int ndst, char* const* dst, long long npack, int scaled, float scale) {
   const long long blocks = (npack + nt - 1) / nt;      // per warp
   if (OP == OP_COPY || (nsrc == 1 && !scaled)) {
@@ -434,29 +435,27 @@ __device__ __forceinline__ void reduce_copy_shift(int nt, int nsrc, const char* 
     else if (blocks > 2) copy_shift<T, OP, 4>(nt, src[0], ndst, dst, npack);
     else copy_shift<T, OP, 2>(nt, src[0], ndst, dst, npack);
   } else if constexpr (OP != OP_COPY) {
-    if (blocks > 2) reduce_shift<T, OP, 4>(nt, nsrc, src, ndst, dst, npack, scaled, scale);
-    else reduce_shift<T, OP, 2>(nt, nsrc, src, ndst, dst, npack, scaled, scale);
+    if (blocks > 2) reduce_shift<T, OP, FLOW, 4>(nt, nsrc, src, ndst, dst, npack, scaled, scale);
+    else reduce_shift<T, OP, FLOW, 2>(nt, nsrc, src, ndst, dst, npack, scaled, scale);
   }
 }
 
-// Element-wise path: the last, partial pack of an action.  All operands are on their way before the first is used: one after the other, eight cost six microseconds at the end of a call.
+// Element-wise path: the last, partial pack of an action, an operand after the other.  (A data flow's has all operands on their way first, exec_flow.cuh.  In this kernel that form, which needs a register
+// for each operand, makes the loops above slower although it hardly ever runs: reduce of 8 x 16 MiB in two rings 111 us, with it 123, in rings of four 101 and 110; 8 x 52 MiB of fp64 averaged by DIRECT 267 and 292.)
 template <typename T, int OP>
 __device__ __noinline__ void reduce_copy_elem(int nt, int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
-                                                 long long first, long long nelem, int scaled, float scale) {
+                                                 long long first, long long nelem, bool do_scale, float scale) {
   typedef typename AccOf<T>::type A;
   for (long long i = first + threadIdx.x; i < nelem; i += nt) {
-    T raw[kMaxActionPeers + 1];
-#pragma unroll
-    for (int s = 0; s < kMaxActionPeers + 1; s++)
-      if (s < nsrc) { const T* p = reinterpret_cast<const T*>(src[s]) + i; raw[s] = (local_src == s) ? *p : *reinterpret_cast<const volatile T*>(p); }
     A acc = A();
-#pragma unroll
-    for (int s = 0; s < kMaxActionPeers + 1; s++)
-      if (s < nsrc) {
-        const A x = scale_operand<T, A>(Cvt<T>::up(raw[s]), scaled, s, scale);
-        acc = (s == 0) ? x : red<OP, A>(acc, x);
-      }
-    T o = Cvt<T>::down(acc);
+    for (int s = 0; s < nsrc; s++) {
+      const T* p = reinterpret_cast<const T*>(src[s]) + i;
+      const T raw = local_src == s ? *p : *reinterpret_cast<const volatile T*>(p);
+      A x = Cvt<T>::up(raw);
+      if (do_scale && local_src == s) x = scale_val<A>(x, scale);
+      acc = s == 0 ? x : red<OP, A>(acc, x);
+    }
+    const T o = Cvt<T>::down(acc);
     for (int d = 0; d < ndst; d++) reinterpret_cast<T*>(dst[d])[i] = o;
   }
 }
@@ -531,9 +530,9 @@ __global__ void __launch_bounds__(kMaxBlock + kCtlThreads, 1) exec_kernel(const 
         const bool do_scale = flags & STEP_SCALE;
         constexpr int N = Pack<T>::N;
         const long long nfull = (SHIFT || (flags & STEP_ALIGNED)) ? len / N : 0;
-        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP>(ndata, nsrc, src, ndst, dst, nfull, do_scale ? 1 << local_src : 0, ka.scale); }
+        if constexpr (SHIFT) { if (nfull && ndst) reduce_copy_shift<T, OP, false>(ndata, nsrc, src, ndst, dst, nfull, do_scale ? 1 << local_src : 0, ka.scale); }
         else if (nfull) move_aligned<T, OP, false>(ndata, src, nsrc, dst, ndst, (int)nfull, do_scale ? 1 << local_src : 0, ka.scale, L2Hints{(flags & STEP_SRC_DONE) != 0, (flags & STEP_DST_DONE) != 0, local_src, st.local_dst});
-        if (nfull * N < len) reduce_copy_elem<T, OP>(ndata, nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale ? 1 << local_src : 0, ka.scale);
+        if (nfull * N < len) reduce_copy_elem<T, OP>(ndata, nsrc, src, local_src, ndst, dst, nfull * N, len, do_scale, ka.scale);
       }
       bar_arrive_n(kDone + d, ndata + 32);
       if (flags & (STEP_END | STEP_FAIL)) return;

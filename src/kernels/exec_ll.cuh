@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
           for (int e = 0; e < E; e++) if (u * E + e < len) un.t[e] = from[u * E + e];
         }
 #pragma unroll
-        for (int e = 0; e < E; e++) v[e] = scale_operand<T, A>(Cvt<T>::up(un.t[e]), scaled, 0, ka.scale);
+        for (int e = 0; e < E; e++) v[e] = scale_operand<T, false>(Cvt<T>::up(un.t[e]), scaled, 0, ka.scale);
       };
       const bool src_whole = (reinterpret_cast<uintptr_t>(lsrc) & 7) == 0, dst_whole = (reinterpret_cast<uintptr_t>(ldst) & 7) == 0;
 
