@@ -9,6 +9,7 @@
 // us through the slots and this, one B200: all-reduce 4 x 25 MiB averaged by recursive doubling 131 / 38, 8 x 64 MiB on the ring 353 / 188, 8 x 280 KB 45 / 4.8, 8 x 4 KB 37 / 4.7; all-gather 4 x 1 MiB at
 // odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34; broadcast 8 x 16 MiB 110 / 27; 8 x 8 MiB 196 / 98; reduce 8 x 16 MiB on the ring 92 / 28, in two rings 120 / 56.
 #include <algorithm>
+#include <array>
 #include <map>
 #include "coll_internal.h"
 
@@ -128,7 +129,22 @@ struct Flow {
 
 }  // namespace
 
-bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops) {
+// Integers: one fold of all operands, whatever the nesting was, in the ranks' order so that all ranks' expressions are alike.  Evaluated as nested expressions, 8-bit elements, sixteen to a pack, were
+// slower than through the slots (us through the slots, nested, and this: maximum of 8 x 16 MiB of bytes in two rings 197, 1018, 35; product of 8 x 5 KB in fours 8.8, 23.6, 4.7; reduce-scatter of 8 x 2 MB on the ring at odd
+// addresses 532, 812, 78).
+static void flatten(FlowOp& op) {
+  std::array<int, kFlowLeaves> order;
+  for (int i = 0; i < op.n_leaf; i++) order[i] = i;
+  std::sort(order.begin(), order.begin() + op.n_leaf, [&](int a, int b) { return std::make_pair(op.leaf_rank[a], op.leaf_off[a]) < std::make_pair(op.leaf_rank[b], op.leaf_off[b]); });
+  const FlowOp was = op;
+  for (int i = 0; i < op.n_leaf; i++) {
+    op.leaf_rank[i] = was.leaf_rank[order[i]]; op.leaf_buf[i] = was.leaf_buf[order[i]]; op.leaf_off[i] = was.leaf_off[order[i]];
+    op.place[i] = i == 0 ? 4 : 0;
+  }
+  op.nested = op.scaled = op.rounded = op.before = 0;
+}
+
+bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, bool integers) {
   const int n = (int)progs.size();
   ops.clear();
   Flow f(progs);
@@ -160,6 +176,7 @@ bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops) {
         if (it != made.end()) at = it->second;
         else {
           f.fold(m, 0);
+          if (integers && f.ok) flatten(f.op);
           for (size_t q = 0; q < ops.size() && f.ok && at < 0; q++) if (ops[q].n_leaf > 1 && alike(ops[q], f.op)) at = (int)q;
         }
       }

@@ -122,8 +122,8 @@ Resolved resolve(Coll coll, Algo algo, int k, int nranks);
 Program compile(const CollArgs& a, int rank);
 
 // The operations of a call, from the programs of ALL its ranks.  The caller vouches that no rank's receive buffer overlaps another rank's buffers or its own send
-// buffer (in place: all-gather and broadcast only).  false: they have no such form.
-bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops);
+// buffer (in place: all-gather and broadcast only).  integers: elements for which operands give the same result in any order, no partial result being rounded.  false: they have no such form.
+bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, bool integers = false);
 
 // Chunking used by allreduce: chunk c covers [displ(c), displ(c)+cnt(c)); chunk
 // starts are multiples of 16 bytes; tail chunks may be short or empty.

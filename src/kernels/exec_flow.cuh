@@ -3,6 +3,7 @@
 // operation each, as many to an SM as there are registers for, launched while the kernel before it ends.  Blocks of the same slice of all operations are neighbours: what several operations
 // read comes from memory once.  Large messages are bound by memory (each operand read and each result written once), small ones by the launch.  Figures in coll/flow.cc.
 #pragma once
+#include <type_traits>
 #include "exec_impl.cuh"
 
 namespace piccl {
@@ -211,8 +212,9 @@ __global__ void __launch_bounds__(kFlowBlock, 3) exec_flow_kernel(const FlowArgs
   const int scaled = fa.avg ? op.scaled | op.rounded << kRoundedShift : 0;
   const long long len = sl.hi - sl.lo, nfull = len / N;
   const bool dst_done = fa.leave_first & 2;
-  if (OP != OP_COPY && op.nested) {
-    if constexpr (OP != OP_COPY) {
+  constexpr bool NESTED = OP != OP_COPY && !std::is_integral<T>::value;      // (integers are folded flat)
+  if (NESTED && op.nested) {
+    if constexpr (NESTED) {
       if constexpr (SHIFT) flow_tree_shift<T, OP>(op, s_src, s_dst, nfull, scaled, fa.scale);
       else if (op.n_leaf <= 4) flow_tree<T, OP, 4, 2>(op, s_src, s_dst, (int)nfull, scaled, fa.scale, dst_done);
       else flow_tree<T, OP, 8, 1>(op, s_src, s_dst, (int)nfull, scaled, fa.scale, dst_done);

@@ -541,7 +541,8 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
   CollArgs a; a.coll = d0.coll; a.algo = d0.algo; a.k = d0.k; a.nranks = n; a.root = d0.root; a.count = count; a.elem_size = esz;
   a.in_place = !reducing && d0.send == d0.recv;              // (an all-gather's rank 0: its block is the buffer's first; may_flow: all ranks or none)
   ProgKey k{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, 0};
-  k.flow = 1;
+  const bool integers = reducing && d0.dtype != DT_F16 && d0.dtype != DT_F32 && d0.dtype != DT_F64 && d0.dtype != DT_BF16;
+  k.flow = integers ? 2 : 1;
   ProgEntry* e = nullptr;
   {
     std::lock_guard<std::mutex> l(c0->mu);
@@ -554,7 +555,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
       for (int r = 0; r < n; r++) progs.push_back(compile(a, r));
       std::vector<FlowOp> ops;
       ProgEntry x;
-      if (data_flow(progs, ops)) {
+      if (data_flow(progs, ops, integers)) {
         for (const FlowOp& o : ops) {
           x.most = std::max<long long>(x.most, o.count);
           for (int i = 0; i < o.n_leaf; i++) x.offsets_aligned &= o.leaf_off[i] * esz % 16 == 0;

@@ -3,7 +3,9 @@
 run, README.md:40-44)."""
 import itertools
 import json
+import subprocess
 import xml.etree.ElementTree as ET
+from pathlib import Path
 
 import pytest
 
@@ -221,3 +223,18 @@ def test_sums_in_place_have_no_data_flow():
     """A rank could overwrite what another is still to read."""
     assert all(not S.validate(c, "RING", 4, 100, in_place=True, flow=True).ok for c in ("allreduce", "reduce", "reduce_scatter"))
     assert not S.validate("allgather", "RING", 9, 100, flow=True).ok
+
+
+@pytest.fixture(scope="module")
+def flow_main(tmp_path_factory):
+    out = tmp_path_factory.mktemp("flow") / "flow_main"
+    root = Path(__file__).resolve().parent.parent
+    cmd = ["g++", "-std=c++17", "-O1", "-g", "-Wall", "-Werror", f"-I{root / 'src' / 'include'}", *map(str, sorted((root / "src" / "coll").glob("*.cc"))), str(root / "tests" / "native" / "flow_main.cc"), "-o", str(out)]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    return lambda what: subprocess.run([str(out), what], capture_output=True, text=True, timeout=120).stdout.strip()
+
+
+def test_data_flow_of_integers_is_one_fold(flow_main):
+    """Nothing is rounded on the way, so the nesting of the programs does not show in the result."""
+    assert flow_main("integers") == "OK"
