@@ -393,24 +393,23 @@ struct LocalPolicy {
   static constexpr int EXTRA_BYTES = 0, NSTAGE = 1;
   static constexpr bool K_RANKS = RS;
   __device__ LocalPolicy(const TpArgs& args)
-      : a(args), mb_per_shard(args.M / args.n / TP_BM), blocks(RS ? mb_per_shard : args.M / TP_BM), rp((blocks + 1) / 2), num_n(args.N / TN), kb_per_rank(args.K / TP_BK) {}
+      : a(args), mb_per_shard(args.M / args.n / TP_BM), blocks(args.M / TP_BM), rp((blocks + 1) / 2), num_n(args.N / TN), kb_per_rank(args.K / TP_BK) {}
   __device__ void begin() const {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
   __device__ void report(int role) const { for (int i = 0; i < a.nv; i++) atomicExch(a.r[i].status, role); }
-  __device__ int num_tiles() const { return a.nv * rp * num_n; }
+  __device__ int num_tiles() const { return (RS ? 1 : a.nv) * rp * num_n; }
   // ag_gemm: one rank after the other; bands of 16 pairs of row blocks, inside a band rows fastest.  gemm_rs: bands of 8 pairs across owners, so that a wave of the grid is about as many
-  // rows as columns: each wave reads all ranks' k of them.
+  // rows as columns: each wave reads all ranks' k of them.  A pair of CTAs may work for two owners: with one row block to each of eight ranks half of the CTAs would multiply for nothing.
   __device__ void tile(int idx, int v, int& m_blk, int& n_blk) {
     if (RS) {
       constexpr int BAND = 8;
-      const int band = idx / (BAND * num_n), in_band = min(BAND, a.nv * rp - band * BAND), w = idx % (BAND * num_n), pair = band * BAND + w % in_band;
+      const int band = idx / (BAND * num_n), in_band = min(BAND, rp - band * BAND), w = idx % (BAND * num_n), i = 2 * (band * BAND + w % in_band) + v;
       n_blk = w / in_band;
-      rank = pair / rp;
+      rank = min(i, blocks - 1) / mb_per_shard;
       R = &a.r[rank];
-      const int i = 2 * (pair % rp) + v;
-      m_blk = i < blocks ? i : -1;
+      m_blk = i < blocks ? i % mb_per_shard : -1;
       return;
     }
     constexpr int BAND = 16;
@@ -504,15 +503,27 @@ static bool tp_local(piccl_comm** cs, int n, const void* const* A, const void* c
   }
   return true;
 }
-// Tile width: waves of the persistent grid times the clocks of a tile, which are those of the plain GEMM (gemm_sm100.cu: choose).
-static int tp_local_width(int n, int M, int N, int K, int which, int pairs) {
-  const long long blocks = which ? M / TP_BM : M / n / TP_BM, kb = (which ? K : (long long)n * K) / TP_BK;
+static long long tp_local_tiles(int n, int M, int N, int which, int tn) { return (long long)(which ? n : 1) * ((M / TP_BM + 1) / 2) * (N / tn); }
+// Tile width (index into kLocal[which]) for operands read where they are: waves of the persistent grid times the clocks of a tile, which are those of the plain GEMM (gemm_sm100.cu: choose).
+// *exchange: the exchanging form is the faster one.  That is so for gemm_rs with a long k and few tiles: summing all ranks' k in one accumulator has 1 / n of the tiles, each n times as long, and leaves the chip idle
+// where the ranks' own products would fill it.  The exchange costs a fifth more than its tiles and 8 us.  Of 89 shapes the rule picks the slower form, by more than 2 %, for none (us, exchanging and
+// reading: 8 ranks 1024 x 256 x 4096 40 / 94, 2048 x 256 x 4096 47 / 95, 2048 x 1280 x 1664 68 / 72, 4 ranks 1024 x 1024 x 4096 39 / 51, 3 ranks 384 x 512 x 4096 33 / 37; on the other side 8 ranks 3072 x 1024 x 4096
+// 174 / 165, 1024 x 512 x 960 28.7 / 25.5, 4 ranks 512 x 2048 x 4096 57 / 50, 2 ranks 512 x 256 x 4096 33 / 26).
+static int tp_local_width(int n, int M, int N, int K, int which, int pairs, bool* exchange) {
+  const long long kb = (which ? K : (long long)n * K) / TP_BK;
   int best = 0; double best_cost = 0;
+  auto waves = [&](long long tiles) { return (double)((tiles + pairs - 1) / pairs); };
   for (int v = 0; v < 3; v++) {
     const int tn = kLocal[which][v].tn;
-    const long long tiles = n * ((blocks + 1) / 2) * (N / tn);
-    const double cost = (double)((tiles + pairs - 1) / pairs) * ((tn == 256 ? 136 : tn == 128 ? 84 : 70) * 4.0 * kb + 10.0 * tn);
+    const double cost = waves(tp_local_tiles(n, M, N, which, tn)) * ((tn == 256 ? 136 : tn == 128 ? 84 : 70) * 4.0 * kb + 10.0 * tn);
     if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
+  }
+  *exchange = false;
+  if (which == 0) {
+    const long long mb = M / n / TP_BM, tiles = n * (((n - 1) * mb + 1) / 2 + (mb + 1) / 2) * (N / TP_BN);      // (pairs of row blocks for others and of own ones)
+    const double other = waves(tiles) * (136 * 4.0 * (K / TP_BK) + 10.0 * TP_BN);
+    // (the narrowest tiles of a long chain take 80 clocks: the ring of stages is shorter than memory is far)
+    *exchange = best_cost * (kLocal[0][best].tn == 64 ? 80.0 / 70.0 : 1.0) > 1.2 * other + 15000;
   }
   return best;
 }
@@ -553,8 +564,14 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
   }
   a.nv = n; a.one_gpu = n == nr;
   bool ok = true;
-  const bool local = tp_local(cs, n, A, B, out, M, N, K, which);
-  const LocalVariant& lv = kLocal[which][local ? tp_local_width(n, M, N, K, which, c0->tp_pairs[which]) : 0];
+  bool local = tp_local(cs, n, A, B, out, M, N, K, which), exchange = false;
+  const LocalVariant& lv = kLocal[which][local ? tp_local_width(n, M, N, K, which, c0->tp_pairs[which], &exchange) : 0];
+  if (local && exchange) {
+    // (not while the stream is being captured: the exchange's epoch is a launch argument, a replay would reuse it)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusNone; }
+    local = cap != cudaStreamCaptureStatusNone;
+  }
   for (int i = 0; i < n && ok; i++) {
     piccl_comm* c = cs[i];
     TpRank& R = a.r[i];
@@ -581,7 +598,7 @@ static int tp_launch(piccl_comm** cs, int n, const void* const* A, const void* c
       if (cudaFuncSetAttribute((const void*)lv.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lv.smem) != cudaSuccess) return fail(PICCL_CUDA_ERROR, "cannot get %d bytes of shared memory", lv.smem);
       c0->tp_local_ready |= bit;
     }
-    const long long tiles = n * ((((which ? M : M / n) / TP_BM) + 1) / 2) * (long long)(N / lv.tn);
+    const long long tiles = tp_local_tiles(n, M, N, which, lv.tn);
     cfg.gridDim = dim3(2 * (unsigned)std::min<long long>(tiles, c0->tp_pairs[which])); cfg.blockDim = dim3(PAIR_THREADS); cfg.dynamicSmemBytes = lv.smem;
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
@@ -615,6 +632,12 @@ int piccl_tp_flag_range(int which, int nranks, int M, int N, int parity, long lo
   if (nranks * per_src * 4 > TP_FLAG_CALL) return fail(PICCL_UNSUPPORTED, "too many tiles for the flag area");
   *begin = base + tp_flag_at(parity, 0, per_src, 0); *end = base + tp_flag_at(parity, nranks - 1, per_src, per_src - 1) + 4;
   return PICCL_OK;
+}
+// Columns of a tile where a launch carries all ranks on one GPU with `pairs` pairs of CTAs; 0: the ranks exchange.
+int piccl_test_tp_width(int which, int nranks, int M, int N, int K, int pairs) {
+  bool exchange = false;
+  const int v = tp_local_width(nranks, M, N, K, which, pairs, &exchange);
+  return exchange ? 0 : kLocal[which][v].tn;
 }
 int piccl_gemm_rs(piccl_comm_t* c, const void* A, const void* B, void* out, int M, int N, int K_local, void* stream) {
   if (!c) return fail(PICCL_INVALID_ARGUMENT, "null communicator");
