@@ -3,7 +3,8 @@
 // A program says which operands are combined where, in which order, and through which slots the values travel.  Between GPUs that way is the point; on one GPU it is
 // several passes over memory for each hop.  `data_flow` follows the entries of all ranks' programs back and keeps what they compute: each element of a
 // receive buffer as an expression over the send buffers, with the operands of each action in its order and each partial result rounded to the element type where it would
-// have been put into a slot, so that the results are bit for bit those of the programs.  A sum that one rank makes and others receive, or that several ranks make alike, is
+// have been put into a slot, so that the results are bit for bit those of the programs.  (But for bf16 averages among 2, 4 or 8 ranks of elements whose share is
+// below 2^-126, its normal range: such shares are not rounded on their way.)  A sum that one rank makes and others receive, or that several ranks make alike, is
 // computed once and stored in all their buffers.  Nothing in such a call waits (kernels/exec_flow.cuh).
 //
 // us through the slots and this, one B200: all-reduce 4 x 25 MiB averaged by recursive doubling 131 / 38, 8 x 64 MiB on the ring 353 / 188, 8 x 280 KB 45 / 4.8, 8 x 4 KB 37 / 4.7; all-gather 4 x 1 MiB at
@@ -24,7 +25,8 @@ struct Flow {
   std::vector<std::vector<std::vector<Ref>>> producer;      // [rank][action][receive operand]
   FlowOp op;                                                // the expression being built
   bool ok = true;
-  explicit Flow(const std::vector<Program>& p) : progs(p), producer(p.size()) {}
+  FlowKind kind;
+  Flow(const std::vector<Program>& p, FlowKind k) : progs(p), producer(p.size()), kind(k) {}
 
   // the k-th entry pushed on a connection is the k-th one popped; false: the programs do not fit together
   bool match() {
@@ -80,8 +82,9 @@ struct Flow {
     op.leaf_rank[i] = (uint8_t)rank; op.leaf_buf[i] = buf; op.leaf_off[i] = off;
     op.place[i] = (uint8_t)(level | (first ? 4 : 0));
     if (scaled) op.scaled |= (uint8_t)(1u << i);
-    // (one half, quarter or eighth of an element is itself an element but where it is too small for one: not rounding it there loses nothing, and all ranks' averages are the same)
-    if (scaled && rounded && (progs.size() & (progs.size() - 1)) != 0) op.rounded |= (uint8_t)(1u << i);
+    // One half, quarter or eighth of an element is itself an element unless it is below the normal range.  Where it is taken for one all ranks' averages are one expression; otherwise each rank's own share is the
+    // one that is not rounded in its own result (fp16, us: 4 x 25 MiB by recursive doubling 37 and 45.6, through the slots 131; 8 x 8 MB in eights 24 and 68, 202).
+    if (scaled && (kind == FLOW_ALL_SHARES || (rounded && (kind == FLOW_SMALL_SHARES || (progs.size() & (progs.size() - 1)) != 0)))) op.rounded |= (uint8_t)(1u << i);
   }
   void event(bool merge) {                                  // after the last leaf
     uint8_t& p = op.place[op.n_leaf - 1];
@@ -144,10 +147,10 @@ static void flatten(FlowOp& op) {
   op.nested = op.scaled = op.rounded = op.before = 0;
 }
 
-bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, bool integers) {
+bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, FlowKind kind) {
   const int n = (int)progs.size();
   ops.clear();
-  Flow f(progs);
+  Flow f(progs, kind);
   if (n < 2 || n > kFlowLeaves || !f.match()) return false;
   std::map<Ref, int> made;                                  // the operation of what an action makes
   auto alike = [](const FlowOp& a, const FlowOp& b) {
@@ -176,7 +179,7 @@ bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, bool
         if (it != made.end()) at = it->second;
         else {
           f.fold(m, 0);
-          if (integers && f.ok) flatten(f.op);
+          if (kind == FLOW_INTEGERS && f.ok) flatten(f.op);
           for (size_t q = 0; q < ops.size() && f.ok && at < 0; q++) if (ops[q].n_leaf > 1 && alike(ops[q], f.op)) at = (int)q;
         }
       }

@@ -75,7 +75,7 @@ ValidateResult run(const CollArgs& a, int op_, bool with_data, int fifo_cap, int
 
   std::vector<FlowOp> ops;
   if (flow) {
-    if (!with_data || (a.in_place && a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) || !data_flow(progs, ops, std::is_integral<T>::value)) { res.error = "no data flow"; return res; }
+    if (!with_data || (a.in_place && a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) || !data_flow(progs, ops, std::is_integral<T>::value ? FLOW_INTEGERS : FLOW_FLOATS)) { res.error = "no data flow"; return res; }
     for (const FlowOp& op : ops) {
       for (int i = 0; i < op.n_leaf; i++) if (op.leaf_off[i] < 0 || op.leaf_off[i] + op.count > (op.leaf_buf[i] == BUF_IN ? sz.in_elems : sz.out_elems)) { res.error = "leaf out of bounds"; return res; }
       for (int i = 0; i < op.n_dst; i++) if (op.dst_off[i] < 0 || op.dst_off[i] + op.count > sz.out_elems) { res.error = "destination range out of bounds"; return res; }

@@ -100,7 +100,9 @@ int piccl_broadcast(piccl_comm_t* c, const void* send, void* recv, size_t count,
  * the same device (virtual ranks) as a single cooperative kernel launch.  Used
  * to exercise the multi-rank protocol on one GPU.  With all ranks in the launch,
  * and buffers that do not overlap, what the ranks' programs compute is computed
- * straight from the send buffers, bit for bit the same. */
+ * straight from the send buffers, bit for bit the same (but for bf16 averages
+ * among 2, 4 or 8 ranks of elements whose share is below 2^-126: such shares are
+ * rounded once less). */
 int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const void* const* send, void* const* recv,
                            size_t count, int dtype, int op, int root, int algo, int k, void* stream);
 

@@ -122,8 +122,14 @@ Resolved resolve(Coll coll, Algo algo, int k, int nranks);
 Program compile(const CollArgs& a, int rank);
 
 // The operations of a call, from the programs of ALL its ranks.  The caller vouches that no rank's receive buffer overlaps another rank's buffers or its own send
-// buffer (in place: all-gather and broadcast only).  integers: elements for which operands give the same result in any order, no partial result being rounded.  false: they have no such form.
-bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, bool integers = false);
+// buffer (in place: all-gather and broadcast only).  false: they have no such form.
+enum FlowKind : int {
+  FLOW_FLOATS = 1,          // among 2, 4 and 8 ranks an average's shares are taken as elements, which they are unless they are below the type's normal range
+  FLOW_INTEGERS = 2,        // operands give the same result in any order, no partial result being rounded
+  FLOW_SMALL_SHARES = 3,    // averages of a type whose normal range ends where data may lie (fp16): shares that cross between ranks are rounded among any number of them
+  FLOW_ALL_SHARES = 4,      // averages of 16-bit types as the low-latency kernels have them: every share is rounded, a rank's own too
+};
+bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, FlowKind kind = FLOW_FLOATS);
 
 // Chunking used by allreduce: chunk c covers [displ(c), displ(c)+cnt(c)); chunk
 // starts are multiples of 16 bytes; tail chunks may be short or empty.

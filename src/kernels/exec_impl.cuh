@@ -124,7 +124,7 @@ template <> __device__ __forceinline__ float scale_val<float>(float v, float s) 
 template <> __device__ __forceinline__ double scale_val<double>(double v, float s) { return v * (double)s; }
 
 // Operands to scale (avg): bit s, operand s is an original contribution; bit 8 + s, of another rank, which would have put it into a slot: it is rounded to the
-// element type as it would be there, so that a call's result does not depend on how its operands came.  FLOW: only a data flow has such operands; in the executor, where the lone operand to scale is the
+// element type as it would be there, so that a call's result does not depend on how its operands came (coll/flow.cc says where it need not be rounded).  FLOW: only a data flow has such operands; in the executor, where the lone operand to scale is the
 // rank's own, the test for them cost the loops of 16-bit types a tenth, also those that scale nothing (reduce of 8 x 16 MiB of bf16 in two rings 120 us, with it 133; reduce-scatter of 8 x 8 MiB averaged on the ring 211 and 218).
 constexpr int kRoundedShift = 8;
 template <typename T, bool FLOW, typename A> __device__ __forceinline__ A scale_operand(A v, int scaled, int s, float scale) {

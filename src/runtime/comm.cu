@@ -526,6 +526,31 @@ static bool ll_plan(piccl_comm** comms, int n, Algo algo, int k, LLArgs* out) {
   return p.usable;
 }
 
+// Is this a small exchange-type all-reduce, which the low-latency kernel takes (flags travel inside the data lines)?  Its call-independent arguments then.
+static bool ll_takes(piccl_comm** comms, int n, const CallDesc& d, int esz, LLArgs* la) {
+  piccl_comm* c0 = comms[0];
+  if (d.coll != COLL_ALLREDUCE || c0->ll_max_bytes <= 0 || (long long)d.count * esz > c0->ll_max_bytes) return false;
+  if (d.algo != ALGO_RD && d.algo != ALGO_RM && d.algo != ALGO_PRD && d.algo != ALGO_PRM) return false;
+  if (!ll_plan(comms, n, d.algo, d.k, la)) return false;
+  const int E = 8 / esz;
+  const long long nlines = ((long long)d.count + E - 1) / E;
+  // (the persistent server is one CTA: what fits one goes to it)
+  la->n_cta = env().launch_persistent && nlines <= ll_lines_per_cta() ? 1 : ll_ctas(nlines, ll_lines_per_cta(), c0->sm_count / n);
+  return n * la->n_cta <= c0->sm_count;
+}
+// A small all-gather / reduce-scatter whose schedule is one exchange with every rank (DIRECT, or RM / PRM with a radix of at least the rank count): the low-latency exchange kernel.
+static bool llx_takes(piccl_comm** comms, int n, const CallDesc& d, int esz, LLXArgs* xa) {
+  piccl_comm* c0 = comms[0];
+  if ((d.coll != COLL_ALLGATHER && d.coll != COLL_REDUCE_SCATTER) || c0->ll_max_bytes <= 0 || c0->nranks < 2 ||
+      (long long)d.count * esz > std::min<long long>(c0->ll_max_bytes, (long long)env().llx_kb * 1024)) return false;
+  if (d.algo != ALGO_DIRECT && !((d.algo == ALGO_RM || d.algo == ALGO_PRM) && d.k >= c0->nranks)) return false;
+  memset(xa, 0, sizeof *xa);
+  xa->count = d.coll == COLL_ALLGATHER ? (long long)d.count * esz : (long long)d.count;
+  const long long nlines = d.coll == COLL_ALLGATHER ? (xa->count + 7) / 8 : ((long long)d.count + (8 / esz) - 1) / (8 / esz);
+  xa->n_cta = ll_ctas(nlines, llx_lines_per_cta(), c0->sm_count / n);
+  return n * xa->n_cta <= c0->sm_count;
+}
+
 // Slices to an operation: blocks of 4 KiB, one 16-byte pack a thread, while there are SMs for more of them, and no larger than 64 KiB, so that the last wave is short (figures in flow.cc).
 static int flow_slices(const piccl_comm* c, long long bytes, long long ops, long long* slice_bytes) {
   const long long even = (ops * bytes / (12LL * c->sm_count) + 4095) / 4096 * 4096;
@@ -533,16 +558,17 @@ static int flow_slices(const piccl_comm* c, long long bytes, long long ops, long
   return (int)std::max<long long>(1, (bytes + *slice_bytes - 1) / *slice_bytes);
 }
 
-// The call's data flow, all ranks in this launch.  PICCL_UNSUPPORTED: nothing was done, the ranks' programs are to run.
-static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long count, int esz, int op, bool avg, bool capturing, cudaStream_t stream) {
+// The call's data flow, all ranks in this launch; ll: of a call that a low-latency kernel would take, whose averages it gives.  PICCL_UNSUPPORTED: nothing was done, the ranks' programs are to run.
+static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long count, int esz, int op, bool avg, bool ll, bool capturing, cudaStream_t stream) {
   piccl_comm* c0 = comms[0];
   const CallDesc& d0 = calls[0];
   const bool reducing = d0.coll == COLL_ALLREDUCE || d0.coll == COLL_REDUCE || d0.coll == COLL_REDUCE_SCATTER;
   CollArgs a; a.coll = d0.coll; a.algo = d0.algo; a.k = d0.k; a.nranks = n; a.root = d0.root; a.count = count; a.elem_size = esz;
   a.in_place = !reducing && d0.send == d0.recv;              // (an all-gather's rank 0: its block is the buffer's first; may_flow: all ranks or none)
   ProgKey k{(int)a.coll, (int)a.algo, a.k, a.root, a.elem_size, a.in_place ? 1 : 0, a.count, 0};
-  const bool integers = reducing && d0.dtype != DT_F16 && d0.dtype != DT_F32 && d0.dtype != DT_F64 && d0.dtype != DT_BF16;
-  k.flow = integers ? 2 : 1;
+  const bool floats = !reducing || d0.dtype == DT_F16 || d0.dtype == DT_F32 || d0.dtype == DT_F64 || d0.dtype == DT_BF16;
+  const FlowKind kind = !floats ? FLOW_INTEGERS : !avg || esz != 2 ? FLOW_FLOATS : ll ? FLOW_ALL_SHARES : d0.dtype == DT_F16 ? FLOW_SMALL_SHARES : FLOW_FLOATS;
+  k.flow = kind;
   ProgEntry* e = nullptr;
   {
     std::lock_guard<std::mutex> l(c0->mu);
@@ -555,7 +581,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
       for (int r = 0; r < n; r++) progs.push_back(compile(a, r));
       std::vector<FlowOp> ops;
       ProgEntry x;
-      if (data_flow(progs, ops, integers)) {
+      if (data_flow(progs, ops, kind)) {
         for (const FlowOp& o : ops) {
           x.most = std::max<long long>(x.most, o.count);
           for (int i = 0; i < o.n_leaf; i++) x.offsets_aligned &= o.leaf_off[i] * esz % 16 == 0;
@@ -640,64 +666,52 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
   // for by its algorithm stays on the kernel that is made for it.
   constexpr long long kOwnKernelBytes = 16384;
   const bool flows = !env().launch_persistent && d0.algo != ALGO_NVLS && env().proto != 3 && may_flow(comms, n, calls, (long long)d0.count * esz_real);
-  // small exchange-type all-reduces take the low-latency kernel (flags travel inside the data lines)
-  // (not while the stream is being captured: the call epoch is a launch argument, a replay would reuse it)
+  // (the low-latency kernels not while the stream is being captured: the call epoch is a launch argument, a replay would reuse it)
   cudaStreamCaptureStatus cap_state = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap_state) != cudaSuccess) { cudaGetLastError(); cap_state = cudaStreamCaptureStatusNone; }
-  if (cap_state == cudaStreamCaptureStatusNone && d0.coll == COLL_ALLREDUCE && c0->ll_max_bytes > 0 && (long long)d0.count * esz_real <= c0->ll_max_bytes &&
-      (d0.algo == ALGO_RD || d0.algo == ALGO_RM || d0.algo == ALGO_PRD || d0.algo == ALGO_PRM)) {
-    if (flows && (long long)d0.count * esz_real > kOwnKernelBytes) { const int rc = run_flow(comms, n, calls, count, esz, op, avg, false, stream); if (rc != PICCL_UNSUPPORTED) return rc; }
-    LLKernelFn lf = ll_kernel_for(d0.dtype, op);
-    LLArgs la;
-    if (lf && ll_plan(comms, n, d0.algo, d0.k, &la)) {
+  const bool capturing = cap_state != cudaStreamCaptureStatusNone;
+  LLArgs la;
+  LLXArgs xa;
+  const bool ll = ll_takes(comms, n, d0, esz_real, &la), llx = llx_takes(comms, n, d0, esz_real, &xa);
+  if (flows && !capturing && (ll ? (long long)d0.count * esz_real > kOwnKernelBytes : llx)) {
+    const int rc = run_flow(comms, n, calls, count, esz, op, avg, true, false, stream);
+    if (rc != PICCL_UNSUPPORTED) return rc;
+  }
+  if (ll && !capturing) {
+    if (LLKernelFn lf = ll_kernel_for(d0.dtype, op)) {
       la.avg = avg ? 1 : 0; la.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
       la.count = (long long)d0.count; la.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
-      const int E = 8 / esz_real;
-      long long nlines = ((long long)d0.count + E - 1) / E;
-      // (the persistent server is one CTA: what fits one goes to it)
-      la.n_cta = env().launch_persistent && nlines <= ll_lines_per_cta() ? 1 : ll_ctas(nlines, ll_lines_per_cta(), c0->sm_count / n);
-      if (n * la.n_cta <= c0->sm_count) {
-        bool skip = false;
-        for (int i = 0; i < n; i++) {
-          piccl_comm* c = comms[i];
-          std::lock_guard<std::mutex> l(c->mu);
-          la.r[i].ctx = c->d_ctx; la.r[i].in = calls[i].send; la.r[i].out = calls[i].recv;
-          la.epoch = ++c->ll_epoch;
-          c->stats.launches++; c->stats.calls[COLL_ALLREDUCE]++; c->stats.bytes[COLL_ALLREDUCE] += (unsigned long long)d0.count * esz_real;
-          skip |= fault_now(c); c->call_index++;
-        }
-        if (skip) return PICCL_OK;
-        if (env().launch_persistent) {
-          const void* ins[kMaxVRanks]; void* outs[kMaxVRanks];
-          for (int i = 0; i < n; i++) { ins[i] = calls[i].send; outs[i] = calls[i].recv; }
-          if (persist_allreduce(comms, n, la, ins, outs, (long long)d0.count, d0.dtype, op, avg ? 1 : 0, (int)d0.algo, d0.k, stream) == PICCL_OK) { c0->stats.persistent_calls++; return PICCL_OK; }
-        }
-        nvtxRangePushA("allreduce_ll");
-        void* args[] = {&la};
-        cudaError_t e;
-        if (n > 1) e = cudaLaunchCooperativeKernel((const void*)lf, dim3(n * la.n_cta), dim3(kLLBlock), args, 0, stream);
-        else e = cudaLaunchKernel((const void*)lf, dim3(la.n_cta), dim3(kLLBlock), args, 0, stream);
-        nvtxRangePop();
-        if (e != cudaSuccess) return fail(PICCL_CUDA_ERROR, "low-latency launch failed: %s", cudaGetErrorString(e));
-        return PICCL_OK;
+      bool skip = false;
+      for (int i = 0; i < n; i++) {
+        piccl_comm* c = comms[i];
+        std::lock_guard<std::mutex> l(c->mu);
+        la.r[i].ctx = c->d_ctx; la.r[i].in = calls[i].send; la.r[i].out = calls[i].recv;
+        la.epoch = ++c->ll_epoch;
+        c->stats.launches++; c->stats.calls[COLL_ALLREDUCE]++; c->stats.bytes[COLL_ALLREDUCE] += (unsigned long long)d0.count * esz_real;
+        skip |= fault_now(c); c->call_index++;
       }
+      if (skip) return PICCL_OK;
+      if (env().launch_persistent) {
+        const void* ins[kMaxVRanks]; void* outs[kMaxVRanks];
+        for (int i = 0; i < n; i++) { ins[i] = calls[i].send; outs[i] = calls[i].recv; }
+        if (persist_allreduce(comms, n, la, ins, outs, (long long)d0.count, d0.dtype, op, avg ? 1 : 0, (int)d0.algo, d0.k, stream) == PICCL_OK) { c0->stats.persistent_calls++; return PICCL_OK; }
+      }
+      nvtxRangePushA("allreduce_ll");
+      void* args[] = {&la};
+      cudaError_t e;
+      if (n > 1) e = cudaLaunchCooperativeKernel((const void*)lf, dim3(n * la.n_cta), dim3(kLLBlock), args, 0, stream);
+      else e = cudaLaunchKernel((const void*)lf, dim3(la.n_cta), dim3(kLLBlock), args, 0, stream);
+      nvtxRangePop();
+      if (e != cudaSuccess) return fail(PICCL_CUDA_ERROR, "low-latency launch failed: %s", cudaGetErrorString(e));
+      return PICCL_OK;
     }
   }
 
-  // small all-gather / reduce-scatter whose schedule is one exchange with every rank (DIRECT, or RM / PRM with a radix of at least
-  // the rank count): the low-latency exchange kernel.  (Not while capturing: the epoch is a launch argument.)
-  if (cap_state == cudaStreamCaptureStatusNone && (d0.coll == COLL_ALLGATHER || d0.coll == COLL_REDUCE_SCATTER) && c0->ll_max_bytes > 0 && c0->nranks >= 2 &&
-      (long long)d0.count * esz_real <= std::min<long long>(c0->ll_max_bytes, (long long)env().llx_kb * 1024) &&
-      (d0.algo == ALGO_DIRECT || ((d0.algo == ALGO_RM || d0.algo == ALGO_PRM) && d0.k >= c0->nranks))) {
-    if (flows) { const int rc = run_flow(comms, n, calls, count, esz, op, avg, false, stream); if (rc != PICCL_UNSUPPORTED) return rc; }
+  if (llx && !capturing) {
     LLXKernelFn xf = d0.coll == COLL_ALLGATHER ? llx_allgather_kernel() : llx_reduce_scatter_kernel_for(d0.dtype, op);
-    LLXArgs xa; memset(&xa, 0, sizeof xa);
     xa.n_vrank = n; xa.avg = avg ? 1 : 0; xa.scale = avg ? 1.0f / (float)c0->nranks : 1.0f;
-    xa.count = d0.coll == COLL_ALLGATHER ? (long long)d0.count * esz_real : (long long)d0.count;
     xa.timeout_ns = (unsigned long long)c0->cfg.timeout_ms * 1000000ull;
-    const long long nlines = d0.coll == COLL_ALLGATHER ? (xa.count + 7) / 8 : ((long long)d0.count + (8 / esz_real) - 1) / (8 / esz_real);
-    xa.n_cta = ll_ctas(nlines, llx_lines_per_cta(), c0->sm_count / n);
-    if (xf && esz_real <= 8 && n * xa.n_cta <= c0->sm_count) {
+    if (xf) {
       bool skip = false;
       for (int i = 0; i < n; i++) {
         piccl_comm* c = comms[i];
@@ -772,7 +786,7 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
   }
 
   if (flows) {
-    const int flow = run_flow(comms, n, calls, count, esz, op, avg, cap_state != cudaStreamCaptureStatusNone, stream);
+    const int flow = run_flow(comms, n, calls, count, esz, op, avg, ll || llx, capturing, stream);
     if (flow != PICCL_UNSUPPORTED) return flow;
   }
 

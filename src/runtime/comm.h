@@ -21,7 +21,7 @@ struct HandleBlob {
 };
 
 struct ProgKey {
-  int coll, algo, k, root, elem_size, in_place; long long count, stride; int flow = 0 /* the call's data flow, kept by rank 0: 1, of integers 2 */;
+  int coll, algo, k, root, elem_size, in_place; long long count, stride; int flow = 0 /* the call's data flow, kept by rank 0: its kind */;
   bool operator==(const ProgKey& o) const {
     return coll == o.coll && algo == o.algo && k == o.k && root == o.root && elem_size == o.elem_size && in_place == o.in_place && count == o.count && stride == o.stride && flow == o.flow;
   }

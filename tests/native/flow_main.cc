@@ -27,7 +27,7 @@ template <class F> static int each_call(F f) {
 static int integers() {
   return each_call([](const CollArgs& a, const std::vector<Program>& progs) {
     std::vector<FlowOp> ops;
-    if (!data_flow(progs, ops, true)) return bad("no data flow", a);
+    if (!data_flow(progs, ops, FLOW_INTEGERS)) return bad("no data flow", a);
     const bool sums = a.coll == COLL_ALLREDUCE || a.coll == COLL_REDUCE || a.coll == COLL_REDUCE_SCATTER;
     for (size_t q = 0; q < ops.size(); q++) {
       const FlowOp& op = ops[q];

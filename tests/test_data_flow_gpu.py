@@ -40,3 +40,31 @@ def test_integers(n, k, dtype):
             a, b = _both(g, coll, xs, count, count, op=op, root=1, algo=algo, k=k)
             assert all(torch.equal(x, y) for x, y in zip(a, b)), (coll, count, algo, op)
     g.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n", [2, 3, 4, 8])
+def test_averages_of_small_values(n, dtype):
+    """Shares below 2^-14, fp16's normal range, lose bits where they cross between ranks: which do is the same in the data flow, and so it is for thirds, which are rounded in either type.
+    Values of 1e-7 to 1, zeros of both signs, the least elements of fp16; lengths that low-latency kernels would take, which round all shares, and longer ones.  The same bits as through the slots."""
+    g = _group(n)
+    for coll, count in itertools.product(["allreduce", "reduce_scatter", "reduce"], [7, 20011, 600013]):
+        n_in = count * (n if coll == "reduce_scatter" else 1)
+        xs = []
+        for r in range(n):
+            gen = torch.Generator(device="cuda").manual_seed(r)
+            x = (torch.rand(n_in, generator=gen, device="cuda") * 2 - 1) * 10.0 ** torch.randint(-7, 1, (n_in,), generator=gen, device="cuda")
+            xs.append(x.to(dtype))
+            xs[-1][::5] = torch.tensor([0.0, -0.0, 2.0 ** -24, -(2.0 ** -24), 3 * 2.0 ** -24], device="cuda", dtype=dtype)[r % 5]
+        for algo, k in itertools.product(ALGOS, [2, 8]):
+            a, b = _both(g, coll, xs, count, count, op="avg", root=1, algo=algo, k=k)
+            assert all(torch.equal(x.view(torch.int16), y.view(torch.int16)) for x, y in zip(a, b)), (coll, count, algo, k)
+            if algo in ("RD", "RM", "PRD", "PRM") and coll == "allreduce" and count > 7:       # captured, it is the same call (what the low-latency kernel runs cannot be captured)
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    g.run(coll, xs, b, count, op="avg", root=1, algo=algo, k=k)
+                for y in b:
+                    y.zero_()
+                graph.replay()
+                assert all(torch.equal(x.view(torch.int16), y.view(torch.int16)) for x, y in zip(a, b)), (coll, count, algo, k)
+    g.close()
