@@ -67,6 +67,7 @@ def _declare(lib: C.CDLL) -> None:
     lib.piccl_group_collective.argtypes = [vp, i, i, vp, vp, sz, i, i, i, i, i, vp]       # the tables: arrays or packed bytes
     lib.piccl_test_leave_first.argtypes = [i, i, i, i, ll]
     lib.piccl_test_slots_only.argtypes = [vp, i]
+    lib.piccl_test_flow_calls.argtypes, lib.piccl_test_flow_calls.restype = [vp], ll
     lib.piccl_test_unmatched_wait.argtypes = [vp, i, vp]
     lib.piccl_algo_from_string.argtypes = [C.c_char_p]
     lib.piccl_sched_xml.argtypes = [i, i, i, i, i, ll, i, C.c_char_p, ll]

@@ -132,6 +132,10 @@ int piccl_test_leave_first(int coll, int nranks, int in_launch, int one_device, 
  * slots, as ranks on several GPUs do, and not the call's data flow. */
 int piccl_test_slots_only(piccl_comm_t* c, int on);
 
+/* Test hook: how many calls of this communicator ran as data flow (statistics and
+ * traces name the algorithm that was asked for). */
+long long piccl_test_flow_calls(const piccl_comm_t* c);
+
 /* Test hook: tile width of a tensor-parallel product all of whose ranks are in one
  * launch (which: 0 gemm_rs, 1 ag_gemm); 0: the ranks exchange all the same. */
 int piccl_test_tp_width(int which, int nranks, int M, int N, int K, int pairs);

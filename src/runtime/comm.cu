@@ -626,7 +626,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
   nvtxRangePop();
   trace_end(c0, tr, stream);
   if (err != cudaSuccess) return fail(PICCL_CUDA_ERROR, "launch of a data flow failed: %s", cudaGetErrorString(err));
-  for (int i = 0; i < n; i++) { comms[i]->stats.calls[d0.coll]++; comms[i]->stats.bytes[d0.coll] += (unsigned long long)count * esz; }
+  for (int i = 0; i < n; i++) { comms[i]->flow_calls++; comms[i]->stats.calls[d0.coll]++; comms[i]->stats.bytes[d0.coll] += (unsigned long long)count * esz; }
   return PICCL_OK;
 }
 
@@ -661,11 +661,12 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
                    : (reducing ? exec_kernel_for(d0.dtype, op) : exec_copy_kernel());
   if (!fn) return fail(PICCL_INTERNAL_ERROR, "no kernel for dtype %d op %d", d0.dtype, op);
 
-  // All ranks in this launch: the call's data flow, where no way between the ranks is asked for by name.  Among eight ranks the low-latency kernels, which are cooperative launches, take 8.2 us for an
+  // All ranks in this launch: the call's data flow, where neither a way between the ranks (PICCL_PROTO, the persistent server, the switch) nor a size of the grid (PICCL_MIN_GRID_SIZE, PICCL_MAX_GRID_SIZE) is asked for by name.  Among eight ranks the low-latency kernels, which are cooperative launches, take 8.2 us for an
   // all-reduce of 64 KiB and for an all-gather of 4 KiB blocks, the data flow 4.9.  At 1 KiB the all-reduce takes 5.9 and 5.1: up to 16 KiB (both ends of a launch, little more) an exchange asked
   // for by its algorithm stays on the kernel that is made for it.
   constexpr long long kOwnKernelBytes = 16384;
-  const bool flows = !env().launch_persistent && d0.algo != ALGO_NVLS && env().proto != 3 && may_flow(comms, n, calls, (long long)d0.count * esz_real);
+  const Env& ev = env();
+  const bool flows = ev.proto == 0 && !ev.launch_persistent && !ev.min_grid_set && !ev.max_grid_set && d0.algo != ALGO_NVLS && may_flow(comms, n, calls, (long long)d0.count * esz_real);
   // (the low-latency kernels not while the stream is being captured: the call epoch is a launch argument, a replay would reuse it)
   cudaStreamCaptureStatus cap_state = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap_state) != cudaSuccess) { cudaGetLastError(); cap_state = cudaStreamCaptureStatusNone; }
@@ -901,6 +902,7 @@ int piccl_test_slots_only(piccl_comm_t* c, int on) {
   c->slots_only = on != 0;
   return PICCL_OK;
 }
+long long piccl_test_flow_calls(const piccl_comm_t* c) { return c ? (long long)c->flow_calls : -1; }
 int piccl_test_unmatched_wait(piccl_comm_t* c, int timeout_ms, void* stream) {
   if (!c || !c->connected) return fail(PICCL_INVALID_USAGE, "communicator is not connected");
   DevGuard g(c->device);

@@ -58,7 +58,7 @@ struct piccl_comm {
   piccl_status_t* h_status = nullptr; piccl_status_t* d_status = nullptr;
   bool ipc_opened[piccl::kMaxRanks] = {false};
   bool connected = false, broken = false, slots_only = false /* everything goes through the ranks' slots, also where one launch carries all ranks (tests) */;
-  unsigned long long call_index = 0;
+  unsigned long long call_index = 0, flow_calls = 0 /* calls whose data flow ran */;
   unsigned tp_epoch_rs = 0, tp_epoch_ag = 0;   // epochs of the fused tensor-parallel kernels
   int* d_tp_status = nullptr;
   int tp_local_ready = 0;              // bit 3 * kernel + width: the kernel has its shared memory

@@ -68,3 +68,30 @@ def test_averages_of_small_values(n, dtype):
                 graph.replay()
                 assert all(torch.equal(x.view(torch.int16), y.view(torch.int16)) for x, y in zip(a, b)), (coll, count, algo, k)
     g.close()
+
+
+@pytest.mark.parametrize("variable,value", [("PICCL_PROTO", "ll"), ("PICCL_PROTO", "simple"), ("PICCL_MAX_GRID_SIZE", "2"), ("PICCL_MIN_GRID_SIZE", "3")])
+def test_a_way_that_is_asked_for_by_name_is_taken(monkeypatch, variable, value):
+    """The data path that PICCL_PROTO narrows, and the grid that the reference's variables size, are the executor's."""
+    g = _group(4)
+    flows = lambda: g._lib.piccl_test_flow_calls(g._hs[0])
+    xs = [torch.full((20000,), float(r + 1), device="cuda") for r in range(4)]
+
+    def run():
+        outs = [torch.zeros_like(x) for x in xs]
+        for algo in ("RING", "PRD"):
+            g.run("allreduce", xs, outs, 20000, algo=algo)
+        torch.cuda.synchronize()
+        assert g.status().aborted == 0 and all(torch.all(o == 10.0) for o in outs)
+    try:
+        before = flows()
+        run()
+        assert flows() == before + 2
+        monkeypatch.setenv(variable, value)
+        g._lib.piccl_env_reload()
+        run()
+        assert flows() == before + 2
+    finally:
+        monkeypatch.undo()
+        g._lib.piccl_env_reload()
+        g.close()
