@@ -184,7 +184,12 @@ bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, Flow
         }
       }
       if (!f.ok) return false;
-      if (at < 0 || ops[at].n_dst == kFlowLeaves) { at = (int)ops.size(); ops.push_back(f.op); }
+      if (at < 0) { at = (int)ops.size(); ops.push_back(f.op); }
+      else if (ops[at].n_dst == kFlowLeaves) {               // the same once more, for further destinations
+        FlowOp again = ops[at];
+        again.n_dst = 0;
+        at = (int)ops.size(); ops.push_back(again);
+      }
       if (b.n_recv != 0) made[m] = at;
       FlowOp& op = ops[at];
       op.dst_rank[op.n_dst] = (uint8_t)r; op.dst_off[op.n_dst++] = a.dst_off;

@@ -41,9 +41,42 @@ static int integers() {
   });
 }
 
+// A sum that eight ranks store at two places each has more destinations than one operation holds: a second one with the same expression.
+static int destinations() {
+  const int n = 8, count = 16;
+  std::vector<Program> progs(n);
+  for (int r = 0; r < n; r++) {
+    progs[r].rank = r; progs[r].nranks = n;
+    Action get, twice;
+    get.count = twice.count = count; get.dst_buf = BUF_OUT;
+    if (r == 0) {
+      get.src_buf = BUF_IN; get.n_recv = get.n_send = n - 1;
+      for (int p = 1; p < n; p++) get.recv_peer[p - 1] = get.send_peer[p - 1] = (uint8_t)p;
+    } else {
+      Action put;
+      put.count = count; put.src_buf = BUF_IN; put.n_send = 1; put.send_peer[0] = 0;
+      progs[r].actions.push_back(put);
+      get.n_recv = 1; get.recv_peer[0] = 0;
+    }
+    twice.src_buf = twice.dst_buf = BUF_OUT; twice.dst_off = count;
+    progs[r].actions.push_back(get);
+    progs[r].actions.push_back(twice);
+  }
+  std::vector<FlowOp> ops;
+  if (!data_flow(progs, ops)) { printf("no data flow\n"); return 1; }
+  int stored[8][2] = {{0}};
+  for (const FlowOp& op : ops) {
+    if (op.n_leaf != n || op.count != count || op.n_dst < 1 || op.n_dst > kFlowLeaves) { printf("an operation of %d operands and %d destinations\n", op.n_leaf, op.n_dst); return 1; }
+    for (int i = 0; i < n; i++) if (op.leaf_rank[i] != i || op.leaf_buf[i] != BUF_IN || op.leaf_off[i] != 0) { printf("wrong operands\n"); return 1; }
+    for (int i = 0; i < op.n_dst; i++) stored[op.dst_rank[i]][op.dst_off[i] / count]++;
+  }
+  for (auto& r : stored) for (int s : r) if (s != 1) { printf("stored %d times\n", s); return 1; }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
-  const int rc = !strcmp(what, "integers") ? integers() : 2;
+  const int rc = !strcmp(what, "integers") ? integers() : !strcmp(what, "destinations") ? destinations() : 2;
   if (rc == 0) printf("OK\n");
   return rc;
 }

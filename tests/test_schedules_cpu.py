@@ -238,3 +238,7 @@ def flow_main(tmp_path_factory):
 def test_data_flow_of_integers_is_one_fold(flow_main):
     """Nothing is rounded on the way, so the nesting of the programs does not show in the result."""
     assert flow_main("integers") == "OK"
+
+
+def test_data_flow_of_a_result_with_many_destinations(flow_main):
+    assert flow_main("destinations") == "OK"
