@@ -229,4 +229,35 @@ bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, Flow
   return !ops.empty();
 }
 
+const char* check_flow(const std::vector<FlowOp>& ops, const CollArgs& a) {
+  const int64_t st = a.block_stride ? a.block_stride : a.count;
+  const int64_t in_elems = a.coll == COLL_REDUCE_SCATTER ? (a.nranks - 1) * st + a.count : a.count, out_elems = a.coll == COLL_ALLGATHER ? (a.nranks - 1) * st + a.count : a.count;
+  for (const FlowOp& op : ops) {
+    if (op.count <= 0 || op.n_leaf < 1 || op.n_leaf > kFlowLeaves || op.n_dst < 1 || op.n_dst > kFlowLeaves) return "bad number of operands, destinations or elements";
+    int level = 0;
+    bool begun[kFlowLevels] = {false};
+    for (int i = 0; i < op.n_leaf; i++) {
+      if (op.leaf_rank[i] >= a.nranks || (a.coll == COLL_BROADCAST && op.leaf_rank[i] != a.root)) return "operand of a rank that has none";
+      if (op.leaf_buf[i] != BUF_IN && !(op.leaf_buf[i] == BUF_OUT && a.in_place)) return "operand that is not in a send buffer";
+      if (op.leaf_off[i] < 0 || op.leaf_off[i] + op.count > (op.leaf_buf[i] == BUF_IN ? in_elems : out_elems)) return "operand outside its buffer";
+      level = op.place[i] & 3;
+      if (((op.place[i] & 4) != 0) == begun[level]) return "an accumulator that is begun twice, or not at all";
+      begun[level] = true;
+      if (!op.nested && (level || (op.place[i] >> 3) || ((op.place[i] & 4) != 0) != (i == 0))) return "a nested expression that says it is flat";
+      for (int k = 0; k < (op.place[i] >> 3 & 3); k++)
+        if (op.place[i] >> (5 + k) & 1) {
+          if (level == 0 || !begun[level - 1]) return "fold into an accumulator that holds nothing";
+          begun[level--] = false;
+        }
+    }
+    if (level != 0) return "accumulators left";
+    for (int i = 1; i < kFlowLevels; i++) if (begun[i]) return "accumulators left";
+    for (int i = 0; i < op.n_dst; i++) {
+      if (op.dst_rank[i] >= a.nranks || (a.coll == COLL_REDUCE && op.dst_rank[i] != a.root)) return "destination of a rank that has none";
+      if (op.dst_off[i] < 0 || op.dst_off[i] + op.count > out_elems) return "destination outside its buffer";
+    }
+  }
+  return nullptr;
+}
+
 }  // namespace piccl

@@ -130,6 +130,8 @@ enum FlowKind : int {
   FLOW_ALL_SHARES = 4,      // averages of 16-bit types as the low-latency kernels have them: every share is rounded, a rank's own too
 };
 bool data_flow(const std::vector<Program>& progs, std::vector<FlowOp>& ops, FlowKind kind = FLOW_FLOATS);
+// What is wrong with the operations of a call: elements outside its buffers, ranks that are not its own, expressions that no kernel could follow.  null: nothing.
+const char* check_flow(const std::vector<FlowOp>& ops, const CollArgs& a);
 
 // Chunking used by allreduce: chunk c covers [displ(c), displ(c)+cnt(c)); chunk
 // starts are multiples of 16 bytes; tail chunks may be short or empty.

@@ -324,7 +324,7 @@ static int after_upload(ProgEntry& e, cudaStream_t stream) {
 }
 
 // PICCL_DEBUG=1: every action of a freshly compiled program is checked against the extents of the
-// buffers of the call before it is ever given to the device (ranges, peers, scratch capacity).
+// buffers of the call before it is ever given to the device (ranges, peers, scratch capacity); a data flow's operations likewise (flow.cc: check_flow).
 static const char* check_program(const Program& p, const CollArgs& a, long long scratch_cap_elems) {
   const long long st = a.block_stride ? a.block_stride : a.count;
   long long in_elems = a.count, out_elems = a.count;
@@ -582,6 +582,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
       std::vector<FlowOp> ops;
       ProgEntry x;
       if (data_flow(progs, ops, kind)) {
+        if (env().debug) if (const char* why = check_flow(ops, a)) return fail(PICCL_INTERNAL_ERROR, "data flow check failed (%s %s): %s", coll_name(a.coll), algo_name(a.algo), why);
         for (const FlowOp& o : ops) {
           x.most = std::max<long long>(x.most, o.count);
           for (int i = 0; i < o.n_leaf; i++) x.offsets_aligned &= o.leaf_off[i] * esz % 16 == 0;

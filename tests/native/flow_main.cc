@@ -74,9 +74,55 @@ static int destinations() {
   return 0;
 }
 
+// Every call's operations pass the check, whole and of every kind; with one of their fields set wrong they do not.
+static int checked() {
+  return each_call([](const CollArgs& given, const std::vector<Program>& given_progs) {
+    CollArgs a = given;
+    std::vector<Program> progs = given_progs;
+    for (bool in_place : {false, true}) {
+      if (in_place) {
+        if (a.coll != COLL_ALLGATHER && a.coll != COLL_BROADCAST) break;
+        a.in_place = true;
+        for (int r = 0; r < a.nranks; r++) progs[r] = compile(a, r);
+      }
+      for (FlowKind kind : {FLOW_FLOATS, FLOW_INTEGERS, FLOW_SMALL_SHARES, FLOW_ALL_SHARES}) {
+        std::vector<FlowOp> ops;
+        if (!data_flow(progs, ops, kind)) return bad("no data flow", a);
+        if (const char* why = check_flow(ops, a)) { printf("%s\n", why); return bad("refused", a); }
+        const int64_t in = a.coll == COLL_REDUCE_SCATTER ? a.nranks * a.count : a.count, out = a.coll == COLL_ALLGATHER ? a.nranks * a.count : a.count;
+        int missed = 0;
+        auto wrong = [&](auto set) {
+          for (size_t q = 0; q < ops.size(); q += 7) {
+            const FlowOp was = ops[q];
+            set(ops[q]);
+            missed += check_flow(ops, a) == nullptr;
+            ops[q] = was;
+          }
+        };
+        wrong([&](FlowOp& op) { op.count = 0; });
+        wrong([&](FlowOp& op) { op.n_leaf = 0; });
+        wrong([&](FlowOp& op) { op.n_leaf = kFlowLeaves + 1; });
+        wrong([&](FlowOp& op) { op.n_dst = 0; });
+        wrong([&](FlowOp& op) { op.n_dst = kFlowLeaves + 1; });
+        wrong([&](FlowOp& op) { op.leaf_rank[0] = (uint8_t)a.nranks; });
+        wrong([&](FlowOp& op) { op.leaf_buf[op.n_leaf - 1] = BUF_SCRATCH; });
+        wrong([&](FlowOp& op) { op.leaf_off[op.n_leaf - 1] = (op.leaf_buf[op.n_leaf - 1] == BUF_IN ? in : out) - op.count + 1; });
+        wrong([&](FlowOp& op) { op.leaf_off[0] = -1; });
+        wrong([&](FlowOp& op) { op.place[0] &= (uint8_t)~4; });
+        wrong([&](FlowOp& op) { op.place[op.n_leaf - 1] = (uint8_t)((op.place[op.n_leaf - 1] & ~3) | 4 | 1); });
+        wrong([&](FlowOp& op) { op.dst_rank[op.n_dst - 1] = (uint8_t)a.nranks; });
+        wrong([&](FlowOp& op) { op.dst_off[op.n_dst - 1] = out - op.count + 1; });
+        wrong([&](FlowOp& op) { op.dst_off[0] = -1; });
+        if (missed) return bad("a wrong operation passed", a);
+      }
+    }
+    return 0;
+  });
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
-  const int rc = !strcmp(what, "integers") ? integers() : !strcmp(what, "destinations") ? destinations() : 2;
+  const int rc = !strcmp(what, "integers") ? integers() : !strcmp(what, "destinations") ? destinations() : !strcmp(what, "checked") ? checked() : 2;
   if (rc == 0) printf("OK\n");
   return rc;
 }

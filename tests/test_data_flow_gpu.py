@@ -95,3 +95,26 @@ def test_a_way_that_is_asked_for_by_name_is_taken(monkeypatch, variable, value):
         monkeypatch.undo()
         g._lib.piccl_env_reload()
         g.close()
+
+
+def test_checks_of_the_debug_mode_pass(monkeypatch):
+    """PICCL_DEBUG=1 checks fresh programs and data flows against the call's buffers; in place too."""
+    monkeypatch.setenv("PICCL_DEBUG", "1")
+    g = _group(8)
+    g._lib.piccl_env_reload()
+    try:
+        xs = [torch.full((8 * 30011,), float(r + 1), device="cuda") for r in range(8)]
+        for coll, algo in itertools.product(["allreduce", "reduce_scatter", "reduce", "allgather", "broadcast"], ALGOS):
+            outs = [torch.zeros(8 * 30011, device="cuda") for _ in xs]
+            before = g._lib.piccl_test_flow_calls(g._hs[0])
+            g.run(coll, xs, outs, 30011, algo=algo, root=3)
+            if coll in ("allgather", "broadcast"):
+                g.run(coll, [o[r * 30011:] if coll == "allgather" else o for r, o in enumerate(outs)], outs, 30011, algo=algo, root=3)
+            torch.cuda.synchronize()
+            assert g.status().aborted == 0 and g._lib.piccl_test_flow_calls(g._hs[0]) > before
+            want = {"allgather": 4.0, "broadcast": 4.0}.get(coll, 36.0)
+            assert torch.all(outs[3][30011 * 3:30011 * 4] == want) if coll == "allgather" else torch.all(outs[3][:30011] == want)
+    finally:
+        monkeypatch.undo()
+        g._lib.piccl_env_reload()
+        g.close()

@@ -242,3 +242,8 @@ def test_data_flow_of_integers_is_one_fold(flow_main):
 
 def test_data_flow_of_a_result_with_many_destinations(flow_main):
     assert flow_main("destinations") == "OK"
+
+
+def test_operations_of_a_data_flow_are_checked(flow_main):
+    """What PICCL_DEBUG=1 runs on a fresh data flow, as it checks fresh programs."""
+    assert flow_main("checked") == "OK"
