@@ -558,10 +558,11 @@ static int flow_slices(const piccl_comm* c, long long bytes, long long ops, long
   return (int)std::max<long long>(1, (bytes + *slice_bytes - 1) / *slice_bytes);
 }
 
-// The call's data flow, all ranks in this launch; ll: of a call that a low-latency kernel would take, whose averages it gives.  PICCL_UNSUPPORTED: nothing was done, the ranks' programs are to run.
-static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long count, int esz, int op, bool avg, bool ll, bool capturing, cudaStream_t stream) {
+// The call's data flow, all ranks in this launch; ll: of a call that a low-latency kernel would take, whose averages it gives; *fresh: it was not known before.  PICCL_UNSUPPORTED: nothing was done, the ranks' programs are to run.
+static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long count, int esz, int op, bool avg, bool ll, bool capturing, bool* fresh, cudaStream_t stream) {
   piccl_comm* c0 = comms[0];
   const CallDesc& d0 = calls[0];
+  *fresh = false;
   const bool reducing = d0.coll == COLL_ALLREDUCE || d0.coll == COLL_REDUCE || d0.coll == COLL_REDUCE_SCATTER;
   CollArgs a; a.coll = d0.coll; a.algo = d0.algo; a.k = d0.k; a.nranks = n; a.root = d0.root; a.count = count; a.elem_size = esz;
   a.in_place = !reducing && d0.send == d0.recv;              // (an all-gather's rank 0: its block is the buffer's first; may_flow: all ranks or none)
@@ -594,6 +595,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
       if (int rc = upload(c0, ops.data(), ops.size() * sizeof(FlowOp), std::max<size_t>(1, ops.size()) * sizeof(FlowOp), stream, x, &dev)) return rc;
       x.ops = static_cast<const FlowOp*>(dev);
       it = c0->cache.emplace(k, x).first;
+      *fresh = true;
       for (int i = 0; i < n; i++) comms[i]->stats.program_cache_misses++;
     } else {
       if (int rc = after_upload(it->second, stream)) return rc;
@@ -676,7 +678,8 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
   LLXArgs xa;
   const bool ll = ll_takes(comms, n, d0, esz_real, &la), llx = llx_takes(comms, n, d0, esz_real, &xa);
   if (flows && !capturing && (ll ? (long long)d0.count * esz_real > kOwnKernelBytes : llx)) {
-    const int rc = run_flow(comms, n, calls, count, esz, op, avg, true, false, stream);
+    bool fresh;
+    const int rc = run_flow(comms, n, calls, count, esz, op, avg, true, false, &fresh, stream);
     if (rc != PICCL_UNSUPPORTED) return rc;
   }
   if (ll && !capturing) {
@@ -787,8 +790,34 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     }
   }
 
+  // the call of rank i on `cur` elements from `done` on
+  auto part_of = [&](int i, long long done, long long cur, const char** s, char** r) {
+    const piccl_comm* c = comms[i]; const CallDesc& d = calls[i];
+    CollArgs a; a.coll = d.coll; a.algo = d.algo; a.k = d.k; a.nranks = c->nranks; a.root = d.root; a.count = cur; a.block_stride = stride; a.elem_size = esz;
+    *s = (const char*)d.send; *r = (char*)d.recv;
+    switch (d.coll) {
+      case COLL_ALLGATHER: a.in_place = (*s == *r + (long long)c->rank * count); *s += done; *r += done; if (stride == 0 && slab != count) a.block_stride = count; break;
+      case COLL_REDUCE_SCATTER: a.in_place = (*r == *s + (long long)c->rank * count * esz); *s += done * esz; *r += done * esz; break;
+      default: a.in_place = (*s == *r); break;
+    }
+    if (d.coll == COLL_REDUCE && c->rank != d.root) a.in_place = false;
+    return a;
+  };
+
   if (flows) {
-    const int flow = run_flow(comms, n, calls, count, esz, op, avg, ll || llx, capturing, stream);
+    bool fresh;
+    const int flow = run_flow(comms, n, calls, count, esz, op, avg, ll || llx, capturing, &fresh, stream);
+    if (flow == PICCL_OK && fresh && !capturing) {
+      // The ranks' programs too: the same call may come again inside a stream capture with buffers that overlap, when nothing can be built any more.  (What cannot be kept is refused there.)
+      int rc = PICCL_OK;
+      for (long long done = 0; done < count && rc == PICCL_OK; done += slab)
+        for (int i = 0; i < n && rc == PICCL_OK; i++) {
+          std::lock_guard<std::mutex> l(comms[i]->mu);
+          const char* s; char* r;
+          const ProgEntry* pe = nullptr;
+          rc = get_program(comms[i], part_of(i, done, std::min(slab, count - done), &s, &r), stream, &pe);
+        }
+    }
     if (flow != PICCL_UNSUPPORTED) return flow;
   }
 
@@ -802,16 +831,10 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
     bool aligned = true;
     CollArgs priorities_of;
     for (int i = 0; i < n && rc == PICCL_OK; i++) {
-      piccl_comm* c = comms[i]; const CallDesc& d = calls[i];
+      piccl_comm* c = comms[i];
       std::lock_guard<std::mutex> l(c->mu);
-      CollArgs a; a.coll = d.coll; a.algo = d.algo; a.k = d.k; a.nranks = c->nranks; a.root = d.root; a.count = cur; a.block_stride = stride; a.elem_size = esz;
-      const char* s = (const char*)d.send; char* r = (char*)d.recv;
-      switch (d.coll) {
-        case COLL_ALLGATHER: a.in_place = (s == r + (long long)c->rank * count); s += done; r += done; if (stride == 0 && slab != count) a.block_stride = count; break;
-        case COLL_REDUCE_SCATTER: a.in_place = (r == s + (long long)c->rank * count * esz); s += done * esz; r += done * esz; break;
-        default: a.in_place = (s == r); break;
-      }
-      if (d.coll == COLL_REDUCE && c->rank != d.root) a.in_place = false;
+      const char* s; char* r;
+      const CollArgs a = part_of(i, done, cur, &s, &r);
       const ProgEntry* pe = nullptr;
       rc = get_program(c, a, stream, &pe); if (rc) break;
       if (i == 0) {

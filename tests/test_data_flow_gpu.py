@@ -118,3 +118,26 @@ def test_checks_of_the_debug_mode_pass(monkeypatch):
         monkeypatch.undo()
         g._lib.piccl_env_reload()
         g.close()
+
+
+@pytest.mark.parametrize("coll", ["allreduce", "reduce"])
+def test_capture_with_other_buffers_than_the_first_call(coll):
+    """The first call's buffers are apart; in the captured one a rank receives into another's send buffer (the ring's sums contain what they overwrite).  The ranks' programs are there although the data flow ran."""
+    n, count = 4, 300000
+    g = _group(n)
+    xs = [torch.randint(-100, 100, (count,), generator=torch.Generator(device="cuda").manual_seed(r), device="cuda").float() for r in range(n)]
+    want = [torch.zeros(count, device="cuda") for _ in range(n)]
+    flows = g._lib.piccl_test_flow_calls(g._hs[0])
+    g.run(coll, xs, want, count, algo="RING", root=1)
+    assert g._lib.piccl_test_flow_calls(g._hs[0]) == flows + 1
+    ys = [x.clone() for x in xs]
+    outs = [torch.zeros(count, device="cuda") for _ in range(n)]
+    outs[0 if coll == "allreduce" else 1] = ys[1 if coll == "allreduce" else 2]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        g.run(coll, ys, outs, count, algo="RING", root=1)
+    assert g._lib.piccl_test_flow_calls(g._hs[0]) == flows + 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert g.status().aborted == 0 and torch.equal(outs[1], want[1])
+    g.close()
