@@ -242,7 +242,7 @@ int piccl_comm_destroy(piccl_comm_t* c) {
             s.calls[0], s.calls[1], s.calls[2], s.calls[3], s.calls[4], s.launches, s.program_cache_hits, s.program_cache_misses, s.fallbacks, s.timeouts);
   }
   for (int p = 0; p < c->nranks; p++) if (c->ipc_opened[p]) cudaIpcCloseMemHandle(c->h_ctx.heap[p]);
-  for (auto& ch : c->chunks) { cudaFree(ch.dev); cudaFreeHost(ch.host); }
+  for (auto* chunks : {&c->chunks, &c->flow_chunks}) for (auto& ch : *chunks) { cudaFree(ch.dev); cudaFreeHost(ch.host); }
   for (auto& kv : c->cache) if (kv.second.ready) cudaEventDestroy(kv.second.ready);
   for (auto& t : c->trace) { if (t.start) cudaEventDestroy(t.start); if (t.stop) cudaEventDestroy(t.stop); }
   if (c->d_tp_status) cudaFree(c->d_tp_status);
@@ -286,17 +286,24 @@ namespace piccl {
 
 struct CallDesc { Coll coll; const void* send; void* recv; size_t count; int dtype, op, root; Algo algo; int k; };
 
+// What is uploaded is kept for the life of the communicator (kernels in flight may read it): programs and data flows may take this much each.
+constexpr size_t kKeptBytes = (size_t)256 << 20;
+static size_t held(const std::vector<ProgChunk>& chunks) {
+  size_t n = 0;
+  for (const auto& ch : chunks) n += ch.cap;
+  return n;
+}
 // `bytes` of `data` on the device; they stay as long as the communicator.
-static int upload(piccl_comm* c, const void* data, size_t data_bytes, size_t bytes, cudaStream_t stream, ProgEntry& e, const void** dev) {
+static int upload(std::vector<ProgChunk>& chunks, const void* data, size_t data_bytes, size_t bytes, cudaStream_t stream, ProgEntry& e, const void** dev) {
   bytes = (bytes + 255) / 256 * 256;
-  if (c->chunks.empty() || c->chunks.back().used + bytes > c->chunks.back().cap) {
+  if (chunks.empty() || chunks.back().used + bytes > chunks.back().cap) {
     ProgChunk ch; ch.cap = std::max<size_t>(1 << 20, bytes); ch.used = 0;
     CUDA_TRY(cudaMalloc(&ch.dev, ch.cap));
     cudaError_t er = cudaHostAlloc(&ch.host, ch.cap, cudaHostAllocDefault);
     if (er != cudaSuccess) { cudaFree(ch.dev); return fail(PICCL_CUDA_ERROR, "cudaHostAlloc: %s", cudaGetErrorString(er)); }
-    c->chunks.push_back(ch);
+    chunks.push_back(ch);
   }
-  ProgChunk& ch = c->chunks.back();
+  ProgChunk& ch = chunks.back();
   memcpy(ch.host + ch.used, data, data_bytes);
   *dev = ch.dev + ch.used; e.origin = stream; e.synced = false;
   if (data_bytes) CUDA_TRY(cudaMemcpyAsync(ch.dev + ch.used, ch.host + ch.used, data_bytes, cudaMemcpyHostToDevice, stream));
@@ -307,7 +314,7 @@ static int upload(piccl_comm* c, const void* data, size_t data_bytes, size_t byt
 }
 static int upload_program(piccl_comm* c, const Program& p, cudaStream_t stream, ProgEntry& e) {
   const void* dev = nullptr;
-  const int rc = upload(c, p.actions.data(), p.actions.size() * sizeof(Action), std::max<size_t>(p.actions.size(), 1) * sizeof(Action), stream, e, &dev);
+  const int rc = upload(c->chunks, p.actions.data(), p.actions.size() * sizeof(Action), std::max<size_t>(p.actions.size(), 1) * sizeof(Action), stream, e, &dev);
   e.dev = static_cast<const Action*>(dev); e.n_actions = (int)p.actions.size(); e.scratch_elems = p.scratch_elems;
   return rc;
 }
@@ -356,12 +363,9 @@ static int get_program(piccl_comm* c, const CollArgs& a, cudaStream_t stream, co
       return fail(PICCL_UNSUPPORTED, "%s %s of %lld elements was never run outside a stream capture: its program cannot be built while capturing", coll_name(a.coll), algo_name(a.algo), a.count);
     }
     cudaGetLastError();
-    // programs are kept for the life of the communicator (kernels in flight may read them): bound what they may take
-    size_t held = 0;
-    for (const auto& ch : c->chunks) held += ch.cap;
-    if (held > ((size_t)256 << 20)) {
+    if (held(c->chunks) > kKeptBytes) {
       c->stats.fallbacks++;
-      return fail(PICCL_UNSUPPORTED, "program cache full (%zu MiB for %zu distinct calls)", held >> 20, c->cache.size());
+      return fail(PICCL_UNSUPPORTED, "program cache full (%zu MiB for %zu distinct calls)", held(c->chunks) >> 20, c->cache.size());
     }
     c->stats.program_cache_misses++;
     Program p = compile(a, c->rank);
@@ -575,9 +579,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
     std::lock_guard<std::mutex> l(c0->mu);
     auto it = c0->cache.find(k);
     if (it == c0->cache.end()) {
-      size_t held = 0;
-      for (const auto& ch : c0->chunks) held += ch.cap;
-      if (capturing || held > ((size_t)256 << 20)) return PICCL_UNSUPPORTED;      // (the programs' path says why)
+      if (capturing || held(c0->flow_chunks) > kKeptBytes) return PICCL_UNSUPPORTED;      // (the programs, which take a fraction of the room, or what their path says)
       std::vector<Program> progs;
       for (int r = 0; r < n; r++) progs.push_back(compile(a, r));
       std::vector<FlowOp> ops;
@@ -592,7 +594,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
         x.n_ops = (int)ops.size();
       }
       const void* dev = nullptr;
-      if (int rc = upload(c0, ops.data(), ops.size() * sizeof(FlowOp), std::max<size_t>(1, ops.size()) * sizeof(FlowOp), stream, x, &dev)) return rc;
+      if (int rc = upload(c0->flow_chunks, ops.data(), ops.size() * sizeof(FlowOp), std::max<size_t>(1, ops.size()) * sizeof(FlowOp), stream, x, &dev)) return rc;
       x.ops = static_cast<const FlowOp*>(dev);
       it = c0->cache.emplace(k, x).first;
       *fresh = true;

@@ -69,7 +69,7 @@ struct piccl_comm {
   long long ll_max_bytes = 0;          // largest message the low-latency path takes (0: off)
   piccl_stats_t stats{};
   std::unordered_map<piccl::ProgKey, piccl::ProgEntry, piccl::ProgKeyHash> cache;
-  std::vector<piccl::ProgChunk> chunks;
+  std::vector<piccl::ProgChunk> chunks, flow_chunks;      // of programs; of data flows
   std::vector<piccl::LLPlan> ll_plans;                                                     // bounded, see comm.cu
   std::unordered_map<piccl::ProgKey, long long, piccl::ProgKeyHash> scratch_need;          // scratch elements of a reduce-scatter by its arguments
   std::vector<piccl::TraceRec> trace;

@@ -141,3 +141,27 @@ def test_capture_with_other_buffers_than_the_first_call(coll):
     torch.cuda.synchronize()
     assert g.status().aborted == 0 and torch.equal(outs[1], want[1])
     g.close()
+
+
+def test_programs_take_over_when_data_flows_are_full():
+    """Data flows are kept up to 256 MiB, about 11 KB for an all-gather among eight ranks.  Programs, which have room of their own, run what comes then; what is kept runs on."""
+    n, most = 8, 26000
+    g = _group(n)
+    flows = lambda: g._lib.piccl_test_flow_calls(g._hs[0])
+    xs = [torch.full((most,), r, device="cuda", dtype=torch.uint8) for r in range(n)]
+    outs = [torch.zeros(n * most, device="cuda", dtype=torch.uint8) for _ in range(n)]
+    for count in range(1, most + 1):
+        before = flows()
+        g.run("allgather", xs, outs, count, algo="RING")
+        if flows() == before:
+            break
+    assert 20000 < count < most, count
+    for c, kept in ((count, False), (count + 1, False), (100, True)):
+        for o in outs:
+            o.zero_()
+        before = flows()
+        g.run("allgather", xs, outs, c, algo="RING")
+        torch.cuda.synchronize()
+        assert g.status().aborted == 0 and flows() == before + kept
+        assert all(torch.equal(o[:n * c].view(n, c).amin(1), o[:n * c].view(n, c).amax(1)) and o[:n * c:c].tolist() == list(range(n)) for o in outs)
+    g.close()
