@@ -94,9 +94,13 @@ def lib() -> C.CDLL:
 
 
 def fastcall():
-    """The module that calls the library with lists of tensors (src/python/fastcall.cc)."""
+    """The module that calls the library with lists of tensors (src/python/fastcall.cc); None where it could not be built for want of Python's headers."""
     with _lock:
         if "fastcall" not in _libs:
+            from . import build as _build
+            if not (_LIB_DIR / "_fastcall.so").exists() and _build.python_headers() is None:
+                _libs["fastcall"] = None
+                return None
             spec = importlib.util.spec_from_file_location("_fastcall", _ensure_built("_fastcall.so"))
             _libs["fastcall"] = importlib.util.module_from_spec(spec)
             spec.loader.exec_module(_libs["fastcall"])

@@ -3,7 +3,7 @@
   piccl_b200/lib/piccl.so        collectives library + NCCL-ABI preload shim + fused TP kernels
   piccl_b200/lib/libpiccl_ops.so model kernels (tcgen05 GEMM, layer norm, cross entropy, AdamW, ...)
   piccl_b200/lib/libpiccl_model.so native training step (launches the kernels of libpiccl_ops.so; attention partly through ATen)
-  piccl_b200/lib/_fastcall.so    calls with lists of tensors for the Python front end
+  piccl_b200/lib/_fastcall.so    calls with lists of tensors for the Python front end (where Python's headers are installed)
   piccl_b200/lib/piccl_sched     schedule dump / validation command line tool
   piccl_b200/lib/coll_bench      OSU-style collective benchmark (fork per GPU, no MPI)
   piccl_b200/lib/loggp_bench     PRTT measurements between two GPUs (input of tools/loggp_param)
@@ -45,8 +45,14 @@ def _sources(*patterns: str) -> list[Path]:
     return out
 
 
+def python_headers() -> Path | None:
+    """Python's development headers, which only _fastcall.so needs (None: not installed, calls then go through ctypes)."""
+    inc = Path(sysconfig.get_paths()["include"])
+    return inc if (inc / "Python.h").exists() else None
+
+
 def targets() -> dict[str, dict]:
-    return {
+    plan = {
         "piccl.so": {
             "src": _sources("coll/*.cc", "runtime/*.cc", "runtime/*.cu", "kernels/*.cu", "tp/*.cu", "piccl.cc"),
             "link": ["-shared", "-cudart", "static", "-ldl", "-lpthread", "-lrt"],
@@ -62,11 +68,6 @@ def targets() -> dict[str, dict]:
             "link": ["-shared", "-cudart", "none", f"-L{OUT}", "-lpiccl_ops", f"-L{TORCH / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
                      "-Xlinker", "-rpath,$ORIGIN", "-Xlinker", f"-rpath,{TORCH / 'lib'}"],
         },
-        "_fastcall.so": {
-            "src": _sources("python/*.cc"),
-            "flags": [f"-I{sysconfig.get_paths()['include']}"],
-            "link": ["-shared", "-cudart", "none"],
-        },
         "piccl_sched": {
             "src": _sources("coll/*.cc", "tools/piccl_sched.cc"),
             "link": [],
@@ -80,6 +81,9 @@ def targets() -> dict[str, dict]:
             "link": ["-cudart", "static", "-ldl", "-lpthread", "-lrt", "-L/usr/lib/x86_64-linux-gnu", "-lnccl", "-Xcompiler", "-rdynamic"],
         },
     }
+    if inc := python_headers():
+        plan["_fastcall.so"] = {"src": _sources("python/*.cc"), "flags": [f"-I{inc}"], "link": ["-shared", "-cudart", "none"]}
+    return plan
 
 
 def _newer(a: Path, b: Path) -> bool:

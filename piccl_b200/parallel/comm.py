@@ -155,7 +155,7 @@ class Communicator(_CommBase):
 class LoopbackGroup(_CommBase):
     """`nranks` virtual ranks on one device; every collective is one launch."""
 
-    _collective = None           # the native call (src/python/fastcall.cc); without it, as with a stand-in for the library, the call goes through ctypes
+    _collective = None           # the native call (src/python/fastcall.cc); without it the call goes through ctypes
 
     def __init__(self, nranks: int, device: Optional[int] = None, config: Optional[N.Config] = None):
         super().__init__()
@@ -165,7 +165,8 @@ class LoopbackGroup(_CommBase):
         self._hs = []
         self._comms = None
         self._pack = struct.Struct(f"{nranks}Q").pack
-        self._collective, self._entry = N.fastcall().collective, N.address(self._lib.piccl_group_collective)
+        if (fast := N.fastcall()) is not None:
+            self._collective, self._entry = fast.collective, N.address(self._lib.piccl_group_collective)
         blobs = []
         for r in range(nranks):
             h = C.c_void_p()
@@ -185,8 +186,7 @@ class LoopbackGroup(_CommBase):
         if self._collective is not None:
             rc = self._collective(self._entry, self.handles(), self.nranks, send, recv, count, N.COLL[coll], _dt(send[0]), N.OP[op], root, _algo(algo), k, _stream_ptr(stream))
         else:
-            rc = self._lib.piccl_group_collective(self.handles(), self.nranks, N.COLL[coll], self._pack(*[t.data_ptr() for t in send]), self._pack(*[0 if t is None else t.data_ptr() for t in recv]), count,
-                                                  _dt(send[0]), N.OP[op], root, _algo(algo), k, _stream_ptr(stream))
+            rc = self._lib.piccl_group_collective(self.handles(), self.nranks, N.COLL[coll], self._pack(*[t.data_ptr() for t in send]), self.table(recv), count, _dt(send[0]), N.OP[op], root, _algo(algo), k, _stream_ptr(stream))
         if rc:
             N.check(rc, f"piccl_group_collective({coll})")
 
@@ -196,6 +196,9 @@ class LoopbackGroup(_CommBase):
         if self._comms is None:
             self._comms = self._pack(*[h.value for h in self._hs])
         return self._comms
+
+    def table(self, tensors: Sequence[Optional[torch.Tensor]]) -> bytes:      # None: a rank that receives nothing
+        return self._pack(*[0 if t is None else t.data_ptr() for t in tensors])
 
     def slots_only(self, on: bool = True) -> "LoopbackGroup":
         """Everything that crosses goes through the ranks' slots and workspaces, as between GPUs, although one launch carries all ranks."""

@@ -73,7 +73,11 @@ def _entry(lib, fn_name: str) -> int:
 
 def _group(fn_name, g: LoopbackGroup, As, Bs, outs, M, N_, K, stream):
     lib = _declare()
-    rc = N.fastcall().product(_entry(lib, fn_name), g.handles(), g.nranks, As, Bs, outs, M, N_, K, _stream_ptr(stream))
+    fast = N.fastcall()
+    if fast is not None:
+        rc = fast.product(_entry(lib, fn_name), g.handles(), g.nranks, As, Bs, outs, M, N_, K, _stream_ptr(stream))
+    else:
+        rc = getattr(lib, fn_name)(g.handles(), g.nranks, g.table(As), g.table(Bs), g.table(outs), M, N_, K, _stream_ptr(stream))
     if rc:
         N.check(rc, fn_name)
 

@@ -165,3 +165,21 @@ def test_programs_take_over_when_data_flows_are_full():
         assert g.status().aborted == 0 and flows() == before + kept
         assert all(torch.equal(o[:n * c].view(n, c).amin(1), o[:n * c].view(n, c).amax(1)) and o[:n * c:c].tolist() == list(range(n)) for o in outs)
     g.close()
+
+
+def test_groups_without_the_native_call_path(monkeypatch):
+    """As where Python's headers are missing: collectives and products go through ctypes."""
+    from piccl_b200 import _native as N
+    from piccl_b200.parallel import tp
+    from piccl_b200.parallel.comm import LoopbackGroup, make_config
+    monkeypatch.setattr(N, "fastcall", lambda: None)
+    g = LoopbackGroup(2, config=make_config(scratch_bytes=1 << 20, timeout_ms=5000, tp_bytes=tp.workspace_bytes("gemm_rs", 2, 256, 256, 64)))
+    xs = [torch.full((5000,), float(r + 1), device="cuda") for r in range(2)]
+    outs = [torch.zeros(5000, device="cuda"), None]
+    g.run("reduce", xs, outs, 5000, root=0)
+    a = [torch.ones(256, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    c = [torch.zeros(128, 256, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    tp.gemm_rs_group(g, a, a, c)
+    torch.cuda.synchronize()
+    assert g.status().aborted == 0 and torch.all(outs[0] == 3.0) and all(torch.all(x == 128.0) for x in c)
+    g.close()
