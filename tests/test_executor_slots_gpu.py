@@ -12,8 +12,7 @@ def through_the_slots():
     class SlotsOnly(comm.LoopbackGroup):
         def __init__(self, *a, **kw):
             super().__init__(*a, **kw)
-            for h in self._hs:
-                self._lib.piccl_test_slots_only(h, 1)
+            self.slots_only()
     with pytest.MonkeyPatch.context() as m:
         m.setattr(comm, "LoopbackGroup", SlotsOnly)
         yield

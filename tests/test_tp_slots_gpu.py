@@ -6,20 +6,16 @@ from test_tp_gpu import *      # noqa: F401,F403
 from test_tp_gpu import _bf, _group, pytestmark      # noqa: F401
 
 
-@pytest.fixture
-def through_the_workspace(monkeypatch):
+@pytest.fixture(autouse=True)
+def through_the_workspace(request, monkeypatch):
     from piccl_b200.parallel import comm
 
     class SlotsOnly(comm.LoopbackGroup):
         def __init__(self, *a, **kw):
             super().__init__(*a, **kw)
-            for h in self._hs:
-                self._lib.piccl_test_slots_only(h, 1)
-    monkeypatch.setattr(comm, "LoopbackGroup", SlotsOnly)
-
-
-for _name in [n for n in dir() if n.startswith("test_")]:
-    globals()[_name] = pytest.mark.usefixtures("through_the_workspace")(globals()[_name])
+            self.slots_only()
+    if request.function is not test_all_ranks_in_one_launch:
+        monkeypatch.setattr(comm, "LoopbackGroup", SlotsOnly)
 
 
 # Tiles of 256, 128 and 64 columns by the number of tiles; one, an odd and an even number of row blocks to a rank, more tiles than pairs of CTAs, one k-block to a rank.
@@ -52,8 +48,7 @@ def test_all_ranks_in_one_launch(which, n, blocks, N, K):
     for r in range(n):
         err = (outs[r].double() - want[r]).abs()
         assert (err <= want[r].abs() * 2.0 ** -8 + n * K * 2.0 ** -20).all(), (r, err.max().item())
-    for h in g._hs:
-        g._lib.piccl_test_slots_only(h, 1)
+    g.slots_only()
     for r, o in enumerate(run()):
         assert (o.double() - want[r]).norm() <= 2.0 ** -6 * want[r].norm()
         if not rs:
