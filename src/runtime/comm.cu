@@ -587,7 +587,7 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
       if (data_flow(progs, ops, kind)) {
         if (env().debug) if (const char* why = check_flow(ops, a)) return fail(PICCL_INTERNAL_ERROR, "data flow check failed (%s %s): %s", coll_name(a.coll), algo_name(a.algo), why);
         for (const FlowOp& o : ops) {
-          x.most = std::max<long long>(x.most, o.count);
+          x.most = std::max<long long>(x.most, o.count); x.leaves = std::max<int>(x.leaves, o.n_leaf);
           for (int i = 0; i < o.n_leaf; i++) x.offsets_aligned &= o.leaf_off[i] * esz % 16 == 0;
           for (int i = 0; i < o.n_dst; i++) x.offsets_aligned &= o.dst_off[i] * esz % 16 == 0;
         }
@@ -614,6 +614,12 @@ static int run_flow(piccl_comm** comms, int n, const CallDesc* calls, long long 
   for (int i = 0; i < n; i++) {
     fa.in[i] = calls[i].send; fa.out[i] = calls[i].recv;
     aligned &= ((reinterpret_cast<uintptr_t>(calls[i].send) | reinterpret_cast<uintptr_t>(calls[i].recv)) & 15) == 0;
+  }
+  // Small sums at odd addresses, whose code takes longer to fetch than their data: those that the low-latency kernels make in one launch too stay with them.  us there and as a data flow: all-reduce of
+  // 20 KB of fp16 among four ranks 6.6 / 8.1, among eight 7.5 / 13.8, of 80 KB 12.3 / 13.9 (160 KB 26.7 / 13.9, four ranks 9.2 / 8.2); reduce of 300 bytes of bf16 among eight in two rings 8.2 / 10.4, of 14 KB 8.9 / 11.2
+  // (40 KB in fours 12.4 / 8.5; up to four ranks 7.4 / 5.0).  (A captured call has nothing else that could run.)
+  if (!aligned && !capturing && ((ll && e->leaves >= 4 && count * esz <= 98304) || (d0.coll == COLL_REDUCE && e->leaves > 4 && count * esz <= 16384))) return PICCL_UNSUPPORTED;
+  for (int i = 0; i < n; i++) {
     std::lock_guard<std::mutex> l(comms[i]->mu);
     comms[i]->stats.launches++;
     skip |= fault_now(comms[i]); comms[i]->call_index++;

@@ -34,7 +34,7 @@ struct ProgKeyHash {
     return (size_t)h;
   }
 };
-struct ProgEntry { const Action* dev = nullptr; int n_actions = 0; const FlowOp* ops = nullptr; int n_ops = 0; long long most = 0 /* elements of its largest operation */; long long scratch_elems = 0; cudaEvent_t ready = nullptr; cudaStream_t origin = nullptr; bool synced = false, offsets_aligned = true /* all offsets into user buffers are multiples of 16 bytes */; };
+struct ProgEntry { const Action* dev = nullptr; int n_actions = 0; const FlowOp* ops = nullptr; int n_ops = 0; long long most = 0 /* elements of its largest operation */; int leaves = 0 /* most operands of one */; long long scratch_elems = 0; cudaEvent_t ready = nullptr; cudaStream_t origin = nullptr; bool synced = false, offsets_aligned = true /* all offsets into user buffers are multiples of 16 bytes */; };
 struct ProgChunk { char* dev = nullptr; char* host = nullptr; size_t cap = 0, used = 0; };
 
 // What a low-latency all-reduce of one algorithm and radix looks like for the communicators of a launch: the arguments that do not

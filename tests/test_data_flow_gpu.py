@@ -183,3 +183,24 @@ def test_groups_without_the_native_call_path(monkeypatch):
     torch.cuda.synchronize()
     assert g.status().aborted == 0 and torch.all(outs[0] == 3.0) and all(torch.all(x == 128.0) for x in c)
     g.close()
+
+
+@pytest.mark.parametrize("coll,n,algo,small,large", [("allreduce", 4, "RD", 10001, 60001), ("allreduce", 8, "PRM", 49152, 49153), ("reduce", 8, "K_RING", 8192, 8193)])
+def test_small_sums_at_odd_addresses(coll, n, algo, small, large):
+    """They stay with the low-latency kernels up to the lines in run_flow, are captured as data flows all the same, and are the same bits whichever runs; two-byte elements, one element into their buffers."""
+    g = _group(n)
+    flows = lambda: g._lib.piccl_test_flow_calls(g._hs[0])
+    for count, flow in ((small, 0), (large, 1)):
+        xs = [torch.rand(count + 1, generator=torch.Generator(device="cuda").manual_seed(r), device="cuda").to(torch.bfloat16)[1:] for r in range(n)]
+        outs = [[torch.zeros(count + 1, device="cuda", dtype=torch.bfloat16)[1:] for _ in range(n)] for _ in range(2)]
+        before = flows()
+        g.run(coll, xs, outs[0], count, algo=algo, k=2, root=1)
+        assert flows() == before + flow
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            g.run(coll, xs, outs[1], count, algo=algo, k=2, root=1)
+        assert flows() == before + flow + 1
+        graph.replay()
+        torch.cuda.synchronize()
+        assert g.status().aborted == 0 and all(torch.equal(x, y) for x, y in zip(*outs))
+    g.close()
