@@ -3,12 +3,13 @@
 // A program says which operands are combined where, in which order, and through which slots the values travel.  Between GPUs that way is the point; on one GPU it is
 // several passes over memory for each hop.  `data_flow` follows the entries of all ranks' programs back and keeps what they compute: each element of a
 // receive buffer as an expression over the send buffers, with the operands of each action in its order and each partial result rounded to the element type where it would
-// have been put into a slot, so that the results are bit for bit those of the programs.  (But for bf16 averages among 2, 4 or 8 ranks of elements whose share is
+// have been put into a slot, so that the results are bit for bit those of the programs,
+// or of the low-latency kernel that a small call would take.  (But for bf16 averages among 2, 4 or 8 ranks of elements whose share is
 // below 2^-126, its normal range: such shares are not rounded on their way.)  A sum that one rank makes and others receive, or that several ranks make alike, is
 // computed once and stored in all their buffers.  Nothing in such a call waits (kernels/exec_flow.cuh).
 //
 // us through the slots and this, one B200: all-reduce 4 x 25 MiB averaged by recursive doubling 131 / 38, 8 x 64 MiB on the ring 353 / 188, 8 x 280 KB 45 / 4.8, 8 x 4 KB 37 / 4.7; all-gather 4 x 1 MiB at
-// odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34; broadcast 8 x 16 MiB 110 / 27; 8 x 8 MiB 196 / 98; reduce 8 x 16 MiB on the ring 92 / 28, in two rings 120 / 56.
+// odd addresses 28.7 / 10.3, 8 x 8 MiB 195 / 98; reduce-scatter 2 x 32 MiB 55.5 / 34, 8 x 8 MiB on the ring 195 / 94; broadcast 8 x 16 MiB 103 / 27; reduce 8 x 16 MiB on the ring 92 / 28, in two rings 120 / 56.
 #include <algorithm>
 #include <array>
 #include <map>

@@ -441,19 +441,27 @@ __device__ __forceinline__ void reduce_copy_shift(int nt, int nsrc, const char* 
 }
 
 // Element-wise path: the last, partial pack of an action, an operand after the other.  (A data flow's has all operands on their way first, exec_flow.cuh.  In this kernel that form, which needs a register
-// for each operand, makes the loops above slower although it hardly ever runs: reduce of 8 x 16 MiB in two rings 111 us, with it 123, in rings of four 101 and 110; 8 x 52 MiB of fp64 averaged by DIRECT 267 and 292.)
+// for each operand, makes the loops above slower although it hardly ever runs: reduce of 8 x 16 MiB in two rings 111 us, with it 123, in rings of four 101 and 110; 8 x 52 MiB of fp64 averaged by DIRECT 267 and 292.
+// With bytes it is the other way round: maximum of 8 x 4 MiB on the ring 73.7, with it 69.9.)
 template <typename T, int OP>
 __device__ __noinline__ void reduce_copy_elem(int nt, int nsrc, const char* const* src, int local_src, int ndst, char* const* dst,
                                                  long long first, long long nelem, bool do_scale, float scale) {
   typedef typename AccOf<T>::type A;
   for (long long i = first + threadIdx.x; i < nelem; i += nt) {
+    auto load = [&](int s) { const T* const p = reinterpret_cast<const T*>(src[s]) + i; return local_src == s ? *p : *reinterpret_cast<const volatile T*>(p); };
     A acc = A();
-    for (int s = 0; s < nsrc; s++) {
-      const T* p = reinterpret_cast<const T*>(src[s]) + i;
-      const T raw = local_src == s ? *p : *reinterpret_cast<const volatile T*>(p);
-      A x = Cvt<T>::up(raw);
-      if (do_scale && local_src == s) x = scale_val<A>(x, scale);
-      acc = s == 0 ? x : red<OP, A>(acc, x);
+    if constexpr (sizeof(T) == 1) {
+      T raw[kMaxActionPeers + 1];
+#pragma unroll
+      for (int s = 0; s < kMaxActionPeers + 1; s++) if (s < nsrc) raw[s] = load(s);
+#pragma unroll
+      for (int s = 0; s < kMaxActionPeers + 1; s++) if (s < nsrc) { const A x = Cvt<T>::up(raw[s]); acc = s == 0 ? x : red<OP, A>(acc, x); }
+    } else {
+      for (int s = 0; s < nsrc; s++) {
+        A x = Cvt<T>::up(load(s));
+        if (do_scale && local_src == s) x = scale_val<A>(x, scale);
+        acc = s == 0 ? x : red<OP, A>(acc, x);
+      }
     }
     const T o = Cvt<T>::down(acc);
     for (int d = 0; d < ndst; d++) reinterpret_cast<T*>(dst[d])[i] = o;

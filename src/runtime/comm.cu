@@ -672,9 +672,10 @@ static int run(piccl_comm** comms, int n, const CallDesc* calls, cudaStream_t st
                    : (reducing ? exec_kernel_for(d0.dtype, op) : exec_copy_kernel());
   if (!fn) return fail(PICCL_INTERNAL_ERROR, "no kernel for dtype %d op %d", d0.dtype, op);
 
-  // All ranks in this launch: the call's data flow, where neither a way between the ranks (PICCL_PROTO, the persistent server, the switch) nor a size of the grid (PICCL_MIN_GRID_SIZE, PICCL_MAX_GRID_SIZE) is asked for by name.  Among eight ranks the low-latency kernels, which are cooperative launches, take 8.2 us for an
-  // all-reduce of 64 KiB and for an all-gather of 4 KiB blocks, the data flow 4.9.  At 1 KiB the all-reduce takes 5.9 and 5.1: up to 16 KiB (both ends of a launch, little more) an exchange asked
-  // for by its algorithm stays on the kernel that is made for it.
+  // All ranks in this launch: the call's data flow, where neither a way between the ranks (PICCL_PROTO, the persistent server, the switch) nor a size of the grid (PICCL_MIN_GRID_SIZE,
+  // PICCL_MAX_GRID_SIZE) is asked for by name.  Among eight ranks the low-latency kernels, which are cooperative launches, take 8.2 us for an all-reduce of 64 KiB and for an all-gather of 4 KiB
+  // blocks, the data flow 4.9.  An exchange of up to 16 KiB would gain as much (1 KiB 5.9 and 5.1, 4 KiB one after the other 8.2 and 4.9): there the kernel that one rank per GPU runs at these sizes
+  // has been kept, so that programs and tests of one GPU run it too.
   constexpr long long kOwnKernelBytes = 16384;
   const Env& ev = env();
   const bool flows = ev.proto == 0 && !ev.launch_persistent && !ev.min_grid_set && !ev.max_grid_set && d0.algo != ALGO_NVLS && may_flow(comms, n, calls, (long long)d0.count * esz_real);
