@@ -113,8 +113,9 @@ int piccl_group_collective(piccl_comm_t** comms, int ncomms, int coll, const voi
  * piccl_gemm_rs:  out[M/n, N] = rows [rank*M/n, (rank+1)*M/n) of  sum_r A_r[M, K_local] * B_r[N, K_local]^T
  * piccl_ag_gemm:  out[M, N_local] = concat_r(A_r[M/n, K]) * B[N_local, K]^T
  * The *_group variants run several communicators of this process (virtual ranks on one device) as a
- * single launch; with all ranks in it, and results apart from operands, operands are read where they are
- * (but in a gemm_rs of few tiles and a long k, where the exchange is faster outside a stream capture). */
+ * single launch; with all ranks in it, and results apart from operands, operands are read where they are,
+ * and a gemm_rs rounds its sums once where exchanged partial tiles are rounded each (but in a gemm_rs of few
+ * tiles and a long k the exchange is faster, and is what runs outside a stream capture). */
 long long piccl_tp_workspace_bytes(int which /*0 gemm_rs, 1 ag_gemm*/, int nranks, int M, int N, int K);
 /* Bytes [begin, end) of the 1 MiB flag area that a call of this shape uses, by the parity of the kernel's call count. */
 int piccl_tp_flag_range(int which, int nranks, int M, int N, int parity, long long* begin, long long* end);
